@@ -7,17 +7,23 @@
 //                            (tcgen05.ld), so max / sum need no shuffles; P_t goes back to TMEM as
 //                            packed bf16 pairs (tcgen05.st)
 //     O_t (+)= P_t V         tcgen05.mma with the A operand in TMEM, 128 x d x 128, V is the MN-major
-//                            B operand as it sits in memory
+//                            B operand as it sits in memory; issued in two halves of 64 keys, the
+//                            first while the exponentials of the second are still being computed
 // P never touches shared memory: with P staged there the kernel was bound by shared-memory
-// bandwidth (128 B/clk: the P stores, the A-operand reads of P V and of Q K^T, the TMA writes),
-// measured as tcgen05.mma issue blocking for 400 / 620 cycles per S / P V group at head_dim 64.
+// bandwidth (128 B/clk: the P stores, the A-operand reads of P V and of Q K^T, the TMA writes).
 // O_t stays in TMEM for the whole key loop; when a row maximum grows the softmax threads rescale
 // it in place (tcgen05.ld / st) before the next P V is issued.
 // Warp roles (384 threads): warp 0 TMA producer, warps 1 / 2 MMA issuers of tile 0 / 1 (warp 1
 // owns the TMEM allocation), warp 3 idle, warps 4-7 softmax of tile 0, warps 8-11 softmax of tile 1.
 // The two tiles run half a period apart (tile 1 starts late on purpose): the exponentials of one
-// then overlap the loads, maxima and waits of the other instead of queueing on the same MUFU unit.  While one tile is in softmax the tensor pipe
-// works on the other.  Layout / masking conventions are those of flash_attn.cu.
+// then overlap the loads, maxima and waits of the other instead of queueing on the same MUFU unit.
+// What bounds it: 16 exponentials per clock per SM are 1024 cycles per 128x128 block against 542 (d = 64)
+// or 1020 (d = 128) cycles of tensor pipe; a tile's softmax, P V and next S follow one another, and two tiles leave
+// gaps on both units.  Measured before / after P left shared memory at d = 128, P V was split and the longest tiles of
+// all heads came first: B8 S2048 32q/4kv d64 286 / 267 us, B1 S8192 32q/8kv d128 644 / 575, B3 S1531 32q/8kv d128 111 / 102.  Scaling and summing use two-wide fp32 instructions and the maximum three-input ones.
+// (A polynomial on the FMA pipe for one pair of exponentials in four was measured slower: 663 against 576 us at B1 S8192
+// 32q/8kv d128, 274 against 266 us at B8 S2048 32q/4kv d64.)
+// Layout / masking conventions are those of flash_attn.cu.
 // All waits are bounded; on expiry a status word is set and the CTA drains and frees its TMEM.
 #include <string.h>
 #include "tcgen05.cuh"
@@ -66,52 +72,44 @@ struct FaFwdParams {
   const unsigned int* kv_flags;  // null, or this rank's block counters [B][kv_brows / 128]
   unsigned int flag_target;
   int tiles_x;                   // query tiles (256 rows) per (batch, head)
+  int group;                     // (batch, head) pairs whose tiles are ordered together
   unsigned long long wait_ns;    // limit of a wait on a key block's arrival flag
 };
 
-// 2^x on the FMA pipe: round to the nearest integer with the 1.5 * 2^23 trick, a degree-4 polynomial
-// for the fraction in [-0.5, 0.5] (relative error 6e-5, far below the bf16 rounding of P), and
-// the integer part added to the exponent field.  Inputs below -126 (masked scores are -inf) give ~0.
-__device__ __forceinline__ float exp2_poly(float x) {
-  x = fmaxf(x, -126.f);
-  const float t = x + 12582912.f;
-  const float f = x - (t - 12582912.f);
-  float p = fmaf(f, 9.6181291e-3f, 5.5504109e-2f);
-  p = fmaf(p, f, 2.4022651e-1f);
-  p = fmaf(p, f, 6.9314718e-1f);
-  p = fmaf(p, f, 1.0f);
-  return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
+// Three-input maximum; a NaN in any input is the result.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.NaN.ftz.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
-// Off by default: measured at B8 S2048 32q/4kv d64, every 2nd / 4th / 8th pair on the polynomial gave
-// 0.394 / 0.333 / 0.335 ms against 0.316 ms with the MUFU alone (the extra FMA-pipe instructions cost
-// more issue slots than the MUFU cycles they free).
-#ifndef LB_FA_POLY_EVERY
-#define LB_FA_POLY_EVERY 0
-#endif
+__device__ __forceinline__ float max2(float a, float b) {
+  float r;
+  asm("max.NaN.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 
 template <int D>
 struct FaCfg {
   static constexpr int BM = 128, BN = 128;
   static constexpr int KS = (D == 64) ? 3 : 2;
-  static constexpr int VS = (D == 64) ? 3 : 1;
+  static constexpr int VS = (D == 64) ? 3 : 2;
   static constexpr int ATOMS = D / 64;
   static constexpr int ATOM_BYTES = 128 * 128;          // 128 rows x 128 B
   static constexpr int TILE_BYTES = ATOMS * ATOM_BYTES; // one Q / K / V tile
   // TMEM columns: S_t fp32 [128], O_t fp32 [D], P_t packed bf16 [64].  With head_dim 64 all six
-  // regions fit in the 512 columns and P never touches shared memory.  With head_dim 128 S and O
-  // fill the 512 columns: P_t is staged in shared memory instead (letting P_t take columns of S_t
-  // was measured slower: S_t of the next key block then has to queue behind P_t V).
-  static constexpr bool P_TMEM = (D == 64);
-  static constexpr int COL_S = 0, COL_O = 256, COL_P = 384;
-  static constexpr int P_STRIDE = 64;
-  static constexpr int P_BYTES = 2 * ATOM_BYTES;        // 128 x 128 bf16 (shared-memory variant)
+  // regions fit in the 512 columns, and S of the next key block is issued as soon as the softmax
+  // threads hold the current one in registers.  With head_dim 128 S and O fill the 512 columns and
+  // P_t takes the first half of S_t's: the next S_t is then issued right behind P_t V (the tensor
+  // pipe runs the two in order), and the other tile's work fills the time of the softmax.
+  static constexpr bool P_ALIAS = (D == 128);
+  static constexpr int COL_S = 0, COL_O = 256, COL_P = P_ALIAS ? 0 : 384;
+  static constexpr int P_STRIDE = P_ALIAS ? 128 : 64;
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_K = OFF_Q + 2 * TILE_BYTES;
   static constexpr int OFF_V = OFF_K + KS * TILE_BYTES;
-  static constexpr int OFF_P = OFF_V + VS * TILE_BYTES;
-  static constexpr int OFF_BAR = OFF_P + (P_TMEM ? 0 : 2 * P_BYTES);
+  static constexpr int OFF_BAR = OFF_V + VS * TILE_BYTES;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
-  static constexpr int NBAR = 1 + 2 * KS + 2 * VS + 8;
+  static constexpr int NBAR = 1 + 2 * KS + 2 * VS + 10;
 };
 
 template <int D>
@@ -180,12 +178,19 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   auto p_full = [&](int t) { return bar1 + 8u * (2 + t); };
   auto pv_done = [&](int t) { return bar1 + 8u * (4 + t); };
   auto s_free = [&](int t) { return bar1 + 8u * (6 + t); };
+  auto p_half = [&](int t) { return bar1 + 8u * (8 + t); };     // first 64 keys of P are in TMEM
 
   // 1-D grid: movers first (they must be resident before anything waits for data), then the
-  // (query tile, head, batch) CTAs with the tile index fastest
+  // (batch, head, query tile) CTAs.  Causal tiles differ in length by up to the number of key blocks, so
+  // the longest tiles of all heads of a group start first and the short ones fill the tail; a group is as
+  // many heads as keep their K / V in L2 together (launch_fa_fwd).
   const int cid = (int)blockIdx.x - push.n_mov;
-  const int mblk = p.tiles_x - 1 - cid % p.tiles_x;   // late (long) causal rows first
-  const int h = (cid / p.tiles_x) % p.hq, b = cid / (p.tiles_x * p.hq);
+  const int grp = cid / (p.tiles_x * p.group);
+  const int in_grp = cid - grp * p.tiles_x * p.group;
+  const int gsize = min(p.group, p.hq * p.B - grp * p.group);
+  const int mblk = p.tiles_x - 1 - in_grp / gsize;
+  const int bh = grp * p.group + in_grp % gsize;
+  const int h = bh % p.hq, b = bh / p.hq;
   const int hk = h / (p.hq / p.hkv);
   const int m0 = mblk * 2 * C::BM;
   const int off = p.Sk - p.Sq;
@@ -206,7 +211,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     mbar_init(q_full, 1);
     for (int s = 0; s < C::KS; s++) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 2); }
     for (int s = 0; s < C::VS; s++) { mbar_init(v_full(s), 1); mbar_init(v_empty(s), 2); }
-    for (int t = 0; t < 2; t++) { mbar_init(s_full(t), 1); mbar_init(p_full(t), 128); mbar_init(pv_done(t), 1); mbar_init(s_free(t), 128); }
+    for (int t = 0; t < 2; t++) { mbar_init(s_full(t), 1); mbar_init(p_full(t), 128); mbar_init(pv_done(t), 1); mbar_init(s_free(t), 128); mbar_init(p_half(t), 128); }
     mbar_init_fence();
     prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv);
   }
@@ -217,17 +222,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   const uint32_t tmem_base = *tmem_slot;
   volatile int* abort_flag = s_abort;
 
-  // (with LB_FA_SETMAXNREG) warps 0-3 (loads, MMA issue) hand registers to the eight softmax warps,
-  // which hold a 128-column row of scores each
-#ifdef LB_FA_SETMAXNREG
-#define FA_REG_DEC() asm volatile("setmaxnreg.dec.sync.aligned.u32 96;")
-#define FA_REG_INC() asm volatile("setmaxnreg.inc.sync.aligned.u32 200;")
-#else
-#define FA_REG_DEC()
-#define FA_REG_INC()
-#endif
   if (warp == 0) {
-    FA_REG_DEC();
     // ------------------------------- TMA producer -------------------------------
     if (lane == 0 && nb_max > 0) {
       mbar_expect_tx(q_full, 2 * C::TILE_BYTES);
@@ -262,14 +257,12 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       if (!ok) atomicExch(&g_fa_status[0], 1u);
     }
   } else if (warp == 1 || warp == 2) {
-    FA_REG_DEC();
     // ------------------------------- MMA issuers -------------------------------
-    // One issuing thread per query tile.  A tcgen05.mma costs its issuer 60-90 cycles whatever its
-    // size (measured: 370 cycles for the four 128x128x16 of one S, 500 for the eight 128x64x16 of
-    // one P V), so a single thread feeding both tiles was the bottleneck of the whole kernel; two
-    // threads issue side by side and each follows the fixed order of its own tile with blocking
-    // waits: S(0); then per key block S(j+1) as soon as the softmax threads hold S(j) in registers,
-    // and P(j) V as soon as P(j) is in TMEM (or, head_dim 128, in shared memory).
+    // One issuing thread per query tile (a single thread feeding both tiles was measured to bound the
+    // kernel: a tcgen05.mma blocks its issuer for about its own execution time).  Each thread follows
+    // the fixed order of its own tile with blocking waits: S(0); then per key block, head_dim 64: S(j+1)
+    // as soon as the softmax threads hold S(j) in registers, and P(j) V in two halves as P(j) arrives;
+    // head_dim 128: P(j) V, then S(j+1) into the columns that P(j) leaves.
     // A K / V stage is free once BOTH tiles have used it, so each thread arrives on the stage's
     // empty barrier for every block, also for blocks its own tile does not need.
     const int t = warp - 1;
@@ -283,7 +276,6 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       const uint32_t s_dst = tmem_base + C::COL_S + t * C::BN;
       const uint32_t o_dst = tmem_base + C::COL_O + t * D;
       const uint32_t pa = tmem_base + C::COL_P + t * C::P_STRIDE;          // 8 columns per K = 16 slice
-      const uint64_t dp0 = make_desc(sbase + C::OFF_P + t * C::P_BYTES, 16, 1024);
       const int n_my = nb[t];
       bool ok = mbar_wait(q_full, 0, abort_flag);
       auto issue_s = [&](int j) -> bool {             // S(j) = Q K(j)^T, then release K(j)'s stage
@@ -302,23 +294,20 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       };
       auto issue_pv = [&](int j) -> bool {            // O += P(j) V(j), then release V(j)'s stage
         const int vs = j % C::VS;
-        if (!mbar_wait(p_full(t), (uint32_t)j & 1u, abort_flag)) return false;
         if (!mbar_wait(v_full(vs), ((uint32_t)(j / C::VS)) & 1u, abort_flag)) return false;
+        if (!mbar_wait(p_half(t), (uint32_t)j & 1u, abort_flag)) return false;
         fence_after();
         const uint64_t va = dv0 + (uint64_t)((vs * C::TILE_BYTES) >> 4);
-        if (C::P_TMEM) {
-          umma_bf16_ta(o_dst, pa, va, idesc_o, j ? 1u : 0u);
+        umma_bf16_ta(o_dst, pa, va, idesc_o, j ? 1u : 0u);
 #pragma unroll
-          for (int s = 1; s < C::BN / 16; s++)
-            umma_bf16_ta(o_dst, pa + 8u * s, va + (uint64_t)((s * 2048) >> 4), idesc_o, 1u);
-        } else {
-          umma_bf16(o_dst, dp0, va, idesc_o, j ? 1u : 0u);
+        for (int s = 1; s < C::BN / 32; s++)
+          umma_bf16_ta(o_dst, pa + 8u * s, va + (uint64_t)((s * 2048) >> 4), idesc_o, 1u);
+        if (!mbar_wait(p_full(t), (uint32_t)j & 1u, abort_flag)) return false;
+        fence_after();
 #pragma unroll
-          for (int s = 1; s < C::BN / 16; s++)
-            umma_bf16(o_dst, dp0 + (uint64_t)(((s >> 2) * C::ATOM_BYTES + (s & 3) * 32) >> 4), va + (uint64_t)((s * 2048) >> 4),
-                      idesc_o, 1u);
-        }
-        umma_commit(pv_done(t));
+        for (int s = C::BN / 32; s < C::BN / 16; s++)
+          umma_bf16_ta(o_dst, pa + 8u * s, va + (uint64_t)((s * 2048) >> 4), idesc_o, 1u);
+        if (!C::P_ALIAS || j == n_my - 1) umma_commit(pv_done(t));
         umma_commit(v_empty(vs));
         return true;
       };
@@ -328,11 +317,12 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       if (ok && t == 1 && nb[0] > 0 && n_my > 0) ok = mbar_wait(s_free(0), 0u, abort_flag);
       if (ok && n_my > 0) ok = issue_s(0);
       for (int j = 0; j < n_my && ok; j++) {
-        if (j + 1 < n_my) {
+        if (!C::P_ALIAS && j + 1 < n_my) {
           ok = mbar_wait(s_free(t), (uint32_t)j & 1u, abort_flag);
           if (ok) ok = issue_s(j + 1);
         }
         if (ok) ok = issue_pv(j);
+        if (C::P_ALIAS && ok && j + 1 < n_my) ok = issue_s(j + 1);
       }
       // blocks that only the other tile needs: keep the stage rings in step
       for (int j = n_my; j < nb_max && ok; j++) {
@@ -343,11 +333,8 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       }
       if (!ok) atomicExch(&g_fa_status[0], 2u);
     }
-  } else if (warp == 3) {
-    FA_REG_DEC();
-  } else {
+  } else if (warp >= 4) {
     // ------------------------------- softmax warps -------------------------------
-    FA_REG_INC();
     const int t = (warp - 4) >> 2;
     const int quad = warp & 3;
     const int rit = quad * 32 + lane;              // row inside the tile
@@ -356,9 +343,8 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     const uint32_t ts_addr = lane_addr + C::COL_S + t * C::BN;
     const uint32_t to_addr = lane_addr + C::COL_O + t * D;
     const uint32_t tp_addr = lane_addr + C::COL_P + t * C::P_STRIDE;
-    uint8_t* sP = smem + C::OFF_P + t * C::P_BYTES;
     const float sl2 = p.scale * 1.4426950408889634f;
-    constexpr int POLY_EVERY = (D == 64) ? LB_FA_POLY_EVERY : 0;   // head_dim 128 has twice the MMA work per exponential
+    const f32x2 sl2x2 = pack2(sl2, sl2);
     float m_i = -INFINITY, l_i = 0.f;
     bool ok = true;
     const int n_my = nb[t];
@@ -377,7 +363,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       const int lim = (p.causal ? min(p.Sk - 1, row + off) : p.Sk - 1) - c0;   // last visible column of this block
       // the row arrives in two halves so that the maximum of the first overlaps the second load;
       // four independent chains keep the 128 comparisons from serialising on their latency
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      float mx4[4] = {m_i, m_i, m_i, m_i};
       tmem_ld32(ts_addr, r);
       tmem_ld32(ts_addr + 32, r + 32);
       tmem_ld_wait();
@@ -388,58 +374,55 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         if (half == 1) {
           tmem_ld_wait();
           fence_before();
-          mbar_arrive(s_free(t));                     // S_t may be overwritten by the next key block
+          if (!C::P_ALIAS || j == 0) mbar_arrive(s_free(t));   // S_t may be overwritten by the next key block
         }
         if (need_mask) {
 #pragma unroll
-          for (int i = half * 64; i < half * 64 + 64; i++) {
+          for (int i = half * 64; i < half * 64 + 64; i++)
             if (i > lim) r[i] = 0xff800000u;           // -inf
-            mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(r[i]));
-          }
-        } else {
-#pragma unroll
-          for (int i = half * 64; i < half * 64 + 64; i++) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(r[i]));
         }
+#pragma unroll
+        for (int i = half * 64; i < half * 64 + 64; i += 2)
+          mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
       }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       FA_T(2);
       // Lazy reference maximum: keep the old one unless the new maximum is more than 2^8 above
       // it, so that O and l rarely need rescaling (values stay below 2^8 relative to it).
-      float m_new = fmaxf(m_i, mx);
+      float m_new = max2(max2(mx4[0], mx4[1]), max2(mx4[2], mx4[3]));
       if (m_i != -INFINITY && (m_new - m_i) * sl2 <= 8.f) m_new = m_i;
-      const float m_s = (m_new == -INFINITY) ? 0.f : m_new * sl2;
+      // (a row with a score of +inf has no softmax: NaN, as inf - inf gives)
+      const float m_s = (m_new == -INFINITY) ? 0.f : (m_new == INFINITY ? __int_as_float(0x7fffffff) : m_new * sl2);
       const float corr = (m_i == -INFINITY) ? 0.f : exp2f(m_i * sl2 - m_s);
       FA_T(3);
       // exponentials; P goes back to TMEM as packed bf16 pairs (column c holds keys 2c, 2c+1), 32
       // columns per store so that the first store is in flight while the second half is computed.
       // The first half is computed BEFORE waiting for the previous P V (which still reads the P
       // columns and owns O): its 64 exponentials overlap the tail of that MMA.
-      float rs2[2] = {0.f, 0.f};
+      const f32x2 nms2 = pack2(-m_s, -m_s);
+      f32x2 rs2[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
 #pragma unroll
       for (int hh = 0; hh < 2; hh++) {
         uint32_t pr[32];
 #pragma unroll
         for (int c = 0; c < 32; c++) {
           const int i = hh * 64 + c * 2;
-          // the MUFU unit (16 exponentials per clock per SM) is this kernel's ceiling at small head
-          // dimensions: every POLY_EVERY-th pair is evaluated on the FMA pipe instead
+          const f32x2 x2 = fma2(pack2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), sl2x2, nms2);
           float e0, e1;
-          if (POLY_EVERY > 0 && (c % (POLY_EVERY > 0 ? POLY_EVERY : 1)) == 0) {
-            e0 = exp2_poly(fmaf(__uint_as_float(r[i]), sl2, -m_s));
-            e1 = exp2_poly(fmaf(__uint_as_float(r[i + 1]), sl2, -m_s));
-          } else {
-            e0 = exp2f(fmaf(__uint_as_float(r[i]), sl2, -m_s));
-            e1 = exp2f(fmaf(__uint_as_float(r[i + 1]), sl2, -m_s));
-          }
-          rs2[c & 1] += e0 + e1;
+          unpack2(x2, e0, e1);
+          e0 = exp2f(e0);
+          e1 = exp2f(e1);
+          rs2[c & 1] = add2(rs2[c & 1], pack2(e0, e1));
           bf162 pk = __floats2bfloat162_rn(e0, e1);
           pr[c] = *reinterpret_cast<uint32_t*>(&pk);
         }
         if (hh == 0 && j > 0) {
-          // previous P V finished: O is stable and the P columns may be overwritten
-          if (!mbar_wait(pv_done(t), (uint32_t)(j - 1) & 1u, abort_flag)) { ok = false; }
-          fence_after();
-          if (ok && __any_sync(0xffffffffu, m_new != m_i)) {
+          // previous P V finished: O is stable and the P columns may be overwritten.  (head_dim 128: S(j) was
+          // issued behind it by the same thread, so its completion says that P V has completed too.)
+          if (!C::P_ALIAS) {
+            if (!mbar_wait(pv_done(t), (uint32_t)(j - 1) & 1u, abort_flag)) { ok = false; }
+            fence_after();
+          }
+          if (ok && __any_sync(0xffffffffu, !(m_new == m_i))) {
 #pragma unroll 1
             for (int c = 0; c < D / 32; c++) {
               uint32_t o[32];
@@ -452,23 +435,18 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             tmem_st_wait();
           }
         }
-        if (C::P_TMEM) {
-          tmem_st32(tp_addr + hh * 32, pr);
-        } else {
-          // keys hh*64 .. +63 of this row are 128 bytes: one row of swizzle atom hh
-#pragma unroll
-          for (int c16 = 0; c16 < 8; c16++)
-            *reinterpret_cast<uint4*>(sP + hh * C::ATOM_BYTES + sw128_off(rit, c16)) =
-                make_uint4(pr[c16 * 4], pr[c16 * 4 + 1], pr[c16 * 4 + 2], pr[c16 * 4 + 3]);
-        }
+        tmem_st32(tp_addr + hh * 32, pr);
+        tmem_st_wait();
+        fence_before();
+        mbar_arrive(hh == 0 ? p_half(t) : p_full(t));
       }
       if (!ok) break;
-      if (C::P_TMEM) tmem_st_wait(); else fence_proxy_async_smem();
-      l_i = l_i * corr + (rs2[0] + rs2[1]);
+      float rs[4];
+      unpack2(rs2[0], rs[0], rs[1]);
+      unpack2(rs2[1], rs[2], rs[3]);
+      l_i = l_i * corr + ((rs[0] + rs[1]) + (rs[2] + rs[3]));
       m_i = m_new;
       FA_T(4);
-      fence_before();
-      mbar_arrive(p_full(t));
       FA_T(5);
       FA_ACC(0, 0, 1); FA_ACC(1, 1, 2); FA_ACC(2, 2, 3); FA_ACC(3, 3, 4); FA_ACC(4, 4, 5);
 #ifdef LB_FA_PROFILE
@@ -480,7 +458,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       for (int i = 0; i < 8; i++) atomicAdd(&g_fa_prof[i], prof[i]);
 #endif
     if (ok && n_my > 0) {
-      if (!mbar_wait(pv_done(t), (uint32_t)(n_my - 1) & 1u, abort_flag)) ok = false;
+      if (!mbar_wait(pv_done(t), C::P_ALIAS ? 0u : (uint32_t)(n_my - 1) & 1u, abort_flag)) ok = false;
     }
     if (ok && n_my > 0) {
       fence_after();
@@ -529,6 +507,10 @@ int launch_fa_fwd(const void* q, const void* k, const void* v, FaFwdParams p, co
     attr = true;
   }
   p.tiles_x = (p.Sq + 255) / 256;
+  // heads ordered together: as many as have their K / V in 48 MB (of 126 MB of L2), whole GQA groups
+  const long long kv_bytes = 4LL * D * p.Sk;
+  const long long kv_heads = kv_bytes >= (48LL << 20) ? 1 : (48LL << 20) / kv_bytes;
+  p.group = (int)(kv_heads * (p.hq / p.hkv) < (long long)p.hq * p.B ? kv_heads * (p.hq / p.hkv) : (long long)p.hq * p.B);
   p.wait_ns = g_lb_flag_wait_ns;
   const long long grid = (long long)push.n_mov + (long long)p.tiles_x * p.hq * p.B;
   if (grid > 2147483647LL) return LB_ERR_SHAPE;

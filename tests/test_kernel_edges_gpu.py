@@ -1,0 +1,74 @@
+"""Sizes at which the tiling, the scheduling or the dispatch of a kernel changes, against float64 PyTorch.
+
+Bounds: a bf16 result is one rounding (2^-9 relative, 2^-9 / sqrt(3) = 1.1e-3 in the 2-norm) of fp32 sums whose bf16 inputs are exact;
+where a bf16 intermediate (P, dS, an activation) enters a further product its rounding adds about as much again
+per factor.  5e-3 covers one such intermediate, 1e-2 a chain of them.
+"""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(*shape, scale=1.0, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, generator=g, device="cuda", dtype=torch.float32) * scale).to(torch.bfloat16)
+
+
+def _rel(got, want):
+    return ((got.double() - want.double()).norm() / want.double().norm().clamp_min(1e-30)).item()
+
+
+def _status_ok():
+    from lightron_b200.ops import native
+    assert native.device_status() == {}
+
+
+# ---- attention -------------------------------------------------------------------------------------
+
+
+def _attention64(q, k, v, do, causal):
+    q, k, v = (t.detach().double().requires_grad_(True) for t in (q, k, v))
+    B, Sq, hq, d = q.shape
+    Sk, rep = k.shape[1], hq // k.shape[2]
+    kk, vv = (t.repeat_interleave(rep, 2).transpose(1, 2) for t in (k, v))
+    s = q.transpose(1, 2) @ kk.transpose(-1, -2) * d ** -0.5
+    if causal:
+        s = s.masked_fill(torch.ones(Sq, Sk, dtype=torch.bool, device="cuda").triu(1 + Sk - Sq), -float("inf"))
+    o = (s.softmax(-1) @ vv).transpose(1, 2)
+    return (o.detach(), *torch.autograd.grad(o, [q, k, v], do.double()))
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("B,Sq,Sk,hq,hkv,causal,scale", [
+    (1, 2, 2, 1, 1, True, 1.0),              # smaller than anything that is tiled
+    (1, 128, 128, 2, 1, True, 1.0),          # one key block, the second query tile empty
+    (2, 129, 129, 4, 2, True, 1.0),          # one row over
+    (1, 255, 640, 2, 2, True, 1.0),          # more keys than queries
+    (1, 300, 77, 2, 1, False, 1.0),          # last key block ragged, no mask
+    (9, 200, 200, 8, 4, True, 1.0),          # 36 (batch, kv head) pairs: past one scheduling group of 32
+    (1, 700, 700, 4, 1, True, 8.0),          # large scores: the running maximum moves, exponents underflow
+])
+def test_attention_tile_edges(B, Sq, Sk, hq, hkv, causal, scale, d):
+    from lightron_b200.ops import functional as OF
+    q, k, v, do = _rand(B, Sq, hq, d, scale=scale, seed=1), _rand(B, Sk, hkv, d, seed=2), _rand(B, Sk, hkv, d, seed=3), _rand(B, Sq, hq, d, seed=4)
+    o, lse = OF.flash_fwd_native(q, k, v, causal, d ** -0.5)
+    got = (o, *OF.flash_bwd_native(q, k, v, o, lse, do, causal, d ** -0.5))
+    _status_ok()
+    for name, g, w in zip(("o", "dq", "dk", "dv"), got, _attention64(q, k, v, do, causal)):
+        if w.norm() > 1e-6:                  # (with one visible key dq and dk vanish)
+            assert _rel(g, w) < 1e-2, name
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_attention_bad_scores_stay_in_their_rows(d, bad):
+    """A key that is not finite spoils the rows that see it, whichever unit computes its exponentials, and no other."""
+    from lightron_b200.ops import functional as OF
+    S = 300
+    for key in (0, 130, 193, 299):
+        q, k, v = _rand(1, S, 1, d, seed=1).abs(), _rand(1, S, 1, d, seed=2), _rand(1, S, 1, d, seed=3)
+        k[0, key, 0, 0] = bad
+        o, _ = OF.flash_fwd_native(q, k, v, True, d ** -0.5)
+        want = torch.arange(S, device="cuda") >= key
+        assert torch.equal(o[0, :, 0].isnan().all(-1), want) and torch.equal(o[0, :, 0].isnan().any(-1), want), key

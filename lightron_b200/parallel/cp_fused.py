@@ -111,8 +111,9 @@ def _bwd_call(q, kbuf, vbuf, Sk, kv_brows, o, lse, do, scale, dk=None, dv=None):
     if dk is None:
         dk = torch.empty(B, Sk, hkv, d, dtype=q.dtype, device=q.device)
         dv = torch.empty_like(dk)
-    delta = torch.empty(B, hq, Sq, dtype=torch.float32, device=q.device)
-    dq_acc = torch.zeros(B * hq * ((Sq + 127) // 128) * 128 * d, dtype=torch.float32, device=q.device)
+    n_pad = B * hq * ((Sq + 127) // 128) * 128
+    delta = torch.empty(2 * n_pad, dtype=torch.float32, device=q.device)
+    dq_acc = torch.empty(n_pad * d, dtype=torch.float32, device=q.device)
     native.call("lb_flash_bwd_cp", q.data_ptr(), kbuf.data_ptr(), vbuf.data_ptr(), o.data_ptr(), do.data_ptr(),
                 lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                 B, Sq, Sk, kv_brows, hq, hkv, d, q.stride(1), kbuf.stride(1), vbuf.stride(1), o.stride(1), do.stride(1),

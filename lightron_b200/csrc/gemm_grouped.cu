@@ -31,11 +31,17 @@ static __device__ unsigned int g_grp_status[4] = {0, 0, 0, 0};
 namespace {
 
 constexpr int BM = 128, BN = 256, BK = 64;
-constexpr int STAGES = 4;
 constexpr int A_BYTES = BM * BK * 2;
-constexpr int B_BYTES = BN * BK * 2;
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+// CG CTAs work on one tile: 1 = a CTA per 128x256 tile, 2 = a pair (tcgen05 cta_group::2) per 256x256 tile, in which
+// each CTA loads its 128 rows of A and half of B.  Per CTA a stage then holds 16 + 16 instead of 16 + 32 KB, and the tensor
+// pipe, whose operand reads from shared memory are what limits and heats it, reads a third less.
+template <int CG>
+struct Cfg {
+  static constexpr int B_BYTES = BN / CG * BK * 2;
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGES = CG == 2 ? 6 : 4;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+};
 constexpr int NUM_THREADS = 192;
 constexpr int GROUP_M = 8;
 constexpr int MAX_PROBLEMS = 8;
@@ -86,67 +92,80 @@ __device__ __forceinline__ void give_up(volatile int* abort_flag, unsigned where
 // as compile-time constants every descriptor field and the number of TMA boxes is a constant (with
 // run-time majors the producer issued predicated-off TMA instructions for the branch not taken and
 // the tensor pipe lost a fifth of its activity), although the tile itself comes from a list in memory.
-template <bool A_MN, bool B_MN>
+// A CTA of a pair loads its own part (m0, n0 are its first row of A and of B) and signals the leader's barrier,
+// which expects the bytes of both.
+template <int CG>
+__device__ __forceinline__ void load_box(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  if constexpr (CG == 2) bw::tma_load_2d_pair(dst, map, x, y, bar);
+  else bw::tma_load_2d(dst, map, x, y, bar);
+}
+template <int CG, bool A_MN, bool B_MN>
 __device__ __forceinline__ bool produce_tile(const CUtensorMap* ta, const CUtensorMap* tb, int m0, int n0, int num_kb,
                                              uint32_t smem_base, uint32_t bar_base, int& stage, uint32_t& phase,
-                                             volatile int* abort_flag, int k_base = 0, int b_split = 0) {
+                                             volatile int* abort_flag, bool leader, int k_base = 0, int b_split = 0) {
+  using C = Cfg<CG>;
   for (int kb = 0; kb < num_kb; kb++) {
-    if (!bw::mbar_wait(bar_base + 8u * (STAGES + stage), phase ^ 1u, abort_flag)) return false;
-    const uint32_t fb = bar_base + 8u * stage;
-    bw::mbar_expect_tx(fb, STAGE_BYTES);
-    const uint32_t sa = smem_base + stage * STAGE_BYTES;
+    if (!bw::mbar_wait(bar_base + 8u * (C::STAGES + stage), phase ^ 1u, abort_flag)) return false;
+    uint32_t fb = bar_base + 8u * stage;
+    if (CG == 1 || leader) bw::mbar_expect_tx(fb, CG * C::STAGE_BYTES);
+    if (CG == 2) fb = bw::leader_bar(fb);
+    const uint32_t sa = smem_base + stage * C::STAGE_BYTES;
     const uint32_t sb = sa + A_BYTES;
     const int k0 = k_base + kb * BK;
     if (!A_MN) {
-      bw::tma_load_2d(sa, ta, k0, m0, fb);                                                      // box {64 k, 128 m}
+      load_box<CG>(sa, ta, k0, m0, fb);                                                              // box {64 k, 128 m}
     } else {
 #pragma unroll
-      for (int j = 0; j < BM / 64; j++) bw::tma_load_2d(sa + j * 8192, ta, m0 + 64 * j, k0, fb);  // box {64 m, 64 k}
+      for (int j = 0; j < BM / 64; j++) load_box<CG>(sa + j * 8192, ta, m0 + 64 * j, k0, fb);        // box {64 m, 64 k}
     }
     if (!B_MN) {
-      if (b_split > 0) {                       // two boxes {64 k, 128 n}: rows n0.. and b_split + n0.. of B
-        bw::tma_load_2d(sb, tb, k0, n0, fb);
-        bw::tma_load_2d(sb + (BN / 2) * BK * 2, tb, k0, b_split + n0, fb);
-      } else {
-        bw::tma_load_2d(sb, tb, k0, n0, fb);                                                    // box {64 k, 256 n}
-      }
+      load_box<CG>(sb, tb, k0, n0, fb);                                                              // box {64 k, 128 n}
+      if (CG == 1)                               // second box: the next 128 rows, or (SwiGLU) the up rows b_split + n0..
+        load_box<CG>(sb + (BN / 2) * BK * 2, tb, k0, n0 + (b_split > 0 ? b_split : BN / 2), fb);
     } else {
 #pragma unroll
-      for (int j = 0; j < BN / 64; j++) bw::tma_load_2d(sb + j * 8192, tb, n0 + 64 * j, k0, fb);  // box {64 n, 64 k}
+      for (int j = 0; j < BN / CG / 64; j++) load_box<CG>(sb + j * 8192, tb, n0 + 64 * j, k0, fb);   // box {64 n, 64 k}
     }
-    if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+    if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
   }
   return true;
 }
 
-template <bool A_MN, bool B_MN>
+template <int CG, bool A_MN, bool B_MN>
 __device__ __forceinline__ bool mma_tile(uint32_t d_tmem, int num_kb, uint32_t smem_base, uint32_t bar_base, int& stage,
                                          uint32_t& phase, volatile int* abort_flag) {
+  using C = Cfg<CG>;
   constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) |
-                             ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+                             ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM * CG >> 4) << 24);
   constexpr uint32_t a_lbo = A_MN ? 8192u : 16u, b_lbo = B_MN ? 8192u : 16u;
   constexpr uint32_t a_kstep = A_MN ? 2048u : 32u, b_kstep = B_MN ? 2048u : 32u;   // bytes per K=16 slice
   for (int kb = 0; kb < num_kb; kb++) {
     if (!bw::mbar_wait(bar_base + 8u * stage, phase, abort_flag)) return false;
     bw::fence_after();
-    const uint32_t sa = smem_base + stage * STAGE_BYTES;
+    const uint32_t sa = smem_base + stage * C::STAGE_BYTES;
     const uint32_t sb = sa + A_BYTES;
 #pragma unroll
     for (int k = 0; k < BK / 16; k++) {
       const uint64_t ad = bw::make_desc(sa + k * a_kstep, a_lbo, 1024u);
       const uint64_t bd = bw::make_desc(sb + k * b_kstep, b_lbo, 1024u);
-      bw::umma_bf16(d_tmem, ad, bd, idesc, (kb | k) ? 1u : 0u);
+      if constexpr (CG == 2) bw::umma_bf16_pair(d_tmem, ad, bd, idesc, (kb | k) ? 1u : 0u);
+      else bw::umma_bf16(d_tmem, ad, bd, idesc, (kb | k) ? 1u : 0u);
     }
-    bw::umma_commit(bar_base + 8u * (STAGES + stage));   // frees this smem stage when the MMAs have read it
-    if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+    // frees this smem stage (of both CTAs) when the MMAs have read it
+    if constexpr (CG == 2) bw::umma_commit_pair(bar_base + 8u * (C::STAGES + stage));
+    else bw::umma_commit(bar_base + 8u * (C::STAGES + stage));
+    if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
   }
   return true;
 }
 
+template <int CG>
 __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __grid_constant__ GroupedParams gp) {
+  using CF = Cfg<CG>;
+  constexpr int STAGES = CF::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * CF::STAGE_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   __shared__ int s_abort[2];     // {abort, extra wait in ms}: see bw::mbar_wait
 
@@ -158,7 +177,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
   auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + 2 + a); };
-  const int item_begin = gp.offsets[blockIdx.x], item_end = gp.offsets[blockIdx.x + 1];
+  const int worker = (int)blockIdx.x / CG;                       // a CTA, or a pair of CTAs that walks one list
+  const int rank = CG == 2 ? (int)bw::cluster_ctarank() : 0;      // 0 = leader: issues the MMAs of the pair
+  const int item_begin = gp.offsets[worker], item_end = gp.offsets[worker + 1];
 
   if (threadIdx.x == 0) {
     s_abort[0] = 0;
@@ -169,13 +190,17 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
     }
     for (int a = 0; a < 2; a++) {
       bw::mbar_init(tfull_bar(a), 1);
-      bw::mbar_init(tempty_bar(a), 4);
+      bw::mbar_init(tempty_bar(a), 4 * CG);
     }
     bw::mbar_init_fence();
   }
-  if (warp == 1) bw::tmem_alloc(bw::smem_u32(tmem_slot), 512);
+  if (warp == 1) {
+    if constexpr (CG == 2) bw::tmem_alloc_pair(bw::smem_u32(tmem_slot), 512);
+    else bw::tmem_alloc(bw::smem_u32(tmem_slot), 512);
+  }
   bw::fence_before();
   __syncthreads();
+  if constexpr (CG == 2) bw::cluster_sync();      // the peer's barriers exist before anything signals them
   bw::fence_after();
   const uint32_t tmem_base = *tmem_slot;
   volatile int* abort_flag = s_abort;
@@ -196,20 +221,29 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
         int tm, tn;
         tile_coords(item & 0xFFFFFF, gp.prob[pi], tm, tn);
         const int split = gp.prob[pi].epi == 1 ? gp.prob[pi].half : 0;
-        const int m0 = tm * BM, n0 = split ? tn * (BN / 2) : tn * BN;
+        // first row of A and of B this CTA loads.  SwiGLU tiles: 128 gate rows and the up rows of the same
+        // index (a pair's leader loads the former, its peer the latter)
+        const int m0 = (tm * CG + rank) * BM;
+        const int n0 = split ? tn * (BN / 2) + (CG == 2 ? rank * split : 0) : tn * BN + rank * (BN / 2);
         const int num_kb = gp.prob[pi].num_kb;
         switch (gp.prob[pi].a_mn * 2 + gp.prob[pi].b_mn) {
-          case 0: ok = produce_tile<false, false>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, 0, split); break;
-          case 1: ok = produce_tile<false, true>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
-          case 2: ok = produce_tile<true, false>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, 0, split); break;
-          default: ok = produce_tile<true, true>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
+          case 0: ok = produce_tile<CG, false, false>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, 0, split); break;
+          case 1: ok = produce_tile<CG, false, true>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0); break;
+          case 2: ok = produce_tile<CG, true, false>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, 0, split); break;
+          default: ok = produce_tile<CG, true, true>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0); break;
         }
         if (!ok) give_up(abort_flag, 1u);
       }
+      // the leader's MMAs release this CTA's stages: all releases have arrived before the CTA may exit
+      if (CG == 2)
+        for (int s = 0; s < STAGES && ok; s++) {
+          ok = bw::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag);
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    if (lane == 0 && rank == 0) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -226,13 +260,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
         bw::fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * BN;
         switch (majors) {
-          case 0: ok = mma_tile<false, false>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
-          case 1: ok = mma_tile<false, true>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
-          case 2: ok = mma_tile<true, false>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
-          default: ok = mma_tile<true, true>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
+          case 0: ok = mma_tile<CG, false, false>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
+          case 1: ok = mma_tile<CG, false, true>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
+          case 2: ok = mma_tile<CG, true, false>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
+          default: ok = mma_tile<CG, true, true>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
         }
-        if (ok) bw::umma_commit(tfull_bar(acc));          // accumulator complete
-        else give_up(abort_flag, 3u);
+        if (!ok) give_up(abort_flag, 3u);
+        else if constexpr (CG == 2) bw::umma_commit_pair(tfull_bar(acc));          // accumulator complete
+        else bw::umma_commit(tfull_bar(acc));
       }
     }
   } else {
@@ -252,7 +287,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
       const long long ldc = gp.prob[pi].ldc;
       const int acc = n & 1;
       const uint32_t acc_phase = (uint32_t)(n >> 1) & 1u;
-      const int row = tm * BM + quad * 32 + lane;
+      const int row = (tm * CG + rank) * BM + quad * 32 + lane;
       const int n0 = tn * BN;
       if (gp.prob[pi].epi == 2 && row < pM) {
         // while the MMAs of this tile run: pull the g | u values its epilogue will read into L2
@@ -305,7 +340,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
         }
         bw::fence_before();
         __syncwarp();
-        if (lane == 0) bw::mbar_arrive(tempty_bar(acc));
+        if (lane == 0) {
+        if constexpr (CG == 2) bw::mbar_arrive_leader(tempty_bar(acc));
+        else bw::mbar_arrive(tempty_bar(acc));
+      }
         continue;
       }
       if (epi == 2) {
@@ -355,7 +393,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
         }
         bw::fence_before();
         __syncwarp();
-        if (lane == 0) bw::mbar_arrive(tempty_bar(acc));
+        if (lane == 0) {
+        if constexpr (CG == 2) bw::mbar_arrive_leader(tempty_bar(acc));
+        else bw::mbar_arrive(tempty_bar(acc));
+      }
         continue;
       }
 #pragma unroll 1
@@ -385,15 +426,20 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
       }
       bw::fence_before();
       __syncwarp();
-      if (lane == 0) bw::mbar_arrive(tempty_bar(acc));
+      if (lane == 0) {
+        if constexpr (CG == 2) bw::mbar_arrive_leader(tempty_bar(acc));
+        else bw::mbar_arrive(tempty_bar(acc));
+      }
     }
   }
 
   bw::fence_before();
   __syncthreads();
+  if constexpr (CG == 2) bw::cluster_sync();      // nothing of the pair is in flight in either CTA
   if (warp == 1) {
     bw::fence_after();
-    bw::tmem_dealloc(tmem_base, 512);
+    if constexpr (CG == 2) bw::tmem_dealloc_pair(tmem_base, 512);
+    else bw::tmem_dealloc(tmem_base, 512);
   }
 }
 
@@ -455,9 +501,11 @@ __device__ __forceinline__ RaggedTile ragged_tile(int t, const RaggedParams& rp,
 }
 
 __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __grid_constant__ RaggedParams rp) {
+  using CF = Cfg<1>;
+  constexpr int STAGES = CF::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * CF::STAGE_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   __shared__ int s_abort[2];     // {abort, extra wait in ms}: see bw::mbar_wait
   __shared__ int s_off[MAX_PROBLEMS], s_tiles[MAX_PROBLEMS];
@@ -518,10 +566,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
         if (rt.e < 0) break;
         if (rt.num_kb == 0) continue;
         if (rp.mode == 0) {
-          if (!rp.b_mn) ok = produce_tile<false, false>(&rp.ta, &rp.tb[rt.e], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
-          else          ok = produce_tile<false, true>(&rp.ta, &rp.tb[rt.e], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
+          if (!rp.b_mn) ok = produce_tile<1, false, false>(&rp.ta, &rp.tb[rt.e], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, true);
+          else          ok = produce_tile<1, false, true>(&rp.ta, &rp.tb[rt.e], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, true);
         } else {
-          ok = produce_tile<true, true>(&rp.ta, &rp.tb[0], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, rt.k_base);
+          ok = produce_tile<1, true, true>(&rp.ta, &rp.tb[0], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, true, rt.k_base);
         }
         if (!ok) give_up(abort_flag, 1u);
       }
@@ -543,10 +591,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
         bw::fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * BN;
         if (rp.mode == 0) {
-          if (!rp.b_mn) ok = mma_tile<false, false>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
-          else          ok = mma_tile<false, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
+          if (!rp.b_mn) ok = mma_tile<1, false, false>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
+          else          ok = mma_tile<1, false, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
         } else {
-          ok = mma_tile<true, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
+          ok = mma_tile<1, true, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
         }
         if (ok) bw::umma_commit(tfull_bar(acc));
         else give_up(abort_flag, 3u);
@@ -613,7 +661,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
 
 // ---- host side: static schedule, cached per (device, shapes) -------------------------------------
 struct Schedule {
-  int grid = 0;
+  int cg = 1;         // CTAs per tile
+  int grid = 0;       // workers (CTAs, or pairs of CTAs)
   int* d_offsets = nullptr;
   int* d_items = nullptr;
   unsigned long long last_use = 0;
@@ -671,10 +720,34 @@ long long assign_items(const Problem* probs, int np, int sms, std::vector<std::v
   return busiest;
 }
 
-int build_schedule(const Problem* probs, int np, int sms, Schedule* out) {
+void set_tiles(Problem* p, int cg) {
+  p->tiles_m = (p->M + BM * cg - 1) / (BM * cg);
+  p->tiles_n = (p->N + BN - 1) / BN;
+  p->num_kb = (p->K + BK - 1) / BK;
+}
+
+// CTAs per tile for this set of problems: pairs unless their coarser tiles make the busiest worker's list more than 5 % longer
+// (few or ragged tiles), which is what a pair's tile gains.  Measured with 16384 rows, CTAs against pairs: N11264 K2048
+// 584 / 546 us, N2560 K2048 134 / 126, N2048 K2048 106 / 103, N2048 K5632 259 / 254; data + weight gradient of these layers 1167 / 1142,
+// 286 / 262, 234 / 214, 623 / 622.  Pairs forced on few tiles lose: 4096 x 2304 x 768 takes 27 us with CTAs, 31 with pairs.
+int choose_cg(Problem* probs, int np, int sms) {
+  if (sms < 2) return 1;
+  long long load[3] = {0, 0, 0};
+  for (int cg = 1; cg <= 2; cg++) {
+    for (int i = 0; i < np; i++) set_tiles(&probs[i], cg);
+    load[cg] = assign_items(probs, np, sms / cg, nullptr, nullptr, nullptr);
+    if (load[cg] < 0) return -1;
+  }
+  return load[2] * 100 <= load[1] * 105 ? 2 : 1;
+}
+
+int build_schedule(Problem* probs, int np, int sms, Schedule* out) {
   std::vector<std::vector<int>> per;
   int total = 0;
-  if (assign_items(probs, np, sms, &per, &total, nullptr) < 0) return LB_ERR_SHAPE;
+  out->cg = choose_cg(probs, np, sms);
+  if (out->cg < 0) return LB_ERR_SHAPE;
+  for (int i = 0; i < np; i++) set_tiles(&probs[i], out->cg);
+  if (assign_items(probs, np, sms / out->cg, &per, &total, nullptr) < 0) return LB_ERR_SHAPE;
   const int grid = (int)per.size();
   std::vector<int> offsets(grid + 1, 0), flat;
   flat.reserve(total);
@@ -691,6 +764,24 @@ int build_schedule(const Problem* probs, int np, int sms, Schedule* out) {
   return LB_OK;
 }
 
+// Launches fn<CG> on `workers` workers; a pair is a cluster of two CTAs.
+template <typename P>
+int launch_pairs(void (*fn)(P), const P& params, int workers, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * workers);
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = Cfg<2>::SMEM_BYTES;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, params);
+  if (e != cudaSuccess) { cudaGetLastError(); g_lb_last_cuda_error = (int)e; return LB_ERR_LAUNCH; }
+  return LB_OK;
+}
+
 }  // namespace
 
 // Copies the status words of the grouped GEMM kernel to host memory and clears them.
@@ -702,7 +793,7 @@ extern "C" int lb_gemm_grouped_status(void* out) {
   return LB_OK;
 }
 
-// Host only (no CUDA call): the schedule lb_gemm_grouped would build for these shapes on `sms` SMs.
+// Host only (no CUDA call): the schedule lb_gemm_grouped would build for these shapes on `sms` SMs with a CTA per tile.
 // out[0] = load of the busiest CTA, out[1] = total work, out[2] = number of CTAs used, all in k-block
 // units of 64 (a tile counts its k-blocks + 6).  busiest * CTAs / total is the imbalance factor.
 // Number of schedules currently cached (never more than MAX_SCHEDULES).
@@ -716,7 +807,8 @@ extern "C" int lb_gemm_grouped_plan(int n, const int* M, const int* N, const int
   Problem probs[MAX_PROBLEMS];
   for (int i = 0; i < n; i++) {
     if (M[i] <= 0 || N[i] <= 0 || K[i] <= 0) return LB_ERR_SHAPE;
-    probs[i].tiles_m = (M[i] + BM - 1) / BM; probs[i].tiles_n = (N[i] + BN - 1) / BN; probs[i].num_kb = (K[i] + BK - 1) / BK;
+    probs[i].M = M[i]; probs[i].N = N[i]; probs[i].K = K[i];
+    set_tiles(&probs[i], 1);
   }
   std::vector<std::vector<int>> per;
   int total = 0;
@@ -764,21 +856,21 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
       if (e == 2 && N[i] != half[i]) return LB_ERR_SHAPE;
       if (accumulate && accumulate[i]) return LB_ERR_ARG;
     }
-    if (!b_mn[i]) rc = bw::make_map_bf16(&gp.tb[i], B[i], (uint64_t)K[i], (uint64_t)N[i], (uint64_t)ldb[i], BK, e == 1 ? BN / 2 : BN);
+    if (!b_mn[i]) rc = bw::make_map_bf16(&gp.tb[i], B[i], (uint64_t)K[i], (uint64_t)N[i], (uint64_t)ldb[i], BK, BN / 2);
     else          rc = bw::make_map_bf16(&gp.tb[i], B[i], (uint64_t)N[i], (uint64_t)K[i], (uint64_t)ldb[i], 64, BK);
     if (rc) return rc;
     Problem& p = gp.prob[i];
     p.C = (bf16*)C[i]; p.ldc = ldc[i]; p.M = M[i]; p.N = N[i]; p.K = K[i];
     p.C2 = e ? (bf16*)C2[i] : nullptr; p.ldc2 = e ? ldc2[i] : 0; p.epi = e; p.half = e ? half[i] : 0;
     p.a_mn = a_mn[i]; p.b_mn = b_mn[i]; p.accumulate = accumulate ? accumulate[i] : 0;
-    p.tiles_m = (M[i] + BM - 1) / BM; p.tiles_n = (N[i] + BN - 1) / BN; p.num_kb = (K[i] + BK - 1) / BK;
     key.push_back(M[i]); key.push_back(N[i]); key.push_back(K[i]);
   }
   {
     std::lock_guard<std::mutex> lock(g_sched_mutex);
     if (g_sms == 0) {
       cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-      cudaFuncSetAttribute(gemm_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+      cudaFuncSetAttribute(gemm_grouped_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
+      cudaFuncSetAttribute(gemm_grouped_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
     }
   }
   Schedule sched;
@@ -805,8 +897,14 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
   }
   gp.offsets = sched.d_offsets;
   gp.items = sched.d_items;
-  gemm_grouped_kernel<<<sched.grid, NUM_THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(gp);
-  LB_CHECK_LAUNCH();
+  for (int i = 0; i < n; i++) set_tiles(&gp.prob[i], sched.cg);
+  if (sched.cg == 2) {
+    const int rc = launch_pairs(gemm_grouped_kernel<2>, gp, sched.grid, (cudaStream_t)stream);
+    if (rc) return rc;
+  } else {
+    gemm_grouped_kernel<1><<<sched.grid, NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream>>>(gp);
+    LB_CHECK_LAUNCH();
+  }
   return LB_OK;
 }
 
@@ -835,7 +933,7 @@ extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, cons
   if (rc) return rc;
   for (int e = 0; e < LE; e++) {
     if ((uintptr_t)B[e] & 15) return LB_ERR_ARG;
-    if (!b_mn) rc = bw::make_map_bf16(&rp.tb[e], B[e], (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, BN);
+    if (!b_mn) rc = bw::make_map_bf16(&rp.tb[e], B[e], (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BK, BN / 2);
     else       rc = bw::make_map_bf16(&rp.tb[e], B[e], (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 64, BK);
     if (rc) return rc;
     rp.C[e] = nullptr;
@@ -847,9 +945,9 @@ extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, cons
   {
     std::lock_guard<std::mutex> lock(g_sched_mutex);
     static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(gemm_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); attr = true; }
+    if (!attr) { cudaFuncSetAttribute(gemm_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES); attr = true; }
   }
-  gemm_ragged_kernel<<<lb_num_sms(), NUM_THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(rp);
+  gemm_ragged_kernel<<<lb_num_sms(), NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream>>>(rp);
   LB_CHECK_LAUNCH();
   return LB_OK;
 }
@@ -877,9 +975,9 @@ extern "C" int lb_gemm_ragged_wgrad(const void* dY, const void* X, void* const* 
   {
     std::lock_guard<std::mutex> lock(g_sched_mutex);
     static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(gemm_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); attr = true; }
+    if (!attr) { cudaFuncSetAttribute(gemm_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES); attr = true; }
   }
-  gemm_ragged_kernel<<<lb_num_sms(), NUM_THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(rp);
+  gemm_ragged_kernel<<<lb_num_sms(), NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream>>>(rp);
   LB_CHECK_LAUNCH();
   return LB_OK;
 }

@@ -72,3 +72,38 @@ def test_attention_bad_scores_stay_in_their_rows(d, bad):
         o, _ = OF.flash_fwd_native(q, k, v, True, d ** -0.5)
         want = torch.arange(S, device="cuda") >= key
         assert torch.equal(o[0, :, 0].isnan().all(-1), want) and torch.equal(o[0, :, 0].isnan().any(-1), want), key
+
+
+# ---- GEMM --------------------------------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("M,N,K", [(5000, 2312, 72), (4096, 2304, 512), (4225, 4104, 200), (130, 520, 1032), (1, 8, 8)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_gemm_pair_tiles(M, N, K, a_mn, b_mn):
+    """Many tiles (CTA pairs, the last tiles ragged in rows and columns) and few (single CTAs), plain and accumulating."""
+    from lightron_b200.ops import functional as OF
+    if a_mn and M % 8:
+        M = M // 8 * 8 + 8
+    a, b, c0 = _rand(M, K, seed=1), _rand(N, K, seed=2), _rand(M, N, seed=3)
+    ops = (a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b)
+    want = a.double() @ b.double().t()
+    assert _rel(OF.gemm(*ops, a_mn=a_mn, b_mn=b_mn), want) < 5e-3
+    out = c0.clone()
+    OF.gemm_grouped([(*ops, a_mn, b_mn, out, True)])
+    _status_ok()
+    assert _rel(out, want + c0.double()) < 5e-3
+
+
+@pytest.mark.parametrize("T,K,I", [(4000, 256, 1288), (70, 512, 264)])
+def test_swiglu_mlp_pair_tiles(T, K, I):
+    from lightron_b200.ops import functional as OF
+    w13 = _rand(2 * I, K, scale=K ** -0.5, seed=2)
+    ins = [t.detach().requires_grad_(True) for t in (_rand(T, K, seed=1), w13[:I], w13[I:], _rand(K, I, scale=I ** -0.5, seed=3))]
+    dy = _rand(T, K, seed=4)
+    y = OF.swiglu_mlp(*ins)
+    got = (y, *torch.autograd.grad(y, ins, dy))
+    _status_ok()
+    x, w1, w3, w2 = (t.detach().double().requires_grad_(True) for t in ins)
+    yd = (torch.nn.functional.silu(x @ w1.t()) * (x @ w3.t())) @ w2.t()
+    for g, w in zip(got, (yd, *torch.autograd.grad(yd, [x, w1, w3, w2], dy.double()))):
+        assert _rel(g, w) < 1e-2

@@ -33,9 +33,66 @@ int lb_num_sms() {
 extern "C" int lb_sm_count() { return lb_num_sms(); }
 
 // ---------------------------------------------------------------------------------------
-// RMSNorm.  One warp per row, two passes over the row (the second hits L1/L2).
+// RMSNorm.  One warp per row.
 //   fwd: h = x (+ res);  rstd = rsqrt(mean(h^2) + eps);  y = h * rstd * w
+// Memory bound (x, res in; h, y out).  Rows of up to 4096 columns stay in registers between the sum of
+// squares and the scaling (NV 16-byte vectors per lane, all loads of a row in flight at once); wider rows are
+// read a second time.  With the residual, read twice / kept: 16384 x 2048 55.4 / 51.4 us (5.2 TB/s), 16384 x 4096 110 / 98.5.
 // ---------------------------------------------------------------------------------------
+template <bool HAS_RES, int NV>
+__global__ void __launch_bounds__(256) rmsnorm_fwd_reg_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res,
+                                                              const bf16* __restrict__ w, bf16* __restrict__ h,
+                                                              bf16* __restrict__ y, float* __restrict__ rstd_out,
+                                                              int rows, int cols, float eps) {
+  const int lane = threadIdx.x & 31;
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int nvec = cols >> 3;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * cols);
+  const uint4* rr = HAS_RES ? reinterpret_cast<const uint4*>(res + (size_t)row * cols) : nullptr;
+  uint4 a[NV], b[HAS_RES ? NV : 1];
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    const int v = lane + 32 * k;
+    a[k] = v < nvec ? xr[v] : make_uint4(0, 0, 0, 0);
+    if (HAS_RES) b[k] = v < nvec ? rr[v] : make_uint4(0, 0, 0, 0);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    float f[8];
+    unpack8(a[k], f);
+    if (HAS_RES) {
+      float g[8];
+      unpack8(b[k], g);
+#pragma unroll
+      for (int i = 0; i < 8; i++) f[i] += g[i];
+      a[k] = pack8(f);
+      if (lane + 32 * k < nvec) reinterpret_cast<uint4*>(h + (size_t)row * cols)[lane + 32 * k] = a[k];
+      unpack8(a[k], f);  // the norm sees the rounded residual stream, as a separate add would
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) ss += f[i] * f[i];
+  }
+  ss = warp_sum(ss);
+  const float rstd = rsqrtf(ss / (float)cols + eps);
+  if (lane == 0) rstd_out[row] = rstd;
+  const uint4* wv = reinterpret_cast<const uint4*>(w);
+  uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * cols);
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    const int v = lane + 32 * k;
+    if (v < nvec) {
+      float f[8], g[8];
+      unpack8(a[k], f);
+      unpack8(wv[v], g);
+#pragma unroll
+      for (int i = 0; i < 8; i++) f[i] = f[i] * rstd * g[i];
+      yr[v] = pack8(f);
+    }
+  }
+}
+
 template <bool HAS_RES>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res,
                                                           const bf16* __restrict__ w, bf16* __restrict__ h,
@@ -82,18 +139,36 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const bf16* __restrict
   }
 }
 
+template <bool HAS_RES>
+static void rmsnorm_fwd_launch(const void* x, const void* res, const void* w, void* h, void* y, void* rstd, int rows, int cols,
+                               float eps, cudaStream_t s) {
+  // fewer warps per block while that still leaves SMs without a block (a short batch)
+  int wpb = 8;
+  while (wpb > 1 && (rows + wpb - 1) / wpb < 2 * lb_num_sms()) wpb >>= 1;
+  const int blocks = (rows + wpb - 1) / wpb;
+#define LB_RMS_FWD(V)                                                                                               \
+  rmsnorm_fwd_reg_kernel<HAS_RES, V><<<blocks, 32 * wpb, 0, s>>>((const bf16*)x, (const bf16*)res, (const bf16*)w,  \
+                                                                 (bf16*)h, (bf16*)y, (float*)rstd, rows, cols, eps)
+  const int nv = (cols / 8 + 31) / 32;
+  if (nv <= 2) LB_RMS_FWD(2);
+  else if (nv <= 4) LB_RMS_FWD(4);
+  else if (nv <= 6) LB_RMS_FWD(6);
+  else if (nv <= 8) LB_RMS_FWD(8);
+  else if (nv <= 12) LB_RMS_FWD(12);
+  else if (nv <= 16) LB_RMS_FWD(16);
+  else {
+    const int b = (rows + 7) / 8 > lb_num_sms() * 8 ? lb_num_sms() * 8 : (rows + 7) / 8;
+    rmsnorm_fwd_kernel<HAS_RES><<<b, 256, 0, s>>>((const bf16*)x, (const bf16*)res, (const bf16*)w, (bf16*)h, (bf16*)y,
+                                                  (float*)rstd, rows, cols, eps);
+  }
+#undef LB_RMS_FWD
+}
+
 extern "C" int lb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* h, void* y, void* rstd, int rows,
                               int cols, float eps, void* stream) {
   if (cols % 8 || rows <= 0) return LB_ERR_SHAPE;
-  int blocks = (rows + 7) / 8;
-  if (blocks > lb_num_sms() * 8) blocks = lb_num_sms() * 8;
-  cudaStream_t s = (cudaStream_t)stream;
-  if (res)
-    rmsnorm_fwd_kernel<true><<<blocks, 256, 0, s>>>((const bf16*)x, (const bf16*)res, (const bf16*)w, (bf16*)h,
-                                                    (bf16*)y, (float*)rstd, rows, cols, eps);
-  else
-    rmsnorm_fwd_kernel<false><<<blocks, 256, 0, s>>>((const bf16*)x, nullptr, (const bf16*)w, nullptr, (bf16*)y,
-                                                     (float*)rstd, rows, cols, eps);
+  if (res) rmsnorm_fwd_launch<true>(x, res, w, h, y, rstd, rows, cols, eps, (cudaStream_t)stream);
+  else rmsnorm_fwd_launch<false>(x, res, w, h, y, rstd, rows, cols, eps, (cudaStream_t)stream);
   LB_CHECK_LAUNCH();
   return LB_OK;
 }
@@ -154,40 +229,60 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict
 }
 
 // Block-per-row version (no shared-memory atomics): the block's T threads cover one row with VPT
-// uint4 each (cols = 8 * T * VPT), so a thread owns the same 8*VPT columns of every row and keeps
-// their dw partial sums in registers.  RB rows are in flight per iteration; their dy / x stay in
+// uint4 each (cols <= 8 * T * VPT, lanes past the end idle), so a thread owns the same 8*VPT columns of every
+// row and keeps their dw partial sums in registers.  RB rows are in flight per iteration; their dy / x stay in
 // registers between the dot product (one block reduction per iteration, double-buffered so a single
-// barrier suffices) and the dx pass.
-template <int VPT, int RB>
-__global__ void __launch_bounds__(256, (VPT == 1 ? 3 : (VPT <= 3 ? 2 : 1))) rmsnorm_bwd_blk_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
-                                                              const bf16* __restrict__ w, const float* __restrict__ rstd,
-                                                              const bf16* __restrict__ dres, bf16* __restrict__ dx,
-                                                              float* __restrict__ partial, int rows, int cols) {
+// barrier suffices) and the dx pass.  Memory bound: the loads of the next RB rows are issued before the
+// reduction of the current ones, so the barrier does not leave the memory idle (16384 x 4096 with the residual gradient,
+// loads behind the barrier / before it: 133 / 92 us for the autograd call).
+template <int VPT>
+struct RmsBwdCfg {
+  static constexpr int RB = VPT == 1 ? 2 : 1;
+  static constexpr int PER_SM = VPT <= 2 ? 2 : 1;        // resident blocks of 256 threads (registers)
+};
+template <int VPT>
+__global__ void __launch_bounds__(256, RmsBwdCfg<VPT>::PER_SM)
+rmsnorm_bwd_blk_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
+                       const float* __restrict__ rstd, const bf16* __restrict__ dres, bf16* __restrict__ dx,
+                       float* __restrict__ partial, int rows, int cols) {
+  constexpr int RB = RmsBwdCfg<VPT>::RB;
   __shared__ float s_red[2][RB][8];
   const int T = blockDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = T >> 5;
+  const int nvec = cols >> 3;
   const float inv_cols = 1.f / (float)cols;
   float wf[VPT][8], acc[VPT][8];
+  bool in[VPT];
 #pragma unroll
   for (int k = 0; k < VPT; k++) {
-    unpack8(reinterpret_cast<const uint4*>(w)[t + T * k], wf[k]);
+    in[k] = t + T * k < nvec;
+    const uint4 wv = in[k] ? reinterpret_cast<const uint4*>(w)[t + T * k] : make_uint4(0, 0, 0, 0);
+    unpack8(wv, wf[k]);
 #pragma unroll
     for (int i = 0; i < 8; i++) acc[k][i] = 0.f;
   }
-  int par = 0;
-  for (int row0 = blockIdx.x * RB; row0 < rows; row0 += gridDim.x * RB, par ^= 1) {
-    uint4 kd[RB][VPT], kx[RB][VPT];
-    float r[RB], dot[RB];
+  uint4 kd[RB][VPT], kx[RB][VPT], ke[RB][VPT];
+  float r[RB];
+  auto load = [&](int row0, uint4 (&d)[RB][VPT], uint4 (&xx)[RB][VPT], uint4 (&e)[RB][VPT], float (&rr)[RB]) {
 #pragma unroll
     for (int rb = 0; rb < RB; rb++) {
       const int row = row0 + rb;
       const bool ok = row < rows;
-      r[rb] = ok ? rstd[row] : 0.f;
+      rr[rb] = ok ? rstd[row] : 0.f;
 #pragma unroll
       for (int k = 0; k < VPT; k++) {
-        kd[rb][k] = ok ? reinterpret_cast<const uint4*>(dy + (size_t)row * cols)[t + T * k] : make_uint4(0, 0, 0, 0);
-        kx[rb][k] = ok ? reinterpret_cast<const uint4*>(x + (size_t)row * cols)[t + T * k] : make_uint4(0, 0, 0, 0);
+        const size_t at = (size_t)row * nvec + t + T * k;
+        d[rb][k] = ok && in[k] ? reinterpret_cast<const uint4*>(dy)[at] : make_uint4(0, 0, 0, 0);
+        xx[rb][k] = ok && in[k] ? reinterpret_cast<const uint4*>(x)[at] : make_uint4(0, 0, 0, 0);
+        e[rb][k] = ok && in[k] && dres ? reinterpret_cast<const uint4*>(dres)[at] : make_uint4(0, 0, 0, 0);
       }
     }
+  };
+  int par = 0;
+  load(blockIdx.x * RB, kd, kx, ke, r);
+  for (int row0 = blockIdx.x * RB; row0 < rows; row0 += gridDim.x * RB, par ^= 1) {
+    uint4 nd[RB][VPT], nx[RB][VPT], ne[RB][VPT];
+    float nr[RB], dot[RB];
+    load(row0 + gridDim.x * RB, nd, nx, ne, nr);
 #pragma unroll
     for (int rb = 0; rb < RB; rb++) {
       float d = 0.f;
@@ -215,50 +310,50 @@ __global__ void __launch_bounds__(256, (VPT == 1 ? 3 : (VPT <= 3 ? 2 : 1))) rmsn
       if (row >= rows) break;
 #pragma unroll
       for (int k = 0; k < VPT; k++) {
-        float a[8], b[8], o[8];
+        float a[8], b[8], o[8], e[8];
         unpack8(kd[rb][k], a);
         unpack8(kx[rb][k], b);
+        unpack8(ke[rb][k], e);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
           const float xhat = b[i] * r[rb];
-          o[i] = r[rb] * (a[i] * wf[k][i] - xhat * dot[rb]);
+          o[i] = r[rb] * (a[i] * wf[k][i] - xhat * dot[rb]) + e[i];
           acc[k][i] += a[i] * xhat;
         }
-        if (dres) {
-          float e[8];
-          unpack8(reinterpret_cast<const uint4*>(dres + (size_t)row * cols)[t + T * k], e);
-#pragma unroll
-          for (int i = 0; i < 8; i++) o[i] += e[i];
-        }
-        reinterpret_cast<uint4*>(dx + (size_t)row * cols)[t + T * k] = pack8(o);
+        if (in[k]) reinterpret_cast<uint4*>(dx)[(size_t)row * nvec + t + T * k] = pack8(o);
       }
+    }
+#pragma unroll
+    for (int rb = 0; rb < RB; rb++) {
+      r[rb] = nr[rb];
+#pragma unroll
+      for (int k = 0; k < VPT; k++) { kd[rb][k] = nd[rb][k]; kx[rb][k] = nx[rb][k]; ke[rb][k] = ne[rb][k]; }
     }
   }
 #pragma unroll
   for (int k = 0; k < VPT; k++) {
+    if (!in[k]) continue;
     float* dst = partial + (size_t)blockIdx.x * cols + (size_t)(t + T * k) * 8;
     *reinterpret_cast<float4*>(dst) = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
     *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[k][4], acc[k][5], acc[k][6], acc[k][7]);
   }
 }
 
-// Launches the block-per-row version when the width fits it (cols = 8 * T * VPT with T a multiple
-// of 32, T <= 256, VPT <= 4); returns false otherwise.
+// Launches the block-per-row version (rows of up to 8192 columns); returns false for wider ones.
 static bool rmsnorm_bwd_blk_dispatch(const void* dy, const void* x, const void* w, const void* rstd, const void* dres,
                                      void* dx, void* partial, int rows, int cols, int nblk, cudaStream_t s) {
   const int nvec = cols / 8;
   const int vpt = (nvec + 255) / 256;
-  if (vpt > 4 || nvec % vpt) return false;
-  const int T = nvec / vpt;
-  if (T % 32) return false;
-#define LB_RMS_BLK(V, R)                                                                                          \
-  rmsnorm_bwd_blk_kernel<V, R><<<nblk, T, 0, s>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)rstd, \
-                                                  (const bf16*)dres, (bf16*)dx, (float*)partial, rows, cols)
+  if (vpt > 4) return false;
+  const int T = ((nvec + vpt - 1) / vpt + 31) / 32 * 32;
+#define LB_RMS_BLK(V)                                                                                             \
+  rmsnorm_bwd_blk_kernel<V><<<nblk, T, 0, s>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)rstd, \
+                                               (const bf16*)dres, (bf16*)dx, (float*)partial, rows, cols)
   switch (vpt) {
-    case 1: LB_RMS_BLK(1, 2); break;
-    case 2: LB_RMS_BLK(2, 2); break;
-    case 3: LB_RMS_BLK(3, 1); break;
-    default: LB_RMS_BLK(4, 1); break;
+    case 1: LB_RMS_BLK(1); break;
+    case 2: LB_RMS_BLK(2); break;
+    case 3: LB_RMS_BLK(3); break;
+    default: LB_RMS_BLK(4); break;
   }
 #undef LB_RMS_BLK
   return true;
@@ -284,15 +379,22 @@ __global__ void __launch_bounds__(1024) rmsnorm_dw_reduce_kernel(const float* __
 
 // Number of blocks (= rows of the `partial` scratch) that lb_rmsnorm_bwd uses for this shape.
 extern "C" int lb_rmsnorm_bwd_blocks(int rows, int cols) {
-  // as many blocks as are resident at once (one wave of the grid-stride loop): the block-per-row
-  // kernel fits 3 / 2 / 2 / 1 blocks per SM for 1 / 2 / 3 / 4 vectors per thread, the atomics
-  // version 2
+  // As many blocks as are resident at once (one wave of the grid-stride loop), and no block without rows: the
+  // block-per-row kernel takes 2 / 1 / 1 / 1 rows per iteration for 1 / 2 / 3 / 4 vectors per thread and
+  // more of its narrow blocks fit; the atomics version has a warp per row.
   const int nvec = cols / 8;
   const int vpt = (nvec + 255) / 256;
-  const bool blk = vpt <= 4 && nvec % vpt == 0 && (nvec / vpt) % 32 == 0;
-  const int per_sm = !blk ? 2 : (vpt == 1 ? 3 : (vpt <= 3 ? 2 : 1));
-  int blocks = (rows + 7) / 8;
-  if (blocks > lb_num_sms() * per_sm) blocks = lb_num_sms() * per_sm;
+  int blocks, cap;
+  if (vpt <= 4) {
+    const int rb = vpt == 1 ? RmsBwdCfg<1>::RB : RmsBwdCfg<2>::RB;
+    const int T = ((nvec + vpt - 1) / vpt + 31) / 32 * 32;
+    blocks = (rows + rb - 1) / rb;
+    cap = lb_num_sms() * (vpt <= 2 ? RmsBwdCfg<1>::PER_SM * (256 / T) : RmsBwdCfg<3>::PER_SM);
+  } else {
+    blocks = (rows + 7) / 8;
+    cap = lb_num_sms() * 2;
+  }
+  if (blocks > cap) blocks = cap;
   return blocks < 1 ? 1 : blocks;
 }
 

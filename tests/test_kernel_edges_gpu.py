@@ -107,3 +107,29 @@ def test_swiglu_mlp_pair_tiles(T, K, I):
     yd = (torch.nn.functional.silu(x @ w1.t()) * (x @ w3.t())) @ w2.t()
     for g, w in zip(got, (yd, *torch.autograd.grad(yd, [x, w1, w3, w2], dy.double()))):
         assert _rel(g, w) < 1e-2
+
+
+# ---- norm ----------------------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 264), (700, 1448), (301, 2056), (130, 4096), (65, 4104), (9, 8192), (5, 8200)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_rmsnorm_widths(rows, cols, residual):
+    from lightron_b200.ops import functional as OF
+    x, r, w = _rand(rows, cols, seed=1), _rand(rows, cols, seed=2), (1 + 0.1 * _rand(cols, seed=3).float()).to(torch.bfloat16)
+    dh, dy = _rand(rows, cols, seed=4), _rand(rows, cols, seed=5)
+
+    def grads(norm, conv):
+        xs = [conv(t).requires_grad_(True) for t in ((x, r, w) if residual else (x, w))]
+        outs = norm(*xs)
+        return (*outs, *torch.autograd.grad(outs, xs, [conv(t) for t in ((dh, dy) if residual else (dy,))]))
+
+    def norm64(*xs):
+        h = xs[0] + xs[1] if residual else xs[0]
+        y = h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-5) * xs[-1]
+        return (h, y) if residual else (y,)
+
+    def norm_native(*xs):
+        return OF.add_rmsnorm(*xs, 1e-5) if residual else (OF.rmsnorm(*xs, 1e-5),)
+    for g, want in zip(grads(norm_native, lambda t: t.clone()), grads(norm64, lambda t: t.double())):
+        assert _rel(g, want) < 5e-3

@@ -669,6 +669,38 @@ extern "C" int lb_ce_stats(const void* logits, const void* tgt, void* mx, void* 
   return LB_OK;
 }
 
+// lse[t] = log-sum-exp of row t, loss[0] = inv_n * sum over the rows whose target counts of (lse - target logit).  One block: the
+// sums of a row are three floats, and a fixed order makes the loss the same every time.
+__global__ void __launch_bounds__(1024) ce_loss_kernel(const float* __restrict__ mx, const float* __restrict__ se,
+                                                       const float* __restrict__ tl, const long long* __restrict__ tgt,
+                                                       float* __restrict__ lse, float* __restrict__ loss, int T, float inv_n,
+                                                       int ignore_index) {
+  float s = 0.f;
+#pragma unroll 4
+  for (int t = threadIdx.x; t < T; t += 1024) {
+    const float l = mx[t] + (float)log((double)se[t]);      // (logf is the approximate one under fast math)
+    lse[t] = l;
+    if (tgt[t] != ignore_index) s += l - tl[t];
+  }
+  s = warp_sum(s);
+  __shared__ float sh[32];
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = warp_sum(sh[threadIdx.x]);
+    if (threadIdx.x == 0) loss[0] = s * inv_n;
+  }
+}
+
+extern "C" int lb_ce_loss(const void* mx, const void* se, const void* tl, const void* tgt, void* lse, void* loss, int T, float inv_n,
+                          int ignore_index, void* stream) {
+  if (T <= 0) return LB_ERR_SHAPE;
+  ce_loss_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>((const float*)mx, (const float*)se, (const float*)tl,
+                                                       (const long long*)tgt, (float*)lse, (float*)loss, T, inv_n, ignore_index);
+  LB_CHECK_LAUNCH();
+  return LB_OK;
+}
+
 extern "C" int lb_ce_grad(const void* logits, const void* tgt, const void* lse, void* dlogits, const void* dloss, int T,
                           int V, long long ld, int v0, float inv_n, int ignore_index, void* stream) {
   if (V % 8 || ld % 8 || T <= 0) return LB_ERR_SHAPE;

@@ -760,11 +760,16 @@ class _CrossEntropy(torch.autograd.Function):
             packed = torch.stack((se * torch.exp(mx - gmx), tl))
             dist.all_reduce(packed, op=dist.ReduceOp.SUM, group=group)
             se, tl, mx = packed[0], packed[1], gmx
-        lse = mx + torch.log(se)
-        valid = tgt != ignore_index
-        n_valid = n_valid_total if n_valid_total is not None else int(valid.sum().item())
-        per_tok = torch.where(valid, lse - tl, torch.zeros_like(lse))
-        loss = per_tok.sum() / max(n_valid, 1)
+        n_valid = n_valid_total if n_valid_total is not None else int((tgt != ignore_index).sum().item())
+        if use_native:
+            lse = torch.empty_like(mx)
+            loss = torch.empty((), dtype=torch.float32, device=logits.device)
+            native.call("lb_ce_loss", mx.data_ptr(), se.data_ptr(), tl.data_ptr(), tgt.data_ptr(), lse.data_ptr(),
+                        loss.data_ptr(), T, 1.0 / max(n_valid, 1), ignore_index, native.stream_ptr())
+        else:
+            lse = mx + torch.log(se)
+            per_tok = torch.where(tgt != ignore_index, lse - tl, torch.zeros_like(lse))
+            loss = per_tok.sum() / max(n_valid, 1)
         ctx.save_for_backward(logits, tgt, lse)
         ctx.meta = (vocab_start, n_valid, ignore_index, use_native)
         return loss

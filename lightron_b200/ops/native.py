@@ -43,6 +43,7 @@ _SIGNATURES = {
     "lb_embedding_fwd": [_P, _P, _P, _I, _I, _I, _I, _P],
     "lb_embedding_bwd": [_P, _P, _P, _I, _I, _I, _I, _P],
     "lb_ce_stats": [_P, _P, _P, _P, _P, _I, _I, _L, _I, _P],
+    "lb_ce_loss": [_P, _P, _P, _P, _P, _P, _I, _F, _I, _P],
     "lb_ce_grad": [_P, _P, _P, _P, _P, _I, _I, _L, _I, _F, _I, _P],
     "lb_adamw": [_P, _P, _P, _P, _P, _L, _F, _F, _F, _F, _F, _F, _F, _F, _I, _P],
     "lb_sumsq": [_P, _L, _P, _I, _P],

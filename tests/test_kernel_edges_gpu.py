@@ -133,3 +133,21 @@ def test_rmsnorm_widths(rows, cols, residual):
         return OF.add_rmsnorm(*xs, 1e-5) if residual else (OF.rmsnorm(*xs, 1e-5),)
     for g, want in zip(grads(norm_native, lambda t: t.clone()), grads(norm64, lambda t: t.double())):
         assert _rel(g, want) < 5e-3
+
+
+# ---- loss ------------------------------------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("T,V", [(1, 8), (33, 264), (1025, 1000), (4100, 64)])
+def test_cross_entropy_loss_rows(T, V):
+    """Fewer rows than threads, more, ignored ones; the loss is an fp32 sum (1e-6) of fp32 rows over bf16 logits."""
+    from lightron_b200.ops import functional as OF
+    logits, tgt = _rand(T, V, scale=3.0, seed=1), torch.randint(0, V, (T,), device="cuda", generator=torch.Generator("cuda").manual_seed(2))
+    tgt[1::7] = -100
+    x = logits.clone().requires_grad_(True)
+    loss = OF.cross_entropy(x * 1, tgt)
+    got, = torch.autograd.grad(loss, x)
+    w = logits.double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(w, tgt)
+    assert abs(loss.item() - want.item()) < 4e-6 * max(1.0, want.item())
+    assert _rel(got, torch.autograd.grad(want, w)[0]) < 5e-3

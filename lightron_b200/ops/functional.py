@@ -19,6 +19,23 @@ import torch.nn.functional as F
 
 from . import native, reference as ref
 
+class _NoGradCtx:
+    """Stands in for the context of an autograd function whose backward cannot be asked for."""
+
+    def save_for_backward(self, *tensors):
+        pass
+
+
+def _apply(fn, *args):
+    """``fn.apply(*args)``; with gradients off, only ``fn.forward``: the autograd function then records nothing, and its
+    Python wrapper is most of the host time of a small call.  Whatever else looks at autograd functions (function transforms, forward-mode
+    derivatives, tracing) still gets the function."""
+    if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or torch._C._get_tracing_state() is not None
+            or torch.autograd.forward_ad._current_level >= 0):
+        return fn.apply(*args)
+    return fn.forward(_NoGradCtx(), *args)
+
+
 # --------------------------------------------------------------------------------------
 # GEMM
 # --------------------------------------------------------------------------------------
@@ -283,7 +300,7 @@ def swiglu_mlp_ok(x: torch.Tensor, w1, w3, w2) -> bool:
 def swiglu_mlp(x: torch.Tensor, w1: torch.Tensor, w3: torch.Tensor, w2: torch.Tensor) -> torch.Tensor:
     """``w2(silu(w1 x) * w3 x)`` for [n, K] weights; the fused-epilogue kernels when they apply."""
     if swiglu_mlp_ok(x, w1, w3, w2):
-        return _SwiGLUMLP.apply(x, w1, w3, w2)
+        return _apply(_SwiGLUMLP, x, w1, w3, w2)
     return linear(swiglu(linear(x, w1, w3)), w2)
 
 
@@ -364,7 +381,7 @@ def grouped_linear(x: torch.Tensor, counts, groups) -> torch.Tensor:
     (one launch for all local experts; the reference applies a single expert, model/model.py:109)."""
     if grouped_linear_ok(x, groups):
         flat = [w for ws in groups for w in ws]
-        return _GroupedLinear.apply(x, list(counts), len(groups[0]), *flat)
+        return _apply(_GroupedLinear, x, list(counts), len(groups[0]), *flat)
     outs, off = [], 0
     for c, ws in zip(counts, groups):
         outs.append(linear(x[off:off + c], *ws))
@@ -377,7 +394,7 @@ def grouped_linear(x: torch.Tensor, counts, groups) -> torch.Tensor:
 def linear(x: torch.Tensor, *ws: torch.Tensor) -> torch.Tensor:
     """x [..., K] times one or more [n_i, K] weights -> [..., sum n_i]."""
     if native.use_native(x) and x.shape[-1] % 8 == 0 and all(w.shape[0] % 8 == 0 for w in ws):
-        return _Linear.apply(x, *ws)
+        return _apply(_Linear, x, *ws)
     # CPU / fp32 oracle path, and GEMMs whose widths are not multiples of 8 (a MoE router with
     # fewer than 8 experts): TMA needs 16-byte rows, and such a GEMM is tiny anyway
     if len(ws) == 1:
@@ -448,14 +465,14 @@ class _RMSNorm(torch.autograd.Function):
 
 def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
     if native.use_native(x):
-        return _RMSNorm.apply(x, None, w, eps)
+        return _apply(_RMSNorm, x, None, w, eps)
     return ref.rmsnorm(x, w, eps)
 
 
 def add_rmsnorm(x: torch.Tensor, res: torch.Tensor, w: torch.Tensor, eps: float) -> Tuple[torch.Tensor, torch.Tensor]:
     """h = x + res; y = rmsnorm(h).  Returns (h, y) from one pass over memory."""
     if native.use_native(x):
-        return _RMSNorm.apply(x, res, w, eps)
+        return _apply(_RMSNorm, x, res, w, eps)
     h = x + res
     return h, ref.rmsnorm(h, w, eps)
 
@@ -495,7 +512,7 @@ def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, positions: Optio
     if native.use_native(x):
         if positions is not None and positions.dtype != torch.int32:
             positions = positions.to(torch.int32)
-        return _Rope.apply(x, cos, sin, positions)
+        return _apply(_Rope, x, cos, sin, positions)
     return ref.rope(x, cos, sin, positions)
 
 
@@ -532,7 +549,7 @@ class _SwiGLU(torch.autograd.Function):
 def swiglu(gu: torch.Tensor) -> torch.Tensor:
     """gu [..., 2I] holding gate | up -> silu(gate) * up [..., I]."""
     if native.use_native(gu):
-        return _SwiGLU.apply(gu)
+        return _apply(_SwiGLU, gu)
     I = gu.shape[-1] // 2
     return ref.swiglu(gu[..., :I], gu[..., I:])
 
@@ -621,7 +638,7 @@ def flash_attention(q, k, v, causal: bool = True, scale: Optional[float] = None)
     """q [B,Sq,hq,d], k/v [B,Sk,hkv,d] -> [B,Sq,hq,d]; GQA by indexing (no repeat_kv)."""
     scale = 1.0 / math.sqrt(q.shape[-1]) if scale is None else scale
     if native.use_native(q):
-        return _FlashAttn.apply(q, k, v, causal, scale)
+        return _apply(_FlashAttn, q, k, v, causal, scale)
     return ref.attention(q, k, v, causal=causal, scale=scale)
 
 
@@ -676,7 +693,7 @@ def rope_attention_qkv(qkv: torch.Tensor, cos, sin, positions, B: int, S: int, h
     if native.use_native(qkv):
         if positions is not None and positions.dtype != torch.int32:
             positions = positions.to(torch.int32)
-        return _RopeAttnQKV.apply(qkv, cos, sin, positions, B, S, hq, hkv, d, scale)
+        return _apply(_RopeAttnQKV, qkv, cos, sin, positions, B, S, hq, hkv, d, scale)
     T = B * S
     q, k, v = qkv.view(T, -1).split([hq * d, hkv * d, hkv * d], dim=-1)
     q = ref.rope(q.reshape(B, S, hq, d), cos, sin, positions)
@@ -720,7 +737,7 @@ def embedding(tokens: torch.Tensor, w: torch.Tensor, vocab_start: int = 0) -> to
     """Rows of ``w`` (which holds vocab ids [vocab_start, vocab_start + w.shape[0])); ids outside
     the range give zero rows (vocab-parallel partial result, parallel/parallel_tp.py:131-143)."""
     if native.use_native(w):
-        return _Embedding.apply(tokens, w, vocab_start)
+        return _apply(_Embedding, tokens, w, vocab_start)
     local = tokens - vocab_start
     mask = (local < 0) | (local >= w.shape[0])
     out = F.embedding(local.masked_fill(mask, 0), w)
@@ -801,4 +818,4 @@ def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int 
     """Mean NLL of [T, V_local] logits.  With ``group`` the vocab dim is sharded across it.
     ``n_valid_total`` (the number of non-ignored targets) avoids a host sync when known."""
     logits2 = logits.reshape(-1, logits.shape[-1])
-    return _CrossEntropy.apply(logits2, targets, vocab_start, group, n_valid_total, ignore_index)
+    return _apply(_CrossEntropy, logits2, targets, vocab_start, group, n_valid_total, ignore_index)

@@ -173,7 +173,9 @@ def measured_peaks() -> dict:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current device's current stream (``torch.cuda.current_stream().cuda_stream`` without building the
+    ``Stream`` object, which costs as much as the launch's argument conversion)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t: Optional[torch.Tensor]) -> int:

@@ -1,0 +1,61 @@
+"""With gradients off the ops call an autograd function's forward directly; everything that looks at autograd functions
+still gets the function."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwAD
+
+from lightron_b200.ops import functional as OF
+
+
+class _Twice(torch.autograd.Function):
+    applied = 0
+
+    @staticmethod
+    def forward(ctx, x, y):
+        ctx.save_for_backward(x, y)
+        ctx.shape = x.shape
+        return 2 * x + y
+
+    @staticmethod
+    def backward(ctx, g):
+        return 2 * g, g
+
+
+@pytest.fixture
+def wrapped(monkeypatch):
+    calls = []
+    real = _Twice.apply
+    monkeypatch.setattr(_Twice, "apply", lambda *a: (calls.append(1), real(*a))[1])
+    return calls
+
+
+def test_gradients_on_uses_the_function(wrapped):
+    x, y = torch.randn(3, requires_grad=True), torch.randn(3)
+    out = OF._apply(_Twice, x, y)
+    out.sum().backward()
+    assert wrapped and torch.equal(x.grad, torch.full((3,), 2.0))
+    saved = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: saved.append(t) or t, lambda t: t):
+        OF._apply(_Twice, x, y)
+    assert len(saved) == 2
+
+
+@pytest.mark.parametrize("mode", [torch.no_grad, torch.inference_mode])
+def test_gradients_off_gives_the_same_values(wrapped, mode):
+    x, y = torch.randn(3, requires_grad=True), torch.randn(3)
+    with mode():
+        got = OF._apply(_Twice, x, y)
+    assert not wrapped and not got.requires_grad and torch.equal(got, 2 * x.detach() + y)
+
+
+def test_transforms_and_tangents_still_reach_the_function(wrapped):
+    x, y = torch.randn(4, 3), torch.randn(4, 3)
+    with torch.no_grad():
+        with pytest.raises(RuntimeError):                       # no vmap rule: refused, not computed on wrappers
+            torch.func.vmap(lambda a, b: OF._apply(_Twice, a, b))(x, y)
+        assert wrapped
+        wrapped.clear()
+        with fwAD.dual_level():
+            with pytest.raises(Exception):                      # no jvp rule: refused, the tangent is not dropped
+                OF._apply(_Twice, fwAD.make_dual(x, torch.ones_like(x)), y)
+        assert wrapped

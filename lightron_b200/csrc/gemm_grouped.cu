@@ -729,7 +729,9 @@ void set_tiles(Problem* p, int cg) {
 // CTAs per tile for this set of problems: pairs unless their coarser tiles make the busiest worker's list more than 5 % longer
 // (few or ragged tiles), which is what a pair's tile gains.  Measured with 16384 rows, CTAs against pairs: N11264 K2048
 // 584 / 546 us, N2560 K2048 134 / 126, N2048 K2048 106 / 103, N2048 K5632 259 / 254; data + weight gradient of these layers 1167 / 1142,
-// 286 / 262, 234 / 214, 623 / 622.  Pairs forced on few tiles lose: 4096 x 2304 x 768 takes 27 us with CTAs, 31 with pairs.
+// 286 / 262, 234 / 214, 623 / 575.  A launch of one or two short tiles per SM (a load below 64 k-blocks) pays more for setting up the
+// pairs than they gain: 512 / 1000 x 2304 x 768 takes 16.7 / 17.3 us with CTAs and 20.6 with pairs, 4096 x 2304 x 768 (load 36) 22.6 to
+// 26.8 and 24.9 to 31.7 (all with the launch).
 int choose_cg(Problem* probs, int np, int sms) {
   if (sms < 2) return 1;
   long long load[3] = {0, 0, 0};
@@ -738,7 +740,7 @@ int choose_cg(Problem* probs, int np, int sms) {
     load[cg] = assign_items(probs, np, sms / cg, nullptr, nullptr, nullptr);
     if (load[cg] < 0) return -1;
   }
-  return load[2] * 100 <= load[1] * 105 ? 2 : 1;
+  return load[2] >= 64 && load[2] * 100 <= load[1] * 105 ? 2 : 1;
 }
 
 int build_schedule(Problem* probs, int np, int sms, Schedule* out) {

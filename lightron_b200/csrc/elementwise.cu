@@ -844,7 +844,7 @@ extern "C" int lb_add_inplace(void* a, const void* b, long long n, void* stream)
 //    blocks may differ (fewer, larger blocks), which changes dw by fp32 rounding only.
 //  * It always runs the general kernel (row per warp, dw partial sums through shared-memory
 //    atomics), not the faster block-per-row kernel that lb_rmsnorm_bwd picks for common widths:
-//    that one needs one scratch row per resident block, up to 444 rows, which would not fit the
+//    that one needs one scratch row per resident block, up to 16 per SM, which would not fit the
 //    128 rows of the fixed array.  Expect roughly 1.5x the run time of lb_rmsnorm_bwd.
 // ---------------------------------------------------------------------------------------
 #define LB_STATIC_SCRATCH_MAX_COLS 8192

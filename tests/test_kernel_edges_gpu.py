@@ -151,3 +151,31 @@ def test_cross_entropy_loss_rows(T, V):
     want = torch.nn.functional.cross_entropy(w, tgt)
     assert abs(loss.item() - want.item()) < 4e-6 * max(1.0, want.item())
     assert _rel(got, torch.autograd.grad(want, w)[0]) < 5e-3
+
+
+# ---- mixture of experts ------------------------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("T,H,E,k", [(1, 64, 4, 2), (70, 264, 5, 1), (300, 512, 40, 3), (65, 2056, 64, 8)])
+def test_moe_router_tiles(T, H, E, k):
+    """Ragged last block of tokens, a width that is no multiple of the column tile, one to eight passes over the experts."""
+    from lightron_b200.ops import native
+    x, wg, dev = _rand(T, H, seed=1), _rand(E, H, scale=H ** -0.5, seed=2), "cuda"
+    lib = native.require()
+    nblk = lib.lb_moe_router_blocks(T)
+    probs, wts = torch.empty(T, E, device=dev), torch.empty(T, k, device=dev)
+    idx, within = torch.empty(T, k, dtype=torch.int32, device=dev), torch.zeros(nblk * 32, k, dtype=torch.int32, device=dev)
+    hist, psum = torch.empty(nblk, E, dtype=torch.int32, device=dev), torch.empty(nblk, E, device=dev)
+    native.call("lb_moe_router", x.data_ptr(), wg.data_ptr(), T, H, E, k, probs.data_ptr(), idx.data_ptr(), wts.data_ptr(),
+                within.data_ptr(), hist.data_ptr(), psum.data_ptr(), native.stream_ptr())
+    xd, wd = x.double().requires_grad_(True), wg.double().requires_grad_(True)
+    want = (xd @ wd.t()).softmax(-1)
+    assert torch.allclose(probs.double(), want, atol=1e-6, rtol=1e-4)          # fp32 sums of H exact products
+    assert torch.equal(torch.gather(probs, 1, idx.long()), wts) and torch.equal(hist.sum(0), torch.bincount(idx.reshape(-1), minlength=E).int())
+    dwts, frac, daux = torch.randn(T, k, device=dev), torch.rand(E, device=dev), torch.tensor([0.7], device=dev)
+    dx, dwg = torch.empty_like(x), torch.zeros(E, H, device=dev)
+    native.call("lb_moe_router_bwd", x.data_ptr(), wg.data_ptr(), probs.data_ptr(), idx.data_ptr(), dwts.data_ptr(), frac.data_ptr(),
+                daux.data_ptr(), dx.data_ptr(), dwg.data_ptr(), T, H, E, k, native.stream_ptr())
+    loss = (want.gather(1, idx.long()) * dwts.double()).sum() + 0.7 * E * (frac.double() * want.mean(0)).sum()
+    gx, gw = torch.autograd.grad(loss, [xd, wd])
+    assert _rel(dx, gx) < 5e-3 and _rel(dwg, gw) < 1e-4

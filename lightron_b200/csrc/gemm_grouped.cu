@@ -608,7 +608,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
     for (int t = blockIdx.x;; t += gridDim.x) {
       const RaggedTile rt = ragged_tile(t, rp, s_off, s_tiles);
       if (rt.e < 0) break;
-      if (rt.num_kb == 0) continue;
+      if (rt.num_kb == 0) {
+        // an expert without rows: its weight gradient is zero (nothing to add when accumulating)
+        const int row = rt.m0 + quad * 32 + lane;
+        if (rp.mode == 1 && !rp.accumulate && row < rp.M_w)
+          for (int c = rt.n0; c < rt.n0 + BN && c < rp.N; c += 8)
+            *reinterpret_cast<uint4*>(rp.C[rt.e] + (size_t)row * rp.ldc + c) = make_uint4(0, 0, 0, 0);
+        continue;
+      }
       const int acc = n & 1;
       const uint32_t acc_phase = (uint32_t)(n >> 1) & 1u;
       if (!bw::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) { give_up(abort_flag, 4u); break; }
@@ -955,7 +962,8 @@ extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, cons
 }
 
 //  Weight gradients: C_e [Nw, Kw] (+)= dY[rows of e, Nw]^T . X[rows of e, Kw]; C: host array of LE
-//  gradient pointers with leading dimension ldc.
+//  gradient pointers with leading dimension ldc.  Without accumulate every C_e is written whole (zeros for an expert
+//  without rows).
 extern "C" int lb_gemm_ragged_wgrad(const void* dY, const void* X, void* const* C, const void* seg, int LE, int cap, int Nw,
                                     int Kw, long long lddy, long long ldx, long long ldc, int accumulate, void* stream) {
   if (LE < 1 || LE > MAX_PROBLEMS || cap <= 0 || Nw <= 0 || Kw <= 0) return LB_ERR_SHAPE;

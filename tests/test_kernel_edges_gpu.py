@@ -179,3 +179,30 @@ def test_moe_router_tiles(T, H, E, k):
     loss = (want.gather(1, idx.long()) * dwts.double()).sum() + 0.7 * E * (frac.double() * want.mean(0)).sum()
     gx, gw = torch.autograd.grad(loss, [xd, wd])
     assert _rel(dx, gx) < 5e-3 and _rel(dwg, gw) < 1e-4
+
+
+def test_moe_expert_without_tokens_gets_zero_gradients():
+    """Gradients outside an arena are written, not accumulated, into memory that holds anything."""
+    from lightron_b200.config import ModelArgs
+    from lightron_b200.models.llama import LightronTransformer, flatten_parameters
+    from lightron_b200.models.moe import MoEFeedForward
+    H, I, E = 256, 520, 4
+    ctx = LightronTransformer(ModelArgs(dim=64, n_layers=0, n_heads=1, vocab_size=64)).ctx
+    layer = MoEFeedForward(ModelArgs(dim=H, n_layers=1, n_heads=4, vocab_size=64, intermediate_size=I, moe_num_experts=E, moe_topk=2,
+                                     moe_layer_freq=1), ctx, dtype=torch.bfloat16, device="cuda")
+    flatten_parameters(layer)
+    x = _rand(300, H, seed=1).abs().requires_grad_(True)
+    with torch.no_grad():
+        for i, p in enumerate(layer.parameters()):
+            p.copy_(_rand(*p.shape, scale=p.shape[1] ** -0.5, seed=10 + i))
+        layer.gate.weight[2] = -1.0                              # x >= 0: expert 2 is never among the best two
+    for p in layer.parameters():
+        p.grad = None
+    junk = [torch.full((E, 2 * I, H), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    del junk
+    names, ps = zip(*layer.named_parameters())
+    grads = dict(zip(names, torch.autograd.grad(layer(x), ps, _rand(300, H, seed=3))))
+    _status_ok()
+    for n, g in grads.items():
+        assert torch.isfinite(g).all(), n
+        assert ("experts.2." in n) == (not g.any()), n

@@ -557,17 +557,31 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ tok, const bf
   }
 }
 
+// WIDE: one 16-byte reduction for 8 columns instead of four atomics (dy and dw on 16-byte boundaries).  The rounding of every
+// element is the same; bound by the number of reductions that L2 takes (16384 x 2048 into 32000 rows, forward and backward with
+// the clear of dw: 108 us with atomics, 92 with the wide reductions).
+template <bool WIDE>
 __global__ void embedding_bwd_kernel(const long long* __restrict__ tok, const bf16* __restrict__ dy,
                                      bf16* __restrict__ dw, int T, int H, int v0, int v1) {
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
-  const int npair = H >> 1;
   for (int t = blockIdx.x * wpb + (threadIdx.x >> 5); t < T; t += gridDim.x * wpb) {
     const long long id = tok[t];
     if (id < v0 || id >= v1) continue;
-    const bf162* src = reinterpret_cast<const bf162*>(dy + (size_t)t * H);
-    bf162* dst = reinterpret_cast<bf162*>(dw + (size_t)(id - v0) * H);
-    for (int v = lane; v < npair; v += 32) atomicAdd(dst + v, src[v]);
+    if (WIDE) {
+      const uint4* src = reinterpret_cast<const uint4*>(dy + (size_t)t * H);
+      uint4* dst = reinterpret_cast<uint4*>(dw + (size_t)(id - v0) * H);
+#pragma unroll 4
+      for (int v = lane; v < (H >> 3); v += 32) {
+        const uint4 a = src[v];
+        asm volatile("red.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(dst + v), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w)
+                     : "memory");
+      }
+    } else {
+      const bf162* src = reinterpret_cast<const bf162*>(dy + (size_t)t * H);
+      bf162* dst = reinterpret_cast<bf162*>(dw + (size_t)(id - v0) * H);
+      for (int v = lane; v < (H >> 1); v += 32) atomicAdd(dst + v, src[v]);
+    }
   }
 }
 
@@ -585,8 +599,10 @@ extern "C" int lb_embedding_bwd(const void* tok, const void* dy, void* dw, int T
   if (H % 8 || T <= 0) return LB_ERR_SHAPE;
   int blocks = (T + 7) / 8;
   if (blocks > lb_num_sms() * 8) blocks = lb_num_sms() * 8;
-  embedding_bwd_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const long long*)tok, (const bf16*)dy, (bf16*)dw, T,
-                                                                 H, v0, v1);
+  if ((((uintptr_t)dy | (uintptr_t)dw) & 15) == 0)
+    embedding_bwd_kernel<true><<<blocks, 256, 0, (cudaStream_t)stream>>>((const long long*)tok, (const bf16*)dy, (bf16*)dw, T, H, v0, v1);
+  else
+    embedding_bwd_kernel<false><<<blocks, 256, 0, (cudaStream_t)stream>>>((const long long*)tok, (const bf16*)dy, (bf16*)dw, T, H, v0, v1);
   LB_CHECK_LAUNCH();
   return LB_OK;
 }

@@ -135,6 +135,24 @@ def test_rmsnorm_widths(rows, cols, residual):
         assert _rel(g, want) < 5e-3
 
 
+# ---- embedding ---------------------------------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("V,H,T,shift", [(50, 264, 300, 0), (50, 264, 300, 2), (2000, 2048, 700, 0), (40, 8, 1, 4)])
+def test_embedding_gradient_alignment(V, H, T, shift):
+    """Gradient rows on 16-byte boundaries and ``shift`` elements off them; ids outside [10, V - 10) belong to other ranks.
+    An id's sum is rounded to bf16 after every one of its occurrences (about ten here: 4 roundings' worth in the 2-norm)."""
+    from lightron_b200.ops import functional as OF
+    lo, hi = (10, V - 10)
+    tok = torch.randint(0, V, (T,), device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    w = _rand(hi - lo, H, seed=2).requires_grad_(True)
+    dy = _rand(T * H + shift, seed=3)[shift:].view(T, H)
+    got, = torch.autograd.grad(OF.embedding(tok, w, lo), w, dy)
+    mine = (tok >= lo) & (tok < hi)
+    want = torch.zeros(hi - lo, H, dtype=torch.float64, device="cuda").index_add_(0, tok[mine] - lo, dy[mine].double())
+    assert (got.double() - want).norm() <= 1e-2 * want.norm()
+
+
 # ---- loss ------------------------------------------------------------------------------------------------
 
 

@@ -802,29 +802,46 @@ extern "C" int lb_gemm_grouped_status(void* out) {
   return LB_OK;
 }
 
-// Host only (no CUDA call): the schedule lb_gemm_grouped would build for these shapes on `sms` SMs with a CTA per tile.
-// out[0] = load of the busiest CTA, out[1] = total work, out[2] = number of CTAs used, all in k-block
-// units of 64 (a tile counts its k-blocks + 6).  busiest * CTAs / total is the imbalance factor.
 // Number of schedules currently cached (never more than MAX_SCHEDULES).
 extern "C" int lb_gemm_grouped_cached() {
   std::lock_guard<std::mutex> lock(g_sched_mutex);
   return (int)g_schedules.size();
 }
 
-extern "C" int lb_gemm_grouped_plan(int n, const int* M, const int* N, const int* K, int sms, long long* out) {
-  if (n < 1 || n > MAX_PROBLEMS || sms < 1) return LB_ERR_SHAPE;
-  Problem probs[MAX_PROBLEMS];
+namespace {
+// Problems of the host-only entry points below; false for sizes that no launch takes.
+bool plan_problems(int n, const int* M, const int* N, const int* K, int sms, Problem* probs) {
+  if (n < 1 || n > MAX_PROBLEMS || sms < 1) return false;
   for (int i = 0; i < n; i++) {
-    if (M[i] <= 0 || N[i] <= 0 || K[i] <= 0) return LB_ERR_SHAPE;
+    if (M[i] <= 0 || N[i] <= 0 || K[i] <= 0) return false;
     probs[i].M = M[i]; probs[i].N = N[i]; probs[i].K = K[i];
-    set_tiles(&probs[i], 1);
   }
+  return true;
+}
+}  // namespace
+
+// Host only (no CUDA call): CTAs per tile, 1 or 2, of the schedule that lb_gemm_grouped builds for these shapes on `sms` SMs.
+extern "C" int lb_gemm_grouped_ctas_per_tile(int n, const int* M, const int* N, const int* K, int sms) {
+  Problem probs[MAX_PROBLEMS];
+  if (!plan_problems(n, M, N, K, sms, probs)) return LB_ERR_SHAPE;
+  const int cg = choose_cg(probs, n, sms);
+  return cg < 0 ? LB_ERR_SHAPE : cg;
+}
+
+// Host only (no CUDA call): that schedule.  out[0] = load of the busiest CTA, out[1] = total work, out[2] = number of CTAs used,
+// all in k-block units of 64 (a tile counts its k-blocks + 6, for each of its CTAs).  busiest * CTAs / total is the imbalance factor.
+extern "C" int lb_gemm_grouped_plan(int n, const int* M, const int* N, const int* K, int sms, long long* out) {
+  Problem probs[MAX_PROBLEMS];
+  if (!plan_problems(n, M, N, K, sms, probs)) return LB_ERR_SHAPE;
+  const int cg = choose_cg(probs, n, sms);
+  if (cg < 0) return LB_ERR_SHAPE;
+  for (int i = 0; i < n; i++) set_tiles(&probs[i], cg);
   std::vector<std::vector<int>> per;
   int total = 0;
   long long work = 0;
-  const long long busiest = assign_items(probs, n, sms, &per, &total, &work);
+  const long long busiest = assign_items(probs, n, sms / cg, &per, &total, &work);
   if (busiest < 0) return LB_ERR_SHAPE;
-  out[0] = busiest; out[1] = work; out[2] = (long long)per.size();
+  out[0] = busiest; out[1] = cg * work; out[2] = cg * (long long)per.size();
   return LB_OK;
 }
 

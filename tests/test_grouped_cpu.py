@@ -35,6 +35,29 @@ def test_schedule_balances_weight_gradient_with_data_gradient():
     assert ctas == 4 and imb == 1.0
 
 
+def _ctas_per_tile(shapes, sms=148):
+    IA = ctypes.c_int * len(shapes)
+    return native._load().lb_gemm_grouped_ctas_per_tile(len(shapes), *(IA(*[s[i] for s in shapes]) for i in range(3)), sms)
+
+
+def test_plan_is_the_schedule_of_the_chosen_form():
+    """One tile's rows decide between a CTA per 128 rows and a pair per 256: the plan counts the form that is launched."""
+    lib = native._load()
+    if lib is None:
+        pytest.skip("native library not built")
+    for shapes, cg, ctas in (([(384, 256, 16384)], 2, 4),            # two 256-row tiles (the second half empty), not three of 128
+                             ([(384, 256, 512)], 1, 3),              # a short launch: CTAs
+                             ([(16384, 2048, 2048)], 2, 148)):
+        IA = ctypes.c_int * 1
+        out = (ctypes.c_longlong * 3)()
+        assert lib.lb_gemm_grouped_plan(1, *(IA(v) for v in shapes[0]), 148, out) == 0
+        kb = shapes[0][2] // 64 + 6
+        tiles = -(-shapes[0][0] // (128 * cg)) * -(-shapes[0][1] // 256)
+        assert _ctas_per_tile(shapes) == cg and out[2] == ctas and out[1] == cg * tiles * kb, shapes
+        assert out[0] == -(-tiles // (ctas // cg)) * kb
+    assert _ctas_per_tile([(0, 8, 8)]) < 0
+
+
 def test_schedule_rejects_bad_arguments():
     lib = native._load()
     if lib is None:

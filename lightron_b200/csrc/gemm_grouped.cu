@@ -688,10 +688,16 @@ int g_sms = 0;
 // that run at the same time adjacent in the problem's L2-friendly order).
 struct Item { int cost, code; };
 
-// The assignment itself (host only): per-CTA item lists, longest tiles first, each to the least
-// loaded CTA.  Returns the load (in k-block units) of the busiest CTA.
-long long assign_items(const Problem* probs, int np, int sms, std::vector<std::vector<int>>* per_out, int* total_out,
-                       long long* work_out) {
+// Modelled time of a tile, in hundredths of a single CTA's k-block: the main loop plus a fixed part, but not less than storing
+// the tile takes.  A pair's k-block takes less of the tensor pipe, its two stores run in step and hide less.
+long long tile_time(int num_kb, int cg) {
+  return cg == 1 ? std::max(100LL * num_kb + 800, 1200LL) : std::max(86LL * num_kb + 800, 25LL * num_kb + 1700);
+}
+
+// The assignment itself (host only): per-worker item lists, longest tiles first, each to the least
+// loaded worker.  Returns the load (in k-block units) of the busiest one; `time` receives its modelled time.
+long long assign_items(const Problem* probs, int np, int cg, int sms, std::vector<std::vector<int>>* per_out, int* total_out,
+                       long long* work_out, long long* time_out) {
   std::vector<Item> items;
   std::vector<int> order(np);
   for (int i = 0; i < np; i++) order[i] = i;
@@ -707,16 +713,19 @@ long long assign_items(const Problem* probs, int np, int sms, std::vector<std::v
     }
   }
   const int total = (int)items.size();
-  const int grid = total < sms ? total : sms;
+  const int workers = sms / cg;
+  const int grid = total < workers ? total : workers;
   typedef std::pair<long long, int> Load;
   std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
   for (int c = 0; c < grid; c++) heap.push({0, c});
   std::vector<std::vector<int>> per(grid);
+  std::vector<long long> time(grid, 0);
   long long busiest = 0;
   for (const Item& it : items) {
     Load l = heap.top();
     heap.pop();
     per[l.second].push_back(it.code);
+    time[l.second] += tile_time(it.cost - 6, cg);
     const long long load = l.first + it.cost;
     if (load > busiest) busiest = load;
     heap.push({load, l.second});
@@ -724,6 +733,7 @@ long long assign_items(const Problem* probs, int np, int sms, std::vector<std::v
   if (per_out) per_out->swap(per);
   if (total_out) *total_out = total;
   if (work_out) *work_out = work;
+  if (time_out) *time_out = *std::max_element(time.begin(), time.end());
   return busiest;
 }
 
@@ -733,21 +743,20 @@ void set_tiles(Problem* p, int cg) {
   p->num_kb = (p->K + BK - 1) / BK;
 }
 
-// CTAs per tile for this set of problems: pairs unless their coarser tiles make the busiest worker's list more than 5 % longer
-// (few or ragged tiles), which is what a pair's tile gains.  Measured with 16384 rows, CTAs against pairs: N11264 K2048
-// 584 / 546 us, N2560 K2048 134 / 126, N2048 K2048 106 / 103, N2048 K5632 259 / 254; data + weight gradient of these layers 1167 / 1142,
-// 286 / 262, 234 / 214, 623 / 575.  A launch of one or two short tiles per SM (a load below 64 k-blocks) pays more for setting up the
-// pairs than they gain: 512 / 1000 x 2304 x 768 takes 16.7 / 17.3 us with CTAs and 20.6 with pairs, 4096 x 2304 x 768 (load 36) 22.6 to
-// 26.8 and 24.9 to 31.7 (all with the launch).
+// CTAs per tile for this set of problems: the form whose busiest worker is modelled to finish first (tile_time, plus 6 k-blocks for
+// setting up the pairs of a launch).  Fitted to 727 launches in both forms: 130 to 16384 rows, N 768 to 11264, K 128 to 8192, all
+// operand majors, data + weight gradients, SwiGLU epilogues; the rule is on average 0.1 % off the better form, and at worst 6 % (launches
+// of one tile per CTA).  CTAs / pairs in us: where the store of a tile outlasts its main loop, 16384 x 4096 x 256 64.6 / 79.8,
+// x 512 80.0 / 88.9, 8192 x 4096 x 768 51.2 / 52.4; where it does not, 8192 x 4096 x 1024 62.1 / 58.7, 16384 x 4096 x 1536 167 / 150,
+// 4096 x 11264 x 4096 287 / 259; short launches, 1000 x 2304 x 768 14.6 / 16.5, 1000 x 768 x 4096 31.2 / 30.3.
 int choose_cg(Problem* probs, int np, int sms) {
   if (sms < 2) return 1;
-  long long load[3] = {0, 0, 0};
+  long long time[3] = {0, 0, 0};
   for (int cg = 1; cg <= 2; cg++) {
     for (int i = 0; i < np; i++) set_tiles(&probs[i], cg);
-    load[cg] = assign_items(probs, np, sms / cg, nullptr, nullptr, nullptr);
-    if (load[cg] < 0) return -1;
+    if (assign_items(probs, np, cg, sms, nullptr, nullptr, nullptr, &time[cg]) < 0) return -1;
   }
-  return load[2] >= 64 && load[2] * 100 <= load[1] * 105 ? 2 : 1;
+  return time[2] + 600 < time[1] ? 2 : 1;
 }
 
 int build_schedule(Problem* probs, int np, int sms, Schedule* out) {
@@ -756,7 +765,7 @@ int build_schedule(Problem* probs, int np, int sms, Schedule* out) {
   out->cg = choose_cg(probs, np, sms);
   if (out->cg < 0) return LB_ERR_SHAPE;
   for (int i = 0; i < np; i++) set_tiles(&probs[i], out->cg);
-  if (assign_items(probs, np, sms / out->cg, &per, &total, nullptr) < 0) return LB_ERR_SHAPE;
+  if (assign_items(probs, np, out->cg, sms, &per, &total, nullptr, nullptr) < 0) return LB_ERR_SHAPE;
   const int grid = (int)per.size();
   std::vector<int> offsets(grid + 1, 0), flat;
   flat.reserve(total);
@@ -839,7 +848,7 @@ extern "C" int lb_gemm_grouped_plan(int n, const int* M, const int* N, const int
   std::vector<std::vector<int>> per;
   int total = 0;
   long long work = 0;
-  const long long busiest = assign_items(probs, n, sms / cg, &per, &total, &work);
+  const long long busiest = assign_items(probs, n, cg, sms, &per, &total, &work, nullptr);
   if (busiest < 0) return LB_ERR_SHAPE;
   out[0] = busiest; out[1] = cg * work; out[2] = cg * (long long)per.size();
   return LB_OK;

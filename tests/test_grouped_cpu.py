@@ -58,6 +58,22 @@ def test_plan_is_the_schedule_of_the_chosen_form():
     assert _ctas_per_tile([(0, 8, 8)]) < 0
 
 
+@pytest.mark.parametrize("shapes,cg", [
+    # the store of a tile outlasts its main loop: pairs were 4 to 24 % slower, whatever the number of tiles
+    ([(16384, 4096, 256)], 1), ([(8192, 5632, 512)], 1), ([(16384, 2304, 768)], 1), ([(4096, 4096, 768)], 1),
+    # it does not: 4 to 11 % faster
+    ([(8192, 4096, 1024)], 2), ([(4096, 4096, 1536)], 2), ([(16384, 768, 1536)], 2), ([(16384, 5632, 4096)], 2),
+    # one or two short tiles per SM: the setup
+    ([(1000, 2304, 768)], 1), ([(4096, 2304, 768)], 1), ([(2048, 2304, 2048)], 1), ([(512, 768, 768), (512, 768, 768)], 1),
+    # the weight gradient's long tiles carry the data gradient's short ones
+    ([(2304, 768, 8192), (8192, 768, 2304)], 2),
+])
+def test_pairs_are_chosen_where_they_are_faster(shapes, cg):
+    if native._load() is None:
+        pytest.skip("native library not built")
+    assert _ctas_per_tile(shapes) == cg
+
+
 def test_schedule_rejects_bad_arguments():
     lib = native._load()
     if lib is None:

@@ -437,8 +437,8 @@ __global__ void __launch_bounds__(256) moe_pull_kernel(const PullParams p) {
 // -------------------------------------------------------------------------------------------
 // Router backward
 // -------------------------------------------------------------------------------------------
-// A block takes 64 tokens x 256 columns: warp w the tokens 8 w .. 8 w + 7, a lane 8 columns.  The gate weights of 8 experts stay in
-// registers over a warp's tokens, and the block's share of the gate gradient is summed over its warps in shared memory
+// A block takes 64 tokens x 256 columns: warp w the tokens 8 w .. 8 w + 7, a lane 8 columns.  A warp's tokens stay in registers over
+// the experts, whose gate weights are fetched once for all of them, and the block's share of the gate gradient is summed over its warps in shared memory
 // before one vector reduction per 4 columns.  (A block per 64 tokens and all columns left most SMs idle and fetched the weights
 // again for every token: T 4096, H 2048, E 8 100 us, now 28.)
 constexpr int RB_TOKENS = 64, RB_COLS = 256, RB_WARPS = 8, RB_TPW = RB_TOKENS / RB_WARPS;
@@ -449,7 +449,7 @@ moe_router_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wg, c
                       const float* __restrict__ daux, bf16* __restrict__ dx, float* __restrict__ dwg_acc, int T, int H,
                       int E, int k) {
   __shared__ float s_dl[RB_TOKENS][MOE_MAX_EXPERTS + 1];
-  __shared__ float s_w[RB_WARPS][RB_COLS];
+  __shared__ __align__(16) float s_w[RB_WARPS][RB_COLS];
   const int t0 = blockIdx.x * RB_TOKENS;
   const int ntok = min(RB_TOKENS, T - t0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

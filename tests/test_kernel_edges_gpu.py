@@ -199,6 +199,24 @@ def test_moe_router_tiles(T, H, E, k):
     assert _rel(dx, gx) < 5e-3 and _rel(dwg, gw) < 1e-4
 
 
+@pytest.mark.parametrize("shift", [0, 1, 2])
+def test_moe_router_gradient_alignment(shift):
+    """The gate gradient is added to a buffer on 16 bytes or ``shift`` elements off it (fp32 sums: 1e-4 as above)."""
+    from lightron_b200.ops import native
+    T, H, E, k, dev = 70, 264, 5, 2, "cuda"
+    x, wg = _rand(T, H, seed=1), _rand(E, H, scale=H ** -0.5, seed=2)
+    probs = torch.rand(T, E, device=dev).softmax(-1)
+    idx = torch.stack([torch.randperm(E, device=dev)[:k] for _ in range(T)]).int()
+    dwts, frac, dx = torch.randn(T, k, device=dev), torch.zeros(E, device=dev), torch.empty_like(x)
+    buf = torch.ones(E * H + 8, device=dev)
+    native.call("lb_moe_router_bwd", x.data_ptr(), wg.data_ptr(), probs.data_ptr(), idx.data_ptr(), dwts.data_ptr(), frac.data_ptr(),
+                0, dx.data_ptr(), buf.data_ptr() + 4 * shift, T, H, E, k, native.stream_ptr())
+    dp = torch.zeros(T, E, dtype=torch.float64, device=dev).scatter_add_(1, idx.long(), dwts.double())
+    dl = probs.double() * (dp - (probs.double() * dp).sum(-1, keepdim=True))
+    assert _rel(buf[shift:shift + E * H].view(E, H), 1 + dl.t() @ x.double()) < 1e-4 and _rel(dx, dl @ wg.double()) < 5e-3
+    assert (buf[:shift] == 1).all() and (buf[shift + E * H:] == 1).all()
+
+
 def test_moe_expert_without_tokens_gets_zero_gradients():
     """Gradients outside an arena are written, not accumulated, into memory that holds anything."""
     from lightron_b200.config import ModelArgs

@@ -54,6 +54,10 @@ __device__ __forceinline__ void moe_fail(unsigned code, unsigned where) {
 // -------------------------------------------------------------------------------------------
 // Router
 // -------------------------------------------------------------------------------------------
+// Latency bound.  IN tokens of a warp go through the gate weights together: a weight vector is fetched once for all of them and their
+// loads are in flight at the same time, but with more than 8 experts the rows are read again for every 8, and IN rows per warp
+// no longer stay in L1 (lb_moe_router has the rule).  The sums of a token are the same for every IN.
+template <int IN>
 __global__ void __launch_bounds__(ROUTER_THREADS)
 moe_router_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wg, int T, int H, int E, int k,
                   float* __restrict__ probs, int* __restrict__ idx, float* __restrict__ wts, int* __restrict__ within,
@@ -66,84 +70,81 @@ moe_router_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wg, int T
   for (int i = threadIdx.x; i < ROUTER_TOKENS * MOE_MAX_TOPK; i += blockDim.x) s_eid[i] = -1;
   __syncthreads();
   const int nvec = H >> 3;
-  // Latency bound: the tokens of a warp go through the weights together, so that a weight vector is fetched once for all
-  // of them and their loads are in flight at the same time (T 4096, H 2048, E 8: 52 us one token after the other, 48 together).
   constexpr int TPW = ROUTER_TOKENS / (ROUTER_THREADS / 32), NW = ROUTER_THREADS / 32;
-  // logits[e] for e = lane, lane + 32 end up in lg[0] / lg[1] (E <= 64)
-  float lg[TPW][2];
+  for (int i0 = 0; i0 < TPW && t0 + warp + i0 * NW < T; i0 += IN) {      // IN tokens of the warp at a time
+    // logits[e] for e = lane, lane + 32 end up in lg[0] / lg[1] (E <= 64)
+    float lg[IN][2];
 #pragma unroll
-  for (int i = 0; i < TPW; i++) lg[i][0] = lg[i][1] = -INFINITY;
-  for (int e0 = 0; e0 < E; e0 += 8) {                     // 8 experts per pass over the rows
-    float acc[TPW][8];
+    for (int i = 0; i < IN; i++) lg[i][0] = lg[i][1] = -INFINITY;
+    for (int e0 = 0; e0 < E; e0 += 8) {                     // 8 experts per pass over the rows
+      float acc[IN][8];
 #pragma unroll
-    for (int i = 0; i < TPW; i++)
+      for (int i = 0; i < IN; i++)
 #pragma unroll
-      for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
-    const int ne = min(8, E - e0);
-    for (int v = lane; v < nvec; v += 32) {
-      uint4 raw[TPW];
+        for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
+      const int ne = min(8, E - e0);
+      for (int v = lane; v < nvec; v += 32) {
+        float xf[IN][8];
 #pragma unroll
-      for (int i = 0; i < TPW; i++) {
-        const int t = t0 + warp + i * NW;
-        raw[i] = t < T ? reinterpret_cast<const uint4*>(x + (size_t)t * H)[v] : make_uint4(0, 0, 0, 0);
-      }
+        for (int i = 0; i < IN; i++) {
+          const int t = t0 + warp + (i0 + i) * NW;
+          unpack8(t < T ? reinterpret_cast<const uint4*>(x + (size_t)t * H)[v] : make_uint4(0, 0, 0, 0), xf[i]);
+        }
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        if (j < ne) {
-          float wf[8];
-          unpack8(__ldg(reinterpret_cast<const uint4*>(wg + (size_t)(e0 + j) * H) + v), wf);
+        for (int j = 0; j < 8; j++) {
+          if (j < ne) {
+            float wf[8];
+            unpack8(__ldg(reinterpret_cast<const uint4*>(wg + (size_t)(e0 + j) * H) + v), wf);
 #pragma unroll
-          for (int i = 0; i < TPW; i++) {
-            float xf[8];
-            unpack8(raw[i], xf);
+            for (int i = 0; i < IN; i++)
 #pragma unroll
-            for (int c = 0; c < 8; c++) acc[i][j] = fmaf(xf[c], wf[c], acc[i][j]);
+              for (int c = 0; c < 8; c++) acc[i][j] = fmaf(xf[i][c], wf[c], acc[i][j]);
           }
         }
       }
+#pragma unroll
+      for (int i = 0; i < IN; i++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const float s = warp_sum(acc[i][j]);
+          if (j < ne) {
+            const int e = e0 + j;
+            if ((e & 31) == lane) { if (e < 32) lg[i][0] = s; else lg[i][1] = s; }
+          }
+        }
     }
 #pragma unroll
-    for (int i = 0; i < TPW; i++)
+    for (int i = 0; i < IN; i++) {
+      const int tl = warp + (i0 + i) * NW, t = t0 + tl;
+      if (t >= T) break;                                   // warp-uniform
+      const float lg0 = lg[i][0], lg1 = lg[i][1];
+      // softmax over experts (fp32), every lane ends with its own probabilities
+      const float mx = warp_max(fmaxf(lg0, lg1));
+      const float ex0 = (lane < E) ? __expf(lg0 - mx) : 0.f;
+      const float ex1 = (lane + 32 < E) ? __expf(lg1 - mx) : 0.f;
+      const float inv = 1.f / warp_sum(ex0 + ex1);
+      const float p0 = ex0 * inv, p1 = ex1 * inv;
+      if (lane < E) probs[(size_t)t * E + lane] = p0;
+      if (lane + 32 < E) probs[(size_t)t * E + lane + 32] = p1;
+      // top-k: k rounds of arg-max (lowest index wins ties)
+      float q0 = (lane < E) ? p0 : -1.f, q1 = (lane + 32 < E) ? p1 : -1.f;
+      for (int s = 0; s < k; s++) {
+        float best = fmaxf(q0, q1);
+        int bi = (q0 >= q1) ? lane : lane + 32;
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const float s = warp_sum(acc[i][j]);
-        if (j < ne) {
-          const int e = e0 + j;
-          if ((e & 31) == lane) { if (e < 32) lg[i][0] = s; else lg[i][1] = s; }
+        for (int o = 16; o > 0; o >>= 1) {
+          const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+          if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
         }
+        if (lane == 0) {
+          idx[(size_t)t * k + s] = bi;
+          wts[(size_t)t * k + s] = best;
+          s_eid[tl * k + s] = bi;
+        }
+        if (bi == lane) q0 = -1.f;
+        if (bi == lane + 32) q1 = -1.f;
       }
-  }
-#pragma unroll
-  for (int i = 0; i < TPW; i++) {
-    const int tl = warp + i * NW, t = t0 + tl;
-    if (t >= T) break;                                   // warp-uniform
-    const float lg0 = lg[i][0], lg1 = lg[i][1];
-    // softmax over experts (fp32), every lane ends with its own probabilities
-    const float mx = warp_max(fmaxf(lg0, lg1));
-    const float ex0 = (lane < E) ? __expf(lg0 - mx) : 0.f;
-    const float ex1 = (lane + 32 < E) ? __expf(lg1 - mx) : 0.f;
-    const float inv = 1.f / warp_sum(ex0 + ex1);
-    const float p0 = ex0 * inv, p1 = ex1 * inv;
-    if (lane < E) probs[(size_t)t * E + lane] = p0;
-    if (lane + 32 < E) probs[(size_t)t * E + lane + 32] = p1;
-    // top-k: k rounds of arg-max (lowest index wins ties)
-    float q0 = (lane < E) ? p0 : -1.f, q1 = (lane + 32 < E) ? p1 : -1.f;
-    for (int s = 0; s < k; s++) {
-      float best = fmaxf(q0, q1);
-      int bi = (q0 >= q1) ? lane : lane + 32;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-      }
-      if (lane == 0) {
-        idx[(size_t)t * k + s] = bi;
-        wts[(size_t)t * k + s] = best;
-        s_eid[tl * k + s] = bi;
-      }
-      if (bi == lane) q0 = -1.f;
-      if (bi == lane + 32) q1 = -1.f;
     }
   }
   __syncthreads();
@@ -564,7 +565,11 @@ extern "C" int lb_moe_push_ctas(int T) { return moe_grid(T); }
 extern "C" int lb_moe_router(const void* x, const void* wg, int T, int H, int E, int k, void* probs, void* idx, void* wts,
                              void* within, void* blk_hist, void* blk_psum, void* stream) {
   if (T <= 0 || (H % 8) || E < 1 || E > MOE_MAX_EXPERTS || k < 1 || k > MOE_MAX_TOPK || k > E) return LB_ERR_SHAPE;
-  moe_router_kernel<<<lb_moe_router_blocks(T), ROUTER_THREADS, 0, (cudaStream_t)stream>>>(
+  // One token at a time where a warp has no second one, and where many experts meet rows that do not stay in L2; four elsewhere.
+  // One / four, us: T 1, H 2048, E 8 10 / 19; T 16384, H 4096, E 64 744 / 1078; T 32768, H 2048, E 64 647 / 737; T 4096, H 2048, E 8
+  // 33 / 28, E 64 235 / 150; T 16384, H 2048, E 64 412 / 363.
+  const bool one = T <= ROUTER_THREADS / 32 || (E > 8 && (long long)T * H > (32LL << 20));
+  (one ? moe_router_kernel<1> : moe_router_kernel<4>)<<<lb_moe_router_blocks(T), ROUTER_THREADS, 0, (cudaStream_t)stream>>>(
       (const bf16*)x, (const bf16*)wg, T, H, E, k, (float*)probs, (int*)idx, (float*)wts, (int*)within, (int*)blk_hist,
       (float*)blk_psum);
   LB_CHECK_LAUNCH();

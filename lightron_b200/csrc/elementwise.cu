@@ -685,35 +685,59 @@ extern "C" int lb_ce_stats(const void* logits, const void* tgt, void* mx, void* 
   return LB_OK;
 }
 
-// lse[t] = log-sum-exp of row t, loss[0] = inv_n * sum over the rows whose target counts of (lse - target logit).  One block: the
-// sums of a row are three floats, and a fixed order makes the loss the same every time.
-__global__ void __launch_bounds__(1024) ce_loss_kernel(const float* __restrict__ mx, const float* __restrict__ se,
-                                                       const float* __restrict__ tl, const long long* __restrict__ tgt,
-                                                       float* __restrict__ lse, float* __restrict__ loss, int T, float inv_n,
-                                                       int ignore_index) {
+// lse[t] = log-sum-exp of row t, loss[0] = inv_n * sum over the rows whose target counts of (lse - target logit).  A fixed order
+// of the sum makes the loss the same every time.  Up to CE_LOSS_ROWS rows one block does it all (8192 rows 14 us, of which
+// half is the launch); beyond, a double-precision logarithm per row is too much for one SM (131072 rows 155 us): a block per
+// CE_LOSS_ROWS / 2 rows leaves its sum in the first of its rows' `se`, which nothing reads any more, and a second kernel adds them.
+constexpr int CE_LOSS_ROWS = 8192;
+
+__device__ __forceinline__ float ce_block_sum(float s) {      // of 1024 threads; complete in thread 0
+  __shared__ float sh[32];
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  return threadIdx.x < 32 ? warp_sum(sh[threadIdx.x]) : 0.f;
+}
+
+__global__ void __launch_bounds__(1024) ce_loss_kernel(const float* __restrict__ mx, const float* se, const float* __restrict__ tl,
+                                                       const long long* __restrict__ tgt, float* __restrict__ lse, float* sum,
+                                                       int T, int rows, float inv_n, int ignore_index) {
+  const long long t0 = (long long)blockIdx.x * rows;
+  const int n = (int)min((long long)rows, T - t0);
   float s = 0.f;
 #pragma unroll 4
-  for (int t = threadIdx.x; t < T; t += 1024) {
+  for (int i = threadIdx.x; i < n; i += 1024) {
+    const long long t = t0 + i;
     const float l = mx[t] + (float)log((double)se[t]);      // (logf is the approximate one under fast math)
     lse[t] = l;
     if (tgt[t] != ignore_index) s += l - tl[t];
   }
-  s = warp_sum(s);
-  __shared__ float sh[32];
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    s = warp_sum(sh[threadIdx.x]);
-    if (threadIdx.x == 0) loss[0] = s * inv_n;
-  }
+  s = ce_block_sum(s);
+  if (threadIdx.x == 0) sum[t0] = s * inv_n;
 }
 
-extern "C" int lb_ce_loss(const void* mx, const void* se, const void* tl, const void* tgt, void* lse, void* loss, int T, float inv_n,
+__global__ void __launch_bounds__(1024) ce_loss_sum_kernel(const float* __restrict__ sum, float* __restrict__ loss, int n, int rows,
+                                                           float inv_n) {
+  float s = 0.f;
+  for (int b = threadIdx.x; b < n; b += 1024) s += sum[(long long)b * rows];
+  s = ce_block_sum(s);
+  if (threadIdx.x == 0) loss[0] = s * inv_n;
+}
+
+// `se` is scratch: beyond CE_LOSS_ROWS rows it is overwritten.
+extern "C" int lb_ce_loss(const void* mx, void* se, const void* tl, const void* tgt, void* lse, void* loss, int T, float inv_n,
                           int ignore_index, void* stream) {
   if (T <= 0) return LB_ERR_SHAPE;
-  ce_loss_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>((const float*)mx, (const float*)se, (const float*)tl,
-                                                       (const long long*)tgt, (float*)lse, (float*)loss, T, inv_n, ignore_index);
+  const bool one = T <= CE_LOSS_ROWS;
+  const int rows = one ? T : CE_LOSS_ROWS / 2, blocks = (T - 1) / rows + 1;
+  ce_loss_kernel<<<blocks, 1024, 0, (cudaStream_t)stream>>>((const float*)mx, (const float*)se, (const float*)tl,
+                                                            (const long long*)tgt, (float*)lse, (float*)(one ? loss : se), T, rows,
+                                                            one ? inv_n : 1.f, ignore_index);
   LB_CHECK_LAUNCH();
+  if (!one) {
+    ce_loss_sum_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>((const float*)se, (float*)loss, blocks, rows, inv_n);
+    LB_CHECK_LAUNCH();
+  }
   return LB_OK;
 }
 

@@ -156,9 +156,9 @@ def test_embedding_gradient_alignment(V, H, T, shift):
 # ---- loss ------------------------------------------------------------------------------------------------
 
 
-@pytest.mark.parametrize("T,V", [(1, 8), (33, 264), (1025, 1000), (4100, 64)])
+@pytest.mark.parametrize("T,V", [(1, 8), (33, 264), (1025, 1000), (4100, 64), (8192, 8), (8193, 8), (140001, 16)])
 def test_cross_entropy_loss_rows(T, V):
-    """Fewer rows than threads, more, ignored ones; the loss is an fp32 sum (1e-6) of fp32 rows over bf16 logits."""
+    """Fewer rows than threads, more, more than one block takes, ignored ones; the loss is an fp32 sum (1e-6) of fp32 rows over bf16 logits."""
     from lightron_b200.ops import functional as OF
     logits, tgt = _rand(T, V, scale=3.0, seed=1), torch.randint(0, V, (T,), device="cuda", generator=torch.Generator("cuda").manual_seed(2))
     tgt[1::7] = -100

@@ -759,6 +759,8 @@ class _CrossEntropy(torch.autograd.Function):
         use_native = native.use_native(logits)
         tgt = targets.reshape(-1).contiguous()
         if use_native:
+            if tgt.numel() != T:        # the kernels read a target per row
+                raise ValueError(f"{tgt.numel()} targets for {T} rows of logits")
             mx = torch.empty(T, dtype=torch.float32, device=logits.device)
             se = torch.empty(T, dtype=torch.float32, device=logits.device)
             tl = torch.empty(T, dtype=torch.float32, device=logits.device)

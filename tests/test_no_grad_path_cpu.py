@@ -59,3 +59,17 @@ def test_transforms_and_tangents_still_reach_the_function(wrapped):
             with pytest.raises(Exception):                      # no jvp rule: refused, the tangent is not dropped
                 OF._apply(_Twice, fwAD.make_dual(x, torch.ones_like(x)), y)
         assert wrapped
+
+
+@pytest.mark.parametrize("n", [3, 5, 1])
+def test_targets_have_to_match_the_rows(monkeypatch, n):
+    """The kernels read a target per row of logits: another number is refused before any of them is launched."""
+    monkeypatch.setattr(OF.native, "use_native", lambda t: True)
+    monkeypatch.setattr(OF.native, "stream_ptr", lambda: 0)
+    calls = []
+    monkeypatch.setattr(OF.native, "call", lambda *a: calls.append(a[0]))
+    with pytest.raises(ValueError):
+        OF.cross_entropy(torch.randn(4, 8), torch.zeros(n, dtype=torch.long))
+    assert not calls
+    OF.cross_entropy(torch.randn(4, 8), torch.zeros(2, 2, dtype=torch.long))
+    assert calls == ["lb_ce_stats", "lb_ce_loss"]

@@ -516,20 +516,24 @@ extern "C" int lb_flash_bwd_status(void* out) {
   return LB_OK;
 }
 
-// Same contract as lb_flash_bwd (flash_attn.cu) except for the scratch, which need not be initialised: dq_acc is fp32
-// of B * hq * ceil(Sq/128) * 128 * d elements (tile-permuted layout, see fa_dq_convert_kernel), delta fp32 of
-// 2 * B * hq * ceil(Sq/128) * 128 (fa_bwd_prep_kernel); both 16-byte aligned.  head_dim 64 or 128; causal needs Sk >= Sq.
+// Bytes of the workspace of lb_flash_bwd_tc_ws / lb_flash_bwd_cp_ws: the row statistics (fa_bwd_prep_kernel), then the fp32 dQ
+// accumulator (fa_dq_convert_kernel has its layout), both in whole 128-query blocks.  0 for sizes that they do not take.
+extern "C" long long lb_flash_bwd_ws_bytes(int B, int Sq, int hq, int d) {
+  if (B <= 0 || Sq <= 0 || hq <= 0 || (d != 64 && d != 128)) return 0;
+  return (long long)B * hq * ((Sq + 127) / 128) * 128 * (2 + d) * (long long)sizeof(float);
+}
+
 static int flash_bwd_tc_impl(int kv_brows, const void* q, const void* k, const void* v, const void* o, const void* dout,
-                               const void* lse, void* delta, void* dq_acc, void* dq, void* dk, void* dv, int B, int Sq,
+                               const void* lse, void* stats, void* dq_acc, void* dq, void* dk, void* dv, int B, int Sq,
                                int Sk, int hq, int hkv, int d, long long q_ts, long long k_ts, long long v_ts,
                                long long o_ts, long long do_ts, long long dq_ts, long long dk_ts, long long dv_ts,
                                float scale, int causal, void* stream) {
   if (B <= 0 || Sq <= 0 || Sk <= 0 || hq % hkv) return LB_ERR_SHAPE;
   if ((q_ts | k_ts | v_ts | o_ts | do_ts | dq_ts | dk_ts | dv_ts) % 8) return LB_ERR_SHAPE;
   if (causal && Sk < Sq) return LB_ERR_SHAPE;
-  if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)dout | (uintptr_t)dq | (uintptr_t)dk | (uintptr_t)dv | (uintptr_t)o | (uintptr_t)delta | (uintptr_t)dq_acc) & 15)
+  if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)dout | (uintptr_t)dq | (uintptr_t)dk | (uintptr_t)dv | (uintptr_t)o | (uintptr_t)stats | (uintptr_t)dq_acc) & 15)
     return LB_ERR_ARG;
-  FaBwdParams p{(const bf16*)o, (const bf16*)dout, (const float*)lse, (float*)delta, (float*)dq_acc,
+  FaBwdParams p{(const bf16*)o, (const bf16*)dout, (const float*)lse, (float*)stats, (float*)dq_acc,
                 (bf16*)dq, (bf16*)dk, (bf16*)dv, B, Sq, Sk, hq, hkv, o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal,
                 kv_brows};
   cudaStream_t s = (cudaStream_t)stream;
@@ -540,23 +544,57 @@ static int flash_bwd_tc_impl(int kv_brows, const void* q, const void* k, const v
   }
 }
 
-extern "C" int lb_flash_bwd_tc(const void* q, const void* k, const void* v, const void* o, const void* dout,
-                               const void* lse, void* delta, void* dq_acc, void* dq, void* dk, void* dv, int B, int Sq,
-                               int Sk, int hq, int hkv, int d, long long q_ts, long long k_ts, long long v_ts,
-                               long long o_ts, long long do_ts, long long dq_ts, long long dk_ts, long long dv_ts,
-                               float scale, int causal, void* stream) {
-  return flash_bwd_tc_impl(Sk, q, k, v, o, dout, lse, delta, dq_acc, dq, dk, dv, B, Sq, Sk, hq, hkv, d, q_ts, k_ts, v_ts,
-                           o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal, stream);
+// Same contract as lb_flash_bwd (flash_attn.cu) except for the scratch: a workspace of ws_bytes >= lb_flash_bwd_ws_bytes(), 16-byte
+// aligned, that need not be initialised.  head_dim 64 or 128; causal needs Sk >= Sq.  K/V are the first Sk rows of every
+// batch of a buffer with kv_brows rows per batch (the context-parallel gather buffers; Sk for plain tensors); dk / dv
+// stay [B, Sk, hkv, d].
+extern "C" int lb_flash_bwd_cp_ws(const void* q, const void* k, const void* v, const void* o, const void* dout,
+                                  const void* lse, void* ws, long long ws_bytes, void* dq, void* dk, void* dv, int B, int Sq,
+                                  int Sk, int kv_brows, int hq, int hkv, int d, long long q_ts, long long k_ts, long long v_ts,
+                                  long long o_ts, long long do_ts, long long dq_ts, long long dk_ts, long long dv_ts,
+                                  float scale, int causal, void* stream) {
+  if (kv_brows < Sk) return LB_ERR_SHAPE;
+  const long long need = lb_flash_bwd_ws_bytes(B, Sq, hq, d);
+  if (!need) return LB_ERR_SHAPE;
+  if (ws_bytes < need) return LB_ERR_CAPACITY;
+  const long long n_pad = (long long)B * hq * ((Sq + 127) / 128) * 128;
+  return flash_bwd_tc_impl(kv_brows, q, k, v, o, dout, lse, ws, (float*)ws + 2 * n_pad, dq, dk, dv, B, Sq, Sk, hq, hkv, d,
+                           q_ts, k_ts, v_ts, o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal, stream);
 }
 
-// Same, for K/V that are the first Sk rows of every batch of a longer buffer (kv_brows rows per
-// batch): the context-parallel gather buffers.  dk / dv stay [B, Sk, hkv, d].
+extern "C" int lb_flash_bwd_tc_ws(const void* q, const void* k, const void* v, const void* o, const void* dout,
+                                  const void* lse, void* ws, long long ws_bytes, void* dq, void* dk, void* dv, int B, int Sq,
+                                  int Sk, int hq, int hkv, int d, long long q_ts, long long k_ts, long long v_ts,
+                                  long long o_ts, long long do_ts, long long dq_ts, long long dk_ts, long long dv_ts,
+                                  float scale, int causal, void* stream) {
+  return lb_flash_bwd_cp_ws(q, k, v, o, dout, lse, ws, ws_bytes, dq, dk, dv, B, Sq, Sk, Sk, hq, hkv, d, q_ts, k_ts, v_ts, o_ts,
+                            do_ts, dq_ts, dk_ts, dv_ts, scale, causal, stream);
+}
+
+// The forms for callers that bring delta (fp32 [B, hq, Sq], not used) and dq_acc (fp32, B * hq * ceil(Sq/128) * 128 * d elements) as
+// scratch: the row statistics need twice the padded rows, so they are allocated on the stream here.
 extern "C" int lb_flash_bwd_cp(const void* q, const void* k, const void* v, const void* o, const void* dout,
                                const void* lse, void* delta, void* dq_acc, void* dq, void* dk, void* dv, int B, int Sq,
                                int Sk, int kv_brows, int hq, int hkv, int d, long long q_ts, long long k_ts,
                                long long v_ts, long long o_ts, long long do_ts, long long dq_ts, long long dk_ts,
                                long long dv_ts, float scale, int causal, void* stream) {
-  if (kv_brows < Sk) return LB_ERR_SHAPE;
-  return flash_bwd_tc_impl(kv_brows, q, k, v, o, dout, lse, delta, dq_acc, dq, dk, dv, B, Sq, Sk, hq, hkv, d, q_ts, k_ts,
-                           v_ts, o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal, stream);
+  (void)delta;
+  if (kv_brows < Sk || !lb_flash_bwd_ws_bytes(B, Sq, hq, d)) return LB_ERR_SHAPE;
+  void* stats = nullptr;
+  cudaError_t e = cudaMallocAsync(&stats, (size_t)B * hq * ((Sq + 127) / 128) * 256 * sizeof(float), (cudaStream_t)stream);
+  if (e != cudaSuccess) { cudaGetLastError(); g_lb_last_cuda_error = (int)e; return LB_ERR_LAUNCH; }
+  const int rc = flash_bwd_tc_impl(kv_brows, q, k, v, o, dout, lse, stats, dq_acc, dq, dk, dv, B, Sq, Sk, hq, hkv, d, q_ts, k_ts,
+                                   v_ts, o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal, stream);
+  e = cudaFreeAsync(stats, (cudaStream_t)stream);
+  if (rc == LB_OK && e != cudaSuccess) { g_lb_last_cuda_error = (int)e; return LB_ERR_LAUNCH; }
+  return rc;
+}
+
+extern "C" int lb_flash_bwd_tc(const void* q, const void* k, const void* v, const void* o, const void* dout,
+                               const void* lse, void* delta, void* dq_acc, void* dq, void* dk, void* dv, int B, int Sq,
+                               int Sk, int hq, int hkv, int d, long long q_ts, long long k_ts, long long v_ts,
+                               long long o_ts, long long do_ts, long long dq_ts, long long dk_ts, long long dv_ts,
+                               float scale, int causal, void* stream) {
+  return lb_flash_bwd_cp(q, k, v, o, dout, lse, delta, dq_acc, dq, dk, dv, B, Sq, Sk, Sk, hq, hkv, d, q_ts, k_ts, v_ts,
+                         o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal, stream);
 }

@@ -605,17 +605,16 @@ def flash_bwd_native(q, k, v, o, lse, do, causal: bool, scale: float, dq=None, d
     for t in (dq, dk, dv):
         _check_attn_layout(t)
     use_tc = d in (64, 128) and not (causal and Sk < Sq) and os.environ.get("LIGHTRON_FA_BWD", "tc") == "tc"
-    if use_tc:      # scratch in 128-query records / tiles, initialised by the kernels
-        n_pad = B * hq * ((Sq + 127) // 128) * 128
-        delta = torch.empty(2 * n_pad, dtype=torch.float32, device=q.device)
-        dq_acc = torch.empty(n_pad * d, dtype=torch.float32, device=q.device)
+    tail = (dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, Sq, Sk, hq, hkv, d, q.stride(1), k.stride(1), v.stride(1), o.stride(1),
+            do.stride(1), dq.stride(1), dk.stride(1), dv.stride(1), float(scale), int(causal), native.stream_ptr())
+    head = (q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr())
+    if use_tc:
+        ws = native.flash_bwd_workspace(B, Sq, hq, d, q.device)
+        native.call("lb_flash_bwd_tc_ws", *head, ws.data_ptr(), ws.numel(), *tail)
     else:
         delta = torch.empty(B, hq, Sq, dtype=torch.float32, device=q.device)
         dq_acc = torch.zeros(B * Sq * hq * d, dtype=torch.float32, device=q.device)
-    native.call("lb_flash_bwd_tc" if use_tc else "lb_flash_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
-                delta.data_ptr(), dq_acc.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                B, Sq, Sk, hq, hkv, d, q.stride(1), k.stride(1), v.stride(1), o.stride(1), do.stride(1),
-                dq.stride(1), dk.stride(1), dv.stride(1), float(scale), int(causal), native.stream_ptr())
+        native.call("lb_flash_bwd", *head, delta.data_ptr(), dq_acc.data_ptr(), *tail)
     return dq, dk, dv
 
 

@@ -28,7 +28,7 @@ def lib_path() -> str:
 
 _P, _I, _L, _F = c_void_p, c_int, c_int64, c_float
 
-# name -> argtypes (all return int)
+# name -> argtypes (all return int, those that count bytes 64 bits of it)
 _SIGNATURES = {
     "lb_last_error": [],
     "lb_sm_count": [],
@@ -91,6 +91,11 @@ _SIGNATURES = {
                         _L, _L, _I, _I, _P, _P, _P, _I, _P],
     "lb_flash_bwd_cp": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I,
                         _L, _L, _L, _L, _L, _L, _L, _L, _F, _I, _P],
+    "lb_flash_bwd_cp_ws": [_P, _P, _P, _P, _P, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I,
+                           _L, _L, _L, _L, _L, _L, _L, _L, _F, _I, _P],
+    "lb_flash_bwd_tc_ws": [_P, _P, _P, _P, _P, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I,
+                           _L, _L, _L, _L, _L, _L, _L, _L, _F, _I, _P],
+    "lb_flash_bwd_ws_bytes": [_I, _I, _I, _I],
     "lb_flash_bwd_status": [_P],
     "lb_flash_bwd_tc": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
                         _L, _L, _L, _L, _L, _L, _L, _L, _F, _I, _P],
@@ -117,7 +122,7 @@ def _load() -> Optional[ctypes.CDLL]:
         if fn is None:
             continue
         fn.argtypes = args
-        fn.restype = c_int
+        fn.restype = _L if name.endswith("_bytes") else c_int
     _LIB = lib
     wait_ms = os.environ.get("LIGHTRON_FLAG_WAIT_MS")     # limit of every device-side wait for a peer
     if wait_ms and hasattr(lib, "lb_set_flag_wait_ns"):
@@ -177,6 +182,11 @@ def stream_ptr() -> int:
     """Handle of the current device's current stream (``torch.cuda.current_stream().cuda_stream`` without building the
     ``Stream`` object, which costs as much as the launch's argument conversion)."""
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def flash_bwd_workspace(B: int, Sq: int, hq: int, d: int, device) -> torch.Tensor:
+    """Scratch of one attention backward call (``lb_flash_bwd_tc_ws`` / ``lb_flash_bwd_cp_ws``), uninitialised."""
+    return torch.empty(require().lb_flash_bwd_ws_bytes(B, Sq, hq, d), dtype=torch.uint8, device=device)
 
 
 def ptr(t: Optional[torch.Tensor]) -> int:

@@ -111,11 +111,9 @@ def _bwd_call(q, kbuf, vbuf, Sk, kv_brows, o, lse, do, scale, dk=None, dv=None):
     if dk is None:
         dk = torch.empty(B, Sk, hkv, d, dtype=q.dtype, device=q.device)
         dv = torch.empty_like(dk)
-    n_pad = B * hq * ((Sq + 127) // 128) * 128
-    delta = torch.empty(2 * n_pad, dtype=torch.float32, device=q.device)
-    dq_acc = torch.empty(n_pad * d, dtype=torch.float32, device=q.device)
-    native.call("lb_flash_bwd_cp", q.data_ptr(), kbuf.data_ptr(), vbuf.data_ptr(), o.data_ptr(), do.data_ptr(),
-                lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+    ws = native.flash_bwd_workspace(B, Sq, hq, d, q.device)
+    native.call("lb_flash_bwd_cp_ws", q.data_ptr(), kbuf.data_ptr(), vbuf.data_ptr(), o.data_ptr(), do.data_ptr(),
+                lse.data_ptr(), ws.data_ptr(), ws.numel(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                 B, Sq, Sk, kv_brows, hq, hkv, d, q.stride(1), kbuf.stride(1), vbuf.stride(1), o.stride(1), do.stride(1),
                 dq.stride(1), dk.stride(1), dv.stride(1), float(scale), 1, native.stream_ptr())
     return dq, dk, dv

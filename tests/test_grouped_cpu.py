@@ -84,6 +84,20 @@ def test_schedule_rejects_bad_arguments():
     assert lib.lb_gemm_grouped_plan(9, IA(8), IA(8), IA(8), 148, out) != 0
 
 
+def test_attention_backward_refuses_a_short_workspace():
+    """The size travels with the pointer: a workspace that is too small is refused before anything is launched."""
+    lib = native._load()
+    if lib is None:
+        pytest.skip("native library not built")
+    need = lib.lb_flash_bwd_ws_bytes(2, 129, 3, 64)
+    assert need == 2 * 3 * 256 * (2 + 64) * 4 and lib.lb_flash_bwd_ws_bytes(1, 8, 1, 32) == 0
+    assert lib.lb_flash_bwd_ws_bytes(8, 1 << 20, 64, 128) == 8 * 64 * (1 << 20) * 130 * 4          # past 32 bits
+    strides = [192] * 8
+    assert lib.lb_flash_bwd_tc_ws(*[0] * 7, need - 1, 0, 0, 0, 2, 129, 129, 3, 3, 64, *strides, 1.0, 1, 0) == -6
+    assert lib.lb_flash_bwd_cp_ws(*[0] * 7, need - 1, 0, 0, 0, 2, 129, 129, 200, 3, 3, 64, *strides, 1.0, 1, 0) == -6
+    assert lib.lb_flash_bwd_cp_ws(*[0] * 7, need, 0, 0, 0, 2, 129, 129, 100, 3, 3, 64, *strides, 1.0, 1, 0) == -3
+
+
 def _fake_gemm_grouped(problems):
     outs = []
     for a, b, a_mn, b_mn, out, acc in problems:

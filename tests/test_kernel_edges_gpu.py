@@ -60,6 +60,32 @@ def test_attention_tile_edges(B, Sq, Sk, hq, hkv, causal, scale, d):
             assert _rel(g, w) < 1e-2, name
 
 
+@pytest.mark.parametrize("B,Sq,d,shift", [(1, 2, 64, 0), (2, 129, 128, 1)])
+def test_attention_backward_scratch_of_the_caller(B, Sq, d, shift):
+    """The form whose caller brings one value per row (4-byte aligned) and the accumulator leaves what lies behind them alone; rows
+    that are not on 16 bytes are refused."""
+    from lightron_b200.ops import functional as OF, native
+    h = 2
+    q, k, v, do = (_rand(B, Sq, h, d, seed=i) for i in range(4))
+    o, lse = OF.flash_fwd_native(q, k, v, True, d ** -0.5)
+    n, n_acc = B * h * Sq, B * h * -(-Sq // 128) * 128 * d
+    delta, acc = torch.full((shift + 4 * n + 4096,), 7.0, device="cuda"), torch.zeros(n_acc + 4096, device="cuda")
+    out = [torch.empty_like(q) for _ in range(3)]
+
+    def call(o_ptr):
+        native.call("lb_flash_bwd_tc", q.data_ptr(), k.data_ptr(), v.data_ptr(), o_ptr, do.data_ptr(), lse.data_ptr(),
+                    delta.data_ptr() + 4 * shift, acc.data_ptr(), *(t.data_ptr() for t in out), B, Sq, Sq, h, h, d, *[h * d] * 8, d ** -0.5, 1,
+                    native.stream_ptr())
+    call(o.data_ptr())
+    assert (delta[:shift] == 7).all() and (delta[shift + n:] == 7).all() and (acc[n_acc:] == 0).all()
+    for g, w in zip(out, _attention64(q, k, v, do, True)[1:]):
+        assert _rel(g, w) < 1e-2
+    for g, w in zip(out, OF.flash_bwd_native(q, k, v, o, lse, do, True, d ** -0.5)):
+        assert _rel(g, w) < 5e-3
+    with pytest.raises(native.NativeError):
+        call(o.data_ptr() + 2)
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 def test_attention_bad_scores_stay_in_their_rows(d, bad):

@@ -240,8 +240,10 @@ class _FusedMoE(torch.autograd.Function):
         else:
             # written whole by the kernel: adding into cleared buffers read and wrote every gradient twice more, and with few
             # rows per expert the epilogue's reads set the pace (4096 tokens, 8 x (2048 -> 4096): layer 1988 / 1508 us)
-            g_up = torch.empty(LE, 2 * I, H, dtype=_BF16, device=dev).unbind(0)
-            g_down = torch.empty(LE, H, I, dtype=_BF16, device=dev).unbind(0)
+            # (a buffer per expert: a gradient that is kept keeps no other expert's memory).  Gradients in the optimizer's arena are
+            # still added to, since the arena may hold those of earlier micro-batches.
+            g_up = [torch.empty(2 * I, H, dtype=_BF16, device=dev) for _ in range(LE)]
+            g_down = [torch.empty(H, I, dtype=_BF16, device=dev) for _ in range(LE)]
         ups = [OF._as_strided_cat(expert_ws[3 * e:3 * e + 2]) for e in range(LE)]
         downs = [expert_ws[3 * e + 2] for e in range(LE)]
         # down projection: da = dy W2, dW2 += dy^T a

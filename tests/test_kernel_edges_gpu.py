@@ -269,4 +269,5 @@ def test_moe_expert_without_tokens_gets_zero_gradients():
     _status_ok()
     for n, g in grads.items():
         assert torch.isfinite(g).all(), n
+        assert "experts." not in n or g.untyped_storage().nbytes() <= 2 * 2 * I * H, n        # kept without the other experts' memory
         assert ("experts.2." in n) == (not g.any()), n

@@ -37,7 +37,7 @@ extern "C" int lb_sm_count() { return lb_num_sms(); }
 //   fwd: h = x (+ res);  rstd = rsqrt(mean(h^2) + eps);  y = h * rstd * w
 // Memory bound (x, res in; h, y out).  Rows of up to 4096 columns stay in registers between the sum of
 // squares and the scaling (NV 16-byte vectors per lane, all loads of a row in flight at once); wider rows are
-// read a second time.  With the residual, read twice / kept: 16384 x 2048 55.4 / 51.4 us (5.2 TB/s), 16384 x 4096 110 / 98.5.
+// read a second time.  With the residual, read twice / kept: 16384 x 2048 55.7 / 49.4 us (5.4 TB/s), 16384 x 4096 113 / 94.
 // ---------------------------------------------------------------------------------------
 template <bool HAS_RES, int NV>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_reg_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res,
@@ -142,19 +142,24 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const bf16* __restrict
 template <bool HAS_RES>
 static void rmsnorm_fwd_launch(const void* x, const void* res, const void* w, void* h, void* y, void* rstd, int rows, int cols,
                                float eps, cudaStream_t s) {
-  // fewer warps per block while that still leaves SMs without a block (a short batch)
-  int wpb = 8;
+  // Small blocks: the registers of a row are many, and with 256 threads a block they leave a good part of an SM's unused (rows with
+  // the residual, 8 / 2 warps per block: 16384 x 3072 82 / 68 us, which was more than reading twice takes at 8192 x 3072, 45 / 39 against
+  // 44; x 4096 100 / 94).  Four for the narrowest rows, whose blocks are over too soon (16384 x 256 9.1 / 9.9); one where that
+  // still leaves SMs without a block (a short batch).
+  const int nv = (cols / 8 + 31) / 32;
+  int wpb = nv <= 2 ? 4 : 2;
   while (wpb > 1 && (rows + wpb - 1) / wpb < 2 * lb_num_sms()) wpb >>= 1;
   const int blocks = (rows + wpb - 1) / wpb;
 #define LB_RMS_FWD(V)                                                                                               \
   rmsnorm_fwd_reg_kernel<HAS_RES, V><<<blocks, 32 * wpb, 0, s>>>((const bf16*)x, (const bf16*)res, (const bf16*)w,  \
                                                                  (bf16*)h, (bf16*)y, (float*)rstd, rows, cols, eps)
-  const int nv = (cols / 8 + 31) / 32;
   if (nv <= 2) LB_RMS_FWD(2);
   else if (nv <= 4) LB_RMS_FWD(4);
   else if (nv <= 6) LB_RMS_FWD(6);
   else if (nv <= 8) LB_RMS_FWD(8);
+  else if (nv <= 10) LB_RMS_FWD(10);
   else if (nv <= 12) LB_RMS_FWD(12);
+  else if (nv <= 14) LB_RMS_FWD(14);
   else if (nv <= 16) LB_RMS_FWD(16);
   else {
     const int b = (rows + 7) / 8 > lb_num_sms() * 8 ? lb_num_sms() * 8 : (rows + 7) / 8;

@@ -138,7 +138,8 @@ def test_swiglu_mlp_pair_tiles(T, K, I):
 # ---- norm ----------------------------------------------------------------------------------
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 264), (700, 1448), (301, 2056), (130, 4096), (65, 4104), (9, 8192), (5, 8200)])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 264), (700, 1448), (301, 2056), (130, 4096), (65, 4104), (9, 8192), (5, 8200),
+                                       (600, 520), (1187, 256), (301, 2312), (301, 2568), (301, 3336), (301, 3592), (700, 4104), (700, 6152), (700, 8192)])
 @pytest.mark.parametrize("residual", [False, True])
 def test_rmsnorm_widths(rows, cols, residual):
     from lightron_b200.ops import functional as OF

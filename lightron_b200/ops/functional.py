@@ -19,6 +19,7 @@ import torch.nn.functional as F
 
 from . import native, reference as ref
 
+
 class _NoGradCtx:
     """Stands in for the context of an autograd function whose backward cannot be asked for."""
 
@@ -26,12 +27,20 @@ class _NoGradCtx:
         pass
 
 
+try:        # not public: a torch without them keeps the autograd functions
+    _transforms_active, _tracing_state, _fwd_ad = (torch._C._are_functorch_transforms_active, torch._C._get_tracing_state,
+                                                   torch.autograd.forward_ad)
+    _fwd_ad._current_level
+except AttributeError:
+    _fwd_ad = None
+
+
 def _apply(fn, *args):
     """``fn.apply(*args)``; with gradients off, only ``fn.forward``: the autograd function then records nothing, and its
     Python wrapper is most of the host time of a small call.  Whatever else looks at autograd functions (function transforms, forward-mode
     derivatives, tracing) still gets the function."""
-    if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or torch._C._get_tracing_state() is not None
-            or torch.autograd.forward_ad._current_level >= 0):
+    if (torch.is_grad_enabled() or _fwd_ad is None or _transforms_active() or _tracing_state() is not None
+            or _fwd_ad._current_level >= 0):
         return fn.apply(*args)
     return fn.forward(_NoGradCtx(), *args)
 

@@ -178,10 +178,18 @@ def measured_peaks() -> dict:
         return {"hbm_gbs": 7700.0, "bf16_tflops": 2250.0, "bf16_tflops_sustained": 2250.0, "source": "nominal"}
 
 
+try:        # not public: without them the Stream object is built
+    _raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+except AttributeError:
+    _raw_stream = None
+
+
 def stream_ptr() -> int:
     """Handle of the current device's current stream (``torch.cuda.current_stream().cuda_stream`` without building the
     ``Stream`` object, which costs as much as the launch's argument conversion)."""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 def flash_bwd_workspace(B: int, Sq: int, hq: int, d: int, device) -> torch.Tensor:

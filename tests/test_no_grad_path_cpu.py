@@ -1,5 +1,9 @@
 """With gradients off the ops call an autograd function's forward directly; everything that looks at autograd functions
 still gets the function."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 import torch.autograd.forward_ad as fwAD
@@ -59,6 +63,37 @@ def test_transforms_and_tangents_still_reach_the_function(wrapped):
             with pytest.raises(Exception):                      # no jvp rule: refused, the tangent is not dropped
                 OF._apply(_Twice, fwAD.make_dual(x, torch.ones_like(x)), y)
         assert wrapped
+
+
+def test_tracing_still_reaches_the_function(wrapped):
+    x, y = torch.randn(3), torch.randn(3)
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda a, b: OF._apply(_Twice, a, b), (x, y), check_trace=False)
+    assert wrapped and torch.equal(traced(x, y), 2 * x + y)
+
+
+def test_a_torch_without_the_private_names_uses_public_ones():
+    """Neither the short path nor the stream handle is needed: without the names that they read, the public way is taken."""
+    code = """
+import torch
+import torch.autograd.forward_ad
+del torch.autograd.forward_ad._current_level
+if hasattr(torch._C, "_cuda_getCurrentRawStream"): del torch._C._cuda_getCurrentRawStream
+from lightron_b200.ops import functional as OF, native
+class F(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        ctx.set_materialize_grads(False)        # only the real context has it
+        return 2 * x
+with torch.no_grad():
+    assert torch.equal(OF._apply(F, torch.ones(2)), torch.full((2,), 2.0))
+class S: cuda_stream = 7
+torch.cuda.current_stream = S
+assert native.stream_ptr() == 7
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 @pytest.mark.parametrize("n", [3, 5, 1])

@@ -46,7 +46,7 @@ def _attention64(q, k, v, do, causal):
     (2, 129, 129, 4, 2, True, 1.0),          # one row over
     (1, 255, 640, 2, 2, True, 1.0),          # more keys than queries
     (1, 300, 77, 2, 1, False, 1.0),          # last key block ragged, no mask
-    (9, 200, 200, 8, 4, True, 1.0),          # 36 (batch, kv head) pairs: past one scheduling group of 32
+    (9, 200, 200, 8, 4, True, 1.0),          # 36 (batch, kv head) pairs: past one of the backward's groups of 32
     (1, 700, 700, 4, 1, True, 8.0),          # large scores: the running maximum moves, exponents underflow
 ])
 def test_attention_tile_edges(B, Sq, Sk, hq, hkv, causal, scale, d):
@@ -58,6 +58,45 @@ def test_attention_tile_edges(B, Sq, Sk, hq, hkv, causal, scale, d):
     for name, g, w in zip(("o", "dq", "dk", "dv"), got, _attention64(q, k, v, do, causal)):
         if w.norm() > 1e-6:                  # (with one visible key dq and dk vanish)
             assert _rel(g, w) < 1e-2, name
+
+
+def test_attention_forward_second_group_of_heads():
+    """Longest tiles first within as many heads as have 48 MB of keys and values: 24 of these 32, the second group smaller."""
+    from lightron_b200.ops import functional as OF
+    B, Sq, Sk, hq, hkv, d = 2, 300, 8192, 16, 8, 128
+    q, k, v = _rand(B, Sq, hq, d, seed=1), _rand(B, Sk, hkv, d, seed=2), _rand(B, Sk, hkv, d, seed=3)
+    o, lse = OF.flash_fwd_native(q, k, v, True, d ** -0.5)
+    _status_ok()
+    for b in range(B):
+        for h in range(hq):
+            s = (q[b, :, h].double() @ k[b, :, h // 2].double().t()) * d ** -0.5
+            s.masked_fill_(torch.ones(Sq, Sk, dtype=torch.bool, device="cuda").triu(1 + Sk - Sq), -float("inf"))
+            assert _rel(o[b, :, h], s.softmax(-1) @ v[b, :, h // 2].double()) < 5e-3, (b, h)
+            assert torch.allclose(lse[b, h].double(), s.logsumexp(-1), atol=1e-4), (b, h)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("n,Sk,S", [(128, 384, 512), (200, 300, 640)])
+def test_attention_over_a_prefix_of_longer_buffers(n, Sk, S, d):
+    """Context parallelism: the first Sk keys of every batch of a gather buffer of S rows, each 128-key block behind a counter (which
+    has been reached here: one rank waits for nobody), and the backward over the same buffers."""
+    from lightron_b200.ops import functional as OF, native
+    from lightron_b200.parallel import cp_fused
+    B, hq, hkv = 2, 4, 2
+    q, do = _rand(B, n, hq, d, seed=1), _rand(B, n, hq, d, seed=4)
+    kb, vb = _rand(B, S, hkv, d, seed=2), _rand(B, S, hkv, d, seed=3)
+    kb[:, Sk:], vb[:, Sk:] = 100.0, -100.0                               # not yet keys of this prefix
+    o, lse = torch.empty_like(q), torch.empty(B, hq, n, device="cuda")
+    flags = torch.full((B, S // 128), 5, dtype=torch.int32, device="cuda")
+    native.call("lb_flash_fwd_cp", q.data_ptr(), kb.data_ptr(), vb.data_ptr(), o.data_ptr(), lse.data_ptr(), B, n, Sk, S, hq, hkv, d,
+                hq * d, hq * d, d ** -0.5, 1, flags.data_ptr(), 5, 0, 0, 0, 0, 0, 1, 0, None, None, None, 0, native.stream_ptr())
+    got = (o, *cp_fused._bwd_call(q, kb, vb, Sk, S, o, lse, do, d ** -0.5))
+    _status_ok()
+    want = _attention64(q, kb[:, :Sk].contiguous(), vb[:, :Sk].contiguous(), do, True)
+    for name, g, w in zip(("o", "dq", "dk", "dv"), got, want):
+        assert _rel(g, w) < 1e-2, name
+    o2, _ = OF.flash_fwd_native(q, kb[:, :Sk].contiguous(), vb[:, :Sk].contiguous(), True, d ** -0.5)
+    assert torch.equal(o, o2)
 
 
 @pytest.mark.parametrize("B,Sq,d,shift", [(1, 2, 64, 0), (2, 129, 128, 1)])
@@ -103,13 +142,27 @@ def test_attention_bad_scores_stay_in_their_rows(d, bad):
 # ---- GEMM --------------------------------------------------------------------------------------------
 
 
-@pytest.mark.parametrize("M,N,K", [(5000, 2312, 72), (4096, 2304, 512), (4225, 4104, 200), (130, 520, 1032), (1, 8, 8)])
+def _ctas_per_tile(*problems):
+    """1 or 2: the form of the grouped GEMM that these (M, N, K) are launched in on this device."""
+    import ctypes
+    from lightron_b200.ops import native
+    IA = ctypes.c_int * len(problems)
+    return native.require().lb_gemm_grouped_ctas_per_tile(len(problems), *(IA(*[p[i] for p in problems]) for i in range(3)), native.sm_count())
+
+
+@pytest.mark.parametrize("M,N,K,ctas", [
+    (9000, 2312, 1032, 2),                   # several tiles per pair, the last ones ragged in rows, columns and depth
+    (4225, 4104, 2056, 2),
+    (130, 520, 4104, 2), (1, 8, 4096, 2),    # one tile: the second CTA's rows beyond the matrix
+    (5000, 2312, 72, 1), (4096, 2304, 512, 1), (4225, 4104, 200, 1), (130, 520, 1032, 1), (1, 8, 8, 1),
+])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
-def test_gemm_pair_tiles(M, N, K, a_mn, b_mn):
-    """Many tiles (CTA pairs, the last tiles ragged in rows and columns) and few (single CTAs), plain and accumulating."""
+def test_gemm_pair_tiles(M, N, K, ctas, a_mn, b_mn):
+    """Pairs of CTAs and single ones, plain and accumulating; which form ran is part of the test."""
     from lightron_b200.ops import functional as OF
     if a_mn and M % 8:
         M = M // 8 * 8 + 8
+    assert _ctas_per_tile((M, N, K)) == ctas
     a, b, c0 = _rand(M, K, seed=1), _rand(N, K, seed=2), _rand(M, N, seed=3)
     ops = (a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b)
     want = a.double() @ b.double().t()
@@ -120,9 +173,12 @@ def test_gemm_pair_tiles(M, N, K, a_mn, b_mn):
     assert _rel(out, want + c0.double()) < 5e-3
 
 
-@pytest.mark.parametrize("T,K,I", [(4000, 256, 1288), (70, 512, 264)])
-def test_swiglu_mlp_pair_tiles(T, K, I):
+@pytest.mark.parametrize("T,K,I,ctas", [(300, 4096, 264, 2), (2100, 1032, 2312, 2), (4000, 256, 1288, 1), (70, 512, 264, 1)])
+def test_swiglu_mlp_pair_tiles(T, K, I, ctas):
+    """The activation in the epilogue of pairs, whose peer loads the up rows, and of single CTAs; ragged in every size."""
     from lightron_b200.ops import functional as OF
+    assert _ctas_per_tile((T, 2 * I, K)) == ctas
+    assert ctas == 1 or _ctas_per_tile((K, I, T), (T, I, K)) == 2       # down projection: weight gradient and dg | du
     w13 = _rand(2 * I, K, scale=K ** -0.5, seed=2)
     ins = [t.detach().requires_grad_(True) for t in (_rand(T, K, seed=1), w13[:I], w13[I:], _rand(K, I, scale=I ** -0.5, seed=3))]
     dy = _rand(T, K, seed=4)

@@ -4,11 +4,13 @@
 // the tensor pipe.  Per 128-key block:
 //     S_t = Q_t K^T          tcgen05.mma, 128x128xd, operands in 128B-swizzled smem (TMA), D in TMEM
 //     softmax(S_t)           one thread per query row reads its row straight from TMEM
-//                            (tcgen05.ld), so max / sum need no shuffles; P_t goes back as packed
-//                            bf16 pairs, to TMEM (d = 64) or to swizzled smem (d = 128, FaCfg)
-//     O_t (+)= P_t V         tcgen05.mma with P_t as the A operand, 128 x d x 128, V is the MN-major
+//                            (tcgen05.ld), so max / sum need no shuffles; P_t goes back to TMEM as
+//                            packed bf16 pairs (tcgen05.st)
+//     O_t (+)= P_t V         tcgen05.mma with the A operand in TMEM, 128 x d x 128, V is the MN-major
 //                            B operand as it sits in memory; issued in two halves of 64 keys, the
 //                            first while the exponentials of the second are still being computed
+// P never touches shared memory: with P staged there the kernel was bound by shared-memory
+// bandwidth (128 B/clk: the P stores, the A-operand reads of P V and of Q K^T, the TMA writes).
 // O_t stays in TMEM for the whole key loop; when a row maximum grows the softmax threads rescale
 // it in place (tcgen05.ld / st) before the next P V is issued.
 // Warp roles (384 threads): warp 0 TMA producer, warps 1 / 2 MMA issuers of tile 0 / 1 (warp 1
@@ -16,11 +18,9 @@
 // The two tiles run half a period apart (tile 1 starts late on purpose): the exponentials of one
 // then overlap the loads, maxima and waits of the other instead of queueing on the same MUFU unit.
 // What bounds it: 16 exponentials per clock per SM are 1024 cycles per 128x128 block against 542 (d = 64)
-// or 1020 (d = 128) cycles of tensor pipe; a tile's softmax, P V and next softmax follow one another, and two tiles leave
-// gaps on both units; full launches at d = 128 also run at the power limit.  Measured in loops of 0.35 s before / after P V was split
-// and the longest tiles of all heads came first, with the SM clock: B8 S2048 32q/4kv d64 286 / 265 us (1965 MHz), B1 S8192 32q/8kv
-// d128 655 / 591 (1935 / 1815 MHz), B3 S1531 32q/8kv d128 112 / 88 (1965 MHz).  Scaling and summing use two-wide fp32
-// instructions and the maximum three-input ones.
+// or 1020 (d = 128) cycles of tensor pipe; a tile's softmax, P V and next S follow one another, and two tiles leave
+// gaps on both units.  Measured before / after P left shared memory at d = 128, P V was split and the longest tiles of
+// all heads came first: B8 S2048 32q/4kv d64 286 / 267 us, B1 S8192 32q/8kv d128 644 / 575, B3 S1531 32q/8kv d128 111 / 102.  Scaling and summing use two-wide fp32 instructions and the maximum three-input ones.
 // (A polynomial on the FMA pipe for one pair of exponentials in four was measured slower: 663 against 576 us at B1 S8192
 // 32q/8kv d128, 274 against 266 us at B8 S2048 32q/4kv d64.)
 // Layout / masking conventions are those of flash_attn.cu.
@@ -92,24 +92,22 @@ template <int D>
 struct FaCfg {
   static constexpr int BM = 128, BN = 128;
   static constexpr int KS = (D == 64) ? 3 : 2;
-  static constexpr int VS = (D == 64) ? 3 : 1;
+  static constexpr int VS = (D == 64) ? 3 : 2;
   static constexpr int ATOMS = D / 64;
   static constexpr int ATOM_BYTES = 128 * 128;          // 128 rows x 128 B
   static constexpr int TILE_BYTES = ATOMS * ATOM_BYTES; // one Q / K / V tile
   // TMEM columns: S_t fp32 [128], O_t fp32 [D], P_t packed bf16 [64].  With head_dim 64 all six
-  // regions fit in the 512 columns and P never touches shared memory.  With head_dim 128 S and O fill
-  // them and P_t is staged in shared memory, so that S of the next key block is issued as soon as the
-  // softmax threads hold the current one in registers.  (P_t in columns of S_t, with the next S_t behind
-  // P_t V: one CTA with 32 key blocks 84.6 us against 76.7, B1 S8192 32q/8kv 581 against 553.)
-  static constexpr bool P_SMEM = (D == 128);
-  static constexpr int COL_S = 0, COL_O = 256, COL_P = 384;
-  static constexpr int P_STRIDE = 64;
+  // regions fit in the 512 columns, and S of the next key block is issued as soon as the softmax
+  // threads hold the current one in registers.  With head_dim 128 S and O fill the 512 columns and
+  // P_t takes the first half of S_t's: the next S_t is then issued right behind P_t V (the tensor
+  // pipe runs the two in order), and the other tile's work fills the time of the softmax.
+  static constexpr bool P_ALIAS = (D == 128);
+  static constexpr int COL_S = 0, COL_O = 256, COL_P = P_ALIAS ? 0 : 384;
+  static constexpr int P_STRIDE = P_ALIAS ? 128 : 64;
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_K = OFF_Q + 2 * TILE_BYTES;
   static constexpr int OFF_V = OFF_K + KS * TILE_BYTES;
-  static constexpr int P_BYTES = P_SMEM ? 2 * ATOM_BYTES : 0;       // 128 x 128 bf16
-  static constexpr int OFF_P = OFF_V + VS * TILE_BYTES;
-  static constexpr int OFF_BAR = OFF_P + 2 * P_BYTES;
+  static constexpr int OFF_BAR = OFF_V + VS * TILE_BYTES;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
   static constexpr int NBAR = 1 + 2 * KS + 2 * VS + 10;
 };
@@ -180,7 +178,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   auto p_full = [&](int t) { return bar1 + 8u * (2 + t); };
   auto pv_done = [&](int t) { return bar1 + 8u * (4 + t); };
   auto s_free = [&](int t) { return bar1 + 8u * (6 + t); };
-  auto p_half = [&](int t) { return bar1 + 8u * (8 + t); };     // first 64 keys of P are written
+  auto p_half = [&](int t) { return bar1 + 8u * (8 + t); };     // first 64 keys of P are in TMEM
 
   // 1-D grid: movers first (they must be resident before anything waits for data), then the
   // (batch, head, query tile) CTAs.  Causal tiles differ in length by up to the number of key blocks, so
@@ -262,8 +260,9 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     // ------------------------------- MMA issuers -------------------------------
     // One issuing thread per query tile (a single thread feeding both tiles was measured to bound the
     // kernel: a tcgen05.mma blocks its issuer for about its own execution time).  Each thread follows
-    // the fixed order of its own tile with blocking waits: S(0); then per key block S(j+1) as soon as the
-    // softmax threads hold S(j) in registers, and P(j) V in two halves as P(j) arrives.
+    // the fixed order of its own tile with blocking waits: S(0); then per key block, head_dim 64: S(j+1)
+    // as soon as the softmax threads hold S(j) in registers, and P(j) V in two halves as P(j) arrives;
+    // head_dim 128: P(j) V, then S(j+1) into the columns that P(j) leaves.
     // A K / V stage is free once BOTH tiles have used it, so each thread arrives on the stage's
     // empty barrier for every block, also for blocks its own tile does not need.
     const int t = warp - 1;
@@ -277,7 +276,6 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       const uint32_t s_dst = tmem_base + C::COL_S + t * C::BN;
       const uint32_t o_dst = tmem_base + C::COL_O + t * D;
       const uint32_t pa = tmem_base + C::COL_P + t * C::P_STRIDE;          // 8 columns per K = 16 slice
-      const uint64_t dp0 = make_desc(sbase + C::OFF_P + t * C::P_BYTES, 16, 1024);
       const int n_my = nb[t];
       bool ok = mbar_wait(q_full, 0, abort_flag);
       auto issue_s = [&](int j) -> bool {             // S(j) = Q K(j)^T, then release K(j)'s stage
@@ -300,20 +298,16 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         if (!mbar_wait(p_half(t), (uint32_t)j & 1u, abort_flag)) return false;
         fence_after();
         const uint64_t va = dv0 + (uint64_t)((vs * C::TILE_BYTES) >> 4);
-        auto pv = [&](int s) {                        // 16 keys
-          if (C::P_SMEM)
-            umma_bf16(o_dst, dp0 + (uint64_t)(((s >> 2) * C::ATOM_BYTES + (s & 3) * 32) >> 4), va + (uint64_t)((s * 2048) >> 4), idesc_o,
-                      j | s ? 1u : 0u);
-          else
-            umma_bf16_ta(o_dst, pa + 8u * s, va + (uint64_t)((s * 2048) >> 4), idesc_o, j | s ? 1u : 0u);
-        };
+        umma_bf16_ta(o_dst, pa, va, idesc_o, j ? 1u : 0u);
 #pragma unroll
-        for (int s = 0; s < C::BN / 32; s++) pv(s);
+        for (int s = 1; s < C::BN / 32; s++)
+          umma_bf16_ta(o_dst, pa + 8u * s, va + (uint64_t)((s * 2048) >> 4), idesc_o, 1u);
         if (!mbar_wait(p_full(t), (uint32_t)j & 1u, abort_flag)) return false;
         fence_after();
 #pragma unroll
-        for (int s = C::BN / 32; s < C::BN / 16; s++) pv(s);
-        umma_commit(pv_done(t));
+        for (int s = C::BN / 32; s < C::BN / 16; s++)
+          umma_bf16_ta(o_dst, pa + 8u * s, va + (uint64_t)((s * 2048) >> 4), idesc_o, 1u);
+        if (!C::P_ALIAS || j == n_my - 1) umma_commit(pv_done(t));
         umma_commit(v_empty(vs));
         return true;
       };
@@ -323,11 +317,12 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       if (ok && t == 1 && nb[0] > 0 && n_my > 0) ok = mbar_wait(s_free(0), 0u, abort_flag);
       if (ok && n_my > 0) ok = issue_s(0);
       for (int j = 0; j < n_my && ok; j++) {
-        if (j + 1 < n_my) {
+        if (!C::P_ALIAS && j + 1 < n_my) {
           ok = mbar_wait(s_free(t), (uint32_t)j & 1u, abort_flag);
           if (ok) ok = issue_s(j + 1);
         }
         if (ok) ok = issue_pv(j);
+        if (C::P_ALIAS && ok && j + 1 < n_my) ok = issue_s(j + 1);
       }
       // blocks that only the other tile needs: keep the stage rings in step
       for (int j = n_my; j < nb_max && ok; j++) {
@@ -348,7 +343,6 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     const uint32_t ts_addr = lane_addr + C::COL_S + t * C::BN;
     const uint32_t to_addr = lane_addr + C::COL_O + t * D;
     const uint32_t tp_addr = lane_addr + C::COL_P + t * C::P_STRIDE;
-    uint8_t* sP = smem + C::OFF_P + t * C::P_BYTES;
     const float sl2 = p.scale * 1.4426950408889634f;
     const f32x2 sl2x2 = pack2(sl2, sl2);
     float m_i = -INFINITY, l_i = 0.f;
@@ -380,7 +374,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         if (half == 1) {
           tmem_ld_wait();
           fence_before();
-          mbar_arrive(s_free(t));                     // S_t may be overwritten by the next key block
+          if (!C::P_ALIAS || j == 0) mbar_arrive(s_free(t));   // S_t may be overwritten by the next key block
         }
         if (need_mask) {
 #pragma unroll
@@ -400,10 +394,10 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       const float m_s = (m_new == -INFINITY) ? 0.f : (m_new == INFINITY ? __int_as_float(0x7fffffff) : m_new * sl2);
       const float corr = (m_i == -INFINITY) ? 0.f : exp2f(m_i * sl2 - m_s);
       FA_T(3);
-      // exponentials; P goes back as packed bf16 pairs (in TMEM column c holds keys 2c, 2c+1), 64 keys at a
-      // time, so that P V of the first half runs while the second is computed.  The first half is computed
-      // BEFORE waiting for the previous P V (which still reads P and owns O): its 64 exponentials overlap
-      // the tail of that MMA.
+      // exponentials; P goes back to TMEM as packed bf16 pairs (column c holds keys 2c, 2c+1), 32
+      // columns per store so that the first store is in flight while the second half is computed.
+      // The first half is computed BEFORE waiting for the previous P V (which still reads the P
+      // columns and owns O): its 64 exponentials overlap the tail of that MMA.
       const f32x2 nms2 = pack2(-m_s, -m_s);
       f32x2 rs2[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
 #pragma unroll
@@ -422,9 +416,12 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
           pr[c] = *reinterpret_cast<uint32_t*>(&pk);
         }
         if (hh == 0 && j > 0) {
-          // previous P V finished: O is stable and P may be overwritten
-          if (!mbar_wait(pv_done(t), (uint32_t)(j - 1) & 1u, abort_flag)) { ok = false; }
-          fence_after();
+          // previous P V finished: O is stable and the P columns may be overwritten.  (head_dim 128: S(j) was
+          // issued behind it by the same thread, so its completion says that P V has completed too.)
+          if (!C::P_ALIAS) {
+            if (!mbar_wait(pv_done(t), (uint32_t)(j - 1) & 1u, abort_flag)) { ok = false; }
+            fence_after();
+          }
           if (ok && __any_sync(0xffffffffu, !(m_new == m_i))) {
 #pragma unroll 1
             for (int c = 0; c < D / 32; c++) {
@@ -438,17 +435,8 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             tmem_st_wait();
           }
         }
-        if (C::P_SMEM) {
-          // keys hh * 64 .. + 63 of this row are 128 bytes: one row of swizzle atom hh
-#pragma unroll
-          for (int c = 0; c < 8; c++)
-            *reinterpret_cast<uint4*>(sP + hh * C::ATOM_BYTES + sw128_off(rit, c)) =
-                make_uint4(pr[c * 4], pr[c * 4 + 1], pr[c * 4 + 2], pr[c * 4 + 3]);
-          fence_proxy_async_smem();
-        } else {
-          tmem_st32(tp_addr + hh * 32, pr);
-          tmem_st_wait();
-        }
+        tmem_st32(tp_addr + hh * 32, pr);
+        tmem_st_wait();
         fence_before();
         mbar_arrive(hh == 0 ? p_half(t) : p_full(t));
       }
@@ -470,7 +458,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       for (int i = 0; i < 8; i++) atomicAdd(&g_fa_prof[i], prof[i]);
 #endif
     if (ok && n_my > 0) {
-      if (!mbar_wait(pv_done(t), (uint32_t)(n_my - 1) & 1u, abort_flag)) ok = false;
+      if (!mbar_wait(pv_done(t), C::P_ALIAS ? 0u : (uint32_t)(n_my - 1) & 1u, abort_flag)) ok = false;
     }
     if (ok && n_my > 0) {
       fence_after();

@@ -19,9 +19,11 @@
 // their own: TMEM -> registers -> staging -> asynchronous bulk reduce-add (cp.reduce.async.bulk .add.f32)
 // into an fp32 accumulator in global memory, whose layout is the staging layout (un-permuted by the final
 // convert kernel), so no atomic instructions pass through the load/store pipe.
-// Bound by shared-memory bandwidth at head_dim 128 (about 3700 cycles per block of operand reads, dS and dQ staging against
-// 2560 of tensor pipe).  Measured whole (statistics, main, convert), the earlier form / this one: B8 S2048 32q/4kv d64 935 / 615 us,
-// B1 S8192 32q/8kv d128 2632 / 1475, B3 S1531 32q/8kv d128 438 / 250.
+// No unit is full (counters at B4 S2048 32q/8kv d128 / B8 S2048 32q/4kv d64: tensor pipe 46 / 32 % of the active cycles, L1 and shared
+// memory 58 / 39 %, exponentials 20 / 28 %): what bounds it is the order of a block's phases, of which one CTA per SM holds one block, and
+// at d = 128 the dQ that waits for its drain in dP's columns, besides the power limit.  Loops of 0.35 s of all its kernels with the SM clock, the
+// earlier form / this one: B8 S2048 32q/4kv d64 934 (1965 MHz) / 658 us (1830 MHz), B1 S8192 32q/8kv d128 2650 (1965) / 1664 (1670),
+// B3 S1531 32q/8kv d128 438 (1965) / 244 (1705).
 // Warp roles (512 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4-11 math, 12-15 dQ drain.
 // All waits are bounded; on expiry a status word is set and the CTA drains and frees its TMEM.
 #include "tcgen05.cuh"

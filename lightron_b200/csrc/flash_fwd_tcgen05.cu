@@ -9,8 +9,7 @@
 //     O_t (+)= P_t V         tcgen05.mma with the A operand in TMEM, 128 x d x 128, V is the MN-major
 //                            B operand as it sits in memory; issued in two halves of 64 keys, the
 //                            first while the exponentials of the second are still being computed
-// P never touches shared memory: with P staged there the kernel was bound by shared-memory
-// bandwidth (128 B/clk: the P stores, the A-operand reads of P V and of Q K^T, the TMA writes).
+// P never touches shared memory, whose bandwidth (128 B/clk) the operand reads and the TMA writes share.
 // O_t stays in TMEM for the whole key loop; when a row maximum grows the softmax threads rescale
 // it in place (tcgen05.ld / st) before the next P V is issued.
 // Warp roles (384 threads): warp 0 TMA producer, warps 1 / 2 MMA issuers of tile 0 / 1 (warp 1
@@ -19,10 +18,14 @@
 // then overlap the loads, maxima and waits of the other instead of queueing on the same MUFU unit.
 // What bounds it: 16 exponentials per clock per SM are 1024 cycles per 128x128 block against 542 (d = 64)
 // or 1020 (d = 128) cycles of tensor pipe; a tile's softmax, P V and next S follow one another, and two tiles leave
-// gaps on both units.  Measured before / after P left shared memory at d = 128, P V was split and the longest tiles of
-// all heads came first: B8 S2048 32q/4kv d64 286 / 267 us, B1 S8192 32q/8kv d128 644 / 575, B3 S1531 32q/8kv d128 111 / 102.  Scaling and summing use two-wide fp32 instructions and the maximum three-input ones.
+// gaps on both units (counters at B8 S2048 32q/4kv d64 / B4 S2048 32q/8kv d128: exponentials 52 / 37 % of the active cycles, tensor pipe
+// 25 / 36 %).  Loops of 0.35 s with the SM clock, before / after P left shared memory at d = 128, P V was split and the longest tiles of
+// all heads came first: B8 S2048 32q/4kv d64 286 / 265 us (1965 MHz), B1 S8192 32q/8kv d128 655 (1935) / 606 (1880), B3 S1531
+// 32q/8kv d128 112 / 89 (1965).  Scaling and summing use two-wide fp32 instructions and the maximum three-input ones.
 // (A polynomial on the FMA pipe for one pair of exponentials in four was measured slower: 663 against 576 us at B1 S8192
-// 32q/8kv d128, 274 against 266 us at B8 S2048 32q/4kv d64.)
+// 32q/8kv d128, 274 against 266 us at B8 S2048 32q/4kv d64.  P in shared memory at d = 128 with the next scores ahead of P V and one V
+// stage: 2 to 9 % faster where K and V are in L2 and there are less than two CTAs per SM, 2 to 5 % slower where they are not,
+// B3 S1531 92.8 against 95.2 us; not kept.)
 // Layout / masking conventions are those of flash_attn.cu.
 // All waits are bounded; on expiry a status word is set and the CTA drains and frees its TMEM.
 #include <string.h>

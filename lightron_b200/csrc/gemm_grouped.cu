@@ -6,13 +6,15 @@
 // full).  Launching the data gradient and the weight gradient of a linear layer together, or
 // the GEMMs of all local experts of a MoE layer, gives the scheduler short tiles to fill those
 // holes.  The host computes a static schedule (longest tiles first, each to the least loaded
-// CTA), uploads it once per shape, and every role of a CTA walks the same list, so no
-// intra-kernel tile broadcast is needed.
+// worker), uploads it once per shape, and every role of a worker walks the same list, so no
+// intra-kernel tile broadcast is needed.  A worker is a CTA with tiles of 128x256 or a pair of CTAs
+// (tcgen05 cta_group::2) with tiles of 256x256: Cfg has the two forms, choose_cg the choice.
 //
-// The main loop is the one of gemm_tcgen05.cu: TMA (128-byte swizzle, no multicast) -> 4-stage
-// mbarrier ring -> tcgen05.mma 128x256x16 -> two 256-column TMEM accumulators -> tcgen05.ld
-// epilogue overlapped with the next tile.  `accumulate` adds the old contents of C in the
-// epilogue (gradient accumulation over micro-batches without a separate add).
+// The main loop is the one of gemm_tcgen05.cu: TMA (128-byte swizzle, no multicast) -> mbarrier ring
+// of 4 (CTA) or 6 (pair) stages -> tcgen05.mma 128x256x16 / 256x256x16 -> two 256-column TMEM accumulators
+// per CTA -> tcgen05.ld epilogue overlapped with the next tile.  `accumulate` adds the old contents of C in
+// the epilogue (gradient accumulation over micro-batches without a separate add).
+// The ragged kernel (lb_gemm_ragged, lb_gemm_ragged_wgrad) uses the CTA form and takes its tiles from device memory.
 // Every wait is bounded; on expiry the kernel records a status code (lb_gemm_grouped_status),
 // stops issuing work, frees its TMEM and returns.
 #include <cuda.h>
@@ -341,9 +343,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
         bw::fence_before();
         __syncwarp();
         if (lane == 0) {
-        if constexpr (CG == 2) bw::mbar_arrive_leader(tempty_bar(acc));
-        else bw::mbar_arrive(tempty_bar(acc));
-      }
+          if constexpr (CG == 2) bw::mbar_arrive_leader(tempty_bar(acc));
+          else bw::mbar_arrive(tempty_bar(acc));
+        }
         continue;
       }
       if (epi == 2) {
@@ -394,9 +396,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
         bw::fence_before();
         __syncwarp();
         if (lane == 0) {
-        if constexpr (CG == 2) bw::mbar_arrive_leader(tempty_bar(acc));
-        else bw::mbar_arrive(tempty_bar(acc));
-      }
+          if constexpr (CG == 2) bw::mbar_arrive_leader(tempty_bar(acc));
+          else bw::mbar_arrive(tempty_bar(acc));
+        }
         continue;
       }
 #pragma unroll 1

@@ -439,9 +439,10 @@ __global__ void __launch_bounds__(256) moe_pull_kernel(const PullParams p) {
 // Router backward
 // -------------------------------------------------------------------------------------------
 // A block takes 64 tokens x 256 columns: warp w the tokens 8 w .. 8 w + 7, a lane 8 columns.  A warp's tokens stay in registers over
-// the experts, whose gate weights are fetched once for all of them, and the block's share of the gate gradient is summed over its warps in shared memory
-// before one vector reduction per 4 columns (four atomics where the gradient does not start on 16 bytes).  (A block per 64 tokens and all columns left most SMs idle and fetched the weights
-// again for every token: T 4096, H 2048, E 8 100 us, now 28.)
+// the experts, whose gate weights are fetched once for all of them, and the block's share of the gate gradient is summed over its
+// warps in shared memory before one vector reduction per 4 columns (four atomics where the gradient does not start on 16 bytes).
+// (A block per 64 tokens and all columns left most SMs idle and fetched the weights again for every token: T 4096, H 2048, inputs
+// not in L2, E 8 108 us, now 35; E 64 688, now 184.)
 constexpr int RB_TOKENS = 64, RB_COLS = 256, RB_WARPS = 8, RB_TPW = RB_TOKENS / RB_WARPS;
 
 __global__ void __launch_bounds__(RB_WARPS * 32)

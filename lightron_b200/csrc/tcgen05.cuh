@@ -248,7 +248,7 @@ __device__ __forceinline__ void named_bar_sync(int id, int count) {
 
 // Bulk (non-tensor) asynchronous reduce-add of contiguous fp32 from shared to global memory.
 // Addresses 16-byte aligned, size a multiple of 16.  The data is read by the async proxy: call
-// fence_proxy_async_smem() after writing it, and bulk_wait_read() before reusing the buffer.
+// fence_proxy_async_smem() after writing it, and bulk_wait_read_but<0>() (or <PENDING>, of several buffers) before reusing it.
 __device__ __forceinline__ void bulk_reduce_add_f32(void* gdst, uint32_t ssrc, uint32_t bytes) {
   asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(gdst), "r"(ssrc), "r"(bytes)
                : "memory");
@@ -257,7 +257,6 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 template <int PENDING>
 __device__ __forceinline__ void bulk_wait_read_but() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
 // Bulk (non-tensor) copy global -> this CTA's shared memory, counted on `bar`.  Addresses and size in units of 16 bytes.
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {

@@ -1,31 +1,30 @@
 // FlashAttention forward on the 5th-generation tensor cores (sm_100a), head_dim 64 or 128.
 //
-// One CTA owns 256 consecutive queries of one (batch, head): two 128-row tiles that ping-pong on
-// the tensor pipe.  Per 128-key block:
-//     S_t = Q_t K^T          tcgen05.mma, 128x128xd, operands in 128B-swizzled smem (TMA), D in TMEM
-//     softmax(S_t)           one thread per query row reads its row straight from TMEM
-//                            (tcgen05.ld), so max / sum need no shuffles; P_t goes back to TMEM as
-//                            packed bf16 pairs (tcgen05.st)
-//     O_t (+)= P_t V         tcgen05.mma with the A operand in TMEM, 128 x d x 128, V is the MN-major
-//                            B operand as it sits in memory; issued in two halves of 64 keys, the
-//                            first while the exponentials of the second are still being computed
+// A CTA works on one tile of 128 queries of one (batch, head) at a time; two CTAs share an SM.  Per 128-key block:
+//     S = Q K^T          tcgen05.mma, 128x128xd, operands in 128B-swizzled smem (TMA), D in TMEM
+//     softmax(S)         one thread per query row reads its row straight from TMEM
+//                        (tcgen05.ld), so max / sum need no shuffles; P goes back to TMEM as
+//                        packed bf16 pairs (tcgen05.st)
+//     O (+)= P V         tcgen05.mma with the A operand in TMEM, 128 x d x 128, V is the MN-major
+//                        B operand as it sits in memory; issued in two halves of 64 keys, the
+//                        first while the exponentials of the second are still being computed
 // P never touches shared memory, whose bandwidth (128 B/clk) the operand reads and the TMA writes share.
-// O_t stays in TMEM for the whole key loop; when a row maximum grows the softmax threads rescale
+// O stays in TMEM for the whole key loop; when a row maximum grows the softmax threads rescale
 // it in place (tcgen05.ld / st) before the next P V is issued.
-// Warp roles (384 threads): warp 0 TMA producer, warps 1 / 2 MMA issuers of tile 0 / 1 (warp 1
-// owns the TMEM allocation), warp 3 idle, warps 4-7 softmax of tile 0, warps 8-11 softmax of tile 1.
-// The two tiles run half a period apart (tile 1 starts late on purpose): the exponentials of one
-// then overlap the loads, maxima and waits of the other instead of queueing on the same MUFU unit.
+// Warp roles (256 threads): warp 0 TMA producer, warp 1 MMA issuer and owner of the TMEM allocation, warps 2-3 idle, warps 4-7 softmax.
 // What bounds it: 16 exponentials per clock per SM are 1024 cycles per 128x128 block against 542 (d = 64)
-// or 1020 (d = 128) cycles of tensor pipe; a tile's softmax, P V and next S follow one another, and two tiles leave
-// gaps on both units (counters at B8 S2048 32q/4kv d64 / B4 S2048 32q/8kv d128: exponentials 52 / 37 % of the active cycles, tensor pipe
-// 25 / 36 %).  Loops of 0.35 s with the SM clock, before / after P left shared memory at d = 128, P V was split and the longest tiles of
-// all heads came first: B8 S2048 32q/4kv d64 286 / 265 us (1965 MHz), B1 S8192 32q/8kv d128 655 (1935) / 606 (1880), B3 S1531
-// 32q/8kv d128 112 / 89 (1965).  Scaling and summing use two-wide fp32 instructions and the maximum three-input ones.
-// (A polynomial on the FMA pipe for one pair of exponentials in four was measured slower: 663 against 576 us at B1 S8192
-// 32q/8kv d128, 274 against 266 us at B8 S2048 32q/4kv d64.  P in shared memory at d = 128 with the next scores ahead of P V and one V
-// stage: 2 to 9 % faster where K and V are in L2 and there are less than two CTAs per SM, 2 to 5 % slower where they are not,
-// B3 S1531 92.8 against 95.2 us; not kept.)
+// or 1020 (d = 128) cycles of tensor pipe.  A tile's softmax, P V and next S follow one another, and the two CTAs of an SM fill each
+// other's gaps: a block of a tile that has the SM to itself takes 2350 cycles (d = 64) / 3050 (d = 128), one of two tiles 3200 / 3700 on
+// average.  At d = 128 the power limit comes on top (long loops run at 1.55 GHz).  What the single cycles went into, and what each was worth:
+//   * MMAs and loads are issued by an elected thread (elect_one): 8 MMAs in 590 instead of 1170 cycles;
+//   * one CTA per tile instead of two tiles per CTA and CTAs that go on with the next tile (cluster launch control): prologue and
+//     stores of a tile run under the other tile's blocks (d = 64 alone 265 -> 233 us);
+//   * waits that are sure to succeed are put ahead of the one that is not (some 150 cycles each), O leaves through TMA stores.
+// Loops of 0.35 s, two tiles per CTA / now, on one GPU: B8 S2048 32q/4kv d64 266 / 227 us, B1 S8192 32q/8kv d128 619 / 578,
+// B3 S1531 32q/8kv d128 92 / 82, B1 S4096 8q/8kv d128 82 / 62.  Scaling and summing use two-wide fp32 instructions and the maximum
+// three-input ones.  (Measured and not kept: a polynomial on the FMA pipe for one pair of exponentials in four; four tiles of 64-key blocks per
+// SM at d = 64, 236 us, and two score buffers of 64 keys at d = 128, 753 us, which load each K and V byte in smaller boxes and
+// leave one thread to issue everything; lists fixed in advance instead of launch control, 233 us against 224.)
 // Layout / masking conventions are those of flash_attn.cu.
 // All waits are bounded; on expiry a status word is set and the CTA drains and frees its TMEM.
 #include <string.h>
@@ -33,17 +32,6 @@
 #include "comm.cuh"
 
 static __device__ unsigned int g_fa_status[4] = {0, 0, 0, 0};
-
-// Developer instrumentation (build with -DLB_FA_PROFILE): cycles that lane 0 of every softmax warp
-// spends in each phase of the key-block loop, summed over the grid.  lb_flash_prof() reads and clears.
-#ifdef LB_FA_PROFILE
-static __device__ unsigned long long g_fa_prof[16];
-#define FA_T(i) const long long tp##i = clock64()
-#define FA_ACC(slot, a, b) prof[slot] += (unsigned long long)(tp##b - tp##a)
-#else
-#define FA_T(i)
-#define FA_ACC(slot, a, b)
-#endif
 
 namespace {
 using namespace bw;
@@ -55,7 +43,11 @@ using namespace bw;
 // destination's flag word.  The attention CTAs gate every 128-key block on its flag, so the
 // exchange overlaps the softmax / MMA work on blocks that have already arrived.
 constexpr int FA_MAX_RANKS = 8;
-constexpr int FA_FWD_THREADS = 384;
+constexpr int FA_FWD_THREADS = 256;
+// Registers per thread of the two warpgroups.  Two CTAs of 256 threads leave 128 per thread at launch; the issuing warpgroup gives most
+// of its share to the softmax threads, of which each holds a row of 128 scores.
+constexpr int FA_REGS_ISSUE = 56, FA_REGS_SOFTMAX = 200;
+static_assert(FA_REGS_ISSUE + FA_REGS_SOFTMAX <= 2 * 128, "a CTA has 256 x 128 registers");
 struct FaPush {
   int n_mov, n_ranks, rank, chunk_rows, row_elems;   // row_elems = hkv * d
   const bf16 *k_src, *v_src;                         // this rank's [B, 2*chunk_rows, hkv, d], token strides below
@@ -64,6 +56,18 @@ struct FaPush {
   bf16* v_dst[FA_MAX_RANKS];
   unsigned int* flags[FA_MAX_RANKS];                 // rank r's block counters [B][S_full / 128]
 };
+// Division of 0 <= x < 2^31 by a divisor that is fixed for the launch: a multiplication (the host finds m, which is exact for such x).
+struct FastDiv {
+  unsigned int d, m, s;
+  void set(unsigned int div) {
+    d = div;
+    s = 0;
+    while (s < 31 && (1u << s) < div) s++;                                        // 2^(s-1) < d <= 2^s
+    m = (unsigned int)((((unsigned long long)1 << (31 + s)) + div - 1) / div);    // < 2^32
+  }
+  __device__ __forceinline__ int div(int x) const { return (int)(((unsigned long long)(unsigned)x * m) >> (31 + s)); }
+};
+
 struct FaFwdParams {
   bf16* o;
   float* lse;
@@ -74,9 +78,11 @@ struct FaFwdParams {
   int kv_brows;                  // rows between consecutive batches in the K/V tensor maps (>= Sk)
   const unsigned int* kv_flags;  // null, or this rank's block counters [B][kv_brows / 128]
   unsigned int flag_target;
-  int tiles_x;                   // query tiles (256 rows) per (batch, head)
+  int tiles_x;                   // query tiles (128 rows) per (batch, head)
+  int steal;                     // CTAs go on with entries that have not been started
   int group;                     // (batch, head) pairs whose tiles are ordered together
   unsigned long long wait_ns;    // limit of a wait on a key block's arrival flag
+  FastDiv by_grp, by_group, by_last, by_hq, by_rep;    // entries of a group, heads of a group / of the last one, hq, hq / hkv
 };
 
 // Three-input maximum; a NaN in any input is the result.
@@ -94,31 +100,30 @@ __device__ __forceinline__ float max2(float a, float b) {
 template <int D>
 struct FaCfg {
   static constexpr int BM = 128, BN = 128;
-  static constexpr int KS = (D == 64) ? 3 : 2;
-  static constexpr int VS = (D == 64) ? 3 : 2;
   static constexpr int ATOMS = D / 64;
-  static constexpr int ATOM_BYTES = 128 * 128;          // 128 rows x 128 B
-  static constexpr int TILE_BYTES = ATOMS * ATOM_BYTES; // one Q / K / V tile
-  // TMEM columns: S_t fp32 [128], O_t fp32 [D], P_t packed bf16 [64].  With head_dim 64 all six
-  // regions fit in the 512 columns, and S of the next key block is issued as soon as the softmax
-  // threads hold the current one in registers.  With head_dim 128 S and O fill the 512 columns and
-  // P_t takes the first half of S_t's: the next S_t is then issued right behind P_t V (the tensor
-  // pipe runs the two in order), and the other tile's work fills the time of the softmax.
+  static constexpr int SLOT_BYTES = 128 * 128;          // K: 128 keys x 64 columns; V: 128 keys x 64 columns or 64 keys x 128 columns
+  static constexpr int SLOTS = 6 - ATOMS;               // 5 / 4
+  static constexpr int UNITS = 2 * ATOMS;               // slots that a key block takes, K before V
+  // TMEM columns: S fp32 [128], O fp32 [D], P packed bf16 [64], in the 256 that leave room for a second CTA.  With head_dim 64
+  // P has columns of its own and S of the next key block is issued as soon as the softmax threads hold the current one in
+  // registers.  With head_dim 128 P takes the first half of S's: the next S is then issued right behind P V (the tensor
+  // pipe runs the two in order), and the other CTA's work fills the time of the softmax.
   static constexpr bool P_ALIAS = (D == 128);
-  static constexpr int COL_S = 0, COL_O = 256, COL_P = P_ALIAS ? 0 : 384;
-  static constexpr int P_STRIDE = P_ALIAS ? 128 : 64;
+  static constexpr int COL_S = 0, COL_O = 128, COL_P = P_ALIAS ? 0 : 192, TMEM_COLS = 256;
   static constexpr int OFF_Q = 0;
-  static constexpr int OFF_K = OFF_Q + 2 * TILE_BYTES;
-  static constexpr int OFF_V = OFF_K + KS * TILE_BYTES;
-  static constexpr int OFF_BAR = OFF_V + VS * TILE_BYTES;
-  static constexpr int SMEM = OFF_BAR + 256 + 1024;
-  static constexpr int NBAR = 1 + 2 * KS + 2 * VS + 10;
+  static constexpr int OFF_RING = OFF_Q + ATOMS * SLOT_BYTES;
+  static constexpr int OFF_OUT = OFF_RING + SLOTS * SLOT_BYTES;   // 64 columns of O on their way out, 4 KB per softmax warp
+  static constexpr int OFF_BAR = OFF_OUT + SLOT_BYTES;
+  static constexpr int NBAR = 2 + 2 * SLOTS + 9;
+  static constexpr int SMEM = OFF_BAR + 256;
 };
+static_assert(FaCfg<64>::SMEM <= 115712 && FaCfg<128>::SMEM <= 115712, "two CTAs per SM");
 
 template <int D>
-__global__ void __launch_bounds__(FA_FWD_THREADS, 1)
+__global__ void __launch_bounds__(FA_FWD_THREADS, 2)
 fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
-                 const __grid_constant__ CUtensorMap tv, const FaFwdParams p, const FaPush push) {
+                 const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap to, const FaFwdParams p,
+                 const FaPush push) {
   using C = FaCfg<D>;
   if ((int)blockIdx.x < push.n_mov) {
     // ------------------------------- K/V mover CTAs -------------------------------
@@ -161,271 +166,314 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     }
     return;
   }
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NBAR);
-  __shared__ int s_abort[2];     // {abort, extra wait in ms}: see bw::mbar_wait
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NBAR + 5);     // behind two 16-byte answers
+  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);     // {abort, extra wait in ms}: see bw::mbar_wait
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform over the warp)
   const uint32_t sbase = smem_u32(smem);
+  if (sbase & 1023u) {                                       // the swizzled tiles need it; nothing has been started yet
+    if (threadIdx.x == 0) atomicExch(&g_fa_status[0], 4u);
+    return;
+  }
   const uint32_t bar0 = smem_u32(bars);
   // barrier map
-  const uint32_t q_full = bar0;
-  auto k_full = [&](int s) { return bar0 + 8u * (1 + s); };
-  auto k_empty = [&](int s) { return bar0 + 8u * (1 + C::KS + s); };
-  auto v_full = [&](int s) { return bar0 + 8u * (1 + 2 * C::KS + s); };
-  auto v_empty = [&](int s) { return bar0 + 8u * (1 + 2 * C::KS + C::VS + s); };
-  const uint32_t bar1 = bar0 + 8u * (1 + 2 * C::KS + 2 * C::VS);
-  auto s_full = [&](int t) { return bar1 + 8u * t; };
-  auto p_full = [&](int t) { return bar1 + 8u * (2 + t); };
-  auto pv_done = [&](int t) { return bar1 + 8u * (4 + t); };
-  auto s_free = [&](int t) { return bar1 + 8u * (6 + t); };
-  auto p_half = [&](int t) { return bar1 + 8u * (8 + t); };     // first 64 keys of P are in TMEM
+  const uint32_t q_full = bar0, q_empty = bar0 + 8;
+  auto full = [&](int s) { return bar0 + 8u * (2 + s); };
+  auto empty = [&](int s) { return bar0 + 8u * (2 + C::SLOTS + s); };
+  const uint32_t bar1 = bar0 + 8u * (2 + 2 * C::SLOTS);
+  const uint32_t s_full = bar1, s_free = bar1 + 8, p_half = bar1 + 16, p_full = bar1 + 24, pv_done = bar1 + 32;   // p_half: P of 64 keys
+  auto next_full = [&](int i) { return bar1 + 40u + 8u * i; };
+  auto next_empty = [&](int i) { return bar1 + 56u + 8u * i; };
+  const uint32_t next_slot = (bar0 + 8u * C::NBAR + 15u) & ~15u;
 
-  // 1-D grid: movers first (they must be resident before anything waits for data), then the
-  // (batch, head, query tile) CTAs.  Causal tiles differ in length by up to the number of key blocks, so
-  // the longest tiles of all heads of a group start first and the short ones fill the tail; a group is as
-  // many heads as keep their K / V in L2 together (launch_fa_fwd).
-  const int cid = (int)blockIdx.x - push.n_mov;
-  const int grp = cid / (p.tiles_x * p.group);
-  const int in_grp = cid - grp * p.tiles_x * p.group;
-  const int gsize = min(p.group, p.hq * p.B - grp * p.group);
-  const int mblk = p.tiles_x - 1 - in_grp / gsize;
-  const int bh = grp * p.group + in_grp % gsize;
-  const int h = bh % p.hq, b = bh / p.hq;
-  const int hk = h / (p.hq / p.hkv);
-  const int m0 = mblk * 2 * C::BM;
+  // Grid: movers first (they must be resident before anything waits for data), then one entry per (batch, head, query tile).  Causal
+  // tiles differ in length by up to the number of key blocks, so the longest tiles of all heads of a group come first and
+  // the short ones fill the tail; a group is as many heads as keep their K / V in L2 together (launch_fa_fwd).  A resident CTA goes
+  // on with entries that have not been started yet (cluster launch control: it cancels their launch and takes their place): the
+  // loads and the first scores of a tile then run under the last softmax and the stores of the one before it, and no list is fixed in advance
+  // (lists of equal length gave SMs that were done 12 % later than the mean).
+  volatile int* abort_flag = s_abort;
   const int off = p.Sk - p.Sq;
-  const int kv_blocks = (p.Sk + C::BN - 1) / C::BN;
-  int nb[2];
-#pragma unroll
-  for (int t = 0; t < 2; t++) {
-    const int r0 = m0 + t * C::BM;
-    int n = kv_blocks;
-    if (p.causal) n = min(n, (r0 + C::BM - 1 + off) / C::BN + 1);
-    nb[t] = (r0 < p.Sq) ? n : 0;
-  }
-  const int nb_max = max(nb[0], nb[1]);
+  struct Tile { int m0, b, h, hk, nb; };
+  auto tile_of = [&](int cta) {
+    Tile t;
+    const int cid = cta - push.n_mov;
+    const int grp = p.by_grp.div(cid);
+    const int in_grp = cid - grp * (int)p.by_grp.d;
+    const FastDiv& heads = (grp + 1) * p.group <= p.hq * p.B ? p.by_group : p.by_last;
+    const int row = heads.div(in_grp);
+    const int bh = grp * p.group + in_grp - row * (int)heads.d;
+    t.m0 = (p.tiles_x - 1 - row) * C::BM;
+    t.b = p.by_hq.div(bh);
+    t.h = bh - t.b * p.hq;
+    t.hk = p.by_rep.div(t.h);
+    t.nb = (p.Sk + C::BN - 1) / C::BN;
+    if (p.causal) t.nb = min(t.nb, (t.m0 + C::BM - 1 + off) / C::BN + 1);
+    return t;
+  };
+  // Entry n + 1 of this CTA: the answer to request n, or -1 at the end.
+  auto next_cta = [&](int n) -> int {
+    if (!p.steal || !mbar_wait(next_full(n & 1), (uint32_t)(n >> 1) & 1u, abort_flag)) return -1;
+    const int cta = cancel_result(next_slot + 16u * (n & 1));
+    fence_proxy_async_smem();
+    return cta;
+  };
 
   if (threadIdx.x == 0) {
     s_abort[0] = 0;
     s_abort[1] = p.kv_flags ? wait_extra_ms(p.wait_ns) : 0;
     mbar_init(q_full, 1);
-    for (int s = 0; s < C::KS; s++) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 2); }
-    for (int s = 0; s < C::VS; s++) { mbar_init(v_full(s), 1); mbar_init(v_empty(s), 2); }
-    for (int t = 0; t < 2; t++) { mbar_init(s_full(t), 1); mbar_init(p_full(t), 128); mbar_init(pv_done(t), 1); mbar_init(s_free(t), 128); mbar_init(p_half(t), 128); }
+    mbar_init(q_empty, 1);
+    for (int s = 0; s < C::SLOTS; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+    mbar_init(s_full, 1);
+    mbar_init(pv_done, 1);
+    mbar_init(s_free, 4);
+    mbar_init(p_half, 4);
+    mbar_init(p_full, 4);
+    for (int i = 0; i < 2; i++) { mbar_init(next_full(i), 1); mbar_init(next_empty(i), 5); }   // the issuer and four softmax warps read
     mbar_init_fence();
-    prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv);
+    prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&to);
   }
-  if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
+  if (warp == 1) tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
   fence_before();
   __syncthreads();
   fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  volatile int* abort_flag = s_abort;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
-  if (warp == 0) {
-    // ------------------------------- TMA producer -------------------------------
-    if (lane == 0 && nb_max > 0) {
-      mbar_expect_tx(q_full, 2 * C::TILE_BYTES);
+  if (warp < 4) {
+    reg_dec<FA_REGS_ISSUE>();
+    if (warp == 0) {
+      // ------------------------------- TMA producer -------------------------------
+      if (elect_one()) {
+        bool ok = true;
+        int slot = 0;
+        uint32_t phase = 0;
+        int asked = 0;
+        for (int n = 0, cta = (int)blockIdx.x; ok && cta >= 0; n++) {
+          if (p.steal) {
+            if (!mbar_wait(next_empty(n & 1), ((uint32_t)(n >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+            mbar_expect_tx(next_full(n & 1), 16);
+            cancel_next(next_slot + 16u * (n & 1), next_full(n & 1));
+            asked = n + 1;
+          }
+          const Tile t = tile_of(cta);
+          if (!mbar_wait(q_empty, (uint32_t)(n & 1) ^ 1u, abort_flag)) { ok = false; break; }
+          mbar_expect_tx(q_full, C::ATOMS * C::SLOT_BYTES);
 #pragma unroll
-      for (int t = 0; t < 2; t++)
+          for (int a = 0; a < C::ATOMS; a++)
+            tma_load_2d(sbase + C::OFF_Q + a * C::SLOT_BYTES, &tq, t.h * D + a * 64, t.b * p.Sq + t.m0, q_full);
+          for (int j = 0; j < t.nb && ok; j++) {
+            if (p.kv_flags) {
+              // this 128-key block is pushed by its owner: wait for its counter, then order the
+              // peer's generic-proxy writes before the TMA (async proxy) reads
+              if (!lbcomm::flag_wait_ge(p.kv_flags + (long long)t.b * (p.kv_brows >> 7) + j, p.flag_target, p.wait_ns)) { *abort_flag = 1; ok = false; break; }
+              asm volatile("fence.proxy.async;" ::: "memory");
+            }
+            const int row = t.b * p.kv_brows + j * C::BN;
 #pragma unroll
-        for (int a = 0; a < C::ATOMS; a++)
-          tma_load_2d(sbase + C::OFF_Q + t * C::TILE_BYTES + a * C::ATOM_BYTES, &tq, h * D + a * 64,
-                      b * p.Sq + m0 + t * C::BM, q_full);
-      bool ok = true;
-      for (int j = 0; j < nb_max && ok; j++) {
-        const int ks = j % C::KS, vs = j % C::VS;
-        if (!mbar_wait(k_empty(ks), (((uint32_t)(j / C::KS)) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-        if (p.kv_flags) {
-          // this 128-key block is pushed by its owner: wait for its counter, then order the
-          // peer's generic-proxy writes before the TMA (async proxy) reads
-          if (!lbcomm::flag_wait_ge(p.kv_flags + (long long)b * (p.kv_brows >> 7) + j, p.flag_target, p.wait_ns)) { *abort_flag = 1; ok = false; break; }
-          asm volatile("fence.proxy.async;" ::: "memory");
+            for (int u = 0; u < C::UNITS; u++) {
+              if (ok && !mbar_wait(empty(slot), phase ^ 1u, abort_flag)) ok = false;
+              if (!ok) break;
+              const uint32_t dst = sbase + C::OFF_RING + slot * C::SLOT_BYTES, bar = full(slot);
+              mbar_expect_tx(bar, C::SLOT_BYTES);
+              if (u < C::ATOMS) {
+                tma_load_2d(dst, &tk, t.hk * D + u * 64, row, bar);               // box 128 keys x 64 columns
+              } else {
+                const int half = u - C::ATOMS;                                    // head_dim 128: keys 0-63, then 64-127
+#pragma unroll
+                for (int a = 0; a < 2; a++)                                       // boxes 64 keys x 64 columns
+                  tma_load_2d(dst + a * 8192, &tv, t.hk * D + (D == 128 ? a * 64 : 0), row + (D == 128 ? half * 64 : a * 64), bar);
+              }
+              if (++slot == C::SLOTS) { slot = 0; phase ^= 1u; }
+            }
+          }
+          if (ok) cta = next_cta(n);
         }
-        mbar_expect_tx(k_full(ks), C::TILE_BYTES);
-#pragma unroll
-        for (int a = 0; a < C::ATOMS; a++)
-          tma_load_2d(sbase + C::OFF_K + ks * C::TILE_BYTES + a * C::ATOM_BYTES, &tk, hk * D + a * 64,
-                      b * p.kv_brows + j * C::BN, k_full(ks));
-        if (!mbar_wait(v_empty(vs), (((uint32_t)(j / C::VS)) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-        mbar_expect_tx(v_full(vs), C::TILE_BYTES);
-#pragma unroll
-        for (int a = 0; a < C::ATOMS; a++)
-          tma_load_2d(sbase + C::OFF_V + vs * C::TILE_BYTES + a * C::ATOM_BYTES, &tv, hk * D + a * 64,
-                      b * p.kv_brows + j * C::BN, v_full(vs));
+        if (!ok) {
+          atomicExch(&g_fa_status[0], 1u);
+          if (asked) mbar_wait(next_full((asked - 1) & 1), (uint32_t)((asked - 1) >> 1) & 1u, abort_flag);   // nothing arrives after the CTA's end
+        }
       }
-      if (!ok) atomicExch(&g_fa_status[0], 1u);
+    } else if (warp == 1) {
+      // ------------------------------- MMA issuer -------------------------------
+      // Blocking waits in a fixed order.  Per tile S(0); then per key block, head_dim 64: S(j+1) as soon as the softmax threads hold S(j) in
+      // registers, and P(j) V in two halves as P(j) arrives; head_dim 128: P(j) V, then S(j+1) into the columns that P(j) leaves.
+      if (elect_one()) {
+        const uint32_t idesc_s = make_idesc(C::BM, C::BN, 0, 0);
+        const uint32_t idesc_o = make_idesc(C::BM, D, 0, 1);
+        // descriptor bases; a slot / k-step only changes the 16-byte-granular start address
+        const uint64_t qa = make_desc(sbase + C::OFF_Q, 16, 1024);
+        const uint64_t dk0 = make_desc(sbase + C::OFF_RING, 16, 1024);
+        const uint64_t dv0 = make_desc(sbase + C::OFF_RING, 8192, 1024);
+        const uint32_t s_dst = tmem_base + C::COL_S;
+        const uint32_t o_dst = tmem_base + C::COL_O;
+        const uint32_t pa = tmem_base + C::COL_P;          // 8 columns per K = 16 slice
+        bool ok = true;
+        // slots are taken in load order: K (ATOMS slots), then V of every block; head_dim 64 takes K of the next block before V of the current
+        auto ring = [&](int& slot, uint32_t& phase, int step) { slot += step; if (slot >= C::SLOTS) { slot -= C::SLOTS; phase ^= 1u; } };
+        int ks = 0, vs = C::ATOMS;                      // next slot of K and of V, and their phases
+        uint32_t kp = 0, vp = 0;
+        uint32_t g = 0;                                 // key blocks so far, over all tiles: the phase of the per-block barriers
+        auto k_ready = [&]() -> bool {                  // the next block's K has arrived
+          if (!mbar_wait(full(ks), kp, abort_flag)) return false;
+          if (C::ATOMS == 1) return true;
+          const bool wrap = ks + 1 == C::SLOTS;
+          return mbar_wait(full(wrap ? 0 : ks + 1), wrap ? kp ^ 1u : kp, abort_flag);
+        };
+        auto issue_s = [&](bool last) {                 // S = Q K^T of the next block (K is there), then release its slots of K (and Q)
+          fence_after();
+#pragma unroll
+          for (int a = 0; a < C::ATOMS; a++) {
+            const uint64_t ka = dk0 + (uint64_t)((ks * C::SLOT_BYTES) >> 4);
+#pragma unroll
+            for (int s = 0; s < 4; s++)
+              umma_bf16(s_dst, qa + (uint64_t)((a * C::SLOT_BYTES + s * 32) >> 4), ka + (uint64_t)((s * 32) >> 4), idesc_s, (a | s) ? 1u : 0u);
+            if (a == C::ATOMS - 1) umma_commit(s_full);
+            umma_commit(empty(ks));
+            ring(ks, kp, a == C::ATOMS - 1 ? C::UNITS - C::ATOMS + 1 : 1);
+          }
+          if (last) umma_commit(q_empty);
+        };
+        // O += P V of block g, then release its slots of V.  What a step waits for is waited for ahead of the wait for P, which is
+        // the last to come: a wait takes some 150 cycles even where there is nothing to wait for.
+        auto issue_pv = [&](bool first, bool last) -> bool {
+#pragma unroll
+          for (int half = 0; half < 2; half++) {
+            if ((D == 128 || half == 0) && !mbar_wait(full(vs), vp, abort_flag)) return false;
+            if (half == 1 && C::P_ALIAS && !last && !k_ready()) return false;
+            if (!mbar_wait(half ? p_full : p_half, g & 1u, abort_flag)) return false;
+            fence_after();
+            const uint64_t va = dv0 + (uint64_t)((vs * C::SLOT_BYTES + (D == 128 ? 0 : half * 8192)) >> 4);
+#pragma unroll
+            for (int s = 0; s < 4; s++)
+              umma_bf16_ta(o_dst, pa + 8u * (half * 4 + s), va + (uint64_t)((s * 2048) >> 4), idesc_o, (half | s) ? 1u : (first ? 0u : 1u));
+            if (half && (!C::P_ALIAS || last)) umma_commit(pv_done);
+            if (D == 128 || half) {
+              umma_commit(empty(vs));
+              ring(vs, vp, half ? C::ATOMS + 1 : 1);
+            }
+          }
+          return true;
+        };
+        for (int n = 0, cta = (int)blockIdx.x; ok && cta >= 0; n++) {
+          const Tile t = tile_of(cta);
+          ok = k_ready() && mbar_wait(q_full, (uint32_t)n & 1u, abort_flag);
+          if (ok && !C::P_ALIAS && n > 0) ok = mbar_wait(s_free, (g - 1) & 1u, abort_flag);
+          if (ok) issue_s(t.nb == 1);
+          for (int j = 0; j < t.nb && ok; j++, g++) {
+            const bool last = j + 1 == t.nb;
+            if (!C::P_ALIAS && !last) {
+              ok = k_ready() && mbar_wait(s_free, g & 1u, abort_flag);
+              if (ok) issue_s(j + 2 == t.nb);
+            }
+            if (ok) ok = issue_pv(j == 0, last);
+            if (C::P_ALIAS && ok && !last) issue_s(j + 2 == t.nb);
+          }
+          if (!ok) break;
+          cta = next_cta(n);
+          if (cta >= 0) mbar_arrive(next_empty(n & 1));
+        }
+        if (!ok) atomicExch(&g_fa_status[0], 2u);
+      }
     }
-  } else if (warp == 1 || warp == 2) {
-    // ------------------------------- MMA issuers -------------------------------
-    // One issuing thread per query tile (a single thread feeding both tiles was measured to bound the
-    // kernel: a tcgen05.mma blocks its issuer for about its own execution time).  Each thread follows
-    // the fixed order of its own tile with blocking waits: S(0); then per key block, head_dim 64: S(j+1)
-    // as soon as the softmax threads hold S(j) in registers, and P(j) V in two halves as P(j) arrives;
-    // head_dim 128: P(j) V, then S(j+1) into the columns that P(j) leaves.
-    // A K / V stage is free once BOTH tiles have used it, so each thread arrives on the stage's
-    // empty barrier for every block, also for blocks its own tile does not need.
-    const int t = warp - 1;
-    if (lane == 0 && nb_max > 0) {
-      const uint32_t idesc_s = make_idesc(C::BM, C::BN, 0, 0);
-      const uint32_t idesc_o = make_idesc(C::BM, D, 0, 1);
-      // descriptor bases; a stage / k-step only changes the 16-byte-granular start address
-      const uint64_t qa = make_desc(sbase + C::OFF_Q + t * C::TILE_BYTES, 16, 1024);
-      const uint64_t dk0 = make_desc(sbase + C::OFF_K, 16, 1024);
-      const uint64_t dv0 = make_desc(sbase + C::OFF_V, C::ATOM_BYTES, 1024);
-      const uint32_t s_dst = tmem_base + C::COL_S + t * C::BN;
-      const uint32_t o_dst = tmem_base + C::COL_O + t * D;
-      const uint32_t pa = tmem_base + C::COL_P + t * C::P_STRIDE;          // 8 columns per K = 16 slice
-      const int n_my = nb[t];
-      bool ok = mbar_wait(q_full, 0, abort_flag);
-      auto issue_s = [&](int j) -> bool {             // S(j) = Q K(j)^T, then release K(j)'s stage
-        const int ks = j % C::KS;
-        if (!mbar_wait(k_full(ks), ((uint32_t)(j / C::KS)) & 1u, abort_flag)) return false;
-        fence_after();
-        const uint64_t ka = dk0 + (uint64_t)((ks * C::TILE_BYTES) >> 4);
-#pragma unroll
-        for (int s = 0; s < D / 16; s++) {
-          const uint64_t o = (uint64_t)(((s >> 2) * C::ATOM_BYTES + (s & 3) * 32) >> 4);
-          umma_bf16(s_dst, qa + o, ka + o, idesc_s, s ? 1u : 0u);
-        }
-        umma_commit(s_full(t));
-        umma_commit(k_empty(ks));
-        return true;
-      };
-      auto issue_pv = [&](int j) -> bool {            // O += P(j) V(j), then release V(j)'s stage
-        const int vs = j % C::VS;
-        if (!mbar_wait(v_full(vs), ((uint32_t)(j / C::VS)) & 1u, abort_flag)) return false;
-        if (!mbar_wait(p_half(t), (uint32_t)j & 1u, abort_flag)) return false;
-        fence_after();
-        const uint64_t va = dv0 + (uint64_t)((vs * C::TILE_BYTES) >> 4);
-        umma_bf16_ta(o_dst, pa, va, idesc_o, j ? 1u : 0u);
-#pragma unroll
-        for (int s = 1; s < C::BN / 32; s++)
-          umma_bf16_ta(o_dst, pa + 8u * s, va + (uint64_t)((s * 2048) >> 4), idesc_o, 1u);
-        if (!mbar_wait(p_full(t), (uint32_t)j & 1u, abort_flag)) return false;
-        fence_after();
-#pragma unroll
-        for (int s = C::BN / 32; s < C::BN / 16; s++)
-          umma_bf16_ta(o_dst, pa + 8u * s, va + (uint64_t)((s * 2048) >> 4), idesc_o, 1u);
-        if (!C::P_ALIAS || j == n_my - 1) umma_commit(pv_done(t));
-        umma_commit(v_empty(vs));
-        return true;
-      };
-      // stagger: tile 1 starts once tile 0 holds its first S in registers (two tiles marching in
-      // step were measured to spend 2300 cycles per block together in the exponentials and then
-      // idle together; half a period apart each has the MUFU unit to itself)
-      if (ok && t == 1 && nb[0] > 0 && n_my > 0) ok = mbar_wait(s_free(0), 0u, abort_flag);
-      if (ok && n_my > 0) ok = issue_s(0);
-      for (int j = 0; j < n_my && ok; j++) {
-        if (!C::P_ALIAS && j + 1 < n_my) {
-          ok = mbar_wait(s_free(t), (uint32_t)j & 1u, abort_flag);
-          if (ok) ok = issue_s(j + 1);
-        }
-        if (ok) ok = issue_pv(j);
-        if (C::P_ALIAS && ok && j + 1 < n_my) ok = issue_s(j + 1);
-      }
-      // blocks that only the other tile needs: keep the stage rings in step
-      for (int j = n_my; j < nb_max && ok; j++) {
-        ok = mbar_wait(k_full(j % C::KS), ((uint32_t)(j / C::KS)) & 1u, abort_flag);
-        if (ok) mbar_arrive(k_empty(j % C::KS));
-        if (ok) ok = mbar_wait(v_full(j % C::VS), ((uint32_t)(j / C::VS)) & 1u, abort_flag);
-        if (ok) mbar_arrive(v_empty(j % C::VS));
-      }
-      if (!ok) atomicExch(&g_fa_status[0], 2u);
-    }
-  } else if (warp >= 4) {
+  } else {
     // ------------------------------- softmax warps -------------------------------
-    const int t = (warp - 4) >> 2;
+    reg_inc<FA_REGS_SOFTMAX>();
     const int quad = warp & 3;
-    const int rit = quad * 32 + lane;              // row inside the tile
-    const int row = m0 + t * C::BM + rit;          // query index inside the sequence
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const uint32_t ts_addr = lane_addr + C::COL_S + t * C::BN;
-    const uint32_t to_addr = lane_addr + C::COL_O + t * D;
-    const uint32_t tp_addr = lane_addr + C::COL_P + t * C::P_STRIDE;
+    const uint32_t ts_addr = lane_addr + C::COL_S;
+    const uint32_t to_addr = lane_addr + C::COL_O;
+    const uint32_t tp_addr = lane_addr + C::COL_P;
     const float sl2 = p.scale * 1.4426950408889634f;
     const f32x2 sl2x2 = pack2(sl2, sl2);
-    float m_i = -INFINITY, l_i = 0.f;
     bool ok = true;
-    const int n_my = nb[t];
-#ifdef LB_FA_PROFILE
-    unsigned long long prof[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#endif
-    for (int j = 0; j < n_my; j++) {
-      FA_T(0);
-      if (!mbar_wait(s_full(t), (uint32_t)j & 1u, abort_flag)) { ok = false; break; }
-      fence_after();
-      FA_T(1);
-      uint32_t r[128];
-      const int c0 = j * C::BN;
-      const int warp_row0 = m0 + t * C::BM + quad * 32;
-      const bool need_mask = (c0 + C::BN > p.Sk) || (p.causal && (c0 + C::BN - 1 > warp_row0 + off));
-      const int lim = (p.causal ? min(p.Sk - 1, row + off) : p.Sk - 1) - c0;   // last visible column of this block
-      // the row arrives in two halves so that the maximum of the first overlaps the second load;
-      // four independent chains keep the 128 comparisons from serialising on their latency
-      float mx4[4] = {m_i, m_i, m_i, m_i};
-      tmem_ld32(ts_addr, r);
-      tmem_ld32(ts_addr + 32, r + 32);
-      tmem_ld_wait();
-      tmem_ld32(ts_addr + 64, r + 64);
-      tmem_ld32(ts_addr + 96, r + 96);
+    auto arrive = [&](uint32_t bar) {              // once per warp
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    uint32_t g = 0;                                // key blocks so far, over all tiles
+    bool s_ready = false;                          // S of the next block was seen complete
+    for (int n = 0, cta = (int)blockIdx.x; ok && cta >= 0; n++) {
+      const Tile t = tile_of(cta);
+      const int m0 = t.m0, nb = t.nb;
+      const int row = m0 + quad * 32 + lane;         // query index inside the sequence
+      float m_i = -INFINITY, m_s = 0.f, l_i = 0.f;
+      for (int j = 0; j < nb; j++, g++) {
+        if (!s_ready && !mbar_wait(s_full, g & 1u, abort_flag)) { ok = false; break; }
+        fence_after();
+        uint32_t r[128];
+        const int c0 = j * C::BN;
+        const int warp_row0 = m0 + quad * 32;
+        const bool need_mask = (c0 + C::BN > p.Sk) || (p.causal && (c0 + C::BN - 1 > warp_row0 + off));
+        const int lim = (p.causal ? min(p.Sk - 1, row + off) : p.Sk - 1) - c0;   // last visible column of this block
+        auto mask = [&](int i0) {
+          if (need_mask) {
 #pragma unroll
-      for (int half = 0; half < 2; half++) {
-        if (half == 1) {
-          tmem_ld_wait();
-          fence_before();
-          if (!C::P_ALIAS || j == 0) mbar_arrive(s_free(t));   // S_t may be overwritten by the next key block
-        }
-        if (need_mask) {
+            for (int i = i0; i < i0 + 64; i++)
+              if (i > lim) r[i] = 0xff800000u;           // -inf
+          }
+        };
+        // exponentials of 64 columns, packed as bf16 pairs (column c of P holds keys 2c, 2c+1)
+        auto exps = [&](int i0, uint32_t* pr, f32x2* rs2) {
+          const f32x2 nms2 = pack2(-m_s, -m_s);
+          rs2[0] = rs2[1] = pack2(0.f, 0.f);
 #pragma unroll
-          for (int i = half * 64; i < half * 64 + 64; i++)
-            if (i > lim) r[i] = 0xff800000u;           // -inf
-        }
+          for (int c = 0; c < 32; c++) {
+            const int i = i0 + c * 2;
+            float e0, e1;
+            unpack2(fma2(pack2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), sl2x2, nms2), e0, e1);
+            e0 = exp2f(e0);
+            e1 = exp2f(e1);
+            rs2[c & 1] = add2(rs2[c & 1], pack2(e0, e1));
+            bf162 pk = __floats2bfloat162_rn(e0, e1);
+            pr[c] = *reinterpret_cast<uint32_t*>(&pk);
+          }
+        };
+        auto row_max = [&]() {                           // four independent chains
+          float mx4[4] = {m_i, m_i, m_i, m_i};
 #pragma unroll
-        for (int i = half * 64; i < half * 64 + 64; i += 2)
-          mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
-      }
-      FA_T(2);
-      // Lazy reference maximum: keep the old one unless the new maximum is more than 2^8 above
-      // it, so that O and l rarely need rescaling (values stay below 2^8 relative to it).
-      float m_new = max2(max2(mx4[0], mx4[1]), max2(mx4[2], mx4[3]));
-      if (m_i != -INFINITY && (m_new - m_i) * sl2 <= 8.f) m_new = m_i;
-      // (a row with a score of +inf has no softmax: NaN, as inf - inf gives)
-      const float m_s = (m_new == -INFINITY) ? 0.f : (m_new == INFINITY ? __int_as_float(0x7fffffff) : m_new * sl2);
-      const float corr = (m_i == -INFINITY) ? 0.f : exp2f(m_i * sl2 - m_s);
-      FA_T(3);
-      // exponentials; P goes back to TMEM as packed bf16 pairs (column c holds keys 2c, 2c+1), 32
-      // columns per store so that the first store is in flight while the second half is computed.
-      // The first half is computed BEFORE waiting for the previous P V (which still reads the P
-      // columns and owns O): its 64 exponentials overlap the tail of that MMA.
-      const f32x2 nms2 = pack2(-m_s, -m_s);
-      f32x2 rs2[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
-#pragma unroll
-      for (int hh = 0; hh < 2; hh++) {
+          for (int i = 0; i < 128; i += 2) mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+          return max2(max2(mx4[0], mx4[1]), max2(mx4[2], mx4[3]));
+        };
+        tmem_ld32(ts_addr, r);
+        tmem_ld32(ts_addr + 32, r + 32);
+        tmem_ld32(ts_addr + 64, r + 64);
+        tmem_ld32(ts_addr + 96, r + 96);
+        tmem_ld_wait();
+        if (!C::P_ALIAS) arrive(s_free);                 // S may be overwritten by the next key block
+        mask(0);
+        mask(64);
+        // Lazy reference maximum: the old one stays unless the new maximum is more than 2^8 above it, so that O and l rarely
+        // need rescaling (values stay below 2^8 relative to it).  So the first 64 exponentials are computed with the old one, while the
+        // maximum that tells whether it may stay is still being found, and once more in the rare block where it may not.
         uint32_t pr[32];
-#pragma unroll
-        for (int c = 0; c < 32; c++) {
-          const int i = hh * 64 + c * 2;
-          const f32x2 x2 = fma2(pack2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), sl2x2, nms2);
-          float e0, e1;
-          unpack2(x2, e0, e1);
-          e0 = exp2f(e0);
-          e1 = exp2f(e1);
-          rs2[c & 1] = add2(rs2[c & 1], pack2(e0, e1));
-          bf162 pk = __floats2bfloat162_rn(e0, e1);
-          pr[c] = *reinterpret_cast<uint32_t*>(&pk);
+        f32x2 rs2[2], rt2[2];
+        const bool pv_ready = !C::P_ALIAS && j > 0 && mbar_test_wait(pv_done, (g - 1) & 1u);   // asked ahead of its use
+        if (j > 0) exps(0, pr, rs2);
+        float m_new = row_max();
+        const bool grow = !(m_i != -INFINITY && (m_new - m_i) * sl2 <= 8.f);
+        const bool any_grow = __any_sync(0xffffffffu, grow);
+        float corr = 1.f;
+        if (any_grow) {
+          if (!grow) m_new = m_i;
+          // (a row with a score of +inf has no softmax: NaN, as inf - inf gives)
+          m_s = (m_new == -INFINITY) ? 0.f : (m_new == INFINITY ? __int_as_float(0x7fffffff) : m_new * sl2);
+          corr = (m_i == -INFINITY) ? 0.f : exp2f(m_i * sl2 - m_s);
+          l_i *= corr;
+          m_i = m_new;
+          exps(0, pr, rs2);
         }
-        if (hh == 0 && j > 0) {
+        if (j > 0) {
           // previous P V finished: O is stable and the P columns may be overwritten.  (head_dim 128: S(j) was
           // issued behind it by the same thread, so its completion says that P V has completed too.)
           if (!C::P_ALIAS) {
-            if (!mbar_wait(pv_done(t), (uint32_t)(j - 1) & 1u, abort_flag)) { ok = false; }
+            if (!pv_ready && !mbar_wait(pv_done, (g - 1) & 1u, abort_flag)) { ok = false; break; }
             fence_after();
           }
-          if (ok && __any_sync(0xffffffffu, !(m_new == m_i))) {
+          if (any_grow) {
 #pragma unroll 1
             for (int c = 0; c < D / 32; c++) {
               uint32_t o[32];
@@ -438,51 +486,60 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
             tmem_st_wait();
           }
         }
-        tmem_st32(tp_addr + hh * 32, pr);
+        // P goes back to TMEM, the first half in flight while the second is computed
+        tmem_st32(tp_addr, pr);
         tmem_st_wait();
-        fence_before();
-        mbar_arrive(hh == 0 ? p_half(t) : p_full(t));
+        arrive(p_half);
+        s_ready = !C::P_ALIAS && j + 1 < nb && mbar_test_wait(s_full, (g + 1) & 1u);
+        exps(64, pr, rt2);
+        tmem_st32(tp_addr + 32, pr);
+        tmem_st_wait();
+        arrive(p_full);
+        rs2[0] = add2(rs2[0], rt2[0]);
+        rs2[1] = add2(rs2[1], rt2[1]);
+        float rs[4];
+        unpack2(rs2[0], rs[0], rs[1]);
+        unpack2(rs2[1], rs[2], rs[3]);
+        l_i += (rs[0] + rs[1]) + (rs[2] + rs[3]);
       }
+      if (ok) {
+        cta = next_cta(n);
+        __syncwarp();
+        if (lane == 0 && cta >= 0) mbar_arrive(next_empty(n & 1));
+      }
+      if (ok && !mbar_wait(pv_done, C::P_ALIAS ? (uint32_t)n & 1u : (g - 1) & 1u, abort_flag)) ok = false;
       if (!ok) break;
-      float rs[4];
-      unpack2(rs2[0], rs[0], rs[1]);
-      unpack2(rs2[1], rs[2], rs[3]);
-      l_i = l_i * corr + ((rs[0] + rs[1]) + (rs[2] + rs[3]));
-      m_i = m_new;
-      FA_T(4);
-      FA_T(5);
-      FA_ACC(0, 0, 1); FA_ACC(1, 1, 2); FA_ACC(2, 2, 3); FA_ACC(3, 3, 4); FA_ACC(4, 4, 5);
-#ifdef LB_FA_PROFILE
-      prof[5] += 1;
-#endif
-    }
-#ifdef LB_FA_PROFILE
-    if (lane == 0)
-      for (int i = 0; i < 8; i++) atomicAdd(&g_fa_prof[i], prof[i]);
-#endif
-    if (ok && n_my > 0) {
-      if (!mbar_wait(pv_done(t), C::P_ALIAS ? 0u : (uint32_t)(n_my - 1) & 1u, abort_flag)) ok = false;
-    }
-    if (ok && n_my > 0) {
       fence_after();
       const float inv = l_i > 0.f ? 1.f / l_i : 0.f;
-      bf16* orow = p.o + ((long long)b * p.Sq + row) * p.o_ts + (long long)h * D;
-#pragma unroll 1
-      for (int c = 0; c < D / 32; c++) {
-        uint32_t r[32];
-        tmem_ld32(to_addr + c * 32, r);
+      // 64 columns at a time through shared memory: a row per lane stored straight to memory is 32 separate lines for every 16 bytes
+      // per lane, which kept the load/store unit busy for as long as one and a half key blocks take
+      uint8_t* out = smem + C::OFF_OUT + quad * 4096;
+#pragma unroll
+      for (int c = 0; c < D / 64; c++) {
+        uint32_t r[64];
+        tmem_ld32(to_addr + c * 64, r);
+        tmem_ld32(to_addr + c * 64 + 32, r + 32);
         tmem_ld_wait();
-        if (row < p.Sq) {
-          float f[32];
+        if (lane == 0) bulk_wait_read_but<0>();
+        __syncwarp();
 #pragma unroll
-          for (int i = 0; i < 32; i++) f[i] = __uint_as_float(r[i]) * inv;
+        for (int g8 = 0; g8 < 8; g8++) {
+          float f[8];
 #pragma unroll
-          for (int g = 0; g < 4; g++) *reinterpret_cast<uint4*>(orow + c * 32 + g * 8) = pack8(f + g * 8);
+          for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[g8 * 8 + i]) * inv;
+          *reinterpret_cast<uint4*>(out + sw128_off(lane, g8)) = pack8(f);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && m0 + quad * 32 < p.Sq) {
+          tma_store_3d(&to, smem_u32(out), t.h * D + c * 64, m0 + quad * 32, t.b);
+          bulk_commit();
         }
       }
       if (row < p.Sq)
-        p.lse[((long long)b * p.hq + h) * p.Sq + row] = (l_i > 0.f) ? m_i * p.scale + logf(l_i) : -INFINITY;
+        p.lse[((long long)t.b * p.hq + t.h) * p.Sq + row] = (l_i > 0.f) ? m_i * p.scale + logf(l_i) : -INFINITY;
     }
+    if (lane == 0) bulk_wait_read_but<0>();        // nothing reads shared memory after the CTA's end
     if (!ok && lane == 0) atomicExch(&g_fa_status[0], 3u);
   }
 
@@ -490,7 +547,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   __syncthreads();
   if (warp == 1) {
     fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, C::TMEM_COLS);
   }
 }
 
@@ -498,18 +555,22 @@ template <int D>
 int launch_fa_fwd(const void* q, const void* k, const void* v, FaFwdParams p, const FaPush& push, long long q_ts,
                   long long k_ts, long long v_ts, cudaStream_t s) {
   using C = FaCfg<D>;
-  CUtensorMap tq, tk, tv;
+  CUtensorMap tq, tk, tv, to;
   int rc;
   const uint64_t kv_rows = (uint64_t)(p.B - 1) * p.kv_brows + p.Sk;
   if ((rc = make_map_bf16(&tq, q, (uint64_t)p.hq * D, (uint64_t)p.B * p.Sq, (uint64_t)q_ts, 64, 128))) return rc;
   if ((rc = make_map_bf16(&tk, k, (uint64_t)p.hkv * D, kv_rows, (uint64_t)k_ts, 64, 128))) return rc;
-  if ((rc = make_map_bf16(&tv, v, (uint64_t)p.hkv * D, kv_rows, (uint64_t)v_ts, 64, 128))) return rc;
+  if ((rc = make_map_bf16(&tv, v, (uint64_t)p.hkv * D, kv_rows, (uint64_t)v_ts, 64, 64))) return rc;
+  if ((rc = make_map_bf16_3d(&to, p.o, (uint64_t)p.hq * D, (uint64_t)p.Sq, (uint64_t)p.B, (uint64_t)p.o_ts, 64, 32))) return rc;
   static bool attr = false;
   if (!attr) {
+    // the register split must fit in what the launch allocates, or it would wait for registers that nobody gives back
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, fa_fwd_tc_kernel<D>) != cudaSuccess || (fa.numRegs + 7) / 8 * 8 * 2 < FA_REGS_ISSUE + FA_REGS_SOFTMAX) return LB_ERR_LAUNCH;
     cudaFuncSetAttribute(fa_fwd_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
     attr = true;
   }
-  p.tiles_x = (p.Sq + 255) / 256;
+  p.tiles_x = (p.Sq + 127) / 128;
   // heads ordered together: as many as have their K / V in 48 MB (of 126 MB of L2), whole GQA groups
   const long long kv_bytes = 4LL * D * p.Sk;
   const long long kv_heads = kv_bytes >= (48LL << 20) ? 1 : (48LL << 20) / kv_bytes;
@@ -517,7 +578,13 @@ int launch_fa_fwd(const void* q, const void* k, const void* v, FaFwdParams p, co
   p.wait_ns = g_lb_flag_wait_ns;
   const long long grid = (long long)push.n_mov + (long long)p.tiles_x * p.hq * p.B;
   if (grid > 2147483647LL) return LB_ERR_SHAPE;
-  fa_fwd_tc_kernel<D><<<(unsigned)grid, FA_FWD_THREADS, C::SMEM, s>>>(tq, tk, tv, p, push);
+  p.by_grp.set((unsigned)(p.tiles_x * p.group));
+  p.by_group.set((unsigned)p.group);
+  p.by_last.set((unsigned)(p.hq * p.B % p.group ? p.hq * p.B % p.group : p.group));
+  p.by_hq.set((unsigned)p.hq);
+  p.by_rep.set((unsigned)(p.hq / p.hkv));
+  p.steal = push.n_mov == 0;       // (a mover's place is not to be taken)
+  fa_fwd_tc_kernel<D><<<(unsigned)grid, FA_FWD_THREADS, C::SMEM, s>>>(tq, tk, tv, to, p, push);
   LB_CHECK_LAUNCH();
   return LB_OK;
 }
@@ -533,14 +600,6 @@ extern "C" int lb_flash_status(void* out) {
   return LB_OK;
 }
 
-#ifdef LB_FA_PROFILE
-extern "C" int lb_flash_prof(void* out) {
-  cudaMemcpyFromSymbol(out, g_fa_prof, sizeof(unsigned long long) * 16);
-  unsigned long long zeros[16] = {0};
-  cudaMemcpyToSymbol(g_fa_prof, zeros, sizeof(zeros));
-  return LB_OK;
-}
-#endif
 
 // Same contract as lb_flash_fwd (flash_attn.cu); head_dim 64 or 128, all pointers 16-byte
 // aligned, token strides multiples of 8, causal needs Sk >= Sq.  Returns LB_ERR_SHAPE otherwise.

@@ -84,6 +84,13 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
+// Tile of shared memory -> global memory; elements outside the tensor are not written.  Written by the async proxy: call
+// fence_proxy_async_smem() after filling the tile, bulk_commit() after the store, and bulk_wait_read_but<>() before reusing it.
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(map), "r"(x), "r"(y), "r"(z),
+               "r"(src)
+               : "memory");
+}
 // The same load issued by one CTA of a pair (cta_group::2): the tile goes to this CTA's shared memory, `bar` may be
 // the barrier of the pair's leader (leader_bar()).
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
@@ -239,7 +246,51 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
       "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// One thread of a converged warp, chosen by the hardware.  Where the issuing thread of MMAs and TMA loads is chosen this way (and not
+// as lane 0 of a divergent branch) the compiler keeps descriptors in uniform registers: 32 instead of 46 cycles per issued MMA.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
+// Cluster launch control: asks for a CTA of this grid that has not been started; the 16-byte answer goes to shared memory and is counted on
+// `bar`.  No further request after one that found none.  The answer is written by the async proxy: fence_proxy_async_smem()
+// between reading it and the next request into the same place.
+__device__ __forceinline__ void cancel_next(uint32_t dst, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(dst), "r"(bar)
+               : "memory");
+}
+// blockIdx.x of the CTA whose place may be taken, or -1.
+__device__ __forceinline__ int cancel_result(uint32_t src) {
+  int x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 a;\n\t"
+      "ld.shared.b128 a, [%1];\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, a;\n\t}"
+      : "=r"(x)
+      : "r"(src)
+      : "memory");
+  return x;
+}
+
+// Moves registers between the warpgroups of a CTA: executed by all warps of a warpgroup.  The shares must add up to no more than
+// the CTA was launched with.
+template <int N>
+__device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // Named barrier among `count` threads (a multiple of 32) of the CTA; ids 1..15 (0 is __syncthreads).
 __device__ __forceinline__ void named_bar_sync(int id, int count) {
@@ -311,11 +362,10 @@ inline EncodeTiledFn get_encode() {
   return fn;
 }
 
-// 2-D bf16 tensor map with 128-byte swizzle: `inner` contiguous elements, `outer` rows of `ld`
-// elements; box = box_inner x box_outer.  Binds the CUDA context to the calling thread first (the
+// bf16 tensor map of `rank` 2 or 3 with 128-byte swizzle.  Binds the CUDA context to the calling thread first (the
 // driver call needs one; autograd worker threads may not have touched the runtime yet).
-inline int make_map_bf16(CUtensorMap* m, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
-                         uint32_t box_inner, uint32_t box_outer) {
+inline int make_map_bf16_nd(CUtensorMap* m, const void* base, uint32_t rank, const cuuint64_t* dims, const cuuint64_t* strides,
+                            const cuuint32_t* box) {
   static thread_local bool ctx_bound = false;
   if (!ctx_bound) {
     cudaFree(0);
@@ -323,11 +373,8 @@ inline int make_map_bf16(CUtensorMap* m, const void* base, uint64_t inner, uint6
   }
   EncodeTiledFn enc = get_encode();
   if (!enc) return LB_ERR_DRIVER;
-  cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {ld * 2};
-  cuuint32_t box[2] = {box_inner, box_outer};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
@@ -335,6 +382,20 @@ inline int make_map_bf16(CUtensorMap* m, const void* base, uint64_t inner, uint6
     return LB_ERR_TMAP;
   }
   return LB_OK;
+}
+// `inner` contiguous elements, `outer` rows of `ld` elements; box = box_inner x box_outer.
+inline int make_map_bf16(CUtensorMap* m, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
+                         uint32_t box_inner, uint32_t box_outer) {
+  const cuuint64_t dims[2] = {inner, outer}, strides[1] = {ld * 2};
+  const cuuint32_t box[2] = {box_inner, box_outer};
+  return make_map_bf16_nd(m, base, 2, dims, strides, box);
+}
+// `batches` matrices of `rows` rows one behind the other: a tile that is stored ends with its own matrix.
+inline int make_map_bf16_3d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint64_t batches, uint64_t ld,
+                            uint32_t box_inner, uint32_t box_rows) {
+  const cuuint64_t dims[3] = {inner, rows, batches}, strides[2] = {ld * 2, rows * ld * 2};
+  const cuuint32_t box[3] = {box_inner, box_rows, 1};
+  return make_map_bf16_nd(m, base, 3, dims, strides, box);
 }
 
 }  // namespace bw

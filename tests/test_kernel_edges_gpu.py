@@ -60,6 +60,27 @@ def test_attention_tile_edges(B, Sq, Sk, hq, hkv, causal, scale, d):
             assert _rel(g, w) < 1e-2, name
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("B,S,hq,hkv", [
+    (2, 1100, 20, 4),        # 360 query tiles: more than two per SM, so that CTAs go on with a second one; 8 to 9 key blocks, ragged
+    (6, 130, 40, 8),         # 480 tiles of one and two key blocks, the second tile two rows long
+])
+def test_attention_tiles_taken_over(B, S, hq, hkv, d):
+    """Every tile is done once, and what lies behind the outputs' last rows is not written (tiles end inside them)."""
+    from lightron_b200.ops import functional as OF, native
+    q, k, v, do = _rand(B, S, hq, d, seed=1), _rand(B, S, hkv, d, seed=2), _rand(B, S, hkv, d, seed=3), _rand(B, S, hq, d, seed=4)
+    buf = [torch.full((B * S + 128, h, d), 7.0, dtype=torch.bfloat16, device="cuda") for h in (hq, hq, hkv, hkv)]
+    o, dq, dk, dv = (t[:B * S].view(B, S, -1, d) for t in buf)
+    lse = torch.empty(B, hq, S, dtype=torch.float32, device="cuda")
+    native.call("lb_flash_fwd_tc", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), B, S, S, hq, hkv, d,
+                q.stride(1), k.stride(1), v.stride(1), o.stride(1), d ** -0.5, 1, native.stream_ptr())
+    OF.flash_bwd_native(q, k, v, o, lse, do, True, d ** -0.5, dq, dk, dv)
+    _status_ok()
+    for name, g, w in zip(("o", "dq", "dk", "dv"), (o, dq, dk, dv), _attention64(q, k, v, do, True)):
+        assert _rel(g, w) < 1e-2, name
+    assert all(bool((t[B * S:] == 7.0).all()) for t in buf)
+
+
 def test_attention_forward_second_group_of_heads():
     """Longest tiles first within as many heads as have 48 MB of keys and values: 24 of these 32, the second group smaller."""
     from lightron_b200.ops import functional as OF

@@ -16,14 +16,17 @@
 // those of dP^T.  The tensor pipe runs MMAs in issue order, so a region is reused without a wait when both uses are MMAs:
 //     dV(i) | S(i+1) | dK(i) | dQ(i) | dP(i+1)      (head_dim 64: dP(i+1) before dQ(i))
 // The exponentials of block i+1 therefore run under dK / dQ of block i.  Each dQ tile is drained by four warps of
-// their own: TMEM -> registers -> staging -> asynchronous bulk reduce-add (cp.reduce.async.bulk .add.f32)
-// into an fp32 accumulator in global memory, whose layout is the staging layout (un-permuted by the final
-// convert kernel), so no atomic instructions pass through the load/store pipe.
-// No unit is full (counters at B4 S2048 32q/8kv d128 / B8 S2048 32q/4kv d64: tensor pipe 46 / 32 % of the active cycles, L1 and shared
-// memory 58 / 39 %, exponentials 20 / 28 %): what bounds it is the order of a block's phases, of which one CTA per SM holds one block, and
-// at d = 128 the dQ that waits for its drain in dP's columns, besides the power limit.  Loops of 0.35 s of all its kernels with the SM clock, the
-// earlier form / this one: B8 S2048 32q/4kv d64 934 (1965 MHz) / 658 us (1830 MHz), B1 S8192 32q/8kv d128 2650 (1965) / 1664 (1670),
-// B3 S1531 32q/8kv d128 438 (1965) / 244 (1705).
+// their own: TMEM -> registers (a whole row, so that the columns are free at once) -> staging -> asynchronous bulk reduce-add
+// (cp.reduce.async.bulk .add.f32) into an fp32 accumulator in global memory, whose layout is the staging layout (un-permuted by the final
+// convert kernel), so no atomic instructions pass through the load/store pipe (16-byte reductions straight from the registers held
+// up every other access of the SM: 5360 against 3750 cycles a block at d = 128).
+// What bounds it.  Cycles of a block: d = 64 2770, of which the math warps are never idle (exponentials 1330, dS 480, the rest waits, stores
+// and tensor-memory accesses); d = 128 3750, the chain dS -> dK, dQ -> drain -> dP of the next block, which shares dQ's columns, against 2560 of
+// tensor pipe.  Both run at the power limit in long loops (1.49 / 1.31 GHz).  What it took to get there from 3150 / 4500: an elected thread
+// that issues (elect_one), one arrival per warp, waits that are sure to succeed ahead of the one that is not, no divisions in the loops,
+// dQ's columns freed after 110 instead of 800 cycles, dK and dV through TMA stores (prologue and stores of a CTA: 12000 / 16000 cycles before).
+// Loops of 0.35 s of all its kernels, before / now, on one GPU: B8 S2048 32q/4kv d64 670 / 561 us, B1 S8192 32q/8kv d128
+// 1683 / 1480, B3 S1531 32q/8kv d128 248 / 232, B1 S4096 8q/8kv d128 119 / 107.
 // Warp roles (512 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4-11 math, 12-15 dQ drain.
 // All waits are bounded; on expiry a status word is set and the CTA drains and frees its TMEM.
 #include "tcgen05.cuh"
@@ -60,45 +63,56 @@ struct BwdCfg {
   static constexpr int ATOMS = D / 64;
   static constexpr int ATOM_BYTES = 128 * 128;
   static constexpr int TILE_BYTES = ATOMS * ATOM_BYTES;
-  static constexpr int STG_BYTES = 32 * 32 * 4;         // one 32 x 32 chunk of dQ; two per drain warp
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = OFF_K + TILE_BYTES;
   static constexpr int OFF_Q = OFF_V + TILE_BYTES;              // [QS]
   static constexpr int OFF_DO = OFF_Q + QS * TILE_BYTES;        // [DS]
   static constexpr int OFF_DS = OFF_DO + DS * TILE_BYTES;
+  static constexpr int STG_BYTES = 32 * 32 * 4;                 // one 32 x 32 chunk of dQ; two per drain warp
   static constexpr int OFF_STG = OFF_DS + 2 * ATOM_BYTES;
   static constexpr int OFF_ST = OFF_STG + 8 * STG_BYTES;        // [QS] row statistics of a query block
   static constexpr int OFF_BAR = OFF_ST + QS * 1024;
   static constexpr int SMEM = OFF_BAR + 256;
   static constexpr int NBAR = 1 + 2 * QS + 2 * DS + 6;
   static constexpr int NTHREADS = 512;
+  // Registers per thread: loads and MMAs / math / drain, which holds a whole row of dQ so that its columns are free at once
+  static constexpr int REGS_ISSUE = 96, REGS_MATH = (D == 64) ? 160 : 128, REGS_DRAIN = (D == 64) ? 96 : 160;
+  static_assert(REGS_ISSUE + 2 * REGS_MATH + REGS_DRAIN <= 4 * 128, "a CTA has 512 x 128 registers");
   // TMEM columns
   static constexpr int COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 256 + D;
   static constexpr int COL_DQ = DQ_ALIAS ? COL_DP : 384;
 };
 static_assert(BwdCfg<128>::SMEM <= 232448, "shared memory of a CTA");
 
-// fp32 dQ accumulator layout: tile (b, h, mblock) -> D / 32 column chunks -> 4 row quads -> 32 lanes -> 32 floats in
-// eight 16-byte pieces, piece c of lane l at c ^ (l & 7) (conflict-free shared-memory stores of the staging).
+// fp32 dQ accumulator layout: tile (b, h, mblock) -> 4 row quads -> D / 4 pieces of 4 columns -> 32 rows: the 16-byte stores of a
+// drain warp (a row per lane) are contiguous, and so are the 16-byte loads of a warp here.
 template <int D>
 __global__ void fa_dq_convert_kernel(const FaBwdParams p) {
-  constexpr int VPR = D / 8;
+  constexpr int CPR = D / 32;                                  // 32-column chunks per row: a thread takes one
   const int n_mblocks = (p.Sq + 127) / 128;
-  const long long total = (long long)p.B * p.Sq * p.hq * VPR;
+  const long long total = (long long)p.B * p.hq * n_mblocks * 128 * CPR;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
-    const int v = (int)(idx % VPR);
-    const long long th = idx / VPR;
-    const int h = (int)(th % p.hq);
-    const long long bi = th / p.hq;
-    const int b = (int)(bi / p.Sq), row = (int)(bi % p.Sq);
-    const int mblock = row >> 7, quad = (row & 127) >> 5, lane = row & 31;
-    const int chunk = v >> 2, c0 = (v & 3) * 2;
-    const float* at = p.dq_acc + (((long long)b * p.hq + h) * n_mblocks + mblock) * (128 * D) + (chunk * 4 + quad) * 1024 + lane * 32;
-    const float4 a = *reinterpret_cast<const float4*>(at + (c0 ^ (lane & 7)) * 4);
-    const float4 c = *reinterpret_cast<const float4*>(at + ((c0 + 1) ^ (lane & 7)) * 4);
-    const float f[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
-    *reinterpret_cast<uint4*>(p.dq + bi * p.dq_ts + (long long)h * D + v * 8) = pack8(f);
+    const int lane = (int)(idx & 31);
+    const long long w = idx >> 5;                              // (tile, quad, chunk): the accumulator's order
+    const int chunk = (int)(w % CPR), quad = (int)((w / CPR) & 3);
+    const long long tile = w / (CPR * 4);
+    const int mblock = (int)(tile % n_mblocks);
+    const long long bh = tile / n_mblocks;
+    const int row = mblock * 128 + quad * 32 + lane;
+    if (row >= p.Sq) continue;
+    const int h = (int)(bh % p.hq);
+    const long long b = bh / p.hq;
+    const float4* at = reinterpret_cast<const float4*>(p.dq_acc) + (w * 8) * 32 + lane;
+    float f[32];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const float4 v = at[k * 32];
+      f[4 * k] = v.x; f[4 * k + 1] = v.y; f[4 * k + 2] = v.z; f[4 * k + 3] = v.w;
+    }
+    bf16* o = p.dq + (b * p.Sq + row) * p.dq_ts + (long long)h * D + chunk * 32;
+#pragma unroll
+    for (int k = 0; k < 4; k++) *reinterpret_cast<uint4*>(o + k * 8) = pack8(f + k * 8);
   }
 }
 
@@ -147,14 +161,15 @@ __global__ void fa_bwd_prep_kernel(const FaBwdParams p) {
 template <int D>
 __global__ void __launch_bounds__(512, 1)
 fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
-                 const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo, const FaBwdParams p) {
+                 const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tdk,
+                 const __grid_constant__ CUtensorMap tdv, const FaBwdParams p) {
   using C = BwdCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NBAR);
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);     // {abort, extra wait in ms}: see bw::mbar_wait
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform over the warp)
   const uint32_t sbase = smem_u32(smem);
   if (sbase & 1023u) {                                       // the swizzled tiles need it; nothing has been started yet
     if (threadIdx.x == 0) atomicExch(&g_fab_status[0], 4u);
@@ -199,23 +214,24 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     for (int s = 0; s < C::DS; s++) { mbar_init(do_full(s), 1); mbar_init(do_empty(s), 1); }
     mbar_init(s_full, 1);
     mbar_init(dp_full, 1);
-    mbar_init(p_full, 256);
-    mbar_init(ds_full, 256);
+    mbar_init(p_full, 8);
+    mbar_init(ds_full, 8);
     mbar_init(dq_full, 1);
-    mbar_init(dq_free, 128);
+    mbar_init(dq_free, 4);
     mbar_init_fence();
-    prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tdo);
+    prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv); prefetch_tmap(&tdo); prefetch_tmap(&tdk); prefetch_tmap(&tdv);
   }
   if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
   fence_before();
   __syncthreads();
   fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   volatile int* abort_flag = s_abort;
 
+  if (warp < 4) reg_dec<C::REGS_ISSUE>();
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------
-    if (lane == 0 && total_it > 0) {
+    if (total_it > 0 && elect_one()) {
       mbar_expect_tx(kv_full, 2 * C::TILE_BYTES);
 #pragma unroll
       for (int a = 0; a < C::ATOMS; a++) {
@@ -223,27 +239,29 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         tma_load_2d(sbase + C::OFF_V + a * C::ATOM_BYTES, &tv, hk * D + a * 64, b * p.kv_brows + n0, kv_full);
       }
       bool ok = true;
+      int h = hk * rep, mb = mb_first, st = 0, dst = 0;
+      uint32_t ph = 1u, dph = 1u;
       for (int it = 0; it < total_it; it++) {
-        const int qs = it % C::QS, ds = it % C::DS;
-        const int h = hk * rep + it / per_head;
-        const int mb = mb_first + it % per_head;
-        if (!mbar_wait(q_empty(qs), (((uint32_t)(it / C::QS)) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-        mbar_expect_tx(q_full(qs), C::TILE_BYTES + 1024);
+        if (!mbar_wait(q_empty(st), ph, abort_flag)) { ok = false; break; }
+        mbar_expect_tx(q_full(st), C::TILE_BYTES + 1024);
 #pragma unroll
         for (int a = 0; a < C::ATOMS; a++)
-          tma_load_2d(sbase + C::OFF_Q + qs * C::TILE_BYTES + a * C::ATOM_BYTES, &tq, h * D + a * 64, b * p.Sq + mb * C::BM, q_full(qs));
-        bulk_load(sbase + C::OFF_ST + qs * 1024, p.stats + (((long long)b * p.hq + h) * n_mblocks + mb) * 256, 1024, q_full(qs));
-        if (!mbar_wait(do_empty(ds), (((uint32_t)(it / C::DS)) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-        mbar_expect_tx(do_full(ds), C::TILE_BYTES);
+          tma_load_2d(sbase + C::OFF_Q + st * C::TILE_BYTES + a * C::ATOM_BYTES, &tq, h * D + a * 64, b * p.Sq + mb * C::BM, q_full(st));
+        bulk_load(sbase + C::OFF_ST + st * 1024, p.stats + (((long long)b * p.hq + h) * n_mblocks + mb) * 256, 1024, q_full(st));
+        if (!mbar_wait(do_empty(dst), dph, abort_flag)) { ok = false; break; }
+        mbar_expect_tx(do_full(dst), C::TILE_BYTES);
 #pragma unroll
         for (int a = 0; a < C::ATOMS; a++)
-          tma_load_2d(sbase + C::OFF_DO + ds * C::TILE_BYTES + a * C::ATOM_BYTES, &tdo, h * D + a * 64, b * p.Sq + mb * C::BM, do_full(ds));
+          tma_load_2d(sbase + C::OFF_DO + dst * C::TILE_BYTES + a * C::ATOM_BYTES, &tdo, h * D + a * 64, b * p.Sq + mb * C::BM, do_full(dst));
+        if (++mb == n_mblocks) { mb = mb_first; h++; }
+        if (++st == C::QS) { st = 0; ph ^= 1u; }
+        if (++dst == C::DS) { dst = 0; dph ^= 1u; }
       }
       if (!ok) atomicExch(&g_fab_status[0], 1u);
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer -------------------------------
-    if (lane == 0 && total_it > 0) {
+    if (total_it > 0 && elect_one()) {
       const uint32_t idesc_s = make_idesc(128, 128, 0, 0);     // S^T, dP^T: K-major A and B
       const uint32_t idesc_kv = make_idesc(128, D, 0, 1);      // dV, dK: A in TMEM, MN-major B
       const uint32_t idesc_dq = make_idesc(128, D, 1, 1);      // dQ: MN-major A and B
@@ -266,93 +284,95 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
           umma_bf16_ta(tmem_base + col, tmem_base + acol + (s >> 2) * 64 + (s & 3) * 8, bop + (uint64_t)(s * 128), idesc_kv,
                        s ? 1u : acc);
       };
-      auto issue_s = [&](int it) -> bool {
-        const int qs = it % C::QS;
-        if (!mbar_wait(q_full(qs), ((uint32_t)(it / C::QS)) & 1u, abort_flag)) return false;
-        fence_after();
-        scores(C::COL_S, kK, kQ + (uint64_t)((qs * C::TILE_BYTES) >> 4));
+      // What a step waits for is waited for ahead of the wait that is the last to come: a wait takes some 100 cycles even where
+      // there is nothing to wait for.
+      auto issue_s = [&](uint64_t so) {                          // (Q is there)
+        scores(C::COL_S, kK, kQ + so);
         umma_commit(s_full);
-        return true;
       };
-      auto issue_dp = [&](int it) -> bool {
-        const int ds = it % C::DS;
-        if (!mbar_wait(do_full(ds), ((uint32_t)(it / C::DS)) & 1u, abort_flag)) return false;
-        if (C::DQ_ALIAS && it > 0 && !mbar_wait(dq_free, (uint32_t)(it - 1) & 1u, abort_flag)) return false;
-        fence_after();
-        scores(C::COL_DP, kV, kDO + (uint64_t)((ds * C::TILE_BYTES) >> 4));
+      auto issue_dp = [&](uint64_t so) {                         // (dO is there, dQ has left the columns)
+        scores(C::COL_DP, kV, kDO + so);
         umma_commit(dp_full);
-        return true;
       };
-      bool ok = mbar_wait(kv_full, 0, abort_flag);
-      if (ok) ok = issue_s(0);
-      if (ok) ok = issue_dp(0);
+      bool ok = mbar_wait(kv_full, 0, abort_flag) && mbar_wait(q_full(0), 0, abort_flag);
+      if (ok) { fence_after(); issue_s(0); ok = mbar_wait(do_full(0), 0, abort_flag); }
+      if (ok) { fence_after(); issue_dp(0); }
+      int st = 0, dst = 0;
+      uint32_t ph = 0, dph = 0;
       for (int it = 0; it < total_it && ok; it++) {
         const bool more = it + 1 < total_it;
-        const uint64_t qo = (uint64_t)(((it % C::QS) * C::TILE_BYTES) >> 4), go = (uint64_t)(((it % C::DS) * C::TILE_BYTES) >> 4);
+        const int sn = st + 1 == C::QS ? 0 : st + 1, dn = dst + 1 == C::DS ? 0 : dst + 1;       // stages of the next block
+        const uint32_t phn = sn ? ph : ph ^ 1u, dphn = dn ? dph : dph ^ 1u;
+        if (more && !(ok = mbar_wait(q_full(sn), phn, abort_flag))) break;
         if (!(ok = mbar_wait(p_full, (uint32_t)it & 1u, abort_flag))) break;
         fence_after();
-        grad_kv(C::COL_DV, C::COL_S, mDO + go, it ? 1u : 0u);            // dV += P^T dO
-        umma_commit(do_empty(it % C::DS));
-        if (more && !(ok = issue_s(it + 1))) break;                      // P^T has been read: S^T of the next block
+        grad_kv(C::COL_DV, C::COL_S, mDO + (uint64_t)((dst * C::TILE_BYTES) >> 4), it ? 1u : 0u);       // dV += P^T dO
+        umma_commit(do_empty(dst));
+        if (more) issue_s((uint64_t)((sn * C::TILE_BYTES) >> 4));        // P^T has been read: S^T of the next block
+        if (!C::DQ_ALIAS && more && !(ok = mbar_wait(do_full(dn), dphn, abort_flag))) break;
+        if (!C::DQ_ALIAS && it > 0 && !(ok = mbar_wait(dq_free, (uint32_t)(it - 1) & 1u, abort_flag))) break;
         if (!(ok = mbar_wait(ds_full, (uint32_t)it & 1u, abort_flag))) break;
         fence_after();
-        grad_kv(C::COL_DK, C::COL_DP, mQ + qo, it ? 1u : 0u);            // dK += dS^T Q
-        umma_commit(q_empty(it % C::QS));
-        if (!C::DQ_ALIAS && more && !(ok = issue_dp(it + 1))) break;
-        if (!C::DQ_ALIAS && it > 0) {
-          if (!(ok = mbar_wait(dq_free, (uint32_t)(it - 1) & 1u, abort_flag))) break;
-          fence_after();
-        }
+        grad_kv(C::COL_DK, C::COL_DP, mQ + (uint64_t)((st * C::TILE_BYTES) >> 4), it ? 1u : 0u);        // dK += dS^T Q
+        umma_commit(q_empty(st));
+        if (!C::DQ_ALIAS && more) issue_dp((uint64_t)((dn * C::TILE_BYTES) >> 4));
 #pragma unroll
         for (int s = 0; s < C::BN / 16; s++)                             // dQ = dS K
           umma_bf16(tmem_base + C::COL_DQ, mDS + (uint64_t)(s * 128), mK + (uint64_t)(s * 128), idesc_dq, s ? 1u : 0u);
         umma_commit(dq_full);
-        if (C::DQ_ALIAS && more) ok = issue_dp(it + 1);
+        if (C::DQ_ALIAS && more) {
+          if (!(ok = mbar_wait(do_full(dn), dphn, abort_flag))) break;
+          if (!(ok = mbar_wait(dq_free, (uint32_t)it & 1u, abort_flag))) break;
+          fence_after();
+          issue_dp((uint64_t)((dn * C::TILE_BYTES) >> 4));
+        }
+        st = sn; ph = phn;
+        dst = dn; dph = dphn;
       }
       if (!ok) atomicExch(&g_fab_status[0], 2u);
     }
   } else if (warp >= 12) {
+    if constexpr (C::REGS_DRAIN > 128) reg_inc<C::REGS_DRAIN>(); else reg_dec<C::REGS_DRAIN>();
     // ------------------------------- dQ drain -------------------------------
     const int quad = warp & 3;
     const uint32_t tdq = tmem_base + ((uint32_t)(quad * 32) << 16) + C::COL_DQ;
     uint8_t* stg = smem + C::OFF_STG + quad * 2 * C::STG_BYTES;
+    float* tile = p.dq_acc + (((long long)b * p.hq + hk * rep) * n_mblocks + mb_first) * (128 * D) + quad * (32 * D);
     bool ok = true;
+    int mb = mb_first;
     for (int it = 0; it < total_it; it++) {
-      const int h = hk * rep + it / per_head;
-      const int mb = mb_first + it % per_head;
-      float* tile = p.dq_acc + (((long long)b * p.hq + h) * n_mblocks + mb) * (128 * D) + quad * 1024;
       if (!mbar_wait(dq_full, (uint32_t)it & 1u, abort_flag)) { ok = false; break; }
       fence_after();
+      uint32_t r[D];
 #pragma unroll
-      for (int c2 = 0; c2 < D / 64; c2++) {
-        uint32_t r[64];
-        tmem_ld32(tdq + c2 * 64, r);
-        tmem_ld32(tdq + c2 * 64 + 32, r + 32);
-        tmem_ld_wait();
-        if (c2 == D / 64 - 1) {
-          fence_before();
-          mbar_arrive(dq_free);
-        }
+      for (int c = 0; c < D / 32; c++) tmem_ld32(tdq + c * 32, r + c * 32);
+      tmem_ld_wait();
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(dq_free);
 #pragma unroll
-        for (int c = 0; c < 2; c++) {
-          if (lane == 0) bulk_wait_read_but<1>();      // this half of the staging has been read
-          __syncwarp();
+      for (int c = 0; c < D / 32; c++) {
+        uint8_t* sp = stg + (c & 1) * C::STG_BYTES;
+        if (lane == 0) bulk_wait_read_but<1>();      // this half of the staging has been read
+        __syncwarp();
 #pragma unroll
-          for (int k = 0; k < 8; k++)
-            *reinterpret_cast<uint4*>(stg + c * C::STG_BYTES + lane * 128 + ((k ^ (lane & 7)) << 4)) =
-                make_uint4(r[c * 32 + k * 4], r[c * 32 + k * 4 + 1], r[c * 32 + k * 4 + 2], r[c * 32 + k * 4 + 3]);
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            bulk_reduce_add_f32(tile + (c2 * 2 + c) * 4096, smem_u32(stg + c * C::STG_BYTES), C::STG_BYTES);
-            bulk_commit();
-          }
+        for (int k = 0; k < 8; k++)
+          *reinterpret_cast<uint4*>(sp + k * 512 + lane * 16) =
+              make_uint4(r[c * 32 + k * 4], r[c * 32 + k * 4 + 1], r[c * 32 + k * 4 + 2], r[c * 32 + k * 4 + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          bulk_reduce_add_f32(tile + c * 1024, smem_u32(sp), C::STG_BYTES);
+          bulk_commit();
         }
       }
+      tile += 128 * D;
+      if (++mb == n_mblocks) { mb = mb_first; tile += (long long)mb_first * (128 * D); }
     }
-    if (lane == 0) bulk_wait_all();
+    if (lane == 0) bulk_wait_read_but<0>();
     if (!ok && lane == 0) atomicExch(&g_fab_status[0], 5u);
   } else if (warp >= 4) {
+    reg_inc<C::REGS_MATH>();
     // ------------------------------- math warps -------------------------------
     const int quad = warp & 3;
     const int wg = (warp - 4) >> 2;                 // which 64 of the 128 query columns
@@ -364,11 +384,12 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     const f32x2 sc = pack2(p.scale, p.scale);
     uint8_t* sds = smem + C::OFF_DS + wg * C::ATOM_BYTES;
     bool ok = true;
+    int mb = mb_first, qs = 0;
+    uint32_t qph = 0;
     for (int it = 0; it < total_it; it++) {
-      const int m0 = (mb_first + it % per_head) * C::BM;
-      const int qs = it % C::QS;
+      const int m0 = mb * C::BM;
       const float4* st = reinterpret_cast<const float4*>(smem + C::OFF_ST + qs * 1024) + wg * 16;
-      if (!mbar_wait(q_full(qs), ((uint32_t)(it / C::QS)) & 1u, abort_flag) ||        // the statistics
+      if (!mbar_wait(q_full(qs), qph, abort_flag) ||        // the statistics
           !mbar_wait(s_full, (uint32_t)it & 1u, abort_flag)) { ok = false; break; }
       fence_after();
       float pf[64];
@@ -406,7 +427,8 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         tmem_st_wait();
       }
       fence_before();
-      mbar_arrive(p_full);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
       if (!mbar_wait(dp_full, (uint32_t)it & 1u, abort_flag)) { ok = false; break; }
       fence_after();
       uint32_t dd[32];
@@ -440,29 +462,42 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       tmem_st_wait();
       fence_before();
       fence_proxy_async_smem();
-      mbar_arrive(ds_full);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ds_full);
+      if (++mb == n_mblocks) mb = mb_first;
+      if (++qs == C::QS) { qs = 0; qph ^= 1u; }
     }
     // dQ of the last block is the last MMA: everything has finished
     if (ok && total_it > 0) ok = mbar_wait(dq_full, (uint32_t)(total_it - 1) & 1u, abort_flag);
-    bf16* orow = wg ? p.dk + ((long long)b * p.Sk + key) * p.dk_ts + (long long)hk * D
-                    : p.dv + ((long long)b * p.Sk + key) * p.dv_ts + (long long)hk * D;
     if (ok && total_it > 0) {
+      // through shared memory (K's tile for dV, V's for dK: nothing reads them any more), 64 columns of 32 keys at a time
       fence_after();
 #pragma unroll 1
-      for (int c = 0; c < D / 32; c++) {
-        uint32_t r[32];
-        tmem_ld32(lane_addr + (wg ? C::COL_DK : C::COL_DV) + c * 32, r);
+      for (int a = 0; a < C::ATOMS; a++) {
+        uint8_t* out = smem + (wg ? C::OFF_V : C::OFF_K) + a * C::ATOM_BYTES + quad * 4096;
+        uint32_t r[64];
+        tmem_ld32(lane_addr + (wg ? C::COL_DK : C::COL_DV) + a * 64, r);
+        tmem_ld32(lane_addr + (wg ? C::COL_DK : C::COL_DV) + a * 64 + 32, r + 32);
         tmem_ld_wait();
-        if (key < p.Sk) {
-          float f[32];
 #pragma unroll
-          for (int i = 0; i < 32; i++) f[i] = __uint_as_float(r[i]);
+        for (int g = 0; g < 8; g++) {
+          float f[8];
 #pragma unroll
-          for (int g = 0; g < 4; g++) *reinterpret_cast<uint4*>(orow + c * 32 + g * 8) = pack8(f + g * 8);
+          for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[g * 8 + i]);
+          *reinterpret_cast<uint4*>(out + sw128_off(lane, g)) = pack8(f);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && n0 + quad * 32 < p.Sk) {
+          tma_store_3d(wg ? &tdk : &tdv, smem_u32(out), hk * D + a * 64, n0 + quad * 32, b);
+          bulk_commit();
         }
       }
+      if (lane == 0) bulk_wait_read_but<0>();        // nothing reads shared memory after the CTA's end
     } else if (total_it == 0 && key < p.Sk) {
       // no query sees these keys: their gradients are zero
+      bf16* orow = wg ? p.dk + ((long long)b * p.Sk + key) * p.dk_ts + (long long)hk * D
+                      : p.dv + ((long long)b * p.Sk + key) * p.dv_ts + (long long)hk * D;
       for (int c = 0; c < D / 8; c++) *reinterpret_cast<uint4*>(orow + c * 8) = make_uint4(0, 0, 0, 0);
     }
     if (!ok && lane == 0) atomicExch(&g_fab_status[0], 3u);
@@ -480,15 +515,20 @@ template <int D>
 int launch_fa_bwd(const void* q, const void* k, const void* v, const FaBwdParams& p, long long q_ts, long long k_ts,
                   long long v_ts, cudaStream_t s) {
   using C = BwdCfg<D>;
-  CUtensorMap tq, tk, tv, tdo;
+  CUtensorMap tq, tk, tv, tdo, tdk, tdv;
   int rc;
   if ((rc = make_map_bf16(&tq, q, (uint64_t)p.hq * D, (uint64_t)p.B * p.Sq, (uint64_t)q_ts, 64, 128))) return rc;
   const uint64_t kv_rows = (uint64_t)(p.B - 1) * p.kv_brows + p.Sk;
   if ((rc = make_map_bf16(&tk, k, (uint64_t)p.hkv * D, kv_rows, (uint64_t)k_ts, 64, 128))) return rc;
   if ((rc = make_map_bf16(&tv, v, (uint64_t)p.hkv * D, kv_rows, (uint64_t)v_ts, 64, 128))) return rc;
   if ((rc = make_map_bf16(&tdo, p.dout, (uint64_t)p.hq * D, (uint64_t)p.B * p.Sq, (uint64_t)p.do_ts, 64, 128))) return rc;
+  if ((rc = make_map_bf16_3d(&tdk, p.dk, (uint64_t)p.hkv * D, (uint64_t)p.Sk, (uint64_t)p.B, (uint64_t)p.dk_ts, 64, 32))) return rc;
+  if ((rc = make_map_bf16_3d(&tdv, p.dv, (uint64_t)p.hkv * D, (uint64_t)p.Sk, (uint64_t)p.B, (uint64_t)p.dv_ts, 64, 32))) return rc;
   static bool attr = false;
   if (!attr) {
+    // the register split must fit in what the launch allocates, or it would wait for registers that nobody gives back
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, fa_bwd_tc_kernel<D>) != cudaSuccess || (fa.numRegs + 7) / 8 * 8 != 128) return LB_ERR_LAUNCH;
     cudaFuncSetAttribute(fa_bwd_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
     attr = true;
   }
@@ -499,9 +539,9 @@ int launch_fa_bwd(const void* q, const void* k, const void* v, const FaBwdParams
   const long long pblocks = (rows + rows_per_block - 1) / rows_per_block;
   fa_bwd_prep_kernel<D><<<(int)(pblocks < cap ? pblocks : cap), 256, 0, s>>>(p);
   LB_CHECK_LAUNCH();
-  fa_bwd_tc_kernel<D><<<(unsigned)grid, C::NTHREADS, C::SMEM, s>>>(tq, tk, tv, tdo, p);
+  fa_bwd_tc_kernel<D><<<(unsigned)grid, C::NTHREADS, C::SMEM, s>>>(tq, tk, tv, tdo, tdk, tdv, p);
   LB_CHECK_LAUNCH();
-  const long long cblocks = ((long long)p.B * p.Sq * p.hq * (D / 8) + 255) / 256;
+  const long long cblocks = (rows * (D / 32) + 255) / 256;
   fa_dq_convert_kernel<D><<<(int)(cblocks < cap ? cblocks : cap), 256, 0, s>>>(p);
   LB_CHECK_LAUNCH();
   return LB_OK;

@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   __shared__ int s_abort[2];     // {abort, extra wait in ms}: see bw::mbar_wait
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);      // (uniform over the warp)
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = bw::smem_u32(smem);
   const uint32_t bar_base = bw::smem_u32(bars);
@@ -204,12 +204,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
   __syncthreads();
   if constexpr (CG == 2) bw::cluster_sync();      // the peer's barriers exist before anything signals them
   bw::fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   volatile int* abort_flag = s_abort;
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (bw::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && bw::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
   __shared__ int s_abort[2];     // {abort, extra wait in ms}: see bw::mbar_wait
   __shared__ int s_off[MAX_PROBLEMS], s_tiles[MAX_PROBLEMS];
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);      // (uniform over the warp)
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = bw::smem_u32(smem);
   const uint32_t bar_base = bw::smem_u32(bars);
@@ -548,12 +548,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
   bw::fence_before();
   __syncthreads();
   bw::fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   volatile int* abort_flag = s_abort;
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (bw::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    if (bw::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;

@@ -27,6 +27,7 @@
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include "comm.cuh"
+#include "gemm_split.h"
 
 static __device__ unsigned int g_grp_status[4] = {0, 0, 0, 0};
 
@@ -670,6 +671,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
 
 // ---- host side: static schedule, cached per (device, shapes) -------------------------------------
 struct Schedule {
+  int split = 0;      // parts of K of a launch that the split form takes (gemm_split.cu; nothing else is set then), or 0
   int cg = 1;         // CTAs per tile
   int grid = 0;       // workers (CTAs, or pairs of CTAs)
   int* d_offsets = nullptr;
@@ -751,21 +753,31 @@ void set_tiles(Problem* p, int cg) {
 // of one tile per CTA).  CTAs / pairs in us: where the store of a tile outlasts its main loop, 16384 x 4096 x 256 64.6 / 79.8,
 // x 512 80.0 / 88.9, 8192 x 4096 x 768 51.2 / 52.4; where it does not, 8192 x 4096 x 1024 62.1 / 58.7, 16384 x 4096 x 1536 167 / 150,
 // 4096 x 11264 x 4096 287 / 259; short launches, 1000 x 2304 x 768 14.6 / 16.5, 1000 x 768 x 4096 31.2 / 30.3.
-int choose_cg(Problem* probs, int np, int sms) {
+int choose_cg(Problem* probs, int np, int sms, long long* best = nullptr) {
   if (sms < 2) return 1;
   long long time[3] = {0, 0, 0};
   for (int cg = 1; cg <= 2; cg++) {
     for (int i = 0; i < np; i++) set_tiles(&probs[i], cg);
     if (assign_items(probs, np, cg, sms, nullptr, nullptr, nullptr, &time[cg]) < 0) return -1;
   }
-  return time[2] + 600 < time[1] ? 2 : 1;
+  const int cg = time[2] + 600 < time[1] ? 2 : 1;
+  if (best) *best = cg == 2 ? time[2] + 600 : time[1];
+  return cg;
+}
+
+int parts_of(const Problem* probs, int np, int sms, long long list_time) {
+  int M[MAX_PROBLEMS], N[MAX_PROBLEMS], K[MAX_PROBLEMS];
+  for (int i = 0; i < np; i++) { M[i] = probs[i].M; N[i] = probs[i].N; K[i] = probs[i].K; }
+  return gemm_split_parts(np, M, N, K, sms, list_time);
 }
 
 int build_schedule(Problem* probs, int np, int sms, Schedule* out) {
   std::vector<std::vector<int>> per;
   int total = 0;
-  out->cg = choose_cg(probs, np, sms);
+  long long time = 0;
+  out->cg = choose_cg(probs, np, sms, &time);
   if (out->cg < 0) return LB_ERR_SHAPE;
+  if (time > 0 && (out->split = parts_of(probs, np, sms, time)) > 0) return LB_OK;
   for (int i = 0; i < np; i++) set_tiles(&probs[i], out->cg);
   if (assign_items(probs, np, out->cg, sms, &per, &total, nullptr, nullptr) < 0) return LB_ERR_SHAPE;
   const int grid = (int)per.size();
@@ -831,6 +843,16 @@ bool plan_problems(int n, const int* M, const int* N, const int* K, int sms, Pro
 }
 }  // namespace
 
+// Host only (no CUDA call): parts of K (1, 2 or 4) with which lb_gemm_grouped gives these shapes to the split form (gemm_split.cu), 0 where
+// it takes the list form, which the two entry points below describe.
+extern "C" int lb_gemm_grouped_parts(int n, const int* M, const int* N, const int* K, int sms) {
+  Problem probs[MAX_PROBLEMS];
+  if (!plan_problems(n, M, N, K, sms, probs)) return LB_ERR_SHAPE;
+  long long time = 0;
+  if (choose_cg(probs, n, sms, &time) < 0) return LB_ERR_SHAPE;
+  return time > 0 ? parts_of(probs, n, sms, time) : 0;
+}
+
 // Host only (no CUDA call): CTAs per tile, 1 or 2, of the schedule that lb_gemm_grouped builds for these shapes on `sms` SMs.
 extern "C" int lb_gemm_grouped_ctas_per_tile(int n, const int* M, const int* N, const int* K, int sms) {
   Problem probs[MAX_PROBLEMS];
@@ -859,7 +881,8 @@ extern "C" int lb_gemm_grouped_plan(int n, const int* M, const int* N, const int
 // n problems (1..8), arrays of length n.  Per problem the rules of lb_gemm_bf16 apply: pointers
 // 16-byte aligned, lda / ldb / ldc / N multiples of 8 (M too when a_mn).  accumulate[i] != 0 adds
 // the product to the old contents of C_i.  The first call with a new set of shapes builds and
-// uploads the schedule (two small device allocations, synchronous copies); later calls only launch.
+// uploads the schedule (two small device allocations, synchronous copies); later calls only launch.  Launches of one or two problems that
+// do not fill the chip go to the split form (gemm_split.cu), which has no schedule to upload.
 //
 // lb_gemm_grouped_epi additionally takes, per problem, an epilogue selector (see `Problem`), a second
 // matrix C2 with its leading dimension, and `half`:
@@ -881,10 +904,6 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
     if (M[i] <= 0 || N[i] <= 0 || K[i] <= 0) return LB_ERR_SHAPE;
     if ((lda[i] % 8) || (ldb[i] % 8) || (ldc[i] % 8) || (N[i] % 8) || (a_mn[i] && (M[i] % 8))) return LB_ERR_SHAPE;
     if (((uintptr_t)A[i] | (uintptr_t)B[i] | (uintptr_t)C[i]) & 15) return LB_ERR_ARG;
-    int rc;
-    if (!a_mn[i]) rc = bw::make_map_bf16(&gp.ta[i], A[i], (uint64_t)K[i], (uint64_t)M[i], (uint64_t)lda[i], BK, BM);
-    else          rc = bw::make_map_bf16(&gp.ta[i], A[i], (uint64_t)M[i], (uint64_t)K[i], (uint64_t)lda[i], 64, BK);
-    if (rc) return rc;
     const int e = epi ? epi[i] : 0;
     if (e < 0 || e > 2) return LB_ERR_ARG;
     if (e) {
@@ -893,9 +912,6 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
       if (e == 2 && N[i] != half[i]) return LB_ERR_SHAPE;
       if (accumulate && accumulate[i]) return LB_ERR_ARG;
     }
-    if (!b_mn[i]) rc = bw::make_map_bf16(&gp.tb[i], B[i], (uint64_t)K[i], (uint64_t)N[i], (uint64_t)ldb[i], BK, BN / 2);
-    else          rc = bw::make_map_bf16(&gp.tb[i], B[i], (uint64_t)N[i], (uint64_t)K[i], (uint64_t)ldb[i], 64, BK);
-    if (rc) return rc;
     Problem& p = gp.prob[i];
     p.C = (bf16*)C[i]; p.ldc = ldc[i]; p.M = M[i]; p.N = N[i]; p.K = K[i];
     p.C2 = e ? (bf16*)C2[i] : nullptr; p.ldc2 = e ? ldc2[i] : 0; p.epi = e; p.half = e ? half[i] : 0;
@@ -931,6 +947,17 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
     }
     it->second.last_use = ++g_sched_clock;
     sched = it->second;
+  }
+  if (sched.split)
+    return lb_gemm_split(n, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, epi, C2, ldc2, half, sched.split, stream);
+  for (int i = 0; i < n; i++) {
+    int rc;
+    if (!a_mn[i]) rc = bw::make_map_bf16(&gp.ta[i], A[i], (uint64_t)K[i], (uint64_t)M[i], (uint64_t)lda[i], BK, BM);
+    else          rc = bw::make_map_bf16(&gp.ta[i], A[i], (uint64_t)M[i], (uint64_t)K[i], (uint64_t)lda[i], 64, BK);
+    if (rc) return rc;
+    if (!b_mn[i]) rc = bw::make_map_bf16(&gp.tb[i], B[i], (uint64_t)K[i], (uint64_t)N[i], (uint64_t)ldb[i], BK, BN / 2);
+    else          rc = bw::make_map_bf16(&gp.tb[i], B[i], (uint64_t)N[i], (uint64_t)K[i], (uint64_t)ldb[i], 64, BK);
+    if (rc) return rc;
   }
   gp.offsets = sched.d_offsets;
   gp.items = sched.d_items;

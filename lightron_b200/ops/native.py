@@ -51,6 +51,8 @@ _SIGNATURES = {
     "lb_gemm_bf16": [_P, _P, _P, _I, _I, _I, _L, _L, _L, _I, _I, _I, _P],
     "lb_gemm_grouped": [_I] + [_P] * 13,
     "lb_gemm_grouped_epi": [_I] + [_P] * 17,
+    "lb_gemm_split": [_I] + [_P] * 16 + [_I, _P],
+    "lb_gemm_split_status": [_P],
     "lb_peer_copy": [_P, _P, _L, _I, _I, _P],
     "lb_peer_copy_flagged": [_P, _P, _L, _I, _I, _L, _P, _P],
     "lb_embed_tp_fwd": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, ctypes.c_uint, _P],
@@ -59,6 +61,7 @@ _SIGNATURES = {
     "lb_gemm_grouped_cached": [],
     "lb_gemm_grouped_plan": [_I, _P, _P, _P, _I, _P],
     "lb_gemm_grouped_ctas_per_tile": [_I, _P, _P, _P, _I],
+    "lb_gemm_grouped_parts": [_I, _P, _P, _P, _I],
     "lb_gemm_ag": [_P, _P, _I, _I, _I, _L, _L, _I, _I, _I, _P, _L, _P, _P, ctypes.c_uint, _I, _P],
     "lb_gemm_rs": [_P, _P, _I, _I, _I, _L, _L, _I, _I, _I, _P, _P, ctypes.c_uint, _P, _L, _P],
     "lb_moe_status": [_P],
@@ -226,6 +229,7 @@ def call(name: str, *args) -> None:
 
 
 _STATUS_READERS = (("lb_device_status", "GEMM / fused collective GEMM"), ("lb_gemm_grouped_status", "grouped GEMM"),
+                   ("lb_gemm_split_status", "GEMM of small launches"),
                    ("lb_flash_status", "attention forward"), ("lb_flash_bwd_status", "attention backward"),
                    ("lb_dp_status", "data-parallel optimizer kernel"),
                    ("lb_moe_status", "expert-parallel routing / dispatch / combine"),

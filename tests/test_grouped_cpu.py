@@ -74,6 +74,20 @@ def test_pairs_are_chosen_where_they_are_faster(shapes, cg):
     assert _ctas_per_tile(shapes) == cg
 
 
+@pytest.mark.parametrize("shapes,parts", [
+    ([(128, 768, 2048)], 4), ([(128, 2048, 5632)], 4), ([(128, 2304, 768)], 1), ([(16, 11264, 2048)], 1), ([(8, 8, 8)], 1),
+    ([(768, 768, 1000), (1000, 768, 768)], 1), ([(1000, 768, 2048)], 2),
+    # enough tiles of 128 x 256 to fill the chip, or more than two problems
+    ([(16384, 2048, 2048)], 0), ([(1000, 4096, 768)], 0), ([(1000, 32000, 768)], 0), ([(2048, 2048, 2048)], 0), ([(128, 768, 2048)] * 3, 0),
+])
+def test_short_launches_are_split(shapes, parts):
+    lib = native._load()
+    if lib is None:
+        pytest.skip("native library not built")
+    IA = ctypes.c_int * len(shapes)
+    assert lib.lb_gemm_grouped_parts(len(shapes), *(IA(*[s[i] for s in shapes]) for i in range(3)), 148) == parts
+
+
 def test_schedule_rejects_bad_arguments():
     lib = native._load()
     if lib is None:

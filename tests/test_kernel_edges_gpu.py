@@ -194,6 +194,54 @@ def test_gemm_pair_tiles(M, N, K, ctas, a_mn, b_mn):
     assert _rel(out, want + c0.double()) < 5e-3
 
 
+def _gemm_split(ks, a, b, a_mn, b_mn, out, accumulate, epi=0, c2=None, half=0):
+    """The split form of a GEMM launch, whatever the rule says about these sizes."""
+    import ctypes
+    from lightron_b200.ops import native
+    P, I, L = (lambda v, t=t: (t * 1)(v) for t in (ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong))
+    M, K = (a.shape[1], a.shape[0]) if a_mn else a.shape
+    native.call("lb_gemm_split", 1, P(a.data_ptr()), P(b.data_ptr()), P(out.data_ptr()), I(M), I(b.shape[1] if b_mn else b.shape[0]), I(K),
+                L(a.stride(0)), L(b.stride(0)), L(out.stride(0)), I(int(a_mn)), I(int(b_mn)), I(int(accumulate)), I(epi),
+                P(c2.data_ptr() if epi else 0), L(c2.stride(0) if epi else 0), I(half), ks, native.stream_ptr())
+
+
+@pytest.mark.parametrize("ks", [1, 2, 4])
+@pytest.mark.parametrize("M,N,K", [
+    (8, 8, 264),             # one row of tiles of which almost nothing exists, 5 k-blocks: parts of 1 and 2
+    (72, 200, 328),          # fewer rows than a tile, loaded without the rest
+    (136, 64, 1032),         # a second tile of 8 rows, one column tile, the last k-block ragged
+    (1000, 776, 256),        # as many k-blocks as parts
+])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+def test_gemm_split_tiles(ks, M, N, K, a_mn, b_mn):
+    """Parts of K summed over a cluster; nothing is written behind the last row."""
+    a, b, c0 = _rand(M, K, seed=1), _rand(N, K, seed=2), _rand(M, N, seed=3)
+    ops = (a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b)
+    want = a.double() @ b.double().t()
+    buf = torch.full((M + 8, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    _gemm_split(ks, *ops, a_mn, b_mn, buf[:M], False)
+    acc = c0.clone()
+    _gemm_split(ks, *ops, a_mn, b_mn, acc, True)
+    _status_ok()
+    assert _rel(buf[:M], want) < 5e-3 and _rel(acc, want + c0.double()) < 5e-3 and bool((buf[M:] == 7.0).all())
+
+
+@pytest.mark.parametrize("ks", [1, 2, 4])
+@pytest.mark.parametrize("T,K,I", [(8, 264, 8), (130, 328, 72), (300, 768, 264)])
+def test_gemm_split_activation(ks, T, K, I):
+    """silu(g) u and its gradient in the epilogue of a split tile, half of whose columns are gate and half are up."""
+    x, w13, dy, w2 = _rand(T, K, seed=1), _rand(2 * I, K, scale=K ** -0.5, seed=2), _rand(T, K, seed=3), _rand(K, I, scale=K ** -0.5, seed=4)
+    gu, h, dgu = (torch.empty(T, n, dtype=torch.bfloat16, device="cuda") for n in (2 * I, I, 2 * I))
+    _gemm_split(ks, x, w13, False, False, gu, False, 1, h, I)
+    _gemm_split(ks, dy, w2, False, True, dgu, False, 2, gu, I)
+    _status_ok()
+    want = x.double() @ w13.double().t()
+    g64 = gu.double().requires_grad_()
+    act = torch.nn.functional.silu(g64[:, :I]) * g64[:, I:]
+    act.backward(dy.double() @ w2.double())
+    assert _rel(gu, want) < 5e-3 and _rel(h, act.detach()) < 5e-3 and _rel(dgu, g64.grad) < 1e-2
+
+
 @pytest.mark.parametrize("T,K,I,ctas", [(300, 4096, 264, 2), (2100, 1032, 2312, 2), (4000, 256, 1288, 1), (70, 512, 264, 1)])
 def test_swiglu_mlp_pair_tiles(T, K, I, ctas):
     """The activation in the epilogue of pairs, whose peer loads the up rows, and of single CTAs; ragged in every size."""

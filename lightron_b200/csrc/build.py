@@ -3,8 +3,9 @@
     python -m lightron_b200.csrc.build [--verbose] [--force] [--sanitize]
 
 The result, ``liblightron_b200.so``, sits beside the sources (git-ignored) and is loaded through
-ctypes by ``lightron_b200.ops.native``.  No torch headers are involved, so a full build takes
-seconds and cross-compiles on a machine without a GPU.
+ctypes by ``lightron_b200.ops.native``.  No torch headers are involved in it, so it takes
+seconds and cross-compiles on a machine without a GPU.  ``_host_ops.so`` (``host_ops.cpp``, the autograd nodes
+that call it) is built against the installed torch, at the same time.
 
 ``--sanitize`` builds ``liblightron_b200_asan.so`` instead: the same sources with the HOST code under
 AddressSanitizer + UndefinedBehaviorSanitizer (device code is unchanged).  Load it with
@@ -20,6 +21,7 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB = os.path.join(HERE, "liblightron_b200.so")
+HOST_SRC, HOST_LIB = os.path.join(HERE, "host_ops.cpp"), os.path.join(HERE, "_host_ops.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -27,11 +29,23 @@ def sources():
     return sorted(glob.glob(os.path.join(HERE, "*.cu")))
 
 
+def host_command(out: str) -> list:
+    """Compiler call for the extension module of the autograd nodes."""
+    import sysconfig
+    import torch
+    base = os.path.dirname(torch.__file__)
+    inc = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+           os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")]
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in inc), HOST_SRC, "-o", out,
+            f"-L{os.path.join(base, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python"]
+
+
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
+    if not (os.path.exists(LIB) and os.path.exists(HOST_LIB)):
         return True
-    t = os.path.getmtime(LIB)
-    deps = sources() + glob.glob(os.path.join(HERE, "*.cuh")) + glob.glob(os.path.join(HERE, "*.h"))
+    t = min(os.path.getmtime(LIB), os.path.getmtime(HOST_LIB))
+    deps = sources() + [HOST_SRC] + glob.glob(os.path.join(HERE, "*.cuh")) + glob.glob(os.path.join(HERE, "*.h"))
     return any(os.path.getmtime(s) > t for s in deps)
 
 
@@ -48,6 +62,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
             cmd.insert(2, "-v")
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True)))
         objs.append(obj)
+    procs.append((HOST_SRC, subprocess.Popen(host_command(HOST_LIB + ".tmp"), stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True)))
     failed = []
     for src, pr in procs:
         out, err = pr.communicate()
@@ -56,13 +71,14 @@ def build(verbose: bool = False, force: bool = False) -> str:
         if pr.returncode:
             failed.append(os.path.basename(src))
     if failed:
-        raise RuntimeError(f"nvcc failed on {', '.join(failed)}")
+        raise RuntimeError(f"compilation failed on {', '.join(failed)}")
     cmd = [nvcc, *ARCH, "-shared", "-o", LIB + ".tmp", *objs, "-lcudart"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("link failed")
     os.replace(LIB + ".tmp", LIB)
+    os.replace(HOST_LIB + ".tmp", HOST_LIB)
     return LIB
 
 

@@ -216,16 +216,52 @@ _LAUNCHES = 0
 
 def launch_count() -> int:
     """Number of native kernel entry points invoked so far in this process."""
-    return _LAUNCHES
+    return _LAUNCHES + (_HOST.launches() if _HOST else 0)
+
+
+def _raise(name: str, rc: int) -> None:
+    raise NativeError(f"{name} failed: {_ERRORS.get(rc, rc)} (cuda error {require().lb_last_error()})")
 
 
 def call(name: str, *args) -> None:
     global _LAUNCHES
-    lib = require()
-    rc = getattr(lib, name)(*args)
+    rc = getattr(require(), name)(*args)
     _LAUNCHES += 1
     if rc != 0:
-        raise NativeError(f"{name} failed: {_ERRORS.get(rc, rc)} (cuda error {lib.lb_last_error()})")
+        _raise(name, rc)
+
+
+# ---- autograd nodes in C++ ----------------------------------------------------------------------------
+_HOST = False               # not looked for yet; then the extension module, or None
+_HOST_ENTRIES = ("lb_rmsnorm_fwd", "lb_rmsnorm_bwd_blocks", "lb_rmsnorm_bwd", "lb_rope", "lb_gemm_grouped_epi", "lb_flash_fwd_tc",
+                 "lb_flash_bwd_ws_bytes", "lb_flash_bwd_tc_ws", "lb_flash_bwd", "lb_embedding_fwd", "lb_embedding_bwd", "lb_ce_stats",
+                 "lb_ce_loss", "lb_ce_grad")
+
+
+def host_ops():
+    """The extension module with the autograd nodes of the plain cases (``csrc/host_ops.cpp``), or None: without a GPU, or with
+    ``LIGHTRON_HOST_OPS=0``.  The ops then run their autograd functions in Python, on the same kernels."""
+    global _HOST
+    if _HOST is False:
+        _HOST = _load_host_ops() if os.environ.get("LIGHTRON_HOST_OPS", "1") != "0" and available() else None
+    return _HOST
+
+
+def _load_host_ops():
+    import importlib.machinery
+    import importlib.util
+    import warnings
+    path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc", "_host_ops.so")
+    try:
+        loader = importlib.machinery.ExtensionFileLoader("_host_ops", path)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_host_ops", path, loader=loader))
+        loader.exec_module(mod)
+        lib = require()
+        mod.init({n: ctypes.cast(getattr(lib, n), _P).value for n in _HOST_ENTRIES}, _raise)
+        return mod
+    except (ImportError, OSError, AttributeError, RuntimeError) as e:
+        warnings.warn(f"{path} cannot be used ({e}): the ops run their autograd functions in Python (run: python -m lightron_b200.csrc.build)")
+        return None
 
 
 _STATUS_READERS = (("lb_device_status", "GEMM / fused collective GEMM"), ("lb_gemm_grouped_status", "grouped GEMM"),

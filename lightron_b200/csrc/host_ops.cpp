@@ -45,6 +45,7 @@ struct Api {
   int (*lb_flash_bwd_tc_ws)(P, P, P, P, P, P, W, L, W, W, W, int, int, int, int, int, int, L, L, L, L, L, L, L, L, float, int, W);
   int (*lb_flash_bwd)(P, P, P, P, P, P, W, W, W, W, W, int, int, int, int, int, int, L, L, L, L, L, L, L, L, float, int, W);
   int (*lb_embedding_fwd)(P, P, W, int, int, int, int, W);
+  int (*lb_clear)(W, L, W);
   int (*lb_embedding_bwd)(P, P, W, int, int, int, int, W);
   int (*lb_ce_stats)(P, P, W, W, W, int, int, L, int, W);
   int (*lb_ce_loss)(P, W, P, P, W, W, int, float, int, W);
@@ -324,7 +325,8 @@ struct Embedding : Function<Embedding> {
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     const Tensor tok = ctx->get_saved_variables()[0], dy = grads[0].contiguous();
     const std::vector<int64_t> s = ctx->saved_data["shape"].toIntVector();
-    Tensor dw = at::zeros({s[0], s[1]}, dy.options());
+    Tensor dw = empty({s[0], s[1]}, dy);
+    LB_CALL(lb_clear, dw.mutable_data_ptr(), (L)dw.nbytes(), stream());
     LB_CALL(lb_embedding_bwd, tok.const_data_ptr(), dy.const_data_ptr(), dw.mutable_data_ptr(), (int)tok.numel(), (int)s[1], (int)s[2],
             (int)(s[2] + s[0]), stream());
     return {Tensor(), dw, Tensor()};
@@ -547,7 +549,7 @@ PyObject* py_init(PyObject*, PyObject* args) {
   };
 #define LB_TAKE(name) take(#name, &api.name)
   LB_TAKE(lb_rmsnorm_fwd); LB_TAKE(lb_rmsnorm_bwd_blocks); LB_TAKE(lb_rmsnorm_bwd); LB_TAKE(lb_rope); LB_TAKE(lb_gemm_grouped_epi);
-  LB_TAKE(lb_flash_fwd_tc); LB_TAKE(lb_flash_bwd_ws_bytes); LB_TAKE(lb_flash_bwd_tc_ws); LB_TAKE(lb_flash_bwd); LB_TAKE(lb_embedding_fwd);
+  LB_TAKE(lb_flash_fwd_tc); LB_TAKE(lb_flash_bwd_ws_bytes); LB_TAKE(lb_flash_bwd_tc_ws); LB_TAKE(lb_flash_bwd); LB_TAKE(lb_embedding_fwd); LB_TAKE(lb_clear);
   LB_TAKE(lb_embedding_bwd); LB_TAKE(lb_ce_stats); LB_TAKE(lb_ce_loss); LB_TAKE(lb_ce_grad);
   if (!ok) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "an entry point of the kernels is missing");

@@ -751,7 +751,8 @@ class _Embedding(torch.autograd.Function):
         dy2 = dy.reshape(-1, H)
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        dw = torch.zeros(V, H, dtype=dy.dtype, device=dy.device)
+        dw = torch.empty(V, H, dtype=dy.dtype, device=dy.device)
+        native.call("lb_clear", dw.data_ptr(), dw.nbytes, native.stream_ptr())
         native.call("lb_embedding_bwd", tok.data_ptr(), dy2.data_ptr(), dw.data_ptr(), tok.numel(), H,
                     ctx.vocab_start, ctx.vocab_start + V, native.stream_ptr())
         return None, dw, None

@@ -41,6 +41,7 @@ _SIGNATURES = {
     "lb_swiglu_fwd": [_P, _P, _I, _I, _L, _P],
     "lb_swiglu_bwd": [_P, _P, _P, _I, _I, _L, _P],
     "lb_embedding_fwd": [_P, _P, _P, _I, _I, _I, _I, _P],
+    "lb_clear": [_P, ctypes.c_longlong, _P],
     "lb_embedding_bwd": [_P, _P, _P, _I, _I, _I, _I, _P],
     "lb_ce_stats": [_P, _P, _P, _P, _P, _I, _I, _L, _I, _P],
     "lb_ce_loss": [_P, _P, _P, _P, _P, _P, _I, _F, _I, _P],
@@ -234,7 +235,7 @@ def call(name: str, *args) -> None:
 # ---- autograd nodes in C++ ----------------------------------------------------------------------------
 _HOST = False               # not looked for yet; then the extension module, or None
 _HOST_ENTRIES = ("lb_rmsnorm_fwd", "lb_rmsnorm_bwd_blocks", "lb_rmsnorm_bwd", "lb_rope", "lb_gemm_grouped_epi", "lb_flash_fwd_tc",
-                 "lb_flash_bwd_ws_bytes", "lb_flash_bwd_tc_ws", "lb_flash_bwd", "lb_embedding_fwd", "lb_embedding_bwd", "lb_ce_stats",
+                 "lb_flash_bwd_ws_bytes", "lb_flash_bwd_tc_ws", "lb_flash_bwd", "lb_embedding_fwd", "lb_clear", "lb_embedding_bwd", "lb_ce_stats",
                  "lb_ce_loss", "lb_ce_grad")
 
 

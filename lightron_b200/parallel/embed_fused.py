@@ -100,7 +100,8 @@ class _PeerEmbedding(torch.autograd.Function):
         (tok,) = ctx.saved_tensors
         group, v0, sp, (V, H) = ctx.meta
         dy = dy.contiguous()
-        dw = torch.zeros(V, H, dtype=dy.dtype, device=dy.device)
+        dw = torch.empty(V, H, dtype=dy.dtype, device=dy.device)
+        native.call("lb_clear", dw.data_ptr(), dw.nbytes, native.stream_ptr())
         T = tok.numel()
         if not sp:          # the gradient is already the same on every rank
             native.call("lb_embedding_bwd", tok.data_ptr(), dy.data_ptr(), dw.data_ptr(), T, H, v0, v0 + V, native.stream_ptr())

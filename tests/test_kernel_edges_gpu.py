@@ -443,3 +443,13 @@ def test_moe_rows_pushed_and_pulled(T, H, k):
                 one(words.data_ptr() + 128), 2, st)
     assert ((out.double() - got.sum(1)).abs() <= 2.0 ** -8 * got.sum(1).abs() + k * 2.0 ** -23 * got.abs().sum(1)).all()
     native.device_status()           # the dropped copies were counted: read and cleared
+
+
+@pytest.mark.parametrize("n", [0, 1, 15, 16, 17, 4095, 4096, 4111, 1 << 20, (1 << 20) + 7])
+def test_clear_writes_its_bytes_and_no_others(n):
+    from lightron_b200.ops import native
+    buf = torch.full((n + 64,), 7, dtype=torch.uint8, device="cuda")
+    native.call("lb_clear", buf.data_ptr() + 16, n, native.stream_ptr())
+    assert not buf[16:16 + n].any() and (buf[:16] == 7).all() and (buf[16 + n:] == 7).all()
+    with pytest.raises(native.NativeError):
+        native.call("lb_clear", buf.data_ptr() + 8, n, native.stream_ptr())

@@ -54,9 +54,9 @@ __device__ __forceinline__ void moe_fail(unsigned code, unsigned where) {
 // -------------------------------------------------------------------------------------------
 // Router
 // -------------------------------------------------------------------------------------------
-// Latency bound.  IN tokens of a warp go through the gate weights together: a weight vector is fetched once for all of them and their
-// loads are in flight at the same time, but with more than 8 experts the rows are read again for every 8, and IN rows per warp
-// no longer stay in L1 (lb_moe_router has the rule).  The sums of a token are the same for every IN.
+// Latency bound.  IN tokens of a warp go through the gate weights together, 8 experts at a time; the IN row vectors and the 8 weight vectors of
+// a step are all loaded before the first is used (behind a branch per expert each load was waited for by itself: T 4096, H 2048, inputs not in
+// L2, E 8 47 us, now 25; E 64 284, now 96).  The sums of a token are the same for every IN.
 template <int IN>
 __global__ void __launch_bounds__(ROUTER_THREADS)
 moe_router_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wg, int T, int H, int E, int k,
@@ -84,17 +84,22 @@ moe_router_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wg, int T
         for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
       const int ne = min(8, E - e0);
       for (int v = lane; v < nvec; v += 32) {
-        float xf[IN][8];
+        uint4 xr[IN], wr[8];
 #pragma unroll
         for (int i = 0; i < IN; i++) {
           const int t = t0 + warp + (i0 + i) * NW;
-          unpack8(t < T ? reinterpret_cast<const uint4*>(x + (size_t)t * H)[v] : make_uint4(0, 0, 0, 0), xf[i]);
+          xr[i] = t < T ? reinterpret_cast<const uint4*>(x + (size_t)t * H)[v] : make_uint4(0, 0, 0, 0);
         }
+#pragma unroll
+        for (int j = 0; j < 8; j++) wr[j] = __ldg(reinterpret_cast<const uint4*>(wg + (size_t)(e0 + min(j, ne - 1)) * H) + v);
+        float xf[IN][8];
+#pragma unroll
+        for (int i = 0; i < IN; i++) unpack8(xr[i], xf[i]);
 #pragma unroll
         for (int j = 0; j < 8; j++) {
           if (j < ne) {
             float wf[8];
-            unpack8(__ldg(reinterpret_cast<const uint4*>(wg + (size_t)(e0 + j) * H) + v), wf);
+            unpack8(wr[j], wf);
 #pragma unroll
             for (int i = 0; i < IN; i++)
 #pragma unroll
@@ -586,10 +591,9 @@ extern "C" int lb_moe_push_ctas(int T) { return moe_grid(T); }
 extern "C" int lb_moe_router(const void* x, const void* wg, int T, int H, int E, int k, void* probs, void* idx, void* wts,
                              void* within, void* blk_hist, void* blk_psum, void* stream) {
   if (T <= 0 || (H % 8) || E < 1 || E > MOE_MAX_EXPERTS || k < 1 || k > MOE_MAX_TOPK || k > E) return LB_ERR_SHAPE;
-  // One token at a time where a warp has no second one, and where many experts meet rows that do not stay in L2; four elsewhere.
-  // One / four, us: T 1, H 2048, E 8 10 / 19; T 16384, H 4096, E 64 744 / 1078; T 32768, H 2048, E 64 647 / 737; T 4096, H 2048, E 8
-  // 33 / 28, E 64 235 / 150; T 16384, H 2048, E 64 412 / 363.
-  const bool one = T <= ROUTER_THREADS / 32 || (E > 8 && (long long)T * H > (32LL << 20));
+  // One token at a time where a warp has no second one, four elsewhere.  One / four, us: T 1, H 2048, E 8 16 / 19; T 16384, H 4096, E 64
+  // 766 / 402; T 32768, H 2048, E 64 625 / 369.
+  const bool one = T <= ROUTER_THREADS / 32;
   (one ? moe_router_kernel<1> : moe_router_kernel<4>)<<<lb_moe_router_blocks(T), ROUTER_THREADS, 0, (cudaStream_t)stream>>>(
       (const bf16*)x, (const bf16*)wg, T, H, E, k, (float*)probs, (int*)idx, (float*)wts, (int*)within, (int*)blk_hist,
       (float*)blk_psum);

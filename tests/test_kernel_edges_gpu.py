@@ -330,7 +330,7 @@ def test_cross_entropy_loss_rows(T, V):
                                      (8200, 4104, 9, 2)])
 def test_moe_router_tiles(T, H, E, k):
     """Ragged last block of tokens, a width that is no multiple of the column tile, one to eight passes over the experts; one token of
-    a warp at a time (up to 8 tokens, or more than 64 MB of rows) and four."""
+    a warp at a time (up to 8 tokens) and four."""
     from lightron_b200.ops import native
     x, wg, dev = _rand(T, H, seed=1), _rand(E, H, scale=H ** -0.5, seed=2), "cuda"
     lib = native.require()

@@ -5,9 +5,10 @@
 //
 // Every function takes the plain case (exact tensors or parameters, CUDA, bf16, contiguous, adjacent weights) and answers
 // NotImplemented for anything else, as also under function transforms, forward-mode derivatives, tracing and dispatch or function modes: the
-// caller then runs the autograd function in Python, which accepts, refuses and traces what it always did.  Outputs, saved tensors (and with
-// them the version checks and the saved-tensor hooks), streams and error types are the same in both forms.  Weights whose gradients go
-// straight into the optimizer's arena stay with the Python form.
+// caller then runs the autograd function in Python, which accepts, refuses and traces what it always did.  Outputs, streams, version checks and
+// error types are the same in both forms, and saved-tensor hooks see the same tensors (an input in its own shape, not flattened to rows).  What such hooks
+// give back is looked at again in backward (operand(), fused_rows()).  Weights whose gradients go straight into the optimizer's arena stay with
+// the Python form.
 #include <Python.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -102,11 +103,46 @@ std::vector<int64_t> with_last(const Tensor& x, int64_t n) {
   return s;
 }
 
+// ---- saved tensors -------------------------------------------------------------------------------
+// Saved-tensor hooks (and an assignment to a parameter's .data) may put another tensor in the place of a saved one, which a kernel would
+// read past its end.  Copies and other strides are fine; other sizes, types or devices are refused.  `last`: size of the last dimension, or -1.
+void check_saved(const Tensor& t, const Tensor& grad, at::ScalarType type, L numel, L last) {
+  TORCH_CHECK(t.defined() && t.has_storage() && t.device() == grad.device() && t.scalar_type() == type && t.numel() == numel &&
+                  (last < 0 || (t.dim() > 0 && t.size(-1) == last)),
+              "a tensor saved for backward has come back with another size, type or device");
+}
+Tensor operand(const Tensor& t, const Tensor& grad, L numel, L last, at::ScalarType type = at::kBFloat16) {
+  check_saved(t, grad, type, numel, last);
+  return t.contiguous();
+}
+// [n_i, K] matrices back to back in one buffer
+bool rows_adjacent(const Tensor* const* ws, size_t n) {
+  for (size_t i = 0; i + 1 < n; i++) {
+    const Tensor &a = *ws[i], &b = *ws[i + 1];
+    if (a.storage().data() != b.storage().data()) return false;
+    if (static_cast<const char*>(a.const_data_ptr()) + a.numel() * 2 != b.const_data_ptr()) return false;
+  }
+  return true;
+}
+// The matrix [W_0; W_1; ...] of n rows that the forward pass read, given by the first of its parts.  Parts that no longer follow one another
+// (each unpacked into memory of its own, as save_on_cpu() does) are refused, as the Python form's view of them is.
+Tensor fused_rows(const Tensor* ws, size_t nw, const Tensor& grad, L n, L K) {
+  const Tensor* p[3];
+  L rows = 0;
+  for (size_t i = 0; i < nw; i++) {
+    check_saved(ws[i], grad, at::kBFloat16, ws[i].defined() ? ws[i].numel() : -1, K);
+    TORCH_CHECK(ws[i].dim() == 2 && (nw == 1 || ws[i].is_contiguous()), "a weight saved for backward has come back with other strides");
+    rows += ws[i].size(0);
+    p[i] = &ws[i];
+  }
+  TORCH_CHECK(rows == n && rows_adjacent(p, nw), "adjacent weights saved for backward have come back as separate tensors");
+  return ws[0].contiguous();
+}
+
 // Gradients of y = x [W_0; W_1; ...]^T: dx (or undefined), then one per weight
-variable_list linear_backward(const Tensor& x, const Tensor* ws, size_t nw, const Tensor& dy, bool need_x, bool need_w) {
-  const L T = rows_of(x), K = x.size(-1);
-  L n = 0;
-  for (size_t i = 0; i < nw; i++) n += ws[i].size(0);
+variable_list linear_backward(const Tensor& saved_x, const Tensor* ws, size_t nw, const Tensor& dy, bool need_x, bool need_w) {
+  const L n = dy.size(-1), T = rows_of(dy), K = saved_x.size(-1);
+  const Tensor x = operand(saved_x, dy, T * K, K);
   variable_list out(1 + nw);
   Gemms g;
   Tensor dw;
@@ -114,9 +150,11 @@ variable_list linear_backward(const Tensor& x, const Tensor* ws, size_t nw, cons
     dw = empty({n, K}, x);
     g.add(dy, x, dw, n, K, T, true, true);
   }
+  Tensor w;
   if (need_x) {
+    w = fused_rows(ws, nw, dy, n, K);
     out[0] = at::empty(x.sizes(), x.options());
-    g.add(dy, ws[0], out[0], T, K, n, false, true);
+    g.add(dy, w, out[0], T, K, n, false, true);
   }
   if (g.n) g.run();
   L off = 0;
@@ -161,9 +199,10 @@ struct SwiGLUMLP : Function<SwiGLUMLP> {
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     const variable_list s = ctx->get_saved_variables();
-    const Tensor &x = s[0], &gu = s[1], &h = s[2], &w2 = s[5];
-    const L T = rows_of(x), I = h.size(1), H = w2.size(0);
+    const Tensor& x = s[0];
     const Tensor dy = grads[0].contiguous();
+    const L T = rows_of(dy), I = s[2].size(-1), H = dy.size(-1);
+    const Tensor gu = operand(s[1], dy, T * 2 * I, 2 * I), h = operand(s[2], dy, T * I, I), w2 = operand(s[5], dy, H * I, I);
     Tensor dgu = at::empty(gu.sizes(), gu.options()), dw2;
     Gemms g;
     if (ctx->needs_input_grad(3)) {
@@ -179,8 +218,9 @@ struct SwiGLUMLP : Function<SwiGLUMLP> {
 };
 
 // ---- RMSNorm -------------------------------------------------------------------------------------
-variable_list rmsnorm_backward(const Tensor& src, const Tensor& w, const Tensor& rstd, const Tensor* dh, const Tensor& dy) {
-  const int rows = (int)rows_of(src), cols = (int)src.size(-1), nblk = api.lb_rmsnorm_bwd_blocks(rows, cols);
+variable_list rmsnorm_backward(const variable_list& saved, const Tensor* dh, const Tensor& dy) {
+  const int rows = (int)rows_of(dy), cols = (int)dy.size(-1), nblk = api.lb_rmsnorm_bwd_blocks(rows, cols);
+  const Tensor src = operand(saved[0], dy, dy.numel(), cols), w = operand(saved[1], dy, cols, cols), rstd = operand(saved[2], dy, rows, rows, at::kFloat);
   const Tensor dyc = dy.contiguous(), dhc = dh ? dh->contiguous() : Tensor();
   Tensor partial = empty_f32({nblk, cols}, src), dx = at::empty(src.sizes(), src.options()), dw = at::empty(w.sizes(), w.options());
   LB_CALL(lb_rmsnorm_bwd, dyc.const_data_ptr(), src.const_data_ptr(), w.const_data_ptr(), rstd.const_data_ptr(),
@@ -197,7 +237,7 @@ struct RMSNorm : Function<RMSNorm> {
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     const variable_list s = ctx->get_saved_variables();
-    variable_list r = rmsnorm_backward(s[0], s[1], s[2], nullptr, grads[0]);
+    variable_list r = rmsnorm_backward(s, nullptr, grads[0]);
     r.push_back(Tensor());
     return r;
   }
@@ -212,7 +252,7 @@ struct AddRMSNorm : Function<AddRMSNorm> {
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     const variable_list s = ctx->get_saved_variables();
-    const variable_list r = rmsnorm_backward(s[0], s[1], s[2], &grads[0], grads[1]);
+    const variable_list r = rmsnorm_backward(s, &grads[0], grads[1]);
     return {r[0], r[0], r[1], Tensor()};
   }
 };
@@ -232,9 +272,10 @@ void attention_forward(const Heads& q, const Heads& k, const Heads& v, const Ten
   LB_CALL(lb_flash_fwd_tc, q.p, k.p, v.p, o.mutable_data_ptr(), lse.mutable_data_ptr(), m.B, m.Sq, m.Sk, m.hq, m.hkv, m.d, q.ts, k.ts, v.ts,
           (L)m.hq * m.d, m.scale, m.causal, stream());
 }
-void attention_backward(const Heads& q, const Heads& k, const Heads& v, const Tensor& o, const Tensor& lse, const Heads& dout, W dq, W dk, W dv,
-                        L dq_ts, L dk_ts, L dv_ts, const AttnDims& m) {
-  const L o_ts = (L)m.hq * m.d;
+void attention_backward(const Heads& q, const Heads& k, const Heads& v, const Tensor& saved_o, const Tensor& saved_lse, const Tensor& grad,
+                        const Heads& dout, W dq, W dk, W dv, L dq_ts, L dk_ts, L dv_ts, const AttnDims& m) {
+  const L o_ts = (L)m.hq * m.d, rows = (L)m.B * m.Sq;
+  const Tensor o = operand(saved_o, grad, rows * o_ts, -1), lse = operand(saved_lse, grad, rows * m.hq, m.Sq, at::kFloat);
   if (env_is_tc("LIGHTRON_FA_BWD")) {
     const L bytes = api.lb_flash_bwd_ws_bytes(m.B, m.Sq, m.hq, m.d);
     Tensor ws = at::empty({bytes}, o.options().dtype(at::kByte));
@@ -263,10 +304,16 @@ struct Attention : Function<Attention> {
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     const variable_list s = ctx->get_saved_variables();
-    const Tensor q = fix_layout(s[0]), k = fix_layout(s[1]), v = fix_layout(s[2]), dout = fix_layout(grads[0]);
+    const Tensor& g = grads[0];
+    check_saved(s[0], g, at::kBFloat16, g.numel(), g.size(3));
+    for (int i = 1; i < 3; i++) check_saved(s[i], g, at::kBFloat16, s[1].defined() ? s[1].numel() : -1, g.size(3));
+    TORCH_CHECK(s[0].sizes().equals(g.sizes()) && s[1].dim() == 4 && s[2].sizes().equals(s[1].sizes()) && s[1].size(0) == g.size(0) &&
+                    s[1].numel() > 0 && g.size(2) % s[1].size(2) == 0,
+                "q, k or v saved for backward has come back with another shape");
+    const Tensor q = fix_layout(s[0]), k = fix_layout(s[1]), v = fix_layout(s[2]), dout = fix_layout(g);
     const AttnDims m = dims_of(q, k, ctx->saved_data["causal"].toBool(), ctx->saved_data["scale"].toDouble());
     Tensor dq = empty(q.sizes(), q), dk = empty(k.sizes(), k), dv = empty(v.sizes(), v);
-    attention_backward({q.const_data_ptr(), q.stride(1)}, {k.const_data_ptr(), k.stride(1)}, {v.const_data_ptr(), v.stride(1)}, s[3], s[4],
+    attention_backward({q.const_data_ptr(), q.stride(1)}, {k.const_data_ptr(), k.stride(1)}, {v.const_data_ptr(), v.stride(1)}, s[3], s[4], g,
                        {dout.const_data_ptr(), dout.stride(1)}, dq.mutable_data_ptr(), dk.mutable_data_ptr(), dv.mutable_data_ptr(), dq.stride(1),
                        dk.stride(1), dv.stride(1), m);
     return {dq, dk, dv, Tensor(), Tensor()};
@@ -290,7 +337,7 @@ struct RopeAttention : Function<RopeAttention> {
     const AttnDims m{(int)B, (int)S, (int)S, (int)hq, (int)hkv, (int)d, 1, (float)scale};
     attention_forward({at_head(qkv, 0, d), row}, {at_head(qkv, hq, d), row}, {at_head(qkv, hq + hkv, d), row}, o, lse, m);
     ctx->save_for_backward({qkv, o, lse, cos, sin, pos});
-    ctx->saved_data["dims"] = std::vector<int64_t>(dims.v, dims.v + 5);
+    ctx->saved_data["dims"] = std::vector<int64_t>{B, S, hq, hkv, d, cos.numel(), sin.numel()};
     ctx->saved_data["scale"] = scale;
     return o;
   }
@@ -299,12 +346,14 @@ struct RopeAttention : Function<RopeAttention> {
     const std::vector<int64_t> dims = ctx->saved_data["dims"].toIntVector();
     const L B = dims[0], S = dims[1], hq = dims[2], hkv = dims[3], d = dims[4], row = (hq + 2 * hkv) * d;
     const AttnDims m{(int)B, (int)S, (int)S, (int)hq, (int)hkv, (int)d, 1, (float)ctx->saved_data["scale"].toDouble()};
-    const Tensor& qkv = s[0];
-    const Tensor dout = fix_layout(grads[0].reshape({B, S, hq, d}));
+    const Tensor& g = grads[0];
+    const Tensor qkv = operand(s[0], g, B * S * row, row), cos = operand(s[3], g, dims[5], d / 2, at::kFloat), sin = operand(s[4], g, dims[6], d / 2, at::kFloat);
+    const Tensor pos = s[5].defined() ? operand(s[5], g, S, -1, at::kInt) : Tensor();
+    const Tensor dout = fix_layout(g.reshape({B, S, hq, d}));
     Tensor dqkv = at::empty(qkv.sizes(), qkv.options());
-    attention_backward({at_head(qkv, 0, d), row}, {at_head(qkv, hq, d), row}, {at_head(qkv, hq + hkv, d), row}, s[1], s[2],
+    attention_backward({at_head(qkv, 0, d), row}, {at_head(qkv, hq, d), row}, {at_head(qkv, hq + hkv, d), row}, s[1], s[2], g,
                        {dout.const_data_ptr(), dout.stride(1)}, at_head(dqkv, 0, d), at_head(dqkv, hq, d), at_head(dqkv, hq + hkv, d), row, row, row, m);
-    rope(dqkv, s[3], s[4], s[5], S, hq + hkv, d, row, 1);
+    rope(dqkv, cos, sin, pos, S, hq + hkv, d, row, 1);
     return {dqkv, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
@@ -323,8 +372,8 @@ struct Embedding : Function<Embedding> {
     return out;
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
-    const Tensor tok = ctx->get_saved_variables()[0], dy = grads[0].contiguous();
     const std::vector<int64_t> s = ctx->saved_data["shape"].toIntVector();
+    const Tensor dy = grads[0].contiguous(), tok = operand(ctx->get_saved_variables()[0], dy, dy.numel() / s[1], -1, at::kLong);
     Tensor dw = empty({s[0], s[1]}, dy);
     LB_CALL(lb_clear, dw.mutable_data_ptr(), (L)dw.nbytes(), stream());
     LB_CALL(lb_embedding_bwd, tok.const_data_ptr(), dy.const_data_ptr(), dw.mutable_data_ptr(), (int)tok.numel(), (int)s[1], (int)s[2],
@@ -342,7 +391,7 @@ struct CrossEntropy : Function<CrossEntropy> {
     LB_CALL(lb_ce_loss, mx.const_data_ptr(), se.mutable_data_ptr(), tl.const_data_ptr(), tgt.const_data_ptr(), lse.mutable_data_ptr(),
             loss.mutable_data_ptr(), (int)T, inv_n(n_valid), (int)ignore, stream());
     ctx->save_for_backward({logits, tgt, lse});
-    ctx->saved_data["meta"] = std::vector<int64_t>{v0, n_valid, ignore};
+    ctx->saved_data["meta"] = std::vector<int64_t>{v0, n_valid, ignore, T, V};
     return loss;
   }
   static float inv_n(int64_t n) { return (float)(1.0 / (double)std::max<int64_t>(n, 1)); }
@@ -350,10 +399,15 @@ struct CrossEntropy : Function<CrossEntropy> {
     const variable_list s = ctx->get_saved_variables();
     const std::vector<int64_t> m = ctx->saved_data["meta"].toIntVector();
     const Tensor dl = grads[0].to(at::kFloat).reshape({1}).contiguous();         // read on the device: no host sync
+    const L T = m[3], V = m[4];
+    check_saved(s[0], grads[0], at::kBFloat16, T * V, V);
+    TORCH_CHECK(s[0].dim() == 2, "logits saved for backward have come back with another shape");
+    const Tensor logits = s[0].stride(1) == 1 ? s[0] : s[0].contiguous();
+    const Tensor tgt = operand(s[1], grads[0], T, T, at::kLong), lse = operand(s[2], grads[0], T, T, at::kFloat);
     // the gradient overwrites the logits, which are dead after the loss
-    LB_CALL(lb_ce_grad, s[0].const_data_ptr(), s[1].const_data_ptr(), s[2].const_data_ptr(), s[0].mutable_data_ptr(), dl.const_data_ptr(),
-            (int)s[0].size(0), (int)s[0].size(1), s[0].stride(0), (int)m[0], inv_n(m[1]), (int)m[2], stream());
-    return {s[0], Tensor(), Tensor(), Tensor(), Tensor()};
+    LB_CALL(lb_ce_grad, logits.const_data_ptr(), tgt.const_data_ptr(), lse.const_data_ptr(), logits.mutable_data_ptr(), dl.const_data_ptr(), (int)T,
+            (int)V, logits.stride(0), (int)m[0], inv_n(m[1]), (int)m[2], stream());
+    return {logits, Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -384,15 +438,6 @@ bool in_arena(PyObject* o, const Tensor& w) {
   const int yes = PyObject_IsTrue(a);
   Py_DECREF(a);
   return yes != 0;
-}
-// [n_i, K] matrices back to back in one buffer
-bool rows_adjacent(const Tensor* const* ws, size_t n) {
-  for (size_t i = 0; i + 1 < n; i++) {
-    const Tensor &a = *ws[i], &b = *ws[i + 1];
-    if (a.storage().data() != b.storage().data()) return false;
-    if (static_cast<const char*>(a.const_data_ptr()) + a.numel() * 2 != b.const_data_ptr()) return false;
-  }
-  return true;
 }
 bool weight_ok(const Tensor* w, int64_t K) {
   return plain(w) && w->dim() == 2 && w->size(1) == K && w->size(0) % 8 == 0 && w->size(0) <= INT_MAX;

@@ -239,6 +239,101 @@ def test_observers_see_what_they_did(monkeypatch):
     assert host.launches() == n0
 
 
+def _strided(t):
+    """The same values two elements apart."""
+    buf = torch.zeros(*t.shape, 2, dtype=t.dtype, device=t.device)
+    buf[..., 0] = t
+    return buf[..., 0]
+
+
+def _op_cases():
+    """name -> (op, its differentiable inputs, its output's shape)"""
+    cos, sin = _tables(48, 64)
+    pos = torch.arange(48, device=DEV, dtype=torch.int32).flip(0)
+    tok, tgt = torch.arange(24, device=DEV) % 16, torch.arange(24, device=DEV)
+    qkv = lambda: [_t(2, 24, h, 64, seed=i) for i, h in enumerate((4, 2, 2))]
+    return {
+        "linear": (OF.linear, lambda: [_t(24, 64, seed=1), _t(16, 64, seed=2)], (24, 16)),
+        "rmsnorm": (lambda x, w: OF.rmsnorm(x, w, 1e-5), lambda: [_t(24, 64, seed=1), _t(64, seed=2)], (24, 64)),
+        "add_rmsnorm": (lambda x, r, w: OF.add_rmsnorm(x, r, w, 1e-5)[1], lambda: [_t(24, 64, seed=1), _t(24, 64, seed=2), _t(64, seed=3)], (24, 64)),
+        "attention": (OF.flash_attention, qkv, (2, 24, 4, 64)),
+        "rope_attention": (lambda t: OF.rope_attention_qkv(t * 1, cos, sin, pos, 1, 48, 4, 2, 64), lambda: [_t(48, 512, seed=1)], (48, 256)),
+        "embedding": (lambda w: OF.embedding(tok, w), lambda: [_t(32, 64, seed=1)], (24, 64)),
+        "cross_entropy": (lambda x: OF.cross_entropy(x * 1, tgt, n_valid_total=24), lambda: [_t(24, 64, seed=1)], ()),
+    }
+
+
+@pytest.mark.parametrize("name", ["linear", "rmsnorm", "add_rmsnorm", "attention", "rope_attention", "embedding", "cross_entropy"])
+def test_saved_tensors_come_back_otherwise(name):
+    """A copy, and a copy with other strides: the same gradients (attention: dQ is summed with atomics).  Other sizes or types, and batched
+    gradients, which have no memory: refused."""
+    op, make, out = _op_cases()[name]
+    host = native.host_ops()
+    dy = _t(*out, seed=9, grad=False) if out else torch.ones((), device=DEV)
+    n0 = host.launches()
+
+    def grads(unpack):
+        ins = make()
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            y = op(*ins)
+        return torch.autograd.grad(y, ins, dy)
+    want = grads(lambda t: t)
+    for unpack in (lambda t: t.clone(), lambda t: _strided(t)):
+        for g, w in zip(grads(unpack), want):
+            _same(g, w, tol=2e-3 if "attention" in name else None)
+    ins = make()
+    with torch.autograd.graph.save_on_cpu():
+        y = op(*ins)
+    for g, w in zip(torch.autograd.grad(y, ins, dy), want):
+        _same(g, w, tol=2e-3 if "attention" in name else None)
+    for unpack in (lambda t: t[:-1], lambda t: t.double(), lambda t: t.cpu()):
+        with pytest.raises(RuntimeError, match="saved for backward"):
+            grads(unpack)
+    ins = make()
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad(op(*ins), ins, dy.expand(3, *dy.shape), is_grads_batched=True)
+    torch.cuda.synchronize()
+    assert host.launches() > n0
+
+
+@pytest.mark.parametrize("op,n", [(OF.linear, 2), (OF.linear, 3), (OF.swiglu_mlp, 3)])
+def test_adjacent_weights_come_back_apart(monkeypatch, op, n):
+    """The data gradient reads the adjacent weights as one matrix: refused where the hooks give each its own memory, in either form.  What
+    does not need it, and weights that are still adjacent (recomputation), give the same gradients."""
+    from torch.utils.checkpoint import checkpoint
+
+    def make(need_x=True):
+        buf = _t(n * 40, 64, seed=2, scale=0.1, grad=False)
+        ws = [buf[i * 40:i * 40 + 40].detach().requires_grad_() for i in range(n if op is OF.linear else 2)]
+        if op is OF.swiglu_mlp:
+            ws.append(_t(64, 40, seed=3, scale=0.1))
+        return [_t(37, 64, seed=1).requires_grad_(need_x), *ws]
+    dy = _t(*op(*make()).shape, seed=4, grad=False)
+
+    def grads(need_x, ctx, call=op):
+        ins = make(need_x)
+        with ctx:
+            y = call(*ins)
+        return torch.autograd.grad(y, ins if need_x else ins[1:], dy)
+    import contextlib
+    want = grads(True, contextlib.nullcontext())
+    assert native.host_ops() is not None
+    for g, w in zip(grads(True, contextlib.nullcontext(), lambda *a: checkpoint(op, *a, use_reentrant=False)), want):
+        _same(g, w)
+    apart = (torch.autograd.graph.save_on_cpu, lambda: torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t.clone()))
+    for ctx in apart:
+        with pytest.raises(RuntimeError, match="separate tensors"):
+            grads(True, ctx())
+        for g, w in zip(grads(False, ctx()), want[1:]):
+            _same(g, w)
+    with monkeypatch.context() as m:
+        m.setattr(native, "_HOST", None)
+        for ctx in apart:
+            with pytest.raises(RuntimeError, match="out of bounds for storage"):
+                grads(True, ctx())
+    torch.cuda.synchronize()
+
+
 def test_threads_and_streams():
     x, w = _t(64, 512), _t(512, 512, seed=1, scale=0.05)
     want = OF.linear(x.detach(), w.detach())

@@ -437,6 +437,7 @@ bool in_arena(PyObject* o, const Tensor& w) {
   if (!a) { PyErr_Clear(); return false; }
   const int yes = PyObject_IsTrue(a);
   Py_DECREF(a);
+  if (yes < 0) PyErr_Clear();                    // the Python form asks again, and raises
   return yes != 0;
 }
 bool weight_ok(const Tensor* w, int64_t K) {

@@ -189,6 +189,17 @@ def test_what_is_not_plain_goes_the_old_way(monkeypatch):
     assert w.grad.abs().sum() > 0
 
 
+def test_a_mark_without_truth_value_goes_the_old_way(monkeypatch):
+    """The attribute that marks a weight of the arena may be anything: the node declines, without an error of its own."""
+    class Unclear:
+        def __bool__(self):
+            raise ValueError("neither")
+    w = _t(16, 64, seed=2)
+    w._lb_direct_grad = Unclear()
+    new, old = _both(monkeypatch, lambda: OF.linear(_t(8, 64), w).detach(), taken=False)
+    assert torch.equal(new, old)
+
+
 def test_errors_are_the_same():
     with pytest.raises(native.NativeError, match="lb_rmsnorm_fwd failed: unsupported shape"):
         OF.rmsnorm(_t(4, 12), _t(12), 1e-5)

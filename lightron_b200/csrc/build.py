@@ -29,6 +29,19 @@ def sources():
     return sorted(glob.glob(os.path.join(HERE, "*.cu")))
 
 
+def host_tag() -> str:
+    """What ``_host_ops.so`` is built against, as it is written into the file: classes of another torch have another layout."""
+    import torch
+    return f"lightron_b200 host ops: torch {torch.__version__}, python {sys.version_info[0]}.{sys.version_info[1]}."
+
+
+def host_built_for_this_torch() -> bool:
+    if not os.path.exists(HOST_LIB):
+        return False
+    with open(HOST_LIB, "rb") as f:
+        return host_tag().encode() in f.read()
+
+
 def host_command(out: str) -> list:
     """Compiler call for the extension module of the autograd nodes."""
     import sysconfig
@@ -37,12 +50,12 @@ def host_command(out: str) -> list:
     inc = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
            os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")]
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in inc), HOST_SRC, "-o", out,
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DLB_BUILT_FOR="{host_tag()}"', *(f"-I{d}" for d in inc), HOST_SRC, "-o", out,
             f"-L{os.path.join(base, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python"]
 
 
 def needs_build() -> bool:
-    if not (os.path.exists(LIB) and os.path.exists(HOST_LIB)):
+    if not os.path.exists(LIB) or not host_built_for_this_torch():
         return True
     t = min(os.path.getmtime(LIB), os.path.getmtime(HOST_LIB))
     deps = sources() + [HOST_SRC] + glob.glob(os.path.join(HERE, "*.cuh")) + glob.glob(os.path.join(HERE, "*.h"))

@@ -614,6 +614,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host_ops", nullptr, -1, methods, 
 
 }  // namespace
 
+// Read from the file by csrc/build.py before the module is loaded.
+extern "C" __attribute__((used, visibility("default"))) const char lb_host_ops_built_for[] = LB_BUILT_FOR;
+
 PyMODINIT_FUNC PyInit__host_ops() {
   direct_grad = PyUnicode_InternFromString("_lb_direct_grad");
   return direct_grad ? PyModule_Create(&module) : nullptr;

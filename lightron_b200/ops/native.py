@@ -252,8 +252,11 @@ def _load_host_ops():
     import importlib.machinery
     import importlib.util
     import warnings
-    path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc", "_host_ops.so")
+    from ..csrc import build
+    path = build.HOST_LIB
     try:
+        if os.path.exists(path) and not build.host_built_for_this_torch():
+            raise ImportError(f"not built for torch {torch.__version__}")
         loader = importlib.machinery.ExtensionFileLoader("_host_ops", path)
         mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_host_ops", path, loader=loader))
         loader.exec_module(mod)

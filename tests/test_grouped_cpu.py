@@ -266,3 +266,15 @@ def test_host_code_under_address_and_ub_sanitizers(tmp_path):
                UBSAN_OPTIONS="halt_on_error=1:print_stacktrace=1")
     r = subprocess.run([sys.executable, str(script), lib], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "SANITIZED_HOST_OK" in r.stdout, r.stdout[-1500:] + r.stderr[-3000:]
+
+
+def test_host_module_of_another_torch_is_not_loaded(monkeypatch):
+    """The module of the autograd nodes names the torch it was built against: for another one it is rebuilt, and never loaded."""
+    from lightron_b200.csrc import build
+    if not os.path.exists(build.HOST_LIB):
+        pytest.skip("native library not built")
+    assert build.host_built_for_this_torch()
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + "x")
+    assert build.needs_build() and not build.host_built_for_this_torch()
+    with pytest.warns(UserWarning, match="not built for torch"):
+        assert native._load_host_ops() is None

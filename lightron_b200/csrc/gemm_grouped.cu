@@ -681,9 +681,11 @@ struct Schedule {
 // Cache of uploaded schedules, keyed by (device, M, N, K of every problem).  A training run uses a
 // few dozen shape sets; callers whose row counts change from call to call (expert-parallel MoE)
 // use lb_gemm_ragged instead, which takes the counts from device memory and needs no schedule.
-// The cache is still bounded: beyond MAX_SCHEDULES entries the least recently used one is freed.
-constexpr size_t MAX_SCHEDULES = 128;
+// The cache is still bounded: beyond MAX_SCHEDULES entries the least recently used one is freed.  Entries of the split form are only a number
+// on the host: they have a limit of their own and push out no uploaded schedule, which takes allocations and synchronous copies to make again.
+constexpr int MAX_SCHEDULES = 128, MAX_SPLITS = 512;
 std::map<std::vector<int>, Schedule> g_schedules;
+int g_cached[2] = {0, 0};      // entries with a schedule, entries of the split form
 unsigned long long g_sched_clock = 0;
 std::mutex g_sched_mutex;
 int g_sms = 0;
@@ -828,7 +830,7 @@ extern "C" int lb_gemm_grouped_status(void* out) {
 // Number of schedules currently cached (never more than MAX_SCHEDULES).
 extern "C" int lb_gemm_grouped_cached() {
   std::lock_guard<std::mutex> lock(g_sched_mutex);
-  return (int)g_schedules.size();
+  return g_cached[0];
 }
 
 namespace {
@@ -931,18 +933,22 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
     std::lock_guard<std::mutex> lock(g_sched_mutex);
     auto it = g_schedules.find(key);
     if (it == g_schedules.end()) {
-      if (g_schedules.size() >= MAX_SCHEDULES) {
-        // evict the least recently used entry; cudaFree waits for kernels that may still read it
-        auto victim = g_schedules.begin();
-        for (auto j = g_schedules.begin(); j != g_schedules.end(); ++j)
-          if (j->second.last_use < victim->second.last_use) victim = j;
-        cudaFree(victim->second.d_offsets);
-        cudaFree(victim->second.d_items);
-        g_schedules.erase(victim);
-      }
       Schedule s;
       int rc = build_schedule(gp.prob, n, g_sms, &s);
       if (rc) return rc;
+      const bool split = s.split > 0;
+      if (++g_cached[split] > (split ? MAX_SPLITS : MAX_SCHEDULES)) {
+        // evict the least recently used entry of its kind; cudaFree waits for kernels that may still read it
+        auto victim = g_schedules.end();
+        for (auto j = g_schedules.begin(); j != g_schedules.end(); ++j)
+          if ((j->second.split > 0) == split && (victim == g_schedules.end() || j->second.last_use < victim->second.last_use)) victim = j;
+        if (!split) {
+          cudaFree(victim->second.d_offsets);
+          cudaFree(victim->second.d_items);
+        }
+        g_schedules.erase(victim);
+        g_cached[split]--;
+      }
       it = g_schedules.emplace(key, s).first;
     }
     it->second.last_use = ++g_sched_clock;

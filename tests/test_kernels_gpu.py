@@ -255,26 +255,46 @@ def test_peer_copy_kernel_local(mode, nbytes, ctas):
 def test_grouped_gemm_schedule_cache_stays_bounded():
     """Callers whose shapes change from call to call must not grow the schedule cache (or device memory)
     without bound: sweeps over 150 different row counts leave at most the cache's capacity of entries behind,
-    and a second sweep (every entry evicted and rebuilt) does not cost device memory."""
+    and a second sweep (every entry evicted and rebuilt) does not cost device memory.  Launches of the split form, which
+    has no schedule, push none out."""
+    import ctypes
     from lightron_b200.ops import functional as OF, native
     lib = native.require()
     a = _rand(1208, 64, seed=1)
     b = _rand(64, 64, seed=2)
-    out = torch.empty(1208, 64, device="cuda", dtype=torch.bfloat16)
+    outs = [torch.empty(1208, 64, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
 
-    def sweep(check):
+    def parts(n, M):
+        IA = ctypes.c_int * n
+        return lib.lb_gemm_grouped_parts(n, IA(*[M] * n), IA(*[64] * n), IA(*[64] * n), native.sm_count())
+
+    def sweep(n, check=False):
         for i, M in enumerate(range(8, 1208, 8)):                  # 150 shape sets
-            OF.gemm_grouped([(a[:M], b, False, False, out[:M], False)])
+            assert (parts(n, M) == 0) == (n == 3)                  # three problems: the list form, which uploads a schedule
+            OF.gemm_grouped([(a[:M], b, False, False, out[:M], False) for out in outs[:n]])
             if check and i % 37 == 0:
                 want = a[:M].float() @ b.float().t()
-                assert _rel_err(out[:M], want) < 1e-2, M
+                assert all(_rel_err(out[:M], want) < 1e-2 for out in outs[:n]), M
         torch.cuda.synchronize()
 
-    sweep(True)                                                    # also pays every one-time allocation (library handles, ...)
-    assert lib.lb_gemm_grouped_cached() <= 128
+    sweep(3, True)                                                 # also pays every one-time allocation (library handles, ...)
+    assert lib.lb_gemm_grouped_cached() == 128
     free1 = torch.cuda.mem_get_info()[0]
-    sweep(False)
-    assert lib.lb_gemm_grouped_cached() <= 128
+    sweep(3)
+    assert lib.lb_gemm_grouped_cached() == 128
+    assert free1 - torch.cuda.mem_get_info()[0] < (8 << 20)
+    for n in (1, 2):                                               # 300 launches in the split form: the schedules stay
+        sweep(n, True)
+    assert lib.lb_gemm_grouped_cached() == 128
+    for out in outs:
+        out.zero_()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):                                  # (a schedule that has to be uploaded again could not be captured)
+        OF.gemm_grouped([(a[:1200], b, False, False, out[:1200], False) for out in outs])
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(_rel_err(out[:1200], a[:1200].float() @ b.float().t()) < 1e-2 for out in outs)
+    del graph
     assert free1 - torch.cuda.mem_get_info()[0] < (8 << 20)
     assert _gemm_status()[0] == 0
 

@@ -57,15 +57,10 @@ def _grads(out, inputs, dy):
     return torch.autograd.grad(outs, need, dy, allow_unused=True)
 
 
-@pytest.mark.parametrize("shape,widths", [((1, 8), (8,)), ((2, 24, 64), (16, 8, 8)), ((300, 256), (512,)), ((8, 200, 512), (512, 256, 256))])
+@pytest.mark.parametrize("shape,widths", [((1, 8), (8,)), ((2, 24, 64), (16, 8, 8)), ((300, 256), (512,)), ((70, 264), (512, 136, 136)), ((8, 200, 512), (512, 256, 256))])
 @pytest.mark.parametrize("need", [(True, True), (True, False), (False, True), (False, False)])
 @pytest.mark.parametrize("form", ["dense", "expanded", "transposed"])
 def test_linear(monkeypatch, shape, widths, need, form):
-    rows = 1
-    for s in shape[:-1]:
-        rows *= s
-    if rows % 8 and need[1]:
-        need = (need[0], False)             # the weight gradient wants 16-byte rows
     def fn():
         x = _t(*shape, seed=1, grad=need[0])
         buf = _t(sum(widths), shape[-1], seed=2, scale=0.1, grad=False)
@@ -81,7 +76,7 @@ def test_linear(monkeypatch, shape, widths, need, form):
         _same(a, b)
 
 
-@pytest.mark.parametrize("T,K,I", [(8, 8, 8), (104, 264, 136), (512, 512, 1408)])
+@pytest.mark.parametrize("T,K,I", [(1, 8, 8), (8, 8, 8), (37, 264, 136), (104, 264, 136), (512, 512, 1408), (1531, 512, 1408)])
 @pytest.mark.parametrize("need", [(1, 1, 1, 1), (1, 0, 0, 0), (0, 0, 0, 1), (0, 1, 1, 0), (0, 0, 0, 0)])
 def test_swiglu_mlp(monkeypatch, T, K, I, need):
     def fn():
@@ -220,9 +215,9 @@ def test_observers_see_what_they_did(monkeypatch):
     packed = []
     with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t.cpu(), lambda t: t.to(DEV)):
         y = OF.linear(x, w)
-    assert len(packed) == 2
+    assert packed == [x.shape, w.shape]
     y.sum().backward()
-    assert torch.isfinite(x.grad).all()
+    assert torch.equal(x.grad, torch.autograd.grad(OF.linear(x, w).sum(), x)[0])
 
     from torch.utils._python_dispatch import TorchDispatchMode
 

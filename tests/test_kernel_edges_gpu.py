@@ -163,35 +163,42 @@ def test_attention_bad_scores_stay_in_their_rows(d, bad):
 # ---- GEMM --------------------------------------------------------------------------------------------
 
 
-def _ctas_per_tile(*problems):
-    """1 or 2: the form of the grouped GEMM that these (M, N, K) are launched in on this device."""
+def _form(*problems):
+    """(parts, CTAs per tile) of a grouped launch of these (M, N, K) on this device: K in `parts` parts in the split form, or 0 and the
+    list form with 1 or 2 CTAs per tile."""
     import ctypes
     from lightron_b200.ops import native
-    IA = ctypes.c_int * len(problems)
-    return native.require().lb_gemm_grouped_ctas_per_tile(len(problems), *(IA(*[p[i] for p in problems]) for i in range(3)), native.sm_count())
+    lib, IA = native.require(), ctypes.c_int * len(problems)
+    args = (len(problems), *(IA(*[p[i] for p in problems]) for i in range(3)), native.sm_count())
+    parts = lib.lb_gemm_grouped_parts(*args)
+    return parts, 0 if parts else lib.lb_gemm_grouped_ctas_per_tile(*args)
 
 
-@pytest.mark.parametrize("M,N,K,ctas", [
-    (9000, 2312, 1032, 2),                   # several tiles per pair, the last ones ragged in rows, columns and depth
-    (4225, 4104, 2056, 2),
-    (130, 520, 4104, 2), (1, 8, 4096, 2),    # one tile: the second CTA's rows beyond the matrix
-    (5000, 2312, 72, 1), (4096, 2304, 512, 1), (4225, 4104, 200, 1), (130, 520, 1032, 1), (1, 8, 8, 1),
+@pytest.mark.parametrize("M,N,K,n,form", [
+    (9000, 2312, 1032, 1, (0, 2)),           # several tiles per pair, the last ones ragged in rows, columns and depth
+    (4225, 4104, 2056, 1, (0, 2)),
+    (5000, 2312, 72, 1, (0, 1)), (4096, 2304, 512, 1, (0, 1)), (4225, 4104, 200, 1, (0, 1)),
+    # three problems are never split.  One tile each: the second CTA's rows beyond the matrix; then single CTAs
+    (130, 520, 4104, 3, (0, 2)), (1, 8, 4096, 3, (0, 2)), (130, 520, 1032, 3, (0, 1)), (1, 8, 8, 3, (0, 1)),
+    # the same alone
+    (130, 520, 4104, 1, (4, 0)), (1, 8, 4096, 1, (4, 0)), (130, 520, 1032, 1, (4, 0)), (1, 8, 8, 1, (1, 0)),
 ])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
-def test_gemm_pair_tiles(M, N, K, ctas, a_mn, b_mn):
-    """Pairs of CTAs and single ones, plain and accumulating; which form ran is part of the test."""
+def test_gemm_forms(M, N, K, n, form, a_mn, b_mn):
+    """Pairs of CTAs, single ones and the split form, plain and accumulating; which form ran is part of the test."""
     from lightron_b200.ops import functional as OF
     if a_mn and M % 8:
         M = M // 8 * 8 + 8
-    assert _ctas_per_tile((M, N, K)) == ctas
+    assert _form(*[(M, N, K)] * n) == form
     a, b, c0 = _rand(M, K, seed=1), _rand(N, K, seed=2), _rand(M, N, seed=3)
     ops = (a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b)
     want = a.double() @ b.double().t()
-    assert _rel(OF.gemm(*ops, a_mn=a_mn, b_mn=b_mn), want) < 5e-3
-    out = c0.clone()
-    OF.gemm_grouped([(*ops, a_mn, b_mn, out, True)])
-    _status_ok()
-    assert _rel(out, want + c0.double()) < 5e-3
+    for acc in (False, True):
+        outs = [c0.clone() for _ in range(n)]
+        OF.gemm_grouped([(*ops, a_mn, b_mn, out, acc) for out in outs])
+        _status_ok()
+        for out in outs:
+            assert _rel(out, want + c0.double() if acc else want) < 5e-3
 
 
 def _gemm_split(ks, a, b, a_mn, b_mn, out, accumulate, epi=0, c2=None, half=0):
@@ -211,11 +218,16 @@ def _gemm_split(ks, a, b, a_mn, b_mn, out, accumulate, epi=0, c2=None, half=0):
     (72, 200, 328),          # fewer rows than a tile, loaded without the rest
     (136, 64, 1032),         # a second tile of 8 rows, one column tile, the last k-block ragged
     (1000, 776, 256),        # as many k-blocks as parts
+    (133, 72, 261),          # no multiple of 8 in rows or depth (rows of the operands on 16 bytes all the same)
+    (1, 8, 193),             # one row, one element in the last k-block
 ])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
 def test_gemm_split_tiles(ks, M, N, K, a_mn, b_mn):
     """Parts of K summed over a cluster; nothing is written behind the last row."""
-    a, b, c0 = _rand(M, K, seed=1), _rand(N, K, seed=2), _rand(M, N, seed=3)
+    if a_mn and M % 8:
+        M = M // 8 * 8 + 8
+    pad = (K + 7) // 8 * 8
+    a, b, c0 = _rand(M, pad, seed=1)[:, :K], _rand(N, pad, seed=2)[:, :K], _rand(M, N, seed=3)
     ops = (a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b)
     want = a.double() @ b.double().t()
     buf = torch.full((M + 8, N), 7.0, dtype=torch.bfloat16, device="cuda")
@@ -242,12 +254,13 @@ def test_gemm_split_activation(ks, T, K, I):
     assert _rel(gu, want) < 5e-3 and _rel(h, act.detach()) < 5e-3 and _rel(dgu, g64.grad) < 1e-2
 
 
-@pytest.mark.parametrize("T,K,I,ctas", [(300, 4096, 264, 2), (2100, 1032, 2312, 2), (4000, 256, 1288, 1), (70, 512, 264, 1)])
-def test_swiglu_mlp_pair_tiles(T, K, I, ctas):
-    """The activation in the epilogue of pairs, whose peer loads the up rows, and of single CTAs; ragged in every size."""
+@pytest.mark.parametrize("T,K,I,form", [(2100, 1032, 2312, (0, 2)), (4000, 256, 1288, (0, 1)), (300, 4096, 264, (4, 0)), (70, 512, 264, (1, 0))])
+def test_swiglu_mlp_forms(T, K, I, form):
+    """The activation in the epilogue of pairs, whose peer loads the up rows, of single CTAs and of the split form; ragged in every size."""
     from lightron_b200.ops import functional as OF
-    assert _ctas_per_tile((T, 2 * I, K)) == ctas
-    assert ctas == 1 or _ctas_per_tile((K, I, T), (T, I, K)) == 2       # down projection: weight gradient and dg | du
+    assert _form((T, 2 * I, K)) == form
+    if form == (0, 2):
+        assert _form((K, I, T), (T, I, K)) == form           # down projection: weight gradient and dg | du
     w13 = _rand(2 * I, K, scale=K ** -0.5, seed=2)
     ins = [t.detach().requires_grad_(True) for t in (_rand(T, K, seed=1), w13[:I], w13[I:], _rand(K, I, scale=I ** -0.5, seed=3))]
     dy = _rand(T, K, seed=4)
@@ -258,6 +271,25 @@ def test_swiglu_mlp_pair_tiles(T, K, I, ctas):
     yd = (torch.nn.functional.silu(x @ w1.t()) * (x @ w3.t())) @ w2.t()
     for g, w in zip(got, (yd, *torch.autograd.grad(yd, [x, w1, w3, w2], dy.double()))):
         assert _rel(g, w) < 1e-2
+
+
+@pytest.mark.parametrize("T,K,I,ctas", [(300, 4096, 264, 2), (70, 512, 264, 1)])
+def test_activation_in_small_list_tiles(T, K, I, ctas):
+    """Activation epilogues of the list form whose columns are fewer than a tile's: three problems, which are never split."""
+    from lightron_b200.ops import functional as OF
+    assert _form(*[(T, 2 * I, K)] * 3) == (0, ctas) == _form(*[(T, I, K)] * 3)
+    x, w13, dy, w2 = _rand(T, K, seed=1), _rand(2 * I, K, scale=K ** -0.5, seed=2), _rand(T, K, seed=3), _rand(K, I, scale=K ** -0.5, seed=4)
+    new = lambda n: [torch.empty(T, n, dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+    gus, hs, dgus = new(2 * I), new(I), new(2 * I)
+    OF.gemm_grouped([(x, w13, False, False, gu, False, 1, h, I) for gu, h in zip(gus, hs)])
+    OF.gemm_grouped([(dy, w2, False, True, dgu, False, 2, gu, I) for dgu, gu in zip(dgus, gus)])
+    _status_ok()
+    want = x.double() @ w13.double().t()
+    for gu, h, dgu in zip(gus, hs, dgus):
+        g64 = gu.double().requires_grad_()
+        act = torch.nn.functional.silu(g64[:, :I]) * g64[:, I:]
+        act.backward(dy.double() @ w2.double())
+        assert _rel(gu, want) < 5e-3 and _rel(h, act.detach()) < 5e-3 and _rel(dgu, g64.grad) < 1e-2
 
 
 # ---- norm ----------------------------------------------------------------------------------

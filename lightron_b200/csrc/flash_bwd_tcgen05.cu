@@ -22,11 +22,12 @@
 // up every other access of the SM: 5360 against 3750 cycles a block at d = 128).
 // What bounds it.  Cycles of a block: d = 64 2770, of which the math warps are never idle (exponentials 1330, dS 480, the rest waits, stores
 // and tensor-memory accesses); d = 128 3750, the chain dS -> dK, dQ -> drain -> dP of the next block, which shares dQ's columns, against 2560 of
-// tensor pipe.  Both run at the power limit in long loops (1.49 / 1.31 GHz).  What it took to get there from 3150 / 4500: an elected thread
+// tensor pipe.  Both run at the power limit in long loops (1.64 / 1.53 GHz).  Counters: tensor pipe 45 / 58 %, L1 and shared memory 55 / 73 %,
+// exponentials 36 / 23 % of the active cycles (B8 S2048 32q/4kv d64, B4 S2048 32q/8kv d128).  What it took to get there from 3150 / 4500: an elected thread
 // that issues (elect_one), one arrival per warp, waits that are sure to succeed ahead of the one that is not, no divisions in the loops,
 // dQ's columns freed after 110 instead of 800 cycles, dK and dV through TMA stores (prologue and stores of a CTA: 12000 / 16000 cycles before).
-// Loops of 0.35 s of all its kernels, before / now, on one GPU: B8 S2048 32q/4kv d64 670 / 561 us, B1 S8192 32q/8kv d128
-// 1683 / 1480, B3 S1531 32q/8kv d128 248 / 232, B1 S4096 8q/8kv d128 119 / 107.
+// Loops of 0.35 s of all its kernels, before / now, on one GPU: B8 S2048 32q/4kv d64 646 / 547 us, B1 S8192 32q/8kv d128
+// 1624 / 1404, B3 S1531 32q/8kv d128 237 / 221, B1 S4096 8q/8kv d128 117 / 104.
 // Warp roles (512 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4-11 math, 12-15 dQ drain.
 // All waits are bounded; on expiry a status word is set and the CTA drains and frees its TMEM.
 #include "tcgen05.cuh"
@@ -75,7 +76,8 @@ struct BwdCfg {
   static constexpr int SMEM = OFF_BAR + 256;
   static constexpr int NBAR = 1 + 2 * QS + 2 * DS + 6;
   static constexpr int NTHREADS = 512;
-  // Registers per thread: loads and MMAs / math / drain, which holds a whole row of dQ so that its columns are free at once
+  // Registers per thread: loads and MMAs / math / drain, which holds a whole row of dQ so that its columns are free at once.
+  // (Spills by -Xptxas -v: 24 bytes stored and 160 loaded per thread at d = 64, 76 and 100 at d = 128.)
   static constexpr int REGS_ISSUE = 96, REGS_MATH = (D == 64) ? 160 : 128, REGS_DRAIN = (D == 64) ? 96 : 160;
   static_assert(REGS_ISSUE + 2 * REGS_MATH + REGS_DRAIN <= 4 * 128, "a CTA has 512 x 128 registers");
   // TMEM columns

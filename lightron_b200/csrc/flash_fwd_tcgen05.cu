@@ -15,13 +15,15 @@
 // What bounds it: 16 exponentials per clock per SM are 1024 cycles per 128x128 block against 542 (d = 64)
 // or 1020 (d = 128) cycles of tensor pipe.  A tile's softmax, P V and next S follow one another, and the two CTAs of an SM fill each
 // other's gaps: a block of a tile that has the SM to itself takes 2350 cycles (d = 64) / 3050 (d = 128), one of two tiles 3200 / 3700 on
-// average.  At d = 128 the power limit comes on top (long loops run at 1.55 GHz).  What the single cycles went into, and what each was worth:
-//   * MMAs and loads are issued by an elected thread (elect_one): 8 MMAs in 590 instead of 1170 cycles;
+// average.  At d = 128 the power limit comes on top (long loops run at 1.67 GHz).  Counters: exponentials 60 / 48 %, tensor pipe 30 / 48 % of the
+// active cycles (B8 S2048 32q/4kv d64, B4 S2048 32q/8kv d128).  What the single cycles went into, and what each was worth:
+//   * MMAs and loads are issued by an elected thread (elect_one has the cycles): with lane 0 in its place 242 us instead of 228 (B8 S2048
+//     32q/4kv d64) and 557 instead of 488 (B1 S8192 32q/8kv d128);
 //   * one CTA per tile instead of two tiles per CTA and CTAs that go on with the next tile (cluster launch control): prologue and
 //     stores of a tile run under the other tile's blocks (d = 64 alone 265 -> 233 us);
 //   * waits that are sure to succeed are put ahead of the one that is not (some 150 cycles each), O leaves through TMA stores.
-// Loops of 0.35 s, two tiles per CTA / now, on one GPU: B8 S2048 32q/4kv d64 266 / 227 us, B1 S8192 32q/8kv d128 619 / 578,
-// B3 S1531 32q/8kv d128 92 / 82, B1 S4096 8q/8kv d128 82 / 62.  Scaling and summing use two-wide fp32 instructions and the maximum
+// Loops of 0.35 s, two tiles per CTA / now, on one GPU: B8 S2048 32q/4kv d64 266 / 226 us, B1 S8192 32q/8kv d128 595 / 545,
+// B3 S1531 32q/8kv d128 88 / 76, B1 S4096 8q/8kv d128 82 / 63.  Scaling and summing use two-wide fp32 instructions and the maximum
 // three-input ones.  (Measured and not kept: a polynomial on the FMA pipe for one pair of exponentials in four; four tiles of 64-key blocks per
 // SM at d = 64, 236 us, and two score buffers of 64 keys at d = 128, 753 us, which load each K and V byte in smaller boxes and
 // leave one thread to issue everything; lists fixed in advance instead of launch control, 233 us against 224.)
@@ -45,7 +47,8 @@ using namespace bw;
 constexpr int FA_MAX_RANKS = 8;
 constexpr int FA_FWD_THREADS = 256;
 // Registers per thread of the two warpgroups.  Two CTAs of 256 threads leave 128 per thread at launch; the issuing warpgroup gives most
-// of its share to the softmax threads, of which each holds a row of 128 scores.
+// of its share to the softmax threads, of which each holds a row of 128 scores.  (Spills by -Xptxas -v: none at d = 64, 32 bytes
+// stored and 36 loaded per thread at d = 128.)
 constexpr int FA_REGS_ISSUE = 56, FA_REGS_SOFTMAX = 200;
 static_assert(FA_REGS_ISSUE + FA_REGS_SOFTMAX <= 2 * 128, "a CTA has 256 x 128 registers");
 struct FaPush {
@@ -56,7 +59,8 @@ struct FaPush {
   bf16* v_dst[FA_MAX_RANKS];
   unsigned int* flags[FA_MAX_RANKS];                 // rank r's block counters [B][S_full / 128]
 };
-// Division of 0 <= x < 2^31 by a divisor that is fixed for the launch: a multiplication (the host finds m, which is exact for such x).
+// Division of 0 <= x < 2^31 by a divisor that is fixed for the launch: a multiplication by a rounded-up reciprocal (division by invariant
+// integers, Granlund and Montgomery 1994; the host finds m, which is exact for such x).
 struct FastDiv {
   unsigned int d, m, s;
   void set(unsigned int div) {

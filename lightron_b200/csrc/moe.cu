@@ -591,8 +591,9 @@ extern "C" int lb_moe_push_ctas(int T) { return moe_grid(T); }
 extern "C" int lb_moe_router(const void* x, const void* wg, int T, int H, int E, int k, void* probs, void* idx, void* wts,
                              void* within, void* blk_hist, void* blk_psum, void* stream) {
   if (T <= 0 || (H % 8) || E < 1 || E > MOE_MAX_EXPERTS || k < 1 || k > MOE_MAX_TOPK || k > E) return LB_ERR_SHAPE;
-  // One token at a time where a warp has no second one, four elsewhere.  One / four, us: T 1, H 2048, E 8 16 / 19; T 16384, H 4096, E 64
-  // 766 / 402; T 32768, H 2048, E 64 625 / 369.
+  // One token at a time where a warp has no second one, four elsewhere.  One / four, us, single launches between events with inputs that
+  // are not in L2: T 1, H 2048, E 8 16 / 19; T 16384, H 4096, E 64 766 / 402; T 32768, H 2048, E 64 625 / 369.  (The form that waited for each load by
+  // itself took 25, 808 and 664 under the same conditions; with inputs in L2 T 1 takes 17, it took 19.)
   const bool one = T <= ROUTER_THREADS / 32;
   (one ? moe_router_kernel<1> : moe_router_kernel<4>)<<<lb_moe_router_blocks(T), ROUTER_THREADS, 0, (cudaStream_t)stream>>>(
       (const bf16*)x, (const bf16*)wg, T, H, E, k, (float*)probs, (int*)idx, (float*)wts, (int*)within, (int*)blk_hist,

@@ -250,7 +250,8 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // One thread of a converged warp, chosen by the hardware.  Where the issuing thread of MMAs and TMA loads is chosen this way (and not
-// as lane 0 of a divergent branch) the compiler keeps descriptors in uniform registers: 32 instead of 46 cycles per issued MMA.
+// as lane 0 of a divergent branch) the compiler keeps descriptors in uniform registers.  Issuing the scores of a block
+// in the attention forward, by clock64 around MMAs and commits, lane 0 / elected: 4 MMAs (d = 64) 519 / 156 cycles, 8 (d = 128) 734 / 583.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));

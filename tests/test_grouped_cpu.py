@@ -41,7 +41,8 @@ def _ctas_per_tile(shapes, sms=148):
 
 
 def test_plan_is_the_schedule_of_the_chosen_form():
-    """One tile's rows decide between a CTA per 128 rows and a pair per 256: the plan counts the form that is launched."""
+    """One tile's rows decide between a CTA per 128 rows and a pair per 256: the plan counts the one that the list form launches (alone, the
+    first two go to the split form, which has no lists; next to two more problems they do not)."""
     lib = native._load()
     if lib is None:
         pytest.skip("native library not built")
@@ -63,7 +64,7 @@ def test_plan_is_the_schedule_of_the_chosen_form():
     ([(16384, 4096, 256)], 1), ([(8192, 5632, 512)], 1), ([(16384, 2304, 768)], 1), ([(4096, 4096, 768)], 1),
     # it does not: 4 to 11 % faster
     ([(8192, 4096, 1024)], 2), ([(4096, 4096, 1536)], 2), ([(16384, 768, 1536)], 2), ([(16384, 5632, 4096)], 2),
-    # one or two short tiles per SM: the setup
+    # one or two short tiles per SM: the setup (the last one goes to the split form unless a third problem comes with it)
     ([(1000, 2304, 768)], 1), ([(4096, 2304, 768)], 1), ([(2048, 2304, 2048)], 1), ([(512, 768, 768), (512, 768, 768)], 1),
     # the weight gradient's long tiles carry the data gradient's short ones
     ([(2304, 768, 8192), (8192, 768, 2304)], 2),

@@ -30,6 +30,57 @@ int lb_num_sms();
     }                                                       \
   } while (0)
 
+// ---- dependent launches --------------------------------------------------------------------------
+// A kernel launched by lb_launch() may start as soon as every CTA of the kernel before it in the stream has called grid_go() or has ended:
+// its launch, barriers, tensor memory and descriptors then run under the other's tail.  Its first access to memory that
+// another kernel writes or reads comes behind grid_wait(), which returns when the kernels before it have completed and their writes are
+// visible; every thread calls it, so that no bounded wait of a CTA's roles runs meanwhile.  A kernel that allocates tensor memory calls
+// grid_go() behind the allocation: a later kernel's CTA could otherwise hold the columns for which an earlier one waits.  Both are no-ops
+// in a plain launch.  Kernels that wait for other GPUs are launched plainly, and so is one of very many short blocks (a block's grid_wait() takes
+// some 0.3 us: 32000 of clear_kernel 31 instead of 23 us).  No grid_go() in kernels that fill an SM's shared memory or registers: the next one's
+// CTAs would crowd into the SMs that are done first (1000 x 768 feed-forward, four launches, 76 instead of 74 us).
+// (Host time of a launch, 700 bytes of parameters, plain / dependent: 3.05 / 2.48 us.)
+__device__ __forceinline__ void grid_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename T> struct lb_as_is { typedef T type; };      // (arguments convert to the kernel's parameter types)
+// Launches `fn` on clusters of `cluster` CTAs; `dependent` as above.
+template <typename... K>
+inline int lb_launch_cluster(bool dependent, int cluster, void (*fn)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                             const typename lb_as_is<K>::type&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  unsigned n = 0;
+  if (dependent) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = (unsigned)cluster; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1;
+    n++;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = n;
+  void* a[] = {const_cast<void*>(static_cast<const void*>(&args))...};
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(fn), a);
+  if (e != cudaSuccess) { cudaGetLastError(); g_lb_last_cuda_error = (int)e; return LB_ERR_LAUNCH; }
+  return LB_OK;
+}
+template <typename... K>
+inline int lb_launch(void (*fn)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const typename lb_as_is<K>::type&... args) {
+  return lb_launch_cluster(true, 1, fn, grid, block, smem, s, args...);
+}
+#define LB_LAUNCH(...)                                      \
+  do {                                                      \
+    const int rc__ = lb_launch(__VA_ARGS__);                \
+    if (rc__ != LB_OK) return rc__;                         \
+  } while (0)
+
 typedef __nv_bfloat16 bf16;
 typedef __nv_bfloat162 bf162;
 

@@ -44,18 +44,21 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_reg_kernel(const bf16* __rest
                                                               const bf16* __restrict__ w, bf16* __restrict__ h,
                                                               bf16* __restrict__ y, float* __restrict__ rstd_out,
                                                               int rows, int cols, float eps) {
+  grid_go();
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int nvec = cols >> 3;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * cols);
   const uint4* rr = HAS_RES ? reinterpret_cast<const uint4*>(res + (size_t)row * cols) : nullptr;
-  uint4 a[NV], b[HAS_RES ? NV : 1];
+  uint4 a[NV], b[HAS_RES ? NV : 1], c[NV <= 4 ? NV : 1];
 #pragma unroll
   for (int k = 0; k < NV; k++) {
     const int v = lane + 32 * k;
     a[k] = v < nvec ? xr[v] : make_uint4(0, 0, 0, 0);
     if (HAS_RES) b[k] = v < nvec ? rr[v] : make_uint4(0, 0, 0, 0);
+    if (NV <= 4) c[k] = v < nvec ? reinterpret_cast<const uint4*>(w)[v] : make_uint4(0, 0, 0, 0);      // (a narrow row's time is its latency)
   }
   float ss = 0.f;
 #pragma unroll
@@ -85,7 +88,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_reg_kernel(const bf16* __rest
     if (v < nvec) {
       float f[8], g[8];
       unpack8(a[k], f);
-      unpack8(wv[v], g);
+      unpack8(NV <= 4 ? c[k] : wv[v], g);
 #pragma unroll
       for (int i = 0; i < 8; i++) f[i] = f[i] * rstd * g[i];
       yr[v] = pack8(f);
@@ -98,6 +101,8 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const bf16* __restrict
                                                           const bf16* __restrict__ w, bf16* __restrict__ h,
                                                           bf16* __restrict__ y, float* __restrict__ rstd_out,
                                                           int rows, int cols, float eps) {
+  grid_go();
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int warps_per_block = blockDim.x >> 5;
   const int nvec = cols >> 3;
@@ -140,7 +145,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const bf16* __restrict
 }
 
 template <bool HAS_RES>
-static void rmsnorm_fwd_launch(const void* x, const void* res, const void* w, void* h, void* y, void* rstd, int rows, int cols,
+static int rmsnorm_fwd_launch(const void* x, const void* res, const void* w, void* h, void* y, void* rstd, int rows, int cols,
                                float eps, cudaStream_t s) {
   // Small blocks: the registers of a row are many, and with 256 threads a block they leave a good part of an SM's unused (rows with
   // the residual, 8 / 2 warps per block: 16384 x 3072 82 / 68 us, which was more than reading twice takes at 8192 x 3072, 45 / 39 against
@@ -150,9 +155,9 @@ static void rmsnorm_fwd_launch(const void* x, const void* res, const void* w, vo
   int wpb = nv <= 2 ? 4 : 2;
   while (wpb > 1 && (rows + wpb - 1) / wpb < 2 * lb_num_sms()) wpb >>= 1;
   const int blocks = (rows + wpb - 1) / wpb;
-#define LB_RMS_FWD(V)                                                                                               \
-  rmsnorm_fwd_reg_kernel<HAS_RES, V><<<blocks, 32 * wpb, 0, s>>>((const bf16*)x, (const bf16*)res, (const bf16*)w,  \
-                                                                 (bf16*)h, (bf16*)y, (float*)rstd, rows, cols, eps)
+#define LB_RMS_FWD(V)                                                                                                      \
+  LB_LAUNCH(rmsnorm_fwd_reg_kernel<HAS_RES, V>, blocks, 32 * wpb, 0, s, (const bf16*)x, (const bf16*)res, (const bf16*)w,   \
+            (bf16*)h, (bf16*)y, (float*)rstd, rows, cols, eps)
   if (nv <= 2) LB_RMS_FWD(2);
   else if (nv <= 4) LB_RMS_FWD(4);
   else if (nv <= 6) LB_RMS_FWD(6);
@@ -163,19 +168,18 @@ static void rmsnorm_fwd_launch(const void* x, const void* res, const void* w, vo
   else if (nv <= 16) LB_RMS_FWD(16);
   else {
     const int b = (rows + 7) / 8 > lb_num_sms() * 8 ? lb_num_sms() * 8 : (rows + 7) / 8;
-    rmsnorm_fwd_kernel<HAS_RES><<<b, 256, 0, s>>>((const bf16*)x, (const bf16*)res, (const bf16*)w, (bf16*)h, (bf16*)y,
-                                                  (float*)rstd, rows, cols, eps);
+    LB_LAUNCH(rmsnorm_fwd_kernel<HAS_RES>, b, 256, 0, s, (const bf16*)x, (const bf16*)res, (const bf16*)w, (bf16*)h, (bf16*)y, (float*)rstd,
+              rows, cols, eps);
   }
 #undef LB_RMS_FWD
+  return LB_OK;
 }
 
 extern "C" int lb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* h, void* y, void* rstd, int rows,
                               int cols, float eps, void* stream) {
   if (cols % 8 || rows <= 0) return LB_ERR_SHAPE;
-  if (res) rmsnorm_fwd_launch<true>(x, res, w, h, y, rstd, rows, cols, eps, (cudaStream_t)stream);
-  else rmsnorm_fwd_launch<false>(x, res, w, h, y, rstd, rows, cols, eps, (cudaStream_t)stream);
-  LB_CHECK_LAUNCH();
-  return LB_OK;
+  if (res) return rmsnorm_fwd_launch<true>(x, res, w, h, y, rstd, rows, cols, eps, (cudaStream_t)stream);
+  return rmsnorm_fwd_launch<false>(x, res, w, h, y, rstd, rows, cols, eps, (cudaStream_t)stream);
 }
 
 // bwd: g = dy * w; xhat = x * rstd; dx = rstd * (g - xhat * mean(g * xhat)) (+ dres);
@@ -185,6 +189,8 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict
                                                           const bf16* __restrict__ w, const float* __restrict__ rstd,
                                                           const bf16* __restrict__ dres, bf16* __restrict__ dx,
                                                           float* __restrict__ partial, int rows, int cols) {
+  grid_go();
+  grid_wait();
   extern __shared__ float s_dw[];
   for (int j = threadIdx.x; j < cols; j += blockDim.x) s_dw[j] = 0.f;
   __syncthreads();
@@ -250,6 +256,8 @@ __global__ void __launch_bounds__(256, RmsBwdCfg<VPT>::PER_SM)
 rmsnorm_bwd_blk_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
                        const float* __restrict__ rstd, const bf16* __restrict__ dres, bf16* __restrict__ dx,
                        float* __restrict__ partial, int rows, int cols) {
+  grid_go();
+  grid_wait();
   constexpr int RB = RmsBwdCfg<VPT>::RB;
   __shared__ float s_red[2][RB][8];
   const int T = blockDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = T >> 5;
@@ -344,16 +352,16 @@ rmsnorm_bwd_blk_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, 
   }
 }
 
-// Launches the block-per-row version (rows of up to 8192 columns); returns false for wider ones.
-static bool rmsnorm_bwd_blk_dispatch(const void* dy, const void* x, const void* w, const void* rstd, const void* dres,
+// The block-per-row version, for rows of up to 8192 columns (LB_ERR_CAPACITY for wider ones, and nothing is launched).
+static int rmsnorm_bwd_blk_dispatch(const void* dy, const void* x, const void* w, const void* rstd, const void* dres,
                                      void* dx, void* partial, int rows, int cols, int nblk, cudaStream_t s) {
   const int nvec = cols / 8;
   const int vpt = (nvec + 255) / 256;
-  if (vpt > 4) return false;
+  if (vpt > 4) return LB_ERR_CAPACITY;
   const int T = ((nvec + vpt - 1) / vpt + 31) / 32 * 32;
-#define LB_RMS_BLK(V)                                                                                             \
-  rmsnorm_bwd_blk_kernel<V><<<nblk, T, 0, s>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)rstd, \
-                                               (const bf16*)dres, (bf16*)dx, (float*)partial, rows, cols)
+#define LB_RMS_BLK(V)                                                                                                        \
+  LB_LAUNCH(rmsnorm_bwd_blk_kernel<V>, nblk, T, 0, s, (const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)rstd,   \
+            (const bf16*)dres, (bf16*)dx, (float*)partial, rows, cols)
   switch (vpt) {
     case 1: LB_RMS_BLK(1); break;
     case 2: LB_RMS_BLK(2); break;
@@ -361,12 +369,14 @@ static bool rmsnorm_bwd_blk_dispatch(const void* dy, const void* x, const void* 
     default: LB_RMS_BLK(4); break;
   }
 #undef LB_RMS_BLK
-  return true;
+  return LB_OK;
 }
 
 // dw[j] = sum over blocks of partial[b, j]: 32 columns x 32 row lanes per block.
 __global__ void __launch_bounds__(1024) rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, bf16* __restrict__ dw,
                                                                  int nblk, int cols) {
+  grid_go();
+  grid_wait();
   __shared__ float s[32][33];
   const int j = blockIdx.x * 32 + threadIdx.x;
   float v = 0.f;
@@ -409,16 +419,14 @@ extern "C" int lb_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
   if (nblk != lb_rmsnorm_bwd_blocks(rows, cols)) return LB_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   size_t smem = (size_t)cols * sizeof(float);
-  if (rmsnorm_bwd_blk_dispatch(dy, x, w, rstd, dres, dx, partial, rows, cols, nblk, s)) {
-    LB_CHECK_LAUNCH();
-  } else {
+  const int rc = rmsnorm_bwd_blk_dispatch(dy, x, w, rstd, dres, dx, partial, rows, cols, nblk, s);
+  if (rc != LB_OK && rc != LB_ERR_CAPACITY) return rc;
+  if (rc == LB_ERR_CAPACITY) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(rmsnorm_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    rmsnorm_bwd_kernel<<<nblk, 256, smem, s>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)rstd,
-                                               (const bf16*)dres, (bf16*)dx, (float*)partial, rows, cols);
-    LB_CHECK_LAUNCH();
+    LB_LAUNCH(rmsnorm_bwd_kernel, nblk, 256, smem, s, (const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)rstd, (const bf16*)dres,
+              (bf16*)dx, (float*)partial, rows, cols);
   }
-  rmsnorm_dw_reduce_kernel<<<(cols + 31) / 32, dim3(32, 32), 0, s>>>((const float*)partial, (bf16*)dw, nblk, cols);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(rmsnorm_dw_reduce_kernel, (cols + 31) / 32, dim3(32, 32), 0, s, (const float*)partial, (bf16*)dw, nblk, cols);
   return LB_OK;
 }
 
@@ -429,6 +437,8 @@ extern "C" int lb_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
 __global__ void rope_kernel(bf16* __restrict__ t, const float* __restrict__ cosT, const float* __restrict__ sinT,
                             const int* __restrict__ positions, int tokens, int S, int n_heads, int head_dim,
                             long long ld, int inverse) {
+  grid_go();
+  grid_wait();
   const int vec_per_head = head_dim >> 3;
   const long long total = (long long)tokens * n_heads * vec_per_head;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -459,10 +469,8 @@ extern "C" int lb_rope(void* t, const void* cosT, const void* sinT, const void* 
   long long total = (long long)tokens * n_heads * (head_dim / 8);
   int blocks = (int)((total + 255) / 256);
   if (blocks > lb_num_sms() * 16) blocks = lb_num_sms() * 16;
-  rope_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((bf16*)t, (const float*)cosT, (const float*)sinT,
-                                                        (const int*)positions, tokens, S, n_heads, head_dim, ld,
-                                                        inverse);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(rope_kernel, blocks, 256, 0, (cudaStream_t)stream, (bf16*)t, (const float*)cosT, (const float*)sinT, (const int*)positions, tokens,
+            S, n_heads, head_dim, ld, inverse);
   return LB_OK;
 }
 
@@ -471,6 +479,8 @@ extern "C" int lb_rope(void* t, const void* cosT, const void* sinT, const void* 
 // ---------------------------------------------------------------------------------------
 __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, int rows, int I, long long ld,
                                   const int* __restrict__ rows_dev) {
+  grid_go();
+  grid_wait();
   if (rows_dev) rows = max(0, min(rows, *rows_dev));     // row count known only on the device (MoE segments)
   const int vec = I >> 3;
   const long long total = (long long)rows * vec;
@@ -489,6 +499,8 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
 
 __global__ void swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __restrict__ dy, bf16* __restrict__ dgu,
                                   int rows, int I, long long ld, const int* __restrict__ rows_dev) {
+  grid_go();
+  grid_wait();
   if (rows_dev) rows = max(0, min(rows, *rows_dev));
   const int vec = I >> 3;
   const long long total = (long long)rows * vec;
@@ -520,9 +532,8 @@ static inline int ew_blocks(long long total) {
 // rows_dev (or null): device int; only the first min(rows, *rows_dev) rows are processed.
 extern "C" int lb_swiglu_fwd_dev(const void* gu, void* out, int rows, int I, long long ld, const void* rows_dev, void* stream) {
   if (I % 8 || ld % 8 || rows <= 0) return LB_ERR_SHAPE;
-  swiglu_fwd_kernel<<<ew_blocks((long long)rows * (I / 8)), 256, 0, (cudaStream_t)stream>>>((const bf16*)gu, (bf16*)out,
-                                                                                            rows, I, ld, (const int*)rows_dev);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(swiglu_fwd_kernel, ew_blocks((long long)rows * (I / 8)), 256, 0, (cudaStream_t)stream, (const bf16*)gu, (bf16*)out, rows, I, ld,
+            (const int*)rows_dev);
   return LB_OK;
 }
 extern "C" int lb_swiglu_fwd(const void* gu, void* out, int rows, int I, long long ld, void* stream) {
@@ -532,9 +543,8 @@ extern "C" int lb_swiglu_fwd(const void* gu, void* out, int rows, int I, long lo
 extern "C" int lb_swiglu_bwd_dev(const void* gu, const void* dy, void* dgu, int rows, int I, long long ld,
                                  const void* rows_dev, void* stream) {
   if (I % 8 || ld % 8 || rows <= 0) return LB_ERR_SHAPE;
-  swiglu_bwd_kernel<<<ew_blocks((long long)rows * (I / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (const bf16*)gu, (const bf16*)dy, (bf16*)dgu, rows, I, ld, (const int*)rows_dev);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(swiglu_bwd_kernel, ew_blocks((long long)rows * (I / 8)), 256, 0, (cudaStream_t)stream, (const bf16*)gu, (const bf16*)dy, (bf16*)dgu,
+            rows, I, ld, (const int*)rows_dev);
   return LB_OK;
 }
 extern "C" int lb_swiglu_bwd(const void* gu, const void* dy, void* dgu, int rows, int I, long long ld, void* stream) {
@@ -547,6 +557,8 @@ extern "C" int lb_swiglu_bwd(const void* gu, const void* dy, void* dgu, int rows
 // ---------------------------------------------------------------------------------------
 __global__ void embedding_fwd_kernel(const long long* __restrict__ tok, const bf16* __restrict__ w,
                                      bf16* __restrict__ out, int T, int H, int v0, int v1) {
+  grid_go();
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   const int nvec = H >> 3;
@@ -568,6 +580,8 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ tok, const bf
 template <bool WIDE>
 __global__ void embedding_bwd_kernel(const long long* __restrict__ tok, const bf16* __restrict__ dy,
                                      bf16* __restrict__ dw, int T, int H, int v0, int v1) {
+  grid_go();
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   for (int t = blockIdx.x * wpb + (threadIdx.x >> 5); t < T; t += gridDim.x * wpb) {
@@ -591,7 +605,7 @@ __global__ void embedding_bwd_kernel(const long long* __restrict__ tok, const bf
 }
 
 // Zeroes for the dense gradient.  Bound by memory; one 16-byte store per thread, so that a block's stores are all issued at once: 131 MB (32000
-// x 2048) in 23.5 us, as a memset takes and as 32-byte stores do; torch's fill takes 40.
+// x 2048) in 23.5 us, as a memset takes and as 32-byte stores do; torch's fill takes 40.  (Launched plainly: see common.cuh.)
 __global__ void __launch_bounds__(256) clear_kernel(uint4* __restrict__ p, long long nvec, int tail) {
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i < nvec) p[i] = make_uint4(0, 0, 0, 0);
@@ -607,18 +621,14 @@ extern "C" int lb_clear(void* p, long long bytes, void* stream) {
   const int tail = (int)(bytes & 15);
   const long long blocks = (nvec + tail + 255) / 256;
   if (blocks > 0x7fffffffLL) return LB_ERR_SHAPE;
-  clear_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((uint4*)p, nvec, tail);
-  LB_CHECK_LAUNCH();
-  return LB_OK;
+  return lb_launch_cluster(false, 1, clear_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, (uint4*)p, nvec, tail);
 }
 
 extern "C" int lb_embedding_fwd(const void* tok, const void* w, void* out, int T, int H, int v0, int v1, void* stream) {
   if (H % 8 || T <= 0) return LB_ERR_SHAPE;
   int blocks = (T + 7) / 8;
   if (blocks > lb_num_sms() * 8) blocks = lb_num_sms() * 8;
-  embedding_fwd_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const long long*)tok, (const bf16*)w, (bf16*)out, T,
-                                                                 H, v0, v1);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(embedding_fwd_kernel, blocks, 256, 0, (cudaStream_t)stream, (const long long*)tok, (const bf16*)w, (bf16*)out, T, H, v0, v1);
   return LB_OK;
 }
 
@@ -627,10 +637,9 @@ extern "C" int lb_embedding_bwd(const void* tok, const void* dy, void* dw, int T
   int blocks = (T + 7) / 8;
   if (blocks > lb_num_sms() * 8) blocks = lb_num_sms() * 8;
   if ((((uintptr_t)dy | (uintptr_t)dw) & 15) == 0)
-    embedding_bwd_kernel<true><<<blocks, 256, 0, (cudaStream_t)stream>>>((const long long*)tok, (const bf16*)dy, (bf16*)dw, T, H, v0, v1);
+    LB_LAUNCH(embedding_bwd_kernel<true>, blocks, 256, 0, (cudaStream_t)stream, (const long long*)tok, (const bf16*)dy, (bf16*)dw, T, H, v0, v1);
   else
-    embedding_bwd_kernel<false><<<blocks, 256, 0, (cudaStream_t)stream>>>((const long long*)tok, (const bf16*)dy, (bf16*)dw, T, H, v0, v1);
-  LB_CHECK_LAUNCH();
+    LB_LAUNCH(embedding_bwd_kernel<false>, blocks, 256, 0, (cudaStream_t)stream, (const long long*)tok, (const bf16*)dy, (bf16*)dw, T, H, v0, v1);
   return LB_OK;
 }
 
@@ -642,6 +651,8 @@ extern "C" int lb_embedding_bwd(const void* tok, const void* dy, void* dw, int T
 __global__ void __launch_bounds__(256) ce_stats_kernel(const bf16* __restrict__ logits, const long long* __restrict__ tgt,
                                                        float* __restrict__ mx_out, float* __restrict__ se_out,
                                                        float* __restrict__ tl_out, int V, long long ld, int v0) {
+  grid_go();
+  grid_wait();
   const int row = blockIdx.x;
   const uint4* p = reinterpret_cast<const uint4*>(logits + (size_t)row * ld);
   const int nvec = V >> 3;
@@ -682,6 +693,8 @@ __global__ void __launch_bounds__(256) ce_grad_kernel(const bf16* __restrict__ l
                                                       const float* __restrict__ lse, bf16* __restrict__ dlogits,
                                                       const float* __restrict__ dloss, int V, long long ld, int v0,
                                                       float inv_n, int ignore_index) {
+  grid_go();
+  grid_wait();
   const int row = blockIdx.x;
   const long long tg = tgt[row];
   const float scale = (tg == ignore_index) ? 0.f : dloss[0] * inv_n;
@@ -706,9 +719,8 @@ __global__ void __launch_bounds__(256) ce_grad_kernel(const bf16* __restrict__ l
 extern "C" int lb_ce_stats(const void* logits, const void* tgt, void* mx, void* se, void* tl, int T, int V,
                            long long ld, int v0, void* stream) {
   if (V % 8 || ld % 8 || T <= 0) return LB_ERR_SHAPE;
-  ce_stats_kernel<<<T, 256, 0, (cudaStream_t)stream>>>((const bf16*)logits, (const long long*)tgt, (float*)mx,
-                                                       (float*)se, (float*)tl, V, ld, v0);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(ce_stats_kernel, T, 256, 0, (cudaStream_t)stream, (const bf16*)logits, (const long long*)tgt, (float*)mx, (float*)se, (float*)tl, V,
+            ld, v0);
   return LB_OK;
 }
 
@@ -729,6 +741,8 @@ __device__ __forceinline__ float ce_block_sum(float s) {      // of 1024 threads
 __global__ void __launch_bounds__(1024) ce_loss_kernel(const float* __restrict__ mx, const float* se, const float* __restrict__ tl,
                                                        const long long* __restrict__ tgt, float* __restrict__ lse, float* sum,
                                                        int T, int rows, float inv_n, int ignore_index) {
+  grid_go();
+  grid_wait();
   const long long t0 = (long long)blockIdx.x * rows;
   const int n = (int)min((long long)rows, T - t0);
   float s = 0.f;
@@ -745,6 +759,8 @@ __global__ void __launch_bounds__(1024) ce_loss_kernel(const float* __restrict__
 
 __global__ void __launch_bounds__(1024) ce_loss_sum_kernel(const float* __restrict__ sum, float* __restrict__ loss, int n, int rows,
                                                            float inv_n) {
+  grid_go();
+  grid_wait();
   float s = 0.f;
   for (int b = threadIdx.x; b < n; b += 1024) s += sum[(long long)b * rows];
   s = ce_block_sum(s);
@@ -757,13 +773,10 @@ extern "C" int lb_ce_loss(const void* mx, void* se, const void* tl, const void* 
   if (T <= 0) return LB_ERR_SHAPE;
   const bool one = T <= CE_LOSS_ROWS;
   const int rows = one ? T : CE_LOSS_ROWS / 2, blocks = (T - 1) / rows + 1;
-  ce_loss_kernel<<<blocks, 1024, 0, (cudaStream_t)stream>>>((const float*)mx, (const float*)se, (const float*)tl,
-                                                            (const long long*)tgt, (float*)lse, (float*)(one ? loss : se), T, rows,
-                                                            one ? inv_n : 1.f, ignore_index);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(ce_loss_kernel, blocks, 1024, 0, (cudaStream_t)stream, (const float*)mx, (const float*)se, (const float*)tl, (const long long*)tgt,
+            (float*)lse, (float*)(one ? loss : se), T, rows, one ? inv_n : 1.f, ignore_index);
   if (!one) {
-    ce_loss_sum_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>((const float*)se, (float*)loss, blocks, rows, inv_n);
-    LB_CHECK_LAUNCH();
+    LB_LAUNCH(ce_loss_sum_kernel, 1, 1024, 0, (cudaStream_t)stream, (const float*)se, (float*)loss, blocks, rows, inv_n);
   }
   return LB_OK;
 }
@@ -771,10 +784,8 @@ extern "C" int lb_ce_loss(const void* mx, void* se, const void* tl, const void* 
 extern "C" int lb_ce_grad(const void* logits, const void* tgt, const void* lse, void* dlogits, const void* dloss, int T,
                           int V, long long ld, int v0, float inv_n, int ignore_index, void* stream) {
   if (V % 8 || ld % 8 || T <= 0) return LB_ERR_SHAPE;
-  ce_grad_kernel<<<T, 256, 0, (cudaStream_t)stream>>>((const bf16*)logits, (const long long*)tgt, (const float*)lse,
-                                                      (bf16*)dlogits, (const float*)dloss, V, ld, v0, inv_n,
-                                                      ignore_index);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(ce_grad_kernel, T, 256, 0, (cudaStream_t)stream, (const bf16*)logits, (const long long*)tgt, (const float*)lse, (bf16*)dlogits,
+            (const float*)dloss, V, ld, v0, inv_n, ignore_index);
   return LB_OK;
 }
 
@@ -786,6 +797,8 @@ template <typename G>
 __global__ void adamw_kernel(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
                              const G* __restrict__ grad, bf16* __restrict__ param, long long n, float lr, float b1,
                              float b2, float eps, float wd, float bc1, float bc2, float gscale) {
+  grid_go();
+  grid_wait();
   const float inv_bc2_sqrt = rsqrtf(bc2);
   const float step = lr / bc1;
   for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n;
@@ -833,18 +846,19 @@ extern "C" int lb_adamw(void* master, void* m, void* v, const void* grad, void* 
   int blocks = ew_blocks(n / 4);
   cudaStream_t s = (cudaStream_t)stream;
   if (grad_fp32)
-    adamw_kernel<float><<<blocks, 256, 0, s>>>((float*)master, (float*)m, (float*)v, (const float*)grad, (bf16*)param, n,
-                                               lr, b1, b2, eps, wd, bc1, bc2, gscale);
+    LB_LAUNCH(adamw_kernel<float>, blocks, 256, 0, s, (float*)master, (float*)m, (float*)v, (const float*)grad, (bf16*)param, n, lr, b1, b2, eps,
+              wd, bc1, bc2, gscale);
   else
-    adamw_kernel<bf16><<<blocks, 256, 0, s>>>((float*)master, (float*)m, (float*)v, (const bf16*)grad, (bf16*)param, n,
-                                              lr, b1, b2, eps, wd, bc1, bc2, gscale);
-  LB_CHECK_LAUNCH();
+    LB_LAUNCH(adamw_kernel<bf16>, blocks, 256, 0, s, (float*)master, (float*)m, (float*)v, (const bf16*)grad, (bf16*)param, n, lr, b1, b2, eps,
+              wd, bc1, bc2, gscale);
   return LB_OK;
 }
 
 // out[0] += sum(x^2) (fp32).  `zero_first` clears out[0] on the stream before accumulating.
 template <typename G>
 __global__ void sumsq_kernel(const G* __restrict__ x, long long n, float* __restrict__ out) {
+  grid_go();
+  grid_wait();
   float s = 0.f;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const float f = (float)x[i];
@@ -864,12 +878,13 @@ __global__ void sumsq_kernel(const G* __restrict__ x, long long n, float* __rest
 extern "C" int lb_sumsq(const void* x, long long n, void* out, int zero_first, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   if (zero_first) cudaMemsetAsync(out, 0, sizeof(float), s);
-  sumsq_kernel<bf16><<<ew_blocks(n), 256, 0, s>>>((const bf16*)x, n, (float*)out);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(sumsq_kernel<bf16>, ew_blocks(n), 256, 0, s, (const bf16*)x, n, (float*)out);
   return LB_OK;
 }
 
 __global__ void add_inplace_kernel(bf16* __restrict__ a, const bf16* __restrict__ b, long long nvec) {
+  grid_go();
+  grid_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
     float f[8], g[8];
     unpack8(reinterpret_cast<const uint4*>(a)[i], f);
@@ -882,8 +897,7 @@ __global__ void add_inplace_kernel(bf16* __restrict__ a, const bf16* __restrict_
 
 extern "C" int lb_add_inplace(void* a, const void* b, long long n, void* stream) {
   if (n % 8) return LB_ERR_SHAPE;
-  add_inplace_kernel<<<ew_blocks(n / 8), 256, 0, (cudaStream_t)stream>>>((bf16*)a, (const bf16*)b, n / 8);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(add_inplace_kernel, ew_blocks(n / 8), 256, 0, (cudaStream_t)stream, (bf16*)a, (const bf16*)b, n / 8);
   return LB_OK;
 }
 
@@ -946,10 +960,8 @@ extern "C" int lb_rmsnorm_bwd_static(const void* dy, const void* x, const void* 
   cudaStream_t s = (cudaStream_t)stream;
   size_t smem = (size_t)cols * sizeof(float);
   if (smem > 48 * 1024) cudaFuncSetAttribute(rmsnorm_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  rmsnorm_bwd_kernel<<<nblk, 256, smem, s>>>((const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)rstd,
-                                             (const bf16*)dres, (bf16*)dx, partial, rows, cols);
-  LB_CHECK_LAUNCH();
-  rmsnorm_dw_reduce_kernel<<<(cols + 31) / 32, dim3(32, 32), 0, s>>>(partial, (bf16*)dw, nblk, cols);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(rmsnorm_bwd_kernel, nblk, 256, smem, s, (const bf16*)dy, (const bf16*)x, (const bf16*)w, (const float*)rstd, (const bf16*)dres,
+            (bf16*)dx, partial, rows, cols);
+  LB_LAUNCH(rmsnorm_dw_reduce_kernel, (cols + 31) / 32, dim3(32, 32), 0, s, partial, (bf16*)dw, nblk, cols);
   return LB_OK;
 }

@@ -90,6 +90,8 @@ static_assert(BwdCfg<128>::SMEM <= 232448, "shared memory of a CTA");
 // drain warp (a row per lane) are contiguous, and so are the 16-byte loads of a warp here.
 template <int D>
 __global__ void fa_dq_convert_kernel(const FaBwdParams p) {
+  grid_go();
+  grid_wait();
   constexpr int CPR = D / 32;                                  // 32-column chunks per row: a thread takes one
   const int n_mblocks = (p.Sq + 127) / 128;
   const long long total = (long long)p.B * p.hq * n_mblocks * 128 * CPR;
@@ -122,6 +124,8 @@ __global__ void fa_dq_convert_kernel(const FaBwdParams p) {
 // past Sq get (-inf, 0), which makes their P and dS zero.  Also clears the dQ accumulator.  D/8 threads per (token, head).
 template <int D>
 __global__ void fa_bwd_prep_kernel(const FaBwdParams p) {
+  grid_go();
+  grid_wait();
   constexpr int TPR = D / 8;                                   // threads per row: 8 or 16
   const int n_mblocks = (p.Sq + 127) / 128, Sp = n_mblocks * 128;
   const long long total = (long long)p.B * Sp * p.hq;
@@ -229,6 +233,7 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   volatile int* abort_flag = s_abort;
+  grid_wait();
 
   if (warp < 4) reg_dec<C::REGS_ISSUE>();
   if (warp == 0) {
@@ -539,13 +544,10 @@ int launch_fa_bwd(const void* q, const void* k, const void* v, const FaBwdParams
   const long long rows = (long long)p.B * ((p.Sq + 127) / 128 * 128) * p.hq;
   const long long rows_per_block = 256 / (D / 8), cap = lb_num_sms() * 16;
   const long long pblocks = (rows + rows_per_block - 1) / rows_per_block;
-  fa_bwd_prep_kernel<D><<<(int)(pblocks < cap ? pblocks : cap), 256, 0, s>>>(p);
-  LB_CHECK_LAUNCH();
-  fa_bwd_tc_kernel<D><<<(unsigned)grid, C::NTHREADS, C::SMEM, s>>>(tq, tk, tv, tdo, tdk, tdv, p);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(fa_bwd_prep_kernel<D>, (int)(pblocks < cap ? pblocks : cap), 256, 0, s, p);
+  LB_LAUNCH(fa_bwd_tc_kernel<D>, (unsigned)grid, C::NTHREADS, C::SMEM, s, tq, tk, tv, tdo, tdk, tdv, p);
   const long long cblocks = (rows * (D / 32) + 255) / 256;
-  fa_dq_convert_kernel<D><<<(int)(cblocks < cap ? cblocks : cap), 256, 0, s>>>(p);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(fa_dq_convert_kernel<D>, (int)(cblocks < cap ? cblocks : cap), 256, 0, s, p);
   return LB_OK;
 }
 

@@ -245,6 +245,8 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   __syncthreads();
   fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  if (!p.steal) grid_go();
+  grid_wait();
 
   if (warp < 4) {
     reg_dec<FA_REGS_ISSUE>();
@@ -587,10 +589,9 @@ int launch_fa_fwd(const void* q, const void* k, const void* v, FaFwdParams p, co
   p.by_last.set((unsigned)(p.hq * p.B % p.group ? p.hq * p.B % p.group : p.group));
   p.by_hq.set((unsigned)p.hq);
   p.by_rep.set((unsigned)(p.hq / p.hkv));
-  p.steal = push.n_mov == 0;       // (a mover's place is not to be taken)
-  fa_fwd_tc_kernel<D><<<(unsigned)grid, FA_FWD_THREADS, C::SMEM, s>>>(tq, tk, tv, to, p, push);
-  LB_CHECK_LAUNCH();
-  return LB_OK;
+  // (a mover's place is not to be taken; with all tiles resident at once there is none to take)
+  p.steal = push.n_mov == 0 && grid > 2 * lb_num_sms();
+  return lb_launch_cluster(push.n_mov == 0 && !p.kv_flags, 1, fa_fwd_tc_kernel<D>, (unsigned)grid, FA_FWD_THREADS, C::SMEM, s, tq, tk, tv, to, p, push);
 }
 
 }  // namespace

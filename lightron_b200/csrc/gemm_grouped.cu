@@ -207,6 +207,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
   bw::fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   volatile int* abort_flag = s_abort;
+  // (No grid_go(): the next kernel's CTAs would crowd into the SMs that are done first.)
+  grid_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -535,6 +537,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
     }
     bw::mbar_init_fence();
   }
+  if (warp == 1) bw::tmem_alloc(bw::smem_u32(tmem_slot), 512);
+  grid_wait();
   if (threadIdx.x < rp.LE) {
     // segment table -> offsets and tile (mode 0: 128-row tiles) / step (mode 1: 64-row steps) counts,
     // clamped so that no coordinate can pass the end of the buffer
@@ -545,7 +549,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
     s_off[threadIdx.x] = off;
     s_tiles[threadIdx.x] = rp.mode == 0 ? (cnt + BM - 1) / BM : (cnt + BK - 1) / BK;
   }
-  if (warp == 1) bw::tmem_alloc(bw::smem_u32(tmem_slot), 512);
   bw::fence_before();
   __syncthreads();
   bw::fence_after();
@@ -798,24 +801,6 @@ int build_schedule(Problem* probs, int np, int sms, Schedule* out) {
   return LB_OK;
 }
 
-// Launches fn<CG> on `workers` workers; a pair is a cluster of two CTAs.
-template <typename P>
-int launch_pairs(void (*fn)(P), const P& params, int workers, cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * workers);
-  cfg.blockDim = dim3(NUM_THREADS);
-  cfg.dynamicSmemBytes = Cfg<2>::SMEM_BYTES;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, params);
-  if (e != cudaSuccess) { cudaGetLastError(); g_lb_last_cuda_error = (int)e; return LB_ERR_LAUNCH; }
-  return LB_OK;
-}
-
 }  // namespace
 
 // Copies the status words of the grouped GEMM kernel to host memory and clears them.
@@ -968,13 +953,9 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
   gp.offsets = sched.d_offsets;
   gp.items = sched.d_items;
   for (int i = 0; i < n; i++) set_tiles(&gp.prob[i], sched.cg);
-  if (sched.cg == 2) {
-    const int rc = launch_pairs(gemm_grouped_kernel<2>, gp, sched.grid, (cudaStream_t)stream);
-    if (rc) return rc;
-  } else {
-    gemm_grouped_kernel<1><<<sched.grid, NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream>>>(gp);
-    LB_CHECK_LAUNCH();
-  }
+  if (sched.cg == 2)      // a pair is a cluster of two CTAs
+    return lb_launch_cluster(true, 2, gemm_grouped_kernel<2>, 2 * sched.grid, NUM_THREADS, Cfg<2>::SMEM_BYTES, (cudaStream_t)stream, gp);
+  LB_LAUNCH(gemm_grouped_kernel<1>, sched.grid, NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream, gp);
   return LB_OK;
 }
 
@@ -1017,9 +998,7 @@ extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, cons
     static bool attr = false;
     if (!attr) { cudaFuncSetAttribute(gemm_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES); attr = true; }
   }
-  gemm_ragged_kernel<<<lb_num_sms(), NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream>>>(rp);
-  LB_CHECK_LAUNCH();
-  return LB_OK;
+  return lb_launch_cluster(!wait_flag, 1, gemm_ragged_kernel, lb_num_sms(), NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream, rp);
 }
 
 //  Weight gradients: C_e [Nw, Kw] (+)= dY[rows of e, Nw]^T . X[rows of e, Kw]; C: host array of LE
@@ -1048,7 +1027,6 @@ extern "C" int lb_gemm_ragged_wgrad(const void* dY, const void* X, void* const* 
     static bool attr = false;
     if (!attr) { cudaFuncSetAttribute(gemm_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES); attr = true; }
   }
-  gemm_ragged_kernel<<<lb_num_sms(), NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream>>>(rp);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(gemm_ragged_kernel, lb_num_sms(), NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream, rp);
   return LB_OK;
 }

@@ -62,6 +62,8 @@ __global__ void __launch_bounds__(ROUTER_THREADS)
 moe_router_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wg, int T, int H, int E, int k,
                   float* __restrict__ probs, int* __restrict__ idx, float* __restrict__ wts, int* __restrict__ within,
                   int* __restrict__ blk_hist, float* __restrict__ blk_psum) {
+  grid_go();
+  grid_wait();
   __shared__ int s_eid[ROUTER_TOKENS * MOE_MAX_TOPK];
   __shared__ int s_hist[MOE_MAX_EXPERTS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -193,6 +195,8 @@ struct PlanParams {
 };
 
 __global__ void __launch_bounds__(256) moe_plan_kernel(const PlanParams p) {
+  grid_go();
+  grid_wait();
   __shared__ int s_cnt[MOE_MAX_EXPERTS];
   __shared__ float s_ps[MOE_MAX_EXPERTS];
   __shared__ int s_all[MOE_MAX_RANKS * MOE_MAX_EXPERTS];
@@ -292,6 +296,8 @@ struct PushParams {
 };
 
 __global__ void __launch_bounds__(256) moe_push_kernel(const PushParams p) {
+  grid_go();
+  grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const int nvec = p.H >> 3;
   // padding rows of the local segments: rows [off + cnt, off + round_up(cnt, 128)) become zero
@@ -378,6 +384,8 @@ struct PullParams {
 // itself: T 4096, H 2048, k 2 31 us, now 16.)  A sum takes its terms in the same order for every KS.
 template <int KS>
 __global__ void __launch_bounds__(256) moe_pull_kernel(const PullParams p) {
+  grid_go();
+  grid_wait();
   constexpr int U = 8 / KS;
   __shared__ int s_fail;
   if (threadIdx.x == 0) s_fail = 0;
@@ -475,6 +483,8 @@ moe_router_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wg, c
                       const int* __restrict__ idx, const float* __restrict__ dwts, const float* __restrict__ frac,
                       const float* __restrict__ daux, bf16* __restrict__ dx, float* __restrict__ dwg_acc, int T, int H,
                       int E, int k) {
+  grid_go();
+  grid_wait();
   __shared__ float s_dl[RB_TOKENS][MOE_MAX_EXPERTS + 1];
   __shared__ __align__(16) float s_w[RB_WARPS][RB_COLS];
   const int t0 = blockIdx.x * RB_TOKENS;
@@ -595,10 +605,8 @@ extern "C" int lb_moe_router(const void* x, const void* wg, int T, int H, int E,
   // are not in L2: T 1, H 2048, E 8 16 / 19; T 16384, H 4096, E 64 766 / 402; T 32768, H 2048, E 64 625 / 369.  (The form that waited for each load by
   // itself took 25, 808 and 664 under the same conditions; with inputs in L2 T 1 takes 17, it took 19.)
   const bool one = T <= ROUTER_THREADS / 32;
-  (one ? moe_router_kernel<1> : moe_router_kernel<4>)<<<lb_moe_router_blocks(T), ROUTER_THREADS, 0, (cudaStream_t)stream>>>(
-      (const bf16*)x, (const bf16*)wg, T, H, E, k, (float*)probs, (int*)idx, (float*)wts, (int*)within, (int*)blk_hist,
-      (float*)blk_psum);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(one ? moe_router_kernel<1> : moe_router_kernel<4>, lb_moe_router_blocks(T), ROUTER_THREADS, 0, (cudaStream_t)stream, (const bf16*)x,
+            (const bf16*)wg, T, H, E, k, (float*)probs, (int*)idx, (float*)wts, (int*)within, (int*)blk_hist, (float*)blk_psum);
   return LB_OK;
 }
 
@@ -615,9 +623,7 @@ extern "C" int lb_moe_plan(const void* blk_hist, const void* blk_psum, void* blk
   p.nblk = nblk; p.E = E; p.LE = E / n; p.n = n; p.me = me; p.T = T; p.k = k; p.cap = cap;
   for (int r = 0; r < n; r++) { p.cnt_all[r] = (int*)cnt_ptrs[r]; p.flags[r] = (unsigned int*)flag_ptrs[r]; }
   p.parity = parity & 1; p.epoch = epoch; p.wait_ns = g_lb_flag_wait_ns;
-  moe_plan_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(p);
-  LB_CHECK_LAUNCH();
-  return LB_OK;
+  return lb_launch_cluster(n == 1, 1, moe_plan_kernel, 1, 256, 0, (cudaStream_t)stream, p);
 }
 
 // dst_ptrs[r] / arrive_ptrs[r]: rank r's destination buffer [cap, H] bf16 and its arrival word.
@@ -634,9 +640,7 @@ extern "C" int lb_moe_push(const void* src, const void* scale, const void* idx, 
   for (int r = 0; r < n; r++) { p.dst[r] = (bf16*)dst_ptrs[r]; p.arrive[r] = (unsigned int*)arrive_ptrs[r]; }
   p.own = p.dst[me];
   p.T = T; p.H = H; p.E = E; p.LE = E / n; p.k = k; p.n = n; p.me = me; p.cap = cap; p.compute_rows = compute_rows;
-  moe_push_kernel<<<moe_grid(T), 256, 0, (cudaStream_t)stream>>>(p);
-  LB_CHECK_LAUNCH();
-  return LB_OK;
+  return lb_launch_cluster(n == 1, 1, moe_push_kernel, moe_grid(T), 256, 0, (cudaStream_t)stream, p);
 }
 
 // src_ptrs[r]: rank r's source buffer [cap, H] bf16; ready_ptrs[r]: rank r's ready words [n] for
@@ -654,10 +658,8 @@ extern "C" int lb_moe_pull(void* out, const void* w, const void* idx, const void
   for (int r = 0; r < n; r++) { p.src[r] = (const bf16*)src_ptrs[r]; p.ready[r] = (unsigned int*)ready_ptrs[r]; }
   p.epoch = epoch; p.wait_ns = g_lb_flag_wait_ns;
   p.T = T; p.H = H; p.E = E; p.LE = E / n; p.k = k; p.n = n; p.me = me; p.cap = cap;
-  (k == 1 ? moe_pull_kernel<1> : k == 2 ? moe_pull_kernel<2> : k <= 4 ? moe_pull_kernel<4> : moe_pull_kernel<8>)
-      <<<moe_grid(T), 256, 0, (cudaStream_t)stream>>>(p);
-  LB_CHECK_LAUNCH();
-  return LB_OK;
+  return lb_launch_cluster(n == 1, 1, k == 1 ? moe_pull_kernel<1> : k == 2 ? moe_pull_kernel<2> : k <= 4 ? moe_pull_kernel<4> : moe_pull_kernel<8>,
+                           moe_grid(T), 256, 0, (cudaStream_t)stream, p);
 }
 
 // dwts [T, k] fp32: gradient of the loss with respect to the routed weights; daux: device pointer to
@@ -668,9 +670,7 @@ extern "C" int lb_moe_router_bwd(const void* x, const void* wg, const void* prob
                                  void* stream) {
   if (T <= 0 || (H % 8) || E < 1 || E > MOE_MAX_EXPERTS || k < 1 || k > MOE_MAX_TOPK) return LB_ERR_SHAPE;
   const dim3 grid((T + RB_TOKENS - 1) / RB_TOKENS, (H + RB_COLS - 1) / RB_COLS);
-  moe_router_bwd_kernel<<<grid, RB_WARPS * 32, 0, (cudaStream_t)stream>>>(
-      (const bf16*)x, (const bf16*)wg, (const float*)probs, (const int*)idx, (const float*)dwts, (const float*)frac,
-      (const float*)daux, (bf16*)dx, (float*)dwg_acc, T, H, E, k);
-  LB_CHECK_LAUNCH();
+  LB_LAUNCH(moe_router_bwd_kernel, grid, RB_WARPS * 32, 0, (cudaStream_t)stream, (const bf16*)x, (const bf16*)wg, (const float*)probs,
+            (const int*)idx, (const float*)dwts, (const float*)frac, (const float*)daux, (bf16*)dx, (float*)dwg_acc, T, H, E, k);
   return LB_OK;
 }

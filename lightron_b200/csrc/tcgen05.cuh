@@ -84,6 +84,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
+// The same box into L2 only: a hint, which may run while another kernel still writes the matrix.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
 // Tile of shared memory -> global memory; elements outside the tensor are not written.  Written by the async proxy: call
 // fence_proxy_async_smem() after filling the tile, bulk_commit() after the store, and bulk_wait_read_but<>() before reusing it.
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {

@@ -485,3 +485,47 @@ def test_clear_writes_its_bytes_and_no_others(n):
     assert not buf[16:16 + n].any() and (buf[:16] == 7).all() and (buf[16 + n:] == 7).all()
     with pytest.raises(native.NativeError):
         native.call("lb_clear", buf.data_ptr() + 8, n, native.stream_ptr())
+
+
+# ---- dependent launches --------------------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 768, 2048), (1000, 4096, 768), (40, 64, 64)])      # split over K, list form, one tile
+@pytest.mark.parametrize("captured", [False, True])
+def test_launches_see_what_the_ones_before_them_wrote(M, N, K, captured):
+    """A launch starts under the tail of the one before it (and asks for its second operand ahead of time): weights that have just been
+    written, and every step of a chain, are the new ones."""
+    from lightron_b200.ops import functional as OF, native
+    a, w0, step = _rand(M, K, seed=1), _rand(N, K, seed=2), _rand(N, K, seed=3, scale=0.125)
+    norm = torch.ones(N, device="cuda", dtype=torch.bfloat16)
+    w, ys = w0.clone(), []
+
+    def chain():
+        for _ in range(6):
+            native.call("lb_add_inplace", w.data_ptr(), step.data_ptr(), w.numel(), native.stream_ptr())
+            y = OF.gemm(a, w)
+            ys.append((y, OF.rmsnorm(y, norm, 1e-5)))
+
+    if captured:
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            chain()                                  # (the first launch of a size uploads its schedule)
+        torch.cuda.synchronize()
+        w.copy_(w0)
+        ys.clear()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            chain()
+        g.replay()
+    else:
+        chain()
+    torch.cuda.synchronize()
+    _status_ok()
+    want_w = w0.clone()
+    for y, n in ys:
+        want_w = (want_w.float() + step.float()).bfloat16()
+        want = a.double() @ want_w.double().t()
+        # bf16 results: half a unit in the last place is 2^-9 of the value
+        assert _rel(y, want) < 5e-3
+        assert _rel(n, y.double() * torch.rsqrt(y.double().square().mean(-1, keepdim=True) + 1e-5)) < 5e-3
+    assert torch.equal(w, want_w)

@@ -38,9 +38,12 @@ int lb_num_sms();
 // grid_go() behind the allocation: a later kernel's CTA could otherwise hold the columns for which an earlier one waits.  Both are no-ops
 // in a plain launch.  Kernels that wait for other GPUs are launched plainly, and so is one of very many short blocks (a block's grid_wait() takes
 // some 0.3 us: 32000 of clear_kernel 31 instead of 23 us).  No grid_go() in kernels that fill an SM's shared memory or registers: the next one's
-// CTAs would crowd into the SMs that are done first (1000 x 768 feed-forward, four launches, 76 instead of 74 us).
+// CTAs would crowd into the SMs that are done first (1000 x 768 feed-forward, four launches, 76 instead of 74 us); for the same reason it does
+// nothing in a grid of many blocks, whose own time is not that of a launch.
 // (Host time of a launch, 700 bytes of parameters, plain / dependent: 3.05 / 2.48 us.)
-__device__ __forceinline__ void grid_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_go() {
+  if (gridDim.x <= 1024) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename T> struct lb_as_is { typedef T type; };      // (arguments convert to the kernel's parameter types)

@@ -35,6 +35,7 @@ namespace {
 
 constexpr int BM = 128, BN = 256, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;
+constexpr int STG_BYTES = 32 * 128;      // 64 columns of the 32 rows of an epilogue warp
 // CG CTAs work on one tile: 1 = a CTA per 128x256 tile, 2 = a pair (tcgen05 cta_group::2) per 256x256 tile, in which
 // each CTA loads its 128 rows of A and half of B.  Per CTA a stage then holds 16 + 16 instead of 16 + 32 KB, and the tensor
 // pipe, whose operand reads from shared memory are what limits and heats it, reads a third less.
@@ -43,7 +44,9 @@ struct Cfg {
   static constexpr int B_BYTES = BN / CG * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = CG == 2 ? 6 : 4;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+  static constexpr int OFF_STG = STAGES * STAGE_BYTES;              // two buffers of every epilogue warp
+  static constexpr int OFF_BAR = OFF_STG + 8 * STG_BYTES;
+  static constexpr int SMEM_BYTES = OFF_BAR + 1024 + 256;
 };
 constexpr int NUM_THREADS = 192;
 constexpr int GROUP_M = 8;
@@ -57,20 +60,20 @@ constexpr int MAX_PROBLEMS = 8;
 //   2  SwiGLU backward: acc is dh [M, half] of the down projection; the epilogue reads g | u from
 //      C2 [M, 2 * half] and writes dg | du to C [M, 2 * half]; dh itself is never stored.
 struct Problem {
-  bf16* C;
-  long long ldc;
-  bf16* C2;
-  long long ldc2;
+  const bf16* old;      // what the epilogue reads: C when accumulate, C2 (g | u) with epi 2
+  long long ld_old;
   int M, N, K;
   int a_mn, b_mn, accumulate;
   int tiles_m, tiles_n, num_kb;
   int epi, half;
 };
 
+template <int NP>
 struct GroupedParams {
-  CUtensorMap ta[MAX_PROBLEMS];
-  CUtensorMap tb[MAX_PROBLEMS];
-  Problem prob[MAX_PROBLEMS];
+  CUtensorMap ta[NP];
+  CUtensorMap tb[NP];
+  CUtensorMap tc[NP][3];      // where the epilogue stores: C; C's gate columns, its up columns, C2; dg, du
+  Problem prob[NP];
   const int* offsets;   // [grid + 1] first item of every CTA
   const int* items;     // (problem << 24) | tile index inside the problem
 };
@@ -162,13 +165,173 @@ __device__ __forceinline__ bool mma_tile(uint32_t d_tmem, int num_kb, uint32_t s
   return true;
 }
 
-template <int CG>
-__global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __grid_constant__ GroupedParams gp) {
+// ---- epilogue of a warp: 32 rows x 256 columns of an accumulator ------------------------------------
+// 64 columns at a time pass through one of the warp's two 4 KB staging buffers (swizzled, a row per lane) and leave by a TMA store, which ends at
+// the matrix's last row and column.  What is read (the old C, or g | u) comes in by loads that cover a row's 64 columns with eight
+// lanes, a step ahead of its use, and turns in the same buffers.  A row per lane read and written straight from memory is 32 lines for every
+// 16 bytes per lane, and kept the load/store unit busy for as long as a main loop of K = 2048 takes (epi 2).  That form / this, us, feed-forward of 16384
+// x 2048 -> 5632: gate | up 562 / 487, down 250 / 245, its gradients with epi 2 696 / 564, gate | up's 1082 / 1055; of 1000 x 768 -> 2048: 12.4 / 11.6,
+// 22.1 / 17.7 (epi 2), 28.9 / 26.7.
+struct Out {
+  const CUtensorMap* map;
+  const bf16* old;
+  long long ld_old;
+  int row0, rows;      // the warp's first row, rows of the matrix
+  int c0, cols;        // first column, columns (of one half, with an activation)
+};
+
+// EPI as in Problem; 3: C = acc + C.  `turn`: which buffer is next, kept over the tiles (the store before the last one has used it).  ready() waits
+// for the accumulator, release() gives its columns back.
+template <int EPI, typename Ready, typename Release>
+__device__ __forceinline__ bool store_tile(const Out& o, uint32_t taddr, uint8_t* stg, int& turn, int lane, Ready ready, Release release) {
+  constexpr bool READS = EPI >= 2;
+  constexpr int NC = EPI == 1 ? BN / 128 : BN / 64;                   // steps of 64 columns
+  uint4 old[READS ? 8 : 1], old2[EPI == 2 ? 8 : 1];
+  const int lr = lane >> 3, lc = (lane & 7) * 8;                      // loads: row (of every four), column
+  auto fetch = [&](int c) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int row = o.row0 + 4 * i + lr, col = o.c0 + c * 64 + lc;
+      const bool in = row < o.rows && col < o.cols;
+      const bf16* at = o.old + (size_t)row * o.ld_old + col;
+      old[i] = in ? *reinterpret_cast<const uint4*>(at) : make_uint4(0, 0, 0, 0);
+      if constexpr (EPI == 2) old2[i] = in ? *reinterpret_cast<const uint4*>(at + o.cols) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  // a buffer to fill: the store before the last one has read it
+  auto next = [&]() -> uint8_t* {
+    if (lane == 0) bw::bulk_wait_read_but<1>();
+    __syncwarp();
+    uint8_t* buf = stg + turn * STG_BYTES;
+    turn ^= 1;
+    return buf;
+  };
+  auto store = [&](const uint8_t* buf, const CUtensorMap* map, int col) {
+    bw::fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      if (o.row0 < o.rows) bw::tma_store_2d(map, bw::smem_u32(buf), col, o.row0);
+      bw::bulk_commit();
+    }
+  };
+  auto at = [&](uint8_t* buf, int g) { return reinterpret_cast<uint4*>(buf + bw::sw128_off(lane, g)); };
+
+  if constexpr (READS) fetch(0);
+  if (!ready()) return false;
+  if constexpr (EPI == 1) {
+    // g and u are stored, and silu(g) * u computed from the ROUNDED values (what a separate pass over the stored
+    // matrix would see, and what the backward recomputes from)
+#pragma unroll 1
+    for (int c = 0; c < NC; c++) {
+      const int col = o.c0 + c * 64;
+      uint32_t r[64];
+      uint4 pg[8], pu[8];
+      auto take = [&](uint32_t from, uint4* packed) {
+        bw::tmem_ld32(from, r);
+        bw::tmem_ld32(from + 32, r + 32);
+        bw::tmem_ld_wait();
+#pragma unroll
+        for (int g = 0; g < 8; g++) packed[g] = pack8(reinterpret_cast<const float*>(r) + g * 8);
+      };
+      take(taddr + c * 64, pg);
+      take(taddr + BN / 2 + c * 64, pu);
+      if (c == NC - 1 || col + 64 >= o.cols) release();
+      uint8_t* buf = next();
+#pragma unroll
+      for (int g = 0; g < 8; g++) *at(buf, g) = pg[g];
+      store(buf, o.map, col);
+      buf = next();
+#pragma unroll
+      for (int g = 0; g < 8; g++) *at(buf, g) = pu[g];
+      store(buf, o.map + 1, col);
+#pragma unroll
+      for (int g = 0; g < 8; g++) {
+        float fg[8], fu[8], h[8];
+        unpack8(pg[g], fg);
+        unpack8(pu[g], fu);
+#pragma unroll
+        for (int i = 0; i < 8; i++) h[i] = fg[i] / (1.f + __expf(-fg[i])) * fu[i];
+        pg[g] = pack8(h);
+      }
+      buf = next();
+#pragma unroll
+      for (int g = 0; g < 8; g++) *at(buf, g) = pg[g];
+      store(buf, o.map + 2, col);
+      if (col + 64 >= o.cols) break;
+    }
+  } else {
+#pragma unroll 1
+    for (int c = 0; c < NC; c++) {
+      const int col = o.c0 + c * 64;
+      const bool last = c == NC - 1 || col + 64 >= o.cols;
+      uint8_t *buf, *buf2 = nullptr;
+      if constexpr (EPI == 2) {                                       // both buffers, the first of which is stored first
+        if (lane == 0) bw::bulk_wait_read_but<0>();
+        __syncwarp();
+        buf = stg;
+        buf2 = stg + STG_BYTES;
+        turn = 0;
+      } else {
+        buf = next();
+      }
+      if constexpr (READS) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const uint32_t to = bw::sw128_off(4 * i + lr, lane & 7);
+          *reinterpret_cast<uint4*>(buf + to) = old[i];
+          if constexpr (EPI == 2) *reinterpret_cast<uint4*>(buf2 + to) = old2[i];
+        }
+        if (!last) fetch(c + 1);
+      }
+      uint32_t r[64];
+      bw::tmem_ld32(taddr + c * 64, r);
+      bw::tmem_ld32(taddr + c * 64 + 32, r + 32);
+      bw::tmem_ld_wait();
+      if (last) release();
+      if constexpr (READS) __syncwarp();
+#pragma unroll
+      for (int g = 0; g < 8; g++) {
+        float f[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[g * 8 + i]);
+        if constexpr (EPI == 2) {
+          float fg[8], fu[8], dg[8], du[8];
+          unpack8(pack8(f), f);                                       // the value a stored bf16 dh would have had
+          unpack8(*at(buf, g), fg);
+          unpack8(*at(buf2, g), fu);
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const float sig = 1.f / (1.f + __expf(-fg[i]));
+            dg[i] = f[i] * fu[i] * sig * (1.f + fg[i] * (1.f - sig));
+            du[i] = f[i] * fg[i] * sig;
+          }
+          *at(buf, g) = pack8(dg);
+          *at(buf2, g) = pack8(du);
+        } else {
+          if constexpr (EPI == 3) {
+            float e[8];
+            unpack8(*at(buf, g), e);
+#pragma unroll
+            for (int i = 0; i < 8; i++) f[i] += e[i];
+          }
+          *at(buf, g) = pack8(f);
+        }
+      }
+      store(buf, o.map, col);
+      if constexpr (EPI == 2) store(buf2, o.map + 1, col);
+      if (last) break;
+    }
+  }
+  return true;
+}
+
+template <int CG, int NP>
+__global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __grid_constant__ GroupedParams<NP> gp) {
   using CF = Cfg<CG>;
   constexpr int STAGES = CF::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * CF::STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + CF::OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   __shared__ int s_abort[2];     // {abort, extra wait in ms}: see bw::mbar_wait
 
@@ -278,7 +441,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
   } else {
     // ------------------------------ epilogue (4 warps) ------------------------------
     const int quad = warp & 3;
-    int n = 0;
+    uint8_t* stg = smem + CF::OFF_STG + quad * 2 * STG_BYTES;
+    int n = 0, turn = 0;
     int next_item = item_begin < item_end ? gp.items[item_begin] : 0;
     for (int it = item_begin; it < item_end; it++, n++) {
       const int item = next_item;
@@ -286,156 +450,34 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
       const int pi = item >> 24;
       int tm, tn;
       tile_coords(item & 0xFFFFFF, gp.prob[pi], tm, tn);
-      const int pM = gp.prob[pi].M, pN = gp.prob[pi].N;
-      const bool accumulate = gp.prob[pi].accumulate != 0;
-      bf16* const pC = gp.prob[pi].C;
-      const long long ldc = gp.prob[pi].ldc;
+      const Problem& pr = gp.prob[pi];
       const int acc = n & 1;
       const uint32_t acc_phase = (uint32_t)(n >> 1) & 1u;
-      const int row = (tm * CG + rank) * BM + quad * 32 + lane;
-      const int n0 = tn * BN;
-      if (gp.prob[pi].epi == 2 && row < pM) {
-        // while the MMAs of this tile run: pull the g | u values its epilogue will read into L2
-        const bf16* pre = gp.prob[pi].C2 + (size_t)row * gp.prob[pi].ldc2 + n0;
-        const int half = gp.prob[pi].half;
-#pragma unroll
-        for (int l = 0; l < BN / 64; l++) {
-          if (n0 + l * 64 < half) {
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(pre + l * 64));
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(pre + half + l * 64));
-          }
-        }
-      }
-      if (!bw::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) { give_up(abort_flag, 4u); break; }
-      bw::fence_after();
+      const Out out{gp.tc[pi], pr.old, pr.ld_old, (tm * CG + rank) * BM + quad * 32, pr.M, tn * (pr.epi == 1 ? BN / 2 : BN), pr.epi ? pr.half : pr.N};
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * BN;
-      bf16* crow = pC + (size_t)row * ldc + n0;
-      const int epi = gp.prob[pi].epi;
-      if (epi == 1) {
-        // gate | up tile: store both, and silu(g) * u computed from the ROUNDED values (what a
-        // separate pass over the stored matrix would see, and what the backward recomputes from)
-        const int half = gp.prob[pi].half;
-        const int c0 = tn * (BN / 2);
-        bf16* grow = pC + (size_t)row * ldc + c0;
-        bf16* hrow = gp.prob[pi].C2 + (size_t)row * gp.prob[pi].ldc2 + c0;
-#pragma unroll 1
-        for (int c = 0; c < BN / 64; c++) {
-          uint32_t rg[32], ru[32];
-          bw::tmem_ld32(taddr + c * 32, rg);
-          bw::tmem_ld32(taddr + BN / 2 + c * 32, ru);
-          bw::tmem_ld_wait();
-          if (row < pM) {
-#pragma unroll
-            for (int g = 0; g < 4; g++) {
-              if (c0 + c * 32 + g * 8 < half) {
-                float fg[8], fu[8], h[8];
-#pragma unroll
-                for (int i = 0; i < 8; i++) { fg[i] = __uint_as_float(rg[g * 8 + i]); fu[i] = __uint_as_float(ru[g * 8 + i]); }
-                const uint4 pg = pack8(fg), pu = pack8(fu);
-                *reinterpret_cast<uint4*>(grow + c * 32 + g * 8) = pg;
-                *reinterpret_cast<uint4*>(grow + half + c * 32 + g * 8) = pu;
-                unpack8(pg, fg);
-                unpack8(pu, fu);
-#pragma unroll
-                for (int i = 0; i < 8; i++) h[i] = fg[i] / (1.f + __expf(-fg[i])) * fu[i];
-                *reinterpret_cast<uint4*>(hrow + c * 32 + g * 8) = pack8(h);
-              }
-            }
-          }
-        }
+      auto ready = [&]() {
+        if (!bw::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) return false;
+        bw::fence_after();
+        return true;
+      };
+      auto release = [&]() {
         bw::fence_before();
         __syncwarp();
         if (lane == 0) {
           if constexpr (CG == 2) bw::mbar_arrive_leader(tempty_bar(acc));
           else bw::mbar_arrive(tempty_bar(acc));
         }
-        continue;
+      };
+      bool ok;
+      switch (pr.epi == 0 && pr.accumulate ? 3 : pr.epi) {
+        case 0: ok = store_tile<0>(out, taddr, stg, turn, lane, ready, release); break;
+        case 1: ok = store_tile<1>(out, taddr, stg, turn, lane, ready, release); break;
+        case 2: ok = store_tile<2>(out, taddr, stg, turn, lane, ready, release); break;
+        default: ok = store_tile<3>(out, taddr, stg, turn, lane, ready, release); break;
       }
-      if (epi == 2) {
-        // dh tile of the down projection -> dg | du, with g | u read from C2.  The 8 loads of a
-        // 32-column chunk are issued together, and the chunk after it is already in flight, before
-        // anything is stored (a store in between would order the loads behind it).
-        const int half = gp.prob[pi].half;
-        const bf16* gurow = gp.prob[pi].C2 + (size_t)row * gp.prob[pi].ldc2 + n0;
-        const bool row_ok = row < pM;
-        uint4 gq[2][4], uq[2][4];
-        auto fetch = [&](int c, int buf) {
-#pragma unroll
-          for (int g = 0; g < 4; g++) {
-            const bool ok = row_ok && (n0 + c * 32 + g * 8 < half);
-            gq[buf][g] = ok ? __ldg(reinterpret_cast<const uint4*>(gurow + c * 32 + g * 8)) : make_uint4(0, 0, 0, 0);
-            uq[buf][g] = ok ? __ldg(reinterpret_cast<const uint4*>(gurow + half + c * 32 + g * 8)) : make_uint4(0, 0, 0, 0);
-          }
-        };
-        fetch(0, 0);
-#pragma unroll
-        for (int c = 0; c < BN / 32; c++) {
-          if (c + 1 < BN / 32) fetch(c + 1, (c + 1) & 1);
-          uint32_t r[32];
-          bw::tmem_ld32(taddr + c * 32, r);
-          bw::tmem_ld_wait();
-          if (row_ok) {
-#pragma unroll
-            for (int g = 0; g < 4; g++) {
-              if (n0 + c * 32 + g * 8 < half) {
-                float d[8], fg[8], fu[8], dg[8], du[8];
-#pragma unroll
-                for (int i = 0; i < 8; i++) d[i] = __uint_as_float(r[g * 8 + i]);
-                unpack8(pack8(d), d);                 // the value a stored bf16 dh would have had
-                unpack8(gq[c & 1][g], fg);
-                unpack8(uq[c & 1][g], fu);
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                  const float sig = 1.f / (1.f + __expf(-fg[i]));
-                  dg[i] = d[i] * fu[i] * sig * (1.f + fg[i] * (1.f - sig));
-                  du[i] = d[i] * fg[i] * sig;
-                }
-                *reinterpret_cast<uint4*>(crow + c * 32 + g * 8) = pack8(dg);
-                *reinterpret_cast<uint4*>(crow + half + c * 32 + g * 8) = pack8(du);
-              }
-            }
-          }
-        }
-        bw::fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          if constexpr (CG == 2) bw::mbar_arrive_leader(tempty_bar(acc));
-          else bw::mbar_arrive(tempty_bar(acc));
-        }
-        continue;
-      }
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; c++) {
-        uint32_t r[32];
-        bw::tmem_ld32(taddr + c * 32, r);
-        bw::tmem_ld_wait();
-        if (row < pM) {
-#pragma unroll
-          for (int g = 0; g < 4; g++) {
-            const int col = n0 + c * 32 + g * 8;
-            if (col < pN) {
-              float f[8];
-#pragma unroll
-              for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[g * 8 + i]);
-              uint4* dst = reinterpret_cast<uint4*>(crow + c * 32 + g * 8);
-              if (accumulate) {
-                float o[8];
-                unpack8(*dst, o);
-#pragma unroll
-                for (int i = 0; i < 8; i++) f[i] += o[i];
-              }
-              *dst = pack8(f);
-            }
-          }
-        }
-      }
-      bw::fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if constexpr (CG == 2) bw::mbar_arrive_leader(tempty_bar(acc));
-        else bw::mbar_arrive(tempty_bar(acc));
-      }
+      if (!ok) { give_up(abort_flag, 4u); break; }
     }
+    if (lane == 0) bw::bulk_wait_read_but<0>();        // nothing reads shared memory after the CTA's end
   }
 
   bw::fence_before();
@@ -463,8 +505,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
 struct RaggedParams {
   CUtensorMap ta;                      // mode 0: [cap, K] K-major;  mode 1: [cap, Nw] as MN-major A
   CUtensorMap tb[MAX_PROBLEMS];        // mode 0: B_e;               mode 1: tb[0] = [cap, Kw] as MN-major B
-  bf16* C[MAX_PROBLEMS];               // mode 0: C[0] = common [cap, N];  mode 1: C_e
+  CUtensorMap tc[MAX_PROBLEMS];        // mode 0: tc[0..2] as in GroupedParams, of matrices of cap rows;  mode 1: C_e
+  bf16* C[MAX_PROBLEMS];               // mode 1: C_e
   long long ldc;
+  const bf16* old;                     // mode 0, epi 2: g | u
+  long long ld_old;
+  int epi, half;
   const int* seg;
   int LE, M_w, N, K, b_mn, mode, accumulate, cap;
   int tiles_n, tiles_m_w, num_kb;
@@ -487,7 +533,7 @@ __device__ __forceinline__ RaggedTile ragged_tile(int t, const RaggedParams& rp,
         pr.tiles_m = s_tiles[e]; pr.tiles_n = rp.tiles_n;
         int tm, tn;
         tile_coords(t, pr, tm, tn);
-        r.e = e; r.m0 = s_off[e] + tm * BM; r.n0 = tn * BN; r.num_kb = rp.num_kb;
+        r.e = e; r.m0 = s_off[e] + tm * BM; r.n0 = tn * (rp.epi == 1 ? BN / 2 : BN); r.num_kb = rp.num_kb;
         return r;
       }
       t -= nt;
@@ -510,7 +556,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
   constexpr int STAGES = CF::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * CF::STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + CF::OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   __shared__ int s_abort[2];     // {abort, extra wait in ms}: see bw::mbar_wait
   __shared__ int s_off[MAX_PROBLEMS], s_tiles[MAX_PROBLEMS];
@@ -572,7 +618,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
         if (rt.e < 0) break;
         if (rt.num_kb == 0) continue;
         if (rp.mode == 0) {
-          if (!rp.b_mn) ok = produce_tile<1, false, false>(&rp.ta, &rp.tb[rt.e], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, true);
+          if (!rp.b_mn) ok = produce_tile<1, false, false>(&rp.ta, &rp.tb[rt.e], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, true, 0, rp.epi == 1 ? rp.half : 0);
           else          ok = produce_tile<1, false, true>(&rp.ta, &rp.tb[rt.e], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, true);
         } else {
           ok = produce_tile<1, true, true>(&rp.ta, &rp.tb[0], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, true, rt.k_base);
@@ -610,7 +656,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
   } else {
     // ------------------------------ epilogue (4 warps) ------------------------------
     const int quad = warp & 3;
-    int n = 0;
+    uint8_t* stg = smem + CF::OFF_STG + quad * 2 * STG_BYTES;
+    int n = 0, turn = 0;
     for (int t = blockIdx.x;; t += gridDim.x) {
       const RaggedTile rt = ragged_tile(t, rp, s_off, s_tiles);
       if (rt.e < 0) break;
@@ -624,44 +671,32 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
       }
       const int acc = n & 1;
       const uint32_t acc_phase = (uint32_t)(n >> 1) & 1u;
-      if (!bw::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) { give_up(abort_flag, 4u); break; }
-      bw::fence_after();
-      const int row = rt.m0 + quad * 32 + lane;
-      const int row_end = rp.mode == 0 ? rp.cap : rp.M_w;      // mode 0 writes whole 128-row tiles (padding rows are zeros)
-      bf16* const pC = rp.mode == 0 ? rp.C[0] : rp.C[rt.e];
-      const bool accumulate = rp.accumulate != 0;
+      const bool wgrad = rp.mode == 1;
+      // (mode 0 writes whole 128-row tiles: padding rows are zeros)
+      const Out out{wgrad ? &rp.tc[rt.e] : rp.tc, wgrad ? rp.C[rt.e] : rp.old, wgrad ? rp.ldc : rp.ld_old, rt.m0 + quad * 32, wgrad ? rp.M_w : rp.cap,
+                    rt.n0, rp.epi ? rp.half : rp.N};
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * BN;
-      bf16* crow = pC + (size_t)row * rp.ldc + rt.n0;
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; c++) {
-        uint32_t r[32];
-        bw::tmem_ld32(taddr + c * 32, r);
-        bw::tmem_ld_wait();
-        if (row < row_end) {
-#pragma unroll
-          for (int g = 0; g < 4; g++) {
-            const int col = rt.n0 + c * 32 + g * 8;
-            if (col < rp.N) {
-              float f[8];
-#pragma unroll
-              for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[g * 8 + i]);
-              uint4* dst = reinterpret_cast<uint4*>(crow + c * 32 + g * 8);
-              if (accumulate) {
-                float o[8];
-                unpack8(*dst, o);
-#pragma unroll
-                for (int i = 0; i < 8; i++) f[i] += o[i];
-              }
-              *dst = pack8(f);
-            }
-          }
-        }
+      auto ready = [&]() {
+        if (!bw::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) return false;
+        bw::fence_after();
+        return true;
+      };
+      auto release = [&]() {
+        bw::fence_before();
+        __syncwarp();
+        if (lane == 0) bw::mbar_arrive(tempty_bar(acc));
+      };
+      bool ok;
+      switch (wgrad && rp.accumulate ? 3 : rp.epi) {
+        case 0: ok = store_tile<0>(out, taddr, stg, turn, lane, ready, release); break;
+        case 1: ok = store_tile<1>(out, taddr, stg, turn, lane, ready, release); break;
+        case 2: ok = store_tile<2>(out, taddr, stg, turn, lane, ready, release); break;
+        default: ok = store_tile<3>(out, taddr, stg, turn, lane, ready, release); break;
       }
-      bw::fence_before();
-      __syncwarp();
-      if (lane == 0) bw::mbar_arrive(tempty_bar(acc));
+      if (!ok) { give_up(abort_flag, 4u); break; }
       n++;
     }
+    if (lane == 0) bw::bulk_wait_read_but<0>();        // nothing reads shared memory after the CTA's end
   }
 
   bw::fence_before();
@@ -801,6 +836,46 @@ int build_schedule(Problem* probs, int np, int sms, Schedule* out) {
   return LB_OK;
 }
 
+// Map of the 64-column, 32-row boxes that an epilogue warp stores.
+int out_map(CUtensorMap* m, const bf16* base, int cols, int rows, long long ld) {
+  return bw::make_map_bf16(m, base, (uint64_t)cols, (uint64_t)rows, (uint64_t)ld, 64, 32);
+}
+// The maps of a problem's outputs (see GroupedParams::tc).
+int out_maps(CUtensorMap* tc, void* C, void* C2, long long ldc, long long ldc2, int rows, int N, int epi, int half) {
+  bf16* c = (bf16*)C;
+  if (!epi) return out_map(tc, c, N, rows, ldc);
+  int rc = out_map(tc, c, half, rows, ldc);
+  if (!rc) rc = out_map(tc + 1, c + half, half, rows, ldc);
+  if (!rc && epi == 1) rc = out_map(tc + 2, (const bf16*)C2, half, rows, ldc2);
+  return rc;
+}
+
+struct Operands {
+  const void *const *A, *const *B;
+  void *const *C, *const *C2;
+  const long long *lda, *ldb, *ldc, *ldc2;
+};
+template <int NP>
+int launch_grouped(int n, const Problem* probs, const Operands& op, const Schedule& sched, cudaStream_t s) {
+  static thread_local GroupedParams<NP> gp;         // up to 5.5 KB of tensor maps: kept off the stack, one per calling thread
+  for (int i = 0; i < n; i++) {
+    const Problem& p = gp.prob[i] = probs[i];
+    int rc;
+    if (!p.a_mn) rc = bw::make_map_bf16(&gp.ta[i], op.A[i], (uint64_t)p.K, (uint64_t)p.M, (uint64_t)op.lda[i], BK, BM);
+    else         rc = bw::make_map_bf16(&gp.ta[i], op.A[i], (uint64_t)p.M, (uint64_t)p.K, (uint64_t)op.lda[i], 64, BK);
+    if (rc) return rc;
+    if (!p.b_mn) rc = bw::make_map_bf16(&gp.tb[i], op.B[i], (uint64_t)p.K, (uint64_t)p.N, (uint64_t)op.ldb[i], BK, BN / 2);
+    else         rc = bw::make_map_bf16(&gp.tb[i], op.B[i], (uint64_t)p.N, (uint64_t)p.K, (uint64_t)op.ldb[i], 64, BK);
+    if (rc) return rc;
+    if ((rc = out_maps(gp.tc[i], op.C[i], p.epi ? op.C2[i] : nullptr, op.ldc[i], p.epi ? op.ldc2[i] : 0, p.M, p.N, p.epi, p.half))) return rc;
+  }
+  gp.offsets = sched.d_offsets;
+  gp.items = sched.d_items;
+  if (sched.cg == 2)      // a pair is a cluster of two CTAs
+    return lb_launch_cluster(true, 2, gemm_grouped_kernel<2, NP>, 2 * sched.grid, NUM_THREADS, Cfg<2>::SMEM_BYTES, s, gp);
+  return lb_launch(gemm_grouped_kernel<1, NP>, sched.grid, NUM_THREADS, Cfg<1>::SMEM_BYTES, s, gp);
+}
+
 }  // namespace
 
 // Copies the status words of the grouped GEMM kernel to host memory and clears them.
@@ -882,7 +957,7 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
                                    const int* epi, void* const* C2, const long long* ldc2, const int* half,
                                    void* stream) {
   if (n < 1 || n > MAX_PROBLEMS) return LB_ERR_SHAPE;
-  static thread_local GroupedParams gp;         // 2.5 KB of tensor maps: kept off the stack, one per calling thread
+  Problem probs[MAX_PROBLEMS];
   std::vector<int> key;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -899,9 +974,9 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
       if (e == 2 && N[i] != half[i]) return LB_ERR_SHAPE;
       if (accumulate && accumulate[i]) return LB_ERR_ARG;
     }
-    Problem& p = gp.prob[i];
-    p.C = (bf16*)C[i]; p.ldc = ldc[i]; p.M = M[i]; p.N = N[i]; p.K = K[i];
-    p.C2 = e ? (bf16*)C2[i] : nullptr; p.ldc2 = e ? ldc2[i] : 0; p.epi = e; p.half = e ? half[i] : 0;
+    Problem& p = probs[i];
+    p.M = M[i]; p.N = N[i]; p.K = K[i]; p.epi = e; p.half = e ? half[i] : 0;
+    p.old = (const bf16*)(e == 2 ? C2[i] : C[i]); p.ld_old = e == 2 ? ldc2[i] : ldc[i];
     p.a_mn = a_mn[i]; p.b_mn = b_mn[i]; p.accumulate = accumulate ? accumulate[i] : 0;
     key.push_back(M[i]); key.push_back(N[i]); key.push_back(K[i]);
   }
@@ -909,8 +984,10 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
     std::lock_guard<std::mutex> lock(g_sched_mutex);
     if (g_sms == 0) {
       cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-      cudaFuncSetAttribute(gemm_grouped_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
-      cudaFuncSetAttribute(gemm_grouped_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
+      cudaFuncSetAttribute(gemm_grouped_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
+      cudaFuncSetAttribute(gemm_grouped_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
+      cudaFuncSetAttribute(gemm_grouped_kernel<1, MAX_PROBLEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
+      cudaFuncSetAttribute(gemm_grouped_kernel<2, MAX_PROBLEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
     }
   }
   Schedule sched;
@@ -919,7 +996,7 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
     auto it = g_schedules.find(key);
     if (it == g_schedules.end()) {
       Schedule s;
-      int rc = build_schedule(gp.prob, n, g_sms, &s);
+      int rc = build_schedule(probs, n, g_sms, &s);
       if (rc) return rc;
       const bool split = s.split > 0;
       if (++g_cached[split] > (split ? MAX_SPLITS : MAX_SCHEDULES)) {
@@ -941,22 +1018,9 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
   }
   if (sched.split)
     return lb_gemm_split(n, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, epi, C2, ldc2, half, sched.split, stream);
-  for (int i = 0; i < n; i++) {
-    int rc;
-    if (!a_mn[i]) rc = bw::make_map_bf16(&gp.ta[i], A[i], (uint64_t)K[i], (uint64_t)M[i], (uint64_t)lda[i], BK, BM);
-    else          rc = bw::make_map_bf16(&gp.ta[i], A[i], (uint64_t)M[i], (uint64_t)K[i], (uint64_t)lda[i], 64, BK);
-    if (rc) return rc;
-    if (!b_mn[i]) rc = bw::make_map_bf16(&gp.tb[i], B[i], (uint64_t)K[i], (uint64_t)N[i], (uint64_t)ldb[i], BK, BN / 2);
-    else          rc = bw::make_map_bf16(&gp.tb[i], B[i], (uint64_t)N[i], (uint64_t)K[i], (uint64_t)ldb[i], 64, BK);
-    if (rc) return rc;
-  }
-  gp.offsets = sched.d_offsets;
-  gp.items = sched.d_items;
-  for (int i = 0; i < n; i++) set_tiles(&gp.prob[i], sched.cg);
-  if (sched.cg == 2)      // a pair is a cluster of two CTAs
-    return lb_launch_cluster(true, 2, gemm_grouped_kernel<2>, 2 * sched.grid, NUM_THREADS, Cfg<2>::SMEM_BYTES, (cudaStream_t)stream, gp);
-  LB_LAUNCH(gemm_grouped_kernel<1>, sched.grid, NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream, gp);
-  return LB_OK;
+  for (int i = 0; i < n; i++) set_tiles(&probs[i], sched.cg);
+  const Operands op{A, B, C, C2, lda, ldb, ldc, ldc2};
+  return n <= 2 ? launch_grouped<2>(n, probs, op, sched, (cudaStream_t)stream) : launch_grouped<MAX_PROBLEMS>(n, probs, op, sched, (cudaStream_t)stream);
 }
 
 
@@ -989,7 +1053,8 @@ extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, cons
     if (rc) return rc;
     rp.C[e] = nullptr;
   }
-  rp.C[0] = (bf16*)C; rp.ldc = ldc; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = 0; rp.N = N; rp.K = K; rp.b_mn = b_mn;
+  if ((rc = out_maps(rp.tc, C, nullptr, ldc, 0, cap, N, 0, 0))) return rc;
+  rp.ldc = ldc; rp.old = nullptr; rp.ld_old = 0; rp.epi = 0; rp.half = 0; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = 0; rp.N = N; rp.K = K; rp.b_mn = b_mn;
   rp.mode = 0; rp.accumulate = 0; rp.cap = cap;
   rp.tiles_n = (N + BN - 1) / BN; rp.tiles_m_w = 0; rp.num_kb = (K + BK - 1) / BK;
   rp.wait_flag = (const unsigned int*)wait_flag; rp.wait_target = wait_target; rp.wait_ns = g_lb_flag_wait_ns;
@@ -1017,8 +1082,9 @@ extern "C" int lb_gemm_ragged_wgrad(const void* dY, const void* X, void* const* 
   for (int e = 0; e < LE; e++) {
     if ((uintptr_t)C[e] & 15) return LB_ERR_ARG;
     rp.C[e] = (bf16*)C[e];
+    if ((rc = out_map(&rp.tc[e], rp.C[e], Kw, Nw, ldc))) return rc;
   }
-  rp.ldc = ldc; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = Nw; rp.N = Kw; rp.K = 0; rp.b_mn = 1; rp.mode = 1;
+  rp.ldc = ldc; rp.old = nullptr; rp.ld_old = 0; rp.epi = 0; rp.half = 0; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = Nw; rp.N = Kw; rp.K = 0; rp.b_mn = 1; rp.mode = 1;
   rp.accumulate = accumulate; rp.cap = cap;
   rp.tiles_n = (Kw + BN - 1) / BN; rp.tiles_m_w = (Nw + BM - 1) / BM; rp.num_kb = 0;
   rp.wait_flag = nullptr; rp.wait_target = 0; rp.wait_ns = g_lb_flag_wait_ns;

@@ -1037,12 +1037,18 @@ extern "C" int lb_gemm_grouped(int n, const void* const* A, const void* const* B
 //  mode 0: C [cap, N] = A [cap, K] . op(B_e)^T per segment; B: host array of LE weight pointers
 //          ([N, K], or [K, N] with b_mn), all with leading dimension ldb.  wait_flag (or null): device
 //          word that must reach wait_target before A is read.
-extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, const void* seg, int LE, int cap, int N, int K,
-                              long long lda, long long ldb, long long ldc, int b_mn, const void* wait_flag,
-                              unsigned int wait_target, void* stream) {
+//          epi, C2, ldc2 and half as in lb_gemm_grouped_epi (matrices of cap rows).
+extern "C" int lb_gemm_ragged_epi(const void* A, const void* const* B, void* C, const void* seg, int LE, int cap, int N, int K,
+                                  long long lda, long long ldb, long long ldc, int b_mn, int epi, void* C2, long long ldc2, int half,
+                                  const void* wait_flag, unsigned int wait_target, void* stream) {
   if (LE < 1 || LE > MAX_PROBLEMS || cap <= 0 || N <= 0 || K <= 0) return LB_ERR_SHAPE;
   if ((lda % 8) || (ldb % 8) || (ldc % 8) || (N % 8) || (K % 8)) return LB_ERR_SHAPE;
   if (((uintptr_t)A | (uintptr_t)C) & 15) return LB_ERR_ARG;
+  if (epi < 0 || epi > 2) return LB_ERR_ARG;
+  if (epi) {
+    if (!C2 || ((uintptr_t)C2 & 15) || (ldc2 % 8) || half <= 0 || (half % 8)) return LB_ERR_ARG;
+    if (epi == 1 ? (b_mn || N != 2 * half) : N != half) return LB_ERR_SHAPE;
+  }
   static thread_local RaggedParams rp;
   int rc = bw::make_map_bf16(&rp.ta, A, (uint64_t)K, (uint64_t)cap, (uint64_t)lda, BK, BM);
   if (rc) return rc;
@@ -1053,8 +1059,8 @@ extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, cons
     if (rc) return rc;
     rp.C[e] = nullptr;
   }
-  if ((rc = out_maps(rp.tc, C, nullptr, ldc, 0, cap, N, 0, 0))) return rc;
-  rp.ldc = ldc; rp.old = nullptr; rp.ld_old = 0; rp.epi = 0; rp.half = 0; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = 0; rp.N = N; rp.K = K; rp.b_mn = b_mn;
+  if ((rc = out_maps(rp.tc, C, C2, ldc, ldc2, cap, N, epi, half))) return rc;
+  rp.ldc = ldc; rp.old = (const bf16*)C2; rp.ld_old = ldc2; rp.epi = epi; rp.half = half; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = 0; rp.N = N; rp.K = K; rp.b_mn = b_mn;
   rp.mode = 0; rp.accumulate = 0; rp.cap = cap;
   rp.tiles_n = (N + BN - 1) / BN; rp.tiles_m_w = 0; rp.num_kb = (K + BK - 1) / BK;
   rp.wait_flag = (const unsigned int*)wait_flag; rp.wait_target = wait_target; rp.wait_ns = g_lb_flag_wait_ns;
@@ -1064,6 +1070,12 @@ extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, cons
     if (!attr) { cudaFuncSetAttribute(gemm_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES); attr = true; }
   }
   return lb_launch_cluster(!wait_flag, 1, gemm_ragged_kernel, lb_num_sms(), NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream, rp);
+}
+
+extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, const void* seg, int LE, int cap, int N, int K,
+                              long long lda, long long ldb, long long ldc, int b_mn, const void* wait_flag,
+                              unsigned int wait_target, void* stream) {
+  return lb_gemm_ragged_epi(A, B, C, seg, LE, cap, N, K, lda, ldb, ldc, b_mn, 0, nullptr, 0, 0, wait_flag, wait_target, stream);
 }
 
 //  Weight gradients: C_e [Nw, Kw] (+)= dY[rows of e, Nw]^T . X[rows of e, Kw]; C: host array of LE

@@ -72,8 +72,10 @@ _SIGNATURES = {
     "lb_moe_plan": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _I, ctypes.c_uint, _P],
     "lb_moe_push": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P],
     "lb_moe_pull": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, ctypes.c_uint, _P],
+    "lb_moe_pull_add": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, ctypes.c_uint, _P],
     "lb_moe_router_bwd": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
     "lb_gemm_ragged": [_P, _P, _P, _P, _I, _I, _I, _I, _L, _L, _L, _I, _P, ctypes.c_uint, _P],
+    "lb_gemm_ragged_epi": [_P, _P, _P, _P, _I, _I, _I, _I, _L, _L, _L, _I, _I, _P, _L, _I, _P, ctypes.c_uint, _P],
     "lb_gemm_ragged_wgrad": [_P, _P, _P, _P, _I, _I, _I, _I, _L, _L, _L, _I, _P],
     "lb_swiglu_fwd_dev": [_P, _P, _I, _I, _L, _P, _P],
     "lb_swiglu_bwd_dev": [_P, _P, _P, _I, _I, _L, _P, _P],

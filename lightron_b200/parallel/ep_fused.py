@@ -143,10 +143,12 @@ def _ptr_array(tensors: Sequence[torch.Tensor]):
     return arr
 
 
-def _ragged(A, B_list, C, seg, LE, cap, N, K, b_mn, wait_flag=0, wait_target=0):
+def _ragged(A, B_list, C, seg, LE, cap, N, K, b_mn, wait_flag=0, wait_target=0, epi=0, c2=None, half=0):
+    """``epi``, ``c2`` and ``half``: a SwiGLU epilogue, as in ``functional.gemm_grouped``."""
     ldb = B_list[0].stride(0)
-    native.call("lb_gemm_ragged", A.data_ptr(), _ptr_array(B_list), C.data_ptr(), seg.data_ptr(), LE, cap, N, K,
-                A.stride(0), ldb, C.stride(0), int(b_mn), wait_flag, wait_target, native.stream_ptr())
+    native.call("lb_gemm_ragged_epi", A.data_ptr(), _ptr_array(B_list), C.data_ptr(), seg.data_ptr(), LE, cap, N, K,
+                A.stride(0), ldb, C.stride(0), int(b_mn), epi, native.ptr(c2), 0 if c2 is None else c2.stride(0), half,
+                wait_flag, wait_target, native.stream_ptr())
 
 
 def _ragged_wgrad(dY, X, C_list, seg, LE, cap, Nw, Kw, accumulate=True):
@@ -170,14 +172,14 @@ class _FusedMoE(torch.autograd.Function):
         probs = torch.empty(T, E, dtype=_F32, device=dev)
         idx = torch.empty(T, k, dtype=_I32, device=dev)
         wts = torch.empty(T, k, dtype=_F32, device=dev)
-        within = torch.zeros(nblk * 32, k, dtype=_I32, device=dev)
+        within = torch.empty(nblk * 32, k, dtype=_I32, device=dev)
         blk_hist = torch.empty(nblk, E, dtype=_I32, device=dev)
         blk_psum = torch.empty(nblk, E, dtype=_F32, device=dev)
         native.call("lb_moe_router", x.data_ptr(), gate_w.data_ptr(), T, H, E, k, probs.data_ptr(), idx.data_ptr(),
                     wts.data_ptr(), within.data_ptr(), blk_hist.data_ptr(), blk_psum.data_ptr(), st())
         blk_base = torch.empty(nblk, E, dtype=_I32, device=dev)
         dst_row0 = torch.empty(E, dtype=_I32, device=dev)
-        seg = torch.zeros(2 * LE + 2, dtype=_I32, device=dev)
+        seg = torch.empty(2 * LE + 2, dtype=_I32, device=dev)
         frac = torch.empty(E, dtype=_F32, device=dev)
         aux = torch.empty(1, dtype=_F32, device=dev)
         ws.epoch_cnt += 1
@@ -195,10 +197,8 @@ class _FusedMoE(torch.autograd.Function):
         ups = [OF._as_strided_cat(expert_ws[3 * e:3 * e + 2]) for e in range(LE)]       # [2I, H] gate | up
         downs = [expert_ws[3 * e + 2] for e in range(LE)]                               # [H, I]
         gu = torch.empty(cap, 2 * I, dtype=_BF16, device=dev)
-        _ragged(xbuf, ups, gu, seg, LE, cap, 2 * I, H, False, ws.ctrl_ptrs[me] + 64, ws.arr_x)
         a = torch.empty(cap, I, dtype=_BF16, device=dev)
-        rows_dev = seg.data_ptr() + 4 * (2 * LE)                                          # padded end of the last segment
-        native.call("lb_swiglu_fwd_dev", gu.data_ptr(), a.data_ptr(), cap, I, gu.stride(0), rows_dev, st())
+        _ragged(xbuf, ups, gu, seg, LE, cap, 2 * I, H, False, ws.ctrl_ptrs[me] + 64, ws.arr_x, epi=1, c2=a, half=I)
         _ragged(a, downs, ybuf, seg, LE, cap, H, I, False)
         out = torch.empty(T, H, dtype=_BF16, device=dev)
         ws.epoch_y += 1
@@ -246,21 +246,13 @@ class _FusedMoE(torch.autograd.Function):
             g_down = [torch.empty(H, I, dtype=_BF16, device=dev) for _ in range(LE)]
         ups = [OF._as_strided_cat(expert_ws[3 * e:3 * e + 2]) for e in range(LE)]
         downs = [expert_ws[3 * e + 2] for e in range(LE)]
-        # down projection: da = dy W2, dW2 += dy^T a
-        da = torch.empty(cap, I, dtype=_BF16, device=dev)
-        _ragged(dybuf, downs, da, seg, LE, cap, I, H, True, ws.ctrl_ptrs[me] + 68, ws.arr_dy)
-        _ragged_wgrad(dybuf, a, g_down, seg, LE, cap, H, I, direct)
+        # down projection: da = dy W2, stored as the gradients of g | u; dW2 += dy^T a
         dgu = torch.empty(cap, 2 * I, dtype=_BF16, device=dev)
-        rows_dev = seg.data_ptr() + 4 * (2 * LE)
-        native.call("lb_swiglu_bwd_dev", gu.data_ptr(), da.data_ptr(), dgu.data_ptr(), cap, I, gu.stride(0), rows_dev, st())
+        _ragged(dybuf, downs, dgu, seg, LE, cap, I, H, True, ws.ctrl_ptrs[me] + 68, ws.arr_dy, epi=2, c2=gu, half=I)
+        _ragged_wgrad(dybuf, a, g_down, seg, LE, cap, H, I, direct)
         # gate | up projection: dx_rows = dgu [W1; W3], d[W1; W3] += dgu^T x_rows
         _ragged(dgu, ups, dxbuf, seg, LE, cap, H, 2 * I, True)
         _ragged_wgrad(dgu, xbuf, g_up, seg, LE, cap, 2 * I, H, direct)
-        # input gradient: sum of the k rows, read from their owners
-        dx = torch.empty(T, H, dtype=_BF16, device=dev)
-        ws.epoch_dx += 1
-        native.call("lb_moe_pull", dx.data_ptr(), 0, idx.data_ptr(), rows.data_ptr(), 0, 0, T, H, E, k, n, me, cap,
-                    ws.ptrs(ws.dx_ptrs), ws.ptrs(ws.ctrl_ptrs, 192), ws.epoch_dx, st())
         # router
         dx_r = torch.empty(T, H, dtype=_BF16, device=dev)
         dwg = torch.zeros(E, H, dtype=_F32, device=dev)
@@ -270,7 +262,11 @@ class _FusedMoE(torch.autograd.Function):
             daux_ptr = daux.data_ptr()
         native.call("lb_moe_router_bwd", x.data_ptr(), gate_w.data_ptr(), probs.data_ptr(), idx.data_ptr(), dwts.data_ptr(),
                     frac.data_ptr(), daux_ptr, dx_r.data_ptr(), dwg.data_ptr(), T, H, E, k, st())
-        native.call("lb_add_inplace", dx.data_ptr(), dx_r.data_ptr(), dx.numel(), st())
+        # input gradient: the router's and the sum of the k rows, read from their owners
+        dx = torch.empty(T, H, dtype=_BF16, device=dev)
+        ws.epoch_dx += 1
+        native.call("lb_moe_pull_add", dx.data_ptr(), dx_r.data_ptr(), 0, idx.data_ptr(), rows.data_ptr(), 0, 0, T, H, E, k, n, me, cap,
+                    ws.ptrs(ws.dx_ptrs), ws.ptrs(ws.ctrl_ptrs, 192), ws.epoch_dx, st())
         if direct:
             for w in params:
                 for hook in getattr(w, "_lb_grad_hooks", ()):

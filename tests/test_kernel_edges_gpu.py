@@ -477,6 +477,84 @@ def test_moe_rows_pushed_and_pulled(T, H, k):
     native.device_status()           # the dropped copies were counted: read and cleared
 
 
+@pytest.mark.parametrize("T,H,k", [(1, 8, 1), (37, 2056, 2), (9, 264, 5)])
+def test_moe_rows_pulled_onto_another_row(T, H, k):
+    """The k rows and one more, added in fp32 and rounded once."""
+    import ctypes
+    from lightron_b200.ops import native
+    buf, add, out = _rand(T * k, H, seed=1), _rand(T, H, seed=2), torch.empty(T, H, device="cuda", dtype=torch.bfloat16)
+    idx = torch.zeros(T, k, dtype=torch.int32, device="cuda")
+    rows = torch.randperm(T * k, device="cuda").int().view(T, k).contiguous()
+    words = torch.zeros(8, dtype=torch.int32, device="cuda")
+    one = lambda p: (ctypes.c_void_p * 1)(p)
+    native.call("lb_moe_pull_add", out.data_ptr(), add.data_ptr(), 0, idx.data_ptr(), rows.data_ptr(), 0, 0, T, H, 8, k, 1, 0, T * k,
+                one(buf.data_ptr()), one(words.data_ptr()), 1, native.stream_ptr())
+    terms = torch.cat([buf[rows.long()].double(), add[:, None].double()], 1)
+    assert ((out.double() - terms.sum(1)).abs() <= 2.0 ** -8 * terms.sum(1).abs() + (k + 1) * 2.0 ** -23 * terms.abs().sum(1)).all()
+    _status_ok()
+
+
+@pytest.mark.parametrize("nblk,E", [(1, 1), (31, 9), (33, 8), (129, 64), (300, 5)])
+def test_moe_plan_sums_over_blocks(nblk, E):
+    """Numbers of blocks and experts around what a step of the plan takes: exact whole numbers, fp32 sums of the probabilities."""
+    import ctypes
+    from lightron_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(nblk)
+    dev, k = "cuda", 1
+    hist = torch.randint(0, 9, (nblk, E), generator=g, device=dev, dtype=torch.int32)
+    psum = torch.rand(nblk, E, generator=g, device=dev)
+    T = int(hist.sum())
+    base, row0, seg = (torch.full(s, -1, dtype=torch.int32, device=dev) for s in ((nblk, E), (E,), (2 * E + 2,)))
+    frac, aux, words = torch.empty(E, device=dev), torch.empty(1, device=dev), torch.zeros(4096, dtype=torch.int32, device=dev)
+    one = lambda p: (ctypes.c_void_p * 1)(p)
+    native.call("lb_moe_plan", hist.data_ptr(), psum.data_ptr(), base.data_ptr(), row0.data_ptr(), seg.data_ptr(), frac.data_ptr(), aux.data_ptr(),
+                nblk, E, 1, 0, T, k, 1 << 20, one(words.data_ptr() + 4096), one(words.data_ptr()), 1, 1, native.stream_ptr())
+    n = hist.sum(0)
+    assert torch.equal(base, (hist.cumsum(0) - hist).int())
+    start = ((n + 127) // 128 * 128).cumsum(0) - (n + 127) // 128 * 128
+    assert torch.equal(row0, start.int()) and torch.equal(seg[:E], start.int()) and torch.equal(seg[E:2 * E], n.int())
+    assert int(seg[2 * E + 1]) == T
+    want = E * ((n.double() / T) * (psum.double().sum(0) / T)).sum()
+    assert abs(float(aux) / float(want) - 1) < (nblk + 8) * 2.0 ** -23
+    _status_ok()
+
+
+@pytest.mark.parametrize("H,I", [(72, 264), (264, 8), (520, 1032)])
+def test_ragged_activation_epilogues(H, I):
+    """Segments of one to several tiles, without rows and of one row; widths that end inside a tile and inside a step of 64 columns."""
+    from lightron_b200.parallel import ep_fused
+    counts = [130, 0, 1, 300]
+    LE, cap = len(counts), 1024
+    off, seg = 0, []
+    for c in counts:
+        seg.append(off)
+        off += (c + 127) // 128 * 128
+    table = torch.tensor(seg + counts + [off, sum(counts)], dtype=torch.int32, device="cuda")
+    x, dy = _rand(cap, H, seed=1), _rand(cap, H, seed=2)
+    live = torch.zeros(cap, dtype=torch.bool, device="cuda")
+    for o, c in zip(seg, counts):
+        live[o:o + c] = True
+    x[~live] = 0
+    dy[~live] = 0
+    up = [_rand(2 * I, H, scale=H ** -0.5, seed=10 + e) for e in range(LE)]
+    down = [_rand(H, I, scale=I ** -0.5, seed=20 + e) for e in range(LE)]
+    gu, act, dgu = (torch.full((cap, n), 7.0, device="cuda", dtype=torch.bfloat16) for n in (2 * I, I, 2 * I))
+    ep_fused._ragged(x, up, gu, table, LE, cap, 2 * I, H, False, epi=1, c2=act, half=I)
+    ep_fused._ragged(dy, down, dgu, table, LE, cap, I, H, True, epi=2, c2=gu, half=I)
+    _status_ok()
+    assert (gu[off:] == 7).all() and (act[off:] == 7).all() and (dgu[off:] == 7).all()
+    for e, (o, c) in enumerate(zip(seg, counts)):
+        if not c:
+            continue
+        r = slice(o, o + c)
+        assert _rel(gu[r], x[r].double() @ up[e].double().t()) < 5e-3
+        g, u = gu[r].double().split(I, 1)
+        sig = torch.sigmoid(g)
+        assert _rel(act[r], g * sig * u) < 5e-3
+        dh = dy[r].double() @ down[e].double()
+        assert _rel(dgu[r], torch.cat([dh * u * sig * (1 + g * (1 - sig)), dh * g * sig], 1)) < 1e-2        # (dh is rounded to bf16 first)
+
+
 @pytest.mark.parametrize("n", [0, 1, 15, 16, 17, 4095, 4096, 4111, 1 << 20, (1 << 20) + 7])
 def test_clear_writes_its_bytes_and_no_others(n):
     from lightron_b200.ops import native

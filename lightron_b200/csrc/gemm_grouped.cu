@@ -56,9 +56,10 @@ constexpr int MAX_PROBLEMS = 8;
 //   0  C = acc (+ C when accumulate)
 //   1  SwiGLU forward: B is a fused [2 * half, K] gate | up weight.  Tile tn holds 128 gate columns
 //      (accumulator columns 0..127) and the 128 up columns of the same index (128..255): both go to
-//      C [M, 2 * half] as usual (the backward needs them) and silu(g) * u goes to C2 [M, half].
+//      C [M, 2 * half] as usual (the backward needs them; a null C is not stored) and silu(g) * u goes to C2 [M, half].
 //   2  SwiGLU backward: acc is dh [M, half] of the down projection; the epilogue reads g | u from
 //      C2 [M, 2 * half] and writes dg | du to C [M, 2 * half]; dh itself is never stored.
+//   4  C = acc with its first columns rotated (RopeArgs).
 struct Problem {
   const bf16* old;      // what the epilogue reads: C when accumulate, C2 (g | u) with epi 2
   long long ld_old;
@@ -66,6 +67,7 @@ struct Problem {
   int a_mn, b_mn, accumulate;
   int tiles_m, tiles_n, num_kb;
   int epi, half;
+  int keep;             // epi 1: C is stored
 };
 
 template <int NP>
@@ -74,6 +76,7 @@ struct GroupedParams {
   CUtensorMap tb[NP];
   CUtensorMap tc[NP][3];      // where the epilogue stores: C; C's gate columns, its up columns, C2; dg, du
   Problem prob[NP];
+  RopeArgs rope;
   const int* offsets;   // [grid + 1] first item of every CTA
   const int* items;     // (problem << 24) | tile index inside the problem
 };
@@ -178,13 +181,15 @@ struct Out {
   long long ld_old;
   int row0, rows;      // the warp's first row, rows of the matrix
   int c0, cols;        // first column, columns (of one half, with an activation)
+  bool keep;           // EPI 1: g and u are stored
+  const RopeArgs* rope;
 };
 
 // EPI as in Problem; 3: C = acc + C.  `turn`: which buffer is next, kept over the tiles (the store before the last one has used it).  ready() waits
 // for the accumulator, release() gives its columns back.
 template <int EPI, typename Ready, typename Release>
 __device__ __forceinline__ bool store_tile(const Out& o, uint32_t taddr, uint8_t* stg, int& turn, int lane, Ready ready, Release release) {
-  constexpr bool READS = EPI >= 2;
+  constexpr bool READS = EPI == 2 || EPI == 3;
   constexpr int NC = EPI == 1 ? BN / 128 : BN / 64;                   // steps of 64 columns
   uint4 old[READS ? 8 : 1], old2[EPI == 2 ? 8 : 1];
   const int lr = lane >> 3, lc = (lane & 7) * 8;                      // loads: row (of every four), column
@@ -236,14 +241,17 @@ __device__ __forceinline__ bool store_tile(const Out& o, uint32_t taddr, uint8_t
       take(taddr + c * 64, pg);
       take(taddr + BN / 2 + c * 64, pu);
       if (c == NC - 1 || col + 64 >= o.cols) release();
-      uint8_t* buf = next();
+      uint8_t* buf;
+      if (o.keep) {
+        buf = next();
 #pragma unroll
-      for (int g = 0; g < 8; g++) *at(buf, g) = pg[g];
-      store(buf, o.map, col);
-      buf = next();
+        for (int g = 0; g < 8; g++) *at(buf, g) = pg[g];
+        store(buf, o.map, col);
+        buf = next();
 #pragma unroll
-      for (int g = 0; g < 8; g++) *at(buf, g) = pu[g];
-      store(buf, o.map + 1, col);
+        for (int g = 0; g < 8; g++) *at(buf, g) = pu[g];
+        store(buf, o.map + 1, col);
+      }
 #pragma unroll
       for (int g = 0; g < 8; g++) {
         float fg[8], fu[8], h[8];
@@ -260,6 +268,7 @@ __device__ __forceinline__ bool store_tile(const Out& o, uint32_t taddr, uint8_t
       if (col + 64 >= o.cols) break;
     }
   } else {
+    const int pos = EPI == 4 && o.row0 + lane < o.rows ? rope_position(*o.rope, o.row0 + lane) : 0;
 #pragma unroll 1
     for (int c = 0; c < NC; c++) {
       const int col = o.c0 + c * 64;
@@ -313,6 +322,12 @@ __device__ __forceinline__ bool store_tile(const Out& o, uint32_t taddr, uint8_t
             unpack8(*at(buf, g), e);
 #pragma unroll
             for (int i = 0; i < 8; i++) f[i] += e[i];
+          }
+          if constexpr (EPI == 4) {
+            if (col + g * 8 < o.rope->cols) {
+              unpack8(pack8(f), f);                                   // the values a stored C would have
+              rope_rotate8(*o.rope, pos, col + g * 8, f);
+            }
           }
           *at(buf, g) = pack8(f);
         }
@@ -453,7 +468,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
       const Problem& pr = gp.prob[pi];
       const int acc = n & 1;
       const uint32_t acc_phase = (uint32_t)(n >> 1) & 1u;
-      const Out out{gp.tc[pi], pr.old, pr.ld_old, (tm * CG + rank) * BM + quad * 32, pr.M, tn * (pr.epi == 1 ? BN / 2 : BN), pr.epi ? pr.half : pr.N};
+      const Out out{gp.tc[pi], pr.old, pr.ld_old, (tm * CG + rank) * BM + quad * 32, pr.M, tn * (pr.epi == 1 ? BN / 2 : BN), pr.epi == 1 || pr.epi == 2 ? pr.half : pr.N, pr.keep != 0, &gp.rope};
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * BN;
       auto ready = [&]() {
         if (!bw::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) return false;
@@ -473,6 +488,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
         case 0: ok = store_tile<0>(out, taddr, stg, turn, lane, ready, release); break;
         case 1: ok = store_tile<1>(out, taddr, stg, turn, lane, ready, release); break;
         case 2: ok = store_tile<2>(out, taddr, stg, turn, lane, ready, release); break;
+        case 4: ok = store_tile<4>(out, taddr, stg, turn, lane, ready, release); break;
         default: ok = store_tile<3>(out, taddr, stg, turn, lane, ready, release); break;
       }
       if (!ok) { give_up(abort_flag, 4u); break; }
@@ -674,7 +690,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
       const bool wgrad = rp.mode == 1;
       // (mode 0 writes whole 128-row tiles: padding rows are zeros)
       const Out out{wgrad ? &rp.tc[rt.e] : rp.tc, wgrad ? rp.C[rt.e] : rp.old, wgrad ? rp.ldc : rp.ld_old, rt.m0 + quad * 32, wgrad ? rp.M_w : rp.cap,
-                    rt.n0, rp.epi ? rp.half : rp.N};
+                    rt.n0, rp.epi ? rp.half : rp.N, true, nullptr};
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * BN;
       auto ready = [&]() {
         if (!bw::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) return false;
@@ -843,9 +859,9 @@ int out_map(CUtensorMap* m, const bf16* base, int cols, int rows, long long ld) 
 // The maps of a problem's outputs (see GroupedParams::tc).
 int out_maps(CUtensorMap* tc, void* C, void* C2, long long ldc, long long ldc2, int rows, int N, int epi, int half) {
   bf16* c = (bf16*)C;
-  if (!epi) return out_map(tc, c, N, rows, ldc);
-  int rc = out_map(tc, c, half, rows, ldc);
-  if (!rc) rc = out_map(tc + 1, c + half, half, rows, ldc);
+  if (epi == 0 || epi == 4) return out_map(tc, c, N, rows, ldc);
+  int rc = c ? out_map(tc, c, half, rows, ldc) : LB_OK;
+  if (!rc && c) rc = out_map(tc + 1, c + half, half, rows, ldc);
   if (!rc && epi == 1) rc = out_map(tc + 2, (const bf16*)C2, half, rows, ldc2);
   return rc;
 }
@@ -854,6 +870,7 @@ struct Operands {
   const void *const *A, *const *B;
   void *const *C, *const *C2;
   const long long *lda, *ldb, *ldc, *ldc2;
+  const RopeArgs* rope;
 };
 template <int NP>
 int launch_grouped(int n, const Problem* probs, const Operands& op, const Schedule& sched, cudaStream_t s) {
@@ -867,8 +884,9 @@ int launch_grouped(int n, const Problem* probs, const Operands& op, const Schedu
     if (!p.b_mn) rc = bw::make_map_bf16(&gp.tb[i], op.B[i], (uint64_t)p.K, (uint64_t)p.N, (uint64_t)op.ldb[i], BK, BN / 2);
     else         rc = bw::make_map_bf16(&gp.tb[i], op.B[i], (uint64_t)p.N, (uint64_t)p.K, (uint64_t)op.ldb[i], 64, BK);
     if (rc) return rc;
-    if ((rc = out_maps(gp.tc[i], op.C[i], p.epi ? op.C2[i] : nullptr, op.ldc[i], p.epi ? op.ldc2[i] : 0, p.M, p.N, p.epi, p.half))) return rc;
+    if ((rc = out_maps(gp.tc[i], op.C[i], op.C2 ? op.C2[i] : nullptr, op.ldc[i], op.ldc2 ? op.ldc2[i] : 0, p.M, p.N, p.epi, p.half))) return rc;
   }
+  gp.rope = op.rope ? *op.rope : RopeArgs{nullptr, nullptr, nullptr, 1, 64, 0};
   gp.offsets = sched.d_offsets;
   gp.items = sched.d_items;
   if (sched.cg == 2)      // a pair is a cluster of two CTAs
@@ -949,13 +967,11 @@ extern "C" int lb_gemm_grouped_plan(int n, const int* M, const int* N, const int
 // lb_gemm_grouped_epi additionally takes, per problem, an epilogue selector (see `Problem`), a second
 // matrix C2 with its leading dimension, and `half`:
 //   epi 1: B is a fused [2 * half, K] gate | up weight (b_mn = 0), N = 2 * half, C [M, 2 * half] receives
-//          g | u and C2 [M, half] receives silu(g) * u;
+//          g | u (nothing, with a null C) and C2 [M, half] receives silu(g) * u;
 //   epi 2: N = half, the product is dh; C2 [M, 2 * half] holds g | u and C [M, 2 * half] receives dg | du.
-extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* const* B, void* const* C, const int* M,
-                                   const int* N, const int* K, const long long* lda, const long long* ldb,
-                                   const long long* ldc, const int* a_mn, const int* b_mn, const int* accumulate,
-                                   const int* epi, void* const* C2, const long long* ldc2, const int* half,
-                                   void* stream) {
+static int run_grouped(int n, const void* const* A, const void* const* B, void* const* C, const int* M, const int* N, const int* K,
+                       const long long* lda, const long long* ldb, const long long* ldc, const int* a_mn, const int* b_mn, const int* accumulate,
+                       const int* epi, void* const* C2, const long long* ldc2, const int* half, const RopeArgs* rope, void* stream) {
   if (n < 1 || n > MAX_PROBLEMS) return LB_ERR_SHAPE;
   Problem probs[MAX_PROBLEMS];
   std::vector<int> key;
@@ -975,7 +991,7 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
       if (accumulate && accumulate[i]) return LB_ERR_ARG;
     }
     Problem& p = probs[i];
-    p.M = M[i]; p.N = N[i]; p.K = K[i]; p.epi = e; p.half = e ? half[i] : 0;
+    p.M = M[i]; p.N = N[i]; p.K = K[i]; p.epi = rope ? 4 : e; p.half = e ? half[i] : 0; p.keep = C[i] != nullptr;
     p.old = (const bf16*)(e == 2 ? C2[i] : C[i]); p.ld_old = e == 2 ? ldc2[i] : ldc[i];
     p.a_mn = a_mn[i]; p.b_mn = b_mn[i]; p.accumulate = accumulate ? accumulate[i] : 0;
     key.push_back(M[i]); key.push_back(N[i]); key.push_back(K[i]);
@@ -1017,12 +1033,31 @@ extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* cons
     sched = it->second;
   }
   if (sched.split)
-    return lb_gemm_split(n, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, epi, C2, ldc2, half, sched.split, stream);
+    return gemm_split_rope(n, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, epi, C2, ldc2, half, sched.split, rope, stream);
   for (int i = 0; i < n; i++) set_tiles(&probs[i], sched.cg);
-  const Operands op{A, B, C, C2, lda, ldb, ldc, ldc2};
+  const Operands op{A, B, C, epi ? C2 : nullptr, lda, ldb, ldc, epi ? ldc2 : nullptr, rope};
   return n <= 2 ? launch_grouped<2>(n, probs, op, sched, (cudaStream_t)stream) : launch_grouped<MAX_PROBLEMS>(n, probs, op, sched, (cudaStream_t)stream);
 }
 
+
+extern "C" int lb_gemm_grouped_epi(int n, const void* const* A, const void* const* B, void* const* C, const int* M,
+                                   const int* N, const int* K, const long long* lda, const long long* ldb,
+                                   const long long* ldc, const int* a_mn, const int* b_mn, const int* accumulate,
+                                   const int* epi, void* const* C2, const long long* ldc2, const int* half,
+                                   void* stream) {
+  return run_grouped(n, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, epi, C2, ldc2, half, nullptr, stream);
+}
+
+// C [M, N] = X [M, K] W^T (W [N, K]; all matrices contiguous) with the first rope_cols columns, heads of head_dim columns, rotated as
+// lb_rope rotates them: row r is token r of sequences of S tokens.
+extern "C" int lb_gemm_rope(const void* X, const void* W, void* C, int M, int N, int K, const void* cosT, const void* sinT, const void* positions,
+                            int S, int head_dim, int rope_cols, void* stream) {
+  if (S <= 0 || head_dim <= 0 || (head_dim % 8) || rope_cols < 0 || rope_cols > N || (rope_cols % head_dim)) return LB_ERR_SHAPE;
+  const RopeArgs rope{(const float*)cosT, (const float*)sinT, (const int*)positions, S, head_dim, rope_cols};
+  const long long lda = K, ldb = K, ldc = N;
+  const int k_major = 0;
+  return run_grouped(1, &X, &W, &C, &M, &N, &K, &lda, &ldb, &ldc, &k_major, &k_major, nullptr, nullptr, nullptr, nullptr, nullptr, &rope, stream);
+}
 
 extern "C" int lb_gemm_grouped(int n, const void* const* A, const void* const* B, void* const* C, const int* M,
                                const int* N, const int* K, const long long* lda, const long long* ldb,

@@ -34,7 +34,8 @@ constexpr int NUM_THREADS = 192;
 constexpr int MAX_PROBLEMS = 2;
 constexpr int PREFETCH = 16;                             // k-blocks of B that a CTA asks for ahead of its start (38 MB of all CTAs that run at a time)
 
-// epi: 0 C = acc (+ C); 1 gate | up -> C, silu(g) * u -> C2; 2 dh -> dg | du with g | u from C2 (as in gemm_grouped.cu).
+// epi: 0 C = acc (+ C); 1 gate | up -> C (not stored where C is null), silu(g) * u -> C2; 2 dh -> dg | du with g | u from C2; 4 rotation (as in
+// gemm_grouped.cu).
 struct Problem {
   bf16* C;
   long long ldc;
@@ -47,6 +48,7 @@ struct Problem {
 struct Params {
   CUtensorMap ta[MAX_PROBLEMS], tb[MAX_PROBLEMS];
   Problem prob[MAX_PROBLEMS];
+  RopeArgs rope;
   int np, ks;
 };
 
@@ -214,6 +216,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
     const int row = m0 + row_in;
     const bool row_ok = row < pr.M;
     const int n_end = pr.epi == 1 ? pr.half : pr.N;
+    const int pos = pr.epi == 4 && row_ok ? rope_position(gp.rope, row) : 0;
     for (int c = 0; c < w; c += 8) {
       float f[2][8];
 #pragma unroll
@@ -247,9 +250,11 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
         const int col = n0 + cc;
         if (col < n_end) {
           const uint4 pg = pack8(f[0]), pu = pack8(f[1]);
-          bf16* grow = pr.C + (size_t)row * pr.ldc + col;
-          *reinterpret_cast<uint4*>(grow) = pg;
-          *reinterpret_cast<uint4*>(grow + pr.half) = pu;
+          if (pr.C) {
+            bf16* grow = pr.C + (size_t)row * pr.ldc + col;
+            *reinterpret_cast<uint4*>(grow) = pg;
+            *reinterpret_cast<uint4*>(grow + pr.half) = pu;
+          }
           float g[8], u[8], h[8];
           unpack8(pg, g);
           unpack8(pu, u);
@@ -284,6 +289,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
             unpack8(*reinterpret_cast<const uint4*>(dst), o);
 #pragma unroll
             for (int i = 0; i < 8; i++) f[b][i] += o[i];
+          } else if (pr.epi == 4 && col < gp.rope.cols) {
+            unpack8(pack8(f[b]), f[b]);                        // the values a stored C would have
+            rope_rotate8(gp.rope, pos, col, f[b]);
           }
           *reinterpret_cast<uint4*>(dst) = pack8(f[b]);
         }
@@ -317,8 +325,16 @@ extern "C" int lb_gemm_split_status(void* out) {
 extern "C" int lb_gemm_split(int n, const void* const* A, const void* const* B, void* const* C, const int* M, const int* N, const int* K,
                              const long long* lda, const long long* ldb, const long long* ldc, const int* a_mn, const int* b_mn,
                              const int* accumulate, const int* epi, void* const* C2, const long long* ldc2, const int* half, int ks, void* stream) {
+  return gemm_split_rope(n, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, epi, C2, ldc2, half, ks, nullptr, stream);
+}
+
+int gemm_split_rope(int n, const void* const* A, const void* const* B, void* const* C, const int* M, const int* N, const int* K,
+                    const long long* lda, const long long* ldb, const long long* ldc, const int* a_mn, const int* b_mn,
+                    const int* accumulate, const int* epi, void* const* C2, const long long* ldc2, const int* half, int ks, const RopeArgs* rope,
+                    void* stream) {
   if (n < 1 || n > MAX_PROBLEMS || (ks != 1 && ks != 2 && ks != 4)) return LB_ERR_SHAPE;
   Params gp;
+  gp.rope = rope ? *rope : RopeArgs{nullptr, nullptr, nullptr, 1, 64, 0};
   gp.np = n;
   gp.ks = ks;
   long long tiles = 0;
@@ -346,7 +362,7 @@ extern "C" int lb_gemm_split(int n, const void* const* A, const void* const* B, 
     else          rc = bw::make_map_bf16(&gp.tb[i], B[i], (uint64_t)N[i], (uint64_t)K[i], (uint64_t)ldb[i], 64, BK);
     if (rc) return rc;
     p.C = (bf16*)C[i]; p.ldc = ldc[i]; p.C2 = e ? (bf16*)C2[i] : nullptr; p.ldc2 = e ? ldc2[i] : 0;
-    p.M = M[i]; p.N = N[i]; p.a_mn = a_mn[i]; p.b_mn = b_mn[i]; p.accumulate = accumulate ? accumulate[i] : 0; p.epi = e; p.half = e ? half[i] : 0;
+    p.M = M[i]; p.N = N[i]; p.a_mn = a_mn[i]; p.b_mn = b_mn[i]; p.accumulate = accumulate ? accumulate[i] : 0; p.epi = rope ? 4 : e; p.half = e ? half[i] : 0;
     p.tiles_m = (M[i] + BM - 1) / BM;
     p.num_kb = (K[i] + BK - 1) / BK;
     if (p.num_kb < ks) return LB_ERR_SHAPE;

@@ -2,7 +2,36 @@
 #pragma once
 #include "common.cuh"
 
+// Epilogue 4 (no entry point takes it but lb_gemm_rope): the first `cols` columns of C are heads of d columns whose pairs (2i, 2i + 1) are rotated
+// as lb_rope does, from the values that a stored C would have; row r is token r of sequences of S tokens.
+struct RopeArgs {
+  const float *cos, *sin;
+  const int* positions;      // [S] or null: the token's place in its sequence
+  int S, d, cols;
+};
+__device__ __forceinline__ int rope_position(const RopeArgs& r, int row) {
+  const int s = row % r.S;
+  return r.positions ? r.positions[s] : s;
+}
+// 8 columns of C (from `col`, a multiple of 8) of a row at that position
+__device__ __forceinline__ void rope_rotate8(const RopeArgs& r, int pos, int col, float* f) {
+  const int at = pos * (r.d >> 1) + ((col % r.d) >> 1);
+  const float4 c = *reinterpret_cast<const float4*>(r.cos + at), sn = *reinterpret_cast<const float4*>(r.sin + at);
+  float o[8];
+  o[0] = f[0] * c.x - f[1] * sn.x; o[1] = f[0] * sn.x + f[1] * c.x;
+  o[2] = f[2] * c.y - f[3] * sn.y; o[3] = f[2] * sn.y + f[3] * c.y;
+  o[4] = f[4] * c.z - f[5] * sn.z; o[5] = f[4] * sn.z + f[5] * c.z;
+  o[6] = f[6] * c.w - f[7] * sn.w; o[7] = f[6] * sn.w + f[7] * c.w;
+#pragma unroll
+  for (int i = 0; i < 8; i++) f[i] = o[i];
+}
+
 extern "C" int lb_gemm_split(int n, const void* const* A, const void* const* B, void* const* C, const int* M, const int* N, const int* K,
                              const long long* lda, const long long* ldb, const long long* ldc, const int* a_mn, const int* b_mn,
                              const int* accumulate, const int* epi, void* const* C2, const long long* ldc2, const int* half, int ks, void* stream);
+// The same with the rotation of epilogue 4 (n = 1), or with `rope` null.
+int gemm_split_rope(int n, const void* const* A, const void* const* B, void* const* C, const int* M, const int* N, const int* K,
+                    const long long* lda, const long long* ldb, const long long* ldc, const int* a_mn, const int* b_mn,
+                    const int* accumulate, const int* epi, void* const* C2, const long long* ldc2, const int* half, int ks, const RopeArgs* rope,
+                    void* stream);
 int gemm_split_parts(int n, const int* M, const int* N, const int* K, int sms, long long list_time);

@@ -51,6 +51,7 @@ struct Api {
   int (*lb_ce_stats)(P, P, W, W, W, int, int, L, int, W);
   int (*lb_ce_loss)(P, W, P, P, W, W, int, float, int, W);
   int (*lb_ce_grad)(P, P, P, W, P, int, int, L, int, float, int, W);
+  int (*lb_gemm_rope)(P, P, W, int, int, int, P, P, P, int, int, int, W);
 } api;
 PyObject* raise_error = nullptr;                 // (name, code): raises the error of ops/native.py
 PyObject* direct_grad = nullptr;                 // the attribute of a weight whose gradient the optimizer keeps
@@ -580,6 +581,120 @@ PyObject* py_cross_entropy(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// ---- a run of decoder layers without gradients -----------------------------------------------------
+// What models/llama.py does for one GPU with seven ops a layer, in one call: seven launches a layer (the rotation is in the projection's
+// epilogue, g | u are not stored), intermediate results in one workspace.  12 layers of 768 columns over 128 tokens, embedding and
+// head included, were bound by the host's 8 us an op: 808 us, now 516 (kernels 486).
+struct DecoderLayer { Tensor norm1, wqkv, wo, norm2, w13, w2; double eps1, eps2; L I; };
+
+std::pair<Tensor, Tensor> decoder_layers(Tensor h, Tensor delta, const Tensor& cos, const Tensor& sin, const Tensor& positions, Dims dims, double scale,
+                                         const std::vector<DecoderLayer>& layers) {
+  const L B = dims.v[0], S = dims.v[1], hq = dims.v[2], hkv = dims.v[3], d = dims.v[4], T = h.size(0), H = h.size(1), nqkv = (hq + 2 * hkv) * d;
+  L I = 0;
+  for (const DecoderLayer& l : layers) I = std::max(I, l.I);
+  // Of a layer: the normed rows throughout; then qkv, o, the log-sum-exp and the attention's output, and in their place the activation
+  auto up = [](L bytes) { return (bytes + 255) / 256 * 256; };
+  const L at_rstd = up(2 * T * H), at_qkv = at_rstd + up(4 * T), at_o = at_qkv + up(2 * T * nqkv), at_lse = at_o + up(2 * T * hq * d),
+          at_a = at_lse + up(4 * T * hq), end = std::max(at_a + up(2 * T * H), at_qkv + up(2 * T * I));
+  const Tensor ws = at::empty({end}, h.options().dtype(at::kByte));
+  char* base = static_cast<char*>(ws.mutable_data_ptr());
+  W x = base, rstd = base + at_rstd, qkv = base + at_qkv, o = base + at_o, lse = base + at_lse, a = base + at_a, act = qkv;
+  auto head = [&](L n) { return base + at_qkv + n * d * 2; };
+  const Tensor own[2] = {empty({T, H}, h), empty({T, H}, h)};      // the residual stream, each sum in the one that does not hold the last
+  Tensor f = empty({T, H}, h);
+  int turn = 0;
+  auto norm = [&](P add, const Tensor& w, double eps) {            // h (+)= add, x = norm(h)
+    if (add) {
+      LB_CALL(lb_rmsnorm_fwd, add, h.const_data_ptr(), w.const_data_ptr(), own[turn].mutable_data_ptr(), x, rstd, (int)T, (int)H, (float)eps, stream());
+      h = own[turn];
+      turn ^= 1;
+    } else {
+      LB_CALL(lb_rmsnorm_fwd, h.const_data_ptr(), nullptr, w.const_data_ptr(), nullptr, x, rstd, (int)T, (int)H, (float)eps, stream());
+    }
+  };
+  auto gemm = [&](P in, const Tensor& w, W out, L n, L k, int epi = 0, W c2 = nullptr) {
+    const P A[1] = {in}, Bw[1] = {w.const_data_ptr()};
+    const W C[1] = {out}, C2[1] = {c2};
+    const int M[1] = {(int)T}, N[1] = {(int)n}, K[1] = {(int)k}, no[1] = {0}, ep[1] = {epi}, half[1] = {(int)(n / 2)};
+    const L lda[1] = {k}, ldc[1] = {n}, ldc2[1] = {n / 2};
+    LB_CALL(lb_gemm_grouped_epi, 1, A, Bw, C, M, N, K, lda, lda, ldc, no, no, no, ep, C2, ldc2, half, stream());
+  };
+  for (const DecoderLayer& l : layers) {
+    norm(delta.defined() ? delta.const_data_ptr() : nullptr, l.norm1, l.eps1);
+    LB_CALL(lb_gemm_rope, x, l.wqkv.const_data_ptr(), qkv, (int)T, (int)nqkv, (int)H, cos.const_data_ptr(), sin.const_data_ptr(),
+            positions.defined() ? positions.const_data_ptr() : nullptr, (int)S, (int)d, (int)((hq + hkv) * d), stream());
+    LB_CALL(lb_flash_fwd_tc, head(0), head(hq), head(hq + hkv), o, lse, (int)B, (int)S, (int)S, (int)hq, (int)hkv, (int)d, nqkv, nqkv, nqkv, hq * d,
+            (float)scale, 1, stream());
+    gemm(o, l.wo, a, H, hq * d);
+    norm(a, l.norm2, l.eps2);
+    gemm(x, l.w13, nullptr, 2 * l.I, H, 1, act);
+    gemm(act, l.w2, f.mutable_data_ptr(), H, l.I);
+    delta = f;                                                     // (the next layer's first norm reads it before its last GEMM writes it)
+  }
+  return {h, delta};
+}
+
+// (h, delta or None, cos, sin, positions or None, B, S, hq, hkv, d, scale, layers) -> (h, delta).  layers: a list with, per layer, a tuple (attention norm's weight, eps,
+// wq, wk, wv, wo, feed-forward norm's weight, eps, w1, w3, w2).  Without gradients only.
+PyObject* py_decoder_layers(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 12 || at::GradMode::is_enabled() || !PyFloat_Check(a[10]) || !PyList_CheckExact(a[11]) || PyList_GET_SIZE(a[11]) == 0 || !unobserved() ||
+      !env_is_tc("LIGHTRON_FA")) LB_NOT_PLAIN;
+  const Tensor *h = tensor(a[0]), *delta = a[1] == Py_None ? nullptr : tensor(a[1]), *cos = tensor(a[2]), *sin = tensor(a[3]),
+               *pos = a[4] == Py_None ? nullptr : tensor(a[4]);
+  Dims dims;
+  for (int i = 0; i < 5; i++) {
+    if (!PyLong_CheckExact(a[5 + i])) LB_NOT_PLAIN;
+    dims.v[i] = PyLong_AsLongLong(a[5 + i]);
+    if (PyErr_Occurred()) return nullptr;
+    if (dims.v[i] < 1 || dims.v[i] > (1 << 24)) LB_NOT_PLAIN;
+  }
+  const int64_t B = dims.v[0], S = dims.v[1], hq = dims.v[2], hkv = dims.v[3], d = dims.v[4];
+  auto aligned = [](const Tensor& t) { return ((uintptr_t)t.const_data_ptr() & 15) == 0; };
+  if (!plain(h) || h->dim() != 2 || h->size(0) != B * S || h->size(1) % 8 || !aligned(*h) || hq % hkv || (d != 64 && d != 128) ||
+      !fits_int({B * S, h->size(1), (hq + 2 * hkv) * d}) || !table_ok(cos, d) || !table_ok(sin, d)) LB_NOT_PLAIN;
+  if (a[1] != Py_None && (!plain(delta) || !delta->sizes().equals(h->sizes()) || !aligned(*delta))) LB_NOT_PLAIN;
+  if (a[4] != Py_None) {
+    if (!pos || !pos->is_cuda() || pos->scalar_type() != at::kInt || !pos->is_contiguous() || pos->numel() != S) LB_NOT_PLAIN;
+  } else if (cos->size(0) < S || sin->size(0) < S) {
+    LB_NOT_PLAIN;
+  }
+  const int64_t H = h->size(1);
+  std::vector<DecoderLayer> layers((size_t)PyList_GET_SIZE(a[11]));
+  for (size_t i = 0; i < layers.size(); i++) {
+    PyObject* t = PyList_GET_ITEM(a[11], (Py_ssize_t)i);
+    if (!PyTuple_CheckExact(t) || PyTuple_GET_SIZE(t) != 11) LB_NOT_PLAIN;
+    const Tensor* w[11];
+    for (int j = 0; j < 11; j++) {
+      PyObject* o = PyTuple_GET_ITEM(t, j);
+      if (j == 1 || j == 7) {
+        if (!PyFloat_Check(o)) LB_NOT_PLAIN;
+        continue;
+      }
+      w[j] = tensor(o);
+      if (!plain(w[j]) || !aligned(*w[j]) || w[j]->device() != h->device()) LB_NOT_PLAIN;
+    }
+    for (int j : {0, 6})
+      if (w[j]->dim() != 1 || w[j]->size(0) != H) LB_NOT_PLAIN;
+    for (int j : {2, 3, 4, 8, 9})
+      if (!weight_ok(w[j], H)) LB_NOT_PLAIN;
+    if (w[2]->size(0) != hq * d || w[3]->size(0) != hkv * d || w[4]->size(0) != hkv * d || !weight_ok(w[5], hq * d) || w[5]->size(0) != H ||
+        w[8]->size(0) != w[9]->size(0) || !weight_ok(w[10], w[8]->size(0)) || w[10]->size(0) != H || !fits_int({2 * w[8]->size(0)})) LB_NOT_PLAIN;
+    if (!rows_adjacent(w + 2, 3) || !rows_adjacent(w + 8, 2)) LB_NOT_PLAIN;
+    layers[i] = {*w[0], *w[2], *w[5], *w[6], *w[8], *w[10], PyFloat_AsDouble(PyTuple_GET_ITEM(t, 1)), PyFloat_AsDouble(PyTuple_GET_ITEM(t, 7)), w[8]->size(0)};
+  }
+  const double scale = PyFloat_AsDouble(a[10]);
+  std::pair<Tensor, Tensor> r = unlocked([&, h = *h, delta = delta ? *delta : Tensor(), cos = *cos, sin = *sin, pos = pos ? *pos : Tensor()] {
+    return decoder_layers(h, delta, cos, sin, pos, dims, scale, layers);
+  });
+  PyObject* t = PyTuple_New(2);
+  if (!t) return nullptr;
+  PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(r.first)));
+  PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(std::move(r.second)));
+  return t;
+  END_HANDLE_TH_ERRORS
+}
+
 PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromUnsignedLongLong(g_launches.load(std::memory_order_relaxed)); }
 
 // init(addresses: dict of name -> int, raise_error): the kernels' entry points of the library that ops/native.py has loaded
@@ -596,7 +711,7 @@ PyObject* py_init(PyObject*, PyObject* args) {
 #define LB_TAKE(name) take(#name, &api.name)
   LB_TAKE(lb_rmsnorm_fwd); LB_TAKE(lb_rmsnorm_bwd_blocks); LB_TAKE(lb_rmsnorm_bwd); LB_TAKE(lb_rope); LB_TAKE(lb_gemm_grouped_epi);
   LB_TAKE(lb_flash_fwd_tc); LB_TAKE(lb_flash_bwd_ws_bytes); LB_TAKE(lb_flash_bwd_tc_ws); LB_TAKE(lb_flash_bwd); LB_TAKE(lb_embedding_fwd); LB_TAKE(lb_clear);
-  LB_TAKE(lb_embedding_bwd); LB_TAKE(lb_ce_stats); LB_TAKE(lb_ce_loss); LB_TAKE(lb_ce_grad);
+  LB_TAKE(lb_embedding_bwd); LB_TAKE(lb_ce_stats); LB_TAKE(lb_ce_loss); LB_TAKE(lb_ce_grad); LB_TAKE(lb_gemm_rope);
   if (!ok) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "an entry point of the kernels is missing");
     return nullptr;
@@ -608,7 +723,7 @@ PyObject* py_init(PyObject*, PyObject* args) {
 
 #define LB_FAST(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {LB_FAST(linear), LB_FAST(swiglu_mlp), LB_FAST(rmsnorm), LB_FAST(attention), LB_FAST(rope_attention), LB_FAST(embedding),
-                         LB_FAST(cross_entropy), {"launches", py_launches, METH_NOARGS, nullptr}, {"init", py_init, METH_VARARGS, nullptr},
+                         LB_FAST(cross_entropy), LB_FAST(decoder_layers), {"launches", py_launches, METH_NOARGS, nullptr}, {"init", py_init, METH_VARARGS, nullptr},
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host_ops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

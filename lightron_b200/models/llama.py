@@ -23,6 +23,7 @@ What is different by design:
 """
 from __future__ import annotations
 
+import math
 import zlib
 from typing import List, Optional, Tuple
 
@@ -32,6 +33,7 @@ import torch.nn as nn
 from .. import mesh as _mesh
 from ..config import ModelArgs
 from ..ops import functional as OF
+from ..ops import native
 from ..ops import reference as ref
 from ..parallel import comm, fused
 from ..parallel.tp import ColumnParallelLinear, Linear, RowParallelLinear, VocabParallelEmbedding
@@ -155,6 +157,33 @@ class TransformerBlock(nn.Module):
         return h, f
 
 
+def _plain_layers(layers: nn.ModuleDict):
+    """(hq, hkv, d, scale, weights of every layer) of dense blocks on one GPU that nothing hooks into, for ``host_ops.decoder_layers``, which does
+    in one call what their ``forward`` does op by op; None for any other."""
+    if not layers or nn.modules.module._has_any_global_hook():
+        return None
+    weights, shape = [], None
+    for blk in layers._modules.values():
+        mods = blk._modules
+        att, ff = mods.get("attention"), mods.get("feed_forward")
+        if type(blk) is not TransformerBlock or type(att) is not Attention or type(ff) is not MLP:
+            return None
+        if att.tp_group is not None or att.cp_group is not None or ff.tp_group is not None:
+            return None
+        for m in (blk, att, ff):
+            if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__:
+                return None
+        heads = (att.n_heads, att.n_kv_heads, att.head_dim)
+        if shape is not None and heads != shape:
+            return None
+        shape = heads
+        n1, n2, a, f = mods["attention_norm"], mods["ffn_norm"], att._modules, ff._modules
+        weights.append((n1._parameters.get("weight"), n1.eps, a["wq"]._parameters.get("weight"), a["wk"]._parameters.get("weight"),
+                        a["wv"]._parameters.get("weight"), a["wo"]._parameters.get("weight"), n2._parameters.get("weight"), n2.eps,
+                        f["w1"]._parameters.get("weight"), f["w3"]._parameters.get("weight"), f["w2"]._parameters.get("weight")))
+    return (*shape, 1.0 / math.sqrt(shape[2]), weights)
+
+
 class LightronTransformer(nn.Module):
     def __init__(self, args: ModelArgs, ctx: Optional[_mesh.ParallelContext] = None,
                  layer_range: Optional[Tuple[int, int]] = None, first_stage: bool = True, last_stage: bool = True,
@@ -213,6 +242,9 @@ class LightronTransformer(nn.Module):
         cos, sin = self.rope_tables(h.device)
         if positions is not None and h.is_cuda:
             positions = positions.to(device=h.device, dtype=torch.int32)
+        if not torch.is_grad_enabled() and (host := native.host_ops()) is not None and (run := _plain_layers(self.layers)) is not None:
+            if (out := host.decoder_layers(h, delta, cos, sin, positions, B, S, *run)) is not NotImplemented:
+                return out
         for blk in self.layers.values():
             h, delta = blk(h, delta, B, S, cos, sin, positions)
         return h, delta

@@ -52,6 +52,7 @@ _SIGNATURES = {
     "lb_gemm_bf16": [_P, _P, _P, _I, _I, _I, _L, _L, _L, _I, _I, _I, _P],
     "lb_gemm_grouped": [_I] + [_P] * 13,
     "lb_gemm_grouped_epi": [_I] + [_P] * 17,
+    "lb_gemm_rope": [_P, _P, _P, _I, _I, _I, _P, _P, _P, _I, _I, _I, _P],
     "lb_gemm_split": [_I] + [_P] * 16 + [_I, _P],
     "lb_gemm_split_status": [_P],
     "lb_peer_copy": [_P, _P, _L, _I, _I, _P],
@@ -238,7 +239,7 @@ def call(name: str, *args) -> None:
 _HOST = False               # not looked for yet; then the extension module, or None
 _HOST_ENTRIES = ("lb_rmsnorm_fwd", "lb_rmsnorm_bwd_blocks", "lb_rmsnorm_bwd", "lb_rope", "lb_gemm_grouped_epi", "lb_flash_fwd_tc",
                  "lb_flash_bwd_ws_bytes", "lb_flash_bwd_tc_ws", "lb_flash_bwd", "lb_embedding_fwd", "lb_clear", "lb_embedding_bwd", "lb_ce_stats",
-                 "lb_ce_loss", "lb_ce_grad")
+                 "lb_ce_loss", "lb_ce_grad", "lb_gemm_rope")
 
 
 def host_ops():

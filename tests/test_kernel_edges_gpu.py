@@ -254,6 +254,31 @@ def test_gemm_split_activation(ks, T, K, I):
     assert _rel(gu, want) < 5e-3 and _rel(h, act.detach()) < 5e-3 and _rel(dgu, g64.grad) < 1e-2
 
 
+@pytest.mark.parametrize("B,S,hq,hkv,d,K,form", [
+    (1, 37, 3, 1, 64, 72, (1, 0)), (2, 65, 4, 2, 128, 2056, (4, 0)), (3, 1000, 32, 8, 64, 264, (0, 1)), (4, 1100, 24, 4, 128, 1032, (0, 2)),
+])
+@pytest.mark.parametrize("placed", [False, True])
+def test_projection_with_rotation(B, S, hq, hkv, d, K, form, placed):
+    """The rotation in the epilogue against lb_rope on the projection's output: columns that are rotated and columns that are not, ragged rows,
+    positions of the caller's.  One rounding of the same fp32 values, which a contracted multiply and add may move across a boundary."""
+    from lightron_b200.ops import functional as OF, native
+    N, T = (hq + 2 * hkv) * d, B * S
+    assert _form((T, N, K)) == form
+    x, w = _rand(T, K, seed=1), _rand(N, K, scale=K ** -0.5, seed=2)
+    ang = torch.rand(2 * S, d // 2, device="cuda") * 6.28
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    pos = torch.randperm(2 * S, device="cuda")[:S].int().contiguous() if placed else None
+    got, want = torch.empty(T, N, device="cuda", dtype=torch.bfloat16), OF.gemm(x, w)
+    native.call("lb_gemm_rope", x.data_ptr(), w.data_ptr(), got.data_ptr(), T, N, K, cos.data_ptr(), sin.data_ptr(), native.ptr(pos), S, d,
+                (hq + hkv) * d, native.stream_ptr())
+    OF._rope_native_(want, cos, sin, pos, S, hq + hkv, d, False)
+    _status_ok()
+    assert torch.equal(got[:, (hq + hkv) * d:], want[:, (hq + hkv) * d:])
+    # a pair's two products cancel at worst: their fp32 rounding against the pair's size, and one unit in the last place of the result
+    size = want.float().view(T, -1, 2).norm(dim=-1, keepdim=True).expand(-1, -1, 2).reshape(T, N)
+    assert ((got.float() - want.float()).abs() <= 2.0 ** -7 * want.float().abs() + 2.0 ** -22 * size).all()
+
+
 @pytest.mark.parametrize("T,K,I,form", [(2100, 1032, 2312, (0, 2)), (4000, 256, 1288, (0, 1)), (300, 4096, 264, (4, 0)), (70, 512, 264, (1, 0))])
 def test_swiglu_mlp_forms(T, K, I, form):
     """The activation in the epilogue of pairs, whose peer loads the up rows, of single CTAs and of the split form; ragged in every size."""

@@ -96,3 +96,32 @@ def test_flat_arena_makes_qkv_adjacent():
     assert _rows_adjacent((att.wq.weight, att.wk.weight, att.wv.weight))
     ff = m.layers["0"].feed_forward
     assert _rows_adjacent((ff.w1.weight, ff.w3.weight))
+
+
+def test_which_layers_run_in_one_call():
+    """Only dense blocks of one GPU without hooks or a forward of their own."""
+    from lightron_b200.models.llama import _plain_layers
+    m = LightronTransformer(_tiny())
+    hq, hkv, d, scale, weights = _plain_layers(m.layers)
+    assert (hq, hkv, d) == (8, 8, 32) and abs(scale * d ** 0.5 - 1) < 1e-12 and len(weights) == 2
+    blk = m.layers["1"]
+    assert weights[1][2] is blk.attention.wq.weight and weights[1][10] is blk.feed_forward.w2.weight and weights[0][1] == m.args.norm_eps
+    for mod in (blk, blk.attention, blk.feed_forward):
+        for register in (mod.register_forward_hook, mod.register_forward_pre_hook, mod.register_full_backward_hook):
+            h = register(lambda *a: None)
+            assert _plain_layers(m.layers) is None
+            h.remove()
+        mod.forward = mod.forward
+        assert _plain_layers(m.layers) is None
+        del mod.forward
+    h = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    assert _plain_layers(m.layers) is None
+    h.remove()
+    assert _plain_layers(m.layers) is not None
+
+    class Other(type(blk.attention)):
+        pass
+    blk.attention.__class__ = Other
+    assert _plain_layers(m.layers) is None
+    assert _plain_layers(LightronTransformer(_tiny(moe_num_experts=2, moe_topk=1, moe_layer_freq=2)).layers) is None
+    assert _plain_layers(torch.nn.ModuleDict()) is None

@@ -84,3 +84,51 @@ def test_moe_grouped_expert_gemm_matches_per_expert_loop(monkeypatch):
         # flip for a few tokens, which moves every gradient upstream of a MoE layer more than rounding
         # does; the tight check is the one against the per-expert loop above (same routing)
         assert err < 0.3, f"{n}: grouped vs fp32 rel grad err {err.item()}"
+
+
+@pytest.mark.parametrize("dim,heads,kv,hidden,B,S", [
+    (768, 12, 12, None, 1, 128),         # every launch in the split form
+    (512, 4, 2, 1032, 2, 77),            # head_dim 128, ragged tokens
+    (1024, 16, 4, 2816, 3, 700),         # tiles from lists
+    (256, 4, 4, 264, 1, 1),
+])
+def test_layers_without_gradients_in_one_call(dim, heads, kv, hidden, B, S):
+    """The same logits as op by op, from fewer launches; what hooks into a block keeps its call."""
+    from lightron_b200 import mesh
+    from lightron_b200.config import ModelArgs
+    from lightron_b200.models import LightronTransformer, init_weights
+    from lightron_b200.models.llama import flatten_parameters
+    from lightron_b200.ops import native
+    mesh.set_context(None)
+    args = ModelArgs(dim=dim, n_layers=3, n_heads=heads, n_kv_heads=kv, vocab_size=512, intermediate_size=hidden, max_seq_len=2 * S + 16)
+    m = LightronTransformer(args, dtype=torch.bfloat16, device="cuda")
+    init_weights(m, 1, std=dim ** -0.5)
+    flatten_parameters(m)
+    tok = torch.randint(0, args.vocab_size, (B, S), device="cuda")
+    places = torch.arange(3, S + 3, device="cuda")
+    seen = []
+    for positions in (None, places):
+        n0 = native.launch_count()
+        want = m(tok, positions).detach()
+        n1 = native.launch_count()
+        with torch.no_grad():
+            got = m(tok, positions)
+        n2 = native.launch_count()
+        assert n2 - n1 < n1 - n0, "not in one call"
+        # the kernels' bf16 results are the same, but for a rotation's contracted multiply and add, whose flips three layers carry on
+        assert (got.float() - want.float()).norm() < 1e-2 * want.float().norm()
+        hook = m.layers["1"].register_forward_hook(lambda *a: seen.append(a[0]))
+        with torch.no_grad():
+            assert (m(tok, positions).float() - want.float()).norm() < 1e-2 * want.float().norm()
+        hook.remove()
+    assert seen == [m.layers["1"]] * 2
+    # a run that starts with an add that is pending, and leaves its inputs as they are
+    h, d = (torch.randn(B * S, dim, device="cuda").bfloat16() for _ in range(2))
+    h0, d0 = h.clone(), d.clone()
+    want = [t.detach() for t in m.run_layers(h, d, B, S, None)]
+    with torch.no_grad():
+        got = m.run_layers(h, d, B, S, None)
+    assert torch.equal(h, h0) and torch.equal(d, d0)
+    for g, w in zip(got, want):
+        assert (g.float() - w.float()).norm() < 1e-2 * w.float().norm()
+    native.raise_on_device_status()

@@ -14,12 +14,13 @@
 // of 4 (CTA) or 6 (pair) stages -> tcgen05.mma 128x256x16 / 256x256x16 -> two 256-column TMEM accumulators
 // per CTA -> tcgen05.ld epilogue overlapped with the next tile.  `accumulate` adds the old contents of C in
 // the epilogue (gradient accumulation over micro-batches without a separate add).
-// The ragged kernel (lb_gemm_ragged, lb_gemm_ragged_wgrad) uses the CTA form and takes its tiles from device memory.
+// The ragged kernel (lb_gemm_ragged, lb_gemm_ragged_wgrad) takes its tiles from device memory.
 // Every wait is bounded; on expiry the kernel records a status code (lb_gemm_grouped_status),
 // stops issuing work, frees its TMEM and returns.
 #include <cuda.h>
 #include <string.h>
 #include <algorithm>
+#include <cmath>
 #include <map>
 #include <mutex>
 #include <queue>
@@ -538,6 +539,7 @@ struct RaggedParams {
 struct RaggedTile { int e, m0, n0, num_kb, k_base; };
 
 // Tile `t` of the launch, or e < 0 past the end.  seg_* are the CTA's shared copies of the table.
+template <int CG>
 __device__ __forceinline__ RaggedTile ragged_tile(int t, const RaggedParams& rp, const int* s_off, const int* s_tiles) {
   RaggedTile r;
   r.e = -1; r.m0 = r.n0 = r.num_kb = r.k_base = 0;
@@ -549,7 +551,7 @@ __device__ __forceinline__ RaggedTile ragged_tile(int t, const RaggedParams& rp,
         pr.tiles_m = s_tiles[e]; pr.tiles_n = rp.tiles_n;
         int tm, tn;
         tile_coords(t, pr, tm, tn);
-        r.e = e; r.m0 = s_off[e] + tm * BM; r.n0 = tn * (rp.epi == 1 ? BN / 2 : BN); r.num_kb = rp.num_kb;
+        r.e = e; r.m0 = s_off[e] + tm * BM * CG; r.n0 = tn * (rp.epi == 1 ? BN / 2 : BN); r.num_kb = rp.num_kb;
         return r;
       }
       t -= nt;
@@ -559,7 +561,7 @@ __device__ __forceinline__ RaggedTile ragged_tile(int t, const RaggedParams& rp,
     const int e = t / per;
     if (e < rp.LE) {
       const int tt = t - e * per;
-      r.e = e; r.m0 = (tt % rp.tiles_m_w) * BM; r.n0 = (tt / rp.tiles_m_w) * BN;
+      r.e = e; r.m0 = (tt % rp.tiles_m_w) * BM * CG; r.n0 = (tt / rp.tiles_m_w) * BN;
       r.num_kb = s_tiles[e];              // 64-row steps over the segment
       r.k_base = s_off[e];
     }
@@ -567,15 +569,16 @@ __device__ __forceinline__ RaggedTile ragged_tile(int t, const RaggedParams& rp,
   return r;
 }
 
+template <int CG>
 __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __grid_constant__ RaggedParams rp) {
-  using CF = Cfg<1>;
+  using CF = Cfg<CG>;
   constexpr int STAGES = CF::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + CF::OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   __shared__ int s_abort[2];     // {abort, extra wait in ms}: see bw::mbar_wait
-  __shared__ int s_off[MAX_PROBLEMS], s_tiles[MAX_PROBLEMS];
+  __shared__ int s_off[MAX_PROBLEMS], s_tiles[MAX_PROBLEMS], s_end[MAX_PROBLEMS];
 
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);      // (uniform over the warp)
   const int lane = threadIdx.x & 31;
@@ -586,6 +589,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
   auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + 2 + a); };
 
+  const int worker = (int)blockIdx.x / CG, workers = (int)gridDim.x / CG;
+  const int rank = CG == 2 ? (int)bw::cluster_ctarank() : 0;      // 0 = leader: issues the MMAs of the pair
+
   if (threadIdx.x == 0) {
     s_abort[0] = 0;
     s_abort[1] = rp.wait_flag ? bw::wait_extra_ms(rp.wait_ns) : 0;
@@ -595,11 +601,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
     }
     for (int a = 0; a < 2; a++) {
       bw::mbar_init(tfull_bar(a), 1);
-      bw::mbar_init(tempty_bar(a), 4);
+      bw::mbar_init(tempty_bar(a), 4 * CG);
     }
     bw::mbar_init_fence();
   }
-  if (warp == 1) bw::tmem_alloc(bw::smem_u32(tmem_slot), 512);
+  if (warp == 1) {
+    if constexpr (CG == 2) bw::tmem_alloc_pair(bw::smem_u32(tmem_slot), 512);
+    else bw::tmem_alloc(bw::smem_u32(tmem_slot), 512);
+  }
   grid_wait();
   if (threadIdx.x < rp.LE) {
     // segment table -> offsets and tile (mode 0: 128-row tiles) / step (mode 1: 64-row steps) counts,
@@ -609,10 +618,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
     if (cnt < 0) cnt = 0;
     if (off + cnt > rp.cap) cnt = rp.cap - off;
     s_off[threadIdx.x] = off;
-    s_tiles[threadIdx.x] = rp.mode == 0 ? (cnt + BM - 1) / BM : (cnt + BK - 1) / BK;
+    s_tiles[threadIdx.x] = rp.mode == 0 ? (cnt + BM * CG - 1) / (BM * CG) : (cnt + BK - 1) / BK;
+    s_end[threadIdx.x] = min(off + (cnt + BM - 1) / BM * BM, rp.cap);      // (the second CTA's rows may be the next segment's)
   }
   bw::fence_before();
   __syncthreads();
+  if constexpr (CG == 2) bw::cluster_sync();      // the peer's barriers exist before anything signals them
   bw::fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   volatile int* abort_flag = s_abort;
@@ -629,28 +640,37 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
         if (!lbcomm::flag_wait_ge(rp.wait_flag, rp.wait_target, rp.wait_ns)) { give_up(abort_flag, 11u); ok = false; }
         asm volatile("fence.proxy.async;" ::: "memory");
       }
-      for (int t = blockIdx.x; ok; t += gridDim.x) {
-        const RaggedTile rt = ragged_tile(t, rp, s_off, s_tiles);
+      for (int t = worker; ok; t += workers) {
+        const RaggedTile rt = ragged_tile<CG>(t, rp, s_off, s_tiles);
         if (rt.e < 0) break;
         if (rt.num_kb == 0) continue;
+        const int split = rp.epi == 1 ? rp.half : 0;
+        // this CTA's first rows of A and of B (see gemm_grouped_kernel)
+        const int m0 = rt.m0 + rank * BM, n0 = rt.n0 + (CG == 2 ? rank * (split ? split : BN / 2) : 0);
         if (rp.mode == 0) {
-          if (!rp.b_mn) ok = produce_tile<1, false, false>(&rp.ta, &rp.tb[rt.e], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, true, 0, rp.epi == 1 ? rp.half : 0);
-          else          ok = produce_tile<1, false, true>(&rp.ta, &rp.tb[rt.e], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, true);
+          if (!rp.b_mn) ok = produce_tile<CG, false, false>(&rp.ta, &rp.tb[rt.e], m0, n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, 0, split);
+          else          ok = produce_tile<CG, false, true>(&rp.ta, &rp.tb[rt.e], m0, n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0);
         } else {
-          ok = produce_tile<1, true, true>(&rp.ta, &rp.tb[0], rt.m0, rt.n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, true, rt.k_base);
+          ok = produce_tile<CG, true, true>(&rp.ta, &rp.tb[0], m0, n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, rt.k_base);
         }
         if (!ok) give_up(abort_flag, 1u);
       }
+      // the leader's MMAs release this CTA's stages: all releases have arrived before the CTA may exit
+      if (CG == 2)
+        for (int s = 0; s < STAGES && ok; s++) {
+          ok = bw::mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag);
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (bw::elect_one()) {
+    if (rank == 0 && bw::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       int n = 0;
-      for (int t = blockIdx.x; ok; t += gridDim.x) {
-        const RaggedTile rt = ragged_tile(t, rp, s_off, s_tiles);
+      for (int t = worker; ok; t += workers) {
+        const RaggedTile rt = ragged_tile<CG>(t, rp, s_off, s_tiles);
         if (rt.e < 0) break;
         if (rt.num_kb == 0) continue;
         const int acc = n & 1;
@@ -659,13 +679,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
         bw::fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * BN;
         if (rp.mode == 0) {
-          if (!rp.b_mn) ok = mma_tile<1, false, false>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
-          else          ok = mma_tile<1, false, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
+          if (!rp.b_mn) ok = mma_tile<CG, false, false>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
+          else          ok = mma_tile<CG, false, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
         } else {
-          ok = mma_tile<1, true, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
+          ok = mma_tile<CG, true, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
         }
-        if (ok) bw::umma_commit(tfull_bar(acc));
-        else give_up(abort_flag, 3u);
+        if (!ok) give_up(abort_flag, 3u);
+        else if constexpr (CG == 2) bw::umma_commit_pair(tfull_bar(acc));
+        else bw::umma_commit(tfull_bar(acc));
         n++;
       }
     }
@@ -674,12 +695,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
     const int quad = warp & 3;
     uint8_t* stg = smem + CF::OFF_STG + quad * 2 * STG_BYTES;
     int n = 0, turn = 0;
-    for (int t = blockIdx.x;; t += gridDim.x) {
-      const RaggedTile rt = ragged_tile(t, rp, s_off, s_tiles);
+    for (int t = worker;; t += workers) {
+      const RaggedTile rt = ragged_tile<CG>(t, rp, s_off, s_tiles);
       if (rt.e < 0) break;
       if (rt.num_kb == 0) {
         // an expert without rows: its weight gradient is zero (nothing to add when accumulating)
-        const int row = rt.m0 + quad * 32 + lane;
+        const int row = rt.m0 + rank * BM + quad * 32 + lane;
         if (rp.mode == 1 && !rp.accumulate && row < rp.M_w)
           for (int c = rt.n0; c < rt.n0 + BN && c < rp.N; c += 8)
             *reinterpret_cast<uint4*>(rp.C[rt.e] + (size_t)row * rp.ldc + c) = make_uint4(0, 0, 0, 0);
@@ -689,7 +710,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
       const uint32_t acc_phase = (uint32_t)(n >> 1) & 1u;
       const bool wgrad = rp.mode == 1;
       // (mode 0 writes whole 128-row tiles: padding rows are zeros)
-      const Out out{wgrad ? &rp.tc[rt.e] : rp.tc, wgrad ? rp.C[rt.e] : rp.old, wgrad ? rp.ldc : rp.ld_old, rt.m0 + quad * 32, wgrad ? rp.M_w : rp.cap,
+      const Out out{wgrad ? &rp.tc[rt.e] : rp.tc, wgrad ? rp.C[rt.e] : rp.old, wgrad ? rp.ldc : rp.ld_old, rt.m0 + rank * BM + quad * 32, wgrad ? rp.M_w : s_end[rt.e],
                     rt.n0, rp.epi ? rp.half : rp.N, true, nullptr};
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * BN;
       auto ready = [&]() {
@@ -700,7 +721,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
       auto release = [&]() {
         bw::fence_before();
         __syncwarp();
-        if (lane == 0) bw::mbar_arrive(tempty_bar(acc));
+        if (lane == 0) {
+          if constexpr (CG == 2) bw::mbar_arrive_leader(tempty_bar(acc));
+          else bw::mbar_arrive(tempty_bar(acc));
+        }
       };
       bool ok;
       switch (wgrad && rp.accumulate ? 3 : rp.epi) {
@@ -717,9 +741,11 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
 
   bw::fence_before();
   __syncthreads();
+  if constexpr (CG == 2) bw::cluster_sync();      // nothing of the pair is in flight in either CTA
   if (warp == 1) {
     bw::fence_after();
-    bw::tmem_dealloc(tmem_base, 512);
+    if constexpr (CG == 2) bw::tmem_dealloc_pair(tmem_base, 512);
+    else bw::tmem_dealloc(tmem_base, 512);
   }
 }
 
@@ -1067,6 +1093,49 @@ extern "C" int lb_gemm_grouped(int n, const void* const* A, const void* const* B
                              stream);
 }
 
+namespace {
+// CTAs per tile.  The rows are known on the device only: as many as the buffer holds beyond its padding, the same for every expert, half a tile of each
+// wasted.  Both forms' times as tile_time() has them for the lists (a pair's as those of a launch, 6 k-blocks more), 3 % for the
+// unevenness, which costs pairs more.  CTAs / pairs in us, 8 experts, 2048 -> 4096, 2 of them per token, 4096 tokens: gate | up 254 / 220, down 127 / 106, its data
+// gradient 143 / 144, gate | up's 251 / 252; 1024 tokens 88 / 77, 60 / 54, 64 / 60, 107 / 96; 64 tokens 54 / 63, 34 / 33, 38 / 44, 56 / 58; 4096 tokens of 4
+// experts, 1024 -> 4096: 131 / 108, 59 / 55, 124 / 127, 111 / 104.
+int ragged_cg(int LE, int cap, int n, int num_kb, int sms) {
+  if (sms < 2) return 1;
+  const double rows = std::max(1.0, (double)(cap - LE * BM) / LE);
+  const double tn = (n + BN - 1) / BN;
+  double time[3];
+  for (int cg = 1; cg <= 2; cg++) {
+    const double tiles = LE * std::max(1.0, rows / (BM * cg) + 0.5) * tn;
+    time[cg] = std::ceil(tiles / (sms / cg)) * (double)tile_time(num_kb, cg);
+  }
+  return 1.03 * (time[2] + 600) < time[1] ? 2 : 1;
+}
+// Weight gradients: as many tiles whatever the rows are, but with few of them a tile is mostly its store.  CTAs / pairs, down and gate | up: 1024 rows per expert
+// 126 / 118 and 282 / 222, 512 90 / 79 and 158 / 137, 256 48 / 59 and 88 / 105.
+int ragged_wgrad_cg(int LE, int cap, int sms) {
+  return sms >= 2 && (cap - LE * BM) / LE >= 512 ? 2 : 1;
+}
+int launch_ragged(int cg, bool dependent, const RaggedParams& rp, cudaStream_t s) {
+  {
+    std::lock_guard<std::mutex> lock(g_sched_mutex);
+    static bool attr = false;
+    if (!attr) {
+      cudaFuncSetAttribute(gemm_ragged_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
+      cudaFuncSetAttribute(gemm_ragged_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
+      attr = true;
+    }
+  }
+  if (cg == 2) return lb_launch_cluster(dependent, 2, gemm_ragged_kernel<2>, lb_num_sms() / 2 * 2, NUM_THREADS, Cfg<2>::SMEM_BYTES, s, rp);
+  return lb_launch_cluster(dependent, 1, gemm_ragged_kernel<1>, lb_num_sms(), NUM_THREADS, Cfg<1>::SMEM_BYTES, s, rp);
+}
+}  // namespace
+
+// Host only (no CUDA call): CTAs per tile, 1 or 2, of an expert GEMM over a buffer of `cap` rows (K > 0), or of its weight gradient (K = 0), on `sms` SMs.
+extern "C" int lb_gemm_ragged_ctas_per_tile(int LE, int cap, int N, int K, int sms) {
+  if (LE < 1 || LE > MAX_PROBLEMS || cap <= 0 || N <= 0 || K < 0 || sms < 1) return LB_ERR_SHAPE;
+  return K ? ragged_cg(LE, cap, N, (K + BK - 1) / BK, sms) : ragged_wgrad_cg(LE, cap, sms);
+}
+
 // Expert GEMMs over ragged row segments (see gemm_ragged_kernel).  seg: device table of 2 * LE + 2
 // ints (offsets, counts, ...), LE <= 8 local experts.
 //  mode 0: C [cap, N] = A [cap, K] . op(B_e)^T per segment; B: host array of LE weight pointers
@@ -1099,12 +1168,7 @@ extern "C" int lb_gemm_ragged_epi(const void* A, const void* const* B, void* C, 
   rp.mode = 0; rp.accumulate = 0; rp.cap = cap;
   rp.tiles_n = (N + BN - 1) / BN; rp.tiles_m_w = 0; rp.num_kb = (K + BK - 1) / BK;
   rp.wait_flag = (const unsigned int*)wait_flag; rp.wait_target = wait_target; rp.wait_ns = g_lb_flag_wait_ns;
-  {
-    std::lock_guard<std::mutex> lock(g_sched_mutex);
-    static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(gemm_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES); attr = true; }
-  }
-  return lb_launch_cluster(!wait_flag, 1, gemm_ragged_kernel, lb_num_sms(), NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream, rp);
+  return launch_ragged(ragged_cg(LE, cap, N, rp.num_kb, lb_num_sms()), !wait_flag, rp, (cudaStream_t)stream);
 }
 
 extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, const void* seg, int LE, int cap, int N, int K,
@@ -1122,6 +1186,7 @@ extern "C" int lb_gemm_ragged_wgrad(const void* dY, const void* X, void* const* 
   if ((lddy % 8) || (ldx % 8) || (ldc % 8) || (Nw % 8) || (Kw % 8)) return LB_ERR_SHAPE;
   if (((uintptr_t)dY | (uintptr_t)X) & 15) return LB_ERR_ARG;
   static thread_local RaggedParams rp;
+  const int cg = ragged_wgrad_cg(LE, cap, lb_num_sms());
   int rc = bw::make_map_bf16(&rp.ta, dY, (uint64_t)Nw, (uint64_t)cap, (uint64_t)lddy, 64, BK);
   if (rc) return rc;
   rc = bw::make_map_bf16(&rp.tb[0], X, (uint64_t)Kw, (uint64_t)cap, (uint64_t)ldx, 64, BK);
@@ -1133,13 +1198,7 @@ extern "C" int lb_gemm_ragged_wgrad(const void* dY, const void* X, void* const* 
   }
   rp.ldc = ldc; rp.old = nullptr; rp.ld_old = 0; rp.epi = 0; rp.half = 0; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = Nw; rp.N = Kw; rp.K = 0; rp.b_mn = 1; rp.mode = 1;
   rp.accumulate = accumulate; rp.cap = cap;
-  rp.tiles_n = (Kw + BN - 1) / BN; rp.tiles_m_w = (Nw + BM - 1) / BM; rp.num_kb = 0;
+  rp.tiles_n = (Kw + BN - 1) / BN; rp.tiles_m_w = (Nw + BM * cg - 1) / (BM * cg); rp.num_kb = 0;
   rp.wait_flag = nullptr; rp.wait_target = 0; rp.wait_ns = g_lb_flag_wait_ns;
-  {
-    std::lock_guard<std::mutex> lock(g_sched_mutex);
-    static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(gemm_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES); attr = true; }
-  }
-  LB_LAUNCH(gemm_ragged_kernel, lb_num_sms(), NUM_THREADS, Cfg<1>::SMEM_BYTES, (cudaStream_t)stream, rp);
-  return LB_OK;
+  return launch_ragged(cg, true, rp, (cudaStream_t)stream);
 }

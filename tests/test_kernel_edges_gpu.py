@@ -544,17 +544,22 @@ def test_moe_plan_sums_over_blocks(nblk, E):
     _status_ok()
 
 
-@pytest.mark.parametrize("H,I", [(72, 264), (264, 8), (520, 1032)])
-def test_ragged_activation_epilogues(H, I):
-    """Segments of one to several tiles, without rows and of one row; widths that end inside a tile and inside a step of 64 columns."""
+@pytest.mark.parametrize("H,I,counts,ctas", [(72, 264, (130, 0, 1, 300), 1), (264, 8, (130, 0, 1, 300), 1), (520, 1032, (130, 0, 1, 300), 1),
+                                             (4104, 264, (300, 0, 129, 1290), 2)])
+def test_ragged_expert_gemms(H, I, counts, ctas):
+    """Activation epilogues and weight gradients in single CTAs and in pairs, whose last tile may end in the next segment: segments of one to several
+    tiles, without rows and of one row; widths that end inside a tile and inside a step of 64 columns."""
+    from lightron_b200.ops import native
     from lightron_b200.parallel import ep_fused
-    counts = [130, 0, 1, 300]
-    LE, cap = len(counts), 1024
+    LE, cap = len(counts), 1024 if ctas == 1 else 2560
     off, seg = 0, []
     for c in counts:
         seg.append(off)
         off += (c + 127) // 128 * 128
-    table = torch.tensor(seg + counts + [off, sum(counts)], dtype=torch.int32, device="cuda")
+    assert off < cap
+    lib, sms = native.require(), native.sm_count()
+    assert [lib.lb_gemm_ragged_ctas_per_tile(LE, cap, n, k, sms) for n, k in ((2 * I, H), (I, H), (H, 0))] == [ctas] * 3
+    table = torch.tensor([*seg, *counts, off, sum(counts)], dtype=torch.int32, device="cuda")
     x, dy = _rand(cap, H, seed=1), _rand(cap, H, seed=2)
     live = torch.zeros(cap, dtype=torch.bool, device="cuda")
     for o, c in zip(seg, counts):
@@ -566,12 +571,20 @@ def test_ragged_activation_epilogues(H, I):
     gu, act, dgu = (torch.full((cap, n), 7.0, device="cuda", dtype=torch.bfloat16) for n in (2 * I, I, 2 * I))
     ep_fused._ragged(x, up, gu, table, LE, cap, 2 * I, H, False, epi=1, c2=act, half=I)
     ep_fused._ragged(dy, down, dgu, table, LE, cap, I, H, True, epi=2, c2=gu, half=I)
+    old = [_rand(2 * I, H, seed=30 + e) for e in range(LE)]
+    dw = [[w.clone() for w in old] for _ in range(2)]
+    for accumulate in (0, 1):
+        ep_fused._ragged_wgrad(dgu, x, dw[accumulate], table, LE, cap, 2 * I, H, accumulate)
     _status_ok()
     assert (gu[off:] == 7).all() and (act[off:] == 7).all() and (dgu[off:] == 7).all()
     for e, (o, c) in enumerate(zip(seg, counts)):
+        r = slice(o, o + c)
+        grad = dgu[r].double().t() @ x[r].double()
+        for accumulate in (0, 1):
+            want = grad + old[e].double() * accumulate
+            assert _rel(dw[accumulate][e], want) < 5e-3 if want.any() else not dw[accumulate][e].any()
         if not c:
             continue
-        r = slice(o, o + c)
         assert _rel(gu[r], x[r].double() @ up[e].double().t()) < 5e-3
         g, u = gu[r].double().split(I, 1)
         sig = torch.sigmoid(g)

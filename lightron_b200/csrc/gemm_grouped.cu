@@ -326,8 +326,10 @@ __device__ __forceinline__ bool store_tile(const Out& o, uint32_t taddr, uint8_t
           }
           if constexpr (EPI == 4) {
             if (col + g * 8 < o.rope->cols) {
+              float cs[8];
               unpack8(pack8(f), f);                                   // the values a stored C would have
-              rope_rotate8(*o.rope, pos, col + g * 8, f);
+              rope_load8(*o.rope, pos, col + g * 8, cs);
+              rope_rotate8(cs, f);
             }
           }
           *at(buf, g) = pack8(f);

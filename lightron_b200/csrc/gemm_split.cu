@@ -8,11 +8,14 @@
 // 11.7 / 8.0, 128 x 768 x 2048 17.2 / 7.4, 128 x 2048 x 5632 32.7 / 12.8, 1000 x 768 x 2048 18.3 / 12.4; data and weight gradient of
 // 1000 x 768 x 768 13.2 / 10.1.  What is left (6 us for the shortest): launch, barriers and tensor memory, one round trip to memory, stores.
 //
-// A CTA of a split tile leaves the sum over its part of K in tensor memory.  When all CTAs of the cluster are done, each sends the
-// columns that another one owns into that one's shared memory (the pipeline's stages, which nothing uses any more), and adds what it receives to
-// its own in the order of the parts: the result does not depend on timing.  Roles, pipeline, descriptors and epilogues are those of gemm_grouped.cu.
+// A CTA of a split tile leaves the sum over its part of K in tensor memory.  It sends the columns that another CTA of the cluster owns into that one's
+// shared memory, where they are counted on a barrier, and adds what it receives to its own in the order of the parts: the result does not depend on
+// timing.  Roles, pipeline, descriptors and epilogues are those of gemm_grouped.cu.  Cycles from the end of the wait for the kernel before (clock64, 128 x
+// 768 x 768 in 4 parts): first stage 1800, accumulator 3050; then 5300 for two cluster barriers, eight columns at a time and a loop over the parts,
+// which is why the parts are a template's, the columns come in one load and the sums are counted on a barrier.  128 x 2304 x 768 with the rotation: 7300
+// of 13900 cycles were its tables, fetched per eight columns; they are now on their way while the MMAs run.
 // A launch starts under the kernel before it (grid_go(), grid_wait()), and asks for its part of B, which that kernel hardly ever writes, to be brought to
-// L2 meanwhile: the 99 kernels of 12 layers of 768 columns over 128 tokens 575 us launched one after the other, 521 so, 495 with the request.
+// L2 meanwhile: the 99 kernels of 12 layers of 768 columns over 128 tokens 575 us launched one after the other, 521 so, 495 with the request.  (The 87 kernels of the same without gradients: 486, and 471 with what the paragraph above changed.)
 // Every wait is bounded; on expiry the kernel records a status code (lb_gemm_split_status), stops issuing work, frees its TMEM and returns.
 #include <algorithm>
 #include "gemm_split.h"
@@ -25,11 +28,18 @@ namespace {
 constexpr int BM = 128, BN = 64, BK = 64;
 constexpr int HB = BN / 2;                               // columns of a tile's two blocks
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES, STAGES = 4;
-constexpr int OFF_BAR = STAGES * STAGE_BYTES;
-constexpr int SMEM_BYTES = OFF_BAR + 256;
-static_assert(BM * BN * 4 <= STAGES * STAGE_BYTES, "the partial sums fit in the stages");
-static_assert(2 * (SMEM_BYTES + 1024) <= 233472, "two CTAs per SM");
+constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+// KS parts of K.  With four a CTA has few k-blocks, and the place of a fourth stage is where the others' sums arrive.
+template <int KS>
+struct Cfg {
+  static constexpr int STAGES = KS == 4 ? 3 : 4;
+  static constexpr int W = HB / KS;                      // columns of each block that a CTA finishes
+  static constexpr int RECV_BYTES = (KS - 1) * BM * 2 * W * 4;
+  static constexpr int OFF_RECV = STAGES * STAGE_BYTES;
+  static constexpr int OFF_BAR = OFF_RECV + RECV_BYTES;
+  static constexpr int SMEM_BYTES = OFF_BAR + 256;
+  static_assert(2 * (SMEM_BYTES + 1024) <= 233472, "two CTAs per SM");
+};
 constexpr int NUM_THREADS = 192;
 constexpr int MAX_PROBLEMS = 2;
 constexpr int PREFETCH = 16;                             // k-blocks of B that a CTA asks for ahead of its start (38 MB of all CTAs that run at a time)
@@ -49,7 +59,7 @@ struct Params {
   CUtensorMap ta[MAX_PROBLEMS], tb[MAX_PROBLEMS];
   Problem prob[MAX_PROBLEMS];
   RopeArgs rope;
-  int np, ks;
+  int np;
 };
 
 __device__ __forceinline__ void give_up(volatile int* abort_flag, unsigned where) {
@@ -58,7 +68,7 @@ __device__ __forceinline__ void give_up(volatile int* abort_flag, unsigned where
   atomicExch(&g_split_status[1], where);
 }
 
-template <bool A_MN, bool B_MN>
+template <int STAGES, bool A_MN, bool B_MN>
 __device__ __forceinline__ bool produce(const CUtensorMap* ta, const CUtensorMap* tb, int m0, int n0, int n1, int a_rows, int kb0, int n_kb,
                                         uint32_t smem_base, uint32_t bar_base, volatile int* abort_flag) {
   int stage = 0;
@@ -86,7 +96,7 @@ __device__ __forceinline__ bool produce(const CUtensorMap* ta, const CUtensorMap
   return true;
 }
 
-template <bool A_MN, bool B_MN>
+template <int STAGES, bool A_MN, bool B_MN>
 __device__ __forceinline__ bool multiply(uint32_t d_tmem, int n_kb, uint32_t smem_base, uint32_t bar_base, volatile int* abort_flag) {
   constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) |
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
@@ -108,18 +118,21 @@ __device__ __forceinline__ bool multiply(uint32_t d_tmem, int n_kb, uint32_t sme
   return true;
 }
 
+template <int KS>
 __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid_constant__ Params gp) {
+  using C = Cfg<KS>;
+  constexpr int STAGES = C::STAGES, W = C::W, NG = W / 8;      // NG: groups of 8 columns per block that this CTA finishes
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t smem_base = bw::smem_u32(smem);
-  const uint32_t bar_base = smem_base + OFF_BAR;
-  const uint32_t tfull = bar_base + 8u * 2 * STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 8 * (2 * STAGES + 1));
+  const uint32_t bar_base = smem_base + C::OFF_BAR;
+  const uint32_t tfull = bar_base + 8u * 2 * STAGES, received = tfull + 8;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + 8 * (2 * STAGES + 2));
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);        // {abort, extra wait in ms}: see bw::mbar_wait
   volatile int* abort_flag = s_abort;
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);      // (uniform over the warp)
   const int lane = threadIdx.x & 31;
-  const int ks = gp.ks, rank = ks > 1 ? (int)bw::cluster_ctarank() : 0;
-  const int t = (int)blockIdx.x / ks;
+  const int rank = KS > 1 ? (int)bw::cluster_ctarank() : 0;
+  const int t = (int)blockIdx.x / KS;
   const int pi = gp.np > 1 && t >= gp.prob[1].first ? 1 : 0;
   const Problem& pr = gp.prob[pi];
   const int tl = t - pr.first;
@@ -128,7 +141,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
   // the tile's two blocks of columns: neighbours, or the gate and the up columns of the same index
   const int n0 = pr.epi == 1 ? tn * HB : tn * BN;
   const int n1 = pr.epi == 1 ? pr.half + n0 : n0 + HB;
-  const int kb0 = (int)((long long)pr.num_kb * rank / ks), n_kb = (int)((long long)pr.num_kb * (rank + 1) / ks) - kb0;
+  const int kb0 = (int)((long long)pr.num_kb * rank / KS), n_kb = (int)((long long)pr.num_kb * (rank + 1) / KS) - kb0;
 
   if (threadIdx.x == 64) { bw::prefetch_tmap(&gp.ta[pi]); bw::prefetch_tmap(&gp.tb[pi]); }
   if (threadIdx.x == 0) {
@@ -140,11 +153,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
       bw::mbar_init(bar_base + 8u * (STAGES + s), 1);
     }
     bw::mbar_init(tfull, 1);
+    bw::mbar_init(received, 1);
     bw::mbar_init_fence();
+    if (KS > 1) bw::mbar_expect_tx(received, C::RECV_BYTES);
   }
   if (warp == 1) bw::tmem_alloc(bw::smem_u32(tmem_slot), BN);
   bw::fence_before();
   __syncthreads();
+  if constexpr (KS > 1) bw::cluster_sync();                    // the peers' barriers exist before anything is sent
   bw::fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   bool ok = *abort_flag == 0;
@@ -163,137 +179,160 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
   }
   grid_wait();
 
+  const int quad = warp & 3, row_in = quad * 32 + lane;
+  const int row = m0 + row_in;
+  const bool row_ok = row < pr.M;
+  const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
+  float rot[2][NG][8];                                         // epi 4: cosines and sines of this row's columns, loaded ahead
   if (warp == 0) {
     if (ok && bw::elect_one()) {
       const CUtensorMap *ta = &gp.ta[pi], *tb = &gp.tb[pi];
       switch (pr.a_mn * 2 + pr.b_mn) {
-        case 0: ok = produce<false, false>(ta, tb, m0, n0, n1, pr.a_rows, kb0, n_kb, smem_base, bar_base, abort_flag); break;
-        case 1: ok = produce<false, true>(ta, tb, m0, n0, n1, pr.a_rows, kb0, n_kb, smem_base, bar_base, abort_flag); break;
-        case 2: ok = produce<true, false>(ta, tb, m0, n0, n1, pr.a_rows, kb0, n_kb, smem_base, bar_base, abort_flag); break;
-        default: ok = produce<true, true>(ta, tb, m0, n0, n1, pr.a_rows, kb0, n_kb, smem_base, bar_base, abort_flag); break;
+        case 0: ok = produce<STAGES, false, false>(ta, tb, m0, n0, n1, pr.a_rows, kb0, n_kb, smem_base, bar_base, abort_flag); break;
+        case 1: ok = produce<STAGES, false, true>(ta, tb, m0, n0, n1, pr.a_rows, kb0, n_kb, smem_base, bar_base, abort_flag); break;
+        case 2: ok = produce<STAGES, true, false>(ta, tb, m0, n0, n1, pr.a_rows, kb0, n_kb, smem_base, bar_base, abort_flag); break;
+        default: ok = produce<STAGES, true, true>(ta, tb, m0, n0, n1, pr.a_rows, kb0, n_kb, smem_base, bar_base, abort_flag); break;
       }
       if (!ok) give_up(abort_flag, 1u);
     }
   } else if (warp == 1) {
     if (ok && bw::elect_one()) {
       switch (pr.a_mn * 2 + pr.b_mn) {
-        case 0: ok = multiply<false, false>(tmem_base, n_kb, smem_base, bar_base, abort_flag); break;
-        case 1: ok = multiply<false, true>(tmem_base, n_kb, smem_base, bar_base, abort_flag); break;
-        case 2: ok = multiply<true, false>(tmem_base, n_kb, smem_base, bar_base, abort_flag); break;
-        default: ok = multiply<true, true>(tmem_base, n_kb, smem_base, bar_base, abort_flag); break;
+        case 0: ok = multiply<STAGES, false, false>(tmem_base, n_kb, smem_base, bar_base, abort_flag); break;
+        case 1: ok = multiply<STAGES, false, true>(tmem_base, n_kb, smem_base, bar_base, abort_flag); break;
+        case 2: ok = multiply<STAGES, true, false>(tmem_base, n_kb, smem_base, bar_base, abort_flag); break;
+        default: ok = multiply<STAGES, true, true>(tmem_base, n_kb, smem_base, bar_base, abort_flag); break;
       }
       if (ok) bw::umma_commit(tfull);                          // accumulator complete
       else give_up(abort_flag, 2u);
     }
   } else {
+    if (pr.epi == 4) {
+      const int pos = row_ok ? rope_position(gp.rope, row) : 0;
+#pragma unroll
+      for (int b = 0; b < 2; b++)
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+          const int col = (b ? n1 : n0) + rank * W + g * 8;
+          if (col < gp.rope.cols) rope_load8(gp.rope, pos, col, rot[b][g]);
+        }
+    }
     if (ok && !bw::mbar_wait(tfull, 0, abort_flag)) { ok = false; give_up(abort_flag, 3u); }
+    ok = __all_sync(0xffffffffu, ok);
   }
   __syncwarp();
   bw::fence_after();
 
-  const int quad = warp & 3, row_in = quad * 32 + lane;
-  const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
-  const int w = HB / ks;                                       // columns of each block that this CTA finishes (a multiple of 8)
-  if (ks > 1) {
-    bw::cluster_sync();                                        // the MMAs of all parts are done: their stages are free
-    if (warp >= 2) {
-      for (int i = 1; i < ks; i++) {
-        const int s = (rank + i) % ks;                         // the receiver of these columns
-        const uint32_t dst = bw::cluster_addr(smem_base, s) + (uint32_t)(rank * 2 * w * BM * 4 + row_in * 16);
-        for (int b = 0; b < 2; b++)
-          for (int c = 0; c < w; c += 8) {
-            uint32_t r[8];
-            bw::tmem_ld8(taddr + b * HB + s * w + c, r);
-            bw::tmem_ld_wait();
-            bw::st_cluster_v4(dst + (uint32_t)((b * w + c) * BM * 4), r);
-            bw::st_cluster_v4(dst + (uint32_t)((b * w + c + 4) * BM * 4), r + 4);
-          }
+  if constexpr (KS > 1) {
+    if (warp >= 2 && ok) {
+      // 8 columns at a time to the CTA that finishes them
+      const uint32_t mine = smem_base + C::OFF_RECV + (uint32_t)(row_in * 16);
+#pragma unroll
+      for (int b = 0; b < 2; b++) {
+        uint32_t r[32];
+        bw::tmem_ld32(taddr + b * HB, r);
+        bw::tmem_ld_wait();
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+          const int s = g / NG;                                // the receiver; its place for this part: parts in order, its own left out
+          if (s == rank) continue;
+          const int slot = rank < s ? rank : rank - 1;
+          const uint32_t dst = bw::cluster_addr(mine + (uint32_t)((slot * 2 * W + b * W + (g % NG) * 8) * BM * 4), s);
+          const uint32_t bar = bw::cluster_addr(received, s);
+          bw::st_cluster_v4(dst, r + g * 8, bar);
+          bw::st_cluster_v4(dst + BM * 16, r + g * 8 + 4, bar);
+        }
       }
     }
-    bw::cluster_sync();                                        // everything has been received; nobody writes here any more
+    __syncwarp();
+    bw::cluster_arrive();
   }
-  if (warp >= 2 && *abort_flag == 0) {
-    const int row = m0 + row_in;
-    const bool row_ok = row < pr.M;
+  if (warp >= 2 && ok) {
+    float f[2][NG][8];
+#pragma unroll
+    for (int b = 0; b < 2; b++)
+#pragma unroll
+      for (int g = 0; g < NG; g++) bw::tmem_ld8(taddr + b * HB + rank * W + g * 8, reinterpret_cast<uint32_t*>(f[b][g]));
+    bw::tmem_ld_wait();
+    if constexpr (KS > 1) {
+      if (!bw::mbar_wait(received, 0, abort_flag)) { ok = false; give_up(abort_flag, 5u); }
+      bw::fence_cluster();
+      const float4* in = reinterpret_cast<const float4*>(smem + C::OFF_RECV) + row_in;
+#pragma unroll
+      for (int b = 0; b < 2; b++)
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+          float own[8], sum[8];
+#pragma unroll
+          for (int i = 0; i < 8; i++) { own[i] = f[b][g][i]; sum[i] = 0.f; }
+#pragma unroll
+          for (int s = 0; s < KS; s++) {                       // in the order of the parts
+            const int slot = s < rank ? s : s - 1;
+            const float4* q = in + (size_t)((s == rank ? 0 : slot) * 2 * W + b * W + g * 8) / 4 * BM;
+            const float4 x = q[0], y = q[BM];
+            const float part[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+            for (int i = 0; i < 8; i++) sum[i] += s == rank ? own[i] : part[i];
+          }
+#pragma unroll
+          for (int i = 0; i < 8; i++) f[b][g][i] = sum[i];
+        }
+    }
     const int n_end = pr.epi == 1 ? pr.half : pr.N;
-    const int pos = pr.epi == 4 && row_ok ? rope_position(gp.rope, row) : 0;
-    for (int c = 0; c < w; c += 8) {
-      float f[2][8];
+    if (row_ok && ok) {
 #pragma unroll
-      for (int b = 0; b < 2; b++) {
-        uint32_t r[8];
-        bw::tmem_ld8(taddr + b * HB + rank * w + c, r);
-        bw::tmem_ld_wait();
-        if (ks == 1) {
-#pragma unroll
-          for (int i = 0; i < 8; i++) f[b][i] = __uint_as_float(r[i]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; i++) f[b][i] = 0.f;
-          for (int s = 0; s < ks; s++) {                       // in the order of the parts
-            if (s == rank) {
-#pragma unroll
-              for (int i = 0; i < 8; i++) f[b][i] += __uint_as_float(r[i]);
-            } else {
-              const float4* q = reinterpret_cast<const float4*>(smem + (size_t)(s * 2 * w + b * w + c) * BM * 4) + row_in;
-              const float4 x = q[0], y = q[BM];
-              f[b][0] += x.x; f[b][1] += x.y; f[b][2] += x.z; f[b][3] += x.w;
-              f[b][4] += y.x; f[b][5] += y.y; f[b][6] += y.z; f[b][7] += y.w;
+      for (int g = 0; g < NG; g++) {
+        const int cc = rank * W + g * 8;                       // column inside a block
+        if (pr.epi == 1) {
+          // silu(g) * u is computed from the ROUNDED values (what a separate pass over the stored matrix would see)
+          const int col = n0 + cc;
+          if (col < n_end) {
+            const uint4 pg = pack8(f[0][g]), pu = pack8(f[1][g]);
+            if (pr.C) {
+              bf16* grow = pr.C + (size_t)row * pr.ldc + col;
+              *reinterpret_cast<uint4*>(grow) = pg;
+              *reinterpret_cast<uint4*>(grow + pr.half) = pu;
             }
+            float gt[8], u[8], h[8];
+            unpack8(pg, gt);
+            unpack8(pu, u);
+#pragma unroll
+            for (int i = 0; i < 8; i++) h[i] = gt[i] / (1.f + __expf(-gt[i])) * u[i];
+            *reinterpret_cast<uint4*>(pr.C2 + (size_t)row * pr.ldc2 + col) = pack8(h);
           }
+          continue;
         }
-      }
-      const int cc = rank * w + c;                             // column inside a block
-      if (!row_ok) continue;
-      if (pr.epi == 1) {
-        // silu(g) * u is computed from the ROUNDED values (what a separate pass over the stored matrix would see)
-        const int col = n0 + cc;
-        if (col < n_end) {
-          const uint4 pg = pack8(f[0]), pu = pack8(f[1]);
-          if (pr.C) {
-            bf16* grow = pr.C + (size_t)row * pr.ldc + col;
-            *reinterpret_cast<uint4*>(grow) = pg;
-            *reinterpret_cast<uint4*>(grow + pr.half) = pu;
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+          const int col = (b ? n1 : n0) + cc;
+          if (col >= n_end) continue;
+          bf16* dst = pr.C + (size_t)row * pr.ldc + col;
+          if (pr.epi == 2) {
+            const bf16* gu = pr.C2 + (size_t)row * pr.ldc2 + col;
+            float d[8], gt[8], u[8], dg[8], du[8];
+            unpack8(*reinterpret_cast<const uint4*>(gu), gt);
+            unpack8(*reinterpret_cast<const uint4*>(gu + pr.half), u);
+            unpack8(pack8(f[b][g]), d);                        // the value a stored bf16 dh would have had
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+              const float sig = 1.f / (1.f + __expf(-gt[i]));
+              dg[i] = d[i] * u[i] * sig * (1.f + gt[i] * (1.f - sig));
+              du[i] = d[i] * gt[i] * sig;
+            }
+            *reinterpret_cast<uint4*>(dst) = pack8(dg);
+            *reinterpret_cast<uint4*>(dst + pr.half) = pack8(du);
+          } else {
+            if (pr.accumulate) {
+              float o[8];
+              unpack8(*reinterpret_cast<const uint4*>(dst), o);
+#pragma unroll
+              for (int i = 0; i < 8; i++) f[b][g][i] += o[i];
+            } else if (pr.epi == 4 && col < gp.rope.cols) {
+              unpack8(pack8(f[b][g]), f[b][g]);                // the values a stored C would have
+              rope_rotate8(rot[b][g], f[b][g]);
+            }
+            *reinterpret_cast<uint4*>(dst) = pack8(f[b][g]);
           }
-          float g[8], u[8], h[8];
-          unpack8(pg, g);
-          unpack8(pu, u);
-#pragma unroll
-          for (int i = 0; i < 8; i++) h[i] = g[i] / (1.f + __expf(-g[i])) * u[i];
-          *reinterpret_cast<uint4*>(pr.C2 + (size_t)row * pr.ldc2 + col) = pack8(h);
-        }
-        continue;
-      }
-#pragma unroll
-      for (int b = 0; b < 2; b++) {
-        const int col = (b ? n1 : n0) + cc;
-        if (col >= n_end) continue;
-        bf16* dst = pr.C + (size_t)row * pr.ldc + col;
-        if (pr.epi == 2) {
-          const bf16* gu = pr.C2 + (size_t)row * pr.ldc2 + col;
-          float d[8], g[8], u[8], dg[8], du[8];
-          unpack8(*reinterpret_cast<const uint4*>(gu), g);
-          unpack8(*reinterpret_cast<const uint4*>(gu + pr.half), u);
-          unpack8(pack8(f[b]), d);                             // the value a stored bf16 dh would have had
-#pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const float sig = 1.f / (1.f + __expf(-g[i]));
-            dg[i] = d[i] * u[i] * sig * (1.f + g[i] * (1.f - sig));
-            du[i] = d[i] * g[i] * sig;
-          }
-          *reinterpret_cast<uint4*>(dst) = pack8(dg);
-          *reinterpret_cast<uint4*>(dst + pr.half) = pack8(du);
-        } else {
-          if (pr.accumulate) {
-            float o[8];
-            unpack8(*reinterpret_cast<const uint4*>(dst), o);
-#pragma unroll
-            for (int i = 0; i < 8; i++) f[b][i] += o[i];
-          } else if (pr.epi == 4 && col < gp.rope.cols) {
-            unpack8(pack8(f[b]), f[b]);                        // the values a stored C would have
-            rope_rotate8(gp.rope, pos, col, f[b]);
-          }
-          *reinterpret_cast<uint4*>(dst) = pack8(f[b]);
         }
       }
     }
@@ -305,6 +344,20 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
     bw::fence_after();
     bw::tmem_dealloc(tmem_base, BN);
   }
+  __syncwarp();
+  if constexpr (KS > 1) bw::cluster_wait();                    // nobody sends to this CTA any more
+}
+
+template <int KS>
+int launch(const Params& gp, long long tiles, cudaStream_t s) {
+  static bool attr[64] = {false};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return LB_ERR_LAUNCH;
+  if (!attr[dev]) {
+    cudaFuncSetAttribute(gemm_split_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<KS>::SMEM_BYTES);
+    attr[dev] = true;
+  }
+  return lb_launch_cluster(true, KS, gemm_split_kernel<KS>, dim3((unsigned)(tiles * KS)), NUM_THREADS, Cfg<KS>::SMEM_BYTES, s, gp);
 }
 
 long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
@@ -336,7 +389,6 @@ int gemm_split_rope(int n, const void* const* A, const void* const* B, void* con
   Params gp;
   gp.rope = rope ? *rope : RopeArgs{nullptr, nullptr, nullptr, 1, 64, 0};
   gp.np = n;
-  gp.ks = ks;
   long long tiles = 0;
   for (int i = 0; i < n; i++) {
     if (M[i] <= 0 || N[i] <= 0 || K[i] <= 0) return LB_ERR_SHAPE;
@@ -370,14 +422,7 @@ int gemm_split_rope(int n, const void* const* A, const void* const* B, void* con
     tiles += p.tiles_m * (e == 1 ? ceil_div(half[i], HB) : ceil_div(N[i], BN));
     if (tiles * ks > (1 << 30)) return LB_ERR_SHAPE;
   }
-  static bool attr[64] = {false};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return LB_ERR_LAUNCH;
-  if (!attr[dev]) {
-    cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    attr[dev] = true;
-  }
-  return lb_launch_cluster(true, ks, gemm_split_kernel, dim3((unsigned)(tiles * ks)), NUM_THREADS, SMEM_BYTES, (cudaStream_t)stream, gp);
+  return ks == 1 ? launch<1>(gp, tiles, (cudaStream_t)stream) : ks == 2 ? launch<2>(gp, tiles, (cudaStream_t)stream) : launch<4>(gp, tiles, (cudaStream_t)stream);
 }
 
 // Parts of K (1, 2 or 4) with which this form is modelled to beat the list form of gemm_grouped.cu, or 0.  list_time: the latter's modelled

@@ -13,17 +13,19 @@ __device__ __forceinline__ int rope_position(const RopeArgs& r, int row) {
   const int s = row % r.S;
   return r.positions ? r.positions[s] : s;
 }
-// 8 columns of C (from `col`, a multiple of 8) of a row at that position
-__device__ __forceinline__ void rope_rotate8(const RopeArgs& r, int pos, int col, float* f) {
+// Cosines and sines (4 and 4) of 8 columns of C, from `col` (a multiple of 8), of a row at that position, and the rotation
+__device__ __forceinline__ void rope_load8(const RopeArgs& r, int pos, int col, float* cs) {
   const int at = pos * (r.d >> 1) + ((col % r.d) >> 1);
-  const float4 c = *reinterpret_cast<const float4*>(r.cos + at), sn = *reinterpret_cast<const float4*>(r.sin + at);
-  float o[8];
-  o[0] = f[0] * c.x - f[1] * sn.x; o[1] = f[0] * sn.x + f[1] * c.x;
-  o[2] = f[2] * c.y - f[3] * sn.y; o[3] = f[2] * sn.y + f[3] * c.y;
-  o[4] = f[4] * c.z - f[5] * sn.z; o[5] = f[4] * sn.z + f[5] * c.z;
-  o[6] = f[6] * c.w - f[7] * sn.w; o[7] = f[6] * sn.w + f[7] * c.w;
+  *reinterpret_cast<float4*>(cs) = *reinterpret_cast<const float4*>(r.cos + at);
+  *reinterpret_cast<float4*>(cs + 4) = *reinterpret_cast<const float4*>(r.sin + at);
+}
+__device__ __forceinline__ void rope_rotate8(const float* cs, float* f) {
 #pragma unroll
-  for (int i = 0; i < 8; i++) f[i] = o[i];
+  for (int i = 0; i < 4; i++) {
+    const float a = f[2 * i], b = f[2 * i + 1];
+    f[2 * i] = a * cs[i] - b * cs[4 + i];
+    f[2 * i + 1] = a * cs[4 + i] + b * cs[i];
+  }
 }
 
 extern "C" int lb_gemm_split(int n, const void* const* A, const void* const* B, void* const* C, const int* M, const int* N, const int* K,

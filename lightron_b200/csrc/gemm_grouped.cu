@@ -11,7 +11,7 @@
 // (tcgen05 cta_group::2) with tiles of 256x256: Cfg has the two forms, choose_cg the choice.
 //
 // The main loop is the one of gemm_tcgen05.cu: TMA (128-byte swizzle, no multicast) -> mbarrier ring
-// of 4 (CTA) or 6 (pair) stages -> tcgen05.mma 128x256x16 / 256x256x16 -> two 256-column TMEM accumulators
+// of 4 (CTA) or 5 to 6 (pair) stages -> tcgen05.mma 128x256x16 / 256x256x16 -> two 256-column TMEM accumulators
 // per CTA -> tcgen05.ld epilogue overlapped with the next tile.  `accumulate` adds the old contents of C in
 // the epilogue (gradient accumulation over micro-batches without a separate add).
 // The ragged kernel (lb_gemm_ragged, lb_gemm_ragged_wgrad) takes its tiles from device memory.
@@ -40,16 +40,21 @@ constexpr int STG_BYTES = 32 * 128;      // 64 columns of the 32 rows of an epil
 // CG CTAs work on one tile: 1 = a CTA per 128x256 tile, 2 = a pair (tcgen05 cta_group::2) per 256x256 tile, in which
 // each CTA loads its 128 rows of A and half of B.  Per CTA a stage then holds 16 + 16 instead of 16 + 32 KB, and the tensor
 // pipe, whose operand reads from shared memory are what limits and heats it, reads a third less.
-template <int CG>
+// EW epilogue warps, each with a quarter of the accumulator's rows and all or half of its columns: four, or eight for launches with the SwiGLU
+// backward, whose arithmetic is more than a warp per scheduler gets done in a main loop of K = 2048 (the others lose by eight: gate | up of 16384 x 2048 ->
+// 5632 487 / 495 us, its gradients 1033 / 1060, those with the SwiGLU backward 606 / 545).
+template <int CG, int EW>
 struct Cfg {
   static constexpr int B_BYTES = BN / CG * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = CG == 2 ? 6 : 4;
-  static constexpr int OFF_STG = STAGES * STAGE_BYTES;              // two buffers of every epilogue warp
-  static constexpr int OFF_BAR = OFF_STG + 8 * STG_BYTES;
+  static constexpr int STAGES = CG == 1 ? 4 : EW == 4 ? 6 : 5;
+  static constexpr int NBUF = CG == 1 && EW == 8 ? 1 : 2;           // staging buffers of an epilogue warp
+  static constexpr int OFF_STG = STAGES * STAGE_BYTES;
+  static constexpr int OFF_BAR = OFF_STG + EW * NBUF * STG_BYTES;
   static constexpr int SMEM_BYTES = OFF_BAR + 1024 + 256;
+  static constexpr int NUM_THREADS = 64 + 32 * EW;
+  static_assert(SMEM_BYTES + 256 <= 232448, "shared memory of a CTA");
 };
-constexpr int NUM_THREADS = 192;
 constexpr int GROUP_M = 8;
 constexpr int MAX_PROBLEMS = 8;
 
@@ -64,6 +69,8 @@ constexpr int MAX_PROBLEMS = 8;
 struct Problem {
   const bf16* old;      // what the epilogue reads: C when accumulate, C2 (g | u) with epi 2
   long long ld_old;
+  bf16* C;
+  long long ldc;
   int M, N, K;
   int a_mn, b_mn, accumulate;
   int tiles_m, tiles_n, num_kb;
@@ -75,7 +82,7 @@ template <int NP>
 struct GroupedParams {
   CUtensorMap ta[NP];
   CUtensorMap tb[NP];
-  CUtensorMap tc[NP][3];      // where the epilogue stores: C; C's gate columns, its up columns, C2; dg, du
+  CUtensorMap tc[NP][3];      // where the epilogue stores with TMA: C; C's gate columns, its up columns, C2 (epi 1)
   Problem prob[NP];
   RopeArgs rope;
   const int* offsets;   // [grid + 1] first item of every CTA
@@ -109,11 +116,10 @@ __device__ __forceinline__ void load_box(uint32_t dst, const CUtensorMap* map, i
   if constexpr (CG == 2) bw::tma_load_2d_pair(dst, map, x, y, bar);
   else bw::tma_load_2d(dst, map, x, y, bar);
 }
-template <int CG, bool A_MN, bool B_MN>
+template <typename C, int CG, bool A_MN, bool B_MN>
 __device__ __forceinline__ bool produce_tile(const CUtensorMap* ta, const CUtensorMap* tb, int m0, int n0, int num_kb,
                                              uint32_t smem_base, uint32_t bar_base, int& stage, uint32_t& phase,
                                              volatile int* abort_flag, bool leader, int k_base = 0, int b_split = 0) {
-  using C = Cfg<CG>;
   for (int kb = 0; kb < num_kb; kb++) {
     if (!bw::mbar_wait(bar_base + 8u * (C::STAGES + stage), phase ^ 1u, abort_flag)) return false;
     uint32_t fb = bar_base + 8u * stage;
@@ -141,10 +147,9 @@ __device__ __forceinline__ bool produce_tile(const CUtensorMap* ta, const CUtens
   return true;
 }
 
-template <int CG, bool A_MN, bool B_MN>
+template <typename C, int CG, bool A_MN, bool B_MN>
 __device__ __forceinline__ bool mma_tile(uint32_t d_tmem, int num_kb, uint32_t smem_base, uint32_t bar_base, int& stage,
                                          uint32_t& phase, volatile int* abort_flag) {
-  using C = Cfg<CG>;
   constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) |
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM * CG >> 4) << 24);
   constexpr uint32_t a_lbo = A_MN ? 8192u : 16u, b_lbo = B_MN ? 8192u : 16u;
@@ -169,50 +174,119 @@ __device__ __forceinline__ bool mma_tile(uint32_t d_tmem, int num_kb, uint32_t s
   return true;
 }
 
-// ---- epilogue of a warp: 32 rows x 256 columns of an accumulator ------------------------------------
-// 64 columns at a time pass through one of the warp's two 4 KB staging buffers (swizzled, a row per lane) and leave by a TMA store, which ends at
-// the matrix's last row and column.  What is read (the old C, or g | u) comes in by loads that cover a row's 64 columns with eight
-// lanes, a step ahead of its use, and turns in the same buffers.  A row per lane read and written straight from memory is 32 lines for every
-// 16 bytes per lane, and kept the load/store unit busy for as long as a main loop of K = 2048 takes (epi 2).  That form / this, us, feed-forward of 16384
-// x 2048 -> 5632: gate | up 562 / 487, down 250 / 245, its gradients with epi 2 696 / 564, gate | up's 1082 / 1055; of 1000 x 768 -> 2048: 12.4 / 11.6,
-// 22.1 / 17.7 (epi 2), 28.9 / 26.7.
+// ---- epilogue of a warp: 32 rows x 256 or 128 columns of an accumulator ------------------------------------
+// Columns pass through one of the warp's 4 KB staging buffers (swizzled, a row per lane), 64 at a time.  What is only written leaves by a TMA store, which ends at
+// the matrix's last row and column.  Where the epilogue also reads (the old C, or g | u), steps of 32 columns: four lanes read and write a row's part, the
+// loads a step ahead of their use, and rows turn into lanes and back in the buffer.  A row per lane read and written straight from memory is 32
+// lines for every 16 bytes per lane, and kept the load/store unit busy for as long as a main loop of K = 2048 takes (epi 2).  The same
+// launches with that form / this, us: 562 / 487, 696 / 545, 1082 / 1033, and 250 / 245 for the down projection; of 1000 x 768 -> 2048: 12.4 / 11.2, 22.1 / 16.6
+// (SwiGLU backward), 28.9 / 26.5.  (With TMA stores, whose fence waits for loads in flight, the SwiGLU backward took 579; with
+// stores from whole lines of the buffer in their place the forward 505.)
 struct Out {
   const CUtensorMap* map;
-  const bf16* old;
+  const bf16* old;     // EPI 2, 3: what is read and where the result goes
   long long ld_old;
+  bf16* out;
+  long long ld_out;
   int row0, rows;      // the warp's first row, rows of the matrix
-  int c0, cols;        // first column, columns (of one half, with an activation)
+  int c0, cols;        // the warp's first column, columns (of one half, with an activation)
   bool keep;           // EPI 1: g and u are stored
   const RopeArgs* rope;
 };
 
-// EPI as in Problem; 3: C = acc + C.  `turn`: which buffer is next, kept over the tiles (the store before the last one has used it).  ready() waits
-// for the accumulator, release() gives its columns back.
-template <int EPI, typename Ready, typename Release>
+// EPI as in Problem; 3: C = acc + C.  taddr: the warp's first column (EPI 1: of g).  ready() waits for the accumulator, release() gives its columns back.
+// `turn`: the buffer that is next, kept over the tiles.
+template <int EPI, int NBUF, int EW, typename Ready, typename Release>
 __device__ __forceinline__ bool store_tile(const Out& o, uint32_t taddr, uint8_t* stg, int& turn, int lane, Ready ready, Release release) {
-  constexpr bool READS = EPI == 2 || EPI == 3;
-  constexpr int NC = EPI == 1 ? BN / 128 : BN / 64;                   // steps of 64 columns
-  uint4 old[READS ? 8 : 1], old2[EPI == 2 ? 8 : 1];
-  const int lr = lane >> 3, lc = (lane & 7) * 8;                      // loads: row (of every four), column
-  auto fetch = [&](int c) {
+  constexpr int COLS = BN * 4 / EW;                                   // of the warp (EPI 1: half of them of g, half of u)
+  if (o.c0 >= o.cols) {
+    if (!ready()) return false;
+    release();
+    return true;
+  }
+  if constexpr (EPI == 2 || EPI == 3) {
+    const int lr = lane >> 2, lc = (lane & 3) * 8;                    // memory accesses: row (of every eight), column
+    uint8_t* const stg2 = stg + STG_BYTES / 2;
+    // 16-byte piece c of row r: rows are 64 B apart, no bank twice for eight rows' one piece or two rows' four
+    auto at = [&](uint8_t* buf, int r, int c) { return reinterpret_cast<uint4*>(buf + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); };
+    uint4 old[4], old2[EPI == 2 ? 4 : 1];
+    auto inside = [&](int i, int c) { return o.row0 + 8 * i + lr < o.rows && o.c0 + c * 32 + lc < o.cols; };
+    auto fetch = [&](int c) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const int row = o.row0 + 4 * i + lr, col = o.c0 + c * 64 + lc;
-      const bool in = row < o.rows && col < o.cols;
-      const bf16* at = o.old + (size_t)row * o.ld_old + col;
-      old[i] = in ? *reinterpret_cast<const uint4*>(at) : make_uint4(0, 0, 0, 0);
-      if constexpr (EPI == 2) old2[i] = in ? *reinterpret_cast<const uint4*>(at + o.cols) : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < 4; i++) {
+        const bf16* from = o.old + (size_t)(o.row0 + 8 * i + lr) * o.ld_old + o.c0 + c * 32 + lc;
+        const bool in = inside(i, c);
+        old[i] = in ? *reinterpret_cast<const uint4*>(from) : make_uint4(0, 0, 0, 0);
+        if constexpr (EPI == 2) old2[i] = in ? *reinterpret_cast<const uint4*>(from + o.cols) : make_uint4(0, 0, 0, 0);
+      }
+    };
+    fetch(0);
+    if (!ready()) return false;
+    if (lane == 0) bw::bulk_wait_read_but<0>();                       // (stores of another kind of tile)
+    __syncwarp();
+#pragma unroll 1
+    for (int c = 0; c < COLS / 32; c++) {
+      const bool last = c == COLS / 32 - 1 || o.c0 + (c + 1) * 32 >= o.cols;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        *at(stg, 8 * i + lr, lane & 3) = old[i];
+        if constexpr (EPI == 2) *at(stg2, 8 * i + lr, lane & 3) = old2[i];
+      }
+      if (!last) fetch(c + 1);
+      uint32_t r[32];
+      bw::tmem_ld32(taddr + c * 32, r);
+      bw::tmem_ld_wait();
+      if (last) release();
+      __syncwarp();
+#pragma unroll
+      for (int g = 0; g < 4; g++) {
+        float f[8], fg[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[g * 8 + i]);
+        unpack8(*at(stg, lane, g), fg);
+        if constexpr (EPI == 2) {
+          const bw::f32x2 one = bw::pack2(1.f, 1.f), minus = bw::pack2(-1.f, -1.f);
+          float fu[8];
+          unpack8(pack8(f), f);                                       // the value a stored bf16 dh would have had
+          unpack8(*at(stg2, lane, g), fu);
+#pragma unroll
+          for (int i = 0; i < 8; i += 2) {
+            const bw::f32x2 d = bw::pack2(f[i], f[i + 1]), gg = bw::pack2(fg[i], fg[i + 1]), uu = bw::pack2(fu[i], fu[i + 1]);
+            float a, b;
+            bw::unpack2(bw::add2(one, bw::pack2(__expf(-fg[i]), __expf(-fg[i + 1]))), a, b);
+            const bw::f32x2 sig = bw::pack2(1.f / a, 1.f / b);
+            const bw::f32x2 slope = bw::fma2(gg, bw::fma2(sig, minus, one), one);
+            bw::unpack2(bw::mul2(bw::mul2(bw::mul2(d, uu), sig), slope), f[i], f[i + 1]);       // dg
+            bw::unpack2(bw::mul2(bw::mul2(d, gg), sig), fu[i], fu[i + 1]);                      // du
+          }
+          *at(stg2, lane, g) = pack8(fu);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; i++) f[i] += fg[i];
+        }
+        *at(stg, lane, g) = pack8(f);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        bf16* to = o.out + (size_t)(o.row0 + 8 * i + lr) * o.ld_out + o.c0 + c * 32 + lc;
+        if (inside(i, c)) {
+          *reinterpret_cast<uint4*>(to) = *at(stg, 8 * i + lr, lane & 3);
+          if constexpr (EPI == 2) *reinterpret_cast<uint4*>(to + o.cols) = *at(stg2, 8 * i + lr, lane & 3);
+        }
+      }
+      __syncwarp();
+      if (last) break;
     }
-  };
-  // a buffer to fill: the store before the last one has read it
-  auto next = [&]() -> uint8_t* {
-    if (lane == 0) bw::bulk_wait_read_but<1>();
+    return true;
+  }
+  auto store = [&](const uint4* rows8, const CUtensorMap* map, int col) {      // a lane's row of 64 columns
+    if (lane == 0) bw::bulk_wait_read_but<NBUF - 1>();                // the last store from this buffer has read it
     __syncwarp();
     uint8_t* buf = stg + turn * STG_BYTES;
-    turn ^= 1;
-    return buf;
-  };
-  auto store = [&](const uint8_t* buf, const CUtensorMap* map, int col) {
+    if (NBUF > 1) turn ^= 1;
+#pragma unroll
+    for (int g = 0; g < 8; g++) *reinterpret_cast<uint4*>(buf + bw::sw128_off(lane, g)) = rows8[g];
     bw::fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {
@@ -220,132 +294,78 @@ __device__ __forceinline__ bool store_tile(const Out& o, uint32_t taddr, uint8_t
       bw::bulk_commit();
     }
   };
-  auto at = [&](uint8_t* buf, int g) { return reinterpret_cast<uint4*>(buf + bw::sw128_off(lane, g)); };
-
-  if constexpr (READS) fetch(0);
   if (!ready()) return false;
   if constexpr (EPI == 1) {
     // g and u are stored, and silu(g) * u computed from the ROUNDED values (what a separate pass over the stored
     // matrix would see, and what the backward recomputes from)
 #pragma unroll 1
-    for (int c = 0; c < NC; c++) {
+    for (int c = 0; c < COLS / 128; c++) {
       const int col = o.c0 + c * 64;
-      uint32_t r[64];
+      const bool last = c == COLS / 128 - 1 || col + 64 >= o.cols;
       uint4 pg[8], pu[8];
-      auto take = [&](uint32_t from, uint4* packed) {
-        bw::tmem_ld32(from, r);
-        bw::tmem_ld32(from + 32, r + 32);
+      auto take32 = [&](uint32_t from, uint4* p) {
+        float f[32];
+        bw::tmem_ld32(from, reinterpret_cast<uint32_t*>(f));
         bw::tmem_ld_wait();
 #pragma unroll
-        for (int g = 0; g < 8; g++) packed[g] = pack8(reinterpret_cast<const float*>(r) + g * 8);
+        for (int g = 0; g < 4; g++) p[g] = pack8(f + g * 8);
       };
-      take(taddr + c * 64, pg);
-      take(taddr + BN / 2 + c * 64, pu);
-      if (c == NC - 1 || col + 64 >= o.cols) release();
-      uint8_t* buf;
+      take32(taddr + c * 64, pg);
+      take32(taddr + c * 64 + 32, pg + 4);
+      take32(taddr + BN / 2 + c * 64, pu);
+      take32(taddr + BN / 2 + c * 64 + 32, pu + 4);
+      if (last) release();
       if (o.keep) {
-        buf = next();
-#pragma unroll
-        for (int g = 0; g < 8; g++) *at(buf, g) = pg[g];
-        store(buf, o.map, col);
-        buf = next();
-#pragma unroll
-        for (int g = 0; g < 8; g++) *at(buf, g) = pu[g];
-        store(buf, o.map + 1, col);
+        store(pg, o.map, col);
+        store(pu, o.map + 1, col);
       }
 #pragma unroll
       for (int g = 0; g < 8; g++) {
-        float fg[8], fu[8], h[8];
+        float fg[8], fu[8];
         unpack8(pg[g], fg);
         unpack8(pu[g], fu);
 #pragma unroll
-        for (int i = 0; i < 8; i++) h[i] = fg[i] / (1.f + __expf(-fg[i])) * fu[i];
-        pg[g] = pack8(h);
+        for (int i = 0; i < 8; i++) fg[i] = fg[i] / (1.f + __expf(-fg[i])) * fu[i];
+        pg[g] = pack8(fg);
       }
-      buf = next();
-#pragma unroll
-      for (int g = 0; g < 8; g++) *at(buf, g) = pg[g];
-      store(buf, o.map + 2, col);
-      if (col + 64 >= o.cols) break;
+      store(pg, o.map + 2, col);
+      if (last) break;
     }
   } else {
     const int pos = EPI == 4 && o.row0 + lane < o.rows ? rope_position(*o.rope, o.row0 + lane) : 0;
 #pragma unroll 1
-    for (int c = 0; c < NC; c++) {
+    for (int c = 0; c < COLS / 64; c++) {
       const int col = o.c0 + c * 64;
-      const bool last = c == NC - 1 || col + 64 >= o.cols;
-      uint8_t *buf, *buf2 = nullptr;
-      if constexpr (EPI == 2) {                                       // both buffers, the first of which is stored first
-        if (lane == 0) bw::bulk_wait_read_but<0>();
-        __syncwarp();
-        buf = stg;
-        buf2 = stg + STG_BYTES;
-        turn = 0;
-      } else {
-        buf = next();
-      }
-      if constexpr (READS) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const uint32_t to = bw::sw128_off(4 * i + lr, lane & 7);
-          *reinterpret_cast<uint4*>(buf + to) = old[i];
-          if constexpr (EPI == 2) *reinterpret_cast<uint4*>(buf2 + to) = old2[i];
-        }
-        if (!last) fetch(c + 1);
-      }
-      uint32_t r[64];
-      bw::tmem_ld32(taddr + c * 64, r);
-      bw::tmem_ld32(taddr + c * 64 + 32, r + 32);
+      const bool last = c == COLS / 64 - 1 || col + 64 >= o.cols;
+      float f[64];
+      uint4 p[8];
+      bw::tmem_ld32(taddr + c * 64, reinterpret_cast<uint32_t*>(f));
+      bw::tmem_ld32(taddr + c * 64 + 32, reinterpret_cast<uint32_t*>(f) + 32);
       bw::tmem_ld_wait();
       if (last) release();
-      if constexpr (READS) __syncwarp();
 #pragma unroll
       for (int g = 0; g < 8; g++) {
-        float f[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) f[i] = __uint_as_float(r[g * 8 + i]);
-        if constexpr (EPI == 2) {
-          float fg[8], fu[8], dg[8], du[8];
-          unpack8(pack8(f), f);                                       // the value a stored bf16 dh would have had
-          unpack8(*at(buf, g), fg);
-          unpack8(*at(buf2, g), fu);
-#pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const float sig = 1.f / (1.f + __expf(-fg[i]));
-            dg[i] = f[i] * fu[i] * sig * (1.f + fg[i] * (1.f - sig));
-            du[i] = f[i] * fg[i] * sig;
+        p[g] = pack8(f + g * 8);
+        if constexpr (EPI == 4) {
+          if (col + g * 8 < o.rope->cols) {
+            float v[8], cs[8];
+            unpack8(p[g], v);                                         // the values a stored C would have
+            rope_load8(*o.rope, pos, col + g * 8, cs);
+            rope_rotate8(cs, v);
+            p[g] = pack8(v);
           }
-          *at(buf, g) = pack8(dg);
-          *at(buf2, g) = pack8(du);
-        } else {
-          if constexpr (EPI == 3) {
-            float e[8];
-            unpack8(*at(buf, g), e);
-#pragma unroll
-            for (int i = 0; i < 8; i++) f[i] += e[i];
-          }
-          if constexpr (EPI == 4) {
-            if (col + g * 8 < o.rope->cols) {
-              float cs[8];
-              unpack8(pack8(f), f);                                   // the values a stored C would have
-              rope_load8(*o.rope, pos, col + g * 8, cs);
-              rope_rotate8(cs, f);
-            }
-          }
-          *at(buf, g) = pack8(f);
         }
       }
-      store(buf, o.map, col);
-      if constexpr (EPI == 2) store(buf2, o.map + 1, col);
+      store(p, o.map, col);
       if (last) break;
     }
   }
   return true;
 }
 
-template <int CG, int NP>
-__global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __grid_constant__ GroupedParams<NP> gp) {
-  using CF = Cfg<CG>;
+template <int CG, int EW, int NP>
+__global__ void __launch_bounds__(Cfg<CG, EW>::NUM_THREADS, 1) gemm_grouped_kernel(const __grid_constant__ GroupedParams<NP> gp) {
+  using CF = Cfg<CG, EW>;
   constexpr int STAGES = CF::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -374,7 +394,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
     }
     for (int a = 0; a < 2; a++) {
       bw::mbar_init(tfull_bar(a), 1);
-      bw::mbar_init(tempty_bar(a), 4 * CG);
+      bw::mbar_init(tempty_bar(a), EW * CG);
     }
     bw::mbar_init_fence();
   }
@@ -413,10 +433,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
         const int n0 = split ? tn * (BN / 2) + (CG == 2 ? rank * split : 0) : tn * BN + rank * (BN / 2);
         const int num_kb = gp.prob[pi].num_kb;
         switch (gp.prob[pi].a_mn * 2 + gp.prob[pi].b_mn) {
-          case 0: ok = produce_tile<CG, false, false>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, 0, split); break;
-          case 1: ok = produce_tile<CG, false, true>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0); break;
-          case 2: ok = produce_tile<CG, true, false>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, 0, split); break;
-          default: ok = produce_tile<CG, true, true>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0); break;
+          case 0: ok = produce_tile<CF, CG, false, false>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, 0, split); break;
+          case 1: ok = produce_tile<CF, CG, false, true>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0); break;
+          case 2: ok = produce_tile<CF, CG, true, false>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, 0, split); break;
+          default: ok = produce_tile<CF, CG, true, true>(ta, tb, m0, n0, num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0); break;
         }
         if (!ok) give_up(abort_flag, 1u);
       }
@@ -446,10 +466,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
         bw::fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * BN;
         switch (majors) {
-          case 0: ok = mma_tile<CG, false, false>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
-          case 1: ok = mma_tile<CG, false, true>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
-          case 2: ok = mma_tile<CG, true, false>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
-          default: ok = mma_tile<CG, true, true>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
+          case 0: ok = mma_tile<CF, CG, false, false>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
+          case 1: ok = mma_tile<CF, CG, false, true>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
+          case 2: ok = mma_tile<CF, CG, true, false>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
+          default: ok = mma_tile<CF, CG, true, true>(d_tmem, num_kb, smem_base, bar_base, stage, phase, abort_flag); break;
         }
         if (!ok) give_up(abort_flag, 3u);
         else if constexpr (CG == 2) bw::umma_commit_pair(tfull_bar(acc));          // accumulator complete
@@ -457,9 +477,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
       }
     }
   } else {
-    // ------------------------------ epilogue (4 warps) ------------------------------
-    const int quad = warp & 3;
-    uint8_t* stg = smem + CF::OFF_STG + quad * 2 * STG_BYTES;
+    // ------------------------------ epilogue ------------------------------
+    const int quad = warp & 3, part = (warp - 2) >> 2;
+    uint8_t* stg = smem + CF::OFF_STG + (warp - 2) * CF::NBUF * STG_BYTES;
     int n = 0, turn = 0;
     int next_item = item_begin < item_end ? gp.items[item_begin] : 0;
     for (int it = item_begin; it < item_end; it++, n++) {
@@ -471,8 +491,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
       const Problem& pr = gp.prob[pi];
       const int acc = n & 1;
       const uint32_t acc_phase = (uint32_t)(n >> 1) & 1u;
-      const Out out{gp.tc[pi], pr.old, pr.ld_old, (tm * CG + rank) * BM + quad * 32, pr.M, tn * (pr.epi == 1 ? BN / 2 : BN), pr.epi == 1 || pr.epi == 2 ? pr.half : pr.N, pr.keep != 0, &gp.rope};
-      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * BN;
+      const Out out{gp.tc[pi], pr.old, pr.ld_old, pr.C, pr.ldc, (tm * CG + rank) * BM + quad * 32, pr.M,
+                    tn * (pr.epi == 1 ? BN / 2 : BN) + part * (pr.epi == 1 ? BN / 4 : BN / 2), pr.epi == 1 || pr.epi == 2 ? pr.half : pr.N, pr.keep != 0, &gp.rope};
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN + part * (pr.epi == 1 ? BN / 4 : BN / 2));
       auto ready = [&]() {
         if (!bw::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) return false;
         bw::fence_after();
@@ -488,11 +509,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_grouped_kernel(const __gr
       };
       bool ok;
       switch (pr.epi == 0 && pr.accumulate ? 3 : pr.epi) {
-        case 0: ok = store_tile<0>(out, taddr, stg, turn, lane, ready, release); break;
-        case 1: ok = store_tile<1>(out, taddr, stg, turn, lane, ready, release); break;
-        case 2: ok = store_tile<2>(out, taddr, stg, turn, lane, ready, release); break;
-        case 4: ok = store_tile<4>(out, taddr, stg, turn, lane, ready, release); break;
-        default: ok = store_tile<3>(out, taddr, stg, turn, lane, ready, release); break;
+        case 0: ok = store_tile<0, CF::NBUF, EW>(out, taddr, stg, turn, lane, ready, release); break;
+        case 1: ok = store_tile<1, CF::NBUF, EW>(out, taddr, stg, turn, lane, ready, release); break;
+        case 2:
+          if constexpr (EW == 8) ok = store_tile<2, CF::NBUF, EW>(out, taddr, stg, turn, lane, ready, release);      // (launches with it take eight)
+          else ok = false;
+          break;
+        case 4: ok = store_tile<4, CF::NBUF, EW>(out, taddr, stg, turn, lane, ready, release); break;
+        default: ok = store_tile<3, CF::NBUF, EW>(out, taddr, stg, turn, lane, ready, release); break;
       }
       if (!ok) { give_up(abort_flag, 4u); break; }
     }
@@ -525,7 +549,7 @@ struct RaggedParams {
   CUtensorMap ta;                      // mode 0: [cap, K] K-major;  mode 1: [cap, Nw] as MN-major A
   CUtensorMap tb[MAX_PROBLEMS];        // mode 0: B_e;               mode 1: tb[0] = [cap, Kw] as MN-major B
   CUtensorMap tc[MAX_PROBLEMS];        // mode 0: tc[0..2] as in GroupedParams, of matrices of cap rows;  mode 1: C_e
-  bf16* C[MAX_PROBLEMS];               // mode 1: C_e
+  bf16* C[MAX_PROBLEMS];               // mode 0: C[0];  mode 1: C_e
   long long ldc;
   const bf16* old;                     // mode 0, epi 2: g | u
   long long ld_old;
@@ -571,9 +595,9 @@ __device__ __forceinline__ RaggedTile ragged_tile(int t, const RaggedParams& rp,
   return r;
 }
 
-template <int CG>
-__global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __grid_constant__ RaggedParams rp) {
-  using CF = Cfg<CG>;
+template <int CG, int EW>
+__global__ void __launch_bounds__(Cfg<CG, EW>::NUM_THREADS, 1) gemm_ragged_kernel(const __grid_constant__ RaggedParams rp) {
+  using CF = Cfg<CG, EW>;
   constexpr int STAGES = CF::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -603,7 +627,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
     }
     for (int a = 0; a < 2; a++) {
       bw::mbar_init(tfull_bar(a), 1);
-      bw::mbar_init(tempty_bar(a), 4 * CG);
+      bw::mbar_init(tempty_bar(a), EW * CG);
     }
     bw::mbar_init_fence();
   }
@@ -650,10 +674,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
         // this CTA's first rows of A and of B (see gemm_grouped_kernel)
         const int m0 = rt.m0 + rank * BM, n0 = rt.n0 + (CG == 2 ? rank * (split ? split : BN / 2) : 0);
         if (rp.mode == 0) {
-          if (!rp.b_mn) ok = produce_tile<CG, false, false>(&rp.ta, &rp.tb[rt.e], m0, n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, 0, split);
-          else          ok = produce_tile<CG, false, true>(&rp.ta, &rp.tb[rt.e], m0, n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0);
+          if (!rp.b_mn) ok = produce_tile<CF, CG, false, false>(&rp.ta, &rp.tb[rt.e], m0, n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, 0, split);
+          else          ok = produce_tile<CF, CG, false, true>(&rp.ta, &rp.tb[rt.e], m0, n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0);
         } else {
-          ok = produce_tile<CG, true, true>(&rp.ta, &rp.tb[0], m0, n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, rt.k_base);
+          ok = produce_tile<CF, CG, true, true>(&rp.ta, &rp.tb[0], m0, n0, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag, rank == 0, rt.k_base);
         }
         if (!ok) give_up(abort_flag, 1u);
       }
@@ -681,10 +705,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
         bw::fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * BN;
         if (rp.mode == 0) {
-          if (!rp.b_mn) ok = mma_tile<CG, false, false>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
-          else          ok = mma_tile<CG, false, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
+          if (!rp.b_mn) ok = mma_tile<CF, CG, false, false>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
+          else          ok = mma_tile<CF, CG, false, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
         } else {
-          ok = mma_tile<CG, true, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
+          ok = mma_tile<CF, CG, true, true>(d_tmem, rt.num_kb, smem_base, bar_base, stage, phase, abort_flag);
         }
         if (!ok) give_up(abort_flag, 3u);
         else if constexpr (CG == 2) bw::umma_commit_pair(tfull_bar(acc));
@@ -693,9 +717,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
       }
     }
   } else {
-    // ------------------------------ epilogue (4 warps) ------------------------------
-    const int quad = warp & 3;
-    uint8_t* stg = smem + CF::OFF_STG + quad * 2 * STG_BYTES;
+    // ------------------------------ epilogue ------------------------------
+    const int quad = warp & 3, part = (warp - 2) >> 2;
+    uint8_t* stg = smem + CF::OFF_STG + (warp - 2) * CF::NBUF * STG_BYTES;
     int n = 0, turn = 0;
     for (int t = worker;; t += workers) {
       const RaggedTile rt = ragged_tile<CG>(t, rp, s_off, s_tiles);
@@ -704,7 +728,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
         // an expert without rows: its weight gradient is zero (nothing to add when accumulating)
         const int row = rt.m0 + rank * BM + quad * 32 + lane;
         if (rp.mode == 1 && !rp.accumulate && row < rp.M_w)
-          for (int c = rt.n0; c < rt.n0 + BN && c < rp.N; c += 8)
+          for (int c = rt.n0 + part * (BN / 2); c < rt.n0 + (EW == 4 ? BN : (part + 1) * (BN / 2)) && c < rp.N; c += 8)
             *reinterpret_cast<uint4*>(rp.C[rt.e] + (size_t)row * rp.ldc + c) = make_uint4(0, 0, 0, 0);
         continue;
       }
@@ -712,9 +736,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
       const uint32_t acc_phase = (uint32_t)(n >> 1) & 1u;
       const bool wgrad = rp.mode == 1;
       // (mode 0 writes whole 128-row tiles: padding rows are zeros)
-      const Out out{wgrad ? &rp.tc[rt.e] : rp.tc, wgrad ? rp.C[rt.e] : rp.old, wgrad ? rp.ldc : rp.ld_old, rt.m0 + rank * BM + quad * 32, wgrad ? rp.M_w : s_end[rt.e],
-                    rt.n0, rp.epi ? rp.half : rp.N, true, nullptr};
-      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)acc * BN;
+      const Out out{wgrad ? &rp.tc[rt.e] : rp.tc, wgrad ? rp.C[rt.e] : rp.old, wgrad ? rp.ldc : rp.ld_old, wgrad ? rp.C[rt.e] : rp.C[0], rp.ldc, rt.m0 + rank * BM + quad * 32, wgrad ? rp.M_w : s_end[rt.e],
+                    rt.n0 + part * (rp.epi == 1 ? BN / 4 : BN / 2), rp.epi ? rp.half : rp.N, true, nullptr};
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN + part * (rp.epi == 1 ? BN / 4 : BN / 2));
       auto ready = [&]() {
         if (!bw::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) return false;
         bw::fence_after();
@@ -730,10 +754,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_ragged_kernel(const __gri
       };
       bool ok;
       switch (wgrad && rp.accumulate ? 3 : rp.epi) {
-        case 0: ok = store_tile<0>(out, taddr, stg, turn, lane, ready, release); break;
-        case 1: ok = store_tile<1>(out, taddr, stg, turn, lane, ready, release); break;
-        case 2: ok = store_tile<2>(out, taddr, stg, turn, lane, ready, release); break;
-        default: ok = store_tile<3>(out, taddr, stg, turn, lane, ready, release); break;
+        case 0: ok = store_tile<0, CF::NBUF, EW>(out, taddr, stg, turn, lane, ready, release); break;
+        case 1: ok = store_tile<1, CF::NBUF, EW>(out, taddr, stg, turn, lane, ready, release); break;
+        case 2:
+          if constexpr (EW == 8) ok = store_tile<2, CF::NBUF, EW>(out, taddr, stg, turn, lane, ready, release);      // (launches with it take eight)
+          else ok = false;
+          break;
+        default: ok = store_tile<3, CF::NBUF, EW>(out, taddr, stg, turn, lane, ready, release); break;
       }
       if (!ok) { give_up(abort_flag, 4u); break; }
       n++;
@@ -880,18 +907,33 @@ int build_schedule(Problem* probs, int np, int sms, Schedule* out) {
   return LB_OK;
 }
 
-// Map of the 64-column, 32-row boxes that an epilogue warp stores.
+// Map of the boxes of 32 rows that an epilogue warp stores.
 int out_map(CUtensorMap* m, const bf16* base, int cols, int rows, long long ld) {
   return bw::make_map_bf16(m, base, (uint64_t)cols, (uint64_t)rows, (uint64_t)ld, 64, 32);
 }
 // The maps of a problem's outputs (see GroupedParams::tc).
 int out_maps(CUtensorMap* tc, void* C, void* C2, long long ldc, long long ldc2, int rows, int N, int epi, int half) {
   bf16* c = (bf16*)C;
-  if (epi == 0 || epi == 4) return out_map(tc, c, N, rows, ldc);
+  if (epi == 2) return LB_OK;
+  if (epi != 1) return out_map(tc, c, N, rows, ldc);
   int rc = c ? out_map(tc, c, half, rows, ldc) : LB_OK;
   if (!rc && c) rc = out_map(tc + 1, c + half, half, rows, ldc);
-  if (!rc && epi == 1) rc = out_map(tc + 2, (const bf16*)C2, half, rows, ldc2);
-  return rc;
+  return rc ? rc : out_map(tc + 2, (const bf16*)C2, half, rows, ldc2);
+}
+
+// Launches a form of a kernel on `workers` workers; a pair is a cluster of two CTAs.
+template <typename C, typename P>
+int launch_form(void (*fn)(P), C, int cg, int workers, bool dependent, const P& params, cudaStream_t s) {
+  {
+    std::lock_guard<std::mutex> lock(g_sched_mutex);
+    static std::vector<const void*> ready;      // (of this configuration)
+    const void* f = reinterpret_cast<const void*>(fn);
+    if (std::find(ready.begin(), ready.end(), f) == ready.end()) {
+      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess) return LB_ERR_LAUNCH;
+      ready.push_back(f);
+    }
+  }
+  return lb_launch_cluster(dependent, cg, fn, cg * workers, C::NUM_THREADS, C::SMEM_BYTES, s, params);
 }
 
 struct Operands {
@@ -917,9 +959,11 @@ int launch_grouped(int n, const Problem* probs, const Operands& op, const Schedu
   gp.rope = op.rope ? *op.rope : RopeArgs{nullptr, nullptr, nullptr, 1, 64, 0};
   gp.offsets = sched.d_offsets;
   gp.items = sched.d_items;
-  if (sched.cg == 2)      // a pair is a cluster of two CTAs
-    return lb_launch_cluster(true, 2, gemm_grouped_kernel<2, NP>, 2 * sched.grid, NUM_THREADS, Cfg<2>::SMEM_BYTES, s, gp);
-  return lb_launch(gemm_grouped_kernel<1, NP>, sched.grid, NUM_THREADS, Cfg<1>::SMEM_BYTES, s, gp);
+  const bool eight = std::any_of(probs, probs + n, [](const Problem& p) { return p.epi == 2; });
+  if (sched.cg == 2) return eight ? launch_form(gemm_grouped_kernel<2, 8, NP>, Cfg<2, 8>(), 2, sched.grid, true, gp, s)
+                                  : launch_form(gemm_grouped_kernel<2, 4, NP>, Cfg<2, 4>(), 2, sched.grid, true, gp, s);
+  return eight ? launch_form(gemm_grouped_kernel<1, 8, NP>, Cfg<1, 8>(), 1, sched.grid, true, gp, s)
+               : launch_form(gemm_grouped_kernel<1, 4, NP>, Cfg<1, 4>(), 1, sched.grid, true, gp, s);
 }
 
 }  // namespace
@@ -1020,7 +1064,7 @@ static int run_grouped(int n, const void* const* A, const void* const* B, void* 
     }
     Problem& p = probs[i];
     p.M = M[i]; p.N = N[i]; p.K = K[i]; p.epi = rope ? 4 : e; p.half = e ? half[i] : 0; p.keep = C[i] != nullptr;
-    p.old = (const bf16*)(e == 2 ? C2[i] : C[i]); p.ld_old = e == 2 ? ldc2[i] : ldc[i];
+    p.old = (const bf16*)(e == 2 ? C2[i] : C[i]); p.ld_old = e == 2 ? ldc2[i] : ldc[i]; p.C = (bf16*)C[i]; p.ldc = ldc[i];
     p.a_mn = a_mn[i]; p.b_mn = b_mn[i]; p.accumulate = accumulate ? accumulate[i] : 0;
     key.push_back(M[i]); key.push_back(N[i]); key.push_back(K[i]);
   }
@@ -1028,10 +1072,6 @@ static int run_grouped(int n, const void* const* A, const void* const* B, void* 
     std::lock_guard<std::mutex> lock(g_sched_mutex);
     if (g_sms == 0) {
       cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-      cudaFuncSetAttribute(gemm_grouped_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
-      cudaFuncSetAttribute(gemm_grouped_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
-      cudaFuncSetAttribute(gemm_grouped_kernel<1, MAX_PROBLEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
-      cudaFuncSetAttribute(gemm_grouped_kernel<2, MAX_PROBLEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
     }
   }
   Schedule sched;
@@ -1118,17 +1158,11 @@ int ragged_wgrad_cg(int LE, int cap, int sms) {
   return sms >= 2 && (cap - LE * BM) / LE >= 512 ? 2 : 1;
 }
 int launch_ragged(int cg, bool dependent, const RaggedParams& rp, cudaStream_t s) {
-  {
-    std::lock_guard<std::mutex> lock(g_sched_mutex);
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(gemm_ragged_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<1>::SMEM_BYTES);
-      cudaFuncSetAttribute(gemm_ragged_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<2>::SMEM_BYTES);
-      attr = true;
-    }
-  }
-  if (cg == 2) return lb_launch_cluster(dependent, 2, gemm_ragged_kernel<2>, lb_num_sms() / 2 * 2, NUM_THREADS, Cfg<2>::SMEM_BYTES, s, rp);
-  return lb_launch_cluster(dependent, 1, gemm_ragged_kernel<1>, lb_num_sms(), NUM_THREADS, Cfg<1>::SMEM_BYTES, s, rp);
+  const int workers = lb_num_sms() / cg;
+  if (cg == 2) return rp.epi == 2 ? launch_form(gemm_ragged_kernel<2, 8>, Cfg<2, 8>(), 2, workers, dependent, rp, s)
+                                  : launch_form(gemm_ragged_kernel<2, 4>, Cfg<2, 4>(), 2, workers, dependent, rp, s);
+  return rp.epi == 2 ? launch_form(gemm_ragged_kernel<1, 8>, Cfg<1, 8>(), 1, workers, dependent, rp, s)
+                     : launch_form(gemm_ragged_kernel<1, 4>, Cfg<1, 4>(), 1, workers, dependent, rp, s);
 }
 }  // namespace
 
@@ -1166,7 +1200,7 @@ extern "C" int lb_gemm_ragged_epi(const void* A, const void* const* B, void* C, 
     rp.C[e] = nullptr;
   }
   if ((rc = out_maps(rp.tc, C, C2, ldc, ldc2, cap, N, epi, half))) return rc;
-  rp.ldc = ldc; rp.old = (const bf16*)C2; rp.ld_old = ldc2; rp.epi = epi; rp.half = half; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = 0; rp.N = N; rp.K = K; rp.b_mn = b_mn;
+  rp.C[0] = (bf16*)C; rp.ldc = ldc; rp.old = (const bf16*)C2; rp.ld_old = ldc2; rp.epi = epi; rp.half = half; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = 0; rp.N = N; rp.K = K; rp.b_mn = b_mn;
   rp.mode = 0; rp.accumulate = 0; rp.cap = cap;
   rp.tiles_n = (N + BN - 1) / BN; rp.tiles_m_w = 0; rp.num_kb = (K + BK - 1) / BK;
   rp.wait_flag = (const unsigned int*)wait_flag; rp.wait_target = wait_target; rp.wait_ns = g_lb_flag_wait_ns;

@@ -657,17 +657,33 @@ __global__ void __launch_bounds__(256) ce_stats_kernel(const bf16* __restrict__ 
   const uint4* p = reinterpret_cast<const uint4*>(logits + (size_t)row * ld);
   const int nvec = V >> 3;
   float m = -INFINITY, s = 0.f;
-  for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-    float f[8];
-    unpack8(p[v], f);
-    float lm = f[0];
+  // Four vectors at a time, all loaded before the first is used (one by one, 8192 x 32000 110 us; now 99, 5.3 TB/s)
+  for (int v = threadIdx.x; v < nvec; v += 4 * blockDim.x) {
+    uint4 q[4];
 #pragma unroll
-    for (int i = 1; i < 8; i++) lm = fmaxf(lm, f[i]);
-    const float nm = fmaxf(m, lm);
-    float acc = 0.f;
+    for (int k = 0; k < 4; k++) {
+      const int at = v + k * (int)blockDim.x;
+      q[k] = at < nvec ? p[at] : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);      // -inf
+    }
+    float nm = m;
 #pragma unroll
-    for (int i = 0; i < 8; i++) acc += __expf(f[i] - nm);
-    s = s * __expf(m - nm) + acc;
+    for (int k = 0; k < 4; k++) {
+      float f[8];
+      unpack8(q[k], f);
+#pragma unroll
+      for (int i = 0; i < 8; i++) nm = fmaxf(nm, f[i]);
+    }
+    const float ref = nm == -INFINITY ? 0.f : nm;      // (nothing but masked columns so far)
+    float acc[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      float f[8];
+      unpack8(q[k], f);
+      acc[k] = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; i++) acc[k] += __expf(f[i] - ref);
+    }
+    s = s * __expf(m - ref) + ((acc[0] + acc[1]) + (acc[2] + acc[3]));
     m = nm;
   }
   __shared__ float sm[8], ss[8];
@@ -725,10 +741,10 @@ extern "C" int lb_ce_stats(const void* logits, const void* tgt, void* mx, void* 
 }
 
 // lse[t] = log-sum-exp of row t, loss[0] = inv_n * sum over the rows whose target counts of (lse - target logit).  A fixed order
-// of the sum makes the loss the same every time.  Up to CE_LOSS_ROWS rows one block does it all (8192 rows 14 us, of which
-// half is the launch); beyond, a double-precision logarithm per row is too much for one SM (131072 rows 155 us): a block per
-// CE_LOSS_ROWS / 2 rows leaves its sum in the first of its rows' `se`, which nothing reads any more, and a second kernel adds them.
-constexpr int CE_LOSS_ROWS = 8192;
+// of the sum makes the loss the same every time.  Up to CE_LOSS_ROWS rows one block does it all; beyond, a double-precision logarithm per
+// row is too much for one SM (8192 rows 12.5 us): a block per CE_LOSS_ROWS / 2 rows leaves its sum in the first of its rows' `se`, which nothing reads any
+// more, and a second kernel adds them (3.4 + 3.6 us).
+constexpr int CE_LOSS_ROWS = 1024;
 
 __device__ __forceinline__ float ce_block_sum(float s) {      // of 1024 threads; complete in thread 0
   __shared__ float sh[32];

@@ -380,6 +380,26 @@ def test_cross_entropy_loss_rows(T, V):
     assert _rel(got, torch.autograd.grad(want, w)[0]) < 5e-3
 
 
+@pytest.mark.parametrize("V", [8, 2040, 2056, 8184, 8200, 32000])
+@pytest.mark.parametrize("masked", [None, -float("inf"), torch.finfo(torch.bfloat16).min])
+def test_cross_entropy_widths(V, masked):
+    """Widths around what a step of the row statistics takes, with masked columns in whole steps and in parts of them."""
+    from lightron_b200.ops import functional as OF
+    T = 5
+    logits, tgt = _rand(T, V, scale=3.0, seed=1), torch.full((T,), V - 1, device="cuda")
+    if masked is not None:
+        logits[:, :V - 3] = masked
+        logits[1, :] = _rand(V, seed=2)
+        logits[2, 3:V // 2] = 1.0
+    x = logits.clone().requires_grad_(True)
+    loss = OF.cross_entropy(x * 1, tgt, n_valid_total=T)
+    got, = torch.autograd.grad(loss, x)
+    w = logits.double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(w, tgt)
+    assert abs(loss.item() - want.item()) < 4e-6 * max(1.0, want.item())
+    assert _rel(got, torch.autograd.grad(want, w)[0]) < 5e-3
+
+
 # ---- mixture of experts ------------------------------------------------------------------------------------
 
 

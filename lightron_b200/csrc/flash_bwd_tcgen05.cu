@@ -28,8 +28,12 @@
 // dQ's columns freed after 110 instead of 800 cycles, dK and dV through TMA stores (prologue and stores of a CTA: 12000 / 16000 cycles before).
 // Loops of 0.35 s of all its kernels, before / now, on one GPU: B8 S2048 32q/4kv d64 646 / 547 us, B1 S8192 32q/8kv d128
 // 1624 / 1404, B3 S1531 32q/8kv d128 237 / 221, B1 S4096 8q/8kv d128 117 / 104.
+// A key block's loop over query blocks may be cut into parts of `chunk` blocks, a CTA each, where whole loops would leave SMs without work (a causal
+// sequence's first key block takes as long as all blocks of the last ones together, and grouped heads make few CTAs of long loops): their dK / dV are then added up in
+// fp32 as dQ is, and converted with it (bwd_chunk() has the rule and the figures).
 // Warp roles (512 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4-11 math, 12-15 dQ drain.
 // All waits are bounded; on expiry a status word is set and the CTA drains and frees its TMEM.
+#include <algorithm>
 #include "tcgen05.cuh"
 
 static __device__ unsigned int g_fab_status[4] = {0, 0, 0, 0};
@@ -47,6 +51,8 @@ struct FaBwdParams {
   float scale;
   int causal;
   int kv_brows;   // rows between consecutive batches in the K/V tensor maps (>= Sk)
+  int chunk;      // query blocks of a CTA, or 0: all of its key block, whose dK / dV it writes
+  float *dk_acc, *dv_acc;      // with chunk: fp32 sums, in the layout of dq_acc
 };
 
 // (batch, kv head) pairs whose key blocks are ordered together: enough to keep the chip busy to the end,
@@ -86,42 +92,50 @@ struct BwdCfg {
 };
 static_assert(BwdCfg<128>::SMEM <= 232448, "shared memory of a CTA");
 
-// fp32 dQ accumulator layout: tile (b, h, mblock) -> 4 row quads -> D / 4 pieces of 4 columns -> 32 rows: the 16-byte stores of a
+// fp32 accumulator layout (dQ, and dK / dV in parts): tile (b, h, block of 128 rows) -> 4 row quads -> D / 4 pieces of 4 columns -> 32 rows: the 16-byte stores of a
 // drain warp (a row per lane) are contiguous, and so are the 16-byte loads of a warp here.
 template <int D>
 __global__ void fa_dq_convert_kernel(const FaBwdParams p) {
   grid_go();
   grid_wait();
   constexpr int CPR = D / 32;                                  // 32-column chunks per row: a thread takes one
-  const int n_mblocks = (p.Sq + 127) / 128;
-  const long long total = (long long)p.B * p.hq * n_mblocks * 128 * CPR;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
+  const int qblocks = (p.Sq + 127) / 128, kblocks = (p.Sk + 127) / 128;
+  const long long nq = (long long)p.B * p.hq * qblocks * 128 * CPR;
+  const long long nk = p.chunk ? (long long)p.B * p.hkv * kblocks * 128 * CPR : 0;
+  for (long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x; at < nq + 2 * nk;
+       at += (long long)gridDim.x * blockDim.x) {
+    // whole warps: the three parts are multiples of 32
+    const int which = at < nq ? 0 : at < nq + nk ? 1 : 2;
+    const long long idx = which == 0 ? at : which == 1 ? at - nq : at - nq - nk;
+    const float* acc = which == 0 ? p.dq_acc : which == 1 ? p.dk_acc : p.dv_acc;
+    bf16* out = which == 0 ? p.dq : which == 1 ? p.dk : p.dv;
+    const long long ts = which == 0 ? p.dq_ts : which == 1 ? p.dk_ts : p.dv_ts;
+    const int S = which == 0 ? p.Sq : p.Sk, heads = which == 0 ? p.hq : p.hkv, blocks = which == 0 ? qblocks : kblocks;
     const int lane = (int)(idx & 31);
     const long long w = idx >> 5;                              // (tile, quad, chunk): the accumulator's order
     const int chunk = (int)(w % CPR), quad = (int)((w / CPR) & 3);
     const long long tile = w / (CPR * 4);
-    const int mblock = (int)(tile % n_mblocks);
-    const long long bh = tile / n_mblocks;
-    const int row = mblock * 128 + quad * 32 + lane;
-    if (row >= p.Sq) continue;
-    const int h = (int)(bh % p.hq);
-    const long long b = bh / p.hq;
-    const float4* at = reinterpret_cast<const float4*>(p.dq_acc) + (w * 8) * 32 + lane;
+    const int block = (int)(tile % blocks);
+    const long long bh = tile / blocks;
+    const int row = block * 128 + quad * 32 + lane;
+    if (row >= S) continue;
+    const int h = (int)(bh % heads);
+    const long long b = bh / heads;
+    const float4* from = reinterpret_cast<const float4*>(acc) + (w * 8) * 32 + lane;
     float f[32];
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-      const float4 v = at[k * 32];
+      const float4 v = from[k * 32];
       f[4 * k] = v.x; f[4 * k + 1] = v.y; f[4 * k + 2] = v.z; f[4 * k + 3] = v.w;
     }
-    bf16* o = p.dq + (b * p.Sq + row) * p.dq_ts + (long long)h * D + chunk * 32;
+    bf16* o = out + (b * S + row) * ts + (long long)h * D + chunk * 32;
 #pragma unroll
     for (int k = 0; k < 4; k++) *reinterpret_cast<uint4*>(o + k * 8) = pack8(f + k * 8);
   }
 }
 
 // Row statistics, one 1 KB record per (b, h, 128-query block): 128 x -lse * log2(e), then 128 x -scale * sum_d o * do.  Rows
-// past Sq get (-inf, 0), which makes their P and dS zero.  Also clears the dQ accumulator.  D/8 threads per (token, head).
+// past Sq get (-inf, 0), which makes their P and dS zero.  Also clears the accumulators.  D/8 threads per (token, head).
 template <int D>
 __global__ void fa_bwd_prep_kernel(const FaBwdParams p) {
   grid_go();
@@ -131,6 +145,11 @@ __global__ void fa_bwd_prep_kernel(const FaBwdParams p) {
   const long long total = (long long)p.B * Sp * p.hq;
   const int rpb = blockDim.x / TPR;                            // rows per block and iteration
   const int sub = threadIdx.x % TPR;
+  if (p.chunk) {      // dk_acc and dv_acc, one behind the other
+    const long long n = 2LL * p.B * p.hkv * ((p.Sk + 127) / 128) * 128 * (D / 4);
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+      reinterpret_cast<float4*>(p.dk_acc)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   // every thread of the block runs the same number of iterations, so the shuffles see whole warps
   for (long long base = (long long)blockIdx.x * rpb; base < total; base += (long long)gridDim.x * rpb) {
     const long long idx = base + threadIdx.x / TPR;
@@ -164,7 +183,17 @@ __global__ void fa_bwd_prep_kernel(const FaBwdParams p) {
   }
 }
 
-template <int D>
+// First 128-query block that sees key block `nblk`, and the parts that its loop is cut into.
+__host__ __device__ __forceinline__ int bwd_first_block(int causal, int nblk, int off) {
+  const int first_row = nblk * 128 - off;
+  return causal && first_row > 0 ? first_row / 128 : 0;
+}
+__host__ __device__ __forceinline__ int bwd_parts(int mb_first, int n_mblocks, int rep, int chunk) {
+  const int its = (n_mblocks > mb_first ? n_mblocks - mb_first : 0) * rep;
+  return its ? (its + chunk - 1) / chunk : 1;
+}
+
+template <int D, bool PARTS>      // PARTS: with chunk
 __global__ void __launch_bounds__(512, 1)
 fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                  const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tdk,
@@ -190,27 +219,39 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   const uint32_t bar1 = bar0 + 8u * (1 + 2 * C::QS + 2 * C::DS);
   const uint32_t s_full = bar1, dp_full = bar1 + 8, p_full = bar1 + 16, ds_full = bar1 + 24, dq_full = bar1 + 32, dq_free = bar1 + 40;
 
-  // 1-D grid.  Under a causal mask the first key block is seen by every query and the last by one block,
-  // so the CTAs of early key blocks of all (batch, kv head) pairs of a group come first (longest first: with
-  // one pair after the other, the last pair's longest CTA started when the chip was almost done).
   const int n_nblk = (p.Sk + C::BN - 1) / C::BN;
-  const int grp = (int)blockIdx.x / (n_nblk * BWD_GROUP);
-  const int in_grp = (int)blockIdx.x - grp * n_nblk * BWD_GROUP;
-  const int gsize = min(BWD_GROUP, p.hkv * p.B - grp * BWD_GROUP);
-  const int nblk = in_grp / gsize;
-  const int pair = grp * BWD_GROUP + in_grp % gsize;
-  const int hk = pair % p.hkv, b = pair / p.hkv;
-  const int n0 = nblk * C::BN;
   const int off = p.Sk - p.Sq;
   const int rep = p.hq / p.hkv;
   const int n_mblocks = (p.Sq + C::BM - 1) / C::BM;
-  int mb_first = 0;
-  if (p.causal) {
-    const int first_row = n0 - off;
-    mb_first = first_row > 0 ? first_row / C::BM : 0;
+  int nblk, pair, part = 0;
+  if constexpr (PARTS) {
+    // parts of all key blocks of a pair, then the next pair
+    const int pairs = p.hkv * p.B;
+    pair = (int)blockIdx.x % pairs;
+    part = (int)blockIdx.x / pairs;
+    for (nblk = 0; nblk + 1 < n_nblk; nblk++) {
+      const int parts = bwd_parts(bwd_first_block(p.causal, nblk, off), n_mblocks, rep, p.chunk);
+      if (part < parts) break;
+      part -= parts;
+    }
+  } else {
+    // 1-D grid.  Under a causal mask the first key block is seen by every query and the last by one block,
+    // so the CTAs of early key blocks of all (batch, kv head) pairs of a group come first (longest first: with
+    // one pair after the other, the last pair's longest CTA started when the chip was almost done).
+    const int grp = (int)blockIdx.x / (n_nblk * BWD_GROUP);
+    const int in_grp = (int)blockIdx.x - grp * n_nblk * BWD_GROUP;
+    const int gsize = min(BWD_GROUP, p.hkv * p.B - grp * BWD_GROUP);
+    nblk = in_grp / gsize;
+    pair = grp * BWD_GROUP + in_grp % gsize;
   }
+  const int hk = pair % p.hkv, b = pair / p.hkv;
+  const int n0 = nblk * C::BN;
+  const int mb_first = bwd_first_block(p.causal, nblk, off);
   const int per_head = n_mblocks > mb_first ? n_mblocks - mb_first : 0;
-  const int total_it = per_head * rep;
+  // query blocks of every head of the group, head by head; a part takes `chunk` of them
+  const int it_first = PARTS ? part * p.chunk : 0;
+  const int total_it = PARTS ? min(p.chunk, per_head * rep - it_first) : per_head * rep;
+  const int h_first = hk * rep + (PARTS && per_head ? it_first / per_head : 0), mb_start = mb_first + (PARTS && per_head ? it_first % per_head : 0);
 
   if (threadIdx.x == 0) {
     s_abort[0] = 0;
@@ -246,7 +287,7 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         tma_load_2d(sbase + C::OFF_V + a * C::ATOM_BYTES, &tv, hk * D + a * 64, b * p.kv_brows + n0, kv_full);
       }
       bool ok = true;
-      int h = hk * rep, mb = mb_first, st = 0, dst = 0;
+      int h = h_first, mb = mb_start, st = 0, dst = 0;
       uint32_t ph = 1u, dph = 1u;
       for (int it = 0; it < total_it; it++) {
         if (!mbar_wait(q_empty(st), ph, abort_flag)) { ok = false; break; }
@@ -344,9 +385,9 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     const int quad = warp & 3;
     const uint32_t tdq = tmem_base + ((uint32_t)(quad * 32) << 16) + C::COL_DQ;
     uint8_t* stg = smem + C::OFF_STG + quad * 2 * C::STG_BYTES;
-    float* tile = p.dq_acc + (((long long)b * p.hq + hk * rep) * n_mblocks + mb_first) * (128 * D) + quad * (32 * D);
+    float* tile = p.dq_acc + (((long long)b * p.hq + h_first) * n_mblocks + mb_start) * (128 * D) + quad * (32 * D);
     bool ok = true;
-    int mb = mb_first;
+    int mb = mb_start;
     for (int it = 0; it < total_it; it++) {
       if (!mbar_wait(dq_full, (uint32_t)it & 1u, abort_flag)) { ok = false; break; }
       fence_after();
@@ -391,7 +432,7 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     const f32x2 sc = pack2(p.scale, p.scale);
     uint8_t* sds = smem + C::OFF_DS + wg * C::ATOM_BYTES;
     bool ok = true;
-    int mb = mb_first, qs = 0;
+    int mb = mb_start, qs = 0;
     uint32_t qph = 0;
     for (int it = 0; it < total_it; it++) {
       const int m0 = mb * C::BM;
@@ -476,7 +517,30 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     }
     // dQ of the last block is the last MMA: everything has finished
     if (ok && total_it > 0) ok = mbar_wait(dq_full, (uint32_t)(total_it - 1) & 1u, abort_flag);
-    if (ok && total_it > 0) {
+    if (PARTS && ok && total_it > 0) {
+      // added to the fp32 sums, 32 columns at a time
+      fence_after();
+      float* sum = (wg ? p.dk_acc : p.dv_acc) + (((long long)b * p.hkv + hk) * n_nblk + nblk) * (128 * D) + quad * (32 * D);
+      uint8_t* out = smem + (wg ? C::OFF_V : C::OFF_K) + quad * C::STG_BYTES;
+#pragma unroll 1
+      for (int c = 0; c < D / 32; c++) {
+        uint32_t r[32];
+        tmem_ld32(lane_addr + (wg ? C::COL_DK : C::COL_DV) + c * 32, r);
+        tmem_ld_wait();
+        if (lane == 0) bulk_wait_read_but<0>();
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          *reinterpret_cast<uint4*>(out + k * 512 + lane * 16) = make_uint4(r[k * 4], r[k * 4 + 1], r[k * 4 + 2], r[k * 4 + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          bulk_reduce_add_f32(sum + c * 1024, smem_u32(out), C::STG_BYTES);
+          bulk_commit();
+        }
+      }
+      if (lane == 0) bulk_wait_read_but<0>();        // nothing reads shared memory after the CTA's end
+    } else if (!PARTS && ok && total_it > 0) {
       // through shared memory (K's tile for dV, V's for dK: nothing reads them any more), 64 columns of 32 keys at a time
       fence_after();
 #pragma unroll 1
@@ -501,7 +565,7 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         }
       }
       if (lane == 0) bulk_wait_read_but<0>();        // nothing reads shared memory after the CTA's end
-    } else if (total_it == 0 && key < p.Sk) {
+    } else if (!PARTS && total_it == 0 && key < p.Sk) {
       // no query sees these keys: their gradients are zero
       bf16* orow = wg ? p.dk + ((long long)b * p.Sk + key) * p.dk_ts + (long long)hk * D
                       : p.dv + ((long long)b * p.Sk + key) * p.dv_ts + (long long)hk * D;
@@ -516,6 +580,42 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+}
+
+// CTAs of a launch in parts of `chunk` query blocks.
+long long bwd_ctas(int B, int Sq, int Sk, int hq, int hkv, int causal, int chunk) {
+  const int n_mblocks = (Sq + 127) / 128, rep = hq / hkv;
+  long long n = 0;
+  for (int k = 0; k < (Sk + 127) / 128; k++) n += bwd_parts(bwd_first_block(causal, k, Sk - Sq), n_mblocks, rep, chunk);
+  return n * hkv * B;
+}
+// Query blocks of a part, or 0 where a CTA per key block is modelled to be as good.  In query blocks: a CTA's fixed part is some 6, adding to the
+// fp32 sums instead of writing dK / dV 3 and their conversion 2 more.  Whole / parts, us, all kernels, causal: B2 S2000 16q/2kv d64 258 / 92, B1 S2000
+// 16q/4kv d64 116 / 51 and d128 159 / 71, B1 S8192 8q/2kv d128 561 / 365 and 2q/2kv 147 / 116, B4 S500 16q/4kv d64 40 / 28, B1 S300 8q/2kv d64 30 / 14; left
+// whole B8 S2048 32q/4kv d64, B1 S8192 32q/8kv d128, B3 S1531 32q/8kv d128, B2 S1728 4q/4kv d64.
+int bwd_chunk(int B, int Sq, int Sk, int hq, int hkv, int causal, int sms) {
+  const int n_mblocks = (Sq + 127) / 128, n_nblk = (Sk + 127) / 128, rep = hq / hkv, pairs = hkv * B;
+  if ((long long)n_nblk * pairs > 4LL * sms) return 0;             // (several CTAs per SM, longest first)
+  long long total = 0, longest = 0;
+  for (int k = 0; k < n_nblk; k++) {
+    const long long its = (long long)std::max(0, n_mblocks - bwd_first_block(causal, k, Sk - Sq)) * rep;
+    total += (its + 6) * pairs;
+    longest = std::max(longest, its + 6);
+  }
+  const double whole = std::max((double)longest, 1.1 * (double)total / sms);
+  int best = 0;
+  double best_time = 0.9 * whole;
+  for (int waves = 1; waves <= 2; waves++) {
+    // the smallest parts that make no more CTAs than that many per SM
+    int lo = 1, hi = n_mblocks * rep;
+    while (lo < hi) {
+      const int mid = (lo + hi) / 2;
+      if (bwd_ctas(B, Sq, Sk, hq, hkv, causal, mid) <= (long long)waves * sms) hi = mid; else lo = mid + 1;
+    }
+    const double time = waves * (lo + 9.0) + 2.0;
+    if (time < best_time && bwd_ctas(B, Sq, Sk, hq, hkv, causal, lo) <= (long long)waves * sms) { best = lo; best_time = time; }
+  }
+  return best;
 }
 
 template <int D>
@@ -534,19 +634,23 @@ int launch_fa_bwd(const void* q, const void* k, const void* v, const FaBwdParams
   static bool attr = false;
   if (!attr) {
     // the register split must fit in what the launch allocates, or it would wait for registers that nobody gives back
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, fa_bwd_tc_kernel<D>) != cudaSuccess || (fa.numRegs + 7) / 8 * 8 != 128) return LB_ERR_LAUNCH;
-    cudaFuncSetAttribute(fa_bwd_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    for (auto fn : {fa_bwd_tc_kernel<D, false>, fa_bwd_tc_kernel<D, true>}) {
+      cudaFuncAttributes fa;
+      if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess || (fa.numRegs + 7) / 8 * 8 != 128) return LB_ERR_LAUNCH;
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    }
     attr = true;
   }
-  const long long grid = (long long)((p.Sk + 127) / 128) * p.hkv * p.B;
+  long long grid = (long long)((p.Sk + 127) / 128) * p.hkv * p.B;
   if (grid > 2147483647LL) return LB_ERR_SHAPE;
+  if (p.chunk) grid = bwd_ctas(p.B, p.Sq, p.Sk, p.hq, p.hkv, p.causal, p.chunk);
   const long long rows = (long long)p.B * ((p.Sq + 127) / 128 * 128) * p.hq;
   const long long rows_per_block = 256 / (D / 8), cap = lb_num_sms() * 16;
   const long long pblocks = (rows + rows_per_block - 1) / rows_per_block;
   LB_LAUNCH(fa_bwd_prep_kernel<D>, (int)(pblocks < cap ? pblocks : cap), 256, 0, s, p);
-  LB_LAUNCH(fa_bwd_tc_kernel<D>, (unsigned)grid, C::NTHREADS, C::SMEM, s, tq, tk, tv, tdo, tdk, tdv, p);
-  const long long cblocks = (rows * (D / 32) + 255) / 256;
+  LB_LAUNCH(p.chunk ? fa_bwd_tc_kernel<D, true> : fa_bwd_tc_kernel<D, false>, (unsigned)grid, C::NTHREADS, C::SMEM, s, tq, tk, tv, tdo, tdk, tdv, p);
+  const long long kv_rows_acc = p.chunk ? 2LL * p.B * ((p.Sk + 127) / 128 * 128) * p.hkv : 0;
+  const long long cblocks = ((rows + kv_rows_acc) * (D / 32) + 255) / 256;
   LB_LAUNCH(fa_dq_convert_kernel<D>, (int)(cblocks < cap ? cblocks : cap), 256, 0, s, p);
   return LB_OK;
 }
@@ -569,8 +673,22 @@ extern "C" long long lb_flash_bwd_ws_bytes(int B, int Sq, int hq, int d) {
   return (long long)B * hq * ((Sq + 127) / 128) * 128 * (2 + d) * (long long)sizeof(float);
 }
 
+// As above with room for fp32 dK / dV where that lets the launch be cut into more parts (zero otherwise): what the caller of lb_flash_bwd_tc_ws should bring.
+// With lb_flash_bwd_ws_bytes() a CTA takes a whole key block.
+extern "C" long long lb_flash_bwd_ws_bytes_kv(int B, int Sq, int Sk, int hq, int hkv, int d, int causal) {
+  const long long q = lb_flash_bwd_ws_bytes(B, Sq, hq, d);
+  if (!q || Sk <= 0 || hkv <= 0 || hq % hkv || !bwd_chunk(B, Sq, Sk, hq, hkv, causal, lb_num_sms())) return q;
+  return q + 2LL * B * hkv * ((Sk + 127) / 128) * 128 * d * (long long)sizeof(float);
+}
+
+// Host only (no CUDA call): query blocks per CTA of the launch for these sizes on `sms` SMs, given that workspace; 0: all of a key block.
+extern "C" int lb_flash_bwd_chunk(int B, int Sq, int Sk, int hq, int hkv, int causal, int sms) {
+  if (B <= 0 || Sq <= 0 || Sk <= 0 || hq <= 0 || hkv <= 0 || hq % hkv || sms <= 0) return LB_ERR_SHAPE;
+  return bwd_chunk(B, Sq, Sk, hq, hkv, causal, sms);
+}
+
 static int flash_bwd_tc_impl(int kv_brows, const void* q, const void* k, const void* v, const void* o, const void* dout,
-                               const void* lse, void* stats, void* dq_acc, void* dq, void* dk, void* dv, int B, int Sq,
+                               const void* lse, void* stats, void* dq_acc, void* dkv_acc, void* dq, void* dk, void* dv, int B, int Sq,
                                int Sk, int hq, int hkv, int d, long long q_ts, long long k_ts, long long v_ts,
                                long long o_ts, long long do_ts, long long dq_ts, long long dk_ts, long long dv_ts,
                                float scale, int causal, void* stream) {
@@ -581,7 +699,11 @@ static int flash_bwd_tc_impl(int kv_brows, const void* q, const void* k, const v
     return LB_ERR_ARG;
   FaBwdParams p{(const bf16*)o, (const bf16*)dout, (const float*)lse, (float*)stats, (float*)dq_acc,
                 (bf16*)dq, (bf16*)dk, (bf16*)dv, B, Sq, Sk, hq, hkv, o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal,
-                kv_brows};
+                kv_brows, 0, nullptr, nullptr};
+  if (dkv_acc && (p.chunk = bwd_chunk(B, Sq, Sk, hq, hkv, causal, lb_num_sms())) > 0) {
+    p.dk_acc = (float*)dkv_acc;
+    p.dv_acc = p.dk_acc + (long long)B * hkv * ((Sk + 127) / 128) * 128 * d;
+  }
   cudaStream_t s = (cudaStream_t)stream;
   switch (d) {
     case 64: return launch_fa_bwd<64>(q, k, v, p, q_ts, k_ts, v_ts, s);
@@ -591,7 +713,7 @@ static int flash_bwd_tc_impl(int kv_brows, const void* q, const void* k, const v
 }
 
 // Same contract as lb_flash_bwd (flash_attn.cu) except for the scratch: a workspace of ws_bytes >= lb_flash_bwd_ws_bytes(), 16-byte
-// aligned, that need not be initialised.  head_dim 64 or 128; causal needs Sk >= Sq.  K/V are the first Sk rows of every
+// aligned, that need not be initialised (with the bytes of lb_flash_bwd_ws_bytes_kv() short launches are cut into more parts).  head_dim 64 or 128; causal needs Sk >= Sq.  K/V are the first Sk rows of every
 // batch of a buffer with kv_brows rows per batch (the context-parallel gather buffers; Sk for plain tensors); dk / dv
 // stay [B, Sk, hkv, d].
 extern "C" int lb_flash_bwd_cp_ws(const void* q, const void* k, const void* v, const void* o, const void* dout,
@@ -604,7 +726,8 @@ extern "C" int lb_flash_bwd_cp_ws(const void* q, const void* k, const void* v, c
   if (!need) return LB_ERR_SHAPE;
   if (ws_bytes < need) return LB_ERR_CAPACITY;
   const long long n_pad = (long long)B * hq * ((Sq + 127) / 128) * 128;
-  return flash_bwd_tc_impl(kv_brows, q, k, v, o, dout, lse, ws, (float*)ws + 2 * n_pad, dq, dk, dv, B, Sq, Sk, hq, hkv, d,
+  float* dkv_acc = ws_bytes >= need + 2LL * B * hkv * ((Sk + 127) / 128) * 128 * d * (long long)sizeof(float) ? (float*)ws + (2 + d) * n_pad : nullptr;
+  return flash_bwd_tc_impl(kv_brows, q, k, v, o, dout, lse, ws, (float*)ws + 2 * n_pad, dkv_acc, dq, dk, dv, B, Sq, Sk, hq, hkv, d,
                            q_ts, k_ts, v_ts, o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal, stream);
 }
 
@@ -629,7 +752,7 @@ extern "C" int lb_flash_bwd_cp(const void* q, const void* k, const void* v, cons
   void* stats = nullptr;
   cudaError_t e = cudaMallocAsync(&stats, (size_t)B * hq * ((Sq + 127) / 128) * 256 * sizeof(float), (cudaStream_t)stream);
   if (e != cudaSuccess) { cudaGetLastError(); g_lb_last_cuda_error = (int)e; return LB_ERR_LAUNCH; }
-  const int rc = flash_bwd_tc_impl(kv_brows, q, k, v, o, dout, lse, stats, dq_acc, dq, dk, dv, B, Sq, Sk, hq, hkv, d, q_ts, k_ts,
+  const int rc = flash_bwd_tc_impl(kv_brows, q, k, v, o, dout, lse, stats, dq_acc, nullptr, dq, dk, dv, B, Sq, Sk, hq, hkv, d, q_ts, k_ts,
                                    v_ts, o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal, stream);
   e = cudaFreeAsync(stats, (cudaStream_t)stream);
   if (rc == LB_OK && e != cudaSuccess) { g_lb_last_cuda_error = (int)e; return LB_ERR_LAUNCH; }

@@ -42,7 +42,7 @@ struct Api {
   int (*lb_gemm_grouped_epi)(int, const P*, const P*, const W*, const int*, const int*, const int*, const L*, const L*, const L*, const int*,
                              const int*, const int*, const int*, const W*, const L*, const int*, W);
   int (*lb_flash_fwd_tc)(P, P, P, W, W, int, int, int, int, int, int, L, L, L, L, float, int, W);
-  L (*lb_flash_bwd_ws_bytes)(int, int, int, int);
+  L (*lb_flash_bwd_ws_bytes_kv)(int, int, int, int, int, int, int);
   int (*lb_flash_bwd_tc_ws)(P, P, P, P, P, P, W, L, W, W, W, int, int, int, int, int, int, L, L, L, L, L, L, L, L, float, int, W);
   int (*lb_flash_bwd)(P, P, P, P, P, P, W, W, W, W, W, int, int, int, int, int, int, L, L, L, L, L, L, L, L, float, int, W);
   int (*lb_embedding_fwd)(P, P, W, int, int, int, int, W);
@@ -278,7 +278,7 @@ void attention_backward(const Heads& q, const Heads& k, const Heads& v, const Te
   const L o_ts = (L)m.hq * m.d, rows = (L)m.B * m.Sq;
   const Tensor o = operand(saved_o, grad, rows * o_ts, -1), lse = operand(saved_lse, grad, rows * m.hq, m.Sq, at::kFloat);
   if (env_is_tc("LIGHTRON_FA_BWD")) {
-    const L bytes = api.lb_flash_bwd_ws_bytes(m.B, m.Sq, m.hq, m.d);
+    const L bytes = api.lb_flash_bwd_ws_bytes_kv(m.B, m.Sq, m.Sk, m.hq, m.hkv, m.d, m.causal);
     Tensor ws = at::empty({bytes}, o.options().dtype(at::kByte));
     LB_CALL(lb_flash_bwd_tc_ws, q.p, k.p, v.p, o.const_data_ptr(), dout.p, lse.const_data_ptr(), ws.mutable_data_ptr(), bytes, dq, dk, dv, m.B, m.Sq,
             m.Sk, m.hq, m.hkv, m.d, q.ts, k.ts, v.ts, o_ts, dout.ts, dq_ts, dk_ts, dv_ts, m.scale, m.causal, stream());
@@ -710,7 +710,7 @@ PyObject* py_init(PyObject*, PyObject* args) {
   };
 #define LB_TAKE(name) take(#name, &api.name)
   LB_TAKE(lb_rmsnorm_fwd); LB_TAKE(lb_rmsnorm_bwd_blocks); LB_TAKE(lb_rmsnorm_bwd); LB_TAKE(lb_rope); LB_TAKE(lb_gemm_grouped_epi);
-  LB_TAKE(lb_flash_fwd_tc); LB_TAKE(lb_flash_bwd_ws_bytes); LB_TAKE(lb_flash_bwd_tc_ws); LB_TAKE(lb_flash_bwd); LB_TAKE(lb_embedding_fwd); LB_TAKE(lb_clear);
+  LB_TAKE(lb_flash_fwd_tc); LB_TAKE(lb_flash_bwd_ws_bytes_kv); LB_TAKE(lb_flash_bwd_tc_ws); LB_TAKE(lb_flash_bwd); LB_TAKE(lb_embedding_fwd); LB_TAKE(lb_clear);
   LB_TAKE(lb_embedding_bwd); LB_TAKE(lb_ce_stats); LB_TAKE(lb_ce_loss); LB_TAKE(lb_ce_grad); LB_TAKE(lb_gemm_rope);
   if (!ok) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "an entry point of the kernels is missing");

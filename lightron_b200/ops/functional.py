@@ -629,7 +629,7 @@ def flash_bwd_native(q, k, v, o, lse, do, causal: bool, scale: float, dq=None, d
             do.stride(1), dq.stride(1), dk.stride(1), dv.stride(1), float(scale), int(causal), native.stream_ptr())
     head = (q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr())
     if use_tc:
-        ws = native.flash_bwd_workspace(B, Sq, hq, d, q.device)
+        ws = native.flash_bwd_workspace(B, Sq, hq, d, q.device, (Sk, hkv, causal))
         native.call("lb_flash_bwd_tc_ws", *head, ws.data_ptr(), ws.numel(), *tail)
     else:
         delta = torch.empty(B, hq, Sq, dtype=torch.float32, device=q.device)

@@ -104,6 +104,8 @@ _SIGNATURES = {
     "lb_flash_bwd_tc_ws": [_P, _P, _P, _P, _P, _P, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I,
                            _L, _L, _L, _L, _L, _L, _L, _L, _F, _I, _P],
     "lb_flash_bwd_ws_bytes": [_I, _I, _I, _I],
+    "lb_flash_bwd_ws_bytes_kv": [_I, _I, _I, _I, _I, _I, _I],
+    "lb_flash_bwd_chunk": [_I, _I, _I, _I, _I, _I, _I],
     "lb_flash_bwd_status": [_P],
     "lb_flash_bwd_tc": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
                         _L, _L, _L, _L, _L, _L, _L, _L, _F, _I, _P],
@@ -130,7 +132,7 @@ def _load() -> Optional[ctypes.CDLL]:
         if fn is None:
             continue
         fn.argtypes = args
-        fn.restype = _L if name.endswith("_bytes") else c_int
+        fn.restype = _L if "_bytes" in name else c_int
     _LIB = lib
     wait_ms = os.environ.get("LIGHTRON_FLAG_WAIT_MS")     # limit of every device-side wait for a peer
     if wait_ms and hasattr(lib, "lb_set_flag_wait_ns"):
@@ -200,9 +202,13 @@ def stream_ptr() -> int:
     return _raw_stream(_current_device())
 
 
-def flash_bwd_workspace(B: int, Sq: int, hq: int, d: int, device) -> torch.Tensor:
-    """Scratch of one attention backward call (``lb_flash_bwd_tc_ws`` / ``lb_flash_bwd_cp_ws``), uninitialised."""
-    return torch.empty(require().lb_flash_bwd_ws_bytes(B, Sq, hq, d), dtype=torch.uint8, device=device)
+def flash_bwd_workspace(B: int, Sq: int, hq: int, d: int, device, kv=None) -> torch.Tensor:
+    """Scratch of one attention backward call (``lb_flash_bwd_tc_ws`` / ``lb_flash_bwd_cp_ws``), uninitialised.  With ``kv = (Sk, hkv, causal)`` it
+    has room for what lets a short launch be cut into more parts."""
+    lib = require()
+    if kv is None:
+        return torch.empty(lib.lb_flash_bwd_ws_bytes(B, Sq, hq, d), dtype=torch.uint8, device=device)
+    return torch.empty(lib.lb_flash_bwd_ws_bytes_kv(B, Sq, kv[0], hq, kv[1], d, int(kv[2])), dtype=torch.uint8, device=device)
 
 
 def ptr(t: Optional[torch.Tensor]) -> int:
@@ -239,7 +245,7 @@ def call(name: str, *args) -> None:
 # ---- autograd nodes in C++ ----------------------------------------------------------------------------
 _HOST = False               # not looked for yet; then the extension module, or None
 _HOST_ENTRIES = ("lb_rmsnorm_fwd", "lb_rmsnorm_bwd_blocks", "lb_rmsnorm_bwd", "lb_rope", "lb_gemm_grouped_epi", "lb_flash_fwd_tc",
-                 "lb_flash_bwd_ws_bytes", "lb_flash_bwd_tc_ws", "lb_flash_bwd", "lb_embedding_fwd", "lb_clear", "lb_embedding_bwd", "lb_ce_stats",
+                 "lb_flash_bwd_ws_bytes_kv", "lb_flash_bwd_tc_ws", "lb_flash_bwd", "lb_embedding_fwd", "lb_clear", "lb_embedding_bwd", "lb_ce_stats",
                  "lb_ce_loss", "lb_ce_grad", "lb_gemm_rope")
 
 

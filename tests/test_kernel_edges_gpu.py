@@ -147,6 +147,40 @@ def test_attention_backward_scratch_of_the_caller(B, Sq, d, shift):
 
 
 @pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("B,Sq,Sk,hq,hkv,causal,parts", [
+    (1, 300, 300, 8, 2, True, True),         # a query block per CTA, ragged last ones
+    (2, 1000, 1000, 16, 2, True, True),      # parts that end inside a head, and the last of a key block shorter
+    (1, 515, 1290, 16, 1, True, True),       # more keys than queries
+    (1, 200, 1100, 16, 2, False, True),
+    (1, 1290, 130, 16, 2, False, True),      # few keys, long loops
+    (8, 640, 640, 8, 8, True, False),        # enough CTAs
+])
+def test_attention_backward_in_parts(B, Sq, Sk, hq, hkv, causal, d, parts):
+    """Key blocks whose loops are cut, against 64 bits and against the launch with the workspace that leaves them whole; rows behind the last are not
+    written.  dK and dV are fp32 sums of the same products in another order, rounded once."""
+    from lightron_b200.ops import functional as OF, native
+    lib = native.require()
+    assert (lib.lb_flash_bwd_chunk(B, Sq, Sk, hq, hkv, int(causal), native.sm_count()) > 0) == parts
+    need = lib.lb_flash_bwd_ws_bytes(B, Sq, hq, d)
+    assert (lib.lb_flash_bwd_ws_bytes_kv(B, Sq, Sk, hq, hkv, d, int(causal)) > need) == parts
+    q, do = _rand(B, Sq, hq, d, seed=1), _rand(B, Sq, hq, d, seed=4)
+    k, v = _rand(B, Sk, hkv, d, seed=2), _rand(B, Sk, hkv, d, seed=3)
+    o, lse = OF.flash_fwd_native(q, k, v, causal, d ** -0.5)
+    buf = [torch.full((B * n + 128, h, d), 7.0, dtype=torch.bfloat16, device="cuda") for n, h in ((Sq, hq), (Sk, hkv), (Sk, hkv))]
+    dq, dk, dv = (t[:B * n].view(B, n, -1, d) for t, n in zip(buf, (Sq, Sk, Sk)))
+    OF.flash_bwd_native(q, k, v, o, lse, do, causal, d ** -0.5, dq, dk, dv)
+    whole = [torch.empty_like(t) for t in (dq, dk, dv)]
+    ws = native.flash_bwd_workspace(B, Sq, hq, d, q.device)
+    native.call("lb_flash_bwd_tc_ws", q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(), ws.data_ptr(), ws.numel(),
+                *(t.data_ptr() for t in whole), B, Sq, Sk, hq, hkv, d, *(t.stride(1) for t in (q, k, v, o, do, *whole)), d ** -0.5, int(causal),
+                native.stream_ptr())
+    _status_ok()
+    for name, g, w, x in zip(("dq", "dk", "dv"), (dq, dk, dv), _attention64(q, k, v, do, causal)[1:], whole):
+        assert _rel(g, w) < 1e-2 and _rel(g, x.double()) < 2.0 ** -8, name
+    assert all(bool((t[B * n:] == 7.0).all()) for t, n in zip(buf, (Sq, Sk, Sk)))
+
+
+@pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 def test_attention_bad_scores_stay_in_their_rows(d, bad):
     """A key that is not finite spoils the rows that see it, whichever unit computes its exponentials, and no other."""

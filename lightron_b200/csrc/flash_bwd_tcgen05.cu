@@ -94,18 +94,18 @@ static_assert(BwdCfg<128>::SMEM <= 232448, "shared memory of a CTA");
 
 // fp32 accumulator layout (dQ, and dK / dV in parts): tile (b, h, block of 128 rows) -> 4 row quads -> D / 4 pieces of 4 columns -> 32 rows: the 16-byte stores of a
 // drain warp (a row per lane) are contiguous, and so are the 16-byte loads of a warp here.
-template <int D>
+template <int D, bool PARTS>
 __global__ void fa_dq_convert_kernel(const FaBwdParams p) {
   grid_go();
   grid_wait();
   constexpr int CPR = D / 32;                                  // 32-column chunks per row: a thread takes one
   const int qblocks = (p.Sq + 127) / 128, kblocks = (p.Sk + 127) / 128;
   const long long nq = (long long)p.B * p.hq * qblocks * 128 * CPR;
-  const long long nk = p.chunk ? (long long)p.B * p.hkv * kblocks * 128 * CPR : 0;
+  const long long nk = PARTS ? (long long)p.B * p.hkv * kblocks * 128 * CPR : 0;
   for (long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x; at < nq + 2 * nk;
        at += (long long)gridDim.x * blockDim.x) {
     // whole warps: the three parts are multiples of 32
-    const int which = at < nq ? 0 : at < nq + nk ? 1 : 2;
+    const int which = !PARTS || at < nq ? 0 : at < nq + nk ? 1 : 2;
     const long long idx = which == 0 ? at : which == 1 ? at - nq : at - nq - nk;
     const float* acc = which == 0 ? p.dq_acc : which == 1 ? p.dk_acc : p.dv_acc;
     bf16* out = which == 0 ? p.dq : which == 1 ? p.dk : p.dv;
@@ -219,25 +219,23 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   const uint32_t bar1 = bar0 + 8u * (1 + 2 * C::QS + 2 * C::DS);
   const uint32_t s_full = bar1, dp_full = bar1 + 8, p_full = bar1 + 16, ds_full = bar1 + 24, dq_full = bar1 + 32, dq_free = bar1 + 40;
 
+  // 1-D grid.  Under a causal mask the first key block is seen by every query and the last by one block,
+  // so the CTAs of early key blocks of all (batch, kv head) pairs of a group come first (longest first: with
+  // one pair after the other, the last pair's longest CTA started when the chip was almost done).  In parts: those of the first key block of all
+  // pairs, then the next.
   const int n_nblk = (p.Sk + C::BN - 1) / C::BN;
-  const int off = p.Sk - p.Sq;
-  const int rep = p.hq / p.hkv;
-  const int n_mblocks = (p.Sq + C::BM - 1) / C::BM;
-  int nblk, pair, part = 0;
+  int nblk, pair, it_first = 0;
   if constexpr (PARTS) {
-    // parts of all key blocks of a pair, then the next pair
     const int pairs = p.hkv * p.B;
     pair = (int)blockIdx.x % pairs;
-    part = (int)blockIdx.x / pairs;
+    int part = (int)blockIdx.x / pairs;
     for (nblk = 0; nblk + 1 < n_nblk; nblk++) {
-      const int parts = bwd_parts(bwd_first_block(p.causal, nblk, off), n_mblocks, rep, p.chunk);
+      const int parts = bwd_parts(bwd_first_block(p.causal, nblk, p.Sk - p.Sq), (p.Sq + C::BM - 1) / C::BM, p.hq / p.hkv, p.chunk);
       if (part < parts) break;
       part -= parts;
     }
+    it_first = part * p.chunk;
   } else {
-    // 1-D grid.  Under a causal mask the first key block is seen by every query and the last by one block,
-    // so the CTAs of early key blocks of all (batch, kv head) pairs of a group come first (longest first: with
-    // one pair after the other, the last pair's longest CTA started when the chip was almost done).
     const int grp = (int)blockIdx.x / (n_nblk * BWD_GROUP);
     const int in_grp = (int)blockIdx.x - grp * n_nblk * BWD_GROUP;
     const int gsize = min(BWD_GROUP, p.hkv * p.B - grp * BWD_GROUP);
@@ -246,10 +244,16 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   }
   const int hk = pair % p.hkv, b = pair / p.hkv;
   const int n0 = nblk * C::BN;
-  const int mb_first = bwd_first_block(p.causal, nblk, off);
+  const int off = p.Sk - p.Sq;
+  const int rep = p.hq / p.hkv;
+  const int n_mblocks = (p.Sq + C::BM - 1) / C::BM;
+  int mb_first = 0;
+  if (p.causal) {
+    const int first_row = n0 - off;
+    mb_first = first_row > 0 ? first_row / C::BM : 0;
+  }
   const int per_head = n_mblocks > mb_first ? n_mblocks - mb_first : 0;
   // query blocks of every head of the group, head by head; a part takes `chunk` of them
-  const int it_first = PARTS ? part * p.chunk : 0;
   const int total_it = PARTS ? min(p.chunk, per_head * rep - it_first) : per_head * rep;
   const int h_first = hk * rep + (PARTS && per_head ? it_first / per_head : 0), mb_start = mb_first + (PARTS && per_head ? it_first % per_head : 0);
 
@@ -651,7 +655,7 @@ int launch_fa_bwd(const void* q, const void* k, const void* v, const FaBwdParams
   LB_LAUNCH(p.chunk ? fa_bwd_tc_kernel<D, true> : fa_bwd_tc_kernel<D, false>, (unsigned)grid, C::NTHREADS, C::SMEM, s, tq, tk, tv, tdo, tdk, tdv, p);
   const long long kv_rows_acc = p.chunk ? 2LL * p.B * ((p.Sk + 127) / 128 * 128) * p.hkv : 0;
   const long long cblocks = ((rows + kv_rows_acc) * (D / 32) + 255) / 256;
-  LB_LAUNCH(fa_dq_convert_kernel<D>, (int)(cblocks < cap ? cblocks : cap), 256, 0, s, p);
+  LB_LAUNCH(p.chunk ? fa_dq_convert_kernel<D, true> : fa_dq_convert_kernel<D, false>, (int)(cblocks < cap ? cblocks : cap), 256, 0, s, p);
   return LB_OK;
 }
 

@@ -781,13 +781,15 @@ __global__ void __launch_bounds__(Cfg<CG, EW>::NUM_THREADS, 1) gemm_ragged_kerne
 // ---- host side: static schedule, cached per (device, shapes) -------------------------------------
 struct Schedule {
   int split = 0;      // parts of K of a launch that the split form takes (gemm_split.cu; nothing else is set then), or 0
+  bool apart = false; // two problems that are launched one after the other (nothing else is set then)
+  bool on_host() const { return split > 0 || apart; }      // nothing has been uploaded
   int cg = 1;         // CTAs per tile
   int grid = 0;       // workers (CTAs, or pairs of CTAs)
   int* d_offsets = nullptr;
   int* d_items = nullptr;
   unsigned long long last_use = 0;
 };
-// Cache of uploaded schedules, keyed by (device, M, N, K of every problem).  A training run uses a
+// Cache of uploaded schedules, keyed by (device, M, N, K, epilogue of every problem).  A training run uses a
 // few dozen shape sets; callers whose row counts change from call to call (expert-parallel MoE)
 // use lb_gemm_ragged instead, which takes the counts from device memory and needs no schedule.
 // The cache is still bounded: beyond MAX_SCHEDULES entries the least recently used one is freed.  Entries of the split form are only a number
@@ -876,10 +878,38 @@ int choose_cg(Problem* probs, int np, int sms, long long* best = nullptr) {
   return cg;
 }
 
-int parts_of(const Problem* probs, int np, int sms, long long list_time) {
+int parts_of(const Problem* probs, int np, int sms, long long list_time, double* us = nullptr) {
   int M[MAX_PROBLEMS], N[MAX_PROBLEMS], K[MAX_PROBLEMS];
-  for (int i = 0; i < np; i++) { M[i] = probs[i].M; N[i] = probs[i].N; K[i] = probs[i].K; }
-  return gemm_split_parts(np, M, N, K, sms, list_time);
+  bool activation = false;
+  for (int i = 0; i < np; i++) {
+    M[i] = probs[i].M; N[i] = probs[i].N; K[i] = probs[i].K;
+    activation |= probs[i].epi == 1 || probs[i].epi == 2;
+  }
+  return gemm_split_parts(np, M, N, K, activation, sms, list_time, us);
+}
+
+// Whether two problems are better launched one after the other: a weight gradient over few rows is many short tiles, its data gradient a few tiles with a
+// long reduction, each of which a list gives to one worker.  On its own the latter is split.  Alone, short tiles take the time of their bytes (5.3 TB/s) and of
+// their waves; 5 us are kept back for the second launch.  Together / apart, us (n x k weights, T rows): 32000 x 768, T 64 149 / 42; 11264 x 2048, T 64 59 / 29, T
+// 256 60 / 40; 28672 x 4096, T 16 182 / 100; 8192 x 1024, T 496 44 / 30; 4096 x 768, T 64 25 / 20.  Passes of launches below 40 us are bound by the host (a
+// feed-forward of 64 x 768 takes 85 us of it and 47 of the GPU), to which a second launch only adds.
+bool better_apart(const Problem* probs, int np, int sms, long long list_time, double joint_us) {
+  if (np != 2 || sms < 4 || joint_us < 40.0) return false;
+  const int longest = std::max((probs[0].K + BK - 1) / BK, (probs[1].K + BK - 1) / BK);
+  if (100.0 * longest + 800 < 0.6 * (double)list_time) return false;
+  double alone = -2.0;
+  for (int i = 0; i < 2; i++) {
+    Problem p = probs[i];
+    long long time = 0;
+    double us = 0;
+    if (choose_cg(&p, 1, sms, &time) < 0) return false;
+    parts_of(&p, 1, sms, time, &us);
+    set_tiles(&p, 1);
+    const double mb = 2e-6 * ((double)p.M * p.K + (double)p.N * p.K + (double)p.M * p.N);
+    const double waves = std::ceil((double)p.tiles_m * p.tiles_n / sms);
+    alone += std::min(us, 5.0 + 0.19 * mb + 0.27 * waves * p.num_kb);
+  }
+  return alone + 5.0 < 0.93 * joint_us;
 }
 
 int build_schedule(Problem* probs, int np, int sms, Schedule* out) {
@@ -888,7 +918,10 @@ int build_schedule(Problem* probs, int np, int sms, Schedule* out) {
   long long time = 0;
   out->cg = choose_cg(probs, np, sms, &time);
   if (out->cg < 0) return LB_ERR_SHAPE;
-  if (time > 0 && (out->split = parts_of(probs, np, sms, time)) > 0) return LB_OK;
+  double us = 0;
+  if (time > 0) out->split = parts_of(probs, np, sms, time, &us);
+  if (time > 0 && better_apart(probs, np, sms, time, us)) { out->split = 0; out->apart = true; }
+  if (out->on_host()) return LB_OK;
   for (int i = 0; i < np; i++) set_tiles(&probs[i], out->cg);
   if (assign_items(probs, np, out->cg, sms, &per, &total, nullptr, nullptr) < 0) return LB_ERR_SHAPE;
   const int grid = (int)per.size();
@@ -990,12 +1023,13 @@ bool plan_problems(int n, const int* M, const int* N, const int* K, int sms, Pro
   for (int i = 0; i < n; i++) {
     if (M[i] <= 0 || N[i] <= 0 || K[i] <= 0) return false;
     probs[i].M = M[i]; probs[i].N = N[i]; probs[i].K = K[i];
+    probs[i].epi = 0;
   }
   return true;
 }
 }  // namespace
 
-// Host only (no CUDA call): parts of K (1, 2 or 4) with which lb_gemm_grouped gives these shapes to the split form (gemm_split.cu), 0 where
+// Host only (no CUDA call): parts of K (1, 2, 4 or 8) with which lb_gemm_grouped gives these shapes to the split form (gemm_split.cu), 0 where
 // it takes the list form, which the two entry points below describe.
 extern "C" int lb_gemm_grouped_parts(int n, const int* M, const int* N, const int* K, int sms) {
   Problem probs[MAX_PROBLEMS];
@@ -1003,6 +1037,17 @@ extern "C" int lb_gemm_grouped_parts(int n, const int* M, const int* N, const in
   long long time = 0;
   if (choose_cg(probs, n, sms, &time) < 0) return LB_ERR_SHAPE;
   return time > 0 ? parts_of(probs, n, sms, time) : 0;
+}
+
+// Host only (no CUDA call): 1 where lb_gemm_grouped launches two plain problems one after the other instead of together.
+extern "C" int lb_gemm_grouped_apart(int n, const int* M, const int* N, const int* K, int sms) {
+  Problem probs[MAX_PROBLEMS];
+  if (!plan_problems(n, M, N, K, sms, probs)) return LB_ERR_SHAPE;
+  long long time = 0;
+  double us = 0;
+  if (choose_cg(probs, n, sms, &time) < 0) return LB_ERR_SHAPE;
+  if (time > 0) parts_of(probs, n, sms, time, &us);
+  return time > 0 && better_apart(probs, n, sms, time, us);
 }
 
 // Host only (no CUDA call): CTAs per tile, 1 or 2, of the schedule that lb_gemm_grouped builds for these shapes on `sms` SMs.
@@ -1066,7 +1111,7 @@ static int run_grouped(int n, const void* const* A, const void* const* B, void* 
     p.M = M[i]; p.N = N[i]; p.K = K[i]; p.epi = rope ? 4 : e; p.half = e ? half[i] : 0; p.keep = C[i] != nullptr;
     p.old = (const bf16*)(e == 2 ? C2[i] : C[i]); p.ld_old = e == 2 ? ldc2[i] : ldc[i]; p.C = (bf16*)C[i]; p.ldc = ldc[i];
     p.a_mn = a_mn[i]; p.b_mn = b_mn[i]; p.accumulate = accumulate ? accumulate[i] : 0;
-    key.push_back(M[i]); key.push_back(N[i]); key.push_back(K[i]);
+    key.push_back(M[i]); key.push_back(N[i]); key.push_back(K[i]); key.push_back(e);
   }
   {
     std::lock_guard<std::mutex> lock(g_sched_mutex);
@@ -1082,12 +1127,12 @@ static int run_grouped(int n, const void* const* A, const void* const* B, void* 
       Schedule s;
       int rc = build_schedule(probs, n, g_sms, &s);
       if (rc) return rc;
-      const bool split = s.split > 0;
+      const bool split = s.on_host();
       if (++g_cached[split] > (split ? MAX_SPLITS : MAX_SCHEDULES)) {
         // evict the least recently used entry of its kind; cudaFree waits for kernels that may still read it
         auto victim = g_schedules.end();
         for (auto j = g_schedules.begin(); j != g_schedules.end(); ++j)
-          if ((j->second.split > 0) == split && (victim == g_schedules.end() || j->second.last_use < victim->second.last_use)) victim = j;
+          if (j->second.on_host() == split && (victim == g_schedules.end() || j->second.last_use < victim->second.last_use)) victim = j;
         if (!split) {
           cudaFree(victim->second.d_offsets);
           cudaFree(victim->second.d_items);
@@ -1099,6 +1144,14 @@ static int run_grouped(int n, const void* const* A, const void* const* B, void* 
     }
     it->second.last_use = ++g_sched_clock;
     sched = it->second;
+  }
+  if (sched.apart) {
+    for (int i = 0; i < n; i++) {
+      const int rc = run_grouped(1, A + i, B + i, C + i, M + i, N + i, K + i, lda + i, ldb + i, ldc + i, a_mn + i, b_mn + i, accumulate ? accumulate + i : nullptr,
+                                 epi ? epi + i : nullptr, C2 ? C2 + i : nullptr, ldc2 ? ldc2 + i : nullptr, half ? half + i : nullptr, nullptr, stream);
+      if (rc) return rc;
+    }
+    return LB_OK;
   }
   if (sched.split)
     return gemm_split_rope(n, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, accumulate, epi, C2, ldc2, half, sched.split, rope, stream);

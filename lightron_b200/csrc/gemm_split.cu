@@ -1,5 +1,5 @@
 // bf16 GEMM for launches that do not fill the chip:  C[M,N] (+)= op(A) op(B)^T with tiles of 128 x 64 whose reduction may be
-// split over a cluster of 2 or 4 CTAs; one or two problems per launch.
+// split over a cluster of 2, 4 or 8 CTAs; one or two problems per launch.
 //
 // Why: with the 128 x 256 tiles of gemm_grouped.cu a small problem is a handful of CTAs, each of which streams its whole K through
 // one SM.  An SM brings in 130 to 150 GB/s (what it has in flight over the latency of memory), so 0.38 us per 64 of K is all that such a launch
@@ -29,12 +29,14 @@ constexpr int BM = 128, BN = 64, BK = 64;
 constexpr int HB = BN / 2;                               // columns of a tile's two blocks
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-// KS parts of K.  With four a CTA has few k-blocks, and the place of a fourth stage is where the others' sums arrive.
+// KS parts of K.  A tile's 8 groups of 8 columns are finished by its CTAs: NG groups of each block by everyone, or, with eight parts, one group each (no
+// activation then, which wants both blocks' columns in one CTA).  With four and more a CTA has few k-blocks at a time in flight, and the place of a
+// fourth stage is where the others' sums arrive.
 template <int KS>
 struct Cfg {
-  static constexpr int STAGES = KS == 4 ? 3 : 4;
-  static constexpr int W = HB / KS;                      // columns of each block that a CTA finishes
-  static constexpr int RECV_BYTES = (KS - 1) * BM * 2 * W * 4;
+  static constexpr int STAGES = KS >= 4 ? 3 : 4;
+  static constexpr int G = 8 / KS, NG = KS == 8 ? 1 : HB / 8 / KS, NB = G / NG;      // groups of a CTA: NB blocks, NG in each
+  static constexpr int RECV_BYTES = (KS - 1) * BM * G * 8 * 4;
   static constexpr int OFF_RECV = STAGES * STAGE_BYTES;
   static constexpr int OFF_BAR = OFF_RECV + RECV_BYTES;
   static constexpr int SMEM_BYTES = OFF_BAR + 256;
@@ -121,7 +123,7 @@ __device__ __forceinline__ bool multiply(uint32_t d_tmem, int n_kb, uint32_t sme
 template <int KS>
 __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid_constant__ Params gp) {
   using C = Cfg<KS>;
-  constexpr int STAGES = C::STAGES, W = C::W, NG = W / 8;      // NG: groups of 8 columns per block that this CTA finishes
+  constexpr int STAGES = C::STAGES, NG = C::NG, NB = C::NB;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t smem_base = bw::smem_u32(smem);
   const uint32_t bar_base = smem_base + C::OFF_BAR;
@@ -141,6 +143,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
   // the tile's two blocks of columns: neighbours, or the gate and the up columns of the same index
   const int n0 = pr.epi == 1 ? tn * HB : tn * BN;
   const int n1 = pr.epi == 1 ? pr.half + n0 : n0 + HB;
+  // group g of its block b: which block, and the first column in it
+  auto block_of = [&](int b) { return KS == 8 ? rank >> 2 : b; };
+  auto column_of = [&](int g) { return KS == 8 ? (rank & 3) * 8 : (rank * NG + g) * 8; };
   const int kb0 = (int)((long long)pr.num_kb * rank / KS), n_kb = (int)((long long)pr.num_kb * (rank + 1) / KS) - kb0;
 
   if (threadIdx.x == 64) { bw::prefetch_tmap(&gp.ta[pi]); bw::prefetch_tmap(&gp.tb[pi]); }
@@ -183,7 +188,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
   const int row = m0 + row_in;
   const bool row_ok = row < pr.M;
   const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
-  float rot[2][NG][8];                                         // epi 4: cosines and sines of this row's columns, loaded ahead
+  float rot[NB][NG][8];                                        // epi 4: cosines and sines of this row's columns, loaded ahead
   if (warp == 0) {
     if (ok && bw::elect_one()) {
       const CUtensorMap *ta = &gp.ta[pi], *tb = &gp.tb[pi];
@@ -210,10 +215,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
     if (pr.epi == 4) {
       const int pos = row_ok ? rope_position(gp.rope, row) : 0;
 #pragma unroll
-      for (int b = 0; b < 2; b++)
+      for (int b = 0; b < NB; b++)
 #pragma unroll
         for (int g = 0; g < NG; g++) {
-          const int col = (b ? n1 : n0) + rank * W + g * 8;
+          const int col = (block_of(b) ? n1 : n0) + column_of(g);
           if (col < gp.rope.cols) rope_load8(gp.rope, pos, col, rot[b][g]);
         }
     }
@@ -234,10 +239,11 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
         bw::tmem_ld_wait();
 #pragma unroll
         for (int g = 0; g < 4; g++) {
-          const int s = g / NG;                                // the receiver; its place for this part: parts in order, its own left out
+          const int s = KS == 8 ? b * 4 + g : g / NG;          // the receiver; its place for this part: parts in order, its own left out
           if (s == rank) continue;
           const int slot = rank < s ? rank : rank - 1;
-          const uint32_t dst = bw::cluster_addr(mine + (uint32_t)((slot * 2 * W + b * W + (g % NG) * 8) * BM * 4), s);
+          const int to = KS == 8 ? 0 : b * NG + g % NG;
+          const uint32_t dst = bw::cluster_addr(mine + (uint32_t)((slot * C::G + to) * 8 * BM * 4), s);
           const uint32_t bar = bw::cluster_addr(received, s);
           bw::st_cluster_v4(dst, r + g * 8, bar);
           bw::st_cluster_v4(dst + BM * 16, r + g * 8 + 4, bar);
@@ -248,18 +254,18 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
     bw::cluster_arrive();
   }
   if (warp >= 2 && ok) {
-    float f[2][NG][8];
+    float f[NB][NG][8];
 #pragma unroll
-    for (int b = 0; b < 2; b++)
+    for (int b = 0; b < NB; b++)
 #pragma unroll
-      for (int g = 0; g < NG; g++) bw::tmem_ld8(taddr + b * HB + rank * W + g * 8, reinterpret_cast<uint32_t*>(f[b][g]));
+      for (int g = 0; g < NG; g++) bw::tmem_ld8(taddr + block_of(b) * HB + column_of(g), reinterpret_cast<uint32_t*>(f[b][g]));
     bw::tmem_ld_wait();
     if constexpr (KS > 1) {
       if (!bw::mbar_wait(received, 0, abort_flag)) { ok = false; give_up(abort_flag, 5u); }
       bw::fence_cluster();
       const float4* in = reinterpret_cast<const float4*>(smem + C::OFF_RECV) + row_in;
 #pragma unroll
-      for (int b = 0; b < 2; b++)
+      for (int b = 0; b < NB; b++)
 #pragma unroll
         for (int g = 0; g < NG; g++) {
           float own[8], sum[8];
@@ -268,7 +274,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
 #pragma unroll
           for (int s = 0; s < KS; s++) {                       // in the order of the parts
             const int slot = s < rank ? s : s - 1;
-            const float4* q = in + (size_t)((s == rank ? 0 : slot) * 2 * W + b * W + g * 8) / 4 * BM;
+            const float4* q = in + (size_t)((s == rank ? 0 : slot) * C::G + b * NG + g) * 2 * BM;
             const float4 x = q[0], y = q[BM];
             const float part[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
 #pragma unroll
@@ -282,12 +288,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
     if (row_ok && ok) {
 #pragma unroll
       for (int g = 0; g < NG; g++) {
-        const int cc = rank * W + g * 8;                       // column inside a block
-        if (pr.epi == 1) {
+        const int cc = column_of(g);                           // column inside a block
+        if (NB == 2 && pr.epi == 1) {
           // silu(g) * u is computed from the ROUNDED values (what a separate pass over the stored matrix would see)
           const int col = n0 + cc;
           if (col < n_end) {
-            const uint4 pg = pack8(f[0][g]), pu = pack8(f[1][g]);
+            const uint4 pg = pack8(f[0][g]), pu = pack8(f[NB - 1][g]);
             if (pr.C) {
               bf16* grow = pr.C + (size_t)row * pr.ldc + col;
               *reinterpret_cast<uint4*>(grow) = pg;
@@ -303,8 +309,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
           continue;
         }
 #pragma unroll
-        for (int b = 0; b < 2; b++) {
-          const int col = (b ? n1 : n0) + cc;
+        for (int b = 0; b < NB; b++) {
+          const int col = (block_of(b) ? n1 : n0) + cc;
           if (col >= n_end) continue;
           bf16* dst = pr.C + (size_t)row * pr.ldc + col;
           if (pr.epi == 2) {
@@ -373,8 +379,8 @@ extern "C" int lb_gemm_split_status(void* out) {
   return LB_OK;
 }
 
-// The arguments of lb_gemm_grouped_epi for n = 1 or 2 problems, with K split over ks = 1, 2 or 4 CTAs (no more than a
-// problem has 64-wide k-blocks).  lb_gemm_grouped_epi calls this with what gemm_split_parts() says.
+// The arguments of lb_gemm_grouped_epi for n = 1 or 2 problems, with K split over ks = 1, 2, 4 or 8 CTAs (no more than a
+// problem has 64-wide k-blocks; 8 without an activation).  lb_gemm_grouped_epi calls this with what gemm_split_parts() says.
 extern "C" int lb_gemm_split(int n, const void* const* A, const void* const* B, void* const* C, const int* M, const int* N, const int* K,
                              const long long* lda, const long long* ldb, const long long* ldc, const int* a_mn, const int* b_mn,
                              const int* accumulate, const int* epi, void* const* C2, const long long* ldc2, const int* half, int ks, void* stream) {
@@ -385,7 +391,7 @@ int gemm_split_rope(int n, const void* const* A, const void* const* B, void* con
                     const long long* lda, const long long* ldb, const long long* ldc, const int* a_mn, const int* b_mn,
                     const int* accumulate, const int* epi, void* const* C2, const long long* ldc2, const int* half, int ks, const RopeArgs* rope,
                     void* stream) {
-  if (n < 1 || n > MAX_PROBLEMS || (ks != 1 && ks != 2 && ks != 4)) return LB_ERR_SHAPE;
+  if (n < 1 || n > MAX_PROBLEMS || (ks != 1 && ks != 2 && ks != 4 && ks != 8)) return LB_ERR_SHAPE;
   Params gp;
   gp.rope = rope ? *rope : RopeArgs{nullptr, nullptr, nullptr, 1, 64, 0};
   gp.np = n;
@@ -401,6 +407,7 @@ int gemm_split_rope(int n, const void* const* A, const void* const* B, void* con
       if (e == 1 && (b_mn[i] || N[i] != 2 * half[i])) return LB_ERR_SHAPE;
       if (e == 2 && N[i] != half[i]) return LB_ERR_SHAPE;
       if (accumulate && accumulate[i]) return LB_ERR_ARG;
+      if (ks == 8) return LB_ERR_SHAPE;
     }
     Problem& p = gp.prob[i];
     // the rows behind the last one of a short matrix are not loaded (what lies in the stage makes rows that are not stored): filling them
@@ -422,16 +429,25 @@ int gemm_split_rope(int n, const void* const* A, const void* const* B, void* con
     tiles += p.tiles_m * (e == 1 ? ceil_div(half[i], HB) : ceil_div(N[i], BN));
     if (tiles * ks > (1 << 30)) return LB_ERR_SHAPE;
   }
-  return ks == 1 ? launch<1>(gp, tiles, (cudaStream_t)stream) : ks == 2 ? launch<2>(gp, tiles, (cudaStream_t)stream) : launch<4>(gp, tiles, (cudaStream_t)stream);
+  cudaStream_t s = (cudaStream_t)stream;
+  switch (ks) {
+    case 1: return launch<1>(gp, tiles, s);
+    case 2: return launch<2>(gp, tiles, s);
+    case 4: return launch<4>(gp, tiles, s);
+    default: return launch<8>(gp, tiles, s);
+  }
 }
 
-// Parts of K (1, 2 or 4) with which this form is modelled to beat the list form of gemm_grouped.cu, or 0.  list_time: the latter's modelled
+// Parts of K (1, 2, 4 or 8) with which this form is modelled to beat the list form of gemm_grouped.cu, or 0.  list_time: the latter's modelled
 // time, in hundredths of a k-block.  Both models are in us and fitted to 189 launches in all forms (16 to 4096 rows, N 768 to 32000, K 16 to
 // 5632; forward, data + weight gradient, activation epilogues; operands from memory): a fixed part, the k-blocks of a CTA, those that
 // it waits for where there are more CTAs than SMs, the CTAs themselves, the bytes.  With the rule none of them is slower than the list form
 // by more than it varies (2 %), they are 1.18x faster on average, and eleven stay up to 24 % behind the better form (the model sees
-// 1000 x 2304 x 768 too late: 12.7, split 10.1).
-int gemm_split_parts(int n, const int* M, const int* N, const int* K, int sms, long long list_time) {
+// 1000 x 2304 x 768 too late: 12.7, split 10.1).  Eight parts are for long reductions of few tiles (four / eight, us: 64 x 768 x 32000 46 / 28, 64 x 2048 x 11264
+// 22 / 16, 64 x 1024 x 8192 16 / 10; where four already fill the chip, 64 x 4096 x 28672, 54 / 60), and not for activations.  `us` (or null) receives the
+// modelled time of the form that is taken.
+int gemm_split_parts(int n, const int* M, const int* N, const int* K, bool activation, int sms, long long list_time, double* us) {
+  if (us) *us = 1e30;
   if (n < 1 || n > MAX_PROBLEMS || sms < 4) return 0;
   double mb = 0;
   long long min_kb = 1LL << 30;
@@ -441,7 +457,7 @@ int gemm_split_parts(int n, const int* M, const int* N, const int* K, int sms, l
   }
   double best = 5.0 + 2.68e-3 * (double)list_time + 0.128 * mb;
   int parts = 0;
-  for (int ks = 1; ks <= 4 && ks <= min_kb; ks *= 2) {
+  for (int ks = 1; ks <= (activation || min_kb < 128 ? 4 : 8) && ks <= min_kb; ks *= 2) {
     double ctas = 0, work = 0, longest = 0;
     for (int i = 0; i < n; i++) {
       const double c = (double)ceil_div(M[i], BM) * ceil_div(N[i], BN) * ks, kb = (double)ceil_div(ceil_div(K[i], BK), ks);
@@ -450,7 +466,9 @@ int gemm_split_parts(int n, const int* M, const int* N, const int* K, int sms, l
       longest = std::max(longest, kb);
     }
     const double t = 3.3 + 0.23 * longest + 0.113 * std::max(0.0, work / sms - longest) + 2.78 * ctas / sms + (ks > 1 ? 1.1 : 0.0) + 0.059 * mb;
-    if (1.03 * t < best) { best = 1.03 * t; parts = ks; }
+    const double margin = ks == 8 ? 1.075 : 1.03;
+    if (margin * t < best) { best = margin * t; parts = ks; }
   }
+  if (us) *us = best;
   return parts;
 }

@@ -36,4 +36,4 @@ int gemm_split_rope(int n, const void* const* A, const void* const* B, void* con
                     const long long* lda, const long long* ldb, const long long* ldc, const int* a_mn, const int* b_mn,
                     const int* accumulate, const int* epi, void* const* C2, const long long* ldc2, const int* half, int ks, const RopeArgs* rope,
                     void* stream);
-int gemm_split_parts(int n, const int* M, const int* N, const int* K, int sms, long long list_time);
+int gemm_split_parts(int n, const int* M, const int* N, const int* K, bool activation, int sms, long long list_time, double* us);

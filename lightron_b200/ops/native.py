@@ -64,6 +64,7 @@ _SIGNATURES = {
     "lb_gemm_grouped_plan": [_I, _P, _P, _P, _I, _P],
     "lb_gemm_grouped_ctas_per_tile": [_I, _P, _P, _P, _I],
     "lb_gemm_grouped_parts": [_I, _P, _P, _P, _I],
+    "lb_gemm_grouped_apart": [_I, _P, _P, _P, _I],
     "lb_gemm_ag": [_P, _P, _I, _I, _I, _L, _L, _I, _I, _I, _P, _L, _P, _P, ctypes.c_uint, _I, _P],
     "lb_gemm_rs": [_P, _P, _I, _I, _I, _L, _L, _I, _I, _I, _P, _P, ctypes.c_uint, _P, _L, _P],
     "lb_moe_status": [_P],

@@ -235,6 +235,22 @@ def test_gemm_forms(M, N, K, n, form, a_mn, b_mn):
             assert _rel(out, want + c0.double() if acc else want) < 5e-3
 
 
+@pytest.mark.parametrize("T,n,k,apart", [(16, 16384, 264, 1), (72, 16384, 520, 1), (264, 11264, 2048, 0), (1000, 2304, 768, 0), (72, 768, 768, 0)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_weight_and_data_gradient_launches(T, n, k, apart, accumulate):
+    """Both gradients of a linear layer, in one launch or, over few rows, in one each."""
+    import ctypes
+    from lightron_b200.ops import functional as OF, native
+    IA = ctypes.c_int * 2
+    assert native.require().lb_gemm_grouped_apart(2, IA(n, T), IA(k, k), IA(T, n), native.sm_count()) == apart
+    x, w, dy, old = _rand(T, k, seed=1), _rand(n, k, seed=2), _rand(T, n, seed=3), _rand(n, k, seed=4)
+    dw = old.clone()
+    _, dx = OF.gemm_grouped([(dy, x, True, True, dw, accumulate), (dy, w, False, True, None, False)])
+    _status_ok()
+    want = dy.double().t() @ x.double()
+    assert _rel(dw, want + old.double() if accumulate else want) < 5e-3 and _rel(dx, dy.double() @ w.double()) < 5e-3
+
+
 def _gemm_split(ks, a, b, a_mn, b_mn, out, accumulate, epi=0, c2=None, half=0):
     """The split form of a GEMM launch, whatever the rule says about these sizes."""
     import ctypes
@@ -270,6 +286,27 @@ def test_gemm_split_tiles(ks, M, N, K, a_mn, b_mn):
     _gemm_split(ks, *ops, a_mn, b_mn, acc, True)
     _status_ok()
     assert _rel(buf[:M], want) < 5e-3 and _rel(acc, want + c0.double()) < 5e-3 and bool((buf[M:] == 7.0).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 8, 513), (72, 200, 1032), (136, 64, 4104), (260, 136, 520)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_gemm_split_in_eight(M, N, K, a_mn, b_mn):
+    """Each CTA of a cluster finishes eight columns; eight parts of one and more k-blocks, ragged ones; activations are refused."""
+    from lightron_b200.ops import native
+    if a_mn and M % 8:
+        M = M // 8 * 8 + 8
+    pad = (K + 7) // 8 * 8
+    a, b, c0 = _rand(M, pad, seed=1)[:, :K], _rand(N, pad, seed=2)[:, :K], _rand(M, N, seed=3)
+    ops = (a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b)
+    want = a.double() @ b.double().t()
+    buf = torch.full((M + 8, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    _gemm_split(8, *ops, a_mn, b_mn, buf[:M], False)
+    acc = c0.clone()
+    _gemm_split(8, *ops, a_mn, b_mn, acc, True)
+    _status_ok()
+    assert _rel(buf[:M], want) < 5e-3 and _rel(acc, want + c0.double()) < 5e-3 and bool((buf[M:] == 7.0).all())
+    with pytest.raises(native.NativeError):
+        _gemm_split(8, a, b, False, False, buf[:M], False, 1, acc, N // 16 * 8)
 
 
 @pytest.mark.parametrize("ks", [1, 2, 4])

@@ -22,15 +22,26 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// CLUSTER: the acquire reaches over the cluster, for phases that other CTAs' threads complete (st_cluster_v4).
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if constexpr (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
   return ok != 0;
 }
 // Non-blocking probe of a phase: unlike try_wait, which may suspend the thread for a
@@ -53,9 +64,10 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
 // Kernels that contain waits for OTHER GPUs set extra_ms to the limit of those waits plus a margin,
 // so that the roles of the pipeline that merely wait for the role that waits for the peer do not give
 // up before it does; kernels without such waits set 0.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   for (uint32_t i = 0; i < WAIT_LIMIT; i++) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     if ((i & 255u) == 255u && *abort_flag) return false;
   }
   const unsigned long long extra_ns = (unsigned long long)(unsigned)abort_flag[1] * 1000000ull;
@@ -63,7 +75,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     unsigned long long t0, t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
     for (;;) {
-      if (mbar_try_wait(bar, parity)) return true;
+      if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
       if (*abort_flag) return false;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
       if (t - t0 > extra_ns) break;
@@ -130,8 +142,8 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* v, 
                "r"(v[2]), "r"(v[3]), "r"(bar)
                : "memory");
 }
-__device__ __forceinline__ void fence_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// (orders no memory: for a CTA that must not end while others still send to it)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Arrive on the barrier at the same offset in the cluster's CTA 0.
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {

@@ -53,6 +53,7 @@ struct FaBwdParams {
   int kv_brows;   // rows between consecutive batches in the K/V tensor maps (>= Sk)
   int chunk;      // query blocks of a CTA, or 0: all of its key block, whose dK / dV it writes
   float *dk_acc, *dv_acc;      // with chunk: fp32 sums, in the layout of dq_acc
+  bool alone;                  // one key block, not in parts: its CTAs write dQ, and nothing uses dq_acc
 };
 
 // (batch, kv head) pairs whose key blocks are ordered together: enough to keep the chip busy to the end,
@@ -161,9 +162,11 @@ __global__ void fa_bwd_prep_kernel(const FaBwdParams p) {
       const long long bi = idx / p.hq;
       b = (int)(bi / Sp);
       i = (int)(bi % Sp);
-      float4* z = reinterpret_cast<float4*>(p.dq_acc + (idx * TPR + sub) * 8);
-      z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-      z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!p.alone) {
+        float4* z = reinterpret_cast<float4*>(p.dq_acc + (idx * TPR + sub) * 8);
+        z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+        z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
       if (i < p.Sq) {
         const long long row = (long long)b * p.Sq + i;
         float a[8], e[8];
@@ -193,12 +196,16 @@ __host__ __device__ __forceinline__ int bwd_parts(int mb_first, int n_mblocks, i
   return its ? (its + chunk - 1) / chunk : 1;
 }
 
-template <int D, bool PARTS>      // PARTS: with chunk
+// What a CTA leaves: WHOLE dK and dV of a key block, and its share of dQ, added to the fp32 sums; PARTS (with chunk) its share of all three; ALONE
+// all three.
+enum : int { WHOLE, PARTS_OF, ALONE };
+template <int D, int FORM>
 __global__ void __launch_bounds__(512, 1)
 fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                  const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tdk,
                  const __grid_constant__ CUtensorMap tdv, const FaBwdParams p) {
   using C = BwdCfg<D>;
+  constexpr bool PARTS = FORM == PARTS_OF;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::NBAR);
@@ -389,7 +396,7 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     const int quad = warp & 3;
     const uint32_t tdq = tmem_base + ((uint32_t)(quad * 32) << 16) + C::COL_DQ;
     uint8_t* stg = smem + C::OFF_STG + quad * 2 * C::STG_BYTES;
-    float* tile = p.dq_acc + (((long long)b * p.hq + h_first) * n_mblocks + mb_start) * (128 * D) + quad * (32 * D);
+    [[maybe_unused]] float* tile = p.dq_acc + (((long long)b * p.hq + h_first) * n_mblocks + mb_start) * (128 * D) + quad * (32 * D);
     bool ok = true;
     int mb = mb_start;
     for (int it = 0; it < total_it; it++) {
@@ -402,6 +409,17 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(dq_free);
+      if constexpr (FORM == ALONE) {
+        // the query block's dQ is complete: a row per lane
+        const int row = mb * C::BM + quad * 32 + lane;
+        if (row < p.Sq) {
+          bf16* o = p.dq + ((long long)b * p.Sq + row) * p.dq_ts + (long long)(h_first + it / n_mblocks) * D;
+#pragma unroll
+          for (int k = 0; k < D / 8; k++) *reinterpret_cast<uint4*>(o + k * 8) = pack8(reinterpret_cast<const float*>(r) + k * 8);
+        }
+        if (++mb == n_mblocks) mb = 0;
+        continue;
+      }
 #pragma unroll
       for (int c = 0; c < D / 32; c++) {
         uint8_t* sp = stg + (c & 1) * C::STG_BYTES;
@@ -638,7 +656,7 @@ int launch_fa_bwd(const void* q, const void* k, const void* v, const FaBwdParams
   static bool attr = false;
   if (!attr) {
     // the register split must fit in what the launch allocates, or it would wait for registers that nobody gives back
-    for (auto fn : {fa_bwd_tc_kernel<D, false>, fa_bwd_tc_kernel<D, true>}) {
+    for (auto fn : {fa_bwd_tc_kernel<D, WHOLE>, fa_bwd_tc_kernel<D, PARTS_OF>, fa_bwd_tc_kernel<D, ALONE>}) {
       cudaFuncAttributes fa;
       if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess || (fa.numRegs + 7) / 8 * 8 != 128) return LB_ERR_LAUNCH;
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
@@ -652,7 +670,8 @@ int launch_fa_bwd(const void* q, const void* k, const void* v, const FaBwdParams
   const long long rows_per_block = 256 / (D / 8), cap = lb_num_sms() * 16;
   const long long pblocks = (rows + rows_per_block - 1) / rows_per_block;
   LB_LAUNCH(fa_bwd_prep_kernel<D>, (int)(pblocks < cap ? pblocks : cap), 256, 0, s, p);
-  LB_LAUNCH(p.chunk ? fa_bwd_tc_kernel<D, true> : fa_bwd_tc_kernel<D, false>, (unsigned)grid, C::NTHREADS, C::SMEM, s, tq, tk, tv, tdo, tdk, tdv, p);
+  LB_LAUNCH(p.chunk ? fa_bwd_tc_kernel<D, PARTS_OF> : p.alone ? fa_bwd_tc_kernel<D, ALONE> : fa_bwd_tc_kernel<D, WHOLE>, (unsigned)grid, C::NTHREADS, C::SMEM, s, tq, tk, tv, tdo, tdk, tdv, p);
+  if (p.alone) return LB_OK;
   const long long kv_rows_acc = p.chunk ? 2LL * p.B * ((p.Sk + 127) / 128 * 128) * p.hkv : 0;
   const long long cblocks = ((rows + kv_rows_acc) * (D / 32) + 255) / 256;
   LB_LAUNCH(p.chunk ? fa_dq_convert_kernel<D, true> : fa_dq_convert_kernel<D, false>, (int)(cblocks < cap ? cblocks : cap), 256, 0, s, p);
@@ -703,11 +722,15 @@ static int flash_bwd_tc_impl(int kv_brows, const void* q, const void* k, const v
     return LB_ERR_ARG;
   FaBwdParams p{(const bf16*)o, (const bf16*)dout, (const float*)lse, (float*)stats, (float*)dq_acc,
                 (bf16*)dq, (bf16*)dk, (bf16*)dv, B, Sq, Sk, hq, hkv, o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal,
-                kv_brows, 0, nullptr, nullptr};
+                kv_brows, 0, nullptr, nullptr, false};
   if (dkv_acc && (p.chunk = bwd_chunk(B, Sq, Sk, hq, hkv, causal, lb_num_sms())) > 0) {
     p.dk_acc = (float*)dkv_acc;
     p.dv_acc = p.dk_acc + (long long)B * hkv * ((Sk + 127) / 128) * 128 * d;
   }
+  // Up to 128 keys a query block's dQ comes from one CTA, which writes it: no sums to clear, to add to and to convert.  Forward and backward, us, before / now,
+  // d 64: B4 S128 12 heads inside its layer 58.5 / 57.0, B8 32 heads 29 / 25, B32 32q/8kv 66.6 / 55, B64 16 heads 97 / 83; B8 S100 16 heads d128 26 / 22.  (In
+  // parts, which few CTAs with long loops get, dK and dV have to be converted all the same.)
+  p.alone = Sk <= 128 && !p.chunk;
   cudaStream_t s = (cudaStream_t)stream;
   switch (d) {
     case 64: return launch_fa_bwd<64>(q, k, v, p, q_ts, k_ts, v_ts, s);

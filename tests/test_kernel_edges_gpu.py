@@ -181,6 +181,35 @@ def test_attention_backward_in_parts(B, Sq, Sk, hq, hkv, causal, d, parts):
 
 
 @pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("B,Sq,Sk,hq,hkv,causal", [
+    (1, 1, 1, 1, 1, True),
+    (2, 128, 128, 3, 3, True),
+    (3, 70, 101, 2, 2, True),
+    (40, 129, 128, 8, 4, False),             # two query blocks of two heads in a CTA, the second block of one row
+    (2, 33, 127, 4, 4, False),
+    (40, 200, 5, 4, 4, False),
+])
+def test_attention_backward_of_one_key_block(B, Sq, Sk, hq, hkv, causal, d):
+    """Up to 128 keys dQ is written by the CTA of its key block: against 64 bits, into rows with a stride, of which nothing else is written."""
+    from lightron_b200.ops import functional as OF, native
+    assert native.require().lb_flash_bwd_chunk(B, Sq, Sk, hq, hkv, int(causal), native.sm_count()) == 0
+    q, do = _rand(B, Sq, hq, d, seed=1), _rand(B, Sq, hq, d, seed=4)
+    k, v = _rand(B, Sk, hkv, d, seed=2), _rand(B, Sk, hkv, d, seed=3)
+    o, lse = OF.flash_fwd_native(q, k, v, causal, d ** -0.5)
+    buf = [torch.full((B * n + 128, h * d + 8), 7.0, dtype=torch.bfloat16, device="cuda") for n, h in ((Sq, hq), (Sk, hkv), (Sk, hkv))]
+    out = [t[:B * n, :-8].unflatten(0, (B, n)).unflatten(2, (-1, d)) for t, n in zip(buf, (Sq, Sk, Sk))]
+    OF.flash_bwd_native(q, k, v, o, lse, do, causal, d ** -0.5, *out)
+    _status_ok()
+    want = _attention64(q, k, v, do, causal)[1:]
+    if Sk == 1:                              # one key: its weight is one, and dQ and dK are rounding
+        want = [torch.zeros_like(want[0]), torch.zeros_like(want[1]), want[2]]
+        assert max(float(g.abs().max()) for g in out[:2]) < 1e-3      # (sums of d products of some 1, in fp32)
+    for name, g, w in zip(("dq", "dk", "dv"), out, want):
+        assert not w.any() or _rel(g, w) < 1e-2, name
+    assert all(bool((t[B * n:] == 7.0).all() and (t[:, -8:] == 7.0).all()) for t, n in zip(buf, (Sq, Sk, Sk)))
+
+
+@pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 def test_attention_bad_scores_stay_in_their_rows(d, bad):
     """A key that is not finite spoils the rows that see it, whichever unit computes its exponentials, and no other."""

@@ -36,13 +36,18 @@ template <int KS>
 struct Cfg {
   static constexpr int STAGES = KS >= 4 ? 3 : 4;
   static constexpr int G = 8 / KS, NG = KS == 8 ? 1 : HB / 8 / KS, NB = G / NG;      // groups of a CTA: NB blocks, NG in each
+  // Groups of a block that a warp finishes.  Where a CTA has one of each block, one warp takes the first block's and one the second's; the pair (activation), or
+  // the only one, is the first warp's.
+  static constexpr int GW = NG > 1 ? NG / 2 : 1;
   static constexpr int RECV_BYTES = (KS - 1) * BM * G * 8 * 4;
   static constexpr int OFF_RECV = STAGES * STAGE_BYTES;
   static constexpr int OFF_BAR = OFF_RECV + RECV_BYTES;
   static constexpr int SMEM_BYTES = OFF_BAR + 256;
   static_assert(2 * (SMEM_BYTES + 1024) <= 233472, "two CTAs per SM");
 };
-constexpr int NUM_THREADS = 192;
+// Warps 0 and 1 load and multiply, the others finish, two for each 32 rows: a warp's epilogue is one chain of instructions, not a stream that the SM's units
+// bound, so half of the columns take half of the time.  @@EW@@
+constexpr int NUM_THREADS = 320;
 constexpr int MAX_PROBLEMS = 2;
 constexpr int PREFETCH = 16;                             // k-blocks of B that a CTA asks for ahead of its start (38 MB of all CTAs that run at a time)
 
@@ -123,7 +128,7 @@ __device__ __forceinline__ bool multiply(uint32_t d_tmem, int n_kb, uint32_t sme
 template <int KS>
 __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid_constant__ Params gp) {
   using C = Cfg<KS>;
-  constexpr int STAGES = C::STAGES, NG = C::NG, NB = C::NB;
+  constexpr int STAGES = C::STAGES, NG = C::NG, NB = C::NB, GW = C::GW;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t smem_base = bw::smem_u32(smem);
   const uint32_t bar_base = smem_base + C::OFF_BAR;
@@ -143,9 +148,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
   // the tile's two blocks of columns: neighbours, or the gate and the up columns of the same index
   const int n0 = pr.epi == 1 ? tn * HB : tn * BN;
   const int n1 = pr.epi == 1 ? pr.half + n0 : n0 + HB;
-  // group g of its block b: which block, and the first column in it
+  // group g of this warp in block b: which block, its place among the CTA's groups of a block, its first column, and whether the warp has that block
+  const int set = warp >= 6 ? 1 : 0;
   auto block_of = [&](int b) { return KS == 8 ? rank >> 2 : b; };
-  auto column_of = [&](int g) { return KS == 8 ? (rank & 3) * 8 : (rank * NG + g) * 8; };
+  auto place_of = [&](int g) { return NG > 1 ? set * GW + g : g; };
+  auto column_of = [&](int g) { return KS == 8 ? (rank & 3) * 8 : (rank * NG + place_of(g)) * 8; };
+  auto mine = [&](int b) { return NG > 1 || (NB == 1 || pr.epi == 1 ? set == 0 : set == b); };
   const int kb0 = (int)((long long)pr.num_kb * rank / KS), n_kb = (int)((long long)pr.num_kb * (rank + 1) / KS) - kb0;
 
   if (threadIdx.x == 64) { bw::prefetch_tmap(&gp.ta[pi]); bw::prefetch_tmap(&gp.tb[pi]); }
@@ -188,7 +196,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
   const int row = m0 + row_in;
   const bool row_ok = row < pr.M;
   const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
-  float rot[NB][NG][8];                                        // epi 4: cosines and sines of this row's columns, loaded ahead
+  float rot[NB][GW][8];                                        // epi 4: cosines and sines of this row's columns, loaded ahead
   if (warp == 0) {
     if (ok && bw::elect_one()) {
       const CUtensorMap *ta = &gp.ta[pi], *tb = &gp.tb[pi];
@@ -217,9 +225,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
 #pragma unroll
       for (int b = 0; b < NB; b++)
 #pragma unroll
-        for (int g = 0; g < NG; g++) {
+        for (int g = 0; g < GW; g++) {
           const int col = (block_of(b) ? n1 : n0) + column_of(g);
-          if (col < gp.rope.cols) rope_load8(gp.rope, pos, col, rot[b][g]);
+          if (mine(b) && col < gp.rope.cols) rope_load8(gp.rope, pos, col, rot[b][g]);
         }
     }
     if (ok && !bw::mbar_wait(tfull, 0, abort_flag)) { ok = false; give_up(abort_flag, 3u); }
@@ -230,35 +238,33 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
 
   if constexpr (KS > 1) {
     if (warp >= 2 && ok) {
-      // 8 columns at a time to the CTA that finishes them
-      const uint32_t mine = smem_base + C::OFF_RECV + (uint32_t)(row_in * 16);
+      // 8 columns at a time to the CTA that finishes them: a block of a quad's rows from either of its warps
+      const uint32_t here = smem_base + C::OFF_RECV + (uint32_t)(row_in * 16);
+      uint32_t r[32];
+      bw::tmem_ld32(taddr + set * HB, r);
+      bw::tmem_ld_wait();
 #pragma unroll
-      for (int b = 0; b < 2; b++) {
-        uint32_t r[32];
-        bw::tmem_ld32(taddr + b * HB, r);
-        bw::tmem_ld_wait();
-#pragma unroll
-        for (int g = 0; g < 4; g++) {
-          const int s = KS == 8 ? b * 4 + g : g / NG;          // the receiver; its place for this part: parts in order, its own left out
-          if (s == rank) continue;
-          const int slot = rank < s ? rank : rank - 1;
-          const int to = KS == 8 ? 0 : b * NG + g % NG;
-          const uint32_t dst = bw::cluster_addr(mine + (uint32_t)((slot * C::G + to) * 8 * BM * 4), s);
-          const uint32_t bar = bw::cluster_addr(received, s);
-          bw::st_cluster_v4(dst, r + g * 8, bar);
-          bw::st_cluster_v4(dst + BM * 16, r + g * 8 + 4, bar);
-        }
+      for (int g = 0; g < 4; g++) {
+        const int s = KS == 8 ? set * 4 + g : g / NG;          // the receiver; its place for this part: parts in order, its own left out
+        if (s == rank) continue;
+        const int slot = rank < s ? rank : rank - 1;
+        const int to = KS == 8 ? 0 : set * NG + g % NG;
+        const uint32_t dst = bw::cluster_addr(here + (uint32_t)((slot * C::G + to) * 8 * BM * 4), s);
+        const uint32_t bar = bw::cluster_addr(received, s);
+        bw::st_cluster_v4(dst, r + g * 8, bar);
+        bw::st_cluster_v4(dst + BM * 16, r + g * 8 + 4, bar);
       }
     }
     __syncwarp();
     bw::cluster_arrive();
   }
   if (warp >= 2 && ok) {
-    float f[NB][NG][8];
+    float f[NB][GW][8];
 #pragma unroll
     for (int b = 0; b < NB; b++)
 #pragma unroll
-      for (int g = 0; g < NG; g++) bw::tmem_ld8(taddr + block_of(b) * HB + column_of(g), reinterpret_cast<uint32_t*>(f[b][g]));
+      for (int g = 0; g < GW; g++)
+        if (mine(b)) bw::tmem_ld8(taddr + block_of(b) * HB + column_of(g), reinterpret_cast<uint32_t*>(f[b][g]));
     bw::tmem_ld_wait();
     if constexpr (KS > 1) {
       // The sums order nothing but themselves: an acquire on their barrier, not a fence over the cluster beside it, and a barrier at the end that only keeps the CTA
@@ -269,14 +275,15 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
 #pragma unroll
       for (int b = 0; b < NB; b++)
 #pragma unroll
-        for (int g = 0; g < NG; g++) {
+        for (int g = 0; g < GW; g++) {
+          if (!mine(b)) continue;
           float own[8], sum[8];
 #pragma unroll
           for (int i = 0; i < 8; i++) { own[i] = f[b][g][i]; sum[i] = 0.f; }
 #pragma unroll
           for (int s = 0; s < KS; s++) {                       // in the order of the parts
             const int slot = s < rank ? s : s - 1;
-            const float4* q = in + (size_t)((s == rank ? 0 : slot) * C::G + b * NG + g) * 2 * BM;
+            const float4* q = in + (size_t)((s == rank ? 0 : slot) * C::G + b * NG + place_of(g)) * 2 * BM;
             const float4 x = q[0], y = q[BM];
             const float part[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
 #pragma unroll
@@ -289,12 +296,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
     const int n_end = pr.epi == 1 ? pr.half : pr.N;
     if (row_ok && ok) {
 #pragma unroll
-      for (int g = 0; g < NG; g++) {
+      for (int g = 0; g < GW; g++) {
         const int cc = column_of(g);                           // column inside a block
         if (NB == 2 && pr.epi == 1) {
           // silu(g) * u is computed from the ROUNDED values (what a separate pass over the stored matrix would see)
           const int col = n0 + cc;
-          if (col < n_end) {
+          if (mine(0) && col < n_end) {
             const uint4 pg = pack8(f[0][g]), pu = pack8(f[NB - 1][g]);
             if (pr.C) {
               bf16* grow = pr.C + (size_t)row * pr.ldc + col;
@@ -313,7 +320,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
 #pragma unroll
         for (int b = 0; b < NB; b++) {
           const int col = (block_of(b) ? n1 : n0) + cc;
-          if (col >= n_end) continue;
+          if (!mine(b) || col >= n_end) continue;
           bf16* dst = pr.C + (size_t)row * pr.ldc + col;
           if (pr.epi == 2) {
             const bf16* gu = pr.C2 + (size_t)row * pr.ldc2 + col;

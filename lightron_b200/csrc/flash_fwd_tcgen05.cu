@@ -557,6 +557,194 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   }
 }
 
+// One key block (Sk <= 128) and no more tiles than run at a time: a launch is then one chain from the loads to the stores, and what it takes is the instructions
+// of a softmax warp, straight-line code for its columns that mostly comes from L2.  So a row is two threads', 64 keys each, in eight warps: maxima and sums meet in
+// shared memory, P takes the columns of S.  The products, the exponentials and the order of the sums are those of fa_fwd_tc_kernel: the results are the same
+// bits.  fa_fwd_tc_kernel / this, us, as graphs: 12 layers of 128 tokens, 12 heads of 64, 455 / 411; forward and backward of 4 x 128 tokens, 12 heads of 64 15.6 / 14.4, of
+// 8 x 100, 16 heads of 128 20.5 / 18.5; the layer around the former 54.7 / 52.6.  With more tiles than run at a time the other kernel's loads and scores of a tile under
+// the last one's softmax count for more.
+constexpr int FA_ONE_THREADS = 320;
+__device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+template <int D>
+struct FaOneCfg {
+  static constexpr int ATOMS = D / 64, SLOT_BYTES = 128 * 128;
+  static constexpr int COL_S = 0, COL_P = 0, COL_O = 128, TMEM_COLS = 256;
+  static constexpr int OFF_Q = 0, OFF_K = ATOMS * SLOT_BYTES, OFF_V = 2 * ATOMS * SLOT_BYTES;
+  static constexpr int OFF_MAX = 3 * ATOMS * SLOT_BYTES;        // [2][128] maxima, then [2][128] x 4 sums
+  static constexpr int OFF_SUM = OFF_MAX + 2 * 128 * 4, OFF_BAR = OFF_SUM + 2 * 128 * 16;
+  static constexpr int SMEM = OFF_BAR + 64;
+};
+static_assert(FaOneCfg<128>::SMEM <= 115712, "two CTAs per SM");
+
+template <int D>
+__global__ void __launch_bounds__(FA_ONE_THREADS, 2)
+fa_fwd_one_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv, const FaFwdParams p) {
+  using C = FaOneCfg<D>;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform over the warp)
+  const uint32_t sbase = smem_u32(smem);
+  if (sbase & 1023u) {                                       // the swizzled tiles need it; nothing has been started yet
+    if (threadIdx.x == 0) atomicExch(&g_fa_status[0], 4u);
+    return;
+  }
+  const uint32_t qk_full = sbase + C::OFF_BAR, v_full = qk_full + 8, s_full = qk_full + 16, p_full = qk_full + 24, o_full = qk_full + 32;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + 40);
+  int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);      // {abort, extra wait in ms}: see bw::mbar_wait
+  volatile int* abort_flag = s_abort;
+  const int m0 = (int)blockIdx.y * 128, bh = (int)blockIdx.x;
+  const int b = p.by_hq.div(bh), h = bh - b * p.hq, hk = p.by_rep.div(h);
+  if (threadIdx.x == 0) {
+    s_abort[0] = s_abort[1] = 0;
+    mbar_init(qk_full, 1);
+    mbar_init(v_full, 1);
+    mbar_init(s_full, 1);
+    mbar_init(p_full, 8);
+    mbar_init(o_full, 1);
+    mbar_init_fence();
+    prefetch_tmap(&tq); prefetch_tmap(&tk); prefetch_tmap(&tv);
+  }
+  if (warp == 1) tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  grid_go();
+  grid_wait();
+
+  if (warp == 0) {
+    if (elect_one()) {
+      const int row = b * p.kv_brows;
+      mbar_expect_tx(qk_full, 2 * C::ATOMS * C::SLOT_BYTES);
+#pragma unroll
+      for (int a = 0; a < C::ATOMS; a++) {
+        tma_load_2d(sbase + C::OFF_Q + a * C::SLOT_BYTES, &tq, h * D + a * 64, b * p.Sq + m0, qk_full);
+        tma_load_2d(sbase + C::OFF_K + a * C::SLOT_BYTES, &tk, hk * D + a * 64, row, qk_full);
+      }
+      mbar_expect_tx(v_full, C::ATOMS * C::SLOT_BYTES);
+#pragma unroll
+      for (int half = 0; half < 2; half++)
+#pragma unroll
+        for (int a = 0; a < C::ATOMS; a++)                   // boxes 64 keys x 64 columns
+          tma_load_2d(sbase + C::OFF_V + (half * C::ATOMS + a) * 8192, &tv, hk * D + a * 64, row + half * 64, v_full);
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc_s = make_idesc(128, 128, 0, 0), idesc_o = make_idesc(128, D, 0, 1);
+      const uint64_t qa = make_desc(sbase + C::OFF_Q, 16, 1024), ka = make_desc(sbase + C::OFF_K, 16, 1024), va = make_desc(sbase + C::OFF_V, 8192, 1024);
+      bool ok = mbar_wait(qk_full, 0, abort_flag);
+      if (ok) {
+        fence_after();
+#pragma unroll
+        for (int i = 0; i < D / 16; i++) {
+          const uint64_t at = (uint64_t)(((i >> 2) * C::SLOT_BYTES + (i & 3) * 32) >> 4);
+          umma_bf16(tmem_base + C::COL_S, qa + at, ka + at, idesc_s, i ? 1u : 0u);
+        }
+        umma_commit(s_full);
+        ok = mbar_wait(v_full, 0, abort_flag) && mbar_wait(p_full, 0, abort_flag);
+      }
+      if (ok) {
+        fence_after();
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          umma_bf16_ta(tmem_base + C::COL_O, tmem_base + C::COL_P + 8u * i, va + (uint64_t)(((i >> 2) * C::ATOMS * 8192 + (i & 3) * 2048) >> 4), idesc_o, i ? 1u : 0u);
+        umma_commit(o_full);
+      } else {
+        atomicExch(&g_fa_status[0], 2u);
+      }
+    }
+  } else {
+    const int set = warp >= 6 ? 1 : 0, quad = warp & 3;
+    const int rit = quad * 32 + lane, row = m0 + rit;        // query row in the tile, and in the sequence
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
+    float* mx = reinterpret_cast<float*>(smem + C::OFF_MAX);
+    float4* sums = reinterpret_cast<float4*>(smem + C::OFF_SUM);
+    const float sl2 = p.scale * 1.4426950408889634f;
+    const f32x2 sl2x2 = pack2(sl2, sl2);
+    const int c0 = set * 64;
+    const int lim = (p.causal ? min(p.Sk - 1, row + p.Sk - p.Sq) : p.Sk - 1) - c0;   // last visible column
+    uint32_t r[64];
+    bool ok = __all_sync(0xffffffffu, mbar_wait(s_full, 0, abort_flag));
+    float m = -INFINITY;
+    if (ok) {
+      fence_after();
+      tmem_ld32(lane_addr + C::COL_S + c0, r);
+      tmem_ld32(lane_addr + C::COL_S + c0 + 32, r + 32);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 64; i++)
+        if (i > lim) r[i] = 0xff800000u;                     // -inf
+      float mx4[4] = {m, m, m, m};
+#pragma unroll
+      for (int i = 0; i < 64; i += 2) mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+      m = max2(max2(mx4[0], mx4[1]), max2(mx4[2], mx4[3]));
+    }
+    mx[set * 128 + rit] = m;
+    fence_before();
+    named_sync(1, 256);                                      // (whether or not the wait ended well; S has been read)
+    fence_after();
+    m = max2(mx[rit], mx[128 + rit]);
+    // (a row with a score of +inf has no softmax: NaN, as inf - inf gives)
+    const float m_s = m == -INFINITY ? 0.f : (m == INFINITY ? __int_as_float(0x7fffffff) : m * sl2);
+    if (ok) {
+      const f32x2 nms2 = pack2(-m_s, -m_s);
+      f32x2 rs2[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
+      uint32_t pr[32];
+#pragma unroll
+      for (int c = 0; c < 32; c++) {
+        float e0, e1;
+        unpack2(fma2(pack2(__uint_as_float(r[2 * c]), __uint_as_float(r[2 * c + 1])), sl2x2, nms2), e0, e1);
+        e0 = exp2f(e0);
+        e1 = exp2f(e1);
+        rs2[c & 1] = add2(rs2[c & 1], pack2(e0, e1));
+        bf162 pk = __floats2bfloat162_rn(e0, e1);
+        pr[c] = *reinterpret_cast<uint32_t*>(&pk);
+      }
+      tmem_st32(lane_addr + C::COL_P + set * 32, pr);
+      tmem_st_wait();
+      float4 s4;
+      unpack2(rs2[0], s4.x, s4.y);
+      unpack2(rs2[1], s4.z, s4.w);
+      sums[set * 128 + rit] = s4;
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+    }
+    named_sync(1, 256);
+    const float4 x = sums[rit], y = sums[128 + rit];
+    const float l = (x.x + y.x + (x.y + y.y)) + (x.z + y.z + (x.w + y.w));
+    ok = ok && mbar_wait(o_full, 0, abort_flag);
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok) {
+      fence_after();
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      uint32_t o[D / 2];
+#pragma unroll
+      for (int c = 0; c < D / 64; c++) tmem_ld32(lane_addr + C::COL_O + set * (D / 2) + c * 32, o + c * 32);
+      tmem_ld_wait();
+      if (row < p.Sq) {
+        bf16* out = p.o + ((long long)b * p.Sq + row) * p.o_ts + (long long)h * D + set * (D / 2);
+#pragma unroll
+        for (int g = 0; g < D / 16; g++) {
+          float f[8];
+#pragma unroll
+          for (int i = 0; i < 8; i++) f[i] = __uint_as_float(o[g * 8 + i]) * inv;
+          *reinterpret_cast<uint4*>(out + g * 8) = pack8(f);
+        }
+        if (set == 0) p.lse[((long long)b * p.hq + h) * p.Sq + row] = l > 0.f ? m * p.scale + logf(l) : -INFINITY;
+      }
+    } else if (lane == 0) {
+      atomicExch(&g_fa_status[0], 3u);
+    }
+  }
+
+  fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    fence_after();
+    tmem_dealloc(tmem_base, C::TMEM_COLS);
+  }
+}
+
 template <int D>
 int launch_fa_fwd(const void* q, const void* k, const void* v, FaFwdParams p, const FaPush& push, long long q_ts,
                   long long k_ts, long long v_ts, cudaStream_t s) {
@@ -574,6 +762,7 @@ int launch_fa_fwd(const void* q, const void* k, const void* v, FaFwdParams p, co
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, fa_fwd_tc_kernel<D>) != cudaSuccess || (fa.numRegs + 7) / 8 * 8 * 2 < FA_REGS_ISSUE + FA_REGS_SOFTMAX) return LB_ERR_LAUNCH;
     cudaFuncSetAttribute(fa_fwd_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    cudaFuncSetAttribute(fa_fwd_one_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaOneCfg<D>::SMEM);
     attr = true;
   }
   p.tiles_x = (p.Sq + 127) / 128;
@@ -591,6 +780,8 @@ int launch_fa_fwd(const void* q, const void* k, const void* v, FaFwdParams p, co
   p.by_rep.set((unsigned)(p.hq / p.hkv));
   // (a mover's place is not to be taken; with all tiles resident at once there is none to take)
   p.steal = push.n_mov == 0 && grid > 2 * lb_num_sms();
+  if (p.Sk <= 128 && push.n_mov == 0 && !p.kv_flags && !p.steal)
+    return lb_launch_cluster(true, 1, fa_fwd_one_kernel<D>, dim3((unsigned)(p.hq * p.B), (unsigned)p.tiles_x), FA_ONE_THREADS, FaOneCfg<D>::SMEM, s, tq, tk, tv, p);
   return lb_launch_cluster(push.n_mov == 0 && !p.kv_flags, 1, fa_fwd_tc_kernel<D>, (unsigned)grid, FA_FWD_THREADS, C::SMEM, s, tq, tk, tv, to, p, push);
 }
 

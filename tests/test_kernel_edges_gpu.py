@@ -210,6 +210,26 @@ def test_attention_backward_of_one_key_block(B, Sq, Sk, hq, hkv, causal, d):
 
 
 @pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("Sq,Sk,hq,hkv,causal", [(1, 1, 1, 1, True), (128, 128, 4, 2, True), (70, 101, 2, 1, True), (65, 128, 2, 2, True), (129, 64, 2, 1, False),
+                                                  (300, 65, 4, 4, False), (5, 127, 1, 1, False)])
+def test_attention_of_one_key_block(Sq, Sk, hq, hkv, causal, d):
+    """Up to 128 keys and few tiles: two threads a row.  The same bits as where tiles are many, for finite scores and others."""
+    from lightron_b200.ops import functional as OF, native
+    n = 2 * native.sm_count() // (hq * ((Sq + 127) // 128)) + 1      # batches with which the other kernel runs
+    q, k, v = _rand(2, Sq, hq, d, seed=1), _rand(2, Sk, hkv, d, seed=2), _rand(2, Sk, hkv, d, seed=3)
+    for bad in (None, float("inf"), float("nan"), -float("inf")):
+        if bad is not None:
+            k[1, Sk // 2, 0, 0] = bad
+        o, lse = OF.flash_fwd_native(q, k, v, causal, d ** -0.5)
+        many = OF.flash_fwd_native(*(t.repeat((n + 1) // 2 + 1, 1, 1, 1) for t in (q, k, v)), causal, d ** -0.5)
+        _status_ok()
+        if bad is None:
+            assert _rel(o, _attention64(q, k, v, torch.zeros_like(q), causal)[0]) < 1e-2
+        for g, w in zip((o, lse), many):
+            assert torch.equal(g.nan_to_num(7.0), w[:2].nan_to_num(7.0)) and torch.equal(g.isnan(), w[:2].isnan()), bad
+
+
+@pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 def test_attention_bad_scores_stay_in_their_rows(d, bad):
     """A key that is not finite spoils the rows that see it, whichever unit computes its exponentials, and no other."""

@@ -562,7 +562,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
 // shared memory, P takes the columns of S.  The products, the exponentials and the order of the sums are those of fa_fwd_tc_kernel: the results are the same
 // bits.  fa_fwd_tc_kernel / this, us, as graphs: 12 layers of 128 tokens, 12 heads of 64, 455 / 411; forward and backward of 4 x 128 tokens, 12 heads of 64 15.6 / 14.4, of
 // 8 x 100, 16 heads of 128 20.5 / 18.5; the layer around the former 54.7 / 52.6.  With more tiles than run at a time the other kernel's loads and scores of a tile under
-// the last one's softmax count for more.
+// the last one's softmax count for more (forward alone, d 64: 256 tiles -> 5.4 here, 320 8.3 / 8.7, 1024 14.6 / 18.1, 4096 47 / 74; d 128, 512 tiles 12.1 / 15.0).
 constexpr int FA_ONE_THREADS = 320;
 __device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 template <int D>

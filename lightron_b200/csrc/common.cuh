@@ -118,3 +118,15 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
   for (int i = 0; i < 4; i++) p[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
   return u;
 }
+
+// RoPE of 8 columns: pairs (a, b) to (a c - b s, a s + b c), with four cosines and four sines; `back`: by the opposite angle.  In each sum one product
+// is rounded and the other is not.  Which one is written out, because the compiler chose differently from place to place, and 2e-5 of the bf16
+// results then differed between the kernels: here as rope_kernel has always had it (the first pair, and every pair on the way back, round a s).
+__device__ __forceinline__ void rope_rotate8(const float* cs, float* f, bool back = false) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const float a = f[2 * i], b = f[2 * i + 1], c = cs[i], s = back ? -cs[4 + i] : cs[4 + i];
+    f[2 * i] = __fmaf_rn(a, c, -__fmul_rn(b, s));
+    f[2 * i + 1] = i == 0 || back ? __fmaf_rn(b, c, __fmul_rn(a, s)) : __fmaf_rn(a, s, __fmul_rn(b, c));
+  }
+}

@@ -450,16 +450,12 @@ __global__ void rope_kernel(bf16* __restrict__ t, const float* __restrict__ cosT
     const int s = (int)(tok % S);
     const int pos = positions ? positions[s] : s;
     uint4* p = reinterpret_cast<uint4*>(t + tok * ld + (long long)head * head_dim + v * 8);
-    float f[8], o[8];
+    float f[8], cs[8];
     unpack8(*p, f);
-    const float4 c = *reinterpret_cast<const float4*>(cosT + (size_t)pos * (head_dim >> 1) + v * 4);
-    float4 sn = *reinterpret_cast<const float4*>(sinT + (size_t)pos * (head_dim >> 1) + v * 4);
-    if (inverse) { sn.x = -sn.x; sn.y = -sn.y; sn.z = -sn.z; sn.w = -sn.w; }
-    o[0] = f[0] * c.x - f[1] * sn.x; o[1] = f[0] * sn.x + f[1] * c.x;
-    o[2] = f[2] * c.y - f[3] * sn.y; o[3] = f[2] * sn.y + f[3] * c.y;
-    o[4] = f[4] * c.z - f[5] * sn.z; o[5] = f[4] * sn.z + f[5] * c.z;
-    o[6] = f[6] * c.w - f[7] * sn.w; o[7] = f[6] * sn.w + f[7] * c.w;
-    *p = pack8(o);
+    *reinterpret_cast<float4*>(cs) = *reinterpret_cast<const float4*>(cosT + (size_t)pos * (head_dim >> 1) + v * 4);
+    *reinterpret_cast<float4*>(cs + 4) = *reinterpret_cast<const float4*>(sinT + (size_t)pos * (head_dim >> 1) + v * 4);
+    rope_rotate8(cs, f, inverse != 0);
+    *p = pack8(f);
   }
 }
 

@@ -13,21 +13,12 @@ __device__ __forceinline__ int rope_position(const RopeArgs& r, int row) {
   const int s = row % r.S;
   return r.positions ? r.positions[s] : s;
 }
-// Cosines and sines (4 and 4) of 8 columns of C, from `col` (a multiple of 8), of a row at that position, and the rotation
+// Cosines and sines (4 and 4) of 8 columns of C, from `col` (a multiple of 8), of a row at that position: what rope_rotate8() takes
 __device__ __forceinline__ void rope_load8(const RopeArgs& r, int pos, int col, float* cs) {
   const int at = pos * (r.d >> 1) + ((col % r.d) >> 1);
   *reinterpret_cast<float4*>(cs) = *reinterpret_cast<const float4*>(r.cos + at);
   *reinterpret_cast<float4*>(cs + 4) = *reinterpret_cast<const float4*>(r.sin + at);
 }
-__device__ __forceinline__ void rope_rotate8(const float* cs, float* f) {
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const float a = f[2 * i], b = f[2 * i + 1];
-    f[2 * i] = a * cs[i] - b * cs[4 + i];
-    f[2 * i + 1] = a * cs[4 + i] + b * cs[i];
-  }
-}
-
 extern "C" int lb_gemm_split(int n, const void* const* A, const void* const* B, void* const* C, const int* M, const int* N, const int* K,
                              const long long* lda, const long long* ldb, const long long* ldc, const int* a_mn, const int* b_mn,
                              const int* accumulate, const int* epi, void* const* C2, const long long* ldc2, const int* half, int ks, void* stream);

@@ -380,7 +380,7 @@ def test_gemm_split_activation(ks, T, K, I):
 @pytest.mark.parametrize("placed", [False, True])
 def test_projection_with_rotation(B, S, hq, hkv, d, K, form, placed):
     """The rotation in the epilogue against lb_rope on the projection's output: columns that are rotated and columns that are not, ragged rows,
-    positions of the caller's.  One rounding of the same fp32 values, which a contracted multiply and add may move across a boundary."""
+    positions of the caller's.  One rounding of the same fp32 values (test_rotation_has_the_same_bits_everywhere has their order)."""
     from lightron_b200.ops import functional as OF, native
     N, T = (hq + 2 * hkv) * d, B * S
     assert _form((T, N, K)) == form
@@ -397,6 +397,38 @@ def test_projection_with_rotation(B, S, hq, hkv, d, K, form, placed):
     # a pair's two products cancel at worst: their fp32 rounding against the pair's size, and one unit in the last place of the result
     size = want.float().view(T, -1, 2).norm(dim=-1, keepdim=True).expand(-1, -1, 2).reshape(T, N)
     assert ((got.float() - want.float()).abs() <= 2.0 ** -7 * want.float().abs() + 2.0 ** -22 * size).all()
+
+
+@pytest.mark.parametrize("B,S,hq,hkv,d,K,form", [
+    (1, 128, 12, 12, 64, 768, (1, 0)), (2, 65, 4, 2, 128, 2056, (4, 0)), (3, 1000, 32, 8, 64, 264, (0, 1)), (4, 1100, 24, 4, 128, 1032, (0, 2)),
+])
+@pytest.mark.parametrize("placed", [False, True])
+def test_rotation_has_the_same_bits_everywhere(B, S, hq, hkv, d, K, form, placed):
+    """The rotation in the epilogue, lb_rope there and lb_rope back, against the order of operations that they state: one product of a sum
+    rounded to fp32 and the other not, in float64 (whose own rounding, 2^-53, moves none of these values)."""
+    from lightron_b200.ops import functional as OF, native
+    N, T, heads = (hq + 2 * hkv) * d, B * S, hq + hkv
+    assert _form((T, N, K)) == form
+    x, w = _rand(T, K, seed=1), _rand(N, K, scale=K ** -0.5, seed=2)
+    ang = torch.rand(2 * S, d // 2, device="cuda") * 6.28
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    pos = torch.randperm(2 * S, device="cuda")[:S].int().contiguous() if placed else None
+    plain, fused = OF.gemm(x, w), torch.empty(T, N, device="cuda", dtype=torch.bfloat16)
+    there, back = plain.clone(), plain.clone()
+    native.call("lb_gemm_rope", x.data_ptr(), w.data_ptr(), fused.data_ptr(), T, N, K, cos.data_ptr(), sin.data_ptr(), native.ptr(pos), S, d,
+                heads * d, native.stream_ptr())
+    OF._rope_native_(there, cos, sin, pos, S, heads, d, False)
+    OF._rope_native_(back, cos, sin, pos, S, heads, d, True)
+    _status_ok()
+    assert torch.equal(fused, there)
+    i = slice(0, S) if pos is None else pos.long()
+    c, s = (t[i].double().view(1, S, 1, d // 8, 4) for t in (cos, sin))
+    a, b = plain[:, :heads * d].double().view(B, S, heads, d // 8, 4, 2).unbind(-1)
+    r32, first = lambda t: t.float().double(), torch.tensor([True, False, False, False], device="cuda")
+    for got, s, rounds_as in ((there, s, first), (back, -s, torch.ones_like(first))):
+        want = torch.stack([a * c - r32(b * s), torch.where(rounds_as, b * c + r32(a * s), a * s + r32(b * c))], -1)
+        assert torch.equal(got[:, :heads * d], want.float().bfloat16().reshape(T, -1))
+        assert torch.equal(got[:, heads * d:], plain[:, heads * d:])
 
 
 @pytest.mark.parametrize("T,K,I,form", [(2100, 1032, 2312, (0, 2)), (4000, 256, 1288, (0, 1)), (300, 4096, 264, (4, 0)), (70, 512, 264, (1, 0))])

@@ -115,7 +115,7 @@ def test_layers_without_gradients_in_one_call(dim, heads, kv, hidden, B, S):
             got = m(tok, positions)
         n2 = native.launch_count()
         assert n2 - n1 < n1 - n0, "not in one call"
-        # the kernels' bf16 results are the same, but for a rotation's contracted multiply and add, whose flips three layers carry on
+        # (the same bits: test_layers_in_one_call_leave_the_same_bits)
         assert (got.float() - want.float()).norm() < 1e-2 * want.float().norm()
         hook = m.layers["1"].register_forward_hook(lambda *a: seen.append(a[0]))
         with torch.no_grad():
@@ -132,3 +132,25 @@ def test_layers_without_gradients_in_one_call(dim, heads, kv, hidden, B, S):
     for g, w in zip(got, want):
         assert (g.float() - w.float()).norm() < 1e-2 * w.float().norm()
     native.raise_on_device_status()
+
+
+@pytest.mark.parametrize("dim,heads,kv,B,S", [(768, 12, 12, 1, 128), (512, 4, 2, 2, 77), (1024, 16, 4, 3, 700)])
+def test_layers_in_one_call_leave_the_same_bits(dim, heads, kv, B, S):
+    """An evaluation's logits do not depend on whether something looks at a block's output."""
+    from lightron_b200 import mesh
+    from lightron_b200.config import ModelArgs
+    from lightron_b200.models import LightronTransformer, init_weights
+    from lightron_b200.models.llama import flatten_parameters
+    mesh.set_context(None)
+    args = ModelArgs(dim=dim, n_layers=4, n_heads=heads, n_kv_heads=kv, vocab_size=512, max_seq_len=2 * S)
+    m = LightronTransformer(args, dtype=torch.bfloat16, device="cuda")
+    init_weights(m, 1, std=dim ** -0.5)
+    flatten_parameters(m)
+    tok = torch.randint(0, args.vocab_size, (B, S), device="cuda")
+    for positions in (None, torch.arange(3, S + 3, device="cuda")):
+        with torch.no_grad():
+            got = m(tok, positions)
+            hook = m.layers["1"].register_forward_hook(lambda *a: None)
+            want = m(tok, positions)
+            hook.remove()
+        assert torch.equal(got, want)

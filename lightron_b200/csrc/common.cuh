@@ -35,8 +35,10 @@ int lb_num_sms();
 // its launch, barriers, tensor memory and descriptors then run under the other's tail.  Its first access to memory that
 // another kernel writes or reads comes behind grid_wait(), which returns when the kernels before it have completed and their writes are
 // visible; every thread calls it, so that no bounded wait of a CTA's roles runs meanwhile.  A kernel that allocates tensor memory calls
-// grid_go() behind the allocation: a later kernel's CTA could otherwise hold the columns for which an earlier one waits.  Both are no-ops
-// in a plain launch.  Kernels that wait for other GPUs are launched plainly, and so is one of very many short blocks (a block's grid_wait() takes
+// grid_go() behind the allocation: a later kernel's CTA could otherwise hold the columns for which an earlier one waits.  grid_wait() does nothing in a
+// plain launch, but grid_go() does: whether the NEXT kernel starts early is that one's attribute.  So kernels that wait for other GPUs are launched
+// plainly and do not call grid_go() either: the next kernel's CTAs would fill the SMs for as long as the peers take, and what runs on other streams, which a
+// peer may be waiting for, would find no room.  Launched plainly, too, is one of very many short blocks (a block's grid_wait() takes
 // some 0.3 us: 32000 of clear_kernel 31 instead of 23 us).  No grid_go() in kernels that fill an SM's shared memory or registers: the next one's
 // CTAs would crowd into the SMs that are done first (1000 x 768 feed-forward, four launches, 76 instead of 74 us); for the same reason it does
 // nothing in a grid of many blocks, whose own time is not that of a launch.

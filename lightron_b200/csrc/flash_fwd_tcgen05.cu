@@ -245,7 +245,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
   __syncthreads();
   fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  if (!p.steal) grid_go();
+  if (!p.steal && !push.n_mov && !p.kv_flags) grid_go();
   grid_wait();
 
   if (warp < 4) {

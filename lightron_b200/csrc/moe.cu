@@ -195,7 +195,7 @@ struct PlanParams {
 };
 
 __global__ void __launch_bounds__(256) moe_plan_kernel(const PlanParams p) {
-  grid_go();
+  if (p.n == 1) grid_go();
   grid_wait();
   __shared__ int s_cnt[MOE_MAX_EXPERTS];
   __shared__ float s_ps[MOE_MAX_EXPERTS];
@@ -309,7 +309,7 @@ struct PushParams {
 };
 
 __global__ void __launch_bounds__(256) moe_push_kernel(const PushParams p) {
-  grid_go();
+  if (p.n == 1) grid_go();
   grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const int nvec = p.H >> 3;
@@ -398,7 +398,7 @@ struct PullParams {
 // itself: T 4096, H 2048, k 2 31 us, now 16.)  A sum takes its terms in the same order for every KS.
 template <int KS>
 __global__ void __launch_bounds__(256) moe_pull_kernel(const PullParams p) {
-  grid_go();
+  if (p.n == 1) grid_go();
   grid_wait();
   constexpr int U = 8 / KS;
   __shared__ int s_fail;

@@ -817,3 +817,55 @@ def test_launches_see_what_the_ones_before_them_wrote(M, N, K, captured):
         assert _rel(y, want) < 5e-3
         assert _rel(n, y.double() * torch.rsqrt(y.double().square().mean(-1, keepdim=True) + 1e-5)) < 5e-3
     assert torch.equal(w, want_w)
+
+
+@pytest.mark.parametrize("kind", ["plan", "pull", "attention"])
+def test_a_wait_for_other_gpus_keeps_no_other_stream_waiting(kind):
+    """While a kernel waits for a peer (whose flag nothing sets here: it gives up after half a second and says so), the launch behind it
+    holds no SMs: a kernel of another stream that needs half of the chip gets it."""
+    import ctypes
+    from lightron_b200.ops import functional as OF, native
+    a, b = _rand(4096, 2048, seed=1), _rand(4096, 2048, seed=2)
+    assert _form((4096, 4096, 2048))[0] == 0                            # a CTA's 200 KB of shared memory on every SM
+    q, do = _rand(1, 512, 8, 128, seed=3), _rand(1, 512, 8, 128, seed=4)
+    o, lse = OF.flash_fwd_native(q, q, q, False, 128 ** -0.5)
+    words, flags = (torch.zeros(4096, dtype=torch.int32, device="cuda") for _ in range(2))
+    two = lambda t, at=0: (ctypes.c_void_p * 2)(t.data_ptr() + at, t.data_ptr() + at)
+    i32, f32 = (lambda *s, t=t: torch.zeros(*s, dtype=t, device="cuda") for t in (torch.int32, torch.float32))
+    buf, out, idx, rows = _rand(128, 64), torch.empty(1, 64, dtype=torch.bfloat16, device="cuda"), i32(1, 1), i32(1, 1)
+    hist, psum, base, row0, seg, frac, aux = i32(1, 2), f32(1, 2), i32(1, 2), i32(2), i32(4), f32(2), f32(1)
+    kv, q1, l1 = _rand(1, 256, 1, 64, seed=5), _rand(1, 128, 1, 64, seed=6), f32(1, 1, 128)
+    o1 = torch.empty_like(q1)
+
+    def waiting(st):
+        if kind == "plan":
+            native.call("lb_moe_plan", hist.data_ptr(), psum.data_ptr(), base.data_ptr(), row0.data_ptr(), seg.data_ptr(), frac.data_ptr(),
+                        aux.data_ptr(), 1, 2, 2, 0, 1, 1, 128, two(words, 4096), two(words), 1, 1, st)
+        elif kind == "pull":
+            native.call("lb_moe_pull", out.data_ptr(), 0, idx.data_ptr(), rows.data_ptr(), 0, 0, 1, 64, 2, 1, 2, 0, 128, two(buf), two(words), 1, st)
+        else:
+            native.call("lb_flash_fwd_cp", q1.data_ptr(), kv.data_ptr(), kv.data_ptr(), o1.data_ptr(), l1.data_ptr(), 1, 128, 256, 256, 1, 1, 64,
+                        64, 64, 0.125, 0, flags.data_ptr(), 1, 0, 0, 0, 0, 0, 1, 0, None, None, None, 0, st)
+
+    def needs_room():
+        OF.flash_bwd_native(q, q, q, o, lse, do, False, 128 ** -0.5)
+    side, done = torch.cuda.Stream(), torch.cuda.Event()
+    OF.gemm(a, b)                                                       # (the first launch of a size uploads its schedule)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        needs_room()
+    torch.cuda.synchronize()
+    native.set_flag_wait_ns(500_000_000)
+    try:
+        waiting(native.stream_ptr())
+        OF.gemm(a, b)
+        done.record()
+        with torch.cuda.stream(side):
+            needs_room()
+        side.synchronize()
+        early = not done.query()
+        torch.cuda.synchronize()
+    finally:
+        native.set_flag_wait_ns(20_000_000_000)
+    assert list(native.device_status()) == ["attention forward" if kind == "attention" else "expert-parallel routing / dispatch / combine"]
+    assert early

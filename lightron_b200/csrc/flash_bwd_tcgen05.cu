@@ -29,8 +29,9 @@
 // Loops of 0.35 s of all its kernels, before / now, on one GPU: B8 S2048 32q/4kv d64 646 / 547 us, B1 S8192 32q/8kv d128
 // 1624 / 1404, B3 S1531 32q/8kv d128 237 / 221, B1 S4096 8q/8kv d128 117 / 104.
 // A key block's loop over query blocks may be cut into parts of `chunk` blocks, a CTA each, where whole loops would leave SMs without work (a causal
-// sequence's first key block takes as long as all blocks of the last ones together, and grouped heads make few CTAs of long loops): their dK / dV are then added up in
-// fp32 as dQ is, and converted with it (bwd_chunk() has the rule and the figures).
+// sequence's first key block takes as long as all blocks of the last ones together, and grouped heads make few CTAs of long loops): each part then leaves its
+// dK / dV in fp32 in a place of its own, and the kernel that converts dQ adds them up, in the order of the parts: dK and dV are the same bits in every run, as
+// those of whole loops are (dQ, to which the key blocks add as they come, is not, beyond 128 keys).  bwd_chunk() has the rule and the figures.
 // Warp roles (512 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 4-11 math, 12-15 dQ drain.
 // All waits are bounded; on expiry a status word is set and the CTA drains and frees its TMEM.
 #include <algorithm>
@@ -52,7 +53,7 @@ struct FaBwdParams {
   int causal;
   int kv_brows;   // rows between consecutive batches in the K/V tensor maps (>= Sk)
   int chunk;      // query blocks of a CTA, or 0: all of its key block, whose dK / dV it writes
-  float *dk_acc, *dv_acc;      // with chunk: fp32 sums, in the layout of dq_acc
+  float *dk_acc, *dv_acc;      // with chunk: a tile in the layout of dq_acc's for every CTA of the launch
   bool alone;                  // one key block, not in parts: its CTAs write dQ, and nothing uses dq_acc
 };
 
@@ -93,50 +94,111 @@ struct BwdCfg {
 };
 static_assert(BwdCfg<128>::SMEM <= 232448, "shared memory of a CTA");
 
-// fp32 accumulator layout (dQ, and dK / dV in parts): tile (b, h, block of 128 rows) -> 4 row quads -> D / 4 pieces of 4 columns -> 32 rows: the 16-byte stores of a
-// drain warp (a row per lane) are contiguous, and so are the 16-byte loads of a warp here.
-template <int D, bool PARTS>
+// First 128-query block that sees key block `nblk`, and the parts that its loop is cut into.
+__host__ __device__ __forceinline__ int bwd_first_block(int causal, int nblk, int off) {
+  const int first_row = nblk * 128 - off;
+  return causal && first_row > 0 ? first_row / 128 : 0;
+}
+__host__ __device__ __forceinline__ int bwd_parts(int mb_first, int n_mblocks, int rep, int chunk) {
+  const int its = (n_mblocks > mb_first ? n_mblocks - mb_first : 0) * rep;
+  return its ? (its + chunk - 1) / chunk : 1;      // (one without work where no query sees the block)
+}
+constexpr int MAX_CUT_BLOCKS = 1024;      // key blocks of a launch in parts
+
+// fp32 accumulator layout: dQ tile (b, h, block of 128 rows), or dK / dV tile of a part -> 4 row quads -> D / 4 pieces of 4 columns -> 32 rows: the 16-byte stores of a
+// drain warp (a row per lane) are contiguous, and so are the 16-byte loads of a warp here.  A thread converts 32 columns of a row of dQ, or adds the parts of COLS
+// columns of dK or dV (0: the launch was not in parts), 64 / COLS of them loaded at a time.  With few tiles their parts are one chain of loads, shorter the more are in
+// flight; with many, the wider pieces of rows count (COLS 8 / 16, backward, graph, us: 1 x 128, 16 / 1 heads, d 64 12.0 / 13.2, 1290 x 130, 16 / 2, d 64 20.9 / 22.7; 4
+// x 500, 16 / 4, d 64 28.3 / 26.4, 1 x 8192, 8 / 2, d 128 373 / 367).
+template <int D, int COLS>
 __global__ void fa_dq_convert_kernel(const FaBwdParams p) {
   grid_go();
   grid_wait();
-  constexpr int CPR = D / 32;                                  // 32-column chunks per row: a thread takes one
-  const int qblocks = (p.Sq + 127) / 128, kblocks = (p.Sk + 127) / 128;
-  const long long nq = (long long)p.B * p.hq * qblocks * 128 * CPR;
-  const long long nk = PARTS ? (long long)p.B * p.hkv * kblocks * 128 * CPR : 0;
-  for (long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x; at < nq + 2 * nk;
-       at += (long long)gridDim.x * blockDim.x) {
-    // whole warps: the three parts are multiples of 32
-    const int which = !PARTS || at < nq ? 0 : at < nq + nk ? 1 : 2;
-    const long long idx = which == 0 ? at : which == 1 ? at - nq : at - nq - nk;
-    const float* acc = which == 0 ? p.dq_acc : which == 1 ? p.dk_acc : p.dv_acc;
-    bf16* out = which == 0 ? p.dq : which == 1 ? p.dk : p.dv;
-    const long long ts = which == 0 ? p.dq_ts : which == 1 ? p.dk_ts : p.dv_ts;
-    const int S = which == 0 ? p.Sq : p.Sk, heads = which == 0 ? p.hq : p.hkv, blocks = which == 0 ? qblocks : kblocks;
-    const int lane = (int)(idx & 31);
-    const long long w = idx >> 5;                              // (tile, quad, chunk): the accumulator's order
+  const int lane = threadIdx.x & 31;
+  long long w0 = 0;                                            // warps' pieces of work ahead of those of dQ
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = ((long long)gridDim.x * blockDim.x) >> 5;
+  if constexpr (COLS > 0) {
+    constexpr int G = D / COLS, U = 64 / COLS, V = COLS / 4;      // U * V 16-byte loads in flight
+    const int off = p.Sk - p.Sq, n_mblocks = (p.Sq + 127) / 128, n_nblk = (p.Sk + 127) / 128, rep = p.hq / p.hkv, pairs = p.hkv * p.B;
+    __shared__ int s_first[MAX_CUT_BLOCKS + 1];                // parts ahead of a key block's
+    if (threadIdx.x < 32) {
+      int run = 0;
+      for (int k0 = 0; k0 <= n_nblk; k0 += 32) {
+        const int k = k0 + lane, own = k < n_nblk ? bwd_parts(bwd_first_block(p.causal, k, off), n_mblocks, rep, p.chunk) : 0;
+        int upto = own;                                        // inclusive sum over the lanes
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, upto, o);
+          if (lane >= o) upto += v;
+        }
+        if (k <= n_nblk) s_first[k] = run + upto - own;
+        run += __shfl_sync(0xffffffffu, upto, 31);
+      }
+    }
+    __syncthreads();
+    const int pieces = 2 * pairs * n_nblk * 4 * G;             // (bwd_chunk() cuts launches of few key blocks)
+    w0 = pieces;
+    for (long long at = warp; at < pieces; at += warps) {      // (dK or dV, key block, pair, quad, COLS columns)
+      const int w = (int)at, g = w % G, quad = (w / G) & 3, tile = w / (4 * G);
+      const int pair = tile % pairs, block = (tile / pairs) % n_nblk, dv = tile / pairs / n_nblk;
+      const int row = block * 128 + quad * 32 + lane;
+      if (row >= p.Sk) continue;
+      // (CTA part * pairs + pair has left its tile at that index; a block that no query sees has one part, which leaves nothing)
+      const int first = s_first[block], end = n_mblocks > bwd_first_block(p.causal, block, off) ? s_first[block + 1] : first;
+      const float4* from = reinterpret_cast<const float4*>(dv ? p.dv_acc : p.dk_acc) + (quad * (D / 4) + V * g) * 32 + lane;
+      float f[COLS];
+#pragma unroll
+      for (int i = 0; i < COLS; i++) f[i] = 0.f;
+      for (int part = first; part < end; part += U) {
+        float4 x[U][V];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const float4* tile_at = from + ((long long)(part + u) * pairs + pair) * (32 * D);
+#pragma unroll
+          for (int k = 0; k < V; k++)
+            if (part + u < end) x[u][k] = tile_at[k * 32];
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (part + u < end) {
+#pragma unroll
+            for (int k = 0; k < V; k++) { f[4 * k] += x[u][k].x; f[4 * k + 1] += x[u][k].y; f[4 * k + 2] += x[u][k].z; f[4 * k + 3] += x[u][k].w; }
+          }
+      }
+      bf16* o = (dv ? p.dv : p.dk) + ((long long)(pair / p.hkv) * p.Sk + row) * (dv ? p.dv_ts : p.dk_ts) + (pair % p.hkv) * D + g * COLS;
+#pragma unroll
+      for (int k = 0; k < COLS / 8; k++) *reinterpret_cast<uint4*>(o + k * 8) = pack8(f + k * 8);
+    }
+  }
+  constexpr int CPR = D / 32;                                  // 32-column chunks per row
+  const int n_mblocks = (p.Sq + 127) / 128;
+  const long long total = w0 + (long long)p.B * p.hq * n_mblocks * 4 * CPR;
+  // (a warp's next piece after those of dK and dV)
+  for (long long at = warp < w0 ? warp + (w0 - warp + warps - 1) / warps * warps : warp; at < total; at += warps) {
+    const long long w = at - w0;                               // (tile, quad, chunk): the accumulator's order
     const int chunk = (int)(w % CPR), quad = (int)((w / CPR) & 3);
     const long long tile = w / (CPR * 4);
-    const int block = (int)(tile % blocks);
-    const long long bh = tile / blocks;
-    const int row = block * 128 + quad * 32 + lane;
-    if (row >= S) continue;
-    const int h = (int)(bh % heads);
-    const long long b = bh / heads;
-    const float4* from = reinterpret_cast<const float4*>(acc) + (w * 8) * 32 + lane;
+    const int mblock = (int)(tile % n_mblocks);
+    const long long bh = tile / n_mblocks;
+    const int row = mblock * 128 + quad * 32 + lane;
+    if (row >= p.Sq) continue;
+    const int h = (int)(bh % p.hq);
+    const long long b = bh / p.hq;
+    const float4* from = reinterpret_cast<const float4*>(p.dq_acc) + (w * 8) * 32 + lane;
     float f[32];
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const float4 v = from[k * 32];
       f[4 * k] = v.x; f[4 * k + 1] = v.y; f[4 * k + 2] = v.z; f[4 * k + 3] = v.w;
     }
-    bf16* o = out + (b * S + row) * ts + (long long)h * D + chunk * 32;
+    bf16* o = p.dq + (b * p.Sq + row) * p.dq_ts + (long long)h * D + chunk * 32;
 #pragma unroll
     for (int k = 0; k < 4; k++) *reinterpret_cast<uint4*>(o + k * 8) = pack8(f + k * 8);
   }
 }
 
 // Row statistics, one 1 KB record per (b, h, 128-query block): 128 x -lse * log2(e), then 128 x -scale * sum_d o * do.  Rows
-// past Sq get (-inf, 0), which makes their P and dS zero.  Also clears the accumulators.  D/8 threads per (token, head).
+// past Sq get (-inf, 0), which makes their P and dS zero.  Also clears dQ's accumulator.  D/8 threads per (token, head).
 template <int D>
 __global__ void fa_bwd_prep_kernel(const FaBwdParams p) {
   grid_go();
@@ -146,11 +208,6 @@ __global__ void fa_bwd_prep_kernel(const FaBwdParams p) {
   const long long total = (long long)p.B * Sp * p.hq;
   const int rpb = blockDim.x / TPR;                            // rows per block and iteration
   const int sub = threadIdx.x % TPR;
-  if (p.chunk) {      // dk_acc and dv_acc, one behind the other
-    const long long n = 2LL * p.B * p.hkv * ((p.Sk + 127) / 128) * 128 * (D / 4);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-      reinterpret_cast<float4*>(p.dk_acc)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
   // every thread of the block runs the same number of iterations, so the shuffles see whole warps
   for (long long base = (long long)blockIdx.x * rpb; base < total; base += (long long)gridDim.x * rpb) {
     const long long idx = base + threadIdx.x / TPR;
@@ -186,17 +243,7 @@ __global__ void fa_bwd_prep_kernel(const FaBwdParams p) {
   }
 }
 
-// First 128-query block that sees key block `nblk`, and the parts that its loop is cut into.
-__host__ __device__ __forceinline__ int bwd_first_block(int causal, int nblk, int off) {
-  const int first_row = nblk * 128 - off;
-  return causal && first_row > 0 ? first_row / 128 : 0;
-}
-__host__ __device__ __forceinline__ int bwd_parts(int mb_first, int n_mblocks, int rep, int chunk) {
-  const int its = (n_mblocks > mb_first ? n_mblocks - mb_first : 0) * rep;
-  return its ? (its + chunk - 1) / chunk : 1;
-}
-
-// What a CTA leaves: WHOLE dK and dV of a key block, and its share of dQ, added to the fp32 sums; PARTS (with chunk) its share of all three; ALONE
+// What a CTA leaves: WHOLE dK and dV of a key block, and its share of dQ, added to the fp32 sums; PARTS (with chunk) that, and its share of dK and dV; ALONE
 // all three.
 enum : int { WHOLE, PARTS_OF, ALONE };
 template <int D, int FORM>
@@ -540,9 +587,9 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
     // dQ of the last block is the last MMA: everything has finished
     if (ok && total_it > 0) ok = mbar_wait(dq_full, (uint32_t)(total_it - 1) & 1u, abort_flag);
     if (PARTS && ok && total_it > 0) {
-      // added to the fp32 sums, 32 columns at a time
+      // to this CTA's place, 32 columns at a time
       fence_after();
-      float* sum = (wg ? p.dk_acc : p.dv_acc) + (((long long)b * p.hkv + hk) * n_nblk + nblk) * (128 * D) + quad * (32 * D);
+      float* sum = (wg ? p.dk_acc : p.dv_acc) + (long long)blockIdx.x * (128 * D) + quad * (32 * D);
       uint8_t* out = smem + (wg ? C::OFF_V : C::OFF_K) + quad * C::STG_BYTES;
 #pragma unroll 1
       for (int c = 0; c < D / 32; c++) {
@@ -557,7 +604,7 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          bulk_reduce_add_f32(sum + c * 1024, smem_u32(out), C::STG_BYTES);
+          bulk_store(sum + c * 1024, smem_u32(out), C::STG_BYTES);
           bulk_commit();
         }
       }
@@ -611,13 +658,15 @@ long long bwd_ctas(int B, int Sq, int Sk, int hq, int hkv, int causal, int chunk
   for (int k = 0; k < (Sk + 127) / 128; k++) n += bwd_parts(bwd_first_block(causal, k, Sk - Sq), n_mblocks, rep, chunk);
   return n * hkv * B;
 }
-// Query blocks of a part, or 0 where a CTA per key block is modelled to be as good.  In query blocks: a CTA's fixed part is some 6, adding to the
-// fp32 sums instead of writing dK / dV 3 and their conversion 2 more.  Whole / parts, us, all kernels, causal: B2 S2000 16q/2kv d64 258 / 92, B1 S2000
+// Query blocks of a part, or 0 where a CTA per key block is modelled to be as good.  In query blocks: a CTA's fixed part is some 6, leaving
+// dK / dV in fp32 instead of writing them 3 and their conversion 2 more.  Whole / parts, us, all kernels, causal: B2 S2000 16q/2kv d64 258 / 92, B1 S2000
 // 16q/4kv d64 116 / 51 and d128 159 / 71, B1 S8192 8q/2kv d128 561 / 365 and 2q/2kv 147 / 116, B4 S500 16q/4kv d64 40 / 28, B1 S300 8q/2kv d64 30 / 14; left
 // whole B8 S2048 32q/4kv d64, B1 S8192 32q/8kv d128, B3 S1531 32q/8kv d128, B2 S1728 4q/4kv d64.
+// (Measured with parts that added to one sum as they came.  Places of their own, whose order is fixed, against that, backward as graphs: B2 S2000 16q/2kv d64 81.0 / 82.4,
+// B1 S2000 16q/4kv d128 66.2 / 69.2, B1 S8192 8q/2kv d128 360 / 367 and 2q/2kv 114 / 120, B4 S500 16q/4kv d64 25.4 / 26.4, B1 S300 8q/2kv d64 11.9 / 12.0.)
 int bwd_chunk(int B, int Sq, int Sk, int hq, int hkv, int causal, int sms) {
   const int n_mblocks = (Sq + 127) / 128, n_nblk = (Sk + 127) / 128, rep = hq / hkv, pairs = hkv * B;
-  if ((long long)n_nblk * pairs > 4LL * sms) return 0;             // (several CTAs per SM, longest first)
+  if ((long long)n_nblk * pairs > 4LL * sms || n_nblk > MAX_CUT_BLOCKS) return 0;      // (several CTAs per SM, longest first)
   long long total = 0, longest = 0;
   for (int k = 0; k < n_nblk; k++) {
     const long long its = (long long)std::max(0, n_mblocks - bwd_first_block(causal, k, Sk - Sq)) * rep;
@@ -672,9 +721,10 @@ int launch_fa_bwd(const void* q, const void* k, const void* v, const FaBwdParams
   LB_LAUNCH(fa_bwd_prep_kernel<D>, (int)(pblocks < cap ? pblocks : cap), 256, 0, s, p);
   LB_LAUNCH(p.chunk ? fa_bwd_tc_kernel<D, PARTS_OF> : p.alone ? fa_bwd_tc_kernel<D, ALONE> : fa_bwd_tc_kernel<D, WHOLE>, (unsigned)grid, C::NTHREADS, C::SMEM, s, tq, tk, tv, tdo, tdk, tdv, p);
   if (p.alone) return LB_OK;
-  const long long kv_rows_acc = p.chunk ? 2LL * p.B * ((p.Sk + 127) / 128 * 128) * p.hkv : 0;
-  const long long cblocks = ((rows + kv_rows_acc) * (D / 32) + 255) / 256;
-  LB_LAUNCH(p.chunk ? fa_dq_convert_kernel<D, true> : fa_dq_convert_kernel<D, false>, (int)(cblocks < cap ? cblocks : cap), 256, 0, s, p);
+  const long long part_rows = p.chunk ? 2LL * p.B * ((p.Sk + 127) / 128 * 128) * p.hkv : 0;
+  const int cols = part_rows * (D / 16) < 32 * 4LL * lb_num_sms() ? 8 : 16;      // (16: four warps on an SM have work)
+  const long long cblocks = (rows * (D / 32) + part_rows * (D / cols) + 255) / 256;
+  LB_LAUNCH(!p.chunk ? fa_dq_convert_kernel<D, 0> : cols == 8 ? fa_dq_convert_kernel<D, 8> : fa_dq_convert_kernel<D, 16>, (int)(cblocks < cap ? cblocks : cap), 256, 0, s, p);
   return LB_OK;
 }
 
@@ -696,12 +746,18 @@ extern "C" long long lb_flash_bwd_ws_bytes(int B, int Sq, int hq, int d) {
   return (long long)B * hq * ((Sq + 127) / 128) * 128 * (2 + d) * (long long)sizeof(float);
 }
 
-// As above with room for fp32 dK / dV where that lets the launch be cut into more parts (zero otherwise): what the caller of lb_flash_bwd_tc_ws should bring.
+// Bytes of one of dk_acc and dv_acc of a launch in parts of `chunk` query blocks, which makes two CTAs per SM at most (39 MB of both, d 128, 148 SMs).
+static long long bwd_parts_bytes(int B, int Sq, int Sk, int hq, int hkv, int d, int causal, int chunk) {
+  return bwd_ctas(B, Sq, Sk, hq, hkv, causal, chunk) * 128 * d * (long long)sizeof(float);
+}
+
+// As above with room for the parts' fp32 dK / dV where the launch is better cut into parts (zero otherwise): what the caller of lb_flash_bwd_tc_ws should bring.
 // With lb_flash_bwd_ws_bytes() a CTA takes a whole key block.
 extern "C" long long lb_flash_bwd_ws_bytes_kv(int B, int Sq, int Sk, int hq, int hkv, int d, int causal) {
   const long long q = lb_flash_bwd_ws_bytes(B, Sq, hq, d);
-  if (!q || Sk <= 0 || hkv <= 0 || hq % hkv || !bwd_chunk(B, Sq, Sk, hq, hkv, causal, lb_num_sms())) return q;
-  return q + 2LL * B * hkv * ((Sk + 127) / 128) * 128 * d * (long long)sizeof(float);
+  if (!q || Sk <= 0 || hkv <= 0 || hq % hkv) return q;
+  const int chunk = bwd_chunk(B, Sq, Sk, hq, hkv, causal, lb_num_sms());
+  return chunk ? q + 2 * bwd_parts_bytes(B, Sq, Sk, hq, hkv, d, causal, chunk) : q;
 }
 
 // Host only (no CUDA call): query blocks per CTA of the launch for these sizes on `sms` SMs, given that workspace; 0: all of a key block.
@@ -711,7 +767,7 @@ extern "C" int lb_flash_bwd_chunk(int B, int Sq, int Sk, int hq, int hkv, int ca
 }
 
 static int flash_bwd_tc_impl(int kv_brows, const void* q, const void* k, const void* v, const void* o, const void* dout,
-                               const void* lse, void* stats, void* dq_acc, void* dkv_acc, void* dq, void* dk, void* dv, int B, int Sq,
+                               const void* lse, void* stats, void* dq_acc, void* dkv_acc, long long dkv_bytes, void* dq, void* dk, void* dv, int B, int Sq,
                                int Sk, int hq, int hkv, int d, long long q_ts, long long k_ts, long long v_ts,
                                long long o_ts, long long do_ts, long long dq_ts, long long dk_ts, long long dv_ts,
                                float scale, int causal, void* stream) {
@@ -723,9 +779,13 @@ static int flash_bwd_tc_impl(int kv_brows, const void* q, const void* k, const v
   FaBwdParams p{(const bf16*)o, (const bf16*)dout, (const float*)lse, (float*)stats, (float*)dq_acc,
                 (bf16*)dq, (bf16*)dk, (bf16*)dv, B, Sq, Sk, hq, hkv, o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal,
                 kv_brows, 0, nullptr, nullptr, false};
-  if (dkv_acc && (p.chunk = bwd_chunk(B, Sq, Sk, hq, hkv, causal, lb_num_sms())) > 0) {
-    p.dk_acc = (float*)dkv_acc;
-    p.dv_acc = p.dk_acc + (long long)B * hkv * ((Sk + 127) / 128) * 128 * d;
+  if (const int chunk = dkv_acc ? bwd_chunk(B, Sq, Sk, hq, hkv, causal, lb_num_sms()) : 0) {
+    const long long bytes = bwd_parts_bytes(B, Sq, Sk, hq, hkv, d, causal, chunk);
+    if (dkv_bytes >= 2 * bytes) {
+      p.chunk = chunk;
+      p.dk_acc = (float*)dkv_acc;
+      p.dv_acc = p.dk_acc + bytes / (long long)sizeof(float);
+    }
   }
   // Up to 128 keys a query block's dQ comes from one CTA, which writes it: no sums to clear, to add to and to convert.  Forward and backward, us, before / now,
   // d 64: B4 S128 12 heads inside its layer 58.5 / 57.0, B8 32 heads 29 / 25, B32 32q/8kv 66.6 / 55, B64 16 heads 97 / 83; B8 S100 16 heads d128 26 / 22.  (In
@@ -753,8 +813,8 @@ extern "C" int lb_flash_bwd_cp_ws(const void* q, const void* k, const void* v, c
   if (!need) return LB_ERR_SHAPE;
   if (ws_bytes < need) return LB_ERR_CAPACITY;
   const long long n_pad = (long long)B * hq * ((Sq + 127) / 128) * 128;
-  float* dkv_acc = ws_bytes >= need + 2LL * B * hkv * ((Sk + 127) / 128) * 128 * d * (long long)sizeof(float) ? (float*)ws + (2 + d) * n_pad : nullptr;
-  return flash_bwd_tc_impl(kv_brows, q, k, v, o, dout, lse, ws, (float*)ws + 2 * n_pad, dkv_acc, dq, dk, dv, B, Sq, Sk, hq, hkv, d,
+  float* dkv_acc = ws_bytes > need ? (float*)ws + (2 + d) * n_pad : nullptr;
+  return flash_bwd_tc_impl(kv_brows, q, k, v, o, dout, lse, ws, (float*)ws + 2 * n_pad, dkv_acc, ws_bytes - need, dq, dk, dv, B, Sq, Sk, hq, hkv, d,
                            q_ts, k_ts, v_ts, o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal, stream);
 }
 
@@ -779,7 +839,7 @@ extern "C" int lb_flash_bwd_cp(const void* q, const void* k, const void* v, cons
   void* stats = nullptr;
   cudaError_t e = cudaMallocAsync(&stats, (size_t)B * hq * ((Sq + 127) / 128) * 256 * sizeof(float), (cudaStream_t)stream);
   if (e != cudaSuccess) { cudaGetLastError(); g_lb_last_cuda_error = (int)e; return LB_ERR_LAUNCH; }
-  const int rc = flash_bwd_tc_impl(kv_brows, q, k, v, o, dout, lse, stats, dq_acc, nullptr, dq, dk, dv, B, Sq, Sk, hq, hkv, d, q_ts, k_ts,
+  const int rc = flash_bwd_tc_impl(kv_brows, q, k, v, o, dout, lse, stats, dq_acc, nullptr, 0, dq, dk, dv, B, Sq, Sk, hq, hkv, d, q_ts, k_ts,
                                    v_ts, o_ts, do_ts, dq_ts, dk_ts, dv_ts, scale, causal, stream);
   e = cudaFreeAsync(stats, (cudaStream_t)stream);
   if (rc == LB_OK && e != cudaSuccess) { g_lb_last_cuda_error = (int)e; return LB_ERR_LAUNCH; }

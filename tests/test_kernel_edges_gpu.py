@@ -180,6 +180,27 @@ def test_attention_backward_in_parts(B, Sq, Sk, hq, hkv, causal, d, parts):
     assert all(bool((t[B * n:] == 7.0).all()) for t, n in zip(buf, (Sq, Sk, Sk)))
 
 
+@pytest.mark.parametrize("B,Sq,Sk,hq,hkv,causal,d", [
+    (1, 2000, 2000, 16, 2, True, 64), (2, 300, 300, 8, 2, True, 128), (1, 515, 1290, 16, 1, True, 64), (1, 1290, 130, 16, 2, False, 128),
+    (1, 128, 128, 16, 1, True, 128), (1, 2000, 77, 4, 1, False, 64),     # one key block: dQ too
+    (1, 640, 4096, 16, 1, True, 64),                                     # many key blocks
+])
+def test_attention_backward_in_parts_repeats_itself(B, Sq, Sk, hq, hkv, causal, d):
+    """dK and dV of key blocks whose loops are cut are the same bits in every run, and dQ too where a key block adds to it alone."""
+    from lightron_b200.ops import functional as OF, native
+    assert native.require().lb_flash_bwd_chunk(B, Sq, Sk, hq, hkv, int(causal), native.sm_count()) > 0
+    q, do = _rand(B, Sq, hq, d, seed=1), _rand(B, Sq, hq, d, seed=4)
+    k, v = _rand(B, Sk, hkv, d, seed=2), _rand(B, Sk, hkv, d, seed=3)
+    o, lse = OF.flash_fwd_native(q, k, v, causal, d ** -0.5)
+    runs = [OF.flash_bwd_native(q, k, v, o, lse, do, causal, d ** -0.5) for _ in range(6)]
+    _status_ok()
+    for name, g, w in zip(("dq", "dk", "dv"), runs[0], _attention64(q, k, v, do, causal)[1:]):
+        assert _rel(g, w) < 1e-2, name
+    for r in runs[1:]:
+        assert torch.equal(r[1], runs[0][1]) and torch.equal(r[2], runs[0][2])
+        assert Sk > 128 or torch.equal(r[0], runs[0][0])
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("B,Sq,Sk,hq,hkv,causal", [
     (1, 1, 1, 1, 1, True),

@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + 8 * (2 * STAGES + 2));
   int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);        // {abort, extra wait in ms}: see bw::mbar_wait
   volatile int* abort_flag = s_abort;
+  int* s_sums = s_abort + 2;                                   // the same for the wait for the other parts' sums, which no abort cuts short
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);      // (uniform over the warp)
   const int lane = threadIdx.x & 31;
   const int rank = KS > 1 ? (int)bw::cluster_ctarank() : 0;
@@ -162,6 +163,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
   if (threadIdx.x == 0) {
     s_abort[0] = 0;
     s_abort[1] = 0;
+    s_sums[0] = 0;
+    s_sums[1] = 2000;                                          // (longer than another CTA's wait for its accumulator)
     if (smem_base & 1023u) { s_abort[0] = 1; atomicExch(&g_split_status[0], 4u); }      // the swizzled tiles need it: nothing is started
     for (int s = 0; s < STAGES; s++) {
       bw::mbar_init(bar_base + 8u * s, 1);
@@ -239,12 +242,19 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
   bw::fence_after();
 
   if constexpr (KS > 1) {
-    if (warp >= 2 && ok) {
-      // 8 columns at a time to the CTA that finishes them: a block of a quad's rows from either of its warps
+    if (warp >= 2) {
+      // 8 columns at a time to the CTA that finishes them: a block of a quad's rows from either of its warps.  Every CTA sends all of its parts, zeros where
+      // its accumulator did not come (the status word says that the result is void), and waits for all that is sent to it: a CTA that left out either could end,
+      // or keep another from ending, while stores to its shared memory are on their way.
       const uint32_t here = smem_base + C::OFF_RECV + (uint32_t)(row_in * 16);
       uint32_t r[32];
-      bw::tmem_ld32(taddr + set * HB, r);
-      bw::tmem_ld_wait();
+      if (ok) {
+        bw::tmem_ld32(taddr + set * HB, r);
+        bw::tmem_ld_wait();
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; i++) r[i] = 0;
+      }
 #pragma unroll
       for (int g = 0; g < 4; g++) {
         const int s = KS == 8 ? set * 4 + g : g / NG;          // the receiver; its place for this part: parts in order, its own left out
@@ -260,19 +270,21 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
     __syncwarp();
     bw::cluster_arrive();
   }
-  if (warp >= 2 && ok) {
+  if (warp >= 2) {
     float f[NB][GW][8];
+    if (ok) {
 #pragma unroll
-    for (int b = 0; b < NB; b++)
+      for (int b = 0; b < NB; b++)
 #pragma unroll
-      for (int g = 0; g < GW; g++)
-        if (mine(b)) bw::tmem_ld8(taddr + block_of(b) * HB + column_of(g), reinterpret_cast<uint32_t*>(f[b][g]));
-    bw::tmem_ld_wait();
+        for (int g = 0; g < GW; g++)
+          if (mine(b)) bw::tmem_ld8(taddr + block_of(b) * HB + column_of(g), reinterpret_cast<uint32_t*>(f[b][g]));
+      bw::tmem_ld_wait();
+    }
     if constexpr (KS > 1) {
       // The sums order nothing but themselves: an acquire on their barrier, not a fence over the cluster beside it, and a barrier at the end that only keeps the CTA
       // there (12 layers of 128 x 768 471 -> 462 us, the MLP of 16 x 2048 81.5 -> 80.7; storing rows by neighbouring lanes gave 10 us of the first and 3 of the
       // second back, although the attention layer of 128 rows took 57.0 instead of 58.5).
-      if (!bw::mbar_wait<true>(received, 0, abort_flag)) { ok = false; give_up(abort_flag, 5u); }
+      if (!bw::mbar_wait<true>(received, 0, s_sums)) { ok = false; give_up(abort_flag, 5u); }
       const float4* in = reinterpret_cast<const float4*>(smem + C::OFF_RECV) + row_in;
 #pragma unroll
       for (int b = 0; b < NB; b++)
@@ -362,7 +374,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel(const __grid
     bw::tmem_dealloc(tmem_base, BN);
   }
   __syncwarp();
-  if constexpr (KS > 1) bw::cluster_wait();                    // nobody sends to this CTA any more
+  if constexpr (KS > 1) bw::cluster_wait();                    // nobody has anything left to send to this CTA
 }
 
 template <int KS>

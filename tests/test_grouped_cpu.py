@@ -279,3 +279,40 @@ def test_host_module_of_another_torch_is_not_loaded(monkeypatch):
     assert build.needs_build() and not build.host_built_for_this_torch()
     with pytest.warns(UserWarning, match="not built for torch"):
         assert native._load_host_ops() is None
+
+
+def _conditions(src, at):
+    """The conditions of the if statements whose braces enclose position ``at`` of ``src``."""
+    out, depth = [], 0
+    for i in range(at, -1, -1):
+        if src[i] == "}":
+            depth += 1
+        elif src[i] == "{" and depth:
+            depth -= 1
+        elif src[i] == "{":
+            head = src[:i].rstrip()
+            if head.endswith(")"):
+                n = 0
+                for j in range(len(head) - 1, -1, -1):
+                    n += (head[j] == ")") - (head[j] == "(")
+                    if n == 0:
+                        break
+                if head[:j].rstrip().split()[-1] in ("if", "constexpr"):
+                    out.append(head[j + 1:-1])
+    return out
+
+
+def test_parts_of_a_reduction_are_exchanged_whatever_failed():
+    """A CTA of the split GEMM that has given up still sends its parts and waits for those of the others, on words that no abort sets: stores
+    into a CTA's shared memory have arrived before it may end.  (Read from the source: no test makes a GPU miss them.)"""
+    from lightron_b200.csrc import build
+    src = open(os.path.join(build.HERE, "gemm_split.cu")).read()
+    src = "\n".join(line.split("//")[0] for line in src.splitlines())
+    body = src[src.index("void __launch_bounds__(NUM_THREADS, 2) gemm_split_kernel"):src.index("int launch(const Params& gp")]
+    sends, waits = [body.index(t) for t in ("st_cluster_v4(dst, r", "mbar_wait<true>(received")]
+    assert _conditions(body, body.index("bw::tmem_ld32(taddr + set * HB, r)"))[0] == "ok"      # (what the search finds where there is one)
+    for at in (sends, waits):
+        assert sorted(_conditions(body, at)) == ["KS > 1", "warp >= 2"]
+    words = body[waits:].split(")")[0].split(",")[-1].strip()
+    assert words == "s_sums" and "give_up(s_sums" not in body and body.count(words + "[0] = ") == 1
+    assert body.index("mbar_wait<true>(received") < body.index("bw::cluster_wait()")

@@ -553,7 +553,7 @@ struct RaggedParams {
   long long ldc;
   const bf16* old;                     // mode 0, epi 2: g | u
   long long ld_old;
-  int epi, half;
+  int epi, half, keep;                 // (keep: see Problem)
   const int* seg;
   int LE, M_w, N, K, b_mn, mode, accumulate, cap;
   int tiles_n, tiles_m_w, num_kb;
@@ -737,7 +737,7 @@ __global__ void __launch_bounds__(Cfg<CG, EW>::NUM_THREADS, 1) gemm_ragged_kerne
       const bool wgrad = rp.mode == 1;
       // (mode 0 writes whole 128-row tiles: padding rows are zeros)
       const Out out{wgrad ? &rp.tc[rt.e] : rp.tc, wgrad ? rp.C[rt.e] : rp.old, wgrad ? rp.ldc : rp.ld_old, wgrad ? rp.C[rt.e] : rp.C[0], rp.ldc, rt.m0 + rank * BM + quad * 32, wgrad ? rp.M_w : s_end[rt.e],
-                    rt.n0 + part * (rp.epi == 1 ? BN / 4 : BN / 2), rp.epi ? rp.half : rp.N, true, nullptr};
+                    rt.n0 + part * (rp.epi == 1 ? BN / 4 : BN / 2), rp.epi ? rp.half : rp.N, rp.keep != 0, nullptr};
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN + part * (rp.epi == 1 ? BN / 4 : BN / 2));
       auto ready = [&]() {
         if (!bw::mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) return false;
@@ -1100,7 +1100,7 @@ static int run_grouped(int n, const void* const* A, const void* const* B, void* 
     if ((lda[i] % 8) || (ldb[i] % 8) || (ldc[i] % 8) || (N[i] % 8) || (a_mn[i] && (M[i] % 8))) return LB_ERR_SHAPE;
     if (((uintptr_t)A[i] | (uintptr_t)B[i] | (uintptr_t)C[i]) & 15) return LB_ERR_ARG;
     const int e = epi ? epi[i] : 0;
-    if (e < 0 || e > 2) return LB_ERR_ARG;
+    if (e < 0 || e > 2 || (!C[i] && e != 1)) return LB_ERR_ARG;
     if (e) {
       if (!C2 || !ldc2 || !half || !C2[i] || ((uintptr_t)C2[i] & 15) || (ldc2[i] % 8) || half[i] <= 0 || (half[i] % 8)) return LB_ERR_ARG;
       if (e == 1 && (b_mn[i] || N[i] != 2 * half[i])) return LB_ERR_SHAPE;
@@ -1115,8 +1115,10 @@ static int run_grouped(int n, const void* const* A, const void* const* B, void* 
   }
   {
     std::lock_guard<std::mutex> lock(g_sched_mutex);
-    if (g_sms == 0) {
-      cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
+    if (g_sms == 0 && cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaGetLastError();
+      g_sms = 0;
+      return LB_ERR_LAUNCH;
     }
   }
   Schedule sched;
@@ -1237,7 +1239,7 @@ extern "C" int lb_gemm_ragged_epi(const void* A, const void* const* B, void* C, 
   if (LE < 1 || LE > MAX_PROBLEMS || cap <= 0 || N <= 0 || K <= 0) return LB_ERR_SHAPE;
   if ((lda % 8) || (ldb % 8) || (ldc % 8) || (N % 8) || (K % 8)) return LB_ERR_SHAPE;
   if (((uintptr_t)A | (uintptr_t)C) & 15) return LB_ERR_ARG;
-  if (epi < 0 || epi > 2) return LB_ERR_ARG;
+  if (epi < 0 || epi > 2 || (!C && epi != 1)) return LB_ERR_ARG;
   if (epi) {
     if (!C2 || ((uintptr_t)C2 & 15) || (ldc2 % 8) || half <= 0 || (half % 8)) return LB_ERR_ARG;
     if (epi == 1 ? (b_mn || N != 2 * half) : N != half) return LB_ERR_SHAPE;
@@ -1253,7 +1255,7 @@ extern "C" int lb_gemm_ragged_epi(const void* A, const void* const* B, void* C, 
     rp.C[e] = nullptr;
   }
   if ((rc = out_maps(rp.tc, C, C2, ldc, ldc2, cap, N, epi, half))) return rc;
-  rp.C[0] = (bf16*)C; rp.ldc = ldc; rp.old = (const bf16*)C2; rp.ld_old = ldc2; rp.epi = epi; rp.half = half; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = 0; rp.N = N; rp.K = K; rp.b_mn = b_mn;
+  rp.C[0] = (bf16*)C; rp.ldc = ldc; rp.old = (const bf16*)C2; rp.ld_old = ldc2; rp.epi = epi; rp.half = half; rp.keep = C != nullptr; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = 0; rp.N = N; rp.K = K; rp.b_mn = b_mn;
   rp.mode = 0; rp.accumulate = 0; rp.cap = cap;
   rp.tiles_n = (N + BN - 1) / BN; rp.tiles_m_w = 0; rp.num_kb = (K + BK - 1) / BK;
   rp.wait_flag = (const unsigned int*)wait_flag; rp.wait_target = wait_target; rp.wait_ns = g_lb_flag_wait_ns;
@@ -1274,6 +1276,8 @@ extern "C" int lb_gemm_ragged_wgrad(const void* dY, const void* X, void* const* 
   if (LE < 1 || LE > MAX_PROBLEMS || cap <= 0 || Nw <= 0 || Kw <= 0) return LB_ERR_SHAPE;
   if ((lddy % 8) || (ldx % 8) || (ldc % 8) || (Nw % 8) || (Kw % 8)) return LB_ERR_SHAPE;
   if (((uintptr_t)dY | (uintptr_t)X) & 15) return LB_ERR_ARG;
+  for (int e = 0; e < LE; e++)
+    if (!C[e] || ((uintptr_t)C[e] & 15)) return LB_ERR_ARG;
   static thread_local RaggedParams rp;
   const int cg = ragged_wgrad_cg(LE, cap, lb_num_sms());
   int rc = bw::make_map_bf16(&rp.ta, dY, (uint64_t)Nw, (uint64_t)cap, (uint64_t)lddy, 64, BK);
@@ -1281,11 +1285,10 @@ extern "C" int lb_gemm_ragged_wgrad(const void* dY, const void* X, void* const* 
   rc = bw::make_map_bf16(&rp.tb[0], X, (uint64_t)Kw, (uint64_t)cap, (uint64_t)ldx, 64, BK);
   if (rc) return rc;
   for (int e = 0; e < LE; e++) {
-    if ((uintptr_t)C[e] & 15) return LB_ERR_ARG;
     rp.C[e] = (bf16*)C[e];
     if ((rc = out_map(&rp.tc[e], rp.C[e], Kw, Nw, ldc))) return rc;
   }
-  rp.ldc = ldc; rp.old = nullptr; rp.ld_old = 0; rp.epi = 0; rp.half = 0; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = Nw; rp.N = Kw; rp.K = 0; rp.b_mn = 1; rp.mode = 1;
+  rp.ldc = ldc; rp.old = nullptr; rp.ld_old = 0; rp.epi = 0; rp.half = 0; rp.keep = 1; rp.seg = (const int*)seg; rp.LE = LE; rp.M_w = Nw; rp.N = Kw; rp.K = 0; rp.b_mn = 1; rp.mode = 1;
   rp.accumulate = accumulate; rp.cap = cap;
   rp.tiles_n = (Kw + BN - 1) / BN; rp.tiles_m_w = (Nw + BM * cg - 1) / (BM * cg); rp.num_kb = 0;
   rp.wait_flag = nullptr; rp.wait_target = 0; rp.wait_ns = g_lb_flag_wait_ns;

@@ -424,7 +424,7 @@ int gemm_split_rope(int n, const void* const* A, const void* const* B, void* con
     if ((lda[i] % 8) || (ldb[i] % 8) || (ldc[i] % 8) || (N[i] % 8) || (a_mn[i] && (M[i] % 8))) return LB_ERR_SHAPE;
     if (((uintptr_t)A[i] | (uintptr_t)B[i] | (uintptr_t)C[i]) & 15) return LB_ERR_ARG;
     const int e = epi ? epi[i] : 0;
-    if (e < 0 || e > 2) return LB_ERR_ARG;
+    if (e < 0 || e > 2 || (!C[i] && e != 1)) return LB_ERR_ARG;
     if (e) {
       if (!C2 || !ldc2 || !half || !C2[i] || ((uintptr_t)C2[i] & 15) || (ldc2[i] % 8) || half[i] <= 0 || (half[i] % 8)) return LB_ERR_ARG;
       if (e == 1 && (b_mn[i] || N[i] != 2 * half[i])) return LB_ERR_SHAPE;

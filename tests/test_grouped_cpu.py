@@ -316,3 +316,23 @@ def test_parts_of_a_reduction_are_exchanged_whatever_failed():
     words = body[waits:].split(")")[0].split(",")[-1].strip()
     assert words == "s_sums" and "give_up(s_sums" not in body and body.count(words + "[0] = ") == 1
     assert body.index("mbar_wait<true>(received") < body.index("bw::cluster_wait()")
+
+
+@pytest.mark.parametrize("epi", [0, 1, 2])
+def test_outputs_that_are_missing(epi):
+    """Only the SwiGLU forward may leave out C; elsewhere a null C is refused before anything is launched (on a machine without a GPU
+    the call that is not refused ends at its first CUDA call)."""
+    if torch.cuda.is_available():
+        pytest.skip("host checks; the addresses are made up")
+    lib = native._load()
+    if lib is None:
+        pytest.skip("native library not built")
+    V, I, L = ctypes.c_void_p * 1, ctypes.c_int * 1, ctypes.c_longlong * 1
+    n, half = (512, 256) if epi == 1 else (256, 256)
+    for C in (0, 4096):
+        head = (1, V(4096), V(4096), V(C), I(256), I(n), I(512), L(512), L(512), L(2 * half), I(0), I(0), I(0), I(epi), V(4096), L(2 * half), I(half))
+        refused = [lib.lb_gemm_grouped_epi(*head, None), lib.lb_gemm_split(*head, 1, None),
+                   lib.lb_gemm_ragged_epi(4096, V(4096), C, 4096, 1, 256, n, 512, 512, 512, 2 * half, 0, epi, 4096, 2 * half, half, None, 0, None)]
+        if epi == 0:
+            refused.append(lib.lb_gemm_ragged_wgrad(4096, 4096, V(C), 4096, 1, 256, 256, 512, 256, 512, 512, 0, None))
+        assert [r == -1 for r in refused] == [C == 0 and epi != 1] * len(refused), (C, refused)

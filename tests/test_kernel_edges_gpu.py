@@ -786,6 +786,26 @@ def test_ragged_expert_gemms(H, I, counts, ctas):
         assert _rel(dgu[r], torch.cat([dh * u * sig * (1 + g * (1 - sig)), dh * g * sig], 1)) < 1e-2        # (dh is rounded to bf16 first)
 
 
+@pytest.mark.parametrize("H,I,counts,ctas", [(72, 264, (130, 0, 1, 300), 1), (4104, 264, (300, 0, 129, 1290), 2)])
+def test_ragged_activation_without_gate_and_up(H, I, counts, ctas):
+    """The activation alone, with a null C: the same bits, and the output of the call before it is left as it is."""
+    from lightron_b200.ops import native
+    from lightron_b200.parallel import ep_fused
+    LE, cap = len(counts), 1024 if ctas == 1 else 2560
+    pad = [(c + 127) // 128 * 128 for c in counts]
+    seg = [sum(pad[:e]) for e in range(LE)]
+    assert native.require().lb_gemm_ragged_ctas_per_tile(LE, cap, 2 * I, H, native.sm_count()) == ctas
+    table = torch.tensor([*seg, *counts, sum(pad), sum(counts)], dtype=torch.int32, device="cuda")
+    x, up = _rand(cap, H, seed=1), [_rand(2 * I, H, scale=H ** -0.5, seed=10 + e) for e in range(LE)]
+    gu, act, alone = (torch.full((cap, n), 7.0, device="cuda", dtype=torch.bfloat16) for n in (2 * I, I, I))
+    ep_fused._ragged(x, up, gu, table, LE, cap, 2 * I, H, False, epi=1, c2=act, half=I)
+    gu.fill_(3.0)
+    native.call("lb_gemm_ragged_epi", x.data_ptr(), ep_fused._ptr_array(up), 0, table.data_ptr(), LE, cap, 2 * I, H, H, H, 2 * I, 0, 1,
+                alone.data_ptr(), I, I, 0, 0, native.stream_ptr())
+    _status_ok()
+    assert torch.equal(alone, act) and bool((gu == 3.0).all())
+
+
 @pytest.mark.parametrize("n", [0, 1, 15, 16, 17, 4095, 4096, 4111, 1 << 20, (1 << 20) + 7])
 def test_clear_writes_its_bytes_and_no_others(n):
     from lightron_b200.ops import native

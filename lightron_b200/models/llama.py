@@ -159,8 +159,8 @@ class TransformerBlock(nn.Module):
 
 def _plain_layers(layers: nn.ModuleDict):
     """(hq, hkv, d, scale, weights of every layer) of dense blocks on one GPU that nothing hooks into, for ``host_ops.decoder_layers``, which does
-    in one call what their ``forward`` does op by op; None for any other."""
-    if not layers or nn.modules.module._has_any_global_hook():
+    in one call what their ``forward`` does op by op, with every fusion switched on; None for any other."""
+    if not layers or not (OF._GROUP_BWD and OF._FUSED_SWIGLU) or nn.modules.module._has_any_global_hook():
         return None
     weights, shape = [], None
     for blk in layers._modules.values():

@@ -125,3 +125,14 @@ def test_which_layers_run_in_one_call():
     assert _plain_layers(m.layers) is None
     assert _plain_layers(LightronTransformer(_tiny(moe_num_experts=2, moe_topk=1, moe_layer_freq=2)).layers) is None
     assert _plain_layers(torch.nn.ModuleDict()) is None
+
+
+@pytest.mark.parametrize("switch", ["_FUSED_SWIGLU", "_GROUP_BWD"])
+def test_a_fusion_that_is_switched_off_stays_off_in_evaluations(monkeypatch, switch):
+    """What compares an evaluation with and without a fusion must not run the same kernels twice."""
+    from lightron_b200.models.llama import _plain_layers
+    from lightron_b200.ops import functional as OF
+    m = LightronTransformer(_tiny())
+    assert _plain_layers(m.layers) is not None
+    monkeypatch.setattr(OF, switch, False)
+    assert _plain_layers(m.layers) is None

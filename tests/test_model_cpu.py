@@ -1,3 +1,4 @@
+import pytest
 import torch
 
 from lightron_b200.config import ModelArgs, PRESETS

@@ -157,10 +157,15 @@ class TransformerBlock(nn.Module):
         return h, f
 
 
+_FORWARDS = tuple((cls, cls.forward) for cls in (TransformerBlock, Attention, MLP))
+
+
 def _plain_layers(layers: nn.ModuleDict):
     """(hq, hkv, d, scale, weights of every layer) of dense blocks on one GPU that nothing hooks into, for ``host_ops.decoder_layers``, which does
     in one call what their ``forward`` does op by op, with every fusion switched on; None for any other."""
     if not layers or not (OF._GROUP_BWD and OF._FUSED_SWIGLU) or nn.modules.module._has_any_global_hook():
+        return None
+    if any(cls.forward is not f for cls, f in _FORWARDS):          # replaced for all of a class
         return None
     weights, shape = [], None
     for blk in layers._modules.values():

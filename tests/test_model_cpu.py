@@ -137,3 +137,14 @@ def test_a_fusion_that_is_switched_off_stays_off_in_evaluations(monkeypatch, swi
     assert _plain_layers(m.layers) is not None
     monkeypatch.setattr(OF, switch, False)
     assert _plain_layers(m.layers) is None
+
+
+def test_a_forward_replaced_for_a_class_is_called(monkeypatch):
+    from lightron_b200.models import llama
+    m = LightronTransformer(_tiny())
+    for cls in (llama.TransformerBlock, llama.Attention, llama.MLP):
+        with monkeypatch.context() as p:
+            plain = cls.forward
+            p.setattr(cls, "forward", lambda self, *a, **kw: plain(self, *a, **kw))
+            assert llama._plain_layers(m.layers) is None
+        assert llama._plain_layers(m.layers) is not None

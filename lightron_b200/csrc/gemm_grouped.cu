@@ -1191,14 +1191,14 @@ extern "C" int lb_gemm_grouped(int n, const void* const* A, const void* const* B
 }
 
 namespace {
-// CTAs per tile.  The rows are known on the device only: as many as the buffer holds beyond its padding, the same for every expert, half a tile of each
-// wasted.  Both forms' times as tile_time() has them for the lists (a pair's as those of a launch, 6 k-blocks more), 3 % for the
+// CTAs per tile.  The rows are known on the device only: as many as the caller expects in all, the same for every expert, half a tile of each
+// wasted.  (Not as many as the buffer holds: between several GPUs its capacity is twice what arrives on average.)  Both forms' times as tile_time() has them for the lists (a pair's as those of a launch, 6 k-blocks more), 3 % for the
 // unevenness, which costs pairs more.  CTAs / pairs in us, 8 experts, 2048 -> 4096, 2 of them per token, 4096 tokens: gate | up 254 / 220, down 127 / 106, its data
 // gradient 143 / 144, gate | up's 251 / 252; 1024 tokens 88 / 77, 60 / 54, 64 / 60, 107 / 96; 64 tokens 54 / 63, 34 / 33, 38 / 44, 56 / 58; 4096 tokens of 4
 // experts, 1024 -> 4096: 131 / 108, 59 / 55, 124 / 127, 111 / 104.
-int ragged_cg(int LE, int cap, int n, int num_kb, int sms) {
+int ragged_cg(int LE, int all_rows, int n, int num_kb, int sms) {
   if (sms < 2) return 1;
-  const double rows = std::max(1.0, (double)(cap - LE * BM) / LE);
+  const double rows = std::max(1.0, (double)all_rows / LE);
   const double tn = (n + BN - 1) / BN;
   double time[3];
   for (int cg = 1; cg <= 2; cg++) {
@@ -1208,10 +1208,13 @@ int ragged_cg(int LE, int cap, int n, int num_kb, int sms) {
   return 1.03 * (time[2] + 600) < time[1] ? 2 : 1;
 }
 // Weight gradients: as many tiles whatever the rows are, but with few of them a tile is mostly its store.  CTAs / pairs, down and gate | up: 1024 rows per expert
-// 126 / 118 and 282 / 222, 512 90 / 79 and 158 / 137, 256 48 / 59 and 88 / 105.
-int ragged_wgrad_cg(int LE, int cap, int sms) {
-  return sms >= 2 && (cap - LE * BM) / LE >= 512 ? 2 : 1;
+// 126 / 118 and 282 / 222, 512 90 / 79 and 158 / 137, 256 48 / 59 and 88 / 105.  (Uneven routing, 8 experts, 512 rows on average 72 / 67 and 135 / 126, 448 65 / 62 and 122 /
+// 116, 384 60 / 59 and 110 / 109, 256 47 / 57 and 86 / 103.)
+int ragged_wgrad_cg(int LE, int all_rows, int sms) {
+  return sms >= 2 && all_rows / LE >= 512 ? 2 : 1;
 }
+// Rows to expect: the caller's number, or, where that is 0, what the buffer holds beyond the padding of its segments.
+int ragged_rows(int LE, int cap, int rows) { return rows > 0 ? rows : cap - LE * BM; }
 int launch_ragged(int cg, bool dependent, const RaggedParams& rp, cudaStream_t s) {
   const int workers = lb_num_sms() / cg;
   if (cg == 2) return rp.epi == 2 ? launch_form(gemm_ragged_kernel<2, 8>, Cfg<2, 8>(), 2, workers, dependent, rp, s)
@@ -1221,10 +1224,12 @@ int launch_ragged(int cg, bool dependent, const RaggedParams& rp, cudaStream_t s
 }
 }  // namespace
 
-// Host only (no CUDA call): CTAs per tile, 1 or 2, of an expert GEMM over a buffer of `cap` rows (K > 0), or of its weight gradient (K = 0), on `sms` SMs.
+// Host only (no CUDA call): CTAs per tile, 1 or 2, of an expert GEMM over a buffer of `cap` rows (K > 0) of which as many are expected as it holds, or of its weight
+// gradient (K = 0), on `sms` SMs.
 extern "C" int lb_gemm_ragged_ctas_per_tile(int LE, int cap, int N, int K, int sms) {
   if (LE < 1 || LE > MAX_PROBLEMS || cap <= 0 || N <= 0 || K < 0 || sms < 1) return LB_ERR_SHAPE;
-  return K ? ragged_cg(LE, cap, N, (K + BK - 1) / BK, sms) : ragged_wgrad_cg(LE, cap, sms);
+  const int rows = ragged_rows(LE, cap, 0);
+  return K ? ragged_cg(LE, rows, N, (K + BK - 1) / BK, sms) : ragged_wgrad_cg(LE, rows, sms);
 }
 
 // Expert GEMMs over ragged row segments (see gemm_ragged_kernel).  seg: device table of 2 * LE + 2
@@ -1233,7 +1238,8 @@ extern "C" int lb_gemm_ragged_ctas_per_tile(int LE, int cap, int N, int K, int s
 //          ([N, K], or [K, N] with b_mn), all with leading dimension ldb.  wait_flag (or null): device
 //          word that must reach wait_target before A is read.
 //          epi, C2, ldc2 and half as in lb_gemm_grouped_epi (matrices of cap rows).
-extern "C" int lb_gemm_ragged_epi(const void* A, const void* const* B, void* C, const void* seg, int LE, int cap, int N, int K,
+//  rows: how many there will be in all segments, as far as the caller can tell, or 0 (as many as fit); it decides which form runs, not what is computed.
+extern "C" int lb_gemm_ragged_epi(const void* A, const void* const* B, void* C, const void* seg, int LE, int cap, int rows, int N, int K,
                                   long long lda, long long ldb, long long ldc, int b_mn, int epi, void* C2, long long ldc2, int half,
                                   const void* wait_flag, unsigned int wait_target, void* stream) {
   if (LE < 1 || LE > MAX_PROBLEMS || cap <= 0 || N <= 0 || K <= 0) return LB_ERR_SHAPE;
@@ -1259,19 +1265,19 @@ extern "C" int lb_gemm_ragged_epi(const void* A, const void* const* B, void* C, 
   rp.mode = 0; rp.accumulate = 0; rp.cap = cap;
   rp.tiles_n = (N + BN - 1) / BN; rp.tiles_m_w = 0; rp.num_kb = (K + BK - 1) / BK;
   rp.wait_flag = (const unsigned int*)wait_flag; rp.wait_target = wait_target; rp.wait_ns = g_lb_flag_wait_ns;
-  return launch_ragged(ragged_cg(LE, cap, N, rp.num_kb, lb_num_sms()), !wait_flag, rp, (cudaStream_t)stream);
+  return launch_ragged(ragged_cg(LE, ragged_rows(LE, cap, rows), N, rp.num_kb, lb_num_sms()), !wait_flag, rp, (cudaStream_t)stream);
 }
 
 extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, const void* seg, int LE, int cap, int N, int K,
                               long long lda, long long ldb, long long ldc, int b_mn, const void* wait_flag,
                               unsigned int wait_target, void* stream) {
-  return lb_gemm_ragged_epi(A, B, C, seg, LE, cap, N, K, lda, ldb, ldc, b_mn, 0, nullptr, 0, 0, wait_flag, wait_target, stream);
+  return lb_gemm_ragged_epi(A, B, C, seg, LE, cap, 0, N, K, lda, ldb, ldc, b_mn, 0, nullptr, 0, 0, wait_flag, wait_target, stream);
 }
 
 //  Weight gradients: C_e [Nw, Kw] (+)= dY[rows of e, Nw]^T . X[rows of e, Kw]; C: host array of LE
 //  gradient pointers with leading dimension ldc.  Without accumulate every C_e is written whole (zeros for an expert
 //  without rows).
-extern "C" int lb_gemm_ragged_wgrad(const void* dY, const void* X, void* const* C, const void* seg, int LE, int cap, int Nw,
+extern "C" int lb_gemm_ragged_wgrad(const void* dY, const void* X, void* const* C, const void* seg, int LE, int cap, int rows, int Nw,
                                     int Kw, long long lddy, long long ldx, long long ldc, int accumulate, void* stream) {
   if (LE < 1 || LE > MAX_PROBLEMS || cap <= 0 || Nw <= 0 || Kw <= 0) return LB_ERR_SHAPE;
   if ((lddy % 8) || (ldx % 8) || (ldc % 8) || (Nw % 8) || (Kw % 8)) return LB_ERR_SHAPE;
@@ -1279,7 +1285,7 @@ extern "C" int lb_gemm_ragged_wgrad(const void* dY, const void* X, void* const* 
   for (int e = 0; e < LE; e++)
     if (!C[e] || ((uintptr_t)C[e] & 15)) return LB_ERR_ARG;
   static thread_local RaggedParams rp;
-  const int cg = ragged_wgrad_cg(LE, cap, lb_num_sms());
+  const int cg = ragged_wgrad_cg(LE, ragged_rows(LE, cap, rows), lb_num_sms());
   int rc = bw::make_map_bf16(&rp.ta, dY, (uint64_t)Nw, (uint64_t)cap, (uint64_t)lddy, 64, BK);
   if (rc) return rc;
   rc = bw::make_map_bf16(&rp.tb[0], X, (uint64_t)Kw, (uint64_t)cap, (uint64_t)ldx, 64, BK);

@@ -143,16 +143,16 @@ def _ptr_array(tensors: Sequence[torch.Tensor]):
     return arr
 
 
-def _ragged(A, B_list, C, seg, LE, cap, N, K, b_mn, wait_flag=0, wait_target=0, epi=0, c2=None, half=0):
-    """``epi``, ``c2`` and ``half``: a SwiGLU epilogue, as in ``functional.gemm_grouped``."""
+def _ragged(A, B_list, C, seg, LE, cap, N, K, b_mn, wait_flag=0, wait_target=0, epi=0, c2=None, half=0, rows=0):
+    """``epi``, ``c2`` and ``half``: a SwiGLU epilogue, as in ``functional.gemm_grouped``.  ``rows``: how many are expected (0: as many as fit)."""
     ldb = B_list[0].stride(0)
-    native.call("lb_gemm_ragged_epi", A.data_ptr(), _ptr_array(B_list), C.data_ptr(), seg.data_ptr(), LE, cap, N, K,
+    native.call("lb_gemm_ragged_epi", A.data_ptr(), _ptr_array(B_list), C.data_ptr(), seg.data_ptr(), LE, cap, rows, N, K,
                 A.stride(0), ldb, C.stride(0), int(b_mn), epi, native.ptr(c2), 0 if c2 is None else c2.stride(0), half,
                 wait_flag, wait_target, native.stream_ptr())
 
 
-def _ragged_wgrad(dY, X, C_list, seg, LE, cap, Nw, Kw, accumulate=True):
-    native.call("lb_gemm_ragged_wgrad", dY.data_ptr(), X.data_ptr(), _ptr_array(C_list), seg.data_ptr(), LE, cap, Nw, Kw,
+def _ragged_wgrad(dY, X, C_list, seg, LE, cap, Nw, Kw, accumulate=True, rows=0):
+    native.call("lb_gemm_ragged_wgrad", dY.data_ptr(), X.data_ptr(), _ptr_array(C_list), seg.data_ptr(), LE, cap, rows, Nw, Kw,
                 dY.stride(0), X.stride(0), C_list[0].stride(0), int(accumulate), native.stream_ptr())
 
 
@@ -162,7 +162,7 @@ class _FusedMoE(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gate_w, meta, *expert_ws):
         ws: Workspace = meta["ws"]
-        E, k, LE, cap, n, me = meta["E"], meta["k"], meta["LE"], ws.cap, ws.n, ws.rank
+        E, k, LE, cap, n, me, expected = meta["E"], meta["k"], meta["LE"], ws.cap, ws.n, ws.rank, meta["rows"]
         T, H = x.shape
         I = expert_ws[0].shape[0]
         dev = x.device
@@ -198,8 +198,8 @@ class _FusedMoE(torch.autograd.Function):
         downs = [expert_ws[3 * e + 2] for e in range(LE)]                               # [H, I]
         gu = torch.empty(cap, 2 * I, dtype=_BF16, device=dev)
         a = torch.empty(cap, I, dtype=_BF16, device=dev)
-        _ragged(xbuf, ups, gu, seg, LE, cap, 2 * I, H, False, ws.ctrl_ptrs[me] + 64, ws.arr_x, epi=1, c2=a, half=I)
-        _ragged(a, downs, ybuf, seg, LE, cap, H, I, False)
+        _ragged(xbuf, ups, gu, seg, LE, cap, 2 * I, H, False, ws.ctrl_ptrs[me] + 64, ws.arr_x, epi=1, c2=a, half=I, rows=expected)
+        _ragged(a, downs, ybuf, seg, LE, cap, H, I, False, rows=expected)
         out = torch.empty(T, H, dtype=_BF16, device=dev)
         ws.epoch_y += 1
         native.call("lb_moe_pull", out.data_ptr(), wts.data_ptr(), idx.data_ptr(), rows.data_ptr(), 0, 0, T, H, E, k, n,
@@ -213,7 +213,7 @@ class _FusedMoE(torch.autograd.Function):
         x, gate_w, probs, idx, wts, rows, seg, frac, gu, a, *expert_ws = ctx.saved_tensors
         meta, slot = ctx.meta, ctx.slot
         ws: Workspace = meta["ws"]
-        E, k, LE, cap, n, me = meta["E"], meta["k"], meta["LE"], ws.cap, ws.n, ws.rank
+        E, k, LE, cap, n, me, expected = meta["E"], meta["k"], meta["LE"], ws.cap, ws.n, ws.rank, meta["rows"]
         T, H = x.shape
         I = expert_ws[0].shape[0]
         dev = x.device
@@ -248,11 +248,11 @@ class _FusedMoE(torch.autograd.Function):
         downs = [expert_ws[3 * e + 2] for e in range(LE)]
         # down projection: da = dy W2, stored as the gradients of g | u; dW2 += dy^T a
         dgu = torch.empty(cap, 2 * I, dtype=_BF16, device=dev)
-        _ragged(dybuf, downs, dgu, seg, LE, cap, I, H, True, ws.ctrl_ptrs[me] + 68, ws.arr_dy, epi=2, c2=gu, half=I)
-        _ragged_wgrad(dybuf, a, g_down, seg, LE, cap, H, I, direct)
+        _ragged(dybuf, downs, dgu, seg, LE, cap, I, H, True, ws.ctrl_ptrs[me] + 68, ws.arr_dy, epi=2, c2=gu, half=I, rows=expected)
+        _ragged_wgrad(dybuf, a, g_down, seg, LE, cap, H, I, direct, expected)
         # gate | up projection: dx_rows = dgu [W1; W3], d[W1; W3] += dgu^T x_rows
-        _ragged(dgu, ups, dxbuf, seg, LE, cap, H, 2 * I, True)
-        _ragged_wgrad(dgu, xbuf, g_up, seg, LE, cap, 2 * I, H, direct)
+        _ragged(dgu, ups, dxbuf, seg, LE, cap, H, 2 * I, True, rows=expected)
+        _ragged_wgrad(dgu, xbuf, g_up, seg, LE, cap, 2 * I, H, direct, expected)
         # router
         dx_r = torch.empty(T, H, dtype=_BF16, device=dev)
         dwg = torch.zeros(E, H, dtype=_F32, device=dev)
@@ -279,6 +279,17 @@ class _FusedMoE(torch.autograd.Function):
         return (dx, dwg.to(gate_w.dtype), None, *egrads)
 
 
+def capacity(T: int, topk: int, n: int, LE: int, capacity_factor: float):
+    """Rows of the exchange buffers of ``n`` ranks of ``T`` tokens each, and how many of them an even routing fills: as many copies
+    arrive as leave."""
+    if n == 1 and capacity_factor >= 1.0:
+        held = rows = _up(T * topk, 128)             # one rank can never receive more than its own copies
+    else:
+        held = _up(int(capacity_factor * T * topk), 128)
+        rows = max(1, min(held, T * topk))
+    return held + LE * 128, rows
+
+
 def fused_moe(x: torch.Tensor, gate_w: torch.Tensor, expert_ws: Sequence[torch.Tensor], num_experts: int, topk: int,
               group, layer_key: int, capacity_factor: float = 2.0):
     """x [T, H] -> (out [T, H], aux loss [1]).  expert_ws: (w1, w3, w2) of every local expert, in
@@ -286,10 +297,7 @@ def fused_moe(x: torch.Tensor, gate_w: torch.Tensor, expert_ws: Sequence[torch.T
     T, H = x.shape
     n = dist.get_world_size(group) if group is not None else 1
     LE = num_experts // n
-    if n == 1 and capacity_factor >= 1.0:
-        cap = _up(T * topk, 128) + LE * 128          # one rank can never receive more than its own copies
-    else:
-        cap = _up(int(capacity_factor * T * topk), 128) + LE * 128
+    cap, rows = capacity(T, topk, n, LE, capacity_factor)
     ws = workspace(group, H, cap, num_experts, x.device)
-    meta = {"ws": ws, "E": num_experts, "k": topk, "LE": LE, "layer_key": layer_key}
+    meta = {"ws": ws, "E": num_experts, "k": topk, "LE": LE, "layer_key": layer_key, "rows": rows}
     return _FusedMoE.apply(x, gate_w, meta, *expert_ws)

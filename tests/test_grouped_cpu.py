@@ -332,7 +332,33 @@ def test_outputs_that_are_missing(epi):
     for C in (0, 4096):
         head = (1, V(4096), V(4096), V(C), I(256), I(n), I(512), L(512), L(512), L(2 * half), I(0), I(0), I(0), I(epi), V(4096), L(2 * half), I(half))
         refused = [lib.lb_gemm_grouped_epi(*head, None), lib.lb_gemm_split(*head, 1, None),
-                   lib.lb_gemm_ragged_epi(4096, V(4096), C, 4096, 1, 256, n, 512, 512, 512, 2 * half, 0, epi, 4096, 2 * half, half, None, 0, None)]
+                   lib.lb_gemm_ragged_epi(4096, V(4096), C, 4096, 1, 256, 0, n, 512, 512, 512, 2 * half, 0, epi, 4096, 2 * half, half, None, 0, None)]
         if epi == 0:
-            refused.append(lib.lb_gemm_ragged_wgrad(4096, 4096, V(C), 4096, 1, 256, 256, 512, 256, 512, 512, 0, None))
+            refused.append(lib.lb_gemm_ragged_wgrad(4096, 4096, V(C), 4096, 1, 256, 0, 256, 512, 256, 512, 512, 0, None))
         assert [r == -1 for r in refused] == [C == 0 and epi != 1] * len(refused), (C, refused)
+
+
+def test_expert_gemms_are_planned_for_the_rows_that_arrive(monkeypatch):
+    """Several ranks' exchange buffers hold twice what an even routing brings (capacity factor 2): the form of the expert GEMMs goes by the latter."""
+    from lightron_b200.parallel import ep_fused
+    lib = native._load()
+    if lib is None:
+        pytest.skip("native library not built")
+    assert ep_fused.capacity(1000, 2, 1, 8, 2.0) == (2048 + 8 * 128, 2048)
+    assert ep_fused.capacity(1000, 2, 4, 2, 2.0) == (4096 + 2 * 128, 2000) and ep_fused.capacity(1000, 2, 4, 2, 0.5) == (1024 + 2 * 128, 1000 + 24)
+    T, topk, LE, H = 1024, 2, 8, 2048                    # 256 rows per expert: weight gradients in pairs take 59 us, in single CTAs 48
+    cap, rows = ep_fused.capacity(T, topk, 8, LE, 2.0)
+    form = lambda held, n, k: lib.lb_gemm_ragged_ctas_per_tile(LE, held, n, k, 148)
+    assert form(cap, H, 0) == 2 and form(rows + LE * 128, H, 0) == 1
+    seen, calls = [], []
+    monkeypatch.setattr(ep_fused, "workspace", lambda *a: None)
+    monkeypatch.setattr(ep_fused._FusedMoE, "apply", lambda *a: seen.append(a[2]))
+    monkeypatch.setattr(ep_fused.dist, "get_world_size", lambda group: 8)
+    ep_fused.fused_moe(torch.zeros(T, H), None, (), 8 * LE, topk, object(), 0)
+    assert seen[0]["rows"] == rows == T * topk
+    monkeypatch.setattr(native, "call", lambda name, *a: calls.append((name, a)))
+    monkeypatch.setattr(native, "stream_ptr", lambda: 0)
+    t = torch.zeros(8, 8, dtype=torch.bfloat16)
+    ep_fused._ragged(t, [t], t, t, LE, cap, H, 512, False, rows=rows)
+    ep_fused._ragged_wgrad(t, t, [t], t, LE, cap, 512, H, False, rows)
+    assert [a[4:9] for _, a in calls] == [(LE, cap, rows, H, 512), (LE, cap, rows, 512, H)]

@@ -800,10 +800,36 @@ def test_ragged_activation_without_gate_and_up(H, I, counts, ctas):
     gu, act, alone = (torch.full((cap, n), 7.0, device="cuda", dtype=torch.bfloat16) for n in (2 * I, I, I))
     ep_fused._ragged(x, up, gu, table, LE, cap, 2 * I, H, False, epi=1, c2=act, half=I)
     gu.fill_(3.0)
-    native.call("lb_gemm_ragged_epi", x.data_ptr(), ep_fused._ptr_array(up), 0, table.data_ptr(), LE, cap, 2 * I, H, H, H, 2 * I, 0, 1,
+    native.call("lb_gemm_ragged_epi", x.data_ptr(), ep_fused._ptr_array(up), 0, table.data_ptr(), LE, cap, 0, 2 * I, H, H, H, 2 * I, 0, 1,
                 alone.data_ptr(), I, I, 0, 0, native.stream_ptr())
     _status_ok()
     assert torch.equal(alone, act) and bool((gu == 3.0).all())
+
+
+@pytest.mark.parametrize("rows,ctas", [(0, 2), (300, 1), (8192, 2)])
+def test_expected_rows_choose_the_form_alone(rows, ctas):
+    """Fewer or more rows than expected are computed all the same."""
+    from lightron_b200.ops import native
+    from lightron_b200.parallel import ep_fused
+    H, N, counts, seg, cap = 2048, 4104, (500, 0, 129, 1290), (0, 512, 512, 768), 2560
+    LE, lib, sms = len(counts), native.require(), native.sm_count()
+    held = rows + LE * 128 if rows else cap
+    assert [lib.lb_gemm_ragged_ctas_per_tile(LE, held, *a, sms) for a in ((N, H), (H, 0))] == [ctas] * 2
+    table = torch.tensor([*seg, *counts, 2176, sum(counts)], dtype=torch.int32, device="cuda")
+    x, dy = torch.zeros(cap, H, dtype=torch.bfloat16, device="cuda"), torch.zeros(cap, N, dtype=torch.bfloat16, device="cuda")
+    for o, c in zip(seg, counts):
+        x[o:o + c], dy[o:o + c] = _rand(c, H, seed=c), _rand(c, N, seed=c + 1)
+    w = [_rand(N, H, scale=H ** -0.5, seed=10 + e) for e in range(LE)]
+    y = torch.full((cap, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    dw = [torch.full((N, H), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(LE)]
+    ep_fused._ragged(x, w, y, table, LE, cap, N, H, False, rows=rows)
+    ep_fused._ragged_wgrad(dy, x, dw, table, LE, cap, N, H, False, rows)
+    _status_ok()
+    assert (y[2176:] == 7).all()
+    for e, (o, c) in enumerate(zip(seg, counts)):
+        r, grad = slice(o, o + c), dy[o:o + c].double().t() @ x[o:o + c].double()
+        assert _rel(dw[e], grad) < 5e-3 if c else not dw[e].any()
+        assert not c or _rel(y[r], x[r].double() @ w[e].double().t()) < 5e-3
 
 
 @pytest.mark.parametrize("n", [0, 1, 15, 16, 17, 4095, 4096, 4111, 1 << 20, (1 << 20) + 7])

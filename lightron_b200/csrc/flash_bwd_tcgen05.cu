@@ -700,8 +700,8 @@ int launch_fa_bwd(const void* q, const void* k, const void* v, const FaBwdParams
   if ((rc = make_map_bf16(&tk, k, (uint64_t)p.hkv * D, kv_rows, (uint64_t)k_ts, 64, 128))) return rc;
   if ((rc = make_map_bf16(&tv, v, (uint64_t)p.hkv * D, kv_rows, (uint64_t)v_ts, 64, 128))) return rc;
   if ((rc = make_map_bf16(&tdo, p.dout, (uint64_t)p.hq * D, (uint64_t)p.B * p.Sq, (uint64_t)p.do_ts, 64, 128))) return rc;
-  if ((rc = make_map_bf16_3d(&tdk, p.dk, (uint64_t)p.hkv * D, (uint64_t)p.Sk, (uint64_t)p.B, (uint64_t)p.dk_ts, 64, 32))) return rc;
-  if ((rc = make_map_bf16_3d(&tdv, p.dv, (uint64_t)p.hkv * D, (uint64_t)p.Sk, (uint64_t)p.B, (uint64_t)p.dv_ts, 64, 32))) return rc;
+  if ((rc = make_map_bf16_3d(&tdk, p.dk, (uint64_t)p.hkv * D, (uint64_t)p.Sk, (uint64_t)p.Sk, (uint64_t)p.B, (uint64_t)p.dk_ts, 64, 32))) return rc;
+  if ((rc = make_map_bf16_3d(&tdv, p.dv, (uint64_t)p.hkv * D, (uint64_t)p.Sk, (uint64_t)p.Sk, (uint64_t)p.B, (uint64_t)p.dv_ts, 64, 32))) return rc;
   static bool attr = false;
   if (!attr) {
     // the register split must fit in what the launch allocates, or it would wait for registers that nobody gives back

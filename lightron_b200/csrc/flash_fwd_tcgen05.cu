@@ -277,7 +277,7 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
               if (!lbcomm::flag_wait_ge(p.kv_flags + (long long)t.b * (p.kv_brows >> 7) + j, p.flag_target, p.wait_ns)) { *abort_flag = 1; ok = false; break; }
               asm volatile("fence.proxy.async;" ::: "memory");
             }
-            const int row = t.b * p.kv_brows + j * C::BN;
+            const int key0 = j * C::BN;
 #pragma unroll
             for (int u = 0; u < C::UNITS; u++) {
               if (ok && !mbar_wait(empty(slot), phase ^ 1u, abort_flag)) ok = false;
@@ -285,12 +285,12 @@ fa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
               const uint32_t dst = sbase + C::OFF_RING + slot * C::SLOT_BYTES, bar = full(slot);
               mbar_expect_tx(bar, C::SLOT_BYTES);
               if (u < C::ATOMS) {
-                tma_load_2d(dst, &tk, t.hk * D + u * 64, row, bar);               // box 128 keys x 64 columns
+                tma_load_2d(dst, &tk, t.hk * D + u * 64, t.b * p.kv_brows + key0, bar);               // box 128 keys x 64 columns
               } else {
                 const int half = u - C::ATOMS;                                    // head_dim 128: keys 0-63, then 64-127
 #pragma unroll
                 for (int a = 0; a < 2; a++)                                       // boxes 64 keys x 64 columns
-                  tma_load_2d(dst + a * 8192, &tv, t.hk * D + (D == 128 ? a * 64 : 0), row + (D == 128 ? half * 64 : a * 64), bar);
+                  tma_load_3d(dst + a * 8192, &tv, t.hk * D + (D == 128 ? a * 64 : 0), key0 + (D == 128 ? half * 64 : a * 64), t.b, bar);
               }
               if (++slot == C::SLOTS) { slot = 0; phase ^= 1u; }
             }
@@ -613,19 +613,18 @@ fa_fwd_one_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant_
 
   if (warp == 0) {
     if (elect_one()) {
-      const int row = b * p.kv_brows;
       mbar_expect_tx(qk_full, 2 * C::ATOMS * C::SLOT_BYTES);
 #pragma unroll
       for (int a = 0; a < C::ATOMS; a++) {
         tma_load_2d(sbase + C::OFF_Q + a * C::SLOT_BYTES, &tq, h * D + a * 64, b * p.Sq + m0, qk_full);
-        tma_load_2d(sbase + C::OFF_K + a * C::SLOT_BYTES, &tk, hk * D + a * 64, row, qk_full);
+        tma_load_2d(sbase + C::OFF_K + a * C::SLOT_BYTES, &tk, hk * D + a * 64, b * p.kv_brows, qk_full);
       }
       mbar_expect_tx(v_full, C::ATOMS * C::SLOT_BYTES);
 #pragma unroll
       for (int half = 0; half < 2; half++)
 #pragma unroll
         for (int a = 0; a < C::ATOMS; a++)                   // boxes 64 keys x 64 columns
-          tma_load_2d(sbase + C::OFF_V + (half * C::ATOMS + a) * 8192, &tv, hk * D + a * 64, row + half * 64, v_full);
+          tma_load_3d(sbase + C::OFF_V + (half * C::ATOMS + a) * 8192, &tv, hk * D + a * 64, half * 64, b, v_full);
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -754,8 +753,9 @@ int launch_fa_fwd(const void* q, const void* k, const void* v, FaFwdParams p, co
   const uint64_t kv_rows = (uint64_t)(p.B - 1) * p.kv_brows + p.Sk;
   if ((rc = make_map_bf16(&tq, q, (uint64_t)p.hq * D, (uint64_t)p.B * p.Sq, (uint64_t)q_ts, 64, 128))) return rc;
   if ((rc = make_map_bf16(&tk, k, (uint64_t)p.hkv * D, kv_rows, (uint64_t)k_ts, 64, 128))) return rc;
-  if ((rc = make_map_bf16(&tv, v, (uint64_t)p.hkv * D, kv_rows, (uint64_t)v_ts, 64, 64))) return rc;
-  if ((rc = make_map_bf16_3d(&to, p.o, (uint64_t)p.hq * D, (uint64_t)p.Sq, (uint64_t)p.B, (uint64_t)p.o_ts, 64, 32))) return rc;
+  // (keys past a sequence's last have weights of zero, but zero times the infinity or NaN of the next sequence's V is NaN: they are loaded as zeros)
+  if ((rc = make_map_bf16_3d(&tv, v, (uint64_t)p.hkv * D, (uint64_t)p.Sk, (uint64_t)p.kv_brows, (uint64_t)p.B, (uint64_t)v_ts, 64, 64))) return rc;
+  if ((rc = make_map_bf16_3d(&to, p.o, (uint64_t)p.hq * D, (uint64_t)p.Sq, (uint64_t)p.Sq, (uint64_t)p.B, (uint64_t)p.o_ts, 64, 32))) return rc;
   static bool attr = false;
   if (!attr) {
     // the register split must fit in what the launch allocates, or it would wait for registers that nobody gives back

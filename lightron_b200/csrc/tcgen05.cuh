@@ -96,6 +96,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
 // The same box into L2 only: a hint, which may run while another kernel still writes the matrix.
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
@@ -409,10 +415,10 @@ inline int make_map_bf16(CUtensorMap* m, const void* base, uint64_t inner, uint6
   const cuuint32_t box[2] = {box_inner, box_outer};
   return make_map_bf16_nd(m, base, 2, dims, strides, box);
 }
-// `batches` matrices of `rows` rows one behind the other: a tile that is stored ends with its own matrix.
-inline int make_map_bf16_3d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint64_t batches, uint64_t ld,
+// `batches` matrices of `rows` rows, `apart` rows from one to the next: a tile ends with its own matrix, where a store stops and a load fills with zeros.
+inline int make_map_bf16_3d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint64_t apart, uint64_t batches, uint64_t ld,
                             uint32_t box_inner, uint32_t box_rows) {
-  const cuuint64_t dims[3] = {inner, rows, batches}, strides[2] = {ld * 2, rows * ld * 2};
+  const cuuint64_t dims[3] = {inner, rows, batches}, strides[2] = {ld * 2, apart * ld * 2};
   const cuuint32_t box[3] = {box_inner, box_rows, 1};
   return make_map_bf16_nd(m, base, 3, dims, strides, box);
 }

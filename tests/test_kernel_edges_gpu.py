@@ -264,6 +264,40 @@ def test_attention_bad_scores_stay_in_their_rows(d, bad):
         assert torch.equal(o[0, :, 0].isnan().all(-1), want) and torch.equal(o[0, :, 0].isnan().any(-1), want), key
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("S,hq,hkv,causal", [(100, 4, 2, True), (100, 200, 200, False), (300, 4, 4, True), (129, 2, 1, False)])
+def test_attention_of_a_sequence_beside_a_bad_one(S, hq, hkv, causal, bad, d):
+    """Keys and values that are not finite stay in their sequence, also where the one before it ends inside a tile (with one key block and few
+    or many tiles, and with several)."""
+    from lightron_b200.ops import functional as OF
+    q, k, v = _rand(3, S, hq, d, seed=1), _rand(3, S, hkv, d, seed=2), _rand(3, S, hkv, d, seed=3)
+    want = OF.flash_fwd_native(q, k, v, causal, d ** -0.5)
+    for t in (k, v):
+        keep = t[1, 0].clone()
+        t[1, 0] = bad
+        for g, w in zip(OF.flash_fwd_native(q, k, v, causal, d ** -0.5), want):
+            assert torch.equal(g[::2], w[::2])
+        t[1, 0] = keep
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_attention_over_a_prefix_before_anything_else(d):
+    """What lies behind the first Sk keys of a longer buffer does not matter, whatever it is."""
+    from lightron_b200.ops import native
+    B, n, Sk, S, hq, hkv = 2, 200, 300, 640, 4, 2
+    q, kb, vb = _rand(B, n, hq, d, seed=1), _rand(B, S, hkv, d, seed=2), _rand(B, S, hkv, d, seed=3)
+    flags, outs = torch.full((B, S // 128), 5, dtype=torch.int32, device="cuda"), []
+    for rest in (0.0, float("nan")):
+        kb[:, Sk:], vb[:, Sk:] = rest, rest
+        o, lse = torch.empty_like(q), torch.empty(B, hq, n, device="cuda")
+        native.call("lb_flash_fwd_cp", q.data_ptr(), kb.data_ptr(), vb.data_ptr(), o.data_ptr(), lse.data_ptr(), B, n, Sk, S, hq, hkv, d,
+                    hq * d, hq * d, d ** -0.5, 1, flags.data_ptr(), 5, 0, 0, 0, 0, 0, 1, 0, None, None, None, 0, native.stream_ptr())
+        outs.append((o, lse))
+    _status_ok()
+    assert all(torch.equal(a, b) for a, b in zip(*outs)) and bool(outs[1][0].isfinite().all())
+
+
 # ---- GEMM --------------------------------------------------------------------------------------------
 
 

@@ -114,10 +114,10 @@ template <int D, int COLS>
 __global__ void fa_dq_convert_kernel(const FaBwdParams p) {
   grid_go();
   grid_wait();
-  const int lane = threadIdx.x & 31;
-  long long w0 = 0;                                            // warps' pieces of work ahead of those of dQ
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long threads = (long long)gridDim.x * blockDim.x;
+  long long start = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if constexpr (COLS > 0) {
+    const int lane = threadIdx.x & 31;
     constexpr int G = D / COLS, U = 64 / COLS, V = COLS / 4;      // U * V 16-byte loads in flight
     const int off = p.Sk - p.Sq, n_mblocks = (p.Sq + 127) / 128, n_nblk = (p.Sk + 127) / 128, rep = p.hq / p.hkv, pairs = p.hkv * p.B;
     __shared__ int s_first[MAX_CUT_BLOCKS + 1];                // parts ahead of a key block's
@@ -137,9 +137,8 @@ __global__ void fa_dq_convert_kernel(const FaBwdParams p) {
     }
     __syncthreads();
     const int pieces = 2 * pairs * n_nblk * 4 * G;             // (bwd_chunk() cuts launches of few key blocks)
-    w0 = pieces;
-    for (long long at = warp; at < pieces; at += warps) {      // (dK or dV, key block, pair, quad, COLS columns)
-      const int w = (int)at, g = w % G, quad = (w / G) & 3, tile = w / (4 * G);
+    for (; start < 32LL * pieces; start += threads) {          // (dK or dV, key block, pair, quad, COLS columns)
+      const int w = (int)(start >> 5), g = w % G, quad = (w / G) & 3, tile = w / (4 * G);
       const int pair = tile % pairs, block = (tile / pairs) % n_nblk, dv = tile / pairs / n_nblk;
       const int row = block * 128 + quad * 32 + lane;
       if (row >= p.Sk) continue;
@@ -169,13 +168,14 @@ __global__ void fa_dq_convert_kernel(const FaBwdParams p) {
 #pragma unroll
       for (int k = 0; k < COLS / 8; k++) *reinterpret_cast<uint4*>(o + k * 8) = pack8(f + k * 8);
     }
+    start -= 32LL * pieces;                                    // dQ's pieces come next
   }
   constexpr int CPR = D / 32;                                  // 32-column chunks per row
   const int n_mblocks = (p.Sq + 127) / 128;
-  const long long total = w0 + (long long)p.B * p.hq * n_mblocks * 4 * CPR;
-  // (a warp's next piece after those of dK and dV)
-  for (long long at = warp < w0 ? warp + (w0 - warp + warps - 1) / warps * warps : warp; at < total; at += warps) {
-    const long long w = at - w0;                               // (tile, quad, chunk): the accumulator's order
+  const long long total = (long long)p.B * p.hq * n_mblocks * 128 * CPR;
+  for (long long idx = start; idx < total; idx += threads) {
+    const int lane = (int)(idx & 31);
+    const long long w = idx >> 5;                              // (tile, quad, chunk): the accumulator's order
     const int chunk = (int)(w % CPR), quad = (int)((w / CPR) & 3);
     const long long tile = w / (CPR * 4);
     const int mblock = (int)(tile % n_mblocks);
@@ -184,11 +184,11 @@ __global__ void fa_dq_convert_kernel(const FaBwdParams p) {
     if (row >= p.Sq) continue;
     const int h = (int)(bh % p.hq);
     const long long b = bh / p.hq;
-    const float4* from = reinterpret_cast<const float4*>(p.dq_acc) + (w * 8) * 32 + lane;
+    const float4* at = reinterpret_cast<const float4*>(p.dq_acc) + (w * 8) * 32 + lane;
     float f[32];
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-      const float4 v = from[k * 32];
+      const float4 v = at[k * 32];
       f[4 * k] = v.x; f[4 * k + 1] = v.y; f[4 * k + 2] = v.z; f[4 * k + 3] = v.w;
     }
     bf16* o = p.dq + (b * p.Sq + row) * p.dq_ts + (long long)h * D + chunk * 32;

@@ -249,7 +249,7 @@ enum : int { WHOLE, PARTS_OF, ALONE };
 template <int D, int FORM>
 __global__ void __launch_bounds__(512, 1)
 fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
-                 const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tdk,
+                 const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tdo_end, const __grid_constant__ CUtensorMap tdk,
                  const __grid_constant__ CUtensorMap tdv, const FaBwdParams p) {
   using C = BwdCfg<D>;
   constexpr bool PARTS = FORM == PARTS_OF;
@@ -341,10 +341,11 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       mbar_expect_tx(kv_full, 2 * C::TILE_BYTES);
 #pragma unroll
       for (int a = 0; a < C::ATOMS; a++) {
-        tma_load_2d(sbase + C::OFF_K + a * C::ATOM_BYTES, &tk, hk * D + a * 64, b * p.kv_brows + n0, kv_full);
-        tma_load_2d(sbase + C::OFF_V + a * C::ATOM_BYTES, &tv, hk * D + a * 64, b * p.kv_brows + n0, kv_full);
+        tma_load_3d(sbase + C::OFF_K + a * C::ATOM_BYTES, &tk, hk * D + a * 64, n0, b, kv_full);
+        tma_load_3d(sbase + C::OFF_V + a * C::ATOM_BYTES, &tv, hk * D + a * 64, n0, b, kv_full);
       }
       bool ok = true;
+      const int ragged = p.Sq % C::BM ? n_mblocks - 1 : -1;
       int h = h_first, mb = mb_start, st = 0, dst = 0;
       uint32_t ph = 1u, dph = 1u;
       for (int it = 0; it < total_it; it++) {
@@ -352,13 +353,14 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
         mbar_expect_tx(q_full(st), C::TILE_BYTES + 1024);
 #pragma unroll
         for (int a = 0; a < C::ATOMS; a++)
-          tma_load_2d(sbase + C::OFF_Q + st * C::TILE_BYTES + a * C::ATOM_BYTES, &tq, h * D + a * 64, b * p.Sq + mb * C::BM, q_full(st));
+          tma_load_3d(sbase + C::OFF_Q + st * C::TILE_BYTES + a * C::ATOM_BYTES, &tq, h * D + a * 64, mb * C::BM, b, q_full(st));
         bulk_load(sbase + C::OFF_ST + st * 1024, p.stats + (((long long)b * p.hq + h) * n_mblocks + mb) * 256, 1024, q_full(st));
         if (!mbar_wait(do_empty(dst), dph, abort_flag)) { ok = false; break; }
         mbar_expect_tx(do_full(dst), C::TILE_BYTES);
 #pragma unroll
         for (int a = 0; a < C::ATOMS; a++)
-          tma_load_2d(sbase + C::OFF_DO + dst * C::TILE_BYTES + a * C::ATOM_BYTES, &tdo, h * D + a * 64, b * p.Sq + mb * C::BM, do_full(dst));
+          if (mb == ragged) tma_load_3d(sbase + C::OFF_DO + dst * C::TILE_BYTES + a * C::ATOM_BYTES, &tdo_end, h * D + a * 64, mb * C::BM, b, do_full(dst));
+          else tma_load_2d(sbase + C::OFF_DO + dst * C::TILE_BYTES + a * C::ATOM_BYTES, &tdo, h * D + a * 64, b * p.Sq + mb * C::BM, do_full(dst));
         if (++mb == n_mblocks) { mb = mb_first; h++; }
         if (++st == C::QS) { st = 0; ph ^= 1u; }
         if (++dst == C::DS) { dst = 0; dph ^= 1u; }
@@ -693,15 +695,19 @@ template <int D>
 int launch_fa_bwd(const void* q, const void* k, const void* v, const FaBwdParams& p, long long q_ts, long long k_ts,
                   long long v_ts, cudaStream_t s) {
   using C = BwdCfg<D>;
-  CUtensorMap tq, tk, tv, tdo, tdk, tdv;
+  CUtensorMap tq, tk, tv, tdo, tdo_end, tdk, tdv;
   int rc;
-  if ((rc = make_map_bf16(&tq, q, (uint64_t)p.hq * D, (uint64_t)p.B * p.Sq, (uint64_t)q_ts, 64, 128))) return rc;
-  const uint64_t kv_rows = (uint64_t)(p.B - 1) * p.kv_brows + p.Sk;
-  if ((rc = make_map_bf16(&tk, k, (uint64_t)p.hkv * D, kv_rows, (uint64_t)k_ts, 64, 128))) return rc;
-  if ((rc = make_map_bf16(&tv, v, (uint64_t)p.hkv * D, kv_rows, (uint64_t)v_ts, 64, 128))) return rc;
-  if ((rc = make_map_bf16(&tdo, p.dout, (uint64_t)p.hq * D, (uint64_t)p.B * p.Sq, (uint64_t)p.do_ts, 64, 128))) return rc;
-  if ((rc = make_map_bf16_3d(&tdk, p.dk, (uint64_t)p.hkv * D, (uint64_t)p.Sk, (uint64_t)p.Sk, (uint64_t)p.B, (uint64_t)p.dk_ts, 64, 32))) return rc;
-  if ((rc = make_map_bf16_3d(&tdv, p.dv, (uint64_t)p.hkv * D, (uint64_t)p.Sk, (uint64_t)p.Sk, (uint64_t)p.B, (uint64_t)p.dv_ts, 64, 32))) return rc;
+  // (sequence by sequence: rows past a sequence's last are zeros.  Their P and dS are zero, but zero times what the next sequence holds is not, where
+  // that is infinite or NaN.  dO only for blocks that end inside a sequence's tile: a load by the map with a third dimension takes longer, and at d 128 a block
+  // waits for dO: 1 x 8192, 32 / 8 heads 1265 us, now 1254.)
+  const uint64_t B = p.B, Sq = p.Sq, Sk = p.Sk, brows = p.kv_brows, q_cols = (uint64_t)p.hq * D, kv_cols = (uint64_t)p.hkv * D;
+  if ((rc = make_map_bf16_3d(&tq, q, q_cols, Sq, Sq, B, (uint64_t)q_ts, 64, 128))) return rc;
+  if ((rc = make_map_bf16_3d(&tk, k, kv_cols, Sk, brows, B, (uint64_t)k_ts, 64, 128))) return rc;
+  if ((rc = make_map_bf16_3d(&tv, v, kv_cols, Sk, brows, B, (uint64_t)v_ts, 64, 128))) return rc;
+  if ((rc = make_map_bf16(&tdo, p.dout, q_cols, B * Sq, (uint64_t)p.do_ts, 64, 128))) return rc;
+  if ((rc = make_map_bf16_3d(&tdo_end, p.dout, q_cols, Sq, Sq, B, (uint64_t)p.do_ts, 64, 128))) return rc;
+  if ((rc = make_map_bf16_3d(&tdk, p.dk, kv_cols, Sk, Sk, B, (uint64_t)p.dk_ts, 64, 32))) return rc;
+  if ((rc = make_map_bf16_3d(&tdv, p.dv, kv_cols, Sk, Sk, B, (uint64_t)p.dv_ts, 64, 32))) return rc;
   static bool attr = false;
   if (!attr) {
     // the register split must fit in what the launch allocates, or it would wait for registers that nobody gives back
@@ -719,7 +725,7 @@ int launch_fa_bwd(const void* q, const void* k, const void* v, const FaBwdParams
   const long long rows_per_block = 256 / (D / 8), cap = lb_num_sms() * 16;
   const long long pblocks = (rows + rows_per_block - 1) / rows_per_block;
   LB_LAUNCH(fa_bwd_prep_kernel<D>, (int)(pblocks < cap ? pblocks : cap), 256, 0, s, p);
-  LB_LAUNCH(p.chunk ? fa_bwd_tc_kernel<D, PARTS_OF> : p.alone ? fa_bwd_tc_kernel<D, ALONE> : fa_bwd_tc_kernel<D, WHOLE>, (unsigned)grid, C::NTHREADS, C::SMEM, s, tq, tk, tv, tdo, tdk, tdv, p);
+  LB_LAUNCH(p.chunk ? fa_bwd_tc_kernel<D, PARTS_OF> : p.alone ? fa_bwd_tc_kernel<D, ALONE> : fa_bwd_tc_kernel<D, WHOLE>, (unsigned)grid, C::NTHREADS, C::SMEM, s, tq, tk, tv, tdo, tdo_end, tdk, tdv, p);
   if (p.alone) return LB_OK;
   const long long part_rows = p.chunk ? 2LL * p.B * ((p.Sk + 127) / 128 * 128) * p.hkv : 0;
   const int cols = part_rows * (D / 16) < 32 * 4LL * lb_num_sms() ? 8 : 16;      // (16: four warps on an SM have work)

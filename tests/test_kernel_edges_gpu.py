@@ -282,6 +282,34 @@ def test_attention_of_a_sequence_beside_a_bad_one(S, hq, hkv, causal, bad, d):
 
 
 @pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("S,Sk,hq,hkv,causal", [(100, 100, 4, 2, True), (300, 300, 4, 4, True), (129, 129, 2, 1, False), (70, 700, 16, 2, False),
+                                                 (40, 50, 200, 200, False)])
+def test_attention_gradients_of_a_sequence_beside_a_bad_one(S, Sk, hq, hkv, causal, bad, d):
+    """The same for what the backward reads, in whole key blocks, parts and the form of one key block.  dK and dV are the same bits; dQ too
+    where one key block adds to it, and else the same fp32 terms in another order, rounded once."""
+    from lightron_b200.ops import functional as OF
+    q, do = _rand(3, S, hq, d, seed=1), _rand(3, S, hq, d, seed=4)
+    k, v = _rand(3, Sk, hkv, d, seed=2), _rand(3, Sk, hkv, d, seed=3)
+
+    def grads():
+        o, lse = OF.flash_fwd_native(q, k, v, causal, d ** -0.5)
+        for g, w in zip((o, lse), fwd):          # (the forward of these two to the bit: what follows is the backward's alone)
+            g[::2] = w[::2]
+        return OF.flash_bwd_native(q, k, v, o, lse, do, causal, d ** -0.5)
+    fwd = OF.flash_fwd_native(q, k, v, causal, d ** -0.5)
+    want = grads()
+    for t in (q, k, v, do):
+        keep = t[1, 0].clone()
+        t[1, 0] = bad
+        got = grads()
+        t[1, 0] = keep
+        for i, (g, w) in enumerate(zip(got, want)):
+            assert torch.equal(g[::2], w[::2]) if i or Sk <= 128 else _rel(g[::2], w[::2]) < 2.0 ** -8
+    _status_ok()
+
+
+@pytest.mark.parametrize("d", [64, 128])
 def test_attention_over_a_prefix_before_anything_else(d):
     """What lies behind the first Sk keys of a longer buffer does not matter, whatever it is."""
     from lightron_b200.ops import native

@@ -473,11 +473,9 @@ extern "C" int lb_rope(void* t, const void* cosT, const void* sinT, const void* 
 // ---------------------------------------------------------------------------------------
 // SwiGLU on a fused [rows, 2I] gate|up matrix (row stride ld).
 // ---------------------------------------------------------------------------------------
-__global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, int rows, int I, long long ld,
-                                  const int* __restrict__ rows_dev) {
+__global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, int rows, int I, long long ld) {
   grid_go();
   grid_wait();
-  if (rows_dev) rows = max(0, min(rows, *rows_dev));     // row count known only on the device (MoE segments)
   const int vec = I >> 3;
   const long long total = (long long)rows * vec;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -494,10 +492,9 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
 }
 
 __global__ void swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __restrict__ dy, bf16* __restrict__ dgu,
-                                  int rows, int I, long long ld, const int* __restrict__ rows_dev) {
+                                  int rows, int I, long long ld) {
   grid_go();
   grid_wait();
-  if (rows_dev) rows = max(0, min(rows, *rows_dev));
   const int vec = I >> 3;
   const long long total = (long long)rows * vec;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -525,26 +522,17 @@ static inline int ew_blocks(long long total) {
   return (int)(b < 1 ? 1 : b);
 }
 
-// rows_dev (or null): device int; only the first min(rows, *rows_dev) rows are processed.
-extern "C" int lb_swiglu_fwd_dev(const void* gu, void* out, int rows, int I, long long ld, const void* rows_dev, void* stream) {
-  if (I % 8 || ld % 8 || rows <= 0) return LB_ERR_SHAPE;
-  LB_LAUNCH(swiglu_fwd_kernel, ew_blocks((long long)rows * (I / 8)), 256, 0, (cudaStream_t)stream, (const bf16*)gu, (bf16*)out, rows, I, ld,
-            (const int*)rows_dev);
-  return LB_OK;
-}
 extern "C" int lb_swiglu_fwd(const void* gu, void* out, int rows, int I, long long ld, void* stream) {
-  return lb_swiglu_fwd_dev(gu, out, rows, I, ld, nullptr, stream);
+  if (I % 8 || ld % 8 || rows <= 0) return LB_ERR_SHAPE;
+  LB_LAUNCH(swiglu_fwd_kernel, ew_blocks((long long)rows * (I / 8)), 256, 0, (cudaStream_t)stream, (const bf16*)gu, (bf16*)out, rows, I, ld);
+  return LB_OK;
 }
 
-extern "C" int lb_swiglu_bwd_dev(const void* gu, const void* dy, void* dgu, int rows, int I, long long ld,
-                                 const void* rows_dev, void* stream) {
+extern "C" int lb_swiglu_bwd(const void* gu, const void* dy, void* dgu, int rows, int I, long long ld, void* stream) {
   if (I % 8 || ld % 8 || rows <= 0) return LB_ERR_SHAPE;
   LB_LAUNCH(swiglu_bwd_kernel, ew_blocks((long long)rows * (I / 8)), 256, 0, (cudaStream_t)stream, (const bf16*)gu, (const bf16*)dy, (bf16*)dgu,
-            rows, I, ld, (const int*)rows_dev);
+            rows, I, ld);
   return LB_OK;
-}
-extern "C" int lb_swiglu_bwd(const void* gu, const void* dy, void* dgu, int rows, int I, long long ld, void* stream) {
-  return lb_swiglu_bwd_dev(gu, dy, dgu, rows, I, ld, nullptr, stream);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -467,26 +467,26 @@ fa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
           for (int k = 0; k < D / 8; k++) *reinterpret_cast<uint4*>(o + k * 8) = pack8(reinterpret_cast<const float*>(r) + k * 8);
         }
         if (++mb == n_mblocks) mb = 0;
-        continue;
-      }
+      } else {
 #pragma unroll
-      for (int c = 0; c < D / 32; c++) {
-        uint8_t* sp = stg + (c & 1) * C::STG_BYTES;
-        if (lane == 0) bulk_wait_read_but<1>();      // this half of the staging has been read
-        __syncwarp();
+        for (int c = 0; c < D / 32; c++) {
+          uint8_t* sp = stg + (c & 1) * C::STG_BYTES;
+          if (lane == 0) bulk_wait_read_but<1>();      // this half of the staging has been read
+          __syncwarp();
 #pragma unroll
-        for (int k = 0; k < 8; k++)
-          *reinterpret_cast<uint4*>(sp + k * 512 + lane * 16) =
-              make_uint4(r[c * 32 + k * 4], r[c * 32 + k * 4 + 1], r[c * 32 + k * 4 + 2], r[c * 32 + k * 4 + 3]);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          bulk_reduce_add_f32(tile + c * 1024, smem_u32(sp), C::STG_BYTES);
-          bulk_commit();
+          for (int k = 0; k < 8; k++)
+            *reinterpret_cast<uint4*>(sp + k * 512 + lane * 16) =
+                make_uint4(r[c * 32 + k * 4], r[c * 32 + k * 4 + 1], r[c * 32 + k * 4 + 2], r[c * 32 + k * 4 + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            bulk_reduce_add_f32(tile + c * 1024, smem_u32(sp), C::STG_BYTES);
+            bulk_commit();
+          }
         }
+        tile += 128 * D;
+        if (++mb == n_mblocks) { mb = mb_first; tile += (long long)mb_first * (128 * D); }
       }
-      tile += 128 * D;
-      if (++mb == n_mblocks) { mb = mb_first; tile += (long long)mb_first * (128 * D); }
     }
     if (lane == 0) bulk_wait_read_but<0>();
     if (!ok && lane == 0) atomicExch(&g_fab_status[0], 5u);

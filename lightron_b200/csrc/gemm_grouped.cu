@@ -14,7 +14,7 @@
 // of 4 (CTA) or 5 to 6 (pair) stages -> tcgen05.mma 128x256x16 / 256x256x16 -> two 256-column TMEM accumulators
 // per CTA -> tcgen05.ld epilogue overlapped with the next tile.  `accumulate` adds the old contents of C in
 // the epilogue (gradient accumulation over micro-batches without a separate add).
-// The ragged kernel (lb_gemm_ragged, lb_gemm_ragged_wgrad) takes its tiles from device memory.
+// The ragged kernel (lb_gemm_ragged_epi, lb_gemm_ragged_wgrad) takes its tiles from device memory.
 // Every wait is bounded; on expiry the kernel records a status code (lb_gemm_grouped_status),
 // stops issuing work, frees its TMEM and returns.
 #include <cuda.h>
@@ -791,7 +791,7 @@ struct Schedule {
 };
 // Cache of uploaded schedules, keyed by (device, M, N, K, epilogue of every problem).  A training run uses a
 // few dozen shape sets; callers whose row counts change from call to call (expert-parallel MoE)
-// use lb_gemm_ragged instead, which takes the counts from device memory and needs no schedule.
+// use the ragged kernel instead, which takes the counts from device memory and needs no schedule.
 // The cache is still bounded: beyond MAX_SCHEDULES entries the least recently used one is freed.  Entries of the split form are only a number
 // on the host: they have a limit of their own and push out no uploaded schedule, which takes allocations and synchronous copies to make again.
 constexpr int MAX_SCHEDULES = 128, MAX_SPLITS = 512;
@@ -1266,12 +1266,6 @@ extern "C" int lb_gemm_ragged_epi(const void* A, const void* const* B, void* C, 
   rp.tiles_n = (N + BN - 1) / BN; rp.tiles_m_w = 0; rp.num_kb = (K + BK - 1) / BK;
   rp.wait_flag = (const unsigned int*)wait_flag; rp.wait_target = wait_target; rp.wait_ns = g_lb_flag_wait_ns;
   return launch_ragged(ragged_cg(LE, ragged_rows(LE, cap, rows), N, rp.num_kb, lb_num_sms()), !wait_flag, rp, (cudaStream_t)stream);
-}
-
-extern "C" int lb_gemm_ragged(const void* A, const void* const* B, void* C, const void* seg, int LE, int cap, int N, int K,
-                              long long lda, long long ldb, long long ldc, int b_mn, const void* wait_flag,
-                              unsigned int wait_target, void* stream) {
-  return lb_gemm_ragged_epi(A, B, C, seg, LE, cap, 0, N, K, lda, ldb, ldc, b_mn, 0, nullptr, 0, 0, wait_flag, wait_target, stream);
 }
 
 //  Weight gradients: C_e [Nw, Kw] (+)= dY[rows of e, Nw]^T . X[rows of e, Kw]; C: host array of LE

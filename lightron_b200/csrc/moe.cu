@@ -22,8 +22,8 @@
 //                        pass can produce the dot products that are the router-weight gradients
 //   moe_router_bwd_kernel  softmax backward, dx = dlogits . Wg, dWg += dlogits^T x
 //
-// The grouped expert GEMM between push and pull (lb_gemm_ragged, gemm_grouped.cu) takes the segment
-// offsets and counts from device memory and waits for the arrival word itself.
+// The expert GEMMs between push and pull (lb_gemm_ragged_epi, gemm_grouped.cu), whose epilogues are the activation and its backward, take the
+// segment offsets and counts from device memory; the first of each direction waits for the arrival word itself.
 //
 // All waits on a peer are bounded (comm.cuh) and report through lb_moe_status(); row indices are
 // checked against the buffer capacity before every store or load (a routing so skewed that a rank

@@ -76,12 +76,9 @@ _SIGNATURES = {
     "lb_moe_pull": [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, ctypes.c_uint, _P],
     "lb_moe_pull_add": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, ctypes.c_uint, _P],
     "lb_moe_router_bwd": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
-    "lb_gemm_ragged": [_P, _P, _P, _P, _I, _I, _I, _I, _L, _L, _L, _I, _P, ctypes.c_uint, _P],
     "lb_gemm_ragged_epi": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _L, _L, _L, _I, _I, _P, _L, _I, _P, ctypes.c_uint, _P],
     "lb_gemm_ragged_ctas_per_tile": [_I, _I, _I, _I, _I],
     "lb_gemm_ragged_wgrad": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _L, _L, _L, _I, _P],
-    "lb_swiglu_fwd_dev": [_P, _P, _I, _I, _L, _P, _P],
-    "lb_swiglu_bwd_dev": [_P, _P, _P, _I, _I, _L, _P, _P],
     "lb_coll_status": [_P],
     "lb_ulysses_a2a": [_I, _P, _L, _L, _L, _L, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, ctypes.c_uint, _P],
     "lb_cp_dkv_reduce": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, ctypes.c_uint, _P],

@@ -8,13 +8,14 @@ router                 ``lb_moe_router``: gate GEMM + softmax + top-k + per-bloc
 count exchange / plan  ``lb_moe_plan``: counts stored into every peer's table (flag per source),
                        destination rows, 128-row-aligned expert segments, load-balance loss
 dispatch               ``lb_moe_push``: token rows stored straight into the owner's buffer
-expert MLPs            ``lb_gemm_ragged`` (waits for the arrival word itself), SwiGLU, ``lb_gemm_ragged``
+expert MLPs            ``lb_gemm_ragged_epi`` twice: gate | up with SwiGLU in its epilogue (waits for the
+                       arrival word itself), then down
 combine                ``lb_moe_pull``: peer loads + top-k weighted sum + un-permute
 =====================  =====================================================================
 
 and the mirror image in backward (``lb_moe_pull`` with dot products for the routed-weight gradients,
-``lb_moe_push`` of the scaled output gradient, ragged data / weight gradients, ``lb_moe_pull`` of the
-input gradient, ``lb_moe_router_bwd``).  Per-expert token counts exist only in device memory: the
+``lb_moe_push`` of the scaled output gradient, ragged data / weight gradients with SwiGLU's backward in
+an epilogue, ``lb_moe_router_bwd``, ``lb_moe_pull_add`` of the input gradient onto the router's).  Per-expert token counts exist only in device memory: the
 host never waits for them, every tensor on the expert side has the static capacity
 ``ceil(capacity_factor * tokens * top_k)`` rows (+ padding), and the copies a routing sends beyond it
 are dropped (not dispatched, no contribution to the combine), counted in a status word that the
